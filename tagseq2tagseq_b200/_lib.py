@@ -12,6 +12,7 @@ from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_
 from . import build as _build
 
 _LIB = None
+_OPS = None
 
 # name -> (restype, argtypes); must list every symbol include/ts2ts_attn.h and include/ts2ts_lm.h declare
 SYMBOLS = {
@@ -66,6 +67,25 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _LIB = handle
     return _LIB
+
+
+def ops():
+    """``torch.ops.ts2ts``: the operators of libts2ts_torch.so (csrc/torch_ops.cpp)."""
+    global _OPS
+    if _OPS is None:
+        import torch
+        lib()
+        if not os.path.exists(_build.TORCH_LIB):
+            _build.build_library(force=True)
+        torch.ops.load_library(_build.TORCH_LIB)
+        _OPS = torch.ops.ts2ts
+    return _OPS
+
+
+def failed_call(e: RuntimeError) -> RuntimeError:
+    """The exception for a call the library refused: the operators report it as a RuntimeError with the status in its text."""
+    text = str(e).partition("\nException raised from")[0]
+    return Ts2tsError(text) if text.startswith("ts2ts_") and "failed with status" in text else e
 
 
 def check(code: int, what: str) -> None:

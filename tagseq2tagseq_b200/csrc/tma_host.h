@@ -28,6 +28,21 @@ inline EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
+// Encoding a map needs a current context, and a thread that has made no CUDA call yet (an autograd worker, say) has none.
+inline void bind_context() {
+  typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
+  static CtxGetCurrentFn fn = nullptr;
+  if (!fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) return;
+    fn = reinterpret_cast<CtxGetCurrentFn>(p);
+  }
+  CUcontext ctx = nullptr;
+  int dev = 0;
+  if (fn(&ctx) == CUDA_SUCCESS && ctx == nullptr && cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
+}
+
 // Tensor [B,H,T,D] with D contiguous and element strides (sb, sh, st); tile = box_rows tokens x box_cols
 // elements of one (b,h), written to shared memory with the 128-byte swizzle.  `elem_bytes` is 2 (bf16)
 // or 4 (fp32); box_cols * elem_bytes must be 128.  Rows past T read as zero and are not written.
@@ -36,6 +51,7 @@ inline int make_tile_map(CUtensorMap* out, const void* base, int elem_bytes, int
                          int64_t sb, int64_t sh, int64_t st, int box_rows, int box_cols) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return -100;
+  bind_context();
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return -101;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)st * elem_bytes, (cuuint64_t)sh * elem_bytes, (cuuint64_t)sb * elem_bytes};

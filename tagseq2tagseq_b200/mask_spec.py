@@ -57,10 +57,6 @@ class BlockMap(NamedTuple):
     full_q_idx: Optional[torch.Tensor] = None
 
 
-def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
-    return None if t is None else t.data_ptr()
-
-
 def _check_mask_tensors(doc_ids, link_bits, q_row_ids, kv_col_ids):
     if doc_ids.dim() != 2 or doc_ids.dtype != torch.int32:
         raise ValueError("doc_ids must be int32 [B,T]")
@@ -81,30 +77,12 @@ def build_block_map(doc_ids: torch.Tensor, link_bits: Optional[torch.Tensor] = N
                     with_lists: bool = False) -> BlockMap:
     """Run the integer pre-pass (``ts2ts_block_map``) on the current stream."""
     _check_mask_tensors(doc_ids, link_bits, q_row_ids, kv_col_ids)
-    L = _lib.lib()
-    doc_ids = doc_ids.contiguous()
-    link_bits = None if link_bits is None else link_bits.contiguous()
-    q_row_ids = None if q_row_ids is None else q_row_ids.contiguous()
-    kv_col_ids = None if kv_col_ids is None else kv_col_ids.contiguous()
-    B, T = doc_ids.shape
-    if T == 0 or B == 0:
+    if doc_ids.numel() == 0:
         raise ValueError("empty sequence")
-    nb = (T + TILE - 1) // TILE
-    dev = doc_ids.device
-    with torch.cuda.device(dev):
-        plan = torch.empty(L.ts2ts_plan_bytes(B, T), dtype=torch.uint8, device=dev)
-        outs = [None] * 9
-        if with_lists:
-            outs[0] = torch.empty((B, nb, nb), dtype=torch.uint8, device=dev)
-            for i in (1, 3, 5, 7):
-                outs[i] = torch.empty((B, nb), dtype=torch.int32, device=dev)
-                outs[i + 1] = torch.empty((B, nb, nb), dtype=torch.int32, device=dev)
-        R, W = (0, 0) if link_bits is None else (link_bits.shape[1], link_bits.shape[2])
-        code = L.ts2ts_block_map(_ptr(doc_ids), _ptr(q_row_ids), _ptr(kv_col_ids), _ptr(link_bits), B, T, R, W,
-                                 plan.data_ptr(), plan.numel(), *[_ptr(o) for o in outs],
-                                 torch.cuda.current_stream(dev).cuda_stream)
-    _lib.check(code, "ts2ts_block_map")
-    return BlockMap(plan, *outs)
+    try:
+        return BlockMap(*_lib.ops().block_map.default(doc_ids, link_bits, q_row_ids, kv_col_ids, with_lists))
+    except RuntimeError as e:
+        raise _lib.failed_call(e) from None
 
 
 def read_status(plan: torch.Tensor) -> int:

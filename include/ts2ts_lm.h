@@ -54,6 +54,24 @@ int ts2ts_ce_fwd(const void* logits, const int64_t* target, float* lse, float* l
 int ts2ts_ce_bwd(void* logits, const int64_t* target, const float* lse, const float* gscale, float inv_n, int64_t N, int V,
                  void* stream);
 
+/* Loss and gradient in one pass over the logits: loss[N] as ts2ts_ce_fwd gives it, logits overwritten with
+ * (softmax - onehot) * inv_n.  Returns -2 for rows of more than 110592 columns, which do not fit shared memory. */
+int ts2ts_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float inv_n, int64_t N, int V, void* stream);
+/* x[n] (fp32) *= gscale[0] in place when out == NULL (no traffic when the device scalar is one); otherwise out[n] (bf16)
+ * = x[n] * gscale[0], n a multiple of 8. */
+int ts2ts_scale(float* x, void* out, const float* gscale, int64_t n, void* stream);
+
+/* dw[V,C] (fp32, overwritten) = the sum of the rows dx[N,C] (fp32) of equal idx[N] (int64; an index outside 0..V-1 is
+ * ignored).  C % 4 == 0.  The order of the additions is not fixed. */
+int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, void* stream);
+
+/* One AdamW step over `count` fp32 tensors.  p, g, m, v: host arrays of device pointers (parameter, gradient, first and
+ * second moment); n: host array of element counts; steps: host array, the number of this step per tensor (from 1).
+ *   p <- p (1 - lr wd);  m <- b1 m + (1 - b1) g;  v <- b2 v + (1 - b2) g^2;
+ *   p <- p - lr / (1 - b1^t) m / (sqrt(v / (1 - b2^t)) + eps) */
+int ts2ts_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,
+                const float* steps, double lr, double beta1, double beta2, double eps, double weight_decay, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

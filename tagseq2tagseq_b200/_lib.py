@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p, POINTER
+from ctypes import c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p, POINTER
 
 from . import build as _build
 
@@ -47,6 +47,10 @@ SYMBOLS = {
     "ts2ts_swiglu_bwd": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_void_p]),
     "ts2ts_ce_fwd": (c_int, [c_void_p] * 4 + [c_int64, c_int, c_void_p]),
     "ts2ts_ce_bwd": (c_int, [c_void_p] * 4 + [c_float, c_int64, c_int, c_void_p]),
+    "ts2ts_ce_fwd_grad": (c_int, [c_void_p] * 3 + [c_float, c_int64, c_int, c_void_p]),
+    "ts2ts_scale": (c_int, [c_void_p] * 3 + [c_int64, c_void_p]),
+    "ts2ts_embedding_bwd": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_void_p]),
+    "ts2ts_adamw": (c_int, [c_int] + [c_void_p] * 6 + [c_double] * 5 + [c_void_p]),
 }
 
 

@@ -36,6 +36,11 @@ cudaError_t launch_swiglu_bwd(const void* gu, const void* dact, void* dgu, int64
 cudaError_t launch_ce_fwd(const void* logits, const int64_t* target, float* lse, float* loss, int N, int V, cudaStream_t stream);
 cudaError_t launch_ce_bwd(void* logits, const int64_t* target, const float* lse, const float* gscale, float inv_n, int N, int V,
                           cudaStream_t stream);
+int launch_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float inv_n, int N, int V, cudaStream_t stream);
+cudaError_t launch_scale(float* x, void* out_bf16, const float* gscale, int64_t n, cudaStream_t stream);
+cudaError_t launch_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, cudaStream_t stream);
+cudaError_t launch_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,
+                         const float* steps, double lr, double beta1, double beta2, double eps, double weight_decay, cudaStream_t stream);
 size_t decode_workspace_bytes(int B, int H, int Tk, int D);
 int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq, const int64_t* sk, const int64_t* sv, int B, int H,
                   int Tk, int D, float scale, MaskArgs M, const int32_t* q_pos, void* out, const int64_t* so, float* lse,
@@ -399,4 +404,43 @@ int ts2ts_ce_bwd(void* logits, const int64_t* target, const float* lse, const fl
   if (!logits || !target || !lse || !gscale) return fail(-3, "ce_bwd: null pointer");
   if (!aligned(logits, 16)) return fail(-5, "ce_bwd: misaligned pointer");
   return launched(launch_ce_bwd(logits, target, lse, gscale, inv_n, (int)N, V, static_cast<cudaStream_t>(stream)), "ce_bwd");
+}
+
+int ts2ts_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float inv_n, int64_t N, int V, void* stream) {
+  int r;
+  if ((r = check_rows(N))) return r;
+  if (V < 8 || V % 8) return fail(-2, "V must be a positive multiple of 8 (got %d)", V);
+  if (!logits || !target || !loss) return fail(-3, "ce_fwd_grad: null pointer");
+  if (!aligned(logits, 16)) return fail(-5, "ce_fwd_grad: misaligned pointer");
+  r = launch_ce_fwd_grad(logits, target, loss, inv_n, (int)N, V, static_cast<cudaStream_t>(stream));
+  if (r == -1000) return fail(-2, "V = %d does not fit shared memory", V);
+  return r ? fail(r, "ce_fwd_grad launch failed: %s", cudaGetErrorString(cudaPeekAtLastError())) : 0;
+}
+
+int ts2ts_scale(float* x, void* out, const float* gscale, int64_t n, void* stream) {
+  if (n <= 0 || n > (int64_t(1) << 40)) return fail(-1, "n must be in 1..2^40 (got %lld)", (long long)n);
+  if (!x || !gscale) return fail(-3, "scale: null pointer");
+  if (out && n % 8) return fail(-2, "n must be a multiple of 8 (got %lld)", (long long)n);
+  if (!aligned(x, 16) || (out && !aligned(out, 16))) return fail(-5, "scale: misaligned pointer");
+  return launched(launch_scale(x, out, gscale, n, static_cast<cudaStream_t>(stream)), "scale");
+}
+
+int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, void* stream) {
+  int r;
+  if ((r = check_rows(N))) return r;
+  if (C < 4 || C % 4 || V <= 0) return fail(-2, "C must be a positive multiple of 4 and V positive (got %d, %lld)", C, (long long)V);
+  if (!idx || !dx || !dw) return fail(-3, "embedding_bwd: null pointer");
+  if (!aligned(dx, 16) || !aligned(dw, 16)) return fail(-5, "embedding_bwd: misaligned pointer");
+  return launched(launch_embedding_bwd(idx, dx, dw, N, C, V, static_cast<cudaStream_t>(stream)), "embedding_bwd");
+}
+
+int ts2ts_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,
+                const float* steps, double lr, double beta1, double beta2, double eps, double weight_decay, void* stream) {
+  if (count < 0) return fail(-1, "count must not be negative");
+  if (count > 0 && (!p || !g || !m || !v || !n || !steps)) return fail(-3, "adamw: null pointer");
+  for (int i = 0; i < count; ++i) {
+    if (n[i] < 0 || (n[i] > 0 && (!p[i] || !g[i] || !m[i] || !v[i]))) return fail(-3, "adamw: tensor %d has a null pointer or a negative size", i);
+    if (!(steps[i] >= 1.f)) return fail(-8, "adamw: steps count from 1");
+  }
+  return launched(launch_adamw(count, p, g, m, v, n, steps, lr, beta1, beta2, eps, weight_decay, static_cast<cudaStream_t>(stream)), "adamw");
 }

@@ -6,8 +6,11 @@
 // the GEMMs rather than chains of element-wise launches.  All arithmetic is fp32; bf16 only in memory.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <math_constants.h>
 #include <stdint.h>
+
+#include "ptx.cuh"
 
 namespace ts2ts {
 namespace {
@@ -115,11 +118,17 @@ __global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x_in, const __n
 // d(x_out) is the gradient of both x_in and a (written in fp32 and, when da is given, in bf16).  Blocks walk the rows
 // with a stride, keep their share of dw in registers and write it to row blockIdx.x of dw_part [gridDim.x, C] at the
 // end (atomics on the C addresses of one dw vector serialise a thousand blocks); a second kernel adds the rows up.
-template <int NV>
-__global__ void add_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const float* __restrict__ dx_up, const float* __restrict__ x,
-                                       const float* __restrict__ w, const float* __restrict__ rstd, float* __restrict__ dx,
-                                       __nv_bfloat16* __restrict__ da, float* __restrict__ dw_part, int N, int C) {
-  __shared__ float red[32];
+//
+// HBM-bound, 16 bytes per element: every load of an iteration is issued before its reduction, kRows rows at a time, and
+// the reduction's scratch alternates so that one barrier per iteration suffices.  With one row in flight and the load of
+// dx_up behind the reduction it ran at 62 % of the copy rate (47 us at 16384 x 768, 268 us at 32768 x 2048).
+template <int NV, int kRows>
+__global__ void __launch_bounds__(1024) add_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const float* __restrict__ dx_up,
+                                                               const float* __restrict__ x, const float* __restrict__ w,
+                                                               const float* __restrict__ rstd, float* __restrict__ dx,
+                                                               __nv_bfloat16* __restrict__ da, float* __restrict__ dw_part, int N, int C) {
+  __shared__ float red[2][kRows][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float4 wv[NV], acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -127,36 +136,59 @@ __global__ void add_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dh, con
     wv[i] = c < C ? *reinterpret_cast<const float4*>(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for (int row = blockIdx.x; row < N; row += gridDim.x) {
-    const size_t base = (size_t)row * C;
-    const float r = rstd[row];
-    float4 xh[NV], g[NV];
-    float dot = 0.f;
+  int buf = 0;
+  for (int row0 = blockIdx.x; row0 < N; row0 += kRows * gridDim.x, buf ^= 1) {
+    float4 xh[kRows][NV], g[kRows][NV], up[kRows][NV];
+    float rs[kRows], dot[kRows];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = (threadIdx.x + i * blockDim.x) * 4;
-      if (c < C) {
-        const float4 xv = *reinterpret_cast<const float4*>(x + base + c);
-        const float4 d = bf16x4_to_float4(*reinterpret_cast<const uint2*>(dh + base + c));
-        xh[i] = make_float4(xv.x * r, xv.y * r, xv.z * r, xv.w * r);
-        g[i] = make_float4(d.x * wv[i].x, d.y * wv[i].y, d.z * wv[i].z, d.w * wv[i].w);
-        dot += g[i].x * xh[i].x + g[i].y * xh[i].y + g[i].z * xh[i].z + g[i].w * xh[i].w;
-        acc[i].x += d.x * xh[i].x; acc[i].y += d.y * xh[i].y; acc[i].z += d.z * xh[i].z; acc[i].w += d.w * xh[i].w;
+    for (int k = 0; k < kRows; ++k) {
+      const int row = row0 + k * gridDim.x;
+      rs[k] = row < N ? rstd[row] : 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = (threadIdx.x + i * blockDim.x) * 4;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        xh[k][i] = zero; g[k][i] = zero; up[k][i] = zero;
+        if (c < C && row < N) {
+          const size_t at = (size_t)row * C + c;
+          xh[k][i] = *reinterpret_cast<const float4*>(x + at);
+          g[k][i] = bf16x4_to_float4(*reinterpret_cast<const uint2*>(dh + at));
+          if (dx_up != nullptr) up[k][i] = *reinterpret_cast<const float4*>(dx_up + at);
+        }
       }
     }
-    dot = block_sum(dot, red) / (float)C;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = (threadIdx.x + i * blockDim.x) * 4;
-      if (c < C) {
-        float4 o = make_float4(r * (g[i].x - xh[i].x * dot), r * (g[i].y - xh[i].y * dot), r * (g[i].z - xh[i].z * dot),
-                               r * (g[i].w - xh[i].w * dot));
-        if (dx_up != nullptr) {
-          const float4 u = *reinterpret_cast<const float4*>(dx_up + base + c);
-          o.x += u.x; o.y += u.y; o.z += u.z; o.w += u.w;
+    for (int k = 0; k < kRows; ++k) {
+      dot[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        float4& h = xh[k][i];
+        float4& d = g[k][i];
+        h.x *= rs[k]; h.y *= rs[k]; h.z *= rs[k]; h.w *= rs[k];
+        acc[i].x += d.x * h.x; acc[i].y += d.y * h.y; acc[i].z += d.z * h.z; acc[i].w += d.w * h.w;
+        d.x *= wv[i].x; d.y *= wv[i].y; d.z *= wv[i].z; d.w *= wv[i].w;
+        dot[k] += d.x * h.x + d.y * h.y + d.z * h.z + d.w * h.w;
+      }
+      dot[k] = warp_sum(dot[k]);
+      if (lane == 0) red[buf][k][warp] = dot[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int row = row0 + k * gridDim.x;
+      dot[k] = warp_sum(lane < nw ? red[buf][k][lane] : 0.f) / (float)C;
+      if (row >= N) continue;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = (threadIdx.x + i * blockDim.x) * 4;
+        if (c < C) {
+          const size_t at = (size_t)row * C + c;
+          const float4 h = xh[k][i], d = g[k][i], u = up[k][i];
+          const float4 o = make_float4(rs[k] * (d.x - h.x * dot[k]) + u.x, rs[k] * (d.y - h.y * dot[k]) + u.y,
+                                       rs[k] * (d.z - h.z * dot[k]) + u.z, rs[k] * (d.w - h.w * dot[k]) + u.w);
+          *reinterpret_cast<float4*>(dx + at) = o;
+          if (da != nullptr) *reinterpret_cast<uint2*>(da + at) = float4_to_bf16x4(o);
         }
-        *reinterpret_cast<float4*>(dx + base + c) = o;
-        if (da != nullptr) *reinterpret_cast<uint2*>(da + base + c) = float4_to_bf16x4(o);
       }
     }
   }
@@ -166,20 +198,37 @@ __global__ void add_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dh, con
     if (c < C) *reinterpret_cast<float4*>(dw_part + (size_t)blockIdx.x * C + c) = acc[i];
   }
 }
-// dw[c] += sum over the rows of dw_part[rows, C].
-__global__ void column_sum_kernel(const float* __restrict__ part, float* dw, int rows, int C) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  int r = 0;
-  for (; r + 3 < rows; r += 4) {
-    s0 += part[(size_t)r * C + c];
-    s1 += part[(size_t)(r + 1) * C + c];
-    s2 += part[(size_t)(r + 2) * C + c];
-    s3 += part[(size_t)(r + 3) * C + c];
+// dw[c] += sum over the rows of dw_part[rows, C].  A block owns 32 columns: eight lanes of a warp read one row's 128
+// bytes, so that 128 rows are in flight per block; one thread per column was a serial chain of loads (66 us per call at
+// 1480 x 768, more than the kernel whose partial sums it adds).
+__global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ part, float* dw, int rows, int C) {
+  __shared__ float4 red[32][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
+  const int c = blockIdx.x * 32 + sub * 4;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < C) {
+#pragma unroll 4
+    for (int r = warp * 4 + (lane >> 3); r < rows; r += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(part + (size_t)r * C + c);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
   }
-  for (; r < rows; ++r) s0 += part[(size_t)r * C + c];
-  dw[c] += (s0 + s1) + (s2 + s3);
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+    s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+  }
+  if (lane < 8) red[warp][lane] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {  // thread = column
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t += reinterpret_cast<const float*>(red[i])[threadIdx.x];
+    const int col = blockIdx.x * 32 + threadIdx.x;
+    if (col < C) dw[col] += t;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------- rotary embedding
@@ -302,6 +351,186 @@ __global__ void ce_bwd_kernel(__nv_bfloat16* logits, const int64_t* __restrict__
   }
 }
 
+// Loss and gradient of a row in one pass: the row (at most kCeRowBytes) is brought into shared memory once, read there
+// for the log-sum-exp and again for the gradient, which is written over the logits.  HBM-bound, 4 bytes per logit
+// instead of the 6 of the two kernels above; two blocks of a 50304-logit row share an SM, so that one's copy overlaps the
+// other's arithmetic.  The gradient is that of the mean loss (times inv_n, not times what reaches the loss from above).
+constexpr int kCeThreads = 512, kCeChunks = 4, kCeRowBytes = 216 * 1024;
+__global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* logits, const int64_t* __restrict__ target,
+                                                                 float* __restrict__ loss, float inv_n, int V) {
+  extern __shared__ __align__(128) uint8_t ce_row[];
+  __shared__ __align__(8) uint64_t bars[kCeChunks];
+  __shared__ float red_m[kCeThreads / 32], red_s[kCeThreads / 32];
+  __shared__ int late;
+  __nv_bfloat16* row = logits + (size_t)blockIdx.x * V;
+  const int n_vec = V / 8, per_chunk = (n_vec + kCeChunks - 1) / kCeChunks;  // in 16-byte vectors
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    late = 0;
+    for (int k = 0; k < kCeChunks; ++k) mbar_init(&bars[k], 1);
+    fence_mbar_init();
+    for (int k = 0; k < kCeChunks; ++k) {
+      const int first = min(k * per_chunk, n_vec), count = min(per_chunk, n_vec - first);
+      mbar_expect_tx(&bars[k], count * 16);
+      if (count > 0) bulk_load(ce_row + first * 16, row + first * 8, count * 16, &bars[k]);
+    }
+  }
+  const int64_t tg = target[blockIdx.x];
+  const bool live = tg >= 0 && tg < V;
+  __syncthreads();
+  const uint4* sv = reinterpret_cast<const uint4*>(ce_row);
+  float m = -CUDART_INF_F, s = 0.f;
+  bool ok = true;
+  for (int k = 0; k < kCeChunks; ++k) {
+    ok = ok && mbar_wait(&bars[k], 0, &late, 1);
+    if (!ok) break;
+    const int end = min((k + 1) * per_chunk, n_vec);
+    for (int c = k * per_chunk + tid; c < end; c += kCeThreads) {
+      float f[8];
+      bf16x8_to_float(sv[c], f);
+      float mx = f[0];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) mx = fmaxf(mx, f[i]);
+      const float m_new = fmaxf(m, mx);
+      if (m_new == -CUDART_INF_F) continue;
+      float add = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) add += __expf(f[i] - m_new);
+      s = s * __expf(m - m_new) + add;
+      m = m_new;
+    }
+  }
+  const float wm = warp_max(m);
+  s = warp_sum(m == -CUDART_INF_F ? 0.f : s * __expf(m - wm));
+  if (lane == 0) { red_m[warp] = wm; red_s[warp] = s; }
+  __syncthreads();
+  const float pm = lane < kCeThreads / 32 ? red_m[lane] : -CUDART_INF_F;
+  const float m_all = warp_max(pm);
+  const float s_all = warp_sum(pm == -CUDART_INF_F ? 0.f : red_s[lane] * __expf(pm - m_all));
+  const float l = m_all + logf(s_all);
+  const float hit = live ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(ce_row)[tg]) : 0.f;
+  if (tid == 0) loss[blockIdx.x] = !ok ? CUDART_NAN_F : live ? l - hit : 0.f;  // a copy that never came shows as a loss that is no number
+  if (!ok) {  // let the copy land before the block's shared memory is released
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    return;
+  }
+  const float g = live ? inv_n : 0.f;
+  for (int c = tid; c < n_vec; c += kCeThreads) {
+    float f[8];
+    bf16x8_to_float(sv[c], f);
+    const int64_t first = (int64_t)c * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (__expf(f[i] - l) - (first + i == tg ? 1.f : 0.f)) * g;
+    reinterpret_cast<uint4*>(row)[c] = float_to_bf16x8(f);
+  }
+}
+
+// x *= gscale[0], and out = bf16(x * gscale[0]).  The first does nothing when the factor is one, which it is unless the
+// caller scaled the loss.
+__global__ void __launch_bounds__(256) scale_f32_kernel(float* x, const float* __restrict__ gscale, int64_t n) {
+  const float g = gscale[0];
+  if (g == 1.f) return;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] *= g;
+}
+__global__ void __launch_bounds__(256) scale_to_bf16_kernel(const float* __restrict__ x, const float* __restrict__ gscale,
+                                                            __nv_bfloat16* __restrict__ out, int64_t n_vec) {
+  const float g = gscale[0];
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_vec) return;
+  float f[8];
+  *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(x)[2 * i];
+  *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(x)[2 * i + 1];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) f[k] *= g;
+  reinterpret_cast<uint4*>(out)[i] = float_to_bf16x8(f);
+}
+
+// ---------------------------------------------------------------------------------------------- embedding
+// dw[idx[n]] += dx[n] for every token: one warp per row, 16-byte reductions in L2.  HBM-bound (dx is read once, the
+// touched rows of the zeroed dw are written back once); sorting the tokens first, as the stock kernel does to add equal
+// ones up in order, took 290 us at 16384 x 768 and 1.4 ms at 32768 x 2048.
+__global__ void __launch_bounds__(256) embedding_bwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ dx, float* dw, int64_t N,
+                                                            int C, int64_t V) {
+  const int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (n >= N) return;
+  const int64_t v = idx[n];
+  if (v < 0 || v >= V) return;
+  const float4* src = reinterpret_cast<const float4*>(dx + n * C);
+  float4* dst = reinterpret_cast<float4*>(dw + v * C);
+#pragma unroll 4
+  for (int c = threadIdx.x & 31; c < C / 4; c += 32) atomicAdd(dst + c, src[c]);
+}
+
+// ---------------------------------------------------------------------------------------------- AdamW
+// One decoupled-weight-decay Adam step over many tensors per launch.  HBM-bound: 28 bytes per parameter.  A block owns
+// kAdamChunk consecutive elements of one tensor and keeps two 16-byte vectors of each of the four arrays in flight per
+// thread and step.
+constexpr int kAdamTensors = 64, kAdamThreads = 256, kAdamChunk = 8192;
+struct AdamTensor {
+  float* p;
+  const float* g;
+  float *m, *v;
+  int64_t n;
+  int first_block;
+  float step_size, inv_sqrt_bc2;  // lr / (1 - beta1^t), 1 / sqrt(1 - beta2^t)
+};
+struct AdamArgs {
+  AdamTensor t[kAdamTensors];
+  int count;
+  float decay, beta1, beta2, rest1, rest2, eps;  // decay = 1 - lr * weight_decay, rest = 1 - beta
+};
+__device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, const AdamArgs& a, const AdamTensor& t) {
+  p *= a.decay;
+  m = a.beta1 * m + a.rest1 * g;
+  v = a.beta2 * v + a.rest2 * g * g;
+  p -= t.step_size * m / (sqrtf(v) * t.inv_sqrt_bc2 + a.eps);
+}
+__global__ void __launch_bounds__(kAdamThreads) adamw_kernel(const __grid_constant__ AdamArgs a) {
+  int lo = 0, hi = a.count - 1;  // last tensor whose first block is not after this one
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.t[mid].first_block <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const AdamTensor& t = a.t[lo];
+  const int64_t begin = (int64_t)((int)blockIdx.x - t.first_block) * kAdamChunk;
+  const int64_t end = min(begin + (int64_t)kAdamChunk, t.n);
+  const bool vec = ((reinterpret_cast<uintptr_t>(t.p) | reinterpret_cast<uintptr_t>(t.g) | reinterpret_cast<uintptr_t>(t.m) |
+                     reinterpret_cast<uintptr_t>(t.v)) & 15u) == 0;
+  int64_t i = begin;
+  if (vec) {
+    const int64_t vend = begin + (end - begin) / 4 * 4;
+    for (int64_t j = begin + 4 * threadIdx.x; j < vend; j += 8 * kAdamThreads) {
+      const int64_t j2 = j + 4 * kAdamThreads;
+      const bool two = j2 < vend;
+      float4 p[2], g[2], m[2], v[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int64_t at = k == 0 || !two ? j : j2;
+        p[k] = *reinterpret_cast<const float4*>(t.p + at); g[k] = __ldcs(reinterpret_cast<const float4*>(t.g + at));
+        m[k] = *reinterpret_cast<const float4*>(t.m + at); v[k] = *reinterpret_cast<const float4*>(t.v + at);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !two) break;
+        adam_one(p[k].x, g[k].x, m[k].x, v[k].x, a, t);
+        adam_one(p[k].y, g[k].y, m[k].y, v[k].y, a, t);
+        adam_one(p[k].z, g[k].z, m[k].z, v[k].z, a, t);
+        adam_one(p[k].w, g[k].w, m[k].w, v[k].w, a, t);
+        const int64_t at = k == 0 ? j : j2;
+        *reinterpret_cast<float4*>(t.p + at) = p[k];
+        *reinterpret_cast<float4*>(t.m + at) = m[k];
+        *reinterpret_cast<float4*>(t.v + at) = v[k];
+      }
+    }
+    i = vend;
+  }
+  for (i += threadIdx.x; i < end; i += kAdamThreads) {
+    float p = t.p[i], m = t.m[i], v = t.v[i];
+    adam_one(p, t.g[i], m, v, a, t);
+    t.p[i] = p; t.m[i] = m; t.v[i] = v;
+  }
+}
+
 int norm_threads(int C) {
   int t = (C / 4 + kMaxVec - 1) / kMaxVec;  // threads needed with kMaxVec float4 each
   t = ((t + 31) / 32) * 32;
@@ -333,24 +562,26 @@ int add_rmsnorm_bwd_blocks(int64_t N, int C) {
     sms = n;
   }
   const int threads = norm_threads(C);
-  const int per_sm = 2048 / threads;  // as many resident blocks as the thread limit allows
+  const int per_sm = threads >= 1024 ? 1 : 1024 / threads;  // resident blocks at up to 64 registers a thread
   const int64_t cap = (int64_t)sms * per_sm;
-  return (int)(N < cap ? N : cap);
+  int64_t want = (N + 3) / 4;  // four rows a block or more, once every SM has two: its partial dw row costs traffic of its own
+  if (want < 2 * sms) want = N < 2 * sms ? N : 2 * sms;
+  return (int)(want < cap ? want : cap);
 }
 
 cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx,
                                    void* da, float* dw, float* dw_part, int N, int C, cudaStream_t stream) {
   const int grid = add_rmsnorm_bwd_blocks(N, C);
   const int threads = norm_threads(C);
+  const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(dh);
+  __nv_bfloat16* a = static_cast<__nv_bfloat16*>(da);
   if (C <= 4 * threads)
-    add_rmsnorm_bwd_kernel<1><<<grid, threads, 0, stream>>>(static_cast<const __nv_bfloat16*>(dh), dx_up, x, w, rstd, dx,
-                                                            static_cast<__nv_bfloat16*>(da), dw_part, N, C);
+    add_rmsnorm_bwd_kernel<1, 2><<<grid, threads, 0, stream>>>(g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
   else
-    add_rmsnorm_bwd_kernel<kMaxVec><<<grid, threads, 0, stream>>>(static_cast<const __nv_bfloat16*>(dh), dx_up, x, w, rstd, dx,
-                                                                  static_cast<__nv_bfloat16*>(da), dw_part, N, C);
+    add_rmsnorm_bwd_kernel<kMaxVec, 1><<<grid, threads, 0, stream>>>(g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  column_sum_kernel<<<(C + 127) / 128, 128, 0, stream>>>(dw_part, dw, grid, C);
+  column_sum_kernel<<<(C + 31) / 32, 1024, 0, stream>>>(dw_part, dw, grid, C);
   return cudaGetLastError();
 }
 
@@ -385,6 +616,65 @@ cudaError_t launch_ce_fwd(const void* logits, const int64_t* target, float* lse,
 cudaError_t launch_ce_bwd(void* logits, const int64_t* target, const float* lse, const float* gscale, float inv_n, int N, int V,
                           cudaStream_t stream) {
   ce_bwd_kernel<<<N, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(logits), target, lse, gscale, inv_n, V);
+  return cudaGetLastError();
+}
+
+// -1000: the row does not fit shared memory (the caller takes the two-kernel path).
+int launch_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float inv_n, int N, int V, cudaStream_t stream) {
+  const int bytes = 2 * V;
+  if (bytes > kCeRowBytes) return -1000;
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return -50;
+  if (!attr_done[dev]) {
+    if (cudaFuncSetAttribute(ce_fwd_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeRowBytes) != cudaSuccess) return -50;
+    attr_done[dev] = true;
+  }
+  ce_fwd_grad_kernel<<<N, kCeThreads, bytes, stream>>>(static_cast<__nv_bfloat16*>(logits), target, loss, inv_n, V);
+  return cudaGetLastError() == cudaSuccess ? 0 : -50;
+}
+
+cudaError_t launch_scale(float* x, void* out_bf16, const float* gscale, int64_t n, cudaStream_t stream) {
+  if (out_bf16 == nullptr) {
+    const int64_t blocks = (n + 1023) / 1024;
+    scale_f32_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, stream>>>(x, gscale, n);
+  } else {
+    scale_to_bf16_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, stream>>>(x, gscale, static_cast<__nv_bfloat16*>(out_bf16), n / 8);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(dw, 0, (size_t)V * C * sizeof(float), stream);
+  if (e != cudaSuccess) return e;
+  embedding_bwd_kernel<<<(unsigned)((N + 7) / 8), 256, 0, stream>>>(idx, dx, dw, N, C, V);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,
+                         const float* steps, double lr, double beta1, double beta2, double eps, double weight_decay, cudaStream_t stream) {
+  AdamArgs a;
+  a.decay = (float)(1.0 - lr * weight_decay); a.beta1 = (float)beta1; a.beta2 = (float)beta2; a.eps = (float)eps;
+  a.rest1 = (float)(1.0 - beta1); a.rest2 = (float)(1.0 - beta2);
+  for (int done = 0; done < count;) {
+    int64_t blocks = 0;
+    a.count = 0;
+    while (done < count && a.count < kAdamTensors) {
+      const int64_t need = (n[done] + kAdamChunk - 1) / kAdamChunk;
+      if (a.count > 0 && blocks + need > 0x7fffffff) break;
+      if (need > 0) {
+        AdamTensor& t = a.t[a.count++];
+        t.p = p[done]; t.g = g[done]; t.m = m[done]; t.v = v[done]; t.n = n[done];
+        t.first_block = (int)blocks;
+        t.step_size = (float)(lr / (1.0 - pow(beta1, (double)steps[done])));
+        t.inv_sqrt_bc2 = (float)(1.0 / sqrt(1.0 - pow(beta2, (double)steps[done])));
+        blocks += need;
+      }
+      ++done;
+    }
+    if (blocks > 0) adamw_kernel<<<(unsigned)blocks, kAdamThreads, 0, stream>>>(a);
+  }
   return cudaGetLastError();
 }
 

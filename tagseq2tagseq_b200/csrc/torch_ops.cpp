@@ -14,6 +14,7 @@
 #include <torch/library.h>
 
 #include <array>
+#include <cmath>
 #include <tuple>
 #include <vector>
 
@@ -211,6 +212,290 @@ std::vector<Tensor> block_map_cuda(const Tensor& doc_ids, const OptTensor& link_
   return r;
 }
 
+// ------------------------------------------------------------------------------------------------ decoder layer
+// Autograd functions around the decoder-layer entry points.  Gradients nobody asked for arrive undefined
+// (set_materialize_grads(false)) instead of as zero tensors of the activation's size.
+using c10::cuda::CUDAGuard;
+
+void need_cuda(const Tensor& t) {
+  TORCH_CHECK(t.is_cuda(), "the decoder-layer kernels run on CUDA tensors only (no CPU path exists)");
+}
+const float* fptr(const Tensor& t) { return t.const_data_ptr<float>(); }
+float* mfptr(const Tensor& t) { return t.mutable_data_ptr<float>(); }
+
+struct AddRMSNorm : torch::autograd::Function<AddRMSNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const OptTensor& a_in, const Tensor& w, double eps) {
+    need_cuda(x_in);
+    TORCH_CHECK_TYPE(x_in.scalar_type() == at::kFloat && w.scalar_type() == at::kFloat && (!a_in.has_value() || a_in->scalar_type() == at::kBFloat16),
+                     "add_rmsnorm: x and w are fp32, a is bf16");
+    at::AutoDispatchBelowADInplaceOrView below;
+    const CUDAGuard guard(x_in.device());
+    const Tensor x = x_in.contiguous(), a = a_in.has_value() ? a_in->contiguous() : Tensor();
+    const int64_t C = x.size(-1), N = x.numel() / C;
+    Tensor x_out = at::empty_like(x), h = at::empty(x.sizes(), x.options().dtype(at::kBFloat16)), rstd = at::empty({N}, x.options());
+    check(ts2ts_add_rmsnorm_fwd(fptr(x), a.defined() ? a.const_data_ptr() : nullptr, fptr(w), mfptr(x_out), h.mutable_data_ptr(), mfptr(rstd),
+                                N, static_cast<int>(C), static_cast<float>(eps), stream_of(x)),
+          "ts2ts_add_rmsnorm_fwd");
+    ctx->save_for_backward({x_out, w, rstd});
+    ctx->saved_data["has_a"] = a.defined();
+    ctx->set_materialize_grads(false);
+    return {x_out, h};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &w = s[1], &rstd = s[2];
+    const CUDAGuard guard(x.device());
+    const int64_t C = x.size(-1), N = x.numel() / C;
+    const bool has_a = ctx->saved_data["has_a"].toBool();
+    const auto bf16 = x.options().dtype(at::kBFloat16);
+    const Tensor dh = grads[1].defined() ? grads[1].contiguous() : at::zeros(x.sizes(), bf16);  // h had no user
+    const Tensor up = grads[0].defined() ? grads[0].contiguous() : Tensor();
+    Tensor dx = at::empty_like(x), da = has_a ? at::empty(x.sizes(), bf16) : Tensor(), dw = at::zeros_like(w);
+    Tensor ws = at::empty({static_cast<int64_t>(ts2ts_add_rmsnorm_bwd_workspace_bytes(N, static_cast<int>(C)))}, x.options().dtype(at::kByte));
+    check(ts2ts_add_rmsnorm_bwd(dh.const_data_ptr(), up.defined() ? fptr(up) : nullptr, fptr(x), fptr(w), fptr(rstd), mfptr(dx),
+                                has_a ? da.mutable_data_ptr() : nullptr, mfptr(dw), ws.mutable_data_ptr(), ws.numel(), N, static_cast<int>(C),
+                                stream_of(x)),
+          "ts2ts_add_rmsnorm_bwd");
+    return {dx, da, dw, Tensor()};
+  }
+};
+std::tuple<Tensor, Tensor> add_rmsnorm(const Tensor& x, const OptTensor& a, const Tensor& w, double eps) {
+  auto r = AddRMSNorm::apply(x, a, w, eps);
+  return {r[0], r[1]};
+}
+
+// Element strides (batch, head, token) of q, k or v inside a packed [B,T,3,H,D] buffer, and of a [B,T,H,D] one.
+struct PackedStrides {
+  int64_t s[3];
+  PackedStrides(int64_t T, int64_t parts, int64_t H, int64_t D) : s{T * parts * H * D, D, parts * H * D} {}
+};
+
+// qkv [B,T,3*H*D] (the fused projection's output) -> attention output [B,T,H*D].  q and k are rotated in place; the
+// attention kernels read q, k, v and write the output, and later dq, dk, dv, through strides of the packed buffers, so no
+// tensor is transposed, split or concatenated in memory.
+struct QKVAttention : torch::autograd::Function<QKVAttention> {
+  static variable_list forward(AutogradContext* ctx, Tensor qkv, const Tensor& cos, const Tensor& sin, const Tensor& doc_ids,
+                               const OptTensor& link_bits, const OptTensor& q_row_ids, const OptTensor& kv_col_ids, const Tensor& plan,
+                               int64_t n_heads, int64_t head_dim) {
+    need_cuda(qkv);
+    TORCH_CHECK_TYPE(qkv.scalar_type() == at::kBFloat16 && qkv.is_contiguous(), "qkv_attention: qkv must be a contiguous bf16 tensor");
+    TORCH_CHECK_VALUE(qkv.dim() == 3 && qkv.size(2) == 3 * n_heads * head_dim, "qkv_attention: last dimension must be 3 * n_heads * head_dim");
+    at::AutoDispatchBelowADInplaceOrView below;
+    const CUDAGuard guard(qkv.device());
+    const int B = qkv.size(0), T = qkv.size(1), H = n_heads, D = head_dim;
+    void* stream = stream_of(qkv);
+    check(ts2ts_rope_qk_inplace(qkv.mutable_data_ptr(), fptr(cos), fptr(sin), B, T, H, D, 1.f, stream), "ts2ts_rope_qk_inplace");
+    ctx->mark_dirty({qkv});
+    Tensor out = at::empty({B, T, n_heads * head_dim}, qkv.options()), lse = at::empty({B, H, T}, qkv.options().dtype(at::kFloat));
+    const PackedStrides in(T, 3, H, D), os(T, 1, H, D);
+    const char* base = static_cast<const char*>(qkv.const_data_ptr());
+    const int64_t part = 2 * n_heads * head_dim;  // bytes from q to k to v of a token
+    const float scale = 1.f / std::sqrt(static_cast<float>(D));
+    const MaskPtrs m(doc_ids, link_bits, q_row_ids, kv_col_ids);
+    check(ts2ts_attn_fwd(base, base + part, base + 2 * part, in.s, in.s, in.s, B, H, T, D, scale, m.doc, m.row, m.col, m.link, m.R, m.W,
+                         plan.const_data_ptr(), plan.numel(), out.mutable_data_ptr(), os.s, mfptr(lse), stream),
+          "ts2ts_attn_fwd");
+    ctx->save_for_backward({qkv, out, lse, cos, sin, doc_ids, link_bits.value_or(Tensor()), q_row_ids.value_or(Tensor()),
+                            kv_col_ids.value_or(Tensor()), plan});
+    ctx->saved_data["H"] = n_heads;
+    ctx->set_materialize_grads(false);
+    return {out, qkv};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list r(10);
+    if (!grads[0].defined()) return r;
+    const auto s = ctx->get_saved_variables();
+    const Tensor &qkv = s[0], &out = s[1], &lse = s[2], &cos = s[3], &sin = s[4], &plan = s[9];
+    const CUDAGuard guard(qkv.device());
+    const int64_t n_heads = ctx->saved_data["H"].toInt(), head_dim = qkv.size(2) / (3 * n_heads);
+    const int B = qkv.size(0), T = qkv.size(1), H = n_heads, D = head_dim;
+    void* stream = stream_of(qkv);
+    const Tensor dout = grads[0].contiguous();
+    Tensor dqkv = at::empty_like(qkv);
+    Tensor ws = at::empty({static_cast<int64_t>(ts2ts_attn_bwd_workspace_bytes(B, H, T, D))}, qkv.options().dtype(at::kByte));
+    const PackedStrides in(T, 3, H, D), os(T, 1, H, D);
+    const char* base = static_cast<const char*>(qkv.const_data_ptr());
+    char* dbase = static_cast<char*>(dqkv.mutable_data_ptr());
+    const int64_t part = 2 * n_heads * head_dim;
+    const MaskPtrs m(s[5], opt(s[6]), opt(s[7]), opt(s[8]));
+    check(ts2ts_attn_bwd(base, base + part, base + 2 * part, out.const_data_ptr(), dout.const_data_ptr(), fptr(lse), in.s, in.s, in.s, os.s,
+                         os.s, B, H, T, D, 1.f / std::sqrt(static_cast<float>(D)), m.doc, m.row, m.col, m.link, m.R, m.W, plan.const_data_ptr(),
+                         plan.numel(), dbase, dbase + part, dbase + 2 * part, in.s, in.s, in.s, ws.mutable_data_ptr(), ws.numel(), stream),
+          "ts2ts_attn_bwd");
+    // gradient of the rotated q, k -> gradient of the projection's output: the inverse rotation, in place
+    check(ts2ts_rope_qk_inplace(dqkv.mutable_data_ptr(), fptr(cos), fptr(sin), B, T, H, D, -1.f, stream), "ts2ts_rope_qk_inplace");
+    r[0] = dqkv;
+    return r;
+  }
+};
+Tensor qkv_attention(Tensor qkv, const Tensor& cos, const Tensor& sin, const Tensor& doc_ids, const OptTensor& link_bits,
+                     const OptTensor& q_row_ids, const OptTensor& kv_col_ids, const Tensor& plan, int64_t n_heads, int64_t head_dim) {
+  return QKVAttention::apply(qkv, cos, sin, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, n_heads, head_dim)[0];
+}
+
+struct SwiGLU : torch::autograd::Function<SwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gate_up) {
+    need_cuda(gate_up);
+    TORCH_CHECK_TYPE(gate_up.scalar_type() == at::kBFloat16, "swiglu: bf16 input");
+    at::AutoDispatchBelowADInplaceOrView below;
+    const CUDAGuard guard(gate_up.device());
+    const Tensor gu = gate_up.contiguous();
+    const int64_t F = gu.size(-1) / 2, N = gu.numel() / (2 * F);
+    auto shape = gu.sizes().vec();
+    shape.back() = F;
+    Tensor act = at::empty(shape, gu.options());
+    check(ts2ts_swiglu_fwd(gu.const_data_ptr(), act.mutable_data_ptr(), N, static_cast<int>(F), stream_of(gu)), "ts2ts_swiglu_fwd");
+    ctx->save_for_backward({gu});
+    return act;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor gu = ctx->get_saved_variables()[0], dact = grads[0].contiguous();
+    const CUDAGuard guard(gu.device());
+    const int64_t F = gu.size(-1) / 2, N = gu.numel() / (2 * F);
+    Tensor dgu = at::empty_like(gu);
+    check(ts2ts_swiglu_bwd(gu.const_data_ptr(), dact.const_data_ptr(), dgu.mutable_data_ptr(), N, static_cast<int>(F), stream_of(gu)), "ts2ts_swiglu_bwd");
+    return {dgu};
+  }
+};
+Tensor swiglu(const Tensor& gate_up) { return SwiGLU::apply(gate_up); }
+
+struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& target_in) {
+    need_cuda(logits);
+    TORCH_CHECK_TYPE(logits.scalar_type() == at::kBFloat16 && logits.dim() == 2 && logits.is_contiguous(),
+                     "cross_entropy: logits must be a contiguous bf16 [N,V] tensor");
+    at::AutoDispatchBelowADInplaceOrView below;
+    const CUDAGuard guard(logits.device());
+    const Tensor target = target_in.to(at::kLong).contiguous();
+    const int64_t N = logits.size(0), V = logits.size(1);
+    Tensor lse = at::empty({N}, logits.options().dtype(at::kFloat)), loss = at::empty({N}, lse.options());
+    check(ts2ts_ce_fwd(logits.const_data_ptr(), target.const_data_ptr<int64_t>(), mfptr(lse), mfptr(loss), N, static_cast<int>(V), stream_of(logits)),
+          "ts2ts_ce_fwd");
+    ctx->save_for_backward({logits, target, lse});
+    return loss.mean();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor& logits = s[0];
+    const CUDAGuard guard(logits.device());
+    const int64_t N = logits.size(0), V = logits.size(1);
+    const Tensor g = grads[0].to(at::kFloat).contiguous();
+    // the logits are not needed again: their buffer becomes the gradient
+    check(ts2ts_ce_bwd(logits.mutable_data_ptr(), s[1].const_data_ptr<int64_t>(), fptr(s[2]), fptr(g), static_cast<float>(1.0 / static_cast<double>(N)), N,
+                       static_cast<int>(V), stream_of(logits)),
+          "ts2ts_ce_bwd");
+    return {logits, Tensor()};
+  }
+};
+Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); }
+
+// y = x w^T with bf16 activations and an fp32 weight.  The weight gradient leaves its GEMM in fp32: no bf16 rounding and no
+// conversion pass (6 bytes per weight) on the way to the parameter.
+struct Linear : torch::autograd::Function<Linear> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
+    need_cuda(x);
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor x2 = x.reshape({-1, x.size(-1)}), wb = w.to(at::kBFloat16);
+    ctx->save_for_backward({x2, wb});
+    auto shape = x.sizes().vec();
+    shape.back() = w.size(0);
+    ctx->saved_data["shape"] = x.sizes().vec();
+    return at::mm(x2, wb.t()).view(shape);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)});
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(ctx->saved_data["shape"].toIntVector());
+    if (ctx->needs_input_grad(1)) dw = at::mm(dy.t(), s[0], at::kFloat);
+    return {dx, dw};
+  }
+};
+Tensor linear(const Tensor& x, const Tensor& w) { return Linear::apply(x, w); }
+
+// Mean cross-entropy of the output head, logits = h w^T.  The loss kernel leaves the gradient of the mean loss in the
+// logits' buffer; what reaches the loss from above multiplies the two small results instead of the logits.
+struct HeadLoss : torch::autograd::Function<HeadLoss> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& target_in) {
+    need_cuda(h);
+    at::AutoDispatchBelowADInplaceOrView below;
+    const CUDAGuard guard(h.device());
+    const Tensor h2 = h.reshape({-1, h.size(-1)}), wb = w.to(at::kBFloat16), target = target_in.reshape({-1}).to(at::kLong).contiguous();
+    const int64_t N = h2.size(0), V = w.size(0);
+    Tensor logits = at::mm(h2, wb.t()), loss = at::empty({N}, h.options().dtype(at::kFloat));
+    check(ts2ts_ce_fwd_grad(logits.mutable_data_ptr(), target.const_data_ptr<int64_t>(), mfptr(loss), static_cast<float>(1.0 / static_cast<double>(N)), N,
+                            static_cast<int>(V), stream_of(h)),
+          "ts2ts_ce_fwd_grad");
+    ctx->save_for_backward({h2, wb, logits});
+    ctx->saved_data["shape"] = h.sizes().vec();
+    return loss.mean();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const CUDAGuard guard(s[0].device());
+    const Tensor g = grads[0].to(at::kFloat).contiguous();
+    void* stream = stream_of(g);
+    Tensor dh, dw;
+    if (ctx->needs_input_grad(0)) {
+      Tensor dh32 = at::mm(s[2], s[1], at::kFloat);
+      dh = at::empty(ctx->saved_data["shape"].toIntVector(), s[0].options());
+      check(ts2ts_scale(mfptr(dh32), dh.mutable_data_ptr(), fptr(g), dh.numel(), stream), "ts2ts_scale");
+    }
+    if (ctx->needs_input_grad(1)) {
+      dw = at::mm(s[2].t(), s[0], at::kFloat);
+      check(ts2ts_scale(mfptr(dw), nullptr, fptr(g), dw.numel(), stream), "ts2ts_scale");
+    }
+    return {dh, dw, Tensor()};
+  }
+};
+Tensor head_loss(const Tensor& h, const Tensor& w, const Tensor& target) { return HeadLoss::apply(h, w, target); }
+
+struct Embedding : torch::autograd::Function<Embedding> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& w, const Tensor& idx) {
+    need_cuda(w);
+    at::AutoDispatchBelowADInplaceOrView below;
+    ctx->save_for_backward({idx});
+    ctx->saved_data["V"] = w.size(0);
+    return at::embedding(w, idx);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor idx = ctx->get_saved_variables()[0].contiguous(), dx = grads[0].contiguous();
+    const CUDAGuard guard(dx.device());
+    const int64_t V = ctx->saved_data["V"].toInt(), C = dx.size(-1);
+    Tensor dw = at::empty({V, C}, dx.options());
+    check(ts2ts_embedding_bwd(idx.const_data_ptr<int64_t>(), fptr(dx), mfptr(dw), idx.numel(), static_cast<int>(C), V, stream_of(dx)),
+          "ts2ts_embedding_bwd");
+    return {dw, Tensor()};
+  }
+};
+Tensor embedding(const Tensor& w, const Tensor& idx) { return Embedding::apply(w, idx); }
+
+// One AdamW step over fp32 CUDA tensors; `steps` are one-element CPU tensors, advanced here.
+void adamw(at::TensorList params, at::TensorList grads, at::TensorList exp_avgs, at::TensorList exp_avg_sqs, at::TensorList steps, double lr,
+           double beta1, double beta2, double eps, double weight_decay) {
+  const size_t n = params.size();
+  TORCH_CHECK_VALUE(grads.size() == n && exp_avgs.size() == n && exp_avg_sqs.size() == n && steps.size() == n, "adamw: lists of equal length");
+  if (n == 0) return;
+  const CUDAGuard guard(params[0].device());
+  std::vector<float*> p(n), m(n), v(n);
+  std::vector<const float*> g(n);
+  std::vector<int64_t> sizes(n);
+  std::vector<float> t(n);
+  for (size_t i = 0; i < n; ++i) {
+    TORCH_CHECK_VALUE(params[i].device() == params[0].device() && steps[i].is_cpu(), "adamw: parameters on one device, steps on the CPU");
+    for (const Tensor* x : {&params[i], &grads[i], &exp_avgs[i], &exp_avg_sqs[i]})
+      TORCH_CHECK_VALUE(x->is_cuda() && x->scalar_type() == at::kFloat && x->is_contiguous() && x->numel() == params[i].numel(),
+                        "adamw: contiguous fp32 CUDA tensors");
+    p[i] = mfptr(params[i]); g[i] = fptr(grads[i]); m[i] = mfptr(exp_avgs[i]); v[i] = mfptr(exp_avg_sqs[i]);
+    sizes[i] = params[i].numel();
+    t[i] = *mfptr(steps[i]) += 1.f;
+  }
+  check(ts2ts_adamw(static_cast<int>(n), p.data(), g.data(), m.data(), v.data(), sizes.data(), t.data(), lr, beta1, beta2, eps, weight_decay,
+                    stream_of(params[0])),
+        "ts2ts_adamw");
+  for (const Tensor& x : params) x.unsafeGetTensorImpl()->bump_version();
+}
+
 }  // namespace
 
 TORCH_LIBRARY(ts2ts, m) {
@@ -221,6 +506,16 @@ TORCH_LIBRARY(ts2ts, m) {
   m.def("masked_attn_decode(Tensor q, Tensor k_cache, Tensor v_cache, Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, "
         "Tensor? kv_col_ids, Tensor? q_pos, float scale) -> (Tensor, Tensor)");
   m.def("block_map(Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, Tensor? kv_col_ids, bool with_lists) -> Tensor[]");
+  m.def("add_rmsnorm(Tensor x, Tensor? a, Tensor w, float eps) -> (Tensor, Tensor)", add_rmsnorm);
+  m.def("qkv_attention(Tensor(a!) qkv, Tensor cos, Tensor sin, Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, Tensor? kv_col_ids, "
+        "Tensor plan, int n_heads, int head_dim) -> Tensor", qkv_attention);
+  m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
+  m.def("cross_entropy(Tensor logits, Tensor target) -> Tensor", cross_entropy);
+  m.def("linear(Tensor x, Tensor w) -> Tensor", linear);
+  m.def("head_loss(Tensor h, Tensor w, Tensor target) -> Tensor", head_loss);
+  m.def("embedding(Tensor w, Tensor idx) -> Tensor", embedding);
+  m.def("adamw(Tensor(a!)[] params, Tensor[] grads, Tensor(b!)[] exp_avgs, Tensor(c!)[] exp_avg_sqs, Tensor(d!)[] steps, float lr, float beta1, "
+        "float beta2, float eps, float weight_decay) -> ()", adamw);
 }
 TORCH_LIBRARY_IMPL(ts2ts, CUDA, m) {
   m.impl("masked_attn_fwd", attn_fwd_cuda);

@@ -6,9 +6,9 @@ cross-entropy) and its DDP settings (main.py:404-415: static graph, no unused pa
 plain pre-norm decoder (RMSNorm, fused QKV, RoPE, SwiGLU) standing in for the reference's tunalab modules, which are
 not available.  Every layer calls the masked-attention kernels on the packed QKV projection (lm_fused.qkv_attention);
 the block plan is built once per micro-batch and shared by all layers, as the reference shares its BlockMask
-(block_mask_creator.py:132-139).  The GEMMs are cuBLAS through torch and the optimizer is torch's fused AdamW; the
-memory-bound pieces between them (residual add + RMSNorm, rotary embedding, SwiGLU, cross-entropy) are single-pass
-kernels of this library, as the reference's are fused modules.
+(block_mask_creator.py:132-139).  The GEMMs are cuBLAS through torch; the memory-bound pieces between them (residual add +
+RMSNorm, rotary embedding, SwiGLU, cross-entropy, the embedding's gradient, AdamW) are single-pass kernels of this library,
+as the reference's are fused modules.
 """
 from __future__ import annotations
 
@@ -19,9 +19,8 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
-from .lm_fused import add_rmsnorm, cross_entropy, qkv_attention, rope_half_tables, swiglu
+from .lm_fused import AdamW, Linear, add_rmsnorm, embedding, head_loss, qkv_attention, rope_half_tables, swiglu
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -79,11 +78,11 @@ class Block(nn.Module):
         hd = cfg.n_heads * cfg.head_dim
         self.cfg = cfg
         self.ln1 = nn.RMSNorm(cfg.d_model)
-        self.qkv = nn.Linear(cfg.d_model, 3 * hd, bias=False)
-        self.proj = nn.Linear(hd, cfg.d_model, bias=False)
+        self.qkv = Linear(cfg.d_model, 3 * hd)
+        self.proj = Linear(hd, cfg.d_model)
         self.ln2 = nn.RMSNorm(cfg.d_model)
-        self.gate_up = nn.Linear(cfg.d_model, 2 * cfg.mlp_hidden, bias=False)
-        self.down = nn.Linear(cfg.mlp_hidden, cfg.d_model, bias=False)
+        self.gate_up = Linear(cfg.d_model, 2 * cfg.mlp_hidden)
+        self.down = Linear(cfg.mlp_hidden, cfg.d_model)
 
     def forward(self, x, a, mask: MaskSpec, cos, sin):
         c = self.cfg
@@ -100,26 +99,28 @@ class DecoderLM(nn.Module):
         self.embed = nn.Embedding(cfg.vocab, cfg.d_model)
         self.blocks = nn.ModuleList(Block(cfg) for _ in range(cfg.n_layers))
         self.norm = nn.RMSNorm(cfg.d_model)
-        self.head = nn.Linear(cfg.d_model, cfg.vocab, bias=False)
+        self.head = Linear(cfg.d_model, cfg.vocab)
         for p in self.parameters():
             if p.dim() >= 2:
                 nn.init.normal_(p, std=0.02)
+        self._rope = None  # the rotation tables of the last sequence length and device
+
+    def _rope_tables(self, T: int, device):
+        if self._rope is None or self._rope[0] != (T, device):
+            self._rope = ((T, device), rope_half_tables(T, self.cfg.head_dim, self.cfg.rope_base, device))
+        return self._rope[1]
 
     def forward(self, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
         """tokens int64 [B, T+1]; returns the mean next-token cross-entropy (training_module.py:195-211).  Runs under
         bf16 autocast: the linear layers compute in bf16, the residual stream, norms, rotary angles and the loss in fp32."""
         inp, tgt = tokens[:, :-1], tokens[:, 1:]
-        T = inp.shape[1]
-        x = self.embed(inp).float()
-        cos, sin = rope_half_tables(T, self.cfg.head_dim, self.cfg.rope_base, inp.device)
+        x = embedding(self.embed.weight, inp).float()
+        cos, sin = self._rope_tables(inp.shape[1], inp.device)
         a = None
         for blk in self.blocks:
             x, a = blk(x, a, mask, cos, sin)
         _, h = add_rmsnorm(x, a, self.norm.weight, RMS_EPS)
-        logits = self.head(h)
-        if logits.dtype != torch.bfloat16:
-            logits = logits.to(torch.bfloat16)
-        return cross_entropy(logits.view(-1, logits.shape[-1]), tgt.reshape(-1))
+        return head_loss(h, self.head.weight, tgt)
 
 
 class TrainStep:
@@ -145,7 +146,7 @@ class TrainStep:
             if self.bf16_grads:
                 from torch.distributed.algorithms.ddp_comm_hooks import default_hooks
                 self.model.register_comm_hook(None, default_hooks.bf16_compress_hook)
-        self.opt = torch.optim.AdamW(model.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1, fused=True)
+        self.opt = AdamW(model.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1)
 
     @property
     def grad_bytes_per_step(self) -> int:

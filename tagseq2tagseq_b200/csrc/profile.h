@@ -17,11 +17,14 @@ struct ProfileScope {
   ProfileSlot& s;
   int which;
   cudaStream_t stream;
-  ProfileScope(int which_, cudaStream_t st) : s(profile_slot()), which(which_), stream(st) {
-    if (s.enabled) cudaEventRecord(s.start[which], stream);
+  bool on;  // not inside a stream capture, where an event cannot be timed
+  ProfileScope(int which_, cudaStream_t st) : s(profile_slot()), which(which_), stream(st), on(s.enabled) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (on && (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)) on = false;
+    if (on) cudaEventRecord(s.start[which], stream);
   }
   ~ProfileScope() {
-    if (s.enabled) {
+    if (on) {
       cudaEventRecord(s.stop[which], stream);
       s.recorded[which] = true;
     }

@@ -217,6 +217,8 @@ std::vector<Tensor> block_map_cuda(const Tensor& doc_ids, const OptTensor& link_
 // (set_materialize_grads(false)) instead of as zero tensors of the activation's size.
 using c10::cuda::CUDAGuard;
 
+// An autograd worker that has made no CUDA call yet has no current context, and cuBLAS asks for one.
+void bind_context(const Tensor& t) { C10_CUDA_CHECK(c10::cuda::SetDevice(t.device().index(), true)); }
 void need_cuda(const Tensor& t) {
   TORCH_CHECK(t.is_cuda(), "the decoder-layer kernels run on CUDA tensors only (no CPU path exists)");
 }
@@ -404,6 +406,7 @@ struct Linear : torch::autograd::Function<Linear> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
+    bind_context(s[0]);
     const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)});
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(ctx->saved_data["shape"].toIntVector());
@@ -433,6 +436,7 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     const CUDAGuard guard(s[0].device());
+    bind_context(s[0]);
     const Tensor g = grads[0].to(at::kFloat).contiguous();
     void* stream = stream_of(g);
     Tensor dh, dw;

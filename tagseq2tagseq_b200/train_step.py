@@ -12,13 +12,14 @@ as the reference's are fused modules.
 """
 from __future__ import annotations
 
-import math
+from collections import OrderedDict
 from contextlib import nullcontext as _nullcontext
 from dataclasses import dataclass
 from typing import Optional
 
 import torch
 import torch.nn as nn
+import torch.nn.modules.module as _module
 
 from .lm_fused import AdamW, Linear, add_rmsnorm, embedding, head_loss, qkv_attention, rope_half_tables, swiglu
 from .mask_spec import MaskSpec
@@ -123,6 +124,54 @@ class DecoderLM(nn.Module):
         return head_loss(h, self.head.weight, tgt)
 
 
+class _StepGraph:
+    """Forward and backward of one micro-batch shape as a CUDA graph: its inputs are copied into buffers of the graph's own,
+    the block plan is part of it, the gradients it writes are handed to the parameters.  Link bits are padded with rows and
+    columns that grant nothing, so that packs with different numbers of documents share a graph."""
+
+    def __init__(self, owner: "TrainStep", tokens: torch.Tensor, mask: MaskSpec, key):
+        own = lambda t: None if t is None else torch.empty_like(t, memory_format=torch.contiguous_format)
+        self.tokens = own(tokens)
+        self.mask = MaskSpec(own(mask.doc_ids), None, own(mask.q_row_ids), own(mask.kv_col_ids))
+        if mask.link_bits is not None:
+            self.mask.link_bits = torch.zeros((mask.link_bits.shape[0],) + key[-2:], dtype=torch.int64, device=tokens.device)
+        self._load(tokens, mask)
+        self.params = list(owner.model.parameters())
+        self.graph = torch.cuda.CUDAGraph()
+        side, here = torch.cuda.Stream(), torch.cuda.current_stream()
+        side.wait_stream(here)
+        with torch.cuda.stream(side):
+            self.graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                self.loss = owner._eager(self.tokens, self.mask)
+            finally:
+                self.graph.capture_end()
+        here.wait_stream(side)
+        self.mask._block_map = None  # built by the graph, into its own pool
+        self.grads = [p.grad for p in self.params]
+
+    def _load(self, tokens, mask):
+        self.tokens.copy_(tokens)
+        m = self.mask
+        m.doc_ids.copy_(mask.doc_ids)
+        if m.q_row_ids is not None:
+            m.q_row_ids.copy_(mask.q_row_ids)
+        if m.kv_col_ids is not None:
+            m.kv_col_ids.copy_(mask.kv_col_ids)
+        if m.link_bits is not None:
+            R, W = mask.link_bits.shape[1:]
+            if m.link_bits.shape[1:] != (R, W):
+                m.link_bits.zero_()
+            m.link_bits[:, :R, :W].copy_(mask.link_bits)
+
+    def run(self, tokens, mask) -> torch.Tensor:
+        self._load(tokens, mask)
+        self.graph.replay()
+        for p, g in zip(self.params, self.grads):
+            p.grad = g
+        return self.loss.clone()
+
+
 class TrainStep:
     """One optimizer step on one packed sequence per rank: forward under bf16 autocast, backward (DDP all-reduces
     the gradients, overlapped with the backward), fused AdamW on fp32 parameters.
@@ -130,7 +179,13 @@ class TrainStep:
     DDP settings follow main.py:404-415 (static graph, no unused parameters, 256 MB buckets; the first bucket keeps
     torch's small default so that the last gradients to be produced start their all-reduce early).  With
     ``bf16_grads`` the buckets are cast to bf16 for the all-reduce and back (torch's ``bf16_compress_hook``), which
-    halves the bytes on NVLink; the parameters and the optimizer state stay fp32."""
+    halves the bytes on NVLink; the parameters and the optimizer state stay fp32.
+
+    On one GPU, a step whose kernels are shorter than the host work of launching them (see ``_use_graph``) is replayed as
+    a CUDA graph from the second micro-batch of its shape on.  ``p.grad`` is then the graph's own buffer, which the next
+    step overwrites.  ``use_graphs = False`` turns that off."""
+
+    MAX_GRAPHS = 2  # micro-batch shapes whose graph, and with it a step's activations, is kept
 
     def __init__(self, cfg: LMConfig, device: torch.device, world: int = 1, lr: float = 3e-4, seed: int = 0,
                  bf16_grads: bool = True, bucket_cap_mb: int = 256):
@@ -147,6 +202,9 @@ class TrainStep:
                 from torch.distributed.algorithms.ddp_comm_hooks import default_hooks
                 self.model.register_comm_hook(None, default_hooks.bf16_compress_hook)
         self.opt = AdamW(model.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1)
+        self.use_graphs = True
+        self._graphs: "OrderedDict[tuple, Optional[_StepGraph]]" = OrderedDict()  # None: shape seen once
+        self._layout = None
 
     @property
     def grad_bytes_per_step(self) -> int:
@@ -157,6 +215,13 @@ class TrainStep:
     def forward_backward(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True) -> torch.Tensor:
         """Loss and gradients without the optimizer step.  ``sync=False`` skips the gradient all-reduce (DDP's
         ``no_sync``): the difference between the two is what the collective costs this rank."""
+        if self.use_graphs and self.world == 1:
+            key = self._graph_key(tokens, mask)
+            if key is not None:
+                return self._graphed(key, tokens, mask)
+        return self._eager(tokens, mask, sync)
+
+    def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True) -> torch.Tensor:
         self.opt.zero_grad(set_to_none=True)
         ctx = self.model.no_sync() if (not sync and self.world > 1) else _nullcontext()
         with ctx:
@@ -164,6 +229,59 @@ class TrainStep:
                 loss = self.model(tokens, mask)
             loss.backward()
         return loss.detach()
+
+    # ------------------------------------------------------------------ CUDA graphs of small steps
+    def _use_graph(self, n_tokens: int) -> bool:
+        """Launching a step takes about half a millisecond of host time per layer and as much for the rest; the GEMMs
+        take 6 FLOPs per parameter and token at 1.2 PFLOP/s or less.  Where the second is shorter, the GPU waits for the
+        host (two layers of d256 at T=1024: 1.38 ms a step, of which 0.38 ms of kernels).  The same bound keeps the
+        activations that a graph holds on to small."""
+        return 6.0 * self.cfg.matmul_params * n_tokens / 1.2e12 < 0.5 * (self.cfg.n_layers + 1)
+
+    def _graph_key(self, tokens: torch.Tensor, mask: MaskSpec):
+        doc, link = mask.doc_ids, mask.link_bits
+        if not (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.int64 and tokens.numel() > 0
+                and doc.shape == (tokens.shape[0], tokens.shape[1] - 1) and tokens.device == self.device == doc.device
+                and torch.cuda.current_device() == self.device.index and self._use_graph(doc.numel())):
+            return None
+        if torch.cuda.is_current_stream_capturing() or not torch.is_grad_enabled() or not self._as_built():
+            return None
+        key = (tokens.shape[0], tokens.shape[1], mask.q_row_ids is not None, mask.kv_col_ids is not None)
+        if link is not None:  # capacities in steps of 64 row classes and of powers of two words
+            key += (-(-link.shape[1] // 64) * 64, 1 << (link.shape[2] - 1).bit_length())
+        return key
+
+    def _as_built(self) -> bool:
+        """Whether the model is still the one the graphs were captured from: the same modules and parameters at the same
+        addresses, and no hooks, which a replay would not call."""
+        if self._layout is None:
+            mods = list(self.model.modules())
+            self._layout = (mods, [(m._modules, dict(m._modules)) for m in mods],
+                            [(m._parameters, n, p, p.data_ptr()) for m in mods for n, p in m._parameters.items() if p is not None])
+            self._graphs.clear()
+        mods, children, params = self._layout
+        if _module._has_any_global_hook() or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in mods):
+            return False
+        same = all(d == kept for d, kept in children) and all(
+            d.get(n) is p and p.data_ptr() == at for d, n, p, at in params)
+        if not same:
+            self._layout = None  # looked over again, and captured again, from the next step on
+            return False
+        return all(p.requires_grad and not p._backward_hooks and not p._post_accumulate_grad_hooks for _, _, p, _ in params)
+
+    def _graphed(self, key, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
+        if key not in self._graphs:  # the first step of a shape runs as it is: libraries set themselves up
+            self._graphs[key] = None
+            while len(self._graphs) > 8:
+                self._graphs.popitem(last=False)
+            return self._eager(tokens, mask)
+        if self._graphs[key] is None:
+            live = [k for k, g in self._graphs.items() if g is not None]
+            if len(live) >= self.MAX_GRAPHS:
+                del self._graphs[live[0]]
+            self._graphs[key] = _StepGraph(self, tokens, mask, key)
+        self._graphs.move_to_end(key)
+        return self._graphs[key].run(tokens, mask)
 
     def step(self, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
         loss = self.forward_backward(tokens, mask)

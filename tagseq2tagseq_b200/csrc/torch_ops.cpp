@@ -13,9 +13,13 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
+#include <algorithm>
 #include <array>
 #include <cmath>
+#include <string>
 #include <tuple>
+#include <unordered_map>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -209,6 +213,206 @@ std::vector<Tensor> block_map_cuda(const Tensor& doc_ids, const OptTensor& link_
   check(ts2ts_block_map(m.doc, m.row, m.col, m.link, B, T, m.R, m.W, r[0].mutable_data_ptr(), r[0].numel(), state, lists[0], lists[1],
                         lists[2], lists[3], lists[4], lists[5], lists[6], lists[7], stream_of(doc_ids)),
         "ts2ts_block_map");
+  return r;
+}
+
+// ------------------------------------------------------------------------------------------------ link scan
+// Candidate links of a token sequence and the tokens of their targets, on the host: ({mid, start, close} int32 [n,3], the
+// targets' tokens mid+1 .. close of all links one after the other, int64).  Candidates and tokens come back together in
+// one wait; sequences too long for that to be cheap fetch the tokens between the first and the last link afterwards.
+constexpr int64_t kTokensAlong = 65536;
+
+std::tuple<Tensor, Tensor> link_candidates(const Tensor& input_ids, int64_t mid_id, at::IntArrayRef start_ids, const Tensor& close_flags,
+                                           int64_t back_limit, int64_t window) {
+  const c10::cuda::CUDAGuard guard(input_ids.device());
+  const auto stream = c10::cuda::getCurrentCUDAStream(input_ids.device().index());
+  const Tensor tokens = input_ids.contiguous();
+  const int64_t T = tokens.size(0);
+  const int bytes = static_cast<int>(tokens.element_size());
+  const auto dev32 = tokens.options().dtype(at::kInt), host32 = at::TensorOptions().dtype(at::kInt).pinned_memory(true);
+  Tensor scratch = at::empty({static_cast<int64_t>(ts2ts_detect_links_scratch_bytes(static_cast<int>(T)))}, dev32.dtype(at::kByte));
+  Tensor host, host_tokens;
+  int64_t max_links = 1024, n = 0, first = 0;
+  if (T <= kTokensAlong) {
+    host_tokens = at::empty({T}, host32.dtype(tokens.scalar_type()));
+    host_tokens.copy_(tokens, /*non_blocking=*/true);
+  }
+  for (;;) {  // a second turn only when the sequence holds more candidates than the first buffer
+    Tensor out = at::empty({4 + 3 * max_links}, dev32);  // count, padding, triples
+    int32_t* o = out.mutable_data_ptr<int32_t>();
+    check(ts2ts_detect_links(tokens.const_data_ptr(), bytes, static_cast<int>(T), mid_id, start_ids.data(), static_cast<int>(start_ids.size()),
+                             close_flags.const_data_ptr<uint8_t>(), static_cast<int>(close_flags.size(0)), static_cast<int>(back_limit),
+                             static_cast<int>(window), scratch.mutable_data_ptr(), scratch.numel(), o + 4, static_cast<int>(max_links), o,
+                             stream.stream()),
+          "ts2ts_detect_links");
+    host = at::empty({out.numel()}, host32);
+    host.copy_(out, /*non_blocking=*/true);
+    stream.synchronize();
+    n = host.const_data_ptr<int32_t>()[0];
+    if (n <= max_links) break;
+    max_links = n;
+  }
+  const int32_t* tri = host.const_data_ptr<int32_t>() + 4;
+  Tensor links = at::empty({n, 3}, at::kInt);
+  std::copy(tri, tri + 3 * n, links.mutable_data_ptr<int32_t>());
+  int64_t total = 0, last = 0;
+  for (int64_t i = 0; i < n; ++i) {
+    total += tri[3 * i + 2] - tri[3 * i];
+    last = std::max<int64_t>(last, tri[3 * i + 2]);
+  }
+  if (n > 0 && !host_tokens.defined()) {
+    first = tri[0] + 1;  // candidates ascend
+    host_tokens = tokens.slice(0, first, last + 1).cpu();
+  }
+  Tensor targets = at::empty({total}, at::kLong);
+  int64_t* dst = targets.mutable_data_ptr<int64_t>();
+  for (int64_t i = 0; i < n; ++i)
+    for (int64_t t = tri[3 * i] + 1; t <= tri[3 * i + 2]; ++t)
+      *dst++ = bytes == 8 ? host_tokens.const_data_ptr<int64_t>()[t - first] : host_tokens.const_data_ptr<int32_t>()[t - first];
+  return {links, targets};
+}
+
+// ------------------------------------------------------------------------------------------------ masks from spans and links
+// Tokens covered by the same set of intervals form one class.  The set only changes where an interval starts or ends, so
+// there are at most 2 G + 1 segments however long the sequence is.  `bounds` [S+1] and `ids` [S] (-1: no interval);
+// classes are numbered in order of first appearance, `sets` holds their member bits, `words` 64-bit words each.
+struct Segments {
+  std::vector<int32_t> bounds, ids;
+  std::vector<uint64_t> sets;
+  int classes = 0;
+  Segments(const std::vector<std::pair<int64_t, int64_t>>& ranges, size_t words) {
+    struct Event { int64_t at; int32_t who; bool opens; };
+    std::vector<Event> ev;
+    ev.reserve(2 * ranges.size());
+    for (size_t g = 0; g < ranges.size(); ++g) {
+      ev.push_back({ranges[g].first, static_cast<int32_t>(g), true});
+      ev.push_back({ranges[g].second, static_cast<int32_t>(g), false});
+    }
+    std::sort(ev.begin(), ev.end(), [](const Event& a, const Event& b) { return a.at < b.at; });
+    std::vector<uint64_t> now(words, 0);
+    std::unordered_map<std::string, int32_t> seen;
+    int64_t open = 0;
+    for (size_t i = 0; i < ev.size();) {
+      const int64_t at = ev[i].at;
+      for (; i < ev.size() && ev[i].at == at; ++i) {
+        now[ev[i].who >> 6] ^= uint64_t(1) << (ev[i].who & 63);
+        open += ev[i].opens ? 1 : -1;
+      }
+      bounds.push_back(static_cast<int32_t>(at));
+      if (i == ev.size()) break;
+      if (open == 0) {
+        ids.push_back(-1);
+        continue;
+      }
+      const auto [it, fresh] = seen.try_emplace(std::string(reinterpret_cast<const char*>(now.data()), words * 8), classes);
+      if (fresh) {
+        sets.insert(sets.end(), now.begin(), now.end());
+        ++classes;
+      }
+      ids.push_back(it->second);
+    }
+    if (bounds.empty()) bounds.push_back(0);
+  }
+};
+
+// {doc_ids [1,T]} or {doc_ids, link_bits [1,R,W], q_row_ids, kv_col_ids} of a pack: spans (start, end, doc id) as they come,
+// links as (position, target doc id) in the order in which they receive grants.  A link at `pos` of the first span with
+// start < pos <= end grants tokens [pos, end) the first span of its target; empty grants take no place, and the first one
+// beyond `cap` ends the list (cross_doc_mask.py:239-294).  The host works on segment tables, which reach the device in one
+// copy with the link bits; one kernel per id array spreads them over the tokens.
+std::vector<Tensor> pack_mask(at::IntArrayRef starts, at::IntArrayRef ends, at::IntArrayRef ids, at::IntArrayRef link_pos,
+                              at::IntArrayRef link_target, int64_t T, int64_t cap, c10::Device device) {
+  const size_t n_spans = starts.size();
+  TORCH_CHECK_VALUE(ends.size() == n_spans && ids.size() == n_spans && link_pos.size() == link_target.size(), "pack_mask: lists of equal length");
+  if (!device.has_index()) device = c10::Device(c10::kCUDA, c10::cuda::current_device());
+  const c10::cuda::CUDAGuard guard(device);
+  std::unordered_map<int64_t, size_t> by_id;
+  for (size_t i = 0; i < n_spans; ++i) by_id.try_emplace(ids[i], i);
+  std::vector<std::pair<int64_t, int64_t>> q, k;
+  int64_t src_pos = 0, src_end = 0;  // the source of the last position, if it has one
+  bool has_src = false;
+  for (size_t l = 0; l < link_pos.size() && static_cast<int64_t>(q.size()) < cap; ++l) {
+    const int64_t pos = link_pos[l];
+    if (l == 0 || pos != src_pos) {
+      src_pos = pos;
+      has_src = false;
+      for (size_t i = 0; i < n_spans; ++i)
+        if (starts[i] < pos && pos <= ends[i]) {
+          has_src = true;
+          src_end = ends[i];
+          break;
+        }
+    }
+    const auto it = by_id.find(link_target[l]);
+    if (!has_src || it == by_id.end()) continue;
+    const int64_t q1 = std::min(T, src_end), k0 = std::max<int64_t>(0, starts[it->second]), k1 = std::min(T, ends[it->second]);
+    if (pos < q1 && k0 < k1) {
+      q.emplace_back(pos, q1);
+      k.emplace_back(k0, k1);
+    }
+  }
+  // documents: later spans overwrite earlier ones, uncovered tokens are -1
+  std::vector<int32_t> db;
+  for (size_t i = 0; i < n_spans; ++i) {
+    const int64_t a = std::max<int64_t>(0, starts[i]), b = std::min(T, ends[i]);
+    if (a < b) {
+      db.push_back(static_cast<int32_t>(a));
+      db.push_back(static_cast<int32_t>(b));
+    }
+  }
+  std::sort(db.begin(), db.end());
+  db.erase(std::unique(db.begin(), db.end()), db.end());
+  if (db.empty()) db.push_back(0);
+  std::vector<int32_t> di(db.size() - 1, -1);
+  for (size_t i = 0; i < n_spans; ++i) {
+    const int64_t a = std::max<int64_t>(0, starts[i]), b = std::min(T, ends[i]);
+    if (a < b)
+      for (auto at = std::lower_bound(db.begin(), db.end(), static_cast<int32_t>(a)); *at < b; ++at) di[at - db.begin()] = static_cast<int32_t>(ids[i]);
+  }
+  const size_t words = (q.size() + 63) / 64;
+  const Segments qs(q, words), ks(k, words);
+  const int64_t R = std::max(1, qs.classes), W = std::max(1, (ks.classes + 63) / 64);
+  const bool linked = !q.empty();
+  // staging: link bits, then the tables (bounds, ids) of documents, rows and columns
+  const std::vector<int32_t>* tables[6] = {&db, &di, &qs.bounds, &qs.ids, &ks.bounds, &ks.ids};
+  const int n_tables = linked ? 6 : 2;
+  int64_t ints = linked ? 2 * R * W : 0, at[6];
+  for (int i = 0; i < n_tables; ++i) {
+    at[i] = ints;
+    ints += static_cast<int64_t>(tables[i]->size());
+  }
+  const auto dev = at::TensorOptions().dtype(at::kInt).device(device);
+  Tensor stage = at::empty({ints}, at::TensorOptions().dtype(at::kInt).pinned_memory(true)), table = at::empty({ints}, dev);
+  int32_t* st = stage.mutable_data_ptr<int32_t>();
+  for (int i = 0; i < n_tables; ++i) std::copy(tables[i]->begin(), tables[i]->end(), st + at[i]);
+  if (linked) {
+    uint64_t* bits = reinterpret_cast<uint64_t*>(st);
+    std::fill(bits, bits + R * W, 0);
+    for (int r = 0; r < qs.classes; ++r)
+      for (int c = 0; c < ks.classes; ++c) {
+        const uint64_t *a = &qs.sets[r * words], *b = &ks.sets[c * words];
+        uint64_t hit = 0;
+        for (size_t w = 0; w < words; ++w) hit |= a[w] & b[w];
+        if (hit) bits[r * W + (c >> 6)] |= uint64_t(1) << (c & 63);
+      }
+  }
+  table.copy_(stage, /*non_blocking=*/true);
+  std::vector<Tensor> r;
+  const int32_t* d = table.const_data_ptr<int32_t>();
+  auto spread = [&](int i) {
+    Tensor out = at::empty({1, T}, dev);
+    if (T == 0) return out;
+    check(ts2ts_segment_ids(d + at[i], d + at[i + 1], static_cast<int>(tables[i + 1]->size()), static_cast<int>(T), out.mutable_data_ptr<int32_t>(),
+                            stream_of(out)),
+          "ts2ts_segment_ids");
+    return out;
+  };
+  r.push_back(spread(0));
+  if (linked) {
+    r.push_back(table.slice(0, 0, 2 * R * W).view(at::kLong).view({1, R, W}));
+    r.push_back(spread(2));
+    r.push_back(spread(4));
+  }
   return r;
 }
 
@@ -510,6 +714,8 @@ TORCH_LIBRARY(ts2ts, m) {
   m.def("masked_attn_decode(Tensor q, Tensor k_cache, Tensor v_cache, Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, "
         "Tensor? kv_col_ids, Tensor? q_pos, float scale) -> (Tensor, Tensor)");
   m.def("block_map(Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, Tensor? kv_col_ids, bool with_lists) -> Tensor[]");
+  m.def("link_candidates(Tensor input_ids, int mid_id, int[] start_ids, Tensor close_flags, int back_limit, int window) -> (Tensor, Tensor)");
+  m.def("pack_mask(int[] starts, int[] ends, int[] ids, int[] link_pos, int[] link_target, int seq_len, int cap, Device device) -> Tensor[]", pack_mask);
   m.def("add_rmsnorm(Tensor x, Tensor? a, Tensor w, float eps) -> (Tensor, Tensor)", add_rmsnorm);
   m.def("qkv_attention(Tensor(a!) qkv, Tensor cos, Tensor sin, Tensor doc_ids, Tensor? link_bits, Tensor? q_row_ids, Tensor? kv_col_ids, "
         "Tensor plan, int n_heads, int head_dim) -> Tensor", qkv_attention);
@@ -526,5 +732,6 @@ TORCH_LIBRARY_IMPL(ts2ts, CUDA, m) {
   m.impl("masked_attn_bwd", attn_bwd_cuda);
   m.impl("masked_attn_decode", attn_decode_cuda);
   m.impl("block_map", block_map_cuda);
+  m.impl("link_candidates", link_candidates);
 }
 TORCH_LIBRARY_IMPL(ts2ts, Autograd, m) { m.impl("masked_attn_fwd", attn_fwd_autograd); }

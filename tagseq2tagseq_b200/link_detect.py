@@ -5,7 +5,7 @@ constructor arguments, same ``detect_links(input_ids) -> List[LinkInfo]`` and ``
 protocol, model/graph_traversal/link_detector.py:22-84), so it can be handed to ``CrossDocLinkMaskCreator``
 unchanged.  The reference walks the sequence with one ``.item()`` per token it looks at; here the positions of every
 "[ ... ](" ... ")" candidate come from ``ts2ts_detect_links`` in one pass over the device tensor, and only the few
-target tokens of each candidate are copied back and decoded (with the reference's own growing-window rule, so the
+target tokens of each candidate are decoded (with the reference's own growing-window rule, so the
 strings and the non-empty test are the reference's).
 
 The per-token table "this token's bytes contain ')'" is built once from ``decode_fn`` over ``vocab_size`` ids.  It is
@@ -13,7 +13,6 @@ exact for byte-level BPE vocabularies (GPT-2's): ')' is a single ASCII byte, whi
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Any, Callable, List, Optional, Tuple
 
 import torch
@@ -58,71 +57,52 @@ class MarkdownLinkDetector:
             self._close_dev[key] = self._close_host.to(device)
         return self._close_dev[key]
 
-    def candidates(self, input_ids: torch.Tensor) -> List[Tuple[int, int, int]]:
-        """(position of '](', position of '[', position of the closing token) for every candidate, ascending."""
+    def _scan(self, input_ids: torch.Tensor):
+        """({mid, start, close} of every candidate, the tokens of all targets one after the other), as lists."""
         if input_ids.dim() != 1:
             raise ValueError("input_ids must be 1-D")
         if not input_ids.is_cuda:
             raise RuntimeError("the link scan runs on the GPU: input_ids must be a CUDA tensor (there is no CPU path)")
         if input_ids.dtype not in (torch.int32, torch.int64):
             raise TypeError("input_ids must be int32 or int64")
-        T = input_ids.shape[0]
-        if T == 0:
-            return []
-        tokens = input_ids.contiguous()
-        L = _lib.lib()
-        dev = tokens.device
-        flags = self._close_flags(dev)
-        starts = sorted(self.link_start_token_ids)
-        start_arr = (ctypes.c_int64 * len(starts))(*starts)
-        with torch.cuda.device(dev):
-            scratch = torch.empty(L.ts2ts_detect_links_scratch_bytes(T), dtype=torch.uint8, device=dev)
-            stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-            max_links = 1024
-            while True:
-                out = torch.empty((max_links, 3), dtype=torch.int32, device=dev)
-                count = torch.zeros(1, dtype=torch.int32, device=dev)
-                _lib.check(L.ts2ts_detect_links(tokens.data_ptr(), tokens.element_size(), T, self.link_mid_token_id, start_arr,
-                                                len(starts), flags.data_ptr(), self.vocab_size, 100, self.window_tokens,
-                                                scratch.data_ptr(), scratch.numel(), out.data_ptr(), max_links,
-                                                count.data_ptr(), stream), "ts2ts_detect_links")
-                n = int(count.item())
-                if n <= max_links:
-                    break
-                max_links = n
-        return [tuple(r) for r in out[:n].cpu().tolist()]
+        if input_ids.shape[0] == 0:
+            return [], []
+        try:
+            links, targets = _lib.ops().link_candidates.default(input_ids, self.link_mid_token_id, sorted(self.link_start_token_ids),
+                                                                self._close_flags(input_ids.device), 100, self.window_tokens)
+        except RuntimeError as e:
+            raise _lib.failed_call(e) from None
+        return links.tolist(), targets.tolist()
+
+    def candidates(self, input_ids: torch.Tensor) -> List[Tuple[int, int, int]]:
+        """(position of '](', position of '[', position of the closing token) for every candidate, ascending."""
+        return [tuple(r) for r in self._scan(input_ids)[0]]
 
     # ------------------------------------------------------------------ protocol
     def detect_links(self, input_ids: torch.Tensor) -> List[LinkInfo]:
-        cands = self.candidates(input_ids)
-        if not cands:
-            return []
-        # one gather of the target windows instead of one .item() per token
-        lo = min(c[0] for c in cands) + 1
-        hi = min(input_ids.shape[0], max(c[0] for c in cands) + 1 + self.window_tokens)
-        host = input_ids[lo:hi].cpu().tolist()
+        cands, targets = self._scan(input_ids)
         links: List[LinkInfo] = []
+        decode, new, done = self.decode_fn, tuple.__new__, 0
         for mid, _start, close in cands:
-            chunk = host[mid + 1 - lo:close + 1 - lo]
-            decoded = self.decode_fn(chunk)
-            idx = decoded.find(")")
-            if idx < 0:
+            n = close - mid
+            target, closed, _ = decode(targets[done:done + n]).partition(")")
+            done += n
+            if not closed:
                 # the per-token table promised a ')' that the joint decoding does not show (not a byte-level
                 # vocabulary): fall back to the reference's growing window for this candidate
-                idx, found = self._grow(host, mid + 1 - lo, min(mid + 1 + self.window_tokens, input_ids.shape[0]) - lo)
-                if idx < 0:
+                target, at = self._grow(input_ids[mid + 1:mid + 1 + self.window_tokens].tolist())
+                if at < 0:
                     continue
-                decoded, close = found[0], found[1] + lo
-            target = decoded[:idx].strip()
+                close = mid + 1 + at
+            target = target.strip()
             if target:
-                links.append(LinkInfo(link_end_pos=close + 1, target_str=target))
+                links.append(new(LinkInfo, (close + 1, target)))
         return links
 
-    def _grow(self, host: List[int], begin: int, end: int):
-        chunk: List[int] = []
-        for j in range(begin, min(end, len(host))):
-            chunk.append(host[j])
-            decoded = self.decode_fn(chunk)
-            if ")" in decoded:
-                return decoded.index(")"), (decoded, j)
-        return -1, None
+    def _grow(self, window: List[int]) -> Tuple[str, int]:
+        """(text before ')', index of the token that closes it) of the shortest decodable prefix, or ("", -1)."""
+        for j in range(len(window)):
+            target, closed, _ = self.decode_fn(window[:j + 1]).partition(")")
+            if closed:
+                return target, j
+        return "", -1

@@ -271,17 +271,17 @@ def from_reference(doc_spans: Sequence[Any], link_to_target: Optional[Dict[int, 
                    max_grants_cap: int = 64, device: Optional[torch.device] = None) -> MaskSpec:
     """MaskSpec equal to the reference's mask for these spans and matched links
     (``doc_causal`` when ``link_to_target`` is None or empty)."""
-    device = torch.device("cuda") if device is None else device
+    device = torch.device("cuda" if device is None else device)
+    if device.type == "cuda":
+        # grants, classes on segment boundaries and link bits in native code (what ordered_grants and grant_segments
+        # do); per-token ids are filled on the device, nothing of length T crosses PCIe
+        pairs = [(int(pos), int(tgt)) for pos in sorted(link_to_target) for tgt in link_to_target[pos]] if link_to_target else []
+        return MaskSpec(*_lib.ops().pack_mask.default(*[[int(getattr(s, n)) for s in doc_spans] for n in ("start", "end", "doc_id")],
+                                                      [p for p, _ in pairs], [t for _, t in pairs], seq_len, max_grants_cap, device))
     ids = torch.from_numpy(build_document_ids(seq_len, doc_spans))[None].to(device)
-    if not link_to_target:
-        return MaskSpec(doc_ids=ids)
-    grants = ordered_grants(seq_len, doc_spans, link_to_target, max_grants_cap)
+    grants = ordered_grants(seq_len, doc_spans, link_to_target, max_grants_cap) if link_to_target else []
     if not grants:
         return MaskSpec(doc_ids=ids)
-    if torch.device(device).type == "cuda":  # classes on segment boundaries (host, O(G^2)); per-token ids filled on the device
-        (qb, qi), (kb, ki), link = grant_segments(grants)
-        return MaskSpec(doc_ids=ids, link_bits=torch.from_numpy(link)[None].to(device),
-                        q_row_ids=segment_ids(qb, qi, seq_len, device), kv_col_ids=segment_ids(kb, ki, seq_len, device))
     row, col, link = grant_classes(seq_len, grants)
     return MaskSpec(doc_ids=ids, link_bits=torch.from_numpy(link)[None].to(device),
                     q_row_ids=torch.from_numpy(row)[None].to(device), kv_col_ids=torch.from_numpy(col)[None].to(device))
@@ -322,10 +322,13 @@ class CrossDocLinkMaskCreator:
             index[self.link_detector.index_doc_span(span)] = (span.doc_id, span.start)
         out: Dict[int, List[int]] = {}
         for link in links:
-            hit = index.get(link.target_str)
-            if hit is None or hit[1] >= link.link_end_pos:
+            hit, pos = index.get(link.target_str), link.link_end_pos
+            if hit is None or hit[1] >= pos:
                 continue
-            out.setdefault(link.link_end_pos, []).append(hit[0])
+            if pos in out:
+                out[pos].append(hit[0])
+            else:
+                out[pos] = [hit[0]]
         return out
 
     def __call__(self, tokens: torch.Tensor, doc_spans: List[Any], **kwargs) -> MaskSpec:

@@ -90,7 +90,7 @@ int ts2ts_attn_fwd(const void* q, const void* k, const void* v, const int64_t* q
  *   doc_ids, q_row_ids, kv_col_ids   int32 [B,Tk] (classes of every cached token; the query's are those at q_pos)
  *   q_pos        device int32[B]: position of the query token, or NULL = Tk - 1
  *   out          bf16 [B,H,1,D]; lse fp32 [B,H] natural log; a token that may read no key gets out = 0, lse = -inf
- *   workspace    ts2ts_attn_decode_workspace_bytes(B,H,Tk,D) bytes, 256-byte aligned
+ *   workspace    not used any more: any pointer, NULL included (ts2ts_attn_decode_workspace_bytes stays valid to call)
  * Keys after q_pos are never read.  No block plan is needed: the mask row is evaluated per key. */
 size_t ts2ts_attn_decode_workspace_bytes(int B, int H, int Tk, int D);
 int ts2ts_attn_decode(const void* q, const void* k_cache, const void* v_cache, const int64_t* q_strides,

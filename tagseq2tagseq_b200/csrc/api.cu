@@ -44,7 +44,7 @@ cudaError_t launch_adamw(int count, float* const* p, const float* const* g, floa
 size_t decode_workspace_bytes(int B, int H, int Tk, int D);
 int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq, const int64_t* sk, const int64_t* sv, int B, int H,
                   int Tk, int D, float scale, MaskArgs M, const int32_t* q_pos, void* out, const int64_t* so, float* lse,
-                  void* workspace, cudaStream_t stream);
+                  cudaStream_t stream);
 
 }  // namespace ts2ts
 
@@ -191,11 +191,9 @@ int ts2ts_attn_decode(const void* q, const void* k_cache, const void* v_cache, c
     return r;
   if (lse == nullptr) return fail(-3, "lse: null pointer");
   if ((r = check_mask(doc_ids, link_bits, R, W))) return r;
-  if (workspace == nullptr || !aligned(workspace, 256)) return fail(-9, "workspace must be a 256-byte aligned device buffer");
-  if (workspace_bytes < decode_workspace_bytes(B, H, Tk, D))
-    return fail(-9, "workspace too small: %zu < %zu", workspace_bytes, decode_workspace_bytes(B, H, Tk, D));
+  (void)workspace; (void)workspace_bytes;  // nothing is kept in global memory between the blocks
   r = launch_decode(q, k_cache, v_cache, q_strides, k_strides, v_strides, B, H, Tk, D, scale,
-                    mask_args(doc_ids, q_row_ids, kv_col_ids, link_bits, R, W), q_pos, out, out_strides, lse, workspace,
+                    mask_args(doc_ids, q_row_ids, kv_col_ids, link_bits, R, W), q_pos, out, out_strides, lse,
                     static_cast<cudaStream_t>(stream));
   if (r) return fail(r, "decode launch failed (code %d, CUDA: %s)", r, cudaGetErrorString(cudaPeekAtLastError()));
   return 0;

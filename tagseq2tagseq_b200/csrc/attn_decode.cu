@@ -7,21 +7,28 @@
 //     allowed(kv) = kv <= q_pos  and  ( doc_ids[q_pos] == doc_ids[kv]  or  bit(link_bits[row(q_pos)], col(kv)) ),
 // the same predicate as the training kernels (cross_doc_mask.py:348-357), evaluated per key; no block plan is needed.
 //
-// HBM-bound work (every allowed key's K and V row is read once, 4 D bytes per key and head), split over the keys:
-//   decode_partial_kernel   grid (key tiles of 128, H, B), 128 threads.  A tile none of whose keys is allowed costs
-//                           one predicate per key and no K / V traffic.  Otherwise a half-warp reads one 2 D-byte K
-//                           row per step (16 bytes per lane), the scores of the tile are softmax-ed locally in base
-//                           2, and each thread accumulates its 8 (D = 128) or 4 (D = 64) output columns over the
-//                           tile's V rows.  Result per tile: running maximum, sum and unnormalised output row.
-//   decode_combine_kernel   grid (H, B), D threads: merges the tiles' partial results and writes out (bf16) and the
-//                           natural-log LSE.  A token that may read no key gets out = 0, LSE = -inf.
+// HBM-bound work: every allowed key's K and V row is read once, 4 D bytes per key and head.  One launch, grid
+// (cluster size, H, B), 16 warps a block.  The warps of a cluster share one (batch, head): warp w of W takes the groups of
+// 32 keys w, w + W, w + 2 W, ..., so that stretches without an allowed key spread over all of them.  It evaluates the mask
+// for up to four groups at a time (lane = key), queues the allowed keys in shared memory, and takes them off the queue
+// kUnroll at a time per row of lanes (D / 8 lanes hold one row, 16 bytes each), the K and V rows of all of them in flight
+// together: masked keys cost no traffic and no lane.  Each row of lanes keeps an online softmax (base 2) of its own; they
+// are merged by shuffles inside a warp, through shared memory inside a block and through distributed shared memory inside
+// the cluster, so no partial result goes to global memory.
+//
+// B = 2, H = 16, Tk = 32768, D = 128, 13.9 k allowed keys a sequence (228 MB): two kernels over fixed 128-key tiles with K
+// before V took 75 + 41 us (a third of the copy rate; the merge walked 256 partial results one after the other).
 #include "plan.h"
+#include "ptx.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
 namespace ts2ts {
+
+namespace cg = cooperative_groups;
 
 struct DecodeParams {
   const __nv_bfloat16 *q, *k, *v;
@@ -29,193 +36,224 @@ struct DecodeParams {
   int64_t k_sb, k_sh, k_st, v_sb, v_sh, v_st;
   MaskArgs mask;                   // per-token arrays are [B,Tk]
   const int32_t* q_pos;            // [B] position of the query token in the cache, or nullptr = Tk - 1
-  float* part;                     // [B,H,NB,2 + D]: m (base-2 exponent), l, o[D]
   __nv_bfloat16* out;              // [B,H,1,D]
   int64_t o_sb, o_sh;
   float* lse;                      // [B,H]
-  int B, H, Tk, NB;
+  int H, Tk;
   float scale_log2;
 };
 
+constexpr int kDecWarps = 16, kDecGroups = 4, kUnroll = 4;
+
+__device__ __forceinline__ void row_dot(const uint4& raw, const float (&q)[8], float& acc) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    acc = fmaf(__uint_as_float(w[i] << 16), q[2 * i], acc);
+    acc = fmaf(__uint_as_float(w[i] & 0xffff0000u), q[2 * i + 1], acc);
+  }
+}
+__device__ __forceinline__ void row_axpy(const uint4& raw, float p, float (&o)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    o[2 * i] = fmaf(p, __uint_as_float(w[i] << 16), o[2 * i]);
+    o[2 * i + 1] = fmaf(p, __uint_as_float(w[i] & 0xffff0000u), o[2 * i + 1]);
+  }
+}
+
 template <int D>
-__global__ void __launch_bounds__(128) decode_partial_kernel(const DecodeParams p) {
-  constexpr int kVec = D / 16;  // bf16 elements per lane when 16 lanes share a row: 8 (16 bytes) or 4 (8 bytes)
-  const int tile = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+__global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeParams p) {
+  constexpr int kLanes = D / 8;            // lanes that share a row
+  constexpr int kRows = 32 / kLanes;       // rows a warp reads at once
+  constexpr int kBatch = kRows * kUnroll;  // keys a warp takes off its queue at once
+  __shared__ int s_queue[kDecWarps][kDecGroups * 32 + kBatch];
+  __shared__ float s_m[kDecWarps], s_l[kDecWarps], s_o[kDecWarps][D];
+  __shared__ float s_block[2 + D];         // the block's maximum, sum and unnormalised output row, read by the cluster's first block
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int h = blockIdx.y, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cs = gridDim.x, W = cs * kDecWarps;
   const int qpos = p.q_pos ? min(max(p.q_pos[b], 0), p.Tk - 1) : p.Tk - 1;
-  float* part = p.part + (((size_t)b * p.H + h) * p.NB + tile) * (2 + D);
-  __shared__ float s_score[kTile];
-  __shared__ float s_o[4][D];
-  __shared__ float s_red[8];
-
-  // mask row of this tile: thread = key
-  const int kv = tile * kTile + tid;
-  bool ok = kv <= qpos;
-  if (ok) {
-    const size_t base = (size_t)b * p.Tk;
-    const int qdoc = p.mask.doc[base + qpos];
-    ok = p.mask.doc[base + kv] == qdoc;
-    if (!ok && p.mask.link != nullptr) {
-      const int row = p.mask.row[base + qpos], col = p.mask.col[base + kv];
-      if (row >= 0 && row < p.mask.R && col >= 0 && col < 64 * p.mask.W)
-        ok = (static_cast<unsigned long long>(p.mask.link[((size_t)b * p.mask.R + row) * p.mask.W + (col >> 6)]) >> (col & 63)) & 1ull;
+  const size_t base = (size_t)b * p.Tk;
+  const int32_t* docs = p.mask.doc + base;
+  const int32_t* cols = p.mask.col + base;
+  const int qdoc = docs[qpos];
+  const int64_t* link_row = nullptr;
+  if (p.mask.link != nullptr) {
+    const int row = p.mask.row[base + qpos];
+    if (row >= 0 && row < p.mask.R) link_row = p.mask.link + ((size_t)b * p.mask.R + row) * p.mask.W;
+  }
+  const int sub = lane / kLanes, at = (lane % kLanes) * 8;
+  const __nv_bfloat16* kbase = p.k + (size_t)b * p.k_sb + (size_t)h * p.k_sh + at;
+  const __nv_bfloat16* vbase = p.v + (size_t)b * p.v_sb + (size_t)h * p.v_sh + at;
+  float q[8], o[8];
+  {
+    const __nv_bfloat16* qrow = p.q + (size_t)b * p.q_sb + (size_t)h * p.q_sh + at;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      q[i] = __bfloat162float(qrow[i]) * p.scale_log2;
+      o[i] = 0.f;
     }
   }
-  if (!__syncthreads_or(ok)) {  // nothing to read in this tile
-    if (tid == 0) { part[0] = -CUDART_INF_F; part[1] = 0.f; }
-    return;
-  }
+  float m = -CUDART_INF_F, l = 0.f;
+  int* queue = s_queue[warp];
+  int queued = 0;
 
-  // scores: a half-warp per key row, 16 rows per warp and step
-  const int sub = lane >> 4, l16 = lane & 15;
-  const __nv_bfloat16* qrow = p.q + (size_t)b * p.q_sb + (size_t)h * p.q_sh + l16 * kVec;
-  float qf[kVec];
+  // `count` keys off the queue from `from`; slots past the last one repeat it with a score of -inf
+  auto take = [&](int from, int count) {
+    uint4 kr[kUnroll], vr[kUnroll];
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) qf[i] = __bfloat162float(qrow[i]);
-  const __nv_bfloat16* kbase = p.k + (size_t)b * p.k_sb + (size_t)h * p.k_sh;
-#pragma unroll 4
-  for (int it = 0; it < 16; ++it) {
-    const int r = warp * 32 + it * 2 + sub;  // key row inside the tile
-    const int key = tile * kTile + r;
-    float acc = 0.f;
-    if (key <= qpos) {
-      const __nv_bfloat16* krow = kbase + (size_t)key * p.k_st + l16 * kVec;
-      if (kVec == 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(krow);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int u = 0; u < kUnroll; ++u) {
+      const int key = queue[from + min(u * kRows + sub, count - 1)];
+      kr[u] = __ldg(reinterpret_cast<const uint4*>(kbase + (size_t)key * p.k_st));
+      vr[u] = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)key * p.v_st));
+    }
+    float s[kUnroll], mx = m;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(h2[i]);
-          acc = fmaf(f.x, qf[2 * i], acc);
-          acc = fmaf(f.y, qf[2 * i + 1], acc);
-        }
-      } else {
-        const uint2 raw = *reinterpret_cast<const uint2*>(krow);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int u = 0; u < kUnroll; ++u) {
+      s[u] = 0.f;
+      row_dot(kr[u], q, s[u]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float2 f = __bfloat1622float2(h2[i]);
-          acc = fmaf(f.x, qf[2 * i], acc);
-          acc = fmaf(f.y, qf[2 * i + 1], acc);
-        }
+      for (int x = kLanes / 2; x > 0; x >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], x);
+      if (u * kRows + sub >= count) s[u] = -CUDART_INF_F;
+      mx = fmaxf(mx, s[u]);
+    }
+    const float safe = mx == -CUDART_INF_F ? 0.f : mx;
+    const float f = fast_exp2(m - safe);  // exp2(-inf) = 0 before the first key
+    m = mx;
+    l *= f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] *= f;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const float pj = fast_exp2(s[u] - safe);
+      l += pj;
+      row_axpy(vr[u], pj, o);
+    }
+  };
+
+  const int n_groups = qpos / 32 + 1;
+  for (int g0 = blockIdx.x * kDecWarps + warp; g0 < n_groups; g0 += kDecGroups * W) {
+    int doc[kDecGroups], col[kDecGroups];
+#pragma unroll
+    for (int u = 0; u < kDecGroups; ++u) {
+      const int kv = (g0 + u * W) * 32 + lane;
+      doc[u] = kv <= qpos ? docs[kv] : 0;
+      col[u] = link_row != nullptr && kv <= qpos ? cols[kv] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kDecGroups; ++u) {
+      const int kv = (g0 + u * W) * 32 + lane;
+      bool ok = false;
+      if (kv <= qpos) {
+        ok = doc[u] == qdoc;
+        if (!ok && col[u] >= 0 && col[u] < 64 * p.mask.W)
+          ok = (static_cast<unsigned long long>(__ldg(link_row + (col[u] >> 6))) >> (col[u] & 63)) & 1ull;
       }
+      const unsigned bal = __ballot_sync(0xffffffffu, ok);
+      if (ok) queue[queued + __popc(bal & ((1u << lane) - 1u))] = kv;
+      queued += __popc(bal);
     }
-#pragma unroll
-    for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (l16 == 0) s_score[r] = acc * p.scale_log2;
+    __syncwarp();
+    int done = 0;
+    for (; queued - done >= kBatch; done += kBatch) take(done, kBatch);
+    const int left = queued - done;
+    const int kept = lane < left ? queue[done + lane] : 0;
+    __syncwarp();
+    if (lane < left) queue[lane] = kept;
+    queued = left;
+    __syncwarp();
   }
-  __syncthreads();
+  if (queued > 0) take(0, queued);
 
-  // softmax over the tile: thread = key again
-  const float sc = ok ? s_score[tid] : -CUDART_INF_F;
-  float m = sc;
+  // rows of lanes -> warp
+  float mw = m;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-  if (lane == 0) s_red[warp] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3]));  // finite: at least one key is allowed
-  const float pj = ok ? exp2f(sc - m) : 0.f;
-  float l = pj;
+  for (int x = kLanes; x < 32; x <<= 1) mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, x));
+  const float fw = m == -CUDART_INF_F ? 0.f : fast_exp2(m - mw);
+  l *= fw;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) l += __shfl_xor_sync(0xffffffffu, l, s);
-  if (lane == 0) s_red[4 + warp] = l;
-  s_score[tid] = pj;  // every thread rewrites only its own entry, which nobody else reads before the barrier
-  __syncthreads();
-  l = (s_red[4] + s_red[5]) + (s_red[6] + s_red[7]);
-
-  // output: the same half-warp per V row layout; each lane keeps kVec columns
-  float of[kVec];
+  for (int i = 0; i < 8; ++i) o[i] *= fw;
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) of[i] = 0.f;
-  const __nv_bfloat16* vbase = p.v + (size_t)b * p.v_sb + (size_t)h * p.v_sh;
-#pragma unroll 4
-  for (int it = 0; it < 16; ++it) {
-    const int r = warp * 32 + it * 2 + sub;
-    const float w = s_score[r];
-    if (w != 0.f) {
-      const __nv_bfloat16* vrow = vbase + (size_t)(tile * kTile + r) * p.v_st + l16 * kVec;
-      if (kVec == 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(vrow);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  for (int x = kLanes; x < 32; x <<= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, x);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(h2[i]);
-          of[2 * i] = fmaf(w, f.x, of[2 * i]);
-          of[2 * i + 1] = fmaf(w, f.y, of[2 * i + 1]);
-        }
-      } else {
-        const uint2 raw = *reinterpret_cast<const uint2*>(vrow);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float2 f = __bfloat1622float2(h2[i]);
-          of[2 * i] = fmaf(w, f.x, of[2 * i]);
-          of[2 * i + 1] = fmaf(w, f.y, of[2 * i + 1]);
-        }
-      }
-    }
+    for (int i = 0; i < 8; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], x);
   }
-#pragma unroll
-  for (int i = 0; i < kVec; ++i) of[i] += __shfl_xor_sync(0xffffffffu, of[i], 16);  // the two half-warps of a warp
   if (sub == 0) {
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) s_o[warp][l16 * kVec + i] = of[i];
+    for (int i = 0; i < 8; ++i) s_o[warp][at + i] = o[i];
   }
+  if (lane == 0) { s_m[warp] = mw; s_l[warp] = l; }
   __syncthreads();
-  if (tid < D) part[2 + tid] = (s_o[0][tid] + s_o[1][tid]) + (s_o[2][tid] + s_o[3][tid]);
-  if (tid == 0) { part[0] = m; part[1] = l; }
-}
-
-template <int D>
-__global__ void __launch_bounds__(D) decode_combine_kernel(const DecodeParams p) {
-  const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
-  const float* part = p.part + ((size_t)b * p.H + h) * p.NB * (2 + D);
-  float m = -CUDART_INF_F;
-  for (int t = 0; t < p.NB; ++t) m = fmaxf(m, part[(size_t)t * (2 + D)]);
-  float l = 0.f, o = 0.f;
-  if (m > -CUDART_INF_F) {
-    for (int t = 0; t < p.NB; ++t) {
-      const float mt = part[(size_t)t * (2 + D)];
-      if (mt == -CUDART_INF_F) continue;
-      const float w = exp2f(mt - m);
-      l = fmaf(w, part[(size_t)t * (2 + D) + 1], l);
-      o = fmaf(w, part[(size_t)t * (2 + D) + 2 + d], o);
+  // warps -> block
+  const int d = threadIdx.x;
+  if (d < D) {
+    float mb = s_m[0];
+#pragma unroll
+    for (int w = 1; w < kDecWarps; ++w) mb = fmaxf(mb, s_m[w]);
+    float lb = 0.f, ob = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) {
+      const float f = s_m[w] == -CUDART_INF_F ? 0.f : fast_exp2(s_m[w] - mb);
+      lb = fmaf(f, s_l[w], lb);
+      ob = fmaf(f, s_o[w][d], ob);
     }
+    if (d == 0) { s_block[0] = mb; s_block[1] = lb; }
+    s_block[2 + d] = ob;
   }
-  p.out[(size_t)b * p.o_sb + (size_t)h * p.o_sh + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
-  if (d == 0) p.lse[(size_t)b * p.H + h] = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -CUDART_INF_F;
+  cluster.sync();
+  // blocks -> out
+  if (blockIdx.x == 0 && d < D) {
+    float mc = -CUDART_INF_F;
+    for (int r = 0; r < cs; ++r) mc = fmaxf(mc, *cluster.map_shared_rank(&s_block[0], r));
+    float lc = 0.f, oc = 0.f;
+    for (int r = 0; r < cs; ++r) {
+      const float mr = *cluster.map_shared_rank(&s_block[0], r);
+      if (mr == -CUDART_INF_F) continue;
+      const float f = fast_exp2(mr - mc);
+      lc = fmaf(f, *cluster.map_shared_rank(&s_block[1], r), lc);
+      oc = fmaf(f, *cluster.map_shared_rank(&s_block[2 + d], r), oc);
+    }
+    p.out[(size_t)b * p.o_sb + (size_t)h * p.o_sh + d] = __float2bfloat16(lc > 0.f ? oc / lc : 0.f);
+    if (d == 0) p.lse[(size_t)b * p.H + h] = lc > 0.f ? (mc + log2f(lc)) * 0.6931471805599453f : -CUDART_INF_F;
+  }
+  cluster.sync();  // the first block has read the others' shared memory
 }
 
-size_t decode_workspace_bytes(int B, int H, int Tk, int D) {
-  const size_t nb = (size_t)((Tk + kTile - 1) / kTile);
-  return plan_align((size_t)B * H * nb * (2 + D) * sizeof(float));
-}
+// No partial results go through global memory; the argument stays part of the interface.
+size_t decode_workspace_bytes(int, int, int, int) { return 256; }
 
 int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq, const int64_t* sk, const int64_t* sv, int B, int H,
                   int Tk, int D, float scale, MaskArgs M, const int32_t* q_pos, void* out, const int64_t* so, float* lse,
-                  void* workspace, cudaStream_t stream) {
+                  cudaStream_t stream) {
   DecodeParams p;
   p.q = static_cast<const __nv_bfloat16*>(q); p.k = static_cast<const __nv_bfloat16*>(k); p.v = static_cast<const __nv_bfloat16*>(v);
   p.q_sb = sq[0]; p.q_sh = sq[1];
   p.k_sb = sk[0]; p.k_sh = sk[1]; p.k_st = sk[2];
   p.v_sb = sv[0]; p.v_sh = sv[1]; p.v_st = sv[2];
   p.mask = M; p.q_pos = q_pos;
-  p.part = static_cast<float*>(workspace);
   p.out = static_cast<__nv_bfloat16*>(out); p.o_sb = so[0]; p.o_sh = so[1];
   p.lse = lse;
-  p.B = B; p.H = H; p.Tk = Tk; p.NB = (Tk + kTile - 1) / kTile;
+  p.H = H; p.Tk = Tk;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const dim3 grid(p.NB, H, B);
-  if (D == 128) {
-    decode_partial_kernel<128><<<grid, 128, 0, stream>>>(p);
-    decode_combine_kernel<128><<<dim3(H, B), 128, 0, stream>>>(p);
-  } else if (D == 64) {
-    decode_partial_kernel<64><<<grid, 128, 0, stream>>>(p);
-    decode_combine_kernel<64><<<dim3(H, B), 64, 0, stream>>>(p);
-  } else {
-    return -142;
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -141;
+  // Blocks per (batch, head): twice the SM count in all, as long as every warp gets two groups of keys; eight is the
+  // largest cluster every part of the chip takes.
+  const long long groups = (Tk + 31) / 32;
+  int cs = 1;
+  while (cs < 8 && (long long)B * H * cs < 2 * 148 && groups >= 2ll * kDecWarps * 2 * cs) cs *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs, H, B);
+  cfg.blockDim = dim3(kDecWarps * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cs; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (D == 128) return cudaLaunchKernelEx(&cfg, decode_kernel<128>, p) == cudaSuccess ? 0 : -141;
+  if (D == 64) return cudaLaunchKernelEx(&cfg, decode_kernel<64>, p) == cudaSuccess ? 0 : -141;
+  return -142;
 }
 
 }  // namespace ts2ts

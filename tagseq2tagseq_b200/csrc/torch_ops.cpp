@@ -178,13 +178,12 @@ std::tuple<Tensor, Tensor> attn_decode_cuda(const Tensor& q_, const Tensor& k_, 
   const Tensor q = rowmajor(q_), k = rowmajor(k_), v = rowmajor(v_);
   const int B = k.size(0), H = k.size(1), Tk = k.size(2), D = k.size(3);
   Tensor out = at::empty({B, H, 1, D}, q.options()), lse = at::empty({B, H}, q.options().dtype(at::kFloat));
-  Tensor ws = at::empty({static_cast<int64_t>(ts2ts_attn_decode_workspace_bytes(B, H, Tk, D))}, q.options().dtype(at::kByte));
   const MaskPtrs m(doc_ids, link_bits, q_row_ids, kv_col_ids);
   const Tensor pos = q_pos.has_value() ? q_pos->contiguous() : Tensor();
   check(ts2ts_attn_decode(q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), Strides3(q).s, Strides3(k).s, Strides3(v).s, B, H, Tk,
                           D, static_cast<float>(scale), m.doc, m.row, m.col, m.link, m.R, m.W,
                           pos.defined() ? pos.const_data_ptr<int32_t>() : nullptr, out.mutable_data_ptr(), Strides3(out).s,
-                          lse.mutable_data_ptr<float>(), ws.mutable_data_ptr(), ws.numel(), stream_of(q)),
+                          lse.mutable_data_ptr<float>(), nullptr, 0, stream_of(q)),
         "ts2ts_attn_decode");
   return {out, lse};
 }

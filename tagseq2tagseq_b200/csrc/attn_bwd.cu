@@ -69,7 +69,6 @@ struct BwdParams {
 
 constexpr int kBwdThreads = 512;  // warps 0-7 exp/dS, 8-11 dQ reduction, 12 TMA producer, 13 MMA issuer, 14-15 idle
 constexpr int kSubQ = 64;         // query columns per compute half
-constexpr int kRunSlotsB = 4;     // runs of a partial query tile that the producer copies to shared memory
 #ifndef TS2TS_BWD_X2
 #define TS2TS_BWD_X2 1
 #endif
@@ -96,7 +95,7 @@ struct BwdSmem {
   // alignment slack.  The kernel declares no static shared memory, so the dynamic region normally starts 1024-byte
   // aligned and the slack stays unused; if it ever does not fit, the kernel reports status 2900 instead of running.
   static constexpr int kTiles = 5 * kTileBytes + kDsBytes + kStageBytes;
-  static constexpr int kSmall = 4 * kTile * 4 + 16 * 8 + 16 + 2 * kRunSlotsB * 16 + 16;  // statistics, barriers, flags, staged runs
+  static constexpr int kSmall = 4 * kTile * 4 + 16 * 8 + 16 + 2 * kMaskRuns * 16;  // statistics, barriers, flags, staged masks
   static constexpr int kSlack = 512;
   static constexpr int kBytes = kTiles + kSmall + kSlack;
   // tensor-memory columns: dV, dK accumulators, S^T (later P^T / dS^T), dP^T (later dQ^T)
@@ -106,50 +105,41 @@ struct BwdSmem {
 template <uint32_t N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// What a backward thread knows about its key: document, column class, and how it looks up "may row class r read my
-// column class": 0 = never (no links, or the key has no class), 1 = words of the transposed table kept in registers
-// (R <= 256), 2 = words of the transposed table read from global memory, 3 = the untransposed table (no transposed
-// one was built).
-struct KeyCtx {
-  int kvdoc, kvcol, mode;
-  unsigned long long lt0, lt1, lt2, lt3;
-  const unsigned long long* lt_row;
-  const int64_t* link_col;  // &link[b][0][kvcol >> 6]
-};
-__device__ __forceinline__ bool row_class_allowed(const KeyCtx& k, const MaskArgs& M, int row) {
-  if (k.mode == 0 || row < 0 || row >= M.R) return false;
-  unsigned long long w;
-  if (k.mode == 1) {
-    const int wi = row >> 6;
-    w = wi == 0 ? k.lt0 : wi == 1 ? k.lt1 : wi == 2 ? k.lt2 : k.lt3;
-    return (w >> (row & 63)) & 1ull;
-  }
-  if (k.mode == 2) return (__ldg(k.lt_row + (row >> 6)) >> (row & 63)) & 1ull;
-  return (static_cast<unsigned long long>(__ldg(k.link_col + (size_t)row * M.W)) >> (k.kvcol & 63)) & 1ull;
-}
-// 128-bit mask of the query rows of tile `qb` that may read this thread's key, before causality.  The first
-// kRunSlotsB runs come from shared memory (`staged`), further ones from the plan in global memory.
-__device__ __forceinline__ void allowed_rows(const PlanView& P, const MaskArgs& M, int b, int qb, const KeyCtx& k,
-                                             const int4* staged, int n, uint32_t (&bits)[4]) {
-  bits[0] = bits[1] = bits[2] = bits[3] = 0u;
-  const Run* runs = P.runs + ((size_t)b * P.NB + qb) * kTile;
-  const int n_valid = min(kTile, P.T - qb * kTile);
-  auto get_run = [&](int r) { return r < kRunSlotsB ? staged[r] : __ldg(reinterpret_cast<const int4*>(runs + r)); };
-  int4 cur = n > 0 ? get_run(0) : make_int4(0, 0, 0, 0);
+// 128-bit mask of the query rows of tile qb that may read key `row` of tile kb, before causality, from the run lists: the
+// way out for keys that the plan's mask table does not cover (see kMaskRuns).  "May row class r read my column class" is
+// looked up in the transposed table where the pre-pass built one.
+__device__ __noinline__ uint4 key_mask(const PlanView& P, const MaskArgs& M, int b, int qb, int kb, int row) {
+  const int kv = kb * kTile + row;
+  if (kv >= P.T) return make_uint4(0u, 0u, 0u, 0u);
+  const int kvdoc = M.doc[(size_t)b * P.T + kv], kvcol = M.col[(size_t)b * P.T + kv];
+  const bool linked = M.link != nullptr && kvcol >= 0 && kvcol < 64 * M.W;
+  const unsigned long long* lt_row = nullptr;
+  const int64_t* link_col = nullptr;
+  if (linked && P.status[kLinkTRows] == M.R && kvcol < kLinkTMaxCols) lt_row = P.link_t + ((size_t)b * kLinkTMaxCols + kvcol) * kLinkTWords;
+  else if (linked) link_col = M.link + (size_t)b * M.R * M.W + (kvcol >> 6);
+  const size_t tq = (size_t)b * P.NB + qb;
+  const int4* runs = reinterpret_cast<const int4*>(P.runs + tq * kTile);
+  const int n = min(__ldg(&P.run_cnt[tq]), kTile), n_valid = min(kTile, P.T - qb * kTile);
+  uint32_t bits[4] = {0u, 0u, 0u, 0u};
+  int4 cur = __ldg(runs);
   uint32_t lo[4];
   prefix_mask(cur.x, lo);
   for (int r = 0; r < n; ++r) {
-    const int4 nx = r + 1 < n ? get_run(r + 1) : make_int4(n_valid, 0, 0, 0);
+    const int4 nx = r + 1 < n ? __ldg(runs + r + 1) : make_int4(n_valid, 0, 0, 0);
     uint32_t hi[4];
     prefix_mask(nx.x, hi);  // the run covers rows [cur.x, nx.x)
-    if (cur.y == k.kvdoc || row_class_allowed(k, M, cur.z)) {
+    bool allowed = cur.y == kvdoc;
+    if (!allowed && linked && cur.z >= 0 && cur.z < M.R)
+      allowed = lt_row != nullptr ? (__ldg(lt_row + (cur.z >> 6)) >> (cur.z & 63)) & 1ull
+                                  : (static_cast<unsigned long long>(__ldg(link_col + (size_t)cur.z * M.W)) >> (kvcol & 63)) & 1ull;
 #pragma unroll
-      for (int w = 0; w < 4; ++w) bits[w] |= hi[w] & ~lo[w];
+    for (int w = 0; w < 4; ++w) {
+      if (allowed) bits[w] |= hi[w] & ~lo[w];
+      lo[w] = hi[w];
     }
-#pragma unroll
-    for (int w = 0; w < 4; ++w) lo[w] = hi[w];
     cur = nx;
   }
+  return make_uint4(bits[0], bits[1], bits[2], bits[3]);
 }
 
 // The per-tile arithmetic of a compute thread, 32 query columns at a time, in two phases so that the first can run
@@ -231,7 +221,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
                 const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV,
-                const __grid_constant__ CUtensorMap mapDQ, const BwdParams p) {
+                const __grid_constant__ CUtensorMap mapDQ, const __grid_constant__ BwdParams p) {
   using Cfg = BwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   // Plain pointer arithmetic (no round trip through an integer) keeps the shared address space visible to the
@@ -259,8 +249,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(reinterpret_cast<uint8_t*>(bars + 16) + 4);
   int* abort_w = const_cast<int*>(abort_ptr);
-  int4* s_runs = reinterpret_cast<int4*>(bars + 18);                  // [2 stages][kRunSlotsB] first runs of a partial query tile
-  int* s_nruns = reinterpret_cast<int*>(s_runs + 2 * kRunSlotsB);     // [2] its number of runs
+  uint4* s_masks = reinterpret_cast<uint4*>(bars + 18);               // [2 stages][kMaskRuns] the pair's masks, by run of the key
   {  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
     int bad = 0;
     const int32_t* stw = p.plan.status;
@@ -350,16 +339,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const int entry = list[i];
         const int qb = min(entry & ~kFullBit, NB - 1);
         const int st = i & 1;
-        if (!(entry & kFullBit)) {
-          // partial tile: its first runs travel with the stage (the arrive below publishes these plain stores)
-          const size_t tq = (size_t)b * NB + qb;
-          const int4* src = reinterpret_cast<const int4*>(P.runs + tq * kTile);
-          const int4 r0 = __ldg(src), r1 = __ldg(src + 1), r2 = __ldg(src + 2), r3 = __ldg(src + 3);
-          s_nruns[st] = min(max(__ldg(&P.run_cnt[tq]), 0), kTile);
-          s_runs[st * kRunSlotsB + 0] = r0; s_runs[st * kRunSlotsB + 1] = r1;
-          s_runs[st * kRunSlotsB + 2] = r2; s_runs[st * kRunSlotsB + 3] = r3;
-        }
-        mbar_expect_tx(&bar_q_full[st], Cfg::kTileBytes + 2 * kTile * 4);
+        const bool masks = !(entry & kFullBit) && P.kv_mask != nullptr;  // partial tile: its masks travel with the stage
+        mbar_expect_tx(&bar_q_full[st], Cfg::kTileBytes + 2 * kTile * 4 + (masks ? kMaskRuns * 16 : 0));
+        if (masks)
+          bulk_load(s_masks + st * kMaskRuns, P.kv_mask + ((size_t)b * ((size_t)NB * (NB + 1) / 2) + mask_pair(qb, kb)) * kMaskRuns, kMaskRuns * 16,
+                    &bar_q_full[st]);
         for (int s = 0; s < Cfg::kSub; ++s)
           tma_load_4d(sQ + st * Cfg::kTileBytes + s * 16384, &mapQ, &bar_q_full[st], s * 64, qb * kTile, h, b);
         const size_t stat = ((size_t)b * p.H + h) * p.Tp + (size_t)qb * kTile;
@@ -519,30 +503,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int row = tid & (kTile - 1), half = tid >> 7;
     const int kv = kb * kTile + row;
     const bool kv_valid = kv < P.T;
-    KeyCtx key;
-    key.kvdoc = kv_valid ? p.mask.doc[(size_t)b * P.T + kv] : INT32_MIN;
-    key.kvcol = kv_valid ? p.mask.col[(size_t)b * P.T + kv] : -1;
-    key.mode = 0;
-    key.lt0 = key.lt1 = key.lt2 = key.lt3 = 0ull;
-    key.lt_row = nullptr;
-    key.link_col = nullptr;
-    if (p.mask.link != nullptr && key.kvcol >= 0 && key.kvcol < 64 * p.mask.W) {
-      const int t_rows = P.status[kLinkTRows];
-      if (t_rows == p.mask.R && key.kvcol < kLinkTMaxCols) {
-        key.lt_row = P.link_t + ((size_t)b * kLinkTMaxCols + key.kvcol) * kLinkTWords;
-        if (t_rows <= 256) {
-          key.mode = 1;
-          key.lt0 = __ldg(key.lt_row);
-          if (t_rows > 64) key.lt1 = __ldg(key.lt_row + 1);
-          if (t_rows > 128) key.lt2 = __ldg(key.lt_row + 2);
-          if (t_rows > 192) key.lt3 = __ldg(key.lt_row + 3);
-        } else {
-          key.mode = 2;
-        }
-      } else {
-        key.mode = 3;
-        key.link_col = p.mask.link + (size_t)b * p.mask.R * p.mask.W + (key.kvcol >> 6);
-      }
+    int run = kMaskRuns;  // this key's row of the mask table: the number of its run inside the tile
+    if (P.kv_mask != nullptr) {
+      const size_t tk = (size_t)b * NB + kb;
+      const int nr = __ldg(&P.run_cnt[tk]);
+#pragma unroll
+      for (int r = 0; r < kMaskRuns + 1; ++r)
+        if (r < nr && __ldg(&P.runs[tk * kTile + r].start) <= row) run = r;
     }
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
@@ -552,10 +519,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const int entry = list[i];
       const int qb = min(entry & ~kFullBit, NB - 1);
       const bool masked = (entry & kFullBit) == 0;
-      if (!(ok = mbar_wait(&bar_q_full[st], (i >> 1) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and staged runs of this tile landed
+      if (!(ok = mbar_wait(&bar_q_full[st], (i >> 1) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
       uint32_t bits[4] = {0, 0, 0, 0};
       if (masked) {
-        allowed_rows(P, p.mask, b, qb, key, s_runs + st * kRunSlotsB, s_nruns[st], bits);
+        const uint4 m4 = run < kMaskRuns ? s_masks[st * kMaskRuns + run] : key_mask(P, p.mask, b, qb, kb, row);
+        bits[0] = m4.x; bits[1] = m4.y; bits[2] = m4.z; bits[3] = m4.w;
         if (!kv_valid) bits[0] = bits[1] = bits[2] = bits[3] = 0u;
         if (kb == qb) {  // causal inside the diagonal tile: query rows row..127
 #pragma unroll

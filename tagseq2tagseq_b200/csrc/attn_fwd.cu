@@ -12,8 +12,8 @@
 //   tcgen05   S = Q K^T                       (bf16 x bf16 -> fp32, 128 columns of tensor memory)
 //   softmax   the row's 128 scores are read into registers in one go and the S columns are handed back at
 //             once, so that the issuer can compute S of the NEXT key tile while this one is being exponentiated;
-//             mask (partial tiles only: one select per element against a per-row 128-bit column mask built from
-//             the tile's runs; 32-column chunks that are masked for a whole warp are skipped), online softmax in
+//             mask (partial tiles only: one select per element against a per-row 128-bit column mask that the pre-pass
+//             worked out; 32-column chunks that are masked for a whole warp are skipped), online softmax in
 //             base 2, P -> bf16 -> shared memory (K-major, 128-byte swizzle)
 //   tcgen05   O += P V                        (both operands from shared memory, V MN-major)
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
@@ -88,7 +88,6 @@ constexpr float kRescaleThreshold = 8.0f;
 #ifndef TS2TS_FWD_DUAL
 #define TS2TS_FWD_DUAL 1
 #endif
-constexpr int kRunSlots = 8;  // runs of a partial tile that travel through shared memory; further ones are read from global memory
 // Barrier among the 128 threads of softmax team t (hardware barrier 1 + t; barrier 0 is __syncthreads).
 __device__ __forceinline__ void team_sync(int t) {
   if (t == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -106,7 +105,7 @@ struct FwdSmem {
   static constexpr int kRing = kP + 2 * kPBytes;             // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
   static constexpr int kBars = 18 + 2 * kStages;
-  static constexpr int kSmallBytes = kBars * 8 + 16 + 4 * kStages + 8 + 8 * kRunSlots * 16;  // barriers, words, run copies
+  static constexpr int kSmallBytes = kBars * 8 + 16 + 4 * kStages;  // barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
 };
 
@@ -177,10 +176,42 @@ struct UnionWalk {
   }
 };
 
+// 128-bit mask of the key columns of tile kb that row `row` of tile qb may read, before causality, from the run lists: the
+// way out for rows that the plan's mask table does not cover.  Kept out of line: it is rare, and the softmax loop's code is
+// what the instruction cache has to hold.
+__device__ __noinline__ uint4 row_mask(const PlanView& P, const MaskArgs& M, int b, int qb, int kb, int row) {
+  const int q = qb * kTile + row;
+  if (q >= P.T) return make_uint4(0u, 0u, 0u, 0u);
+  const int mydoc = M.doc[(size_t)b * P.T + q], myrow = M.row[(size_t)b * P.T + q];
+  const int64_t* link_row = (M.link != nullptr && myrow >= 0 && myrow < M.R) ? M.link + ((size_t)b * M.R + myrow) * M.W : nullptr;
+  const size_t tk = (size_t)b * P.NB + kb;
+  const int4* runs = reinterpret_cast<const int4*>(P.runs + tk * kTile);
+  const int n = min(__ldg(&P.run_cnt[tk]), kTile), n_valid = min(kTile, P.T - kb * kTile);
+  uint32_t bits[4] = {0u, 0u, 0u, 0u};
+  int4 cur = __ldg(runs);
+  uint32_t lo[4];
+  prefix_mask(cur.x, lo);
+  for (int r = 0; r < n; ++r) {
+    const int4 nx = r + 1 < n ? __ldg(runs + r + 1) : make_int4(n_valid, 0, 0, 0);
+    uint32_t hi[4];
+    prefix_mask(nx.x, hi);
+    bool allowed = cur.y == mydoc;
+    if (!allowed && link_row != nullptr && cur.w >= 0 && cur.w < 64 * M.W)
+      allowed = (static_cast<unsigned long long>(__ldg(link_row + (cur.w >> 6))) >> (cur.w & 63)) & 1ull;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      if (allowed) bits[w] |= hi[w] & ~lo[w];
+      lo[w] = hi[w];
+    }
+    cur = nx;
+  }
+  return make_uint4(bits[0], bits[1], bits[2], bits[3]);
+}
+
 template <int D>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
-                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const FwdParams p) {
+                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
   using Cfg = FwdSmem<D>;
   constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -206,7 +237,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
   int* abort_w = s_item + 3;
   uint32_t* s_ring_info = reinterpret_cast<uint32_t*>(s_item + 4);  // [kStages] kRing* bits of what each slot holds
-  int4* s_runs = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(bars) + ((Cfg::kBars * 8 + 16 + 4 * kStages + 15) & ~15));  // [8 warps][kRunSlots]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -390,7 +420,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const uint32_t tSr = tmem + t * kTile + lane_base;
     const uint32_t tOr = tmem + 2 * kTile + t * D + lane_base;
     uint8_t* sPt = sP + t * Cfg::kPBytes;
-    int4* my_runs = s_runs + warp * kRunSlots;  // this warp's copy of the current partial tile's first runs
     uint32_t n_tiles = 0;  // tiles this team has processed so far
     uint32_t n_epi = 0;    // items this team has finished
     FTRACE_ACC_DECL
@@ -419,52 +448,39 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         }
         continue;
       }
-      const int mydoc = q_valid ? p.mask.doc[(size_t)b * P.T + q] : INT32_MIN;
-      const int myrow = q_valid ? p.mask.row[(size_t)b * P.T + q] : -1;
-      // This row's link words stay in registers for the whole item when there are at most four of them (256 column
-      // classes); a lookup is then a select, not a load.
-      const int64_t* link_row = (p.mask.link != nullptr && myrow >= 0 && myrow < p.mask.R) ? p.mask.link + ((size_t)b * p.mask.R + myrow) * p.mask.W : nullptr;
-      const bool link_regs = p.mask.W <= 4;
-      unsigned long long lw0 = 0, lw1 = 0, lw2 = 0, lw3 = 0;
-      if (link_row != nullptr && link_regs) {
-        lw0 = static_cast<unsigned long long>(__ldg(link_row));
-        if (p.mask.W > 1) lw1 = static_cast<unsigned long long>(__ldg(link_row + 1));
-        if (p.mask.W > 2) lw2 = static_cast<unsigned long long>(__ldg(link_row + 2));
-        if (p.mask.W > 3) lw3 = static_cast<unsigned long long>(__ldg(link_row + 3));
+      // Row of the plan's mask table for this query row: the number of its run inside the tile.  Rows of runs past the
+      // table, and all rows of sequences without one, work their masks out from the run lists (row_mask).
+      const uint4* masks = nullptr;
+      if (P.q_mask != nullptr) {  // rows past the sequence take the last run's masks: nothing of theirs is stored
+        const size_t tq = (size_t)b * NB + qb;
+        const int nr = __ldg(&P.run_cnt[tq]);
+        int run = -1;
+#pragma unroll
+        for (int r = 0; r < kMaskRuns + 1; ++r)
+          if (r < nr && __ldg(&P.runs[tq * kTile + r].start) <= row) run = r;
+        if (run < kMaskRuns) masks = P.q_mask + ((size_t)b * ((size_t)NB * (NB + 1) / 2) + mask_pair(qb, 0)) * kMaskRuns + run;
       }
-      // List entries are fetched two tiles ahead and the runs of a partial tile one tile ahead (lanes 0-7 hold one run
-      // each), so that their latency hides behind the sweeps of the tile before.
+      // List entries are fetched two tiles ahead and the mask of a partial tile one tile ahead, so that their latency
+      // hides behind the sweeps of the tile before.
       int e_cur = ld_nc_i32_here(list);
       int e_nxt = n > 1 ? ld_nc_i32_here(list + 1) : 0;
-      int4 r_pf = make_int4(0, 0, 0, 0);
-      int n_pf = 0;
-      auto prefetch_runs = [&](int entry) {
+      int4 mask_pf = make_int4(0, 0, 0, 0);
+      auto prefetch_mask = [&](int entry) {
         if (entry & kFullBit) return;
-        const int kbp = min(max(entry & ~kFullBit, 0), NB - 1);
-        n_pf = ld_nc_i32_here(&P.run_cnt[(size_t)b * NB + kbp]);
-        if (lane < kRunSlots) r_pf = ld_nc_v4_here(P.runs + ((size_t)b * NB + kbp) * kTile + lane);
+        const int kbp = min(max(entry, 0), qb);
+        if (masks != nullptr) mask_pf = ld_nc_v4_here(masks + (size_t)kbp * kMaskRuns);
       };
-      prefetch_runs(e_cur);
+      prefetch_mask(e_cur);
       float m_used = -CUDART_INF_F, l = 0.f;
       FTRACE_ACC(0);
       for (int j = 0; j < n && ok; ++j) {
         const int entry = e_cur;
         e_cur = e_nxt;
-#ifdef TS2TS_EXPERIMENT_NOLIST
-        if (j + 2 < n) e_nxt = (j + 2) | (j + 2 < n - 1 ? kFullBit : 0);
-#else
         if (j + 2 < n) e_nxt = ld_nc_i32_here(list + j + 2);
-#endif
         const int kb = entry & ~kFullBit;
         if (kb < 0 || kb >= NB) { atomicCAS(abort_w, 0, 38); ok = false; break; }
-        int n_runs = 0;
-        if (!(entry & kFullBit)) {  // hand the prefetched runs to the whole warp
-          __syncwarp();
-          if (lane < kRunSlots) my_runs[lane] = r_pf;
-          n_runs = min(n_pf, kTile);
-          __syncwarp();
-        }
-        if (j + 1 < n) prefetch_runs(e_cur);
+        const int4 mask_cur = mask_pf;
+        if (j + 1 < n) prefetch_mask(e_cur);
         FTRACE_ACC(7);
 #if TS2TS_FWD_DUAL
         auto tile = [&](auto masked_tag) {
@@ -475,36 +491,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
         bool dead[4] = {false, false, false, false}, mixed[4] = {false, false, false, false};
         if (kMasked) {
-          // 128-bit mask of the key columns this row may read, before causality: walk the tile's runs
-          bits[0] = bits[1] = bits[2] = bits[3] = 0u;
-          const Run* runs_g = P.runs + ((size_t)b * NB + kb) * kTile;
-          const int n_valid = min(kTile, P.T - kb * kTile);
-          auto get_run = [&](int r) {
-            return r < kRunSlots ? my_runs[r] : __ldg(reinterpret_cast<const int4*>(runs_g + r));
-          };
-          int4 cur = n_runs > 0 ? get_run(0) : make_int4(0, 0, 0, 0);
-          for (int r = 0; r < n_runs; ++r) {
-            const int4 nx = r + 1 < n_runs ? get_run(r + 1) : make_int4(n_valid, 0, 0, 0);
-            const int start = cur.x, doc = cur.y, col = cur.w, end = nx.x;
-            bool allowed = doc == mydoc;
-            if (!allowed && link_row != nullptr && col >= 0 && col < 64 * p.mask.W) {
-              unsigned long long wbits;
-              if (link_regs) {
-                const int wi = col >> 6;
-                wbits = wi == 0 ? lw0 : wi == 1 ? lw1 : wi == 2 ? lw2 : lw3;
-              } else {
-                wbits = static_cast<unsigned long long>(__ldg(link_row + (col >> 6)));
-              }
-              allowed = (wbits >> (col & 63)) & 1ull;
-            }
-            if (allowed) {
-#pragma unroll
-              for (int w = 0; w < 4; ++w) {
-                const int lo = max(start - 32 * w, 0), hi = min(end - 32 * w, 32);
-                if (hi > lo) bits[w] |= (hi - lo == 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << lo;
-              }
-            }
-            cur = nx;
+          // 128-bit mask of the key columns this row may read, before causality
+          if (masks != nullptr) {
+            bits[0] = mask_cur.x; bits[1] = mask_cur.y; bits[2] = mask_cur.z; bits[3] = mask_cur.w;
+          } else {
+            const uint4 m4 = row_mask(P, p.mask, b, qb, kb, row);
+            bits[0] = m4.x; bits[1] = m4.y; bits[2] = m4.z; bits[3] = m4.w;
           }
           if (kb == qb) {  // causal inside the diagonal tile: columns 0..row
 #pragma unroll

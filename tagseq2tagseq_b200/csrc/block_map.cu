@@ -14,6 +14,7 @@
 // ragged last tile is never full.  A diagonal pair always holds its own
 // diagonal (allowed) and the upper triangle (not allowed), so it is partial.
 #include "plan.h"
+#include "ptx.cuh"
 
 #include <cuda_runtime.h>
 
@@ -53,7 +54,8 @@ __global__ void __launch_bounds__(128) runs_kernel(PlanView P, MaskArgs M, int t
     if (t == 0) flag = true;
     else flag = d != M.doc[base + pos - 1] || r != M.row[base + pos - 1] || c != M.col[base + pos - 1];
   }
-  __shared__ int warp_cnt[4];
+  __shared__ int warp_cnt[4], s_start[kMaskRuns + 1];
+  if (t <= kMaskRuns) s_start[t] = min(kTile, P.T - tb * kTile);
   const unsigned bal = __ballot_sync(0xffffffffu, flag);
   const int lane = t & 31, w = t >> 5;
   if (lane == 0) warp_cnt[w] = __popc(bal);
@@ -65,49 +67,146 @@ __global__ void __launch_bounds__(128) runs_kernel(PlanView P, MaskArgs M, int t
     const int idx = off + __popc(bal & ((1u << lane) - 1u));
     Run run; run.start = t; run.doc = d; run.row = r; run.col = c;
     P.runs[((size_t)b * P.NB + tb) * kTile + idx] = run;
+    if (idx <= kMaskRuns) s_start[idx] = t;
   }
   if (t == 0) P.run_cnt[(size_t)b * P.NB + tb] = total;
+  __syncthreads();
+  if (t < kMaskRuns) {  // runs past the last one come out empty
+    uint32_t lo[4], hi[4];
+    prefix_mask(s_start[t], lo);
+    prefix_mask(s_start[t + 1], hi);
+    P.run_mask[((size_t)b * P.NB + tb) * kMaskRuns + t] = make_uint4(hi[0] & ~lo[0], hi[1] & ~lo[1], hi[2] & ~lo[2], hi[3] & ~lo[3]);
+  }
 }
 
-// One thread per (kb, qb, b); the runs of the block's q tile sit in shared memory.  A thread stops at the first proof of a
-// partial tile, and looks at four q-runs at a time so that their link words are fetched together: counting every
-// combination one by one took 21 us on a 16k pack of 240 grants, whose tiles have ten runs and more a side.
-__global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint8_t* state_out) {
-  const int kb = blockIdx.x * blockDim.x + threadIdx.x, qb = blockIdx.y, b = blockIdx.z;
-  __shared__ int4 s_runs[kTile];
-  const size_t tq = (size_t)b * P.NB + qb;
-  const int nq = P.run_cnt[tq];
-  if ((int)(blockIdx.x * blockDim.x) <= qb) {
-    if ((int)threadIdx.x < nq) s_runs[threadIdx.x] = reinterpret_cast<const int4*>(P.runs + tq * kTile)[threadIdx.x];
-  }
-  __syncthreads();
-  if (kb >= P.NB) return;
-  uint8_t st = kSkip;
-  const int nvq = min(kTile, P.T - qb * kTile);
-  if (kb == qb) {
-    st = nvq > 0 ? kPartial : kSkip;
-  } else if (kb < qb) {
-    const int64_t* link_b = M.link ? M.link + (size_t)b * M.R * M.W : nullptr;
-    const int4* kr = reinterpret_cast<const int4*>(P.runs + ((size_t)b * P.NB + kb) * kTile);
-    const int nk = P.run_cnt[(size_t)b * P.NB + kb];
-    bool some = false, none = nvq < kTile;  // allowed / denied combinations seen; kv tiles below the diagonal are complete
-    for (int j = 0; j < nk && !(some && none); ++j) {
-      const int4 kj = kr[j];  // start, doc, row, col
-      for (int i = 0; i < nq && !(some && none); i += 4) {
+// State of every tile pair and the masks of the partial ones (see kMaskRuns in plan.h).  A block walks 32 pairs of one q
+// tile; the runs of the q tile, and the documents, column classes and token masks of the first eight runs of each kv tile
+// sit in shared memory.  Eight lanes share a pair: lane i tests q run i against the kv runs one by one and collects its
+// column mask; votes then tell it, as the lane of kv run i, which q runs may read that one.  The kernel is bound by the
+// instructions it issues (18 us at B = 2, T = 32768 with sixteen lanes a pair and the kv runs passed round by shuffles,
+// 20 us with dependent loads instead).  Tiles of more than eight runs take the loop over the run lists.
+constexpr int kStateKb = 32;
+__device__ __forceinline__ void add_run(uint32_t (&bits)[4], int start, int end) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int4 qi = s_runs[min(i + u, nq - 1)];
-          const bool ok = qi.y == kj.y || link_bit(link_b, M.R, M.W, qi.z, kj.w);
+  for (int w = 0; w < 4; ++w) {
+    const int lo = max(start - 32 * w, 0), hi = min(end - 32 * w, 32);
+    if (hi > lo) bits[w] |= (hi - lo == 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << lo;
+  }
+}
+__global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint8_t* state_out) {
+  const int kb0 = blockIdx.x * kStateKb, qb = blockIdx.y, b = blockIdx.z;
+  const size_t tq = (size_t)b * P.NB + qb;
+  if (kb0 > qb) {  // above the diagonal
+    const int kb = kb0 + threadIdx.x;
+    if (threadIdx.x < kStateKb && kb < P.NB) {
+      P.state[tq * P.NB + kb] = kSkip;
+      if (state_out) state_out[tq * P.NB + kb] = kSkip;
+    }
+    return;
+  }
+  __shared__ int4 s_runs[kTile];  // start, doc, row class, column class
+  __shared__ uint4 s_qmask[kMaskRuns], s_kmask[kStateKb][kMaskRuns + 1];  // + 1: the four pairs of a warp fall on different banks
+  __shared__ int2 s_krun[kStateKb][kMaskRuns + 1];                        // doc, column class
+  __shared__ int s_nk[kStateKb];
+  const size_t tk0 = (size_t)b * P.NB + kb0;
+  const int n_kb = min(kStateKb, min(P.NB - kb0, qb + 1 - kb0));
+  const int nq = min(P.run_cnt[tq], kTile);
+  if (threadIdx.x < kMaskRuns) s_qmask[threadIdx.x] = P.run_mask[tq * kMaskRuns + threadIdx.x];
+  if ((int)threadIdx.x < n_kb) s_nk[threadIdx.x] = min(P.run_cnt[tk0 + threadIdx.x], kTile);
+#pragma unroll
+  for (int i = threadIdx.x; i < kStateKb * kMaskRuns; i += 128) {
+    const int k = i / kMaskRuns, r = i % kMaskRuns;
+    if (k < n_kb) {
+      const int4 run = __ldg(reinterpret_cast<const int4*>(P.runs + (tk0 + k) * kTile) + r);
+      s_krun[k][r] = make_int2(run.y, run.w);
+      s_kmask[k][r] = __ldg(P.run_mask + (tk0 + k) * kMaskRuns + r);
+    }
+  }
+  if ((int)threadIdx.x < nq) s_runs[threadIdx.x] = reinterpret_cast<const int4*>(P.runs + tq * kTile)[threadIdx.x];
+  __syncthreads();
+  const int64_t* link_b = M.link ? M.link + (size_t)b * M.R * M.W : nullptr;
+  const int lane = threadIdx.x & 31, mine = lane & 7;
+  const int nvq = min(kTile, P.T - qb * kTile);
+  const size_t pairs = (size_t)b * ((size_t)P.NB * (P.NB + 1) / 2);
+  const int4 q_run = s_runs[min(mine, nq - 1)];
+  unsigned long long lw[4] = {0ull, 0ull, 0ull, 0ull};  // the first four link words of this lane's q run
+  if (link_b != nullptr && q_run.z >= 0 && q_run.z < M.R) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      if (w < M.W) lw[w] = static_cast<unsigned long long>(__ldg(link_b + (size_t)q_run.z * M.W + w));
+  }
+#pragma unroll 1
+  for (int k = threadIdx.x >> 3; k < kStateKb; k += 16) {
+    const int kb = kb0 + k;
+    const bool below = k < n_kb;
+    const int nk = below ? s_nk[k] : 0;
+    bool some = false, none = false;
+    uint32_t qbits[4] = {0u, 0u, 0u, 0u}, kbits[4] = {0u, 0u, 0u, 0u};  // mask of q run `mine` over keys, of kv run `mine` over query rows
+    const int most = __reduce_max_sync(0xffffffffu, nk);
+    if (nq <= kMaskRuns && most <= kMaskRuns) {
+      unsigned readers = 0;  // the q runs that may read kv run `mine`
+      const bool q_live = mine < nq;
+#pragma unroll 1
+      for (int j = 0; j < most; ++j) {
+        const int2 kr = s_krun[k][j];
+        const uint4 km = s_kmask[k][j];
+        const bool valid = q_live && j < nk;
+        bool ok = kr.x == q_run.y;
+        if (!ok && kr.y >= 0) {
+          if (kr.y < 256) {
+            const int wi = kr.y >> 6;
+            ok = ((wi == 0 ? lw[0] : wi == 1 ? lw[1] : wi == 2 ? lw[2] : lw[3]) >> (kr.y & 63)) & 1ull;
+          } else if (valid) {
+            ok = link_bit(link_b, M.R, M.W, q_run.z, kr.y);
+          }
+        }
+        ok = ok && valid;
+        some |= ok;
+        none |= valid && !ok;
+        if (ok) { qbits[0] |= km.x; qbits[1] |= km.y; qbits[2] |= km.z; qbits[3] |= km.w; }
+        const unsigned bal = __ballot_sync(0xffffffffu, ok);
+        if (mine == j) readers = bal >> (lane & 24);
+      }
+      for (int i = 0; i < nq; ++i)
+        if ((readers >> i) & 1u) {
+          const uint4 q = s_qmask[i];
+          kbits[0] |= q.x; kbits[1] |= q.y; kbits[2] |= q.z; kbits[3] |= q.w;
+        }
+    } else {
+      const int4* kr = reinterpret_cast<const int4*>(P.runs + (tk0 + (below ? k : 0)) * kTile);
+      const int nvk = min(kTile, P.T - kb * kTile);
+#pragma unroll 1
+      for (int i = mine; i < (below ? nq : 0); i += 8)
+#pragma unroll 1
+        for (int j = 0; j < nk; ++j) {
+          const int4 me = s_runs[i], other = kr[j];
+          const bool ok = me.y == other.y || link_bit(link_b, M.R, M.W, me.z, other.w);
           some |= ok;
           none |= !ok;
+          if (ok && i < kMaskRuns) add_run(qbits, other.x, j + 1 < nk ? kr[j + 1].x : nvk);
         }
+      if (below && mine < nk) {
+        const int4 me = kr[mine];
+#pragma unroll 1
+        for (int i = 0; i < nq; ++i)
+          if (me.y == s_runs[i].y || link_bit(link_b, M.R, M.W, s_runs[i].z, me.w)) add_run(kbits, s_runs[i].x, i + 1 < nq ? s_runs[i + 1].x : nvq);
       }
     }
-    st = !some ? kSkip : (none ? kPartial : kFull);
+    const unsigned group = 0xffu << (lane & 24);
+    const bool any_some = (__ballot_sync(0xffffffffu, some) & group) != 0u, any_none = (__ballot_sync(0xffffffffu, none) & group) != 0u;
+    // a ragged q tile is never full, a diagonal pair always partial; kv tiles below the diagonal are complete
+    uint8_t st = !below || !any_some ? kSkip : (any_none || nvq < kTile ? kPartial : kFull);
+    if (kb == qb) st = kPartial;
+    if (mine == 0 && kb < P.NB) {
+      P.state[tq * P.NB + kb] = st;
+      if (state_out) state_out[tq * P.NB + kb] = st;
+    }
+    if (st == kPartial && P.q_mask != nullptr) {
+      const size_t at = (pairs + mask_pair(qb, kb)) * kMaskRuns + mine;
+      if (mine < nq) P.q_mask[at] = make_uint4(qbits[0], qbits[1], qbits[2], qbits[3]);
+      if (mine < nk) P.kv_mask[at] = make_uint4(kbits[0], kbits[1], kbits[2], kbits[3]);
+    }
   }
-  const size_t at = tq * P.NB + kb;
-  P.state[at] = st;
-  if (state_out) state_out[at] = st;
 }
 
 // One warp per line.  transposed == 0: line = q tile, scan kv tiles; 1: line = kv tile, scan q tiles.
@@ -223,7 +322,7 @@ cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t
   const bool t = M.link != nullptr && M.R > 0 && M.R <= kLinkTMaxRows && 64 * M.W <= kLinkTMaxCols;
   const int t_words = t ? (M.R + 63) / 64 : 0;
   runs_kernel<<<dim3(P.NB + t_words * ((64 * M.W + 127) / 128), P.B), 128, 0, stream>>>(P, M, t_words);
-  state_kernel<<<dim3((P.NB + 127) / 128, P.NB, P.B), 128, 0, stream>>>(P, M, state_out);
+  state_kernel<<<dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream>>>(P, M, state_out);
   lists_kernel<<<dim3((P.NB + 3) / 4, P.B, 3), 128, 0, stream>>>(P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
                                                                  ListOutputs{q_cnt, q_idx, full_q_cnt, full_q_idx});
   order_kernel<<<dim3((P.NB + 255) / 256, P.B, 3), 256, 0, stream>>>(P, t ? M.R : 0);

@@ -8,6 +8,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector_types.h>
+
 namespace ts2ts {
 
 constexpr int kTile = 128;
@@ -35,6 +37,14 @@ enum : int {
 // backward thread owns one key, i.e. one column class, and tests many row classes against it; with the transposed
 // table its words are loaded once per CTA.  The table exists when R <= kLinkTMaxRows and 64 W <= kLinkTMaxCols.
 constexpr int kLinkTMaxRows = 1024, kLinkTMaxCols = 1024, kLinkTWords = kLinkTMaxRows / 64;
+// Masks of partial tiles, worked out once by the pre-pass for every head and layer: for tile pair (qb, kb) and each of the
+// first kMaskRuns runs of the q tile the 128-bit mask of the key columns its rows may read (q_mask), and for each of the
+// first kMaskRuns runs of the kv tile the mask of the query rows that may read its keys (kv_mask); causality inside the
+// diagonal tile is left to the reader.  16 bytes a mask, 2 x 128 bytes a pair at or below the diagonal, so 8.4 MB a
+// sequence of 32k; the tables exist up to kMaskMaxTiles tiles, and rows of later runs are worked out from the run lists.
+constexpr int kMaskRuns = 8, kMaskMaxTiles = 512;
+inline __host__ __device__ size_t mask_pair(int qb, int kb) { return (size_t)qb * (qb + 1) / 2 + kb; }
+
 constexpr int32_t kPlanMagic = 0x54533254;  // "TS2T"
 
 struct PlanLayout {
@@ -52,6 +62,9 @@ struct PlanLayout {
   size_t pair_cnt;    // int32[B,NP]      NP = ceil(NB/2): kv tiles that q tile 2p or 2p+1 reads (forward work items)
   size_t pair_order;  // int32[B,NP]      pairs of batch b by descending pair_cnt
   size_t link_t;      // uint64[B,kLinkTMaxCols,kLinkTWords]   transposed link bits (see kLinkTRows)
+  size_t run_mask;    // uint32[B,NB,kMaskRuns,4]   the tokens of each of a tile's first runs, one bit a token
+  size_t q_mask;      // uint32[B,NB(NB+1)/2,kMaskRuns,4]   see kMaskRuns; absent above kMaskMaxTiles
+  size_t kv_mask;     // the same shape
   size_t bytes;
 };
 
@@ -78,6 +91,10 @@ inline PlanLayout plan_layout(int B, int T) {
   L.pair_cnt = off;   off = plan_align(off + b * np * sizeof(int32_t));
   L.pair_order = off; off = plan_align(off + b * np * sizeof(int32_t));
   L.link_t = off;     off = plan_align(off + b * kLinkTMaxCols * kLinkTWords * sizeof(uint64_t));
+  L.run_mask = off;   off = plan_align(off + b * nb * kMaskRuns * 16);
+  const size_t masks = nb <= (size_t)kMaskMaxTiles ? b * (nb * (nb + 1) / 2) * kMaskRuns * 16 : 0;
+  L.q_mask = off;     off = plan_align(off + masks);
+  L.kv_mask = off;    off = plan_align(off + masks);
   L.bytes = off;
   return L;
 }
@@ -98,6 +115,9 @@ struct PlanView {
   int32_t* pair_cnt;
   int32_t* pair_order;
   unsigned long long* link_t;
+  uint4* run_mask;
+  uint4* q_mask;   // nullptr when the tables do not exist
+  uint4* kv_mask;
 };
 
 inline PlanView plan_view(void* base, int B, int T) {
@@ -118,6 +138,9 @@ inline PlanView plan_view(void* base, int B, int T) {
   v.pair_cnt = reinterpret_cast<int32_t*>(p + L.pair_cnt);
   v.pair_order = reinterpret_cast<int32_t*>(p + L.pair_order);
   v.link_t = reinterpret_cast<unsigned long long*>(p + L.link_t);
+  v.run_mask = reinterpret_cast<uint4*>(p + L.run_mask);
+  v.q_mask = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint4*>(p + L.q_mask) : nullptr;
+  v.kv_mask = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint4*>(p + L.kv_mask) : nullptr;
   return v;
 }
 

@@ -71,3 +71,39 @@ def test_plan_orders_are_heaviest_first_over_many_tiles(tiles):
     assert torch.equal(order.sort().values, torch.arange(nb, device="cuda", dtype=torch.int32))
     ranked = cnt[order.long()]
     assert bool((ranked[:-1] >= ranked[1:]).all())
+
+
+@pytest.mark.parametrize("t,d,median,lo", [(640, 64, 16, 12), (1300, 128, 9, 1), (65664, 64, 300, 40)])
+def test_attention_where_tiles_leave_the_mask_table(t, d, median, lo):
+    """Tiles of exactly eight, nine and many runs, and a sequence of more tiles than the table covers (513), forward and
+    backward, against fp64 rows computed for a sample of the queries and, through V = dO = one-hot sums, all keys."""
+    from tagseq2tagseq_b200 import build_block_map, read_status, synth
+    from tagseq2tagseq_b200.attention import masked_attn
+    dev = torch.device("cuda")
+    pack = synth.make_pack(t, t, median, lo, max(4 * median, lo), p_link=0.3)
+    doc = torch.from_numpy(pack.doc_ids).to(dev)
+    link = torch.from_numpy(pack.link_bits).to(dev)
+    g = torch.Generator(device=dev).manual_seed(1)
+    q, k, v, do = (torch.randn(1, 1, t, d, device=dev, generator=g).bfloat16() for _ in range(4))
+    rows = torch.randperm(t, device=dev, generator=g)[:200]
+    keep = torch.zeros(t, dtype=torch.bool, device=dev)
+    keep[rows] = True
+    do[:, :, ~keep] = 0                                    # only the sampled rows send a gradient back
+    qd, kd, vd = (x.clone().requires_grad_(True) for x in (q, k, v))
+    bm = build_block_map(doc[None], link[None])
+    out, lse = masked_attn(qd, kd, vd, doc[None], link[None], plan=bm.plan)
+    out.backward(do)
+    assert read_status(bm.plan) == 0
+    words = link[doc[rows].long()]
+    bits = (torch.gather(words, 1, (doc >> 6).long()[None].expand(rows.numel(), -1)) >> (doc & 63).long()[None]) & 1
+    ok = ((doc[rows][:, None] == doc[None]) | bits.bool()) & (torch.arange(t, device=dev)[None] <= rows[:, None])
+    s = ((q[0, 0, rows].double() @ k[0, 0].double().T) * d ** -0.5).masked_fill(~ok, float("-inf"))
+    p = torch.softmax(s, -1)
+    ref = p @ v[0, 0].double()
+    dor = do[0, 0, rows].double()
+    ds = p * (dor @ v[0, 0].double().T - (dor * ref).sum(-1, keepdim=True)) * d ** -0.5
+    # the operator's tolerances: out 2e-2, lse 1e-2, gradients 1e-2 relative
+    assert (out[0, 0, rows].double() - ref).abs().max().item() <= 2e-2
+    assert (lse[0, 0, rows].double() - torch.logsumexp(s, -1)).abs().max().item() <= 1e-2
+    for got, want in ((qd.grad[0, 0, rows], ds @ k[0, 0].double()), (kd.grad[0, 0], ds.T @ q[0, 0, rows].double()), (vd.grad[0, 0], p.T @ dor)):
+        assert ((got.double() - want).norm() / want.norm()).item() <= 1e-2

@@ -1,7 +1,7 @@
 // Masked flash-attention backward for sm_100a.
 //
 // Three kernels:
-//   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, padded to whole tiles)
+//   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, padded to whole tiles); zeroes dQ
 //   attn_bwd     one CTA per 128-key tile of one (batch, head); walks the non-skipped 128-query tiles of the
 //                transposed block list.  Everything is transposed so that a tensor-memory lane is a key row:
 //                  tcgen05  S^T = K Q^T,  dP^T = V dO^T            [128 keys x 128 queries, fp32 in TMEM, N = 128]
@@ -714,37 +714,52 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   if (warp == 13) tmem_dealloc(tmem, 512);
 }
 
-// One warp per (b, h, t): the negated statistics -delta and -lse2.  Rows t >= T of the padded arrays get
-// -lse2 = -inf (P = 0) and delta = 0.
+// The negated statistics -delta and -lse2 per (b, h, t), and zeros for the dQ accumulator.  Rows t >= T of the padded
+// arrays get -lse2 = -inf (P = 0) and delta = 0.  HBM-bound, 8 D bytes a row: D / 8 lanes share a row (16 bytes each of
+// out and dout), every lane has four rows in flight and writes its 32 bytes of each row's zeros.  A warp per row with
+// 4- or 8-byte loads ran at a third of the copy rate, and the memset was a launch of its own (59 + 23 us at 262144 rows of
+// D = 128).
 template <int D>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout, const float* lse,
-                                                       int64_t o_sb, int64_t o_sh, int64_t o_st, int64_t d_sb, int64_t d_sh,
-                                                       int64_t d_st, int B, int H, int T, int Tp, float* lse2, float* delta) {
-  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= (int64_t)B * H * Tp) return;
-  const int t = (int)(row % Tp);
-  const int64_t bh = row / Tp;
-  const int h = (int)(bh % H), b = (int)(bh / H);
-  float acc = 0.f, l2 = CUDART_INF_F;  // stored negated below: -lse2 (so -inf where P must be 0) and -delta
-  if (t < T) {
-    const __nv_bfloat16* o = out + b * o_sb + h * o_sh + (int64_t)t * o_st;
-    const __nv_bfloat16* d = dout + b * d_sb + h * d_sh + (int64_t)t * d_st;
-    constexpr int kPer = D / 32;  // 2 or 4 elements per lane
+__global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
+                                                       const float* __restrict__ lse, int64_t o_sb, int64_t o_sh, int64_t o_st, int64_t d_sb,
+                                                       int64_t d_sh, int64_t d_st, int H, int T, int Tp, float* __restrict__ lse2,
+                                                       float* __restrict__ delta, float* __restrict__ dq_acc) {
+  constexpr int kLanes = D / 8, kRows = 256 / kLanes, kEach = kTile / kRows < 4 ? kTile / kRows : 4;  // a block covers kRows * kEach rows of one (b, h)
+  const int per_bh = Tp / (kRows * kEach);
+  const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * (kRows * kEach);
+  const int b = bh / H, h = bh - b * H;
+  const int r = threadIdx.x / kLanes, c = threadIdx.x % kLanes;
+  uint4 ov[kEach], dv[kEach];
 #pragma unroll
-    for (int i = 0; i < kPer; i += 2) {
-      const __nv_bfloat162 ov = *reinterpret_cast<const __nv_bfloat162*>(o + lane * kPer + i);
-      const __nv_bfloat162 dv = *reinterpret_cast<const __nv_bfloat162*>(d + lane * kPer + i);
-      acc += __bfloat162float(ov.x) * __bfloat162float(dv.x) + __bfloat162float(ov.y) * __bfloat162float(dv.y);
+  for (int i = 0; i < kEach; ++i) {
+    const int t = t0 + i * kRows + r;
+    ov[i] = dv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < T) {
+      ov[i] = __ldg(reinterpret_cast<const uint4*>(out + b * o_sb + h * o_sh + (int64_t)t * o_st) + c);
+      dv[i] = __ldg(reinterpret_cast<const uint4*>(dout + b * d_sb + h * d_sh + (int64_t)t * d_st) + c);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    const int t = t0 + i * kRows + r;
+    const int64_t row = (int64_t)bh * Tp + t;
+    float4* z = reinterpret_cast<float4*>(dq_acc + row * D);
+    z[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    z[c + kLanes] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w}, dw[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      acc = fmaf(__uint_as_float(ow[w] << 16), __uint_as_float(dw[w] << 16), acc);
+      acc = fmaf(__uint_as_float(ow[w] & 0xffff0000u), __uint_as_float(dw[w] & 0xffff0000u), acc);
     }
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    const float l = lse[bh * T + t];
-    l2 = (l == -CUDART_INF_F) ? CUDART_INF_F : l * 1.4426950408889634f;
-  }
-  if (lane == 0) {
-    lse2[row] = -l2;
-    delta[row] = -acc;
+    for (int s = kLanes / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (c == 0) {
+      const float l = t < T ? lse[(int64_t)bh * T + t] : -CUDART_INF_F;
+      lse2[row] = l == -CUDART_INF_F ? -CUDART_INF_F : -l * 1.4426950408889634f;
+      delta[row] = -acc;
+    }
   }
 }
 
@@ -802,10 +817,10 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
       return -120;
     attr_done[dev] = true;
   }
-  cudaMemsetAsync(dq_acc, 0, rows * D * 4, stream);
-  bwd_prep_kernel<D><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
+  constexpr int kPrepRows = 256 / (D / 8) * (kTile / (256 / (D / 8)) < 4 ? kTile / (256 / (D / 8)) : 4);
+  bwd_prep_kernel<D><<<(unsigned)(rows / kPrepRows), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1],
-      sdo[2], B, H, T, Tp, lse2, delta);
+      sdo[2], H, T, Tp, lse2, delta, dq_acc);
   BwdParams p;
   p.plan = P; p.mask = M; p.lse2 = lse2; p.delta = delta; p.dq_acc = dq_acc;
   p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);

@@ -11,6 +11,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/library.h>
 
 #include <algorithm>
@@ -186,6 +188,44 @@ std::tuple<Tensor, Tensor> attn_decode_cuda(const Tensor& q_, const Tensor& k_, 
                           lse.mutable_data_ptr<float>(), nullptr, 0, stream_of(q)),
         "ts2ts_attn_decode");
   return {out, lse};
+}
+
+// The backward and the decoding step have no derivative: differentiating through their results raises, where an operator
+// without an autograd kernel would leave the gradient out.
+template <size_t N>
+void refuse_gradient(const char* name, const std::array<Tensor, N>& inputs, std::initializer_list<Tensor*> results) {
+  if (!at::GradMode::is_enabled() || std::none_of(inputs.begin(), inputs.end(), [](const Tensor& t) { return t.requires_grad(); })) return;
+  std::shared_ptr<torch::autograd::Node> fn(new torch::autograd::NotImplemented(name), torch::autograd::deleteNode);
+  fn->set_next_edges(torch::autograd::collect_next_edges(at::ArrayRef<Tensor>(inputs)));
+  for (Tensor* t : results) torch::autograd::set_history(*t, fn);
+}
+
+std::tuple<Tensor, Tensor, Tensor> attn_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
+                                                     const Tensor& dout, const Tensor& lse, const Tensor& doc_ids,
+                                                     const OptTensor& link_bits, const OptTensor& q_row_ids, const OptTensor& kv_col_ids,
+                                                     const Tensor& plan, double scale) {
+  std::tuple<Tensor, Tensor, Tensor> r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = bwd_op().call(q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale);
+  }
+  refuse_gradient<6>("ts2ts::masked_attn_bwd", {q, k, v, out, dout, lse}, {&std::get<0>(r), &std::get<1>(r), &std::get<2>(r)});
+  return r;
+}
+
+std::tuple<Tensor, Tensor> attn_decode_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& doc_ids,
+                                                const OptTensor& link_bits, const OptTensor& q_row_ids, const OptTensor& kv_col_ids,
+                                                const OptTensor& q_pos, double scale) {
+  using Sig = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const OptTensor&, const OptTensor&,
+                                         const OptTensor&, const OptTensor&, double);
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("ts2ts::masked_attn_decode", "").typed<Sig>();
+  std::tuple<Tensor, Tensor> r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = op.call(q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, q_pos, scale);
+  }
+  refuse_gradient<3>("ts2ts::masked_attn_decode", {q, k, v}, {&std::get<0>(r), &std::get<1>(r)});
+  return r;
 }
 
 // ------------------------------------------------------------------------------------------------ block plan
@@ -733,4 +773,8 @@ TORCH_LIBRARY_IMPL(ts2ts, CUDA, m) {
   m.impl("block_map", block_map_cuda);
   m.impl("link_candidates", link_candidates);
 }
-TORCH_LIBRARY_IMPL(ts2ts, Autograd, m) { m.impl("masked_attn_fwd", attn_fwd_autograd); }
+TORCH_LIBRARY_IMPL(ts2ts, Autograd, m) {
+  m.impl("masked_attn_fwd", attn_fwd_autograd);
+  m.impl("masked_attn_bwd", attn_bwd_autograd);
+  m.impl("masked_attn_decode", attn_decode_autograd);
+}

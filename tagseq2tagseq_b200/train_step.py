@@ -126,7 +126,7 @@ class DecoderLM(nn.Module):
 
 class _StepGraph:
     """Forward and backward of one micro-batch shape as a CUDA graph: its inputs are copied into buffers of the graph's own,
-    the block plan is part of it, the gradients it writes are handed to the parameters.  Link bits are padded with rows and
+    the block plan is part of it, copies of the gradients it writes are handed to the parameters.  Link bits are padded with rows and
     columns that grant nothing, so that packs with different numbers of documents share a graph."""
 
     def __init__(self, owner: "TrainStep", tokens: torch.Tensor, mask: MaskSpec, key):
@@ -137,6 +137,8 @@ class _StepGraph:
             self.mask.link_bits = torch.zeros((mask.link_bits.shape[0],) + key[-2:], dtype=torch.int64, device=tokens.device)
         self._load(tokens, mask)
         self.params = list(owner.model.parameters())
+        # read by the graph, but allocated outside of it: the model keeps only the last sequence length's
+        self.tables = owner.model._rope_tables(tokens.shape[1] - 1, tokens.device)
         self.graph = torch.cuda.CUDAGraph()
         side, here = torch.cuda.Stream(), torch.cuda.current_stream()
         side.wait_stream(here)
@@ -167,7 +169,9 @@ class _StepGraph:
     def run(self, tokens, mask) -> torch.Tensor:
         self._load(tokens, mask)
         self.graph.replay()
-        for p, g in zip(self.params, self.grads):
+        grads = [torch.empty_like(g) for g in self.grads]  # the graph's own buffers are written again by the next step
+        torch._foreach_copy_(grads, self.grads)
+        for p, g in zip(self.params, grads):
             p.grad = g
         return self.loss.clone()
 
@@ -182,8 +186,7 @@ class TrainStep:
     halves the bytes on NVLink; the parameters and the optimizer state stay fp32.
 
     On one GPU, a step whose kernels are shorter than the host work of launching them (see ``_use_graph``) is replayed as
-    a CUDA graph from the second micro-batch of its shape on.  ``p.grad`` is then the graph's own buffer, which the next
-    step overwrites.  ``use_graphs = False`` turns that off."""
+    a CUDA graph from the second micro-batch of its shape on.  ``use_graphs = False`` turns that off."""
 
     MAX_GRAPHS = 2  # micro-batch shapes whose graph, and with it a step's activations, is kept
 

@@ -56,3 +56,25 @@ def test_hooks_and_replaced_parameters_are_not_replayed_over():
     for i in range(3):
         assert abs(float(ts.forward_backward(*_batch(5, 300))) - 6.2383) <= 1e-3
     assert any(g is not None for g in ts._graphs.values())                   # captured again at the new address
+
+
+def test_gradients_of_a_step_outlive_the_next_one():
+    ts = _make()
+    for i in range(2):
+        ts.forward_backward(*_batch(i, 300))
+    held = [p.grad for p in ts.model.parameters()]
+    before = [g.clone() for g in held]
+    ts.forward_backward(*_batch(2, 300))
+    assert all(torch.equal(g, b) for g, b in zip(held, before))
+    assert any(not torch.equal(p.grad, b) for p, b in zip(ts.model.parameters(), before))
+
+
+def test_graph_keeps_the_rotation_tables_it_reads():
+    ts = _make()
+    for i in range(2):
+        ts.forward_backward(*_batch(i, 300))
+    graph, = [g for g in ts._graphs.values() if g is not None]
+    tables = ts.model._rope[1]
+    ts.forward_backward(*_batch(2, 200))                    # the model now holds another length's tables
+    assert ts.model._rope[1] is not tables
+    assert all(a is b for a, b in zip(graph.tables, tables))

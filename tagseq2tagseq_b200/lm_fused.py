@@ -110,7 +110,8 @@ class AdamW(torch.optim.AdamW):
     @torch.no_grad()
     def step(self, closure=None):
         groups = [(g, [p for p in g["params"] if p.grad is not None]) for g in self.param_groups]
-        if not all(self._native(g, ps) for g, ps in groups if ps):
+        # a captured step would repeat the bias corrections of the step that was captured: torch's refuses
+        if torch.cuda.is_current_stream_capturing() or not all(self._native(g, ps) for g, ps in groups if ps):
             return super().step(closure)
         loss = None
         if closure is not None:

@@ -104,3 +104,17 @@ def test_norm_weight_gradient_over_row_and_column_remainders(n, c):
     torch.autograd.backward([xr * 1.0, F.rms_norm(xr, (c,), wr, 1e-6)], [up.double(), g.double()])
     assert _rel(x.grad, xr.grad) <= 2e-6          # fp32 arithmetic, sums of at most 16384 terms
     assert _rel(w.grad, wr.grad) <= 4e-6
+
+
+def test_optimizer_step_is_refused_during_capture():
+    from tagseq2tagseq_b200.lm_fused import AdamW
+    p = torch.nn.Parameter(torch.ones(64, device=DEV))
+    p.grad = torch.ones_like(p)
+    opt = AdamW([p])
+    opt.step()
+    before = p.detach().clone()
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        kept = torch.zeros(1, device=DEV)  # a graph of something
+        with pytest.raises(RuntimeError, match="capturable"):
+            opt.step()
+    assert kept is not None and torch.equal(p, before) and float(opt.state[p]["step"]) == 1.0

@@ -27,10 +27,15 @@ def _need_cuda(*ts):
 
 
 def _call(op, *args):
+    if torch.compiler.is_compiling():  # the operators run their autograd functions at once: a compiled caller breaks its graph here
+        return _uncompiled(op, *args)
     try:
         return op(*args)
     except RuntimeError as e:
         raise _lib.failed_call(e) from None
+
+
+_uncompiled = torch.compiler.disable(_call)
 
 
 def add_rmsnorm(x: torch.Tensor, a: Optional[torch.Tensor], weight: torch.Tensor, eps: float) -> Tuple[torch.Tensor, torch.Tensor]:

@@ -267,6 +267,10 @@ def segment_ids(bounds: np.ndarray, ids: np.ndarray, seq_len: int, device: torch
     return out
 
 
+def _pack_mask(*args):
+    return _lib.ops().pack_mask.default(*args)
+
+
 def from_reference(doc_spans: Sequence[Any], link_to_target: Optional[Dict[int, List[int]]], seq_len: int,
                    max_grants_cap: int = 64, device: Optional[torch.device] = None) -> MaskSpec:
     """MaskSpec equal to the reference's mask for these spans and matched links
@@ -276,8 +280,9 @@ def from_reference(doc_spans: Sequence[Any], link_to_target: Optional[Dict[int, 
         # grants, classes on segment boundaries and link bits in native code (what ordered_grants and grant_segments
         # do); per-token ids are filled on the device, nothing of length T crosses PCIe
         pairs = [(int(pos), int(tgt)) for pos in sorted(link_to_target) for tgt in link_to_target[pos]] if link_to_target else []
-        return MaskSpec(*_lib.ops().pack_mask.default(*[[int(getattr(s, n)) for s in doc_spans] for n in ("start", "end", "doc_id")],
-                                                      [p for p, _ in pairs], [t for _, t in pairs], seq_len, max_grants_cap, device))
+        pack_mask = _pack_mask if not torch.compiler.is_compiling() else torch.compiler.disable(_pack_mask)
+        return MaskSpec(*pack_mask(*[[int(getattr(s, n)) for s in doc_spans] for n in ("start", "end", "doc_id")],
+                                   [p for p, _ in pairs], [t for _, t in pairs], seq_len, max_grants_cap, device))
     ids = torch.from_numpy(build_document_ids(seq_len, doc_spans))[None].to(device)
     grants = ordered_grants(seq_len, doc_spans, link_to_target, max_grants_cap) if link_to_target else []
     if not grants:

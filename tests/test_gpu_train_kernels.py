@@ -118,3 +118,19 @@ def test_optimizer_step_is_refused_during_capture():
         with pytest.raises(RuntimeError, match="capturable"):
             opt.step()
     assert kept is not None and torch.equal(p, before) and float(opt.state[p]["step"]) == 1.0
+
+
+def test_layer_operators_break_a_compiled_graph_and_run():
+    from tagseq2tagseq_b200.lm_fused import add_rmsnorm, swiglu
+
+    def fn(x, w, p):
+        _, h = add_rmsnorm(x * 1.5, None, w, 1e-6)
+        return (swiglu(h @ p).float() * 2).sum()
+
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    leaves = [torch.randn(s, device=DEV, generator=gen).requires_grad_() for s in ((1, 40, 64), (64,))]
+    p = torch.randn(64, 128, device=DEV, generator=gen).bfloat16()
+    want = torch.autograd.grad(fn(*leaves, p), leaves)
+    got = torch.autograd.grad(torch.compile(fn, backend="aot_eager")(*leaves, p), leaves)
+    for a, b in zip(got, want):
+        assert _rel(a, b) <= 1e-5

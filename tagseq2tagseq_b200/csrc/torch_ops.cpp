@@ -668,6 +668,7 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
     const CUDAGuard guard(h.device());
     const Tensor h2 = h.reshape({-1, h.size(-1)}), wb = w.to(at::kBFloat16), target = target_in.reshape({-1}).to(at::kLong).contiguous();
     const int64_t N = h2.size(0), V = w.size(0);
+    TORCH_CHECK_VALUE(target.numel() == N, "head_loss: one target per row of h");
     Tensor logits = at::mm(h2, wb.t()), loss = at::empty({N}, h.options().dtype(at::kFloat));
     check(ts2ts_ce_fwd_grad(logits.mutable_data_ptr(), target.const_data_ptr<int64_t>(), mfptr(loss), static_cast<float>(1.0 / static_cast<double>(N)), N,
                             static_cast<int>(V), stream_of(h)),

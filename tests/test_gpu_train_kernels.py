@@ -134,3 +134,11 @@ def test_layer_operators_break_a_compiled_graph_and_run():
     got = torch.autograd.grad(torch.compile(fn, backend="aot_eager")(*leaves, p), leaves)
     for a, b in zip(got, want):
         assert _rel(a, b) <= 1e-5
+
+
+def test_head_loss_refuses_a_target_of_another_length():
+    from tagseq2tagseq_b200.lm_fused import head_loss
+    h = torch.zeros(1, 5, 64, device=DEV, dtype=torch.bfloat16)
+    w = torch.zeros(16, 64, device=DEV, requires_grad=True)
+    with pytest.raises(ValueError):
+        head_loss(h, w, torch.zeros(1, 4, device=DEV, dtype=torch.int64))

@@ -363,6 +363,9 @@ std::vector<Tensor> pack_mask(at::IntArrayRef starts, at::IntArrayRef ends, at::
                               at::IntArrayRef link_target, int64_t T, int64_t cap, c10::Device device) {
   const size_t n_spans = starts.size();
   TORCH_CHECK_VALUE(ends.size() == n_spans && ids.size() == n_spans && link_pos.size() == link_target.size(), "pack_mask: lists of equal length");
+  for (size_t i = 0; i < n_spans; ++i)  // ids of spans that cover a token are stored in 32 bits
+    TORCH_CHECK_VALUE(std::max<int64_t>(0, starts[i]) >= std::min(T, ends[i]) || ids[i] == static_cast<int32_t>(ids[i]),
+                      "pack_mask: document id ", ids[i], " does not fit 32 bits");
   if (!device.has_index()) device = c10::Device(c10::kCUDA, c10::cuda::current_device());
   const c10::cuda::CUDAGuard guard(device);
   std::unordered_map<int64_t, size_t> by_id;

@@ -281,8 +281,10 @@ def from_reference(doc_spans: Sequence[Any], link_to_target: Optional[Dict[int, 
         # do); per-token ids are filled on the device, nothing of length T crosses PCIe
         pairs = [(int(pos), int(tgt)) for pos in sorted(link_to_target) for tgt in link_to_target[pos]] if link_to_target else []
         pack_mask = _pack_mask if not torch.compiler.is_compiling() else torch.compiler.disable(_pack_mask)
-        return MaskSpec(*pack_mask(*[[int(getattr(s, n)) for s in doc_spans] for n in ("start", "end", "doc_id")],
-                                   [p for p, _ in pairs], [t for _, t in pairs], seq_len, max_grants_cap, device))
+        starts, ends, ids = ([int(getattr(s, n)) for s in doc_spans] for n in ("start", "end", "doc_id"))
+        if ids and not -2**31 <= min(ids) <= max(ids) < 2**31:
+            build_document_ids(seq_len, doc_spans)  # OverflowError for an id of more than 32 bits on a span that covers a token
+        return MaskSpec(*pack_mask(starts, ends, ids, [p for p, _ in pairs], [t for _, t in pairs], seq_len, max_grants_cap, device))
     ids = torch.from_numpy(build_document_ids(seq_len, doc_spans))[None].to(device)
     grants = ordered_grants(seq_len, doc_spans, link_to_target, max_grants_cap) if link_to_target else []
     if not grants:

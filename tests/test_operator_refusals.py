@@ -1,0 +1,17 @@
+"""What the native operators refuse before anything reaches a device: inputs that a kernel would read past, or that would be
+cut without a word.  CPU tensors stand in for CUDA ones: the checks come first."""
+import pytest
+import torch
+
+from tagseq2tagseq_b200 import DocSpan, _lib, from_reference
+
+OPS = _lib.ops()
+
+
+@pytest.mark.parametrize("doc_id", [2**32 + 1, 2**31, -2**31 - 1])
+def test_document_ids_beyond_32_bits_are_refused(doc_id):
+    spans = [DocSpan(1, "", 0, 40), DocSpan(doc_id, "", 40, 90)]
+    with pytest.raises(OverflowError):
+        from_reference(spans, None, 100, device=torch.device("cuda"))
+    with pytest.raises(ValueError, match="32 bits"):
+        OPS.pack_mask([0, 40], [40, 90], [1, doc_id], [], [], 100, 64, torch.device("cuda", 0))

@@ -61,10 +61,9 @@ class Ts2tsError(RuntimeError):
 def lib() -> ctypes.CDLL:
     global _LIB
     if _LIB is None:
-        path = _build.LIB
-        if not os.path.exists(path):
-            path = _build.build_library()  # raises when nvcc is absent: no CPU path exists
-        handle = ctypes.CDLL(path)
+        if _build.unusable():  # both libraries are brought up to date before either is loaded
+            _build.build_library()  # raises when nvcc is absent: no CPU path exists
+        handle = ctypes.CDLL(_build.LIB)
         for name, (res, args) in SYMBOLS.items():
             fn = getattr(handle, name)
             fn.restype = res
@@ -79,11 +78,16 @@ def ops():
     if _OPS is None:
         import torch
         lib()
-        if not os.path.exists(_build.TORCH_LIB):
-            _build.build_library(force=True)
         torch.ops.load_library(_build.TORCH_LIB)
+        from . import _fake  # noqa: F401  shapes of the results, for compiled callers
         _OPS = torch.ops.ts2ts
     return _OPS
+
+
+def load_if_built() -> None:
+    """Load the operators when that takes no compiler; otherwise the first call does."""
+    if _OPS is None and not _build.unusable():
+        ops()
 
 
 def failed_call(e: RuntimeError) -> RuntimeError:

@@ -29,7 +29,7 @@ def _check_qkv(q, k, v):
         raise ValueError("head dimension must be 64 or 128")
 
 
-_OPS = _lib.ops()
+_lib.load_if_built()  # not inside the first call, which may be a compiled caller's
 
 
 def _call(op, *args):
@@ -43,28 +43,11 @@ def _call(op, *args):
 
 
 def _attn_fwd(q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale: float) -> Tuple[torch.Tensor, torch.Tensor]:
-    return _call(_OPS.masked_attn_fwd.default, q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale)
+    return _call(_lib.ops().masked_attn_fwd.default, q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale)
 
 
 def _attn_bwd(q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    return _call(_OPS.masked_attn_bwd.default, q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale)
-
-
-@torch.library.register_fake("ts2ts::masked_attn_fwd")
-def _(q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale):
-    B, H, T, D = q.shape
-    return q.new_empty((B, H, T, D)), q.new_empty((B, H, T), dtype=torch.float32)
-
-
-@torch.library.register_fake("ts2ts::masked_attn_bwd")
-def _(q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale):
-    return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-
-
-@torch.library.register_fake("ts2ts::masked_attn_decode")
-def _(q, k_cache, v_cache, doc_ids, link_bits, q_row_ids, kv_col_ids, q_pos, scale):
-    B, H, Tk, D = k_cache.shape
-    return q.new_empty((B, H, 1, D)), q.new_empty((B, H), dtype=torch.float32)
+    return _call(_lib.ops().masked_attn_bwd.default, q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale)
 
 
 def masked_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, doc_ids: torch.Tensor,
@@ -122,7 +105,7 @@ def masked_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
         raise ValueError("scale must be positive")
     if q_pos is not None and (q_pos.dtype != torch.int32 or q_pos.shape != (k_cache.shape[0],)):
         raise ValueError("q_pos must be int32 [B]")
-    return _call(_OPS.masked_attn_decode.default, q, k_cache, v_cache, doc_ids, link_bits, q_row_ids, kv_col_ids, q_pos, scale)
+    return _call(_lib.ops().masked_attn_decode.default, q, k_cache, v_cache, doc_ids, link_bits, q_row_ids, kv_col_ids, q_pos, scale)
 
 
 def flex_attention(query, key, value, score_mod=None, block_mask=None, scale=None, enable_gqa=False, return_lse=False,

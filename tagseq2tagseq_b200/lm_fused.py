@@ -16,7 +16,7 @@ from .mask_spec import MaskSpec
 
 __all__ = ["add_rmsnorm", "qkv_attention", "swiglu", "cross_entropy", "head_loss", "embedding", "rope_half_tables", "Linear", "AdamW"]
 
-_OPS = _lib.ops()
+_lib.load_if_built()
 _MAX_HEAD_COLUMNS = 110592  # a row of logits that ts2ts_ce_fwd_grad keeps in shared memory
 
 
@@ -41,7 +41,7 @@ _uncompiled = torch.compiler.disable(_call)
 def add_rmsnorm(x: torch.Tensor, a: Optional[torch.Tensor], weight: torch.Tensor, eps: float) -> Tuple[torch.Tensor, torch.Tensor]:
     """(x + a, rmsnorm(x + a) * weight): the fp32 residual stream and the bf16 input of the next linear layer."""
     _need_cuda(x, a, weight)
-    return _call(_OPS.add_rmsnorm.default, x, a, weight, eps)
+    return _call(_lib.ops().add_rmsnorm.default, x, a, weight, eps)
 
 
 def rope_half_tables(T: int, head_dim: int, base: float, device) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -55,21 +55,21 @@ def qkv_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, mask:
     """Rotary embedding + masked attention on the packed projection qkv [B,T,3*H*D] (bf16, overwritten: q and k are
     rotated in place).  cos / sin: fp32 [T, head_dim/2] from ``rope_half_tables``.  Returns [B,T,H*D]."""
     _need_cuda(qkv, cos, sin)
-    return _call(_OPS.qkv_attention.default, qkv, cos, sin, mask.doc_ids, mask.link_bits, mask.q_row_ids, mask.kv_col_ids, mask.plan,
+    return _call(_lib.ops().qkv_attention.default, qkv, cos, sin, mask.doc_ids, mask.link_bits, mask.q_row_ids, mask.kv_col_ids, mask.plan,
                  n_heads, head_dim)
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up with gate, up = gate_up.chunk(2, dim=-1)."""
     _need_cuda(gate_up)
-    return _call(_OPS.swiglu.default, gate_up)
+    return _call(_lib.ops().swiglu.default, gate_up)
 
 
 def cross_entropy(logits: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of bf16 logits [N,V] against int64 targets [N]; the backward overwrites ``logits`` with
     their gradient, so the caller must not use them afterwards."""
     _need_cuda(logits, target)
-    return _call(_OPS.cross_entropy.default, logits, target)
+    return _call(_lib.ops().cross_entropy.default, logits, target)
 
 
 def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
@@ -78,7 +78,7 @@ def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> to
     V = weight.shape[0]
     if (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad) and h.dtype == torch.bfloat16 and weight.dtype == torch.float32
             and V % 8 == 0 and V <= _MAX_HEAD_COLUMNS and h.shape[-1] % 8 == 0):
-        return _call(_OPS.head_loss.default, h, weight, target)
+        return _call(_lib.ops().head_loss.default, h, weight, target)
     logits = F.linear(h, weight.to(h.dtype))
     return cross_entropy(logits.to(torch.bfloat16).view(-1, V), target.reshape(-1))
 
@@ -86,7 +86,7 @@ def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> to
 def embedding(weight: torch.Tensor, tokens: torch.Tensor) -> torch.Tensor:
     """Rows of an fp32 embedding table."""
     if weight.is_cuda and weight.dtype == torch.float32 and weight.shape[1] % 4 == 0 and tokens.dtype == torch.int64:
-        return _call(_OPS.embedding.default, weight, tokens)
+        return _call(_lib.ops().embedding.default, weight, tokens)
     return F.embedding(tokens, weight)
 
 
@@ -99,7 +99,7 @@ class Linear(nn.Linear):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32:
-            return _call(_OPS.linear.default, x, self.weight)
+            return _call(_lib.ops().linear.default, x, self.weight)
         return super().forward(x)
 
 
@@ -135,6 +135,6 @@ class AdamW(torch.optim.AdamW):
                 elif st["step"].is_cuda:  # a state saved by an optimizer that counts on the device
                     st["step"] = st["step"].float().cpu()
             states = [self.state[p] for p in params]
-            _call(_OPS.adamw.default, params, [p.grad.contiguous() for p in params], [s["exp_avg"] for s in states],
+            _call(_lib.ops().adamw.default, params, [p.grad.contiguous() for p in params], [s["exp_avg"] for s in states],
                   [s["exp_avg_sq"] for s in states], [s["step"] for s in states], g["lr"], *g["betas"], g["eps"], g["weight_decay"])
         return loss

@@ -609,6 +609,7 @@ Tensor swiglu(const Tensor& gate_up) { return SwiGLU::apply(gate_up); }
 
 struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& target_in) {
+    TORCH_CHECK_VALUE(logits.dim() != 2 || target_in.numel() >= logits.size(0), "cross_entropy: one target per row of logits");
     need_cuda(logits);
     TORCH_CHECK_TYPE(logits.scalar_type() == at::kBFloat16 && logits.dim() == 2 && logits.is_contiguous(),
                      "cross_entropy: logits must be a contiguous bf16 [N,V] tensor");

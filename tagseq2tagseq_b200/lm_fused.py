@@ -74,6 +74,8 @@ def cross_entropy(logits: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
 
 def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call."""
+    if target.numel() != h.shape[:-1].numel():
+        raise ValueError("head_loss: one target per row of h")
     _need_cuda(h, weight, target)
     V = weight.shape[0]
     if (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad) and h.dtype == torch.bfloat16 and weight.dtype == torch.float32

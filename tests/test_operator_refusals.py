@@ -15,3 +15,15 @@ def test_document_ids_beyond_32_bits_are_refused(doc_id):
         from_reference(spans, None, 100, device=torch.device("cuda"))
     with pytest.raises(ValueError, match="32 bits"):
         OPS.pack_mask([0, 40], [40, 90], [1, doc_id], [], [], 100, 64, torch.device("cuda", 0))
+
+
+def test_a_target_shorter_than_the_rows_is_refused():
+    """The loss kernel reads one target per row, whichever way a head's loss takes."""
+    from tagseq2tagseq_b200.lm_fused import head_loss
+    with pytest.raises(ValueError, match="target"):
+        OPS.cross_entropy(torch.zeros(4, 16, dtype=torch.bfloat16), torch.zeros(3, dtype=torch.int64))
+    h, w = torch.zeros(2, 4, 64, dtype=torch.bfloat16), torch.zeros(16, 64)
+    for grad in (False, True):
+        for n in (7, 9):
+            with pytest.raises(ValueError, match="target"):
+                head_loss(h, w.requires_grad_(grad), torch.zeros(n, dtype=torch.int64))

@@ -473,6 +473,7 @@ float* mfptr(const Tensor& t) { return t.mutable_data_ptr<float>(); }
 
 struct AddRMSNorm : torch::autograd::Function<AddRMSNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const OptTensor& a_in, const Tensor& w, double eps) {
+    TORCH_CHECK_VALUE(x_in.size(-1) > 0, "add_rmsnorm: x has no columns");
     need_cuda(x_in);
     TORCH_CHECK_TYPE(x_in.scalar_type() == at::kFloat && w.scalar_type() == at::kFloat && (!a_in.has_value() || a_in->scalar_type() == at::kBFloat16),
                      "add_rmsnorm: x and w are fp32, a is bf16");
@@ -583,6 +584,8 @@ Tensor qkv_attention(Tensor qkv, const Tensor& cos, const Tensor& sin, const Ten
 
 struct SwiGLU : torch::autograd::Function<SwiGLU> {
   static Tensor forward(AutogradContext* ctx, const Tensor& gate_up) {
+    // an odd row has no halves: its rows would be taken to begin earlier and earlier, and to be more than there are
+    TORCH_CHECK_VALUE(gate_up.size(-1) > 0 && gate_up.size(-1) % 2 == 0, "swiglu: the last dimension must be even and not empty");
     need_cuda(gate_up);
     TORCH_CHECK_TYPE(gate_up.scalar_type() == at::kBFloat16, "swiglu: bf16 input");
     at::AutoDispatchBelowADInplaceOrView below;

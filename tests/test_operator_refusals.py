@@ -27,3 +27,13 @@ def test_a_target_shorter_than_the_rows_is_refused():
         for n in (7, 9):
             with pytest.raises(ValueError, match="target"):
                 head_loss(h, w.requires_grad_(grad), torch.zeros(n, dtype=torch.int64))
+
+
+def test_rows_that_cannot_be_counted_are_refused():
+    """A division by zero columns would end the process; an odd gate and up row would make the kernel count more rows than
+    there are."""
+    with pytest.raises(ValueError, match="columns"):
+        OPS.add_rmsnorm(torch.zeros(4, 0), None, torch.zeros(0), 1e-6)
+    for f in (0, 17):
+        with pytest.raises(ValueError, match="even"):
+            OPS.swiglu(torch.zeros(16, f, dtype=torch.bfloat16))

@@ -472,14 +472,16 @@ const float* fptr(const Tensor& t) { return t.const_data_ptr<float>(); }
 float* mfptr(const Tensor& t) { return t.mutable_data_ptr<float>(); }
 
 struct AddRMSNorm : torch::autograd::Function<AddRMSNorm> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const OptTensor& a_in, const Tensor& w, double eps) {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const OptTensor& a_in, const Tensor& w_in, double eps) {
     TORCH_CHECK_VALUE(x_in.size(-1) > 0, "add_rmsnorm: x has no columns");
+    TORCH_CHECK_VALUE(w_in.numel() >= x_in.size(-1) && (!a_in.has_value() || a_in->numel() >= x_in.numel()),
+                      "add_rmsnorm: a has the size of x, w one element per column");
     need_cuda(x_in);
-    TORCH_CHECK_TYPE(x_in.scalar_type() == at::kFloat && w.scalar_type() == at::kFloat && (!a_in.has_value() || a_in->scalar_type() == at::kBFloat16),
+    TORCH_CHECK_TYPE(x_in.scalar_type() == at::kFloat && w_in.scalar_type() == at::kFloat && (!a_in.has_value() || a_in->scalar_type() == at::kBFloat16),
                      "add_rmsnorm: x and w are fp32, a is bf16");
     at::AutoDispatchBelowADInplaceOrView below;
     const CUDAGuard guard(x_in.device());
-    const Tensor x = x_in.contiguous(), a = a_in.has_value() ? a_in->contiguous() : Tensor();
+    const Tensor x = x_in.contiguous(), a = a_in.has_value() ? a_in->contiguous() : Tensor(), w = w_in.contiguous();
     const int64_t C = x.size(-1), N = x.numel() / C;
     Tensor x_out = at::empty_like(x), h = at::empty(x.sizes(), x.options().dtype(at::kBFloat16)), rstd = at::empty({N}, x.options());
     check(ts2ts_add_rmsnorm_fwd(fptr(x), a.defined() ? a.const_data_ptr() : nullptr, fptr(w), mfptr(x_out), h.mutable_data_ptr(), mfptr(rstd),
@@ -526,6 +528,11 @@ struct QKVAttention : torch::autograd::Function<QKVAttention> {
   static variable_list forward(AutogradContext* ctx, Tensor qkv, const Tensor& cos, const Tensor& sin, const Tensor& doc_ids,
                                const OptTensor& link_bits, const OptTensor& q_row_ids, const OptTensor& kv_col_ids, const Tensor& plan,
                                int64_t n_heads, int64_t head_dim) {
+    const int64_t angles = qkv.dim() == 3 ? qkv.size(1) * (head_dim / 2) : 0;
+    for (const Tensor* t : {&cos, &sin})
+      TORCH_CHECK_VALUE(t->numel() >= angles && t->is_contiguous(), "qkv_attention: cos and sin must be contiguous [T, head_dim / 2]");
+    for (const Tensor& t : {doc_ids, q_row_ids.value_or(doc_ids), kv_col_ids.value_or(doc_ids)})
+      TORCH_CHECK_VALUE(qkv.dim() != 3 || t.numel() >= qkv.size(0) * qkv.size(1), "qkv_attention: the mask must have an id per token of qkv");
     need_cuda(qkv);
     TORCH_CHECK_TYPE(qkv.scalar_type() == at::kBFloat16 && qkv.is_contiguous(), "qkv_attention: qkv must be a contiguous bf16 tensor");
     TORCH_CHECK_VALUE(qkv.dim() == 3 && qkv.size(2) == 3 * n_heads * head_dim, "qkv_attention: last dimension must be 3 * n_heads * head_dim");

@@ -37,3 +37,16 @@ def test_rows_that_cannot_be_counted_are_refused():
     for f in (0, 17):
         with pytest.raises(ValueError, match="even"):
             OPS.swiglu(torch.zeros(16, f, dtype=torch.bfloat16))
+
+
+def test_norm_and_attention_refuse_operands_they_would_read_past():
+    x = torch.zeros(4, 64)
+    for a, w in ((torch.zeros(3, 64, dtype=torch.bfloat16), torch.zeros(64)), (None, torch.zeros(63))):
+        with pytest.raises(ValueError, match="add_rmsnorm"):
+            OPS.add_rmsnorm(x, a, w, 1e-6)
+    plan, ids = torch.zeros(4, dtype=torch.uint8), torch.zeros(2, 5, dtype=torch.int32)
+    good = torch.zeros(5, 32)
+    for cos, sin, doc, row in ((good[:4], good, ids, None), (good, good[:, :31], ids, None), (good, torch.zeros(5, 64)[:, ::2], ids, None),
+                               (good, good, ids[:1], None), (good, good, ids, ids[:, 1:])):
+        with pytest.raises(ValueError, match="qkv_attention"):
+            OPS.qkv_attention(torch.zeros(2, 5, 3 * 2 * 64, dtype=torch.bfloat16), cos, sin, doc, None, row, None, plan, 2, 64)

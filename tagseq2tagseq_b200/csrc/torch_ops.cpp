@@ -649,25 +649,25 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
 Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); }
 
 // y = x w^T with bf16 activations and an fp32 weight.  The weight gradient leaves its GEMM in fp32: no bf16 rounding and no
-// conversion pass (6 bytes per weight) on the way to the parameter.
+// conversion pass (6 bytes per weight) on the way to the parameter.  x is saved as it was passed, so that writing to it
+// before the backward is noticed; of w only the bf16 copy is needed, and a changed w does not matter.
 struct Linear : torch::autograd::Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
     need_cuda(x);
     at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor x2 = x.reshape({-1, x.size(-1)}), wb = w.to(at::kBFloat16);
-    ctx->save_for_backward({x2, wb});
+    const Tensor wb = w.to(at::kBFloat16);
+    ctx->save_for_backward({x, wb});
     auto shape = x.sizes().vec();
     shape.back() = w.size(0);
-    ctx->saved_data["shape"] = x.sizes().vec();
-    return at::mm(x2, wb.t()).view(shape);
+    return at::mm(x.reshape({-1, x.size(-1)}), wb.t()).view(shape);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     bind_context(s[0]);
     const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)});
     Tensor dx, dw;
-    if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(ctx->saved_data["shape"].toIntVector());
-    if (ctx->needs_input_grad(1)) dw = at::mm(dy.t(), s[0], at::kFloat);
+    if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(s[0].sizes());
+    if (ctx->needs_input_grad(1)) dw = at::mm(dy.t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
     return {dx, dw};
   }
 };
@@ -687,8 +687,7 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
     check(ts2ts_ce_fwd_grad(logits.mutable_data_ptr(), target.const_data_ptr<int64_t>(), mfptr(loss), static_cast<float>(1.0 / static_cast<double>(N)), N,
                             static_cast<int>(V), stream_of(h)),
           "ts2ts_ce_fwd_grad");
-    ctx->save_for_backward({h2, wb, logits});
-    ctx->saved_data["shape"] = h.sizes().vec();
+    ctx->save_for_backward({h, wb, logits});
     return loss.mean();
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -700,11 +699,11 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
     Tensor dh, dw;
     if (ctx->needs_input_grad(0)) {
       Tensor dh32 = at::mm(s[2], s[1], at::kFloat);
-      dh = at::empty(ctx->saved_data["shape"].toIntVector(), s[0].options());
+      dh = at::empty(s[0].sizes(), s[0].options());
       check(ts2ts_scale(mfptr(dh32), dh.mutable_data_ptr(), fptr(g), dh.numel(), stream), "ts2ts_scale");
     }
     if (ctx->needs_input_grad(1)) {
-      dw = at::mm(s[2].t(), s[0], at::kFloat);
+      dw = at::mm(s[2].t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
       check(ts2ts_scale(mfptr(dw), nullptr, fptr(g), dw.numel(), stream), "ts2ts_scale");
     }
     return {dh, dw, Tensor()};

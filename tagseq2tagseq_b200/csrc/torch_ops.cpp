@@ -650,13 +650,18 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossE
 
 // y = x w^T with bf16 activations and an fp32 weight.  The weight gradient leaves its GEMM in fp32: no bf16 rounding and no
 // conversion pass (6 bytes per weight) on the way to the parameter.  x is saved as it was passed, so that writing to it
-// before the backward is noticed; of w only the bf16 copy is needed, and a changed w does not matter.
+// before the backward is noticed; of w only the bf16 copy is needed, and a changed w does not matter.  A gradient that may be
+// differentiated again (create_graph) is made of ordinary operators on x and w themselves.
 struct Linear : torch::autograd::Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
     need_cuda(x);
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor wb = w.to(at::kBFloat16);
     ctx->save_for_backward({x, wb});
+    if (w.requires_grad() && !w.is_inference()) {
+      ctx->saved_data["w"] = w;
+      ctx->saved_data["version"] = static_cast<int64_t>(w._version());
+    }
     auto shape = x.sizes().vec();
     shape.back() = w.size(0);
     return at::mm(x.reshape({-1, x.size(-1)}), wb.t()).view(shape);
@@ -666,6 +671,20 @@ struct Linear : torch::autograd::Function<Linear> {
     bind_context(s[0]);
     const Tensor dy = grads[0].reshape({-1, grads[0].size(-1)});
     Tensor dx, dw;
+    if (at::GradMode::is_enabled()) {
+      const c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+      Tensor wb = s[1];
+      if (ctx->saved_data.count("w")) {
+        const Tensor w = ctx->saved_data["w"].toTensor();
+        TORCH_CHECK(static_cast<int64_t>(w._version()) == ctx->saved_data["version"].toInt(),
+                    "one of the variables needed for gradient computation has been modified by an inplace operation: the weight of a "
+                    "linear layer whose gradient is to be differentiated again");
+        wb = w.to(at::kBFloat16);
+      }
+      if (ctx->needs_input_grad(0)) dx = at::mm(dy, wb).view(s[0].sizes());
+      if (ctx->needs_input_grad(1)) dw = at::mm(dy.t().to(at::kFloat), s[0].reshape({-1, s[0].size(-1)}).to(at::kFloat));
+      return {dx, dw};
+    }
     if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(s[0].sizes());
     if (ctx->needs_input_grad(1)) dw = at::mm(dy.t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
     return {dx, dw};

@@ -39,3 +39,26 @@ def test_a_weight_changed_before_the_backward_does_not_matter():
         lin.weight.zero_()
     y.sum().backward()
     assert (x.grad.float() - want).abs().max() <= 2 ** -8 * want.abs().max()
+
+
+def test_second_derivative_of_a_linear_layer_matches_torch():
+    """A gradient penalty reaches the weight through x, dy and the weight itself."""
+    lin = _linear(64, 32)
+    grads = []
+    for layer in (lambda x: lin(x), lambda x: F.linear(x, lin.weight)):
+        torch.manual_seed(5)
+        x = torch.randn(3, 9, 64, device=DEV).bfloat16().requires_grad_(True)
+        lin.weight.grad = None
+        with torch.autocast("cuda", torch.bfloat16):
+            y = layer(x)
+        gx, gw = torch.autograd.grad((y.float() ** 3).sum(), (x, lin.weight), create_graph=True)
+        (gx.float().pow(2).sum() + gw.float().pow(2).sum()).backward()
+        grads.append((x.grad.double(), lin.weight.grad.double()))
+    for a, b in zip(*grads):
+        assert (a - b).norm() <= 4 * 2 ** -8 * b.norm()     # bf16 products and results on either side, rounded a few times each
+    with torch.autocast("cuda", torch.bfloat16):
+        y = lin(x)
+    with torch.no_grad():
+        lin.weight.add_(1)
+    with pytest.raises(RuntimeError, match="inplace"):
+        torch.autograd.grad(y.sum(), x, create_graph=True)

@@ -192,12 +192,12 @@ std::tuple<Tensor, Tensor> attn_decode_cuda(const Tensor& q_, const Tensor& k_, 
 
 // The backward and the decoding step have no derivative: differentiating through their results raises, where an operator
 // without an autograd kernel would leave the gradient out.
-template <size_t N>
-void refuse_gradient(const char* name, const std::array<Tensor, N>& inputs, std::initializer_list<Tensor*> results) {
-  if (!at::GradMode::is_enabled() || std::none_of(inputs.begin(), inputs.end(), [](const Tensor& t) { return t.requires_grad(); })) return;
+void refuse_gradient(const char* name, at::ArrayRef<Tensor> inputs, std::initializer_list<Tensor*> results) {
+  if (!at::GradMode::is_enabled() || std::none_of(inputs.begin(), inputs.end(), [](const Tensor& t) { return t.defined() && t.requires_grad(); })) return;
   std::shared_ptr<torch::autograd::Node> fn(new torch::autograd::NotImplemented(name), torch::autograd::deleteNode);
-  fn->set_next_edges(torch::autograd::collect_next_edges(at::ArrayRef<Tensor>(inputs)));
-  for (Tensor* t : results) torch::autograd::set_history(*t, fn);
+  fn->set_next_edges(torch::autograd::collect_next_edges(inputs));
+  for (Tensor* t : results)
+    if (t->defined()) torch::autograd::set_history(*t, fn);
 }
 
 std::tuple<Tensor, Tensor, Tensor> attn_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
@@ -209,7 +209,7 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd_autograd(const Tensor& q, const Tens
     at::AutoDispatchBelowADInplaceOrView below;
     r = bwd_op().call(q, k, v, out, dout, lse, doc_ids, link_bits, q_row_ids, kv_col_ids, plan, scale);
   }
-  refuse_gradient<6>("ts2ts::masked_attn_bwd", {q, k, v, out, dout, lse}, {&std::get<0>(r), &std::get<1>(r), &std::get<2>(r)});
+  refuse_gradient("ts2ts::masked_attn_bwd", {q, k, v, out, dout, lse}, {&std::get<0>(r), &std::get<1>(r), &std::get<2>(r)});
   return r;
 }
 
@@ -224,7 +224,7 @@ std::tuple<Tensor, Tensor> attn_decode_autograd(const Tensor& q, const Tensor& k
     at::AutoDispatchBelowADInplaceOrView below;
     r = op.call(q, k, v, doc_ids, link_bits, q_row_ids, kv_col_ids, q_pos, scale);
   }
-  refuse_gradient<3>("ts2ts::masked_attn_decode", {q, k, v}, {&std::get<0>(r), &std::get<1>(r)});
+  refuse_gradient("ts2ts::masked_attn_decode", {q, k, v}, {&std::get<0>(r), &std::get<1>(r)});
   return r;
 }
 
@@ -460,7 +460,8 @@ std::vector<Tensor> pack_mask(at::IntArrayRef starts, at::IntArrayRef ends, at::
 
 // ------------------------------------------------------------------------------------------------ decoder layer
 // Autograd functions around the decoder-layer entry points.  Gradients nobody asked for arrive undefined
-// (set_materialize_grads(false)) instead of as zero tensors of the activation's size.
+// (set_materialize_grads(false)) instead of as zero tensors of the activation's size.  The kernels' gradients have no
+// derivative of their own: made with create_graph they refuse to be differentiated.
 using c10::cuda::CUDAGuard;
 
 // An autograd worker that has made no CUDA call yet has no current context, and cuBLAS asks for one.
@@ -507,6 +508,7 @@ struct AddRMSNorm : torch::autograd::Function<AddRMSNorm> {
                                 has_a ? da.mutable_data_ptr() : nullptr, mfptr(dw), ws.mutable_data_ptr(), ws.numel(), N, static_cast<int>(C),
                                 stream_of(x)),
           "ts2ts_add_rmsnorm_bwd");
+    refuse_gradient("ts2ts::add_rmsnorm backward", {grads[0], grads[1], x, w}, {&dx, &da, &dw});
     return {dx, da, dw, Tensor()};
   }
 };
@@ -580,6 +582,7 @@ struct QKVAttention : torch::autograd::Function<QKVAttention> {
           "ts2ts_attn_bwd");
     // gradient of the rotated q, k -> gradient of the projection's output: the inverse rotation, in place
     check(ts2ts_rope_qk_inplace(dqkv.mutable_data_ptr(), fptr(cos), fptr(sin), B, T, H, D, -1.f, stream), "ts2ts_rope_qk_inplace");
+    refuse_gradient("ts2ts::qkv_attention backward", {grads[0], qkv}, {&dqkv});
     r[0] = dqkv;
     return r;
   }
@@ -612,6 +615,7 @@ struct SwiGLU : torch::autograd::Function<SwiGLU> {
     const int64_t F = gu.size(-1) / 2, N = gu.numel() / (2 * F);
     Tensor dgu = at::empty_like(gu);
     check(ts2ts_swiglu_bwd(gu.const_data_ptr(), dact.const_data_ptr(), dgu.mutable_data_ptr(), N, static_cast<int>(F), stream_of(gu)), "ts2ts_swiglu_bwd");
+    refuse_gradient("ts2ts::swiglu backward", {grads[0], gu}, {&dgu});
     return {dgu};
   }
 };
@@ -643,7 +647,9 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
     check(ts2ts_ce_bwd(logits.mutable_data_ptr(), s[1].const_data_ptr<int64_t>(), fptr(s[2]), fptr(g), static_cast<float>(1.0 / static_cast<double>(N)), N,
                        static_cast<int>(V), stream_of(logits)),
           "ts2ts_ce_bwd");
-    return {logits, Tensor()};
+    Tensor dlogits = logits.detach();  // not the logits' own history
+    refuse_gradient("ts2ts::cross_entropy backward", {grads[0], logits}, {&dlogits});
+    return {dlogits, Tensor()};
   }
 };
 Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); }
@@ -707,24 +713,29 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
                             static_cast<int>(V), stream_of(h)),
           "ts2ts_ce_fwd_grad");
     ctx->save_for_backward({h, wb, logits});
+    ctx->saved_data["w"] = w;
     return loss.mean();
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     const CUDAGuard guard(s[0].device());
     bind_context(s[0]);
-    const Tensor g = grads[0].to(at::kFloat).contiguous();
-    void* stream = stream_of(g);
     Tensor dh, dw;
-    if (ctx->needs_input_grad(0)) {
-      Tensor dh32 = at::mm(s[2], s[1], at::kFloat);
-      dh = at::empty(s[0].sizes(), s[0].options());
-      check(ts2ts_scale(mfptr(dh32), dh.mutable_data_ptr(), fptr(g), dh.numel(), stream), "ts2ts_scale");
+    {
+      const at::AutoGradMode plain(false);
+      const Tensor g = grads[0].to(at::kFloat).contiguous();
+      void* stream = stream_of(g);
+      if (ctx->needs_input_grad(0)) {
+        Tensor dh32 = at::mm(s[2], s[1], at::kFloat);
+        dh = at::empty(s[0].sizes(), s[0].options());
+        check(ts2ts_scale(mfptr(dh32), dh.mutable_data_ptr(), fptr(g), dh.numel(), stream), "ts2ts_scale");
+      }
+      if (ctx->needs_input_grad(1)) {
+        dw = at::mm(s[2].t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
+        check(ts2ts_scale(mfptr(dw), nullptr, fptr(g), dw.numel(), stream), "ts2ts_scale");
+      }
     }
-    if (ctx->needs_input_grad(1)) {
-      dw = at::mm(s[2].t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
-      check(ts2ts_scale(mfptr(dw), nullptr, fptr(g), dw.numel(), stream), "ts2ts_scale");
-    }
+    refuse_gradient("ts2ts::head_loss backward", {grads[0], s[0], ctx->saved_data["w"].toTensor()}, {&dh, &dw});
     return {dh, dw, Tensor()};
   }
 };
@@ -742,6 +753,7 @@ struct Embedding : torch::autograd::Function<Embedding> {
     const Tensor idx = ctx->get_saved_variables()[0].contiguous(), dx = grads[0].contiguous();
     const CUDAGuard guard(dx.device());
     const int64_t V = ctx->saved_data["V"].toInt(), C = dx.size(-1);
+    if (at::GradMode::is_enabled()) return {at::embedding_dense_backward(dx, idx, V, -1, false), Tensor()};  // may be differentiated again
     Tensor dw = at::empty({V, C}, dx.options());
     check(ts2ts_embedding_bwd(idx.const_data_ptr<int64_t>(), fptr(dx), mfptr(dw), idx.numel(), static_cast<int>(C), V, stream_of(dx)),
           "ts2ts_embedding_bwd");

@@ -62,3 +62,42 @@ def test_second_derivative_of_a_linear_layer_matches_torch():
         lin.weight.add_(1)
     with pytest.raises(RuntimeError, match="inplace"):
         torch.autograd.grad(y.sum(), x, create_graph=True)
+
+
+def _layer_losses():
+    from tagseq2tagseq_b200 import lm_fused as lf
+    from tagseq2tagseq_b200.mask_spec import MaskSpec
+    x, w = torch.randn(6, 64, device=DEV, requires_grad=True), torch.randn(64, device=DEV, requires_grad=True)
+    yield "add_rmsnorm", lf.add_rmsnorm(x, None, w, 1e-6)[1].float().pow(2).sum(), x
+    gu = _bf16(6, 128).requires_grad_(True)
+    yield "swiglu", lf.swiglu(gu).float().pow(2).sum(), gu
+    h, wh = _bf16(6, 64).requires_grad_(True), torch.randn(128, 64, device=DEV, requires_grad=True)
+    target = torch.arange(6, device=DEV)
+    yield "head_loss", lf.head_loss(h, wh, target), h
+    yield "head_loss", lf.head_loss(h, wh, target), wh
+    logits = _bf16(6, 128).requires_grad_(True)
+    yield "cross_entropy", lf.cross_entropy(logits * 1, target), logits
+    qkv = _bf16(1, 6, 3 * 64).requires_grad_(True)
+    cos, sin = lf.rope_half_tables(6, 64, 10000.0, DEV)
+    mask = MaskSpec(torch.zeros(1, 6, dtype=torch.int32, device=DEV))
+    yield "qkv_attention", lf.qkv_attention(qkv * 1, cos, sin, mask, 1, 64).float().pow(2).sum(), qkv
+
+
+def test_second_derivatives_of_the_layer_kernels_are_refused():
+    for name, loss, at in _layer_losses():
+        grad, = torch.autograd.grad(loss, at, create_graph=True)
+        with pytest.raises(RuntimeError, match="not implemented"):
+            grad.float().pow(2).sum().backward()
+        assert grad.isfinite().all(), name
+
+
+def test_second_derivative_of_an_embedding_matches_torch():
+    from tagseq2tagseq_b200.lm_fused import embedding
+    idx = torch.tensor([[3, 1, 3, 0]], device=DEV)
+    got = []
+    for f in (embedding, lambda w, i: F.embedding(i, w)):
+        torch.manual_seed(1)
+        w = torch.randn(5, 8, device=DEV, requires_grad=True)
+        g, = torch.autograd.grad(f(w, idx).pow(3).sum(), w, create_graph=True)
+        got.append(torch.autograd.grad(g.pow(2).sum(), w)[0])
+    assert (got[0] - got[1]).norm() <= 1e-6 * got[1].norm()

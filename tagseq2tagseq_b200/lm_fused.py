@@ -10,6 +10,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad as fwAD
 
 from . import _lib
 from .mask_spec import MaskSpec
@@ -92,15 +93,21 @@ def embedding(weight: torch.Tensor, tokens: torch.Tensor) -> torch.Tensor:
     return F.embedding(tokens, weight)
 
 
+def _transformed() -> bool:
+    """Whether a torch.func transform or forward-mode differentiation is active: C++ autograd functions know neither."""
+    return torch._C._functorch.peek_interpreter_stack() is not None or fwAD._current_level >= 0
+
+
 class Linear(nn.Linear):
-    """A bias-free linear layer with an fp32 weight.  bf16 activations multiply the weight's bf16 copy, and the weight
-    gradient is produced in fp32; anything else is torch's own layer."""
+    """A bias-free linear layer with an fp32 weight.  Under bf16 autocast, bf16 activations multiply the weight's bf16 copy,
+    and the weight gradient is produced in fp32; anything else is torch's own layer."""
 
     def __init__(self, in_features: int, out_features: int):
         super().__init__(in_features, out_features, bias=False)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32:
+        if (x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
+                and torch.get_autocast_dtype("cuda") == torch.bfloat16 and (torch.compiler.is_compiling() or not _transformed())):
             return _call(_lib.ops().linear.default, x, self.weight)
         return super().forward(x)
 

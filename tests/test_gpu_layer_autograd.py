@@ -101,3 +101,17 @@ def test_second_derivative_of_an_embedding_matches_torch():
         g, = torch.autograd.grad(f(w, idx).pow(3).sum(), w, create_graph=True)
         got.append(torch.autograd.grad(g.pow(2).sum(), w)[0])
     assert (got[0] - got[1]).norm() <= 1e-6 * got[1].norm()
+
+
+def test_linear_outside_bf16_autocast_is_torchs_layer():
+    lin, x = _linear(), _bf16(4, 64)
+    with pytest.raises(RuntimeError, match="dtype"):
+        lin(x)                                                       # bf16 against an fp32 weight
+    with torch.autocast("cuda", torch.float16):
+        assert torch.equal(lin(x), F.linear(x, lin.weight)) and lin(x).dtype == torch.float16
+    with torch.autocast("cuda", torch.bfloat16):
+        ref = torch.func.grad(lambda t: F.linear(t, lin.weight).float().pow(2).sum())(x)
+        assert torch.equal(torch.func.grad(lambda t: lin(t).float().pow(2).sum())(x), ref)
+        with torch.autograd.forward_ad.dual_level():
+            dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+            assert torch.autograd.forward_ad.unpack_dual(lin(dual)).tangent is not None

@@ -62,7 +62,7 @@ int ts2ts_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float in
 int ts2ts_scale(float* x, void* out, const float* gscale, int64_t n, void* stream);
 
 /* dw[V,C] (fp32, overwritten) = the sum of the rows dx[N,C] (fp32) of equal idx[N] (int64; an index outside 0..V-1 is
- * ignored).  C % 4 == 0.  The order of the additions is not fixed. */
+ * ignored).  C % 4 == 0, V < 2^31.  The additions are made in an order that depends on idx alone. */
 int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, void* stream);
 
 /* One AdamW step over `count` fp32 tensors.  p, g, m, v: host arrays of device pointers (parameter, gradient, first and

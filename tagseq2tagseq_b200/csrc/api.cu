@@ -426,7 +426,8 @@ int ts2ts_scale(float* x, void* out, const float* gscale, int64_t n, void* strea
 int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, void* stream) {
   int r;
   if ((r = check_rows(N))) return r;
-  if (C < 4 || C % 4 || V <= 0) return fail(-2, "C must be a positive multiple of 4 and V positive (got %d, %lld)", C, (long long)V);
+  if (C < 4 || C % 4 || V <= 0 || V > INT32_MAX)
+    return fail(-2, "C must be a positive multiple of 4 and V in 1..2^31-1 (got %d, %lld)", C, (long long)V);
   if (!idx || !dx || !dw) return fail(-3, "embedding_bwd: null pointer");
   if (!aligned(dx, 16) || !aligned(dw, 16)) return fail(-5, "embedding_bwd: misaligned pointer");
   return launched(launch_embedding_bwd(idx, dx, dw, N, C, V, static_cast<cudaStream_t>(stream)), "embedding_bwd");

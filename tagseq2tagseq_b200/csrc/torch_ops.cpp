@@ -782,11 +782,12 @@ void adamw(at::TensorList params, at::TensorList grads, at::TensorList exp_avgs,
                         "adamw: contiguous fp32 CUDA tensors");
     p[i] = mfptr(params[i]); g[i] = fptr(grads[i]); m[i] = mfptr(exp_avgs[i]); v[i] = mfptr(exp_avg_sqs[i]);
     sizes[i] = params[i].numel();
-    t[i] = *mfptr(steps[i]) += 1.f;
+    t[i] = *fptr(steps[i]) + 1.f;
   }
   check(ts2ts_adamw(static_cast<int>(n), p.data(), g.data(), m.data(), v.data(), sizes.data(), t.data(), lr, beta1, beta2, eps, weight_decay,
                     stream_of(params[0])),
         "ts2ts_adamw");
+  for (size_t i = 0; i < n; ++i) *mfptr(steps[i]) = t[i];
   for (const Tensor& x : params) x.unsafeGetTensorImpl()->bump_version();
 }
 

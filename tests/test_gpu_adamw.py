@@ -1,0 +1,18 @@
+"""The native AdamW step: refused calls, loss scaling, states of other optimizers, and its rounding."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def test_a_refused_step_advances_no_counter():
+    from tagseq2tagseq_b200 import _lib
+    p, g, m, v = ([torch.ones(8, device=DEV) for _ in range(2)] for _ in range(4))
+    steps = [torch.zeros(()) for _ in range(2)]
+    g[1] = torch.ones(7, device=DEV)
+    with pytest.raises(ValueError, match="adamw"):
+        _lib.ops().adamw(p, g, m, v, steps, 1e-3, 0.9, 0.95, 1e-8, 0.1)
+    assert [float(s) for s in steps] == [0.0, 0.0] and float(p[0][0]) == 1.0
+    _lib.ops().adamw(p[:1], g[:1], m[:1], v[:1], steps[:1], 1e-3, 0.9, 0.95, 1e-8, 0.1)
+    assert [float(s) for s in steps] == [1.0, 0.0]

@@ -113,9 +113,12 @@ class Linear(nn.Linear):
 
 
 class AdamW(torch.optim.AdamW):
-    """torch.optim.AdamW with its state layout, the step being one launch of ``ts2ts_adamw`` per parameter group."""
+    """torch.optim.AdamW with its state layout, the step being one launch of ``ts2ts_adamw`` per parameter group.  With
+    ``fused=True`` it is torch's step, which a gradient scaler leaves the unscaling and the skipping to."""
 
     def _native(self, group, params) -> bool:
+        if getattr(self, "_step_supports_amp_scaling", False) or getattr(self, "grad_scale", None) is not None or getattr(self, "found_inf", None) is not None:
+            return False
         return (not group["amsgrad"] and not group["maximize"] and not group["capturable"] and not group["differentiable"]
                 and not isinstance(group["lr"], torch.Tensor)
                 and all(p.is_cuda and p.device == params[0].device and p.dtype == torch.float32 and p.is_contiguous() and not p.grad.is_sparse

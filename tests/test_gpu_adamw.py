@@ -16,3 +16,22 @@ def test_a_refused_step_advances_no_counter():
     assert [float(s) for s in steps] == [0.0, 0.0] and float(p[0][0]) == 1.0
     _lib.ops().adamw(p[:1], g[:1], m[:1], v[:1], steps[:1], 1e-3, 0.9, 0.95, 1e-8, 0.1)
     assert [float(s) for s in steps] == [1.0, 0.0]
+
+
+def test_a_gradient_scaler_is_not_passed_by():
+    """With fused=True the scaler hands its scale and its inf flag to the optimizer instead of acting on them itself."""
+    from tagseq2tagseq_b200.lm_fused import AdamW
+    for kw in ({"fused": True}, {}):
+        p = torch.nn.Parameter(torch.ones(16, device=DEV))
+        plain = torch.nn.Parameter(torch.ones(16, device=DEV))
+        opt, ref = AdamW([p], lr=1e-2, eps=1e-3, **kw), torch.optim.AdamW([plain], lr=1e-2, eps=1e-3)
+        scaler = torch.amp.GradScaler("cuda", init_scale=1024.0)
+        scaler.scale(torch.zeros((), device=DEV))
+        p.grad = torch.full_like(p, float("inf"))
+        scaler.step(opt)
+        scaler.update()
+        assert torch.equal(p.detach(), torch.ones_like(p)), kw
+        p.grad, plain.grad = torch.full_like(p, 2e-3 * scaler.get_scale()), torch.full_like(p, 2e-3)
+        scaler.step(opt)
+        ref.step()
+        assert (p - plain).abs().max() <= 1e-6, kw

@@ -28,9 +28,10 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libts2ts_attn.so")
 SELFTEST_LIB = os.path.join(HERE, "libts2ts_selftest.so")  # test-only: the bounded-wait self-test kernel
 TORCH_LIB = os.path.join(HERE, "libts2ts_torch.so")
-SOURCES = ["api.cu", "block_map.cu", "link_scan.cu", "attn_fwd.cu", "attn_bwd.cu", "attn_decode.cu", "lm_fused.cu"]
+SOURCES = ["api.cu", "block_map.cu", "link_scan.cu", "attn_fwd.cu", "attn_bwd.cu", "attn_decode.cu", "lm_fused.cu", "adamw.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v"]
+IEEE_SOURCES = ("adamw.cu",)  # compiled without --use_fast_math
 SELFTEST_FLAGS = [f for f in NVCC_FLAGS if f not in ("-Xptxas", "-v")] + ["-DTS2TS_SPIN_LIMIT=4096u"]
 
 
@@ -62,6 +63,10 @@ def _digest(files, words) -> str:
     return h.hexdigest()
 
 
+def _flags(src: str) -> list:
+    return [f for f in NVCC_FLAGS if f != "--use_fast_math" or src not in IEEE_SOURCES]
+
+
 def _object(src: str) -> str:
     return os.path.join(OBJ, src.replace(".cu", ".o"))
 
@@ -74,9 +79,9 @@ def _wanted(path: str) -> str:
     if path == SELFTEST_LIB:
         return _digest([os.path.join(CSRC, "selftest_wait.cu"), *_headers()], SELFTEST_FLAGS)
     if path == LIB:
-        return _digest([os.path.join(CSRC, s) for s in SOURCES] + _headers(), NVCC_FLAGS)
+        return _digest([os.path.join(CSRC, s) for s in SOURCES] + _headers(), sum(map(_flags, SOURCES), []))
     src = next(s for s in SOURCES if _object(s) == path)
-    return _digest([os.path.join(CSRC, src), *_headers()], NVCC_FLAGS)
+    return _digest([os.path.join(CSRC, src), *_headers()], _flags(src))
 
 
 def _record(path: str) -> str:
@@ -133,7 +138,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
             obj = _object(src)
             if not force and _up_to_date(obj):
                 return ""
-            return _make(obj, lambda out: [_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", out], src)
+            return _make(obj, lambda out: [_nvcc(), *_flags(src), "-c", os.path.join(CSRC, src), "-o", out], src)
 
         if force or not _up_to_date(LIB):
             with ThreadPoolExecutor(max_workers=6) as ex:

@@ -35,3 +35,14 @@ def test_a_gradient_scaler_is_not_passed_by():
         scaler.step(opt)
         ref.step()
         assert (p - plain).abs().max() <= 1e-6, kw
+
+
+def test_subnormal_moments_are_kept():
+    from tagseq2tagseq_b200.lm_fused import AdamW
+    p = torch.nn.Parameter(torch.ones(40, device=DEV))
+    p.grad = torch.full_like(p, 1e-20)
+    opt = AdamW([p], lr=1.0, betas=(0.9, 0.95), eps=1e-25, weight_decay=0.0)
+    opt.step()
+    v = opt.state[p]["exp_avg_sq"].double()
+    assert (v - 0.05e-40).abs().max() <= 2e-45                   # half a unit of the smallest fp32 number, twice
+    assert p.detach().abs().max() <= 2e-3                        # m / sqrt(v) is one after the bias corrections; v has 12 bits here

@@ -62,8 +62,67 @@ __device__ __forceinline__ void row_axpy(const uint4& raw, float p, float (&o)[8
   }
 }
 
+__device__ __forceinline__ bool may_read(const DecodeParams& p, const int64_t* link_row, int qdoc, int doc, int col) {
+  if (doc == qdoc) return true;
+  if (link_row == nullptr || col < 0 || col >= 64 * p.mask.W) return false;
+  return (static_cast<unsigned long long>(__ldg(link_row + (col >> 6))) >> (col & 63)) & 1ull;
+}
+
+// A warp's keys once more, kRows at a time and asking for weights of zero: m, l and o into `r`.  For rows that came out as no
+// number: keys without weight (padded slots, underflow, all before a maximum that outweighs them) add nothing, whatever
+// their values, but 0 * inf is no number.  Asking at every key of the first pass cost everybody (B = 2, H = 16, Tk = 32768,
+// D = 128: 42.1 -> 45.6 us, or 44.1 us with this pass inlined behind it).
 template <int D>
-__global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeParams p) {
+__device__ __noinline__ void read_carefully(const DecodeParams& p, int qpos, float* r) {
+  constexpr int kLanes = D / 8, kRows = 32 / kLanes;
+  const int h = blockIdx.y, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t base = (size_t)b * p.Tk;
+  const int qdoc = p.mask.doc[base + qpos], row = p.mask.row[base + qpos];
+  const int64_t* link_row = p.mask.link != nullptr && row >= 0 && row < p.mask.R ? p.mask.link + ((size_t)b * p.mask.R + row) * p.mask.W : nullptr;
+  const int sub = lane / kLanes, at = (lane % kLanes) * 8;
+  float q[8], o[8], m = -CUDART_INF_F, l = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    q[i] = __bfloat162float(p.q[(size_t)b * p.q_sb + (size_t)h * p.q_sh + at + i]) * p.scale_log2;
+    o[i] = 0.f;
+  }
+#pragma unroll 1
+  for (int g = blockIdx.x * kDecWarps + warp; g < qpos / 32 + 1; g += gridDim.x * kDecWarps) {
+    const int kv = g * 32 + lane;
+    unsigned keys = __ballot_sync(0xffffffffu, kv <= qpos && may_read(p, link_row, qdoc, p.mask.doc[base + kv], p.mask.col[base + kv]));
+#pragma unroll 1
+    while (keys) {
+      int key = g * 32 + __ffs(keys) - 1;  // of the first row of lanes; rows without a key of their own repeat it
+      bool live = sub == 0;
+      keys &= keys - 1;
+#pragma unroll
+      for (int k = 1; k < kRows; ++k) {
+        if (sub == k && keys) { key = g * 32 + __ffs(keys) - 1; live = true; }
+        keys &= keys - 1;
+      }
+      const uint4 kr = __ldg(reinterpret_cast<const uint4*>(p.k + (size_t)b * p.k_sb + (size_t)h * p.k_sh + (size_t)key * p.k_st + at));
+      const uint4 vr = __ldg(reinterpret_cast<const uint4*>(p.v + (size_t)b * p.v_sb + (size_t)h * p.v_sh + (size_t)key * p.v_st + at));
+      float s = 0.f;
+      row_dot(kr, q, s);
+#pragma unroll
+      for (int x = kLanes / 2; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+      if (!live) s = -CUDART_INF_F;
+      const float mx = fmaxf(m, s), safe = mx == -CUDART_INF_F ? 0.f : mx;
+      const float f = fast_exp2(m - safe), w = fast_exp2(s - safe);
+      m = mx;
+      l = l * f + w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = f == 0.f ? 0.f : o[i] * f;
+      if (w != 0.f) row_axpy(vr, w, o);
+    }
+  }
+  r[0] = m; r[1] = l;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[2 + i] = o[i];
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_constant__ DecodeParams p) {
   constexpr int kLanes = D / 8;            // lanes that share a row
   constexpr int kRows = 32 / kLanes;       // rows a warp reads at once
   constexpr int kBatch = kRows * kUnroll;  // keys a warp takes off its queue at once
@@ -165,6 +224,16 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeP
     __syncwarp();
   }
   if (queued > 0) take(0, queued);
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) bad = bad || o[i] != o[i];
+  if (__any_sync(0xffffffffu, bad)) {
+    float r[10];
+    read_carefully<D>(p, qpos, r);
+    m = r[0]; l = r[1];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = r[2 + i];
+  }
 
   // rows of lanes -> warp
   float mw = m;
@@ -173,7 +242,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeP
   const float fw = m == -CUDART_INF_F ? 0.f : fast_exp2(m - mw);
   l *= fw;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] *= fw;
+  for (int i = 0; i < 8; ++i) o[i] = fw == 0.f ? 0.f : o[i] * fw;
 #pragma unroll
   for (int x = kLanes; x < 32; x <<= 1) {
     l += __shfl_xor_sync(0xffffffffu, l, x);
@@ -197,7 +266,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeP
     for (int w = 0; w < kDecWarps; ++w) {
       const float f = s_m[w] == -CUDART_INF_F ? 0.f : fast_exp2(s_m[w] - mb);
       lb = fmaf(f, s_l[w], lb);
-      ob = fmaf(f, s_o[w][d], ob);
+      ob = fmaf(f, f == 0.f ? 0.f : s_o[w][d], ob);
     }
     if (d == 0) { s_block[0] = mb; s_block[1] = lb; }
     s_block[2 + d] = ob;
@@ -209,11 +278,11 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const DecodeP
     for (int r = 0; r < cs; ++r) mc = fmaxf(mc, *cluster.map_shared_rank(&s_block[0], r));
     float lc = 0.f, oc = 0.f;
     for (int r = 0; r < cs; ++r) {
-      const float mr = *cluster.map_shared_rank(&s_block[0], r);
-      if (mr == -CUDART_INF_F) continue;
-      const float f = fast_exp2(mr - mc);
-      lc = fmaf(f, *cluster.map_shared_rank(&s_block[1], r), lc);
-      oc = fmaf(f, *cluster.map_shared_rank(&s_block[2 + d], r), oc);
+      const float mr = *cluster.map_shared_rank(&s_block[0], r), lr = *cluster.map_shared_rank(&s_block[1], r);
+      const float xr = *cluster.map_shared_rank(&s_block[2 + d], r);
+      const float f = mr == -CUDART_INF_F ? 0.f : fast_exp2(mr - mc);
+      lc = fmaf(f, lr, lc);
+      oc = fmaf(f, f == 0.f ? 0.f : xr, oc);
     }
     p.out[(size_t)b * p.o_sb + (size_t)h * p.o_sh + d] = __float2bfloat16(lc > 0.f ? oc / lc : 0.f);
     if (d == 0) p.lse[(size_t)b * p.H + h] = lc > 0.f ? (mc + log2f(lc)) * 0.6931471805599453f : -CUDART_INF_F;

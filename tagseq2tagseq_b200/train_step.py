@@ -21,7 +21,7 @@ import torch
 import torch.nn as nn
 import torch.nn.modules.module as _module
 
-from .lm_fused import AdamW, Linear, add_rmsnorm, embedding, head_loss, qkv_attention, rope_half_tables, swiglu
+from .lm_fused import AdamW, Linear, add_rmsnorm, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -67,6 +67,12 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.T
     h = x.shape[-1] // 2
     rot = torch.cat([-x[..., h:], x[..., :h]], dim=-1)
     return x * cos + rot * sin
+
+
+def _plain(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` is nothing but ``cls.forward``: that class itself, and no hook of anybody's."""
+    return (type(module) is cls and "forward" not in module.__dict__ and not _module._has_any_global_hook()
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
 
 
 class Block(nn.Module):
@@ -115,13 +121,20 @@ class DecoderLM(nn.Module):
         """tokens int64 [B, T+1]; returns the mean next-token cross-entropy (training_module.py:195-211).  Runs under
         bf16 autocast: the linear layers compute in bf16, the residual stream, norms, rotary angles and the loss in fp32."""
         inp, tgt = tokens[:, :-1], tokens[:, 1:]
-        x = embedding(self.embed.weight, inp).float()
+        e = self.embed
+        if _plain(e, nn.Embedding) and e.padding_idx is None and e.max_norm is None and not e.scale_grad_by_freq and not e.sparse:
+            x = embedding(e.weight, inp).float()
+        else:
+            x = e(inp).float()
         cos, sin = self._rope_tables(inp.shape[1], inp.device)
         a = None
         for blk in self.blocks:
             x, a = blk(x, a, mask, cos, sin)
         _, h = add_rmsnorm(x, a, self.norm.weight, RMS_EPS)
-        return head_loss(h, self.head.weight, tgt)
+        if _plain(self.head, Linear) and self.head.bias is None:
+            return head_loss(h, self.head.weight, tgt)
+        logits = self.head(h)
+        return cross_entropy(logits.to(torch.bfloat16).view(-1, logits.shape[-1]), tgt.reshape(-1))
 
 
 class _StepGraph:

@@ -110,23 +110,46 @@ class DecoderLM(nn.Module):
         for p in self.parameters():
             if p.dim() >= 2:
                 nn.init.normal_(p, std=0.02)
-        self._rope = None  # the rotation tables of the last sequence length and device
+
+    _rope = None  # (what they are for, the tables of the last sequence length, the stream that made them, their completion)
+
+    def __getstate__(self):
+        return {**self.__dict__, "_rope": None}
 
     def _rope_tables(self, T: int, device):
-        if self._rope is None or self._rope[0] != (T, device):
-            self._rope = ((T, device), rope_half_tables(T, self.cfg.head_dim, self.cfg.rope_base, device))
-        return self._rope[1]
+        """cos and sin of the rotation angles.  The last length's are kept; whoever reads them on another stream waits for the
+        one that made them.  Tables made under a trace or inside a capture belong to that alone."""
+        key = (T, device, self.cfg.head_dim, self.cfg.rope_base)
+        make = lambda: rope_half_tables(T, self.cfg.head_dim, self.cfg.rope_base, device)
+        cuda = device.type == "cuda"
+        if torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or (cuda and torch.cuda.is_current_stream_capturing()):
+            return make()
+        kept = self._rope  # read once: another thread may put another length's there
+        if kept is None or kept[0] != key:
+            with torch.inference_mode(False):  # they are saved for a backward later on
+                tables = make()
+            here = torch.cuda.current_stream(device) if cuda else None
+            self._rope = (key, tables, here, here.record_event() if cuda else None)
+            return tables
+        _, tables, maker, done = kept
+        if cuda and torch.cuda.current_stream(device) != maker:
+            here = torch.cuda.current_stream(device)
+            here.wait_event(done)
+            for t in tables:
+                t.record_stream(here)
+        return tables
 
-    def forward(self, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
+    def forward(self, tokens: torch.Tensor, mask: MaskSpec, rope=None) -> torch.Tensor:
         """tokens int64 [B, T+1]; returns the mean next-token cross-entropy (training_module.py:195-211).  Runs under
-        bf16 autocast: the linear layers compute in bf16, the residual stream, norms, rotary angles and the loss in fp32."""
+        bf16 autocast: the linear layers compute in bf16, the residual stream, norms, rotary angles and the loss in fp32.
+        ``rope``: the rotation tables, for a caller that keeps them."""
         inp, tgt = tokens[:, :-1], tokens[:, 1:]
         e = self.embed
         if _plain(e, nn.Embedding) and e.padding_idx is None and e.max_norm is None and not e.scale_grad_by_freq and not e.sparse:
             x = embedding(e.weight, inp).float()
         else:
             x = e(inp).float()
-        cos, sin = self._rope_tables(inp.shape[1], inp.device)
+        cos, sin = self._rope_tables(inp.shape[1], inp.device) if rope is None else rope
         a = None
         for blk in self.blocks:
             x, a = blk(x, a, mask, cos, sin)
@@ -152,13 +175,14 @@ class _StepGraph:
         self.params = list(owner.model.parameters())
         # read by the graph, but allocated outside of it: the model keeps only the last sequence length's
         self.tables = owner.model._rope_tables(tokens.shape[1] - 1, tokens.device)
+        torch.cuda.current_stream().synchronize()  # they are there for a replay on whichever stream
         self.graph = torch.cuda.CUDAGraph()
         side, here = torch.cuda.Stream(), torch.cuda.current_stream()
         side.wait_stream(here)
         with torch.cuda.stream(side):
             self.graph.capture_begin(capture_error_mode="thread_local")
             try:
-                self.loss = owner._eager(self.tokens, self.mask)
+                self.loss = owner._eager(self.tokens, self.mask, rope=self.tables)
             finally:
                 self.graph.capture_end()
         here.wait_stream(side)
@@ -237,12 +261,12 @@ class TrainStep:
                 return self._graphed(key, tokens, mask)
         return self._eager(tokens, mask, sync)
 
-    def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True) -> torch.Tensor:
+    def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True, rope=None) -> torch.Tensor:
         self.opt.zero_grad(set_to_none=True)
         ctx = self.model.no_sync() if (not sync and self.world > 1) else _nullcontext()
         with ctx:
             with torch.autocast("cuda", dtype=torch.bfloat16):
-                loss = self.model(tokens, mask)
+                loss = self.model(tokens, mask) if rope is None else self.model(tokens, mask, rope)
             loss.backward()
         return loss.detach()
 

@@ -160,6 +160,40 @@ class DecoderLM(nn.Module):
         return cross_entropy(logits.to(torch.bfloat16).view(-1, logits.shape[-1]), tgt.reshape(-1))
 
 
+_OWN_FORWARD = {cls: cls.forward for cls in (DecoderLM, Block, Linear, nn.RMSNorm, nn.Embedding, nn.ModuleList)}
+
+
+class _Layout:
+    """What a model was made of when this was taken."""
+
+    @staticmethod
+    def _settings(m: nn.Module):
+        if isinstance(m, (DecoderLM, Block)):
+            return (m.cfg, *vars(m.cfg).values())
+        return (m.padding_idx, m.max_norm, m.scale_grad_by_freq, m.sparse) if isinstance(m, nn.Embedding) else ()
+
+    def __init__(self, model: nn.Module):
+        self.mods = list(model.modules())
+        self.own = all(type(m) in _OWN_FORWARD for m in self.mods)
+        self.settings = [self._settings(m) for m in self.mods]
+        self.children = [dict(m._modules) for m in self.mods]
+        self.slots = [dict(m._parameters) for m in self.mods]  # with the empty ones
+        self.params = [(p, p.data_ptr()) for slots in self.slots for p in slots.values() if p is not None]
+
+    def holds(self, model: nn.Module) -> bool:
+        same = lambda now, then: now.keys() == then.keys() and all(now[k] is v for k, v in then.items())
+        return (model is self.mods[0] and self.own == all(type(m) in _OWN_FORWARD for m in self.mods)
+                and all(same(m._modules, c) for m, c in zip(self.mods, self.children))
+                and all(same(m._parameters, s) for m, s in zip(self.mods, self.slots))
+                and all(p.data_ptr() == at for p, at in self.params)
+                and all(self._settings(m) == s for m, s in zip(self.mods, self.settings)))
+
+    def hooked(self) -> bool:
+        """Whether some call inside a step is more than the class's own forward, or some gradient is watched or not wanted."""
+        return (not all(_plain(m, type(m)) for m in self.mods) or any(cls.forward is not f for cls, f in _OWN_FORWARD.items())
+                or not all(p.requires_grad and not p._backward_hooks and not p._post_accumulate_grad_hooks for p, _ in self.params))
+
+
 class _StepGraph:
     """Forward and backward of one micro-batch shape as a CUDA graph: its inputs are copied into buffers of the graph's own,
     the block plan is part of it, copies of the gradients it writes are handed to the parameters.  Link bits are padded with rows and
@@ -292,22 +326,14 @@ class TrainStep:
         return key
 
     def _as_built(self) -> bool:
-        """Whether the model is still the one the graphs were captured from: the same modules and parameters at the same
-        addresses, and no hooks, which a replay would not call."""
-        if self._layout is None:
-            mods = list(self.model.modules())
-            self._layout = (mods, [(m._modules, dict(m._modules)) for m in mods],
-                            [(m._parameters, n, p, p.data_ptr()) for m in mods for n, p in m._parameters.items() if p is not None])
-            self._graphs.clear()
-        mods, children, params = self._layout
-        if _module._has_any_global_hook() or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in mods):
-            return False
-        same = all(d == kept for d, kept in children) and all(
-            d.get(n) is p and p.data_ptr() == at for d, n, p, at in params)
-        if not same:
-            self._layout = None  # looked over again, and captured again, from the next step on
-            return False
-        return all(p.requires_grad and not p._backward_hooks and not p._post_accumulate_grad_hooks for _, _, p, _ in params)
+        """Whether a replay does what the model would do: the model is the one the graphs were captured from, made of this
+        package's modules alone and configured as it was, its parameters are where they were, and nothing hangs on it that
+        a replay would not call."""
+        kept = self._layout
+        if kept is None or not kept.holds(self.model):
+            self._graphs.clear()  # captured again, from a layout taken now
+            self._layout = kept = _Layout(self.model)
+        return kept.own and not kept.hooked()
 
     def _graphed(self, key, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
         if key not in self._graphs:  # the first step of a shape runs as it is: libraries set themselves up

@@ -93,7 +93,7 @@ def embedding(weight: torch.Tensor, tokens: torch.Tensor) -> torch.Tensor:
     return F.embedding(tokens, weight)
 
 
-def _transformed() -> bool:
+def transformed() -> bool:
     """Whether a torch.func transform or forward-mode differentiation is active: C++ autograd functions know neither."""
     return torch._C._functorch.peek_interpreter_stack() is not None or fwAD._current_level >= 0
 
@@ -107,7 +107,7 @@ class Linear(nn.Linear):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if (x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
-                and torch.get_autocast_dtype("cuda") == torch.bfloat16 and (torch.compiler.is_compiling() or not _transformed())):
+                and torch.get_autocast_dtype("cuda") == torch.bfloat16 and (torch.compiler.is_compiling() or not transformed())):
             return _call(_lib.ops().linear.default, x, self.weight)
         return super().forward(x)
 

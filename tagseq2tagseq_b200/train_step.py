@@ -20,8 +20,10 @@ from typing import Optional
 import torch
 import torch.nn as nn
 import torch.nn.modules.module as _module
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
-from .lm_fused import AdamW, Linear, add_rmsnorm, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu
+from .lm_fused import AdamW, Linear, add_rmsnorm, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -194,6 +196,13 @@ class _Layout:
                 or not all(p.requires_grad and not p._backward_hooks and not p._post_accumulate_grad_hooks for p, _ in self.params))
 
 
+def _observed() -> bool:
+    """Whether something of the caller's is called for every operator or saved tensor, or follows derivatives of its own."""
+    return bool(transformed() or torch._C._len_torch_dispatch_stack() or torch.is_anomaly_enabled()
+                or any(not isinstance(m, DeviceContext) for m in _get_current_function_mode_stack())
+                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None)
+
+
 class _StepGraph:
     """Forward and backward of one micro-batch shape as a CUDA graph: its inputs are copied into buffers of the graph's own,
     the block plan is part of it, copies of the gradients it writes are handed to the parameters.  Link bits are padded with rows and
@@ -313,14 +322,22 @@ class TrainStep:
         return 6.0 * self.cfg.matmul_params * n_tokens / 1.2e12 < 0.5 * (self.cfg.n_layers + 1)
 
     def _graph_key(self, tokens: torch.Tensor, mask: MaskSpec):
-        doc, link = mask.doc_ids, mask.link_bits
-        if not (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.int64 and tokens.numel() > 0
-                and doc.shape == (tokens.shape[0], tokens.shape[1] - 1) and tokens.device == self.device == doc.device
-                and torch.cuda.current_device() == self.device.index and self._use_graph(doc.numel())):
+        """What a graph is kept by, or None for a step that has to be launched: inputs that the launched step would look at
+        more closely, or a caller that wants to see its operators."""
+        if type(mask) is not MaskSpec or tokens.dim() != 2:
             return None
-        if torch.cuda.is_current_stream_capturing() or not torch.is_grad_enabled() or not self._as_built():
+        doc, link, rows, cols = mask.doc_ids, mask.link_bits, mask.q_row_ids, mask.kv_col_ids
+        B, T = tokens.shape[0], tokens.shape[1] - 1
+        fits = lambda t, dtype: type(t) is torch.Tensor and t.device == self.device and t.dtype == dtype
+        if not (fits(tokens, torch.int64) and B > 0 and T > 0 and self._use_graph(B * T)
+                and all(fits(t, torch.int32) and t.shape == (B, T) for t in (doc, rows, cols) if t is not None)
+                and (link is None or fits(link, torch.int64) and link.dim() == 3 and link.shape[0] == B and link.numel() > 0)
+                and self.device.type == "cuda" and torch.cuda.current_device() == self.device.index):
             return None
-        key = (tokens.shape[0], tokens.shape[1], mask.q_row_ids is not None, mask.kv_col_ids is not None)
+        if torch.cuda.is_current_stream_capturing() or not torch.is_grad_enabled() or _observed() or not self._as_built():
+            return None
+        key = (B, T, rows is not None, cols is not None, torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction,
+               torch.are_deterministic_algorithms_enabled())
         if link is not None:  # capacities in steps of 64 row classes and of powers of two words
             key += (-(-link.shape[1] // 64) * 64, 1 << (link.shape[2] - 1).bit_length())
         return key

@@ -12,6 +12,7 @@ as the reference's are fused modules.
 """
 from __future__ import annotations
 
+import warnings
 from collections import OrderedDict
 from contextlib import nullcontext as _nullcontext
 from dataclasses import dataclass
@@ -215,22 +216,27 @@ class _StepGraph:
         if mask.link_bits is not None:
             self.mask.link_bits = torch.zeros((mask.link_bits.shape[0],) + key[-2:], dtype=torch.int64, device=tokens.device)
         self._load(tokens, mask)
-        self.params = list(owner.model.parameters())
+        names, self.params = zip(*owner.model.named_parameters())
         # read by the graph, but allocated outside of it: the model keeps only the last sequence length's
         self.tables = owner.model._rope_tables(tokens.shape[1] - 1, tokens.device)
         torch.cuda.current_stream().synchronize()  # they are there for a replay on whichever stream
+        # Aliases stand for the parameters: an autograd graph of the caller's that is still alive keeps the nodes that
+        # collect the parameters' gradients on its own stream, which a capture must not touch.
+        alias = {n: p.detach().requires_grad_() for n, p in zip(names, self.params)}
         self.graph = torch.cuda.CUDAGraph()
         side, here = torch.cuda.Stream(), torch.cuda.current_stream()
         side.wait_stream(here)
         with torch.cuda.stream(side):
             self.graph.capture_begin(capture_error_mode="thread_local")
             try:
-                self.loss = owner._eager(self.tokens, self.mask, rope=self.tables)
+                with torch.autocast("cuda", dtype=torch.bfloat16):
+                    loss = torch.func.functional_call(owner.model, alias, (self.tokens, self.mask, self.tables))
+                self.grads = torch.autograd.grad(loss, tuple(alias.values()))
+                self.loss = loss.detach()
             finally:
                 self.graph.capture_end()
         here.wait_stream(side)
         self.mask._block_map = None  # built by the graph, into its own pool
-        self.grads = [p.grad for p in self.params]
 
     def _load(self, tokens, mask):
         self.tokens.copy_(tokens)
@@ -249,7 +255,7 @@ class _StepGraph:
     def run(self, tokens, mask) -> torch.Tensor:
         self._load(tokens, mask)
         self.graph.replay()
-        grads = [torch.empty_like(g) for g in self.grads]  # the graph's own buffers are written again by the next step
+        grads = [torch.empty_like(p) for p in self.params]  # the graph's own buffers are written again by the next step
         torch._foreach_copy_(grads, self.grads)
         for p, g in zip(self.params, grads):
             p.grad = g
@@ -287,6 +293,7 @@ class TrainStep:
         self.opt = AdamW(model.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1)
         self.use_graphs = True
         self._graphs: "OrderedDict[tuple, Optional[_StepGraph]]" = OrderedDict()  # None: shape seen once
+        self._refused = set()  # shapes that could not be captured
         self._layout = None
 
     @property
@@ -304,12 +311,12 @@ class TrainStep:
                 return self._graphed(key, tokens, mask)
         return self._eager(tokens, mask, sync)
 
-    def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True, rope=None) -> torch.Tensor:
+    def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True) -> torch.Tensor:
         self.opt.zero_grad(set_to_none=True)
         ctx = self.model.no_sync() if (not sync and self.world > 1) else _nullcontext()
         with ctx:
             with torch.autocast("cuda", dtype=torch.bfloat16):
-                loss = self.model(tokens, mask) if rope is None else self.model(tokens, mask, rope)
+                loss = self.model(tokens, mask)
             loss.backward()
         return loss.detach()
 
@@ -349,10 +356,13 @@ class TrainStep:
         kept = self._layout
         if kept is None or not kept.holds(self.model):
             self._graphs.clear()  # captured again, from a layout taken now
+            self._refused.clear()
             self._layout = kept = _Layout(self.model)
         return kept.own and not kept.hooked()
 
     def _graphed(self, key, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
+        if key in self._refused:
+            return self._eager(tokens, mask)
         if key not in self._graphs:  # the first step of a shape runs as it is: libraries set themselves up
             self._graphs[key] = None
             while len(self._graphs) > 8:
@@ -362,7 +372,12 @@ class TrainStep:
             live = [k for k, g in self._graphs.items() if g is not None]
             if len(live) >= self.MAX_GRAPHS:
                 del self._graphs[live[0]]
-            self._graphs[key] = _StepGraph(self, tokens, mask, key)
+            try:
+                self._graphs[key] = _StepGraph(self, tokens, mask, key)
+            except RuntimeError as e:  # a step that cannot be captured, or no memory for it, still runs launch by launch
+                warnings.warn(f"training step of {tuple(tokens.shape)} tokens could not be captured and stays launched: {e}")
+                self._refused.add(key)
+                return self._eager(tokens, mask)
         self._graphs.move_to_end(key)
         return self._graphs[key].run(tokens, mask)
 

@@ -274,7 +274,8 @@ class TrainStep:
     On one GPU, a step whose kernels are shorter than the host work of launching them (see ``_use_graph``) is replayed as
     a CUDA graph from the second micro-batch of its shape on.  ``use_graphs = False`` turns that off."""
 
-    MAX_GRAPHS = 2  # micro-batch shapes whose graph, and with it a step's activations, is kept
+    MAX_GRAPHS = 2   # micro-batch shapes whose graph, and with it a step's activations, is kept
+    IDLE_STEPS = 64  # steps without a replay after which a graph makes room for another shape's
 
     def __init__(self, cfg: LMConfig, device: torch.device, world: int = 1, lr: float = 3e-4, seed: int = 0,
                  bf16_grads: bool = True, bucket_cap_mb: int = 256):
@@ -292,7 +293,9 @@ class TrainStep:
                 self.model.register_comm_hook(None, default_hooks.bf16_compress_hook)
         self.opt = AdamW(model.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1)
         self.use_graphs = True
-        self._graphs: "OrderedDict[tuple, Optional[_StepGraph]]" = OrderedDict()  # None: shape seen once
+        self._graphs: "OrderedDict[tuple, _StepGraph]" = OrderedDict()  # by last use
+        self._seen: "OrderedDict[tuple, None]" = OrderedDict()  # shapes of earlier steps
+        self._steps = 0
         self._refused = set()  # shapes that could not be captured
         self._layout = None
 
@@ -309,6 +312,8 @@ class TrainStep:
             key = self._graph_key(tokens, mask)
             if key is not None:
                 return self._graphed(key, tokens, mask)
+        elif self._graphs:
+            self._graphs.clear()
         return self._eager(tokens, mask, sync)
 
     def _eager(self, tokens: torch.Tensor, mask: MaskSpec, sync: bool = True) -> torch.Tensor:
@@ -324,9 +329,20 @@ class TrainStep:
     def _use_graph(self, n_tokens: int) -> bool:
         """Launching a step takes about half a millisecond of host time per layer and as much for the rest; the GEMMs
         take 6 FLOPs per parameter and token at 1.2 PFLOP/s or less.  Where the second is shorter, the GPU waits for the
-        host (two layers of d256 at T=1024: 1.38 ms a step, of which 0.38 ms of kernels).  The same bound keeps the
-        activations that a graph holds on to small."""
-        return 6.0 * self.cfg.matmul_params * n_tokens / 1.2e12 < 0.5 * (self.cfg.n_layers + 1)
+        host (two layers of d256 at T=1024: 1.38 ms a step, of which 0.38 ms of kernels).  A graph holds on to a step's
+        memory, which a thin model with a large vocabulary makes much of at the same FLOPs: one graph may take a 32nd of
+        the card's."""
+        return (6.0 * self.cfg.matmul_params * n_tokens / 1.2e12 < 0.5 * (self.cfg.n_layers + 1)
+                and self._graph_bytes(n_tokens) <= torch.cuda.get_device_properties(self.device).total_memory / 32)
+
+    def _graph_bytes(self, n_tokens: int) -> int:
+        """About what a step's graph holds on to: weights' copies and gradients, saved activations, logits, and the largest
+        intermediate gradients."""
+        c = self.cfg
+        hd = c.n_heads * c.head_dim
+        layer = 14 * c.d_model + 8 * hd + 4 * c.n_heads + 6 * c.mlp_hidden  # residual twice in fp32, the rest in bf16
+        return (6 * (c.matmul_params + c.d_model * c.vocab)
+                + n_tokens * (c.n_layers * layer + 2 * c.vocab + 24 * c.d_model + 6 * max(c.mlp_hidden, 2 * hd)))
 
     def _graph_key(self, tokens: torch.Tensor, mask: MaskSpec):
         """What a graph is kept by, or None for a step that has to be launched: inputs that the launched step would look at
@@ -361,25 +377,43 @@ class TrainStep:
         return kept.own and not kept.hooked()
 
     def _graphed(self, key, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
-        if key in self._refused:
-            return self._eager(tokens, mask)
-        if key not in self._graphs:  # the first step of a shape runs as it is: libraries set themselves up
-            self._graphs[key] = None
-            while len(self._graphs) > 8:
-                self._graphs.popitem(last=False)
-            return self._eager(tokens, mask)
-        if self._graphs[key] is None:
-            live = [k for k, g in self._graphs.items() if g is not None]
-            if len(live) >= self.MAX_GRAPHS:
-                del self._graphs[live[0]]
+        self._steps += 1
+        graph = self._graphs.get(key)
+        if graph is None:
+            # the first step of a shape runs as it is: libraries set themselves up
+            if key in self._refused or not self._again(key) or not self._room():
+                return self._eager(tokens, mask)
             try:
-                self._graphs[key] = _StepGraph(self, tokens, mask, key)
+                graph = _StepGraph(self, tokens, mask, key)
             except RuntimeError as e:  # a step that cannot be captured, or no memory for it, still runs launch by launch
                 warnings.warn(f"training step of {tuple(tokens.shape)} tokens could not be captured and stays launched: {e}")
                 self._refused.add(key)
                 return self._eager(tokens, mask)
+        self._graphs[key] = graph
         self._graphs.move_to_end(key)
-        return self._graphs[key].run(tokens, mask)
+        graph.used_at = self._steps
+        return graph.run(tokens, mask)
+
+    def _again(self, key) -> bool:
+        """Whether this shape has come before."""
+        before = key in self._seen
+        self._seen[key] = None
+        self._seen.move_to_end(key)
+        while len(self._seen) > 64:
+            self._seen.popitem(last=False)
+        return before
+
+    def _room(self) -> bool:
+        """Whether one more graph may be kept.  The one that was not replayed for longest makes room, but only if it has been
+        idle for IDLE_STEPS: when more shapes take turns than graphs are kept, the others stay launched, and captures cost
+        at most one in that many steps."""
+        if len(self._graphs) < self.MAX_GRAPHS:
+            return True
+        oldest = next(iter(self._graphs))
+        if self._steps - self._graphs[oldest].used_at <= self.IDLE_STEPS:
+            return False
+        del self._graphs[oldest]
+        return True
 
     def step(self, tokens: torch.Tensor, mask: MaskSpec) -> torch.Tensor:
         loss = self.forward_backward(tokens, mask)

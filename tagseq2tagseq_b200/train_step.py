@@ -236,6 +236,7 @@ class _StepGraph:
             finally:
                 self.graph.capture_end()
         here.wait_stream(side)
+        self.stream = here  # of the last use
         self.mask._block_map = None  # built by the graph, into its own pool
 
     def _load(self, tokens, mask):
@@ -253,6 +254,14 @@ class _StepGraph:
             m.link_bits[:, :R, :W].copy_(mask.link_bits)
 
     def run(self, tokens, mask) -> torch.Tensor:
+        here = torch.cuda.current_stream()
+        if here != self.stream:  # the buffers are in use until the last replay is through
+            here.wait_stream(self.stream)
+            m = self.mask
+            for t in (self.tokens, m.doc_ids, m.link_bits, m.q_row_ids, m.kv_col_ids, *self.tables):
+                if t is not None:
+                    t.record_stream(here)
+            self.stream = here
         self._load(tokens, mask)
         self.graph.replay()
         grads = [torch.empty_like(p) for p in self.params]  # the graph's own buffers are written again by the next step

@@ -43,3 +43,22 @@ def test_a_step_that_cannot_be_captured_runs_launched(monkeypatch):
     with pytest.warns(UserWarning, match="could not be captured"):
         for i in range(4):
             assert torch.equal(ts.step(*_batch(seed=i)), want.step(*_batch(seed=i)))
+
+
+def test_replays_on_two_streams_do_not_share_their_inputs():
+    ts, want = _make(), _make()
+    want.use_graphs = False
+    expect = [float(want.forward_backward(*_batch(seed=i))) for i in range(6)]
+    assert len(set(expect)) == 6
+    for _ in range(2):
+        ts.forward_backward(*_batch(seed=0))
+    batches = [_batch(seed=i) for i in range(6)]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in range(2)], []
+    for i, batch in enumerate(batches):
+        with torch.cuda.stream(streams[i % 2]):
+            if i % 2 == 0:
+                torch.cuda._sleep(20_000_000)                               # some ten milliseconds: the other stream is ahead
+            got.append(ts.forward_backward(*batch))
+    torch.cuda.synchronize()
+    assert [float(x) for x in got] == expect

@@ -144,8 +144,13 @@ class AdamW(torch.optim.AdamW):
                     st["step"] = torch.zeros((), dtype=torch.float32, device="cpu")
                     st["exp_avg"] = torch.zeros_like(p, memory_format=torch.contiguous_format)
                     st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.contiguous_format)
-                elif st["step"].is_cuda:  # a state saved by an optimizer that counts on the device
+                    continue
+                # a state saved by an optimizer that counts on the device or in fp64, or from a tensor of other strides
+                if st["step"].is_cuda or st["step"].dtype != torch.float32:
                     st["step"] = st["step"].float().cpu()
+                for name in ("exp_avg", "exp_avg_sq"):
+                    if not st[name].is_contiguous():
+                        st[name] = st[name].contiguous()
             states = [self.state[p] for p in params]
             _call(_lib.ops().adamw.default, params, [p.grad.contiguous() for p in params], [s["exp_avg"] for s in states],
                   [s["exp_avg_sq"] for s in states], [s["step"] for s in states], g["lr"], *g["betas"], g["eps"], g["weight_decay"])

@@ -46,3 +46,25 @@ def test_subnormal_moments_are_kept():
     v = opt.state[p]["exp_avg_sq"].double()
     assert (v - 0.05e-40).abs().max() <= 2e-45                   # half a unit of the smallest fp32 number, twice
     assert p.detach().abs().max() <= 2e-3                        # m / sqrt(v) is one after the bias corrections; v has 12 bits here
+
+
+def test_states_of_other_strides_and_counters_are_taken():
+    from tagseq2tagseq_b200.lm_fused import AdamW
+    torch.manual_seed(0)
+    p = torch.nn.Parameter(torch.randn(24, 40, device=DEV))
+    ref = torch.nn.Parameter(p.detach().clone())
+    a, b = AdamW([p], lr=1e-2), torch.optim.AdamW([ref], lr=1e-2)
+    grads = [torch.randn(24, 40, device=DEV) for _ in range(3)]
+    for g in grads[:2]:
+        p.grad, ref.grad = g.clone(), g.clone()
+        a.step(), b.step()
+    sd = a.state_dict()
+    st = sd["state"][0]
+    st["exp_avg"], st["exp_avg_sq"] = (st[k].t().contiguous().t() for k in ("exp_avg", "exp_avg_sq"))
+    st["step"] = st["step"].double()
+    a = AdamW([p], lr=1e-2)
+    a.load_state_dict(sd)
+    a.state[p]["step"] = a.state[p]["step"].double()
+    p.grad, ref.grad = grads[2].clone(), grads[2].clone()
+    a.step(), b.step()
+    assert (p - ref).abs().max() <= 1e-6 and float(a.state[p]["step"]) == 3.0

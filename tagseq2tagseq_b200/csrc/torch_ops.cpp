@@ -750,12 +750,14 @@ struct Embedding : torch::autograd::Function<Embedding> {
     return at::embedding(w, idx);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor idx = ctx->get_saved_variables()[0].contiguous(), dx = grads[0].contiguous();
+    const Tensor idx = ctx->get_saved_variables()[0].contiguous();
+    Tensor dx = grads[0].contiguous();
     const CUDAGuard guard(dx.device());
     const int64_t V = ctx->saved_data["V"].toInt(), C = dx.size(-1);
     // torch's own where the gradient may be differentiated again, and for sizes the kernel does not take
     if (at::GradMode::is_enabled() || idx.numel() == 0 || idx.numel() > (1 << 30) || V > INT32_MAX)
       return {at::embedding_dense_backward(dx, idx, V, -1, false), Tensor()};
+    if (reinterpret_cast<uintptr_t>(dx.const_data_ptr()) & 15u) dx = dx.clone();
     Tensor dw = at::empty({V, C}, dx.options());
     check(ts2ts_embedding_bwd(idx.const_data_ptr<int64_t>(), fptr(dx), mfptr(dw), idx.numel(), static_cast<int>(C), V, stream_of(dx)),
           "ts2ts_embedding_bwd");

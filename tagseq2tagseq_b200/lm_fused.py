@@ -88,7 +88,8 @@ def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> to
 
 def embedding(weight: torch.Tensor, tokens: torch.Tensor) -> torch.Tensor:
     """Rows of an fp32 embedding table."""
-    if weight.is_cuda and weight.dtype == torch.float32 and weight.shape[1] % 4 == 0 and tokens.dtype == torch.int64:
+    if (weight.is_cuda and weight.dtype == torch.float32 and weight.shape[1] % 4 == 0 and tokens.dtype == torch.int64
+            and (torch.compiler.is_compiling() or not transformed())):
         return _call(_lib.ops().embedding.default, weight, tokens)
     return F.embedding(tokens, weight)
 

@@ -42,3 +42,14 @@ def test_no_tokens_give_a_zero_gradient():
     w = torch.randn(7, 8, device=DEV, requires_grad=True)
     embedding(w, torch.zeros(1, 0, dtype=torch.int64, device=DEV)).sum().backward()
     assert torch.equal(w.grad, torch.zeros_like(w))
+
+
+def test_gradients_at_odd_addresses_and_transforms_are_taken_as_torch_takes_them():
+    from tagseq2tagseq_b200.lm_fused import embedding
+    idx = torch.tensor([[3, 1, 3]], device=DEV)
+    w, g = torch.randn(7, 8, device=DEV, requires_grad=True), torch.randn(25, device=DEV)[1:].view(1, 3, 8)
+    got, = torch.autograd.grad(embedding(w, idx), w, g)
+    want, = torch.autograd.grad(torch.nn.functional.embedding(idx, w), w, g)
+    assert torch.equal(got, want)
+    grad = torch.func.grad(lambda t: (embedding(t, idx) * g).sum())(w.detach())
+    assert torch.equal(grad, want)

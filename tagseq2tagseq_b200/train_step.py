@@ -356,7 +356,7 @@ class TrainStep:
     def _graph_key(self, tokens: torch.Tensor, mask: MaskSpec):
         """What a graph is kept by, or None for a step that has to be launched: inputs that the launched step would look at
         more closely, or a caller that wants to see its operators."""
-        if type(mask) is not MaskSpec or tokens.dim() != 2:
+        if type(mask) is not MaskSpec or tokens.dim() != 2 or self.device.type != "cuda":
             return None
         doc, link, rows, cols = mask.doc_ids, mask.link_bits, mask.q_row_ids, mask.kv_col_ids
         B, T = tokens.shape[0], tokens.shape[1] - 1
@@ -364,7 +364,7 @@ class TrainStep:
         if not (fits(tokens, torch.int64) and B > 0 and T > 0 and self._use_graph(B * T)
                 and all(fits(t, torch.int32) and t.shape == (B, T) for t in (doc, rows, cols) if t is not None)
                 and (link is None or fits(link, torch.int64) and link.dim() == 3 and link.shape[0] == B and link.numel() > 0)
-                and self.device.type == "cuda" and torch.cuda.current_device() == self.device.index):
+                and torch.cuda.current_device() == self.device.index):
             return None
         if torch.cuda.is_current_stream_capturing() or not torch.is_grad_enabled() or _observed() or not self._as_built():
             return None

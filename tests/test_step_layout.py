@@ -52,3 +52,10 @@ def test_hooks_and_replaced_forwards_are_not_replayed_over(step, change):
 def test_a_class_whose_forward_was_replaced_is_noticed(step, monkeypatch):
     monkeypatch.setattr(DecoderLM, "forward", lambda self, *a: 0)
     assert not step._as_built()
+
+
+def test_a_step_on_the_cpu_is_refused_as_the_kernels_refuse_it():
+    from tagseq2tagseq_b200 import MaskSpec
+    ts = TrainStep(LMConfig(**CFG), torch.device("cpu"))
+    with pytest.raises(RuntimeError, match="CUDA"):
+        ts.forward_backward(torch.zeros(1, 5, dtype=torch.int64), MaskSpec(torch.zeros(1, 4, dtype=torch.int32)))

@@ -13,6 +13,7 @@
 // Tokens past T belong to no run, which reproduces torch's pad-with-False: a
 // ragged last tile is never full.  A diagonal pair always holds its own
 // diagonal (allowed) and the upper triangle (not allowed), so it is partial.
+#include "launch.cuh"
 #include "plan.h"
 #include "ptx.cuh"
 
@@ -31,6 +32,7 @@ __device__ __forceinline__ bool link_bit(const int64_t* link_b, int R, int W, in
 // of its own cost more than either.  The first block clears the status words.
 __global__ void __launch_bounds__(128) runs_kernel(PlanView P, MaskArgs M, int t_words) {
   const int tb = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
+  let_next_start();
   if (tb == 0 && b == 0 && t < 64) P.status[t] = 0;
   if (tb >= P.NB) {
     const int per_word = (64 * M.W + 127) / 128, at = tb - P.NB;
@@ -96,6 +98,7 @@ __device__ __forceinline__ void add_run(uint32_t (&bits)[4], int start, int end)
 __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint8_t* state_out) {
   const int kb0 = blockIdx.x * kStateKb, qb = blockIdx.y, b = blockIdx.z;
   const size_t tq = (size_t)b * P.NB + qb;
+  after_previous();
   if (kb0 > qb) {  // above the diagonal
     const int kb = kb0 + threadIdx.x;
     if (threadIdx.x < kStateKb && kb < P.NB) {
@@ -117,9 +120,9 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
   for (int i = threadIdx.x; i < kStateKb * kMaskRuns; i += 128) {
     const int k = i / kMaskRuns, r = i % kMaskRuns;
     if (k < n_kb) {
-      const int4 run = __ldg(reinterpret_cast<const int4*>(P.runs + (tk0 + k) * kTile) + r);
+      const int4 run = reinterpret_cast<const int4*>(P.runs + (tk0 + k) * kTile)[r];
       s_krun[k][r] = make_int2(run.y, run.w);
-      s_kmask[k][r] = __ldg(P.run_mask + (tk0 + k) * kMaskRuns + r);
+      s_kmask[k][r] = P.run_mask[(tk0 + k) * kMaskRuns + r];
     }
   }
   if ((int)threadIdx.x < nq) s_runs[threadIdx.x] = reinterpret_cast<const int4*>(P.runs + tq * kTile)[threadIdx.x];
@@ -220,12 +223,14 @@ struct ListOutputs {
 __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_out, ListOutputs bwd_out) {
   const int transposed = blockIdx.z;
   const int line = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, lane = threadIdx.x & 31;
+  after_previous();
   if (transposed == 2) {
     const int NP = (P.NB + 1) / 2;
     if (line >= NP) return;
     const uint8_t* s0 = P.state + ((size_t)b * P.NB + 2 * line) * P.NB;
     const uint8_t* s1 = (2 * line + 1 < P.NB) ? s0 + P.NB : s0;
     int n = 0;
+#pragma unroll 8
     for (int kb = lane; kb <= min(2 * line + 1, P.NB - 1); kb += 32) n += (s0[kb] | s1[kb]) != kSkip;
     for (int sh = 16; sh > 0; sh >>= 1) n += __shfl_xor_sync(0xffffffffu, n, sh);
     if (lane == 0) P.pair_cnt[(size_t)b * NP + line] = n;
@@ -239,18 +244,28 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
   const size_t lb = (size_t)b * P.NB + line;
   int32_t* m_idx = (transposed ? P.bwd_idx : P.fwd_idx) + lb * P.NB;
   int n_m = 0, n_p = 0, n_f = 0;
-  for (int c0 = 0; c0 < P.NB; c0 += 32) {
-    const int c = c0 + lane;
-    uint8_t st = kSkip;
-    if (c < P.NB) st = transposed ? P.state[((size_t)b * P.NB + c) * P.NB + line] : P.state[lb * P.NB + c];
-    const unsigned bm = __ballot_sync(0xffffffffu, st != kSkip);
-    const unsigned bp = __ballot_sync(0xffffffffu, st == kPartial);
-    const unsigned bf = __ballot_sync(0xffffffffu, st == kFull);
-    const unsigned below = (1u << lane) - 1u;
-    if (st != kSkip) m_idx[n_m + __popc(bm & below)] = c | (st == kFull ? (int)kFullBit : 0);
-    if (part_idx && st == kPartial) part_idx[lb * P.NB + n_p + __popc(bp & below)] = c;
-    if (full_idx && st == kFull) full_idx[lb * P.NB + n_f + __popc(bf & below)] = c;
-    n_m += __popc(bm); n_p += __popc(bp); n_f += __popc(bf);
+  constexpr int kAhead = 8;  // states a lane loads before it counts the first: the loads are what a line waits for
+  for (int c0 = 0; c0 < P.NB; c0 += 32 * kAhead) {
+    uint8_t sts[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + 32 * u + lane;
+      sts[u] = kSkip;
+      if (c < P.NB) sts[u] = transposed ? P.state[((size_t)b * P.NB + c) * P.NB + line] : P.state[lb * P.NB + c];
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + 32 * u + lane;
+      const uint8_t st = sts[u];
+      const unsigned bm = __ballot_sync(0xffffffffu, st != kSkip);
+      const unsigned bp = __ballot_sync(0xffffffffu, st == kPartial);
+      const unsigned bf = __ballot_sync(0xffffffffu, st == kFull);
+      const unsigned below = (1u << lane) - 1u;
+      if (st != kSkip) m_idx[n_m + __popc(bm & below)] = c | (st == kFull ? (int)kFullBit : 0);
+      if (part_idx && st == kPartial) part_idx[lb * P.NB + n_p + __popc(bp & below)] = c;
+      if (full_idx && st == kFull) full_idx[lb * P.NB + n_f + __popc(bf & below)] = c;
+      n_m += __popc(bm); n_p += __popc(bp); n_f += __popc(bf);
+    }
   }
   for (int c = n_m + lane; c < P.NB; c += 32) m_idx[c] = -1;
   if (part_idx) for (int c = n_p + lane; c < P.NB; c += 32) part_idx[lb * P.NB + c] = -1;
@@ -262,21 +277,25 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
   }
 }
 
-// Heaviest-first order inside each batch element: rank by descending count, ties by index.
+// Heaviest-first order inside each batch element: rank by descending count, ties by index.  Eight lanes share a tile and
+// compare its count with an eighth of the others each.
 // which = 0: q tiles by fwd_cnt, 1: kv tiles by bwd_cnt, 2: q-tile pairs by pair_cnt.
+constexpr int kOrderLanes = 8, kOrderTiles = 256 / kOrderLanes;
 __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows) {
-  const int b = blockIdx.y, which = blockIdx.z;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0 && b == 0 && which == 0) {  // this is the last launch of the pre-pass: stamp the plan (see plan.h)
+  const int b = blockIdx.y, which = blockIdx.z, sub = threadIdx.x % kOrderLanes;
+  const int i = blockIdx.x * kOrderTiles + threadIdx.x / kOrderLanes;
+  after_previous();
+  if (blockIdx.x == 0 && threadIdx.x == 0 && b == 0 && which == 0) {  // this is the last launch of the pre-pass: stamp the plan (see plan.h)
     P.status[kStampMagic] = kPlanMagic;
     P.status[kStampB] = P.B;
     P.status[kStampT] = P.T;
     P.status[kLinkTRows] = link_t_rows;
   }
   const int n = which == 2 ? (P.NB + 1) / 2 : P.NB;
+  if ((int)blockIdx.x * kOrderTiles >= n) return;
   const int32_t* cnt = (which == 2 ? P.pair_cnt : which == 1 ? P.bwd_cnt : P.fwd_cnt) + (size_t)b * n;
   int32_t* order = (which == 2 ? P.pair_order : which == 1 ? P.bwd_order : P.fwd_order) + (size_t)b * n;
-  __shared__ int4 s_cnt[256];  // 1024 counts at a time, read by all threads alike
+  __shared__ int4 s_cnt[256];  // 1024 counts at a time
   const int ci = i < n ? cnt[i] : 0;
   int rank = 0;
   for (int j0 = 0; j0 < n; j0 += 1024) {
@@ -284,14 +303,17 @@ __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows)
     for (int j = threadIdx.x; j < 1024; j += blockDim.x) reinterpret_cast<int*>(s_cnt)[j] = j0 + j < n ? cnt[j0 + j] : -1;
     __syncthreads();
     const int m = (min(1024, n - j0) + 3) / 4;  // counts of -1 outrank nobody
-    for (int q = 0; q < m; ++q) {
+#pragma unroll 4
+    for (int q = sub; q < m; q += kOrderLanes) {
       const int4 c = s_cnt[q];
       const int j = j0 + 4 * q;
       rank += (c.x > ci || (c.x == ci && j < i)) + (c.y > ci || (c.y == ci && j + 1 < i)) + (c.z > ci || (c.z == ci && j + 2 < i)) +
               (c.w > ci || (c.w == ci && j + 3 < i));
     }
   }
-  if (i < n) order[rank] = i;
+#pragma unroll
+  for (int x = kOrderLanes / 2; x > 0; x >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, x);
+  if (i < n && sub == 0) order[rank] = i;
 }
 
 // Per-token ids from a sorted table of segments: token t gets ids[j] for bounds[j] <= t < bounds[j + 1], and -1 before
@@ -314,6 +336,8 @@ cudaError_t launch_segment_ids(const int32_t* bounds, const int32_t* ids, int n_
   return cudaGetLastError();
 }
 
+// The four launches depend on one another and take a few microseconds each, so each starts while the one before still runs
+// (launch.cuh): with the lists' loads ahead and the shared ranking 29.0 -> 24.3-25.8 us a call at B = 2, T = 32768 with explicit lists.
 // Host entry: fills the plan; optional BlockMask-shaped outputs may be null.
 cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t* kv_cnt, int32_t* kv_idx,
                              int32_t* full_cnt, int32_t* full_idx, int32_t* q_cnt, int32_t* q_idx, int32_t* full_q_cnt,
@@ -322,11 +346,13 @@ cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t
   const bool t = M.link != nullptr && M.R > 0 && M.R <= kLinkTMaxRows && 64 * M.W <= kLinkTMaxCols;
   const int t_words = t ? (M.R + 63) / 64 : 0;
   runs_kernel<<<dim3(P.NB + t_words * ((64 * M.W + 127) / 128), P.B), 128, 0, stream>>>(P, M, t_words);
-  state_kernel<<<dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream>>>(P, M, state_out);
-  lists_kernel<<<dim3((P.NB + 3) / 4, P.B, 3), 128, 0, stream>>>(P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
-                                                                 ListOutputs{q_cnt, q_idx, full_q_cnt, full_q_idx});
-  order_kernel<<<dim3((P.NB + 255) / 256, P.B, 3), 256, 0, stream>>>(P, t ? M.R : 0);
-  return cudaGetLastError();
+  cudaError_t e = launch_after(state_kernel, dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream, P, M, state_out);
+  if (e == cudaSuccess)
+    e = launch_after(lists_kernel, dim3((P.NB + 3) / 4, P.B, 3), 128, 0, stream, P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
+                     ListOutputs{q_cnt, q_idx, full_q_cnt, full_q_idx});
+  if (e == cudaSuccess) e = launch_after(order_kernel, dim3((P.NB + kOrderTiles - 1) / kOrderTiles, P.B, 3), 256, 0, stream, P, t ? M.R : 0);
+  const cudaError_t last = cudaGetLastError();
+  return e != cudaSuccess ? e : last;
 }
 
 }  // namespace ts2ts

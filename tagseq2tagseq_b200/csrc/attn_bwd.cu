@@ -3,22 +3,22 @@
 // Three kernels:
 //   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, padded to whole tiles); zeroes dQ
 //   attn_bwd     one CTA per 128-key tile of one (batch, head); walks the non-skipped 128-query tiles of the
-//                transposed block list.  Everything is transposed so that a tensor-memory lane is a key row:
-//                  tcgen05  S^T = K Q^T,  dP^T = V dO^T            [128 keys x 128 queries, fp32 in TMEM, N = 128]
+//                transposed block list.  Scores are transposed so that a tensor-memory lane is a key row:
+//                  tcgen05  S^T = K Q^T,  dP^T = V dO^T            [128 keys x 128 queries, fp32 in TMEM]
 //                  warps 0-7 (two threads per key row, 64 queries each), in two phases:
 //                           P^T = exp2(scale S^T - lse2[q]) under the mask, as soon as S^T is complete, written as
-//                           bf16 over the S^T columns just read; then, once dP^T is complete and in two halves of 64
-//                           queries, dS^T = P^T (dP^T - delta[q]) as bf16 next to P^T and to shared memory
-//                  tcgen05  dV += P^T dO,  dK += dS^T Q           (A from TMEM, B MN-major from smem; issued per
-//                           half, so the first half's MMAs overlap the second half's dS^T arithmetic)
-//                           S^T of the NEXT tile, so that its exponentials run under the MMAs that follow
-//                           dQ^T = K^T dS^T                       [D x 128 queries over the consumed dP^T columns]
-//                           dP^T of the next tile once dQ^T has been read out
-//                  warps 8-11 (thread = head-dim lane)  dQ^T -> scaled fp32, 32 queries at a time, through two
-//                           private shared-memory boxes per warp -> TMA reduce-adds into the dQ accumulator
-//                Q tiles are double-buffered in shared memory, dO has one buffer that is reloaded between the dV MMAs of
-//                a tile and dP^T of the next.  dK (scaled) and dV leave through shared memory and TMA stores at the end.
-//   dq_convert   dQ accumulator (fp32, already scaled) -> bf16 dq
+//                           bf16 over the S^T columns just read; then, once dP^T is complete,
+//                           dS^T = P^T (dP^T - delta[q]) as bf16 to shared memory
+//                  tcgen05  dV += P^T dO                          (A from TMEM, B MN-major from smem)
+//                           S^T of the NEXT tile
+//                           dK += dS^T Q,  dQ = dS K              (dS^T from smem: K-major for dK, MN-major for dQ)
+//                           dP^T of the next tile once dQ has been read out of the columns they share
+//                  warps 8-11 (thread = query)  dQ -> fp32, 32 head dimensions at a time, through two
+//                           private shared-memory boxes per warp -> bulk reduce-adds into the dQ accumulator
+//                dV and S^T run while the compute warps form dS^T; dK, dQ and dP^T while they form the exponentials of the
+//                next tile (H = 16, linked 16k: 853 -> 794 us at D = 128, 729 -> 600 at D = 64, against a structure with dV and dK behind
+//                dS^T).  dK (scaled) and dV leave through shared memory and TMA stores at the end.
+//   dq_convert   dQ accumulator (fp32) -> scaled bf16 dq
 //
 // Computes what the reference gets from autograd of PyTorch FlexAttention
 // (torch/_higher_order_ops/flex_attention.py:947-1075): P = exp(S - LSE), dV = P^T dO, dP = dO V^T,
@@ -29,6 +29,8 @@
 #include "tma_host.h"
 
 #include <math_constants.h>
+
+#include <type_traits>
 
 // A debug build may name a private header that defines the hooks below to record clock64() stamps.
 #ifdef TS2TS_BWD_TRACE_HEADER
@@ -57,7 +59,7 @@ struct BwdParams {
   MaskArgs mask;
   const float* lse2;     // [B,H,Tp]
   const float* delta;    // [B,H,Tp]
-  float* dq_acc;         // [B,H,Tp,D]
+  float* dq_acc;         // [B,H,Tp/32][D/4][32 queries][4], unscaled
   __nv_bfloat16* dk;     // for the empty-list path only
   __nv_bfloat16* dv;
   int64_t dk_s[3], dv_s[3];
@@ -69,37 +71,25 @@ struct BwdParams {
 
 constexpr int kBwdThreads = 512;  // warps 0-7 exp/dS, 8-11 dQ reduction, 12 TMA producer, 13 MMA issuer, 14-15 idle
 constexpr int kSubQ = 64;         // query columns per compute half
-#ifndef TS2TS_BWD_X2
-#define TS2TS_BWD_X2 1
-#endif
-#ifndef TS2TS_BWD_LD2
-#define TS2TS_BWD_LD2 0
-#endif
-#ifndef TS2TS_BWD_ELECT
-#define TS2TS_BWD_ELECT 1
-#endif
-#ifndef TS2TS_BWD_DQ_FIRST
-#define TS2TS_BWD_DQ_FIRST 1
-#endif
-#ifndef TS2TS_BWD_SPLIT_ST
-#define TS2TS_BWD_SPLIT_ST 1  // S^T of the next tile in two 64-query halves, the first right behind the first half of dV / dK
-#endif
 
 template <int D>
 struct BwdSmem {
   static constexpr int kSub = D / 64;
   static constexpr int kTileBytes = kTile * D * 2;
   static constexpr int kDsBytes = kTile * kTile * 2;  // dS^T: two halves of [128 key rows x 128 B]
-  static constexpr int kStageBytes = 4 * 2 * 4096;     // dQ staging: per reduction warp two boxes of [32 queries x 32 floats]
-  // K, V, two Q stages, one dO buffer, dS^T, the dQ staging boxes, then row statistics, barriers and flags; plus
+  static constexpr int kQStages = D == 64 ? 3 : 2, kDoStages = D == 64 ? 2 : 1;  // what shared memory holds
+  static constexpr int kSBufs = D == 64 ? 2 : 1;       // S^T buffers: what tensor memory holds
+  static constexpr int kStageBytes = 4 * 2 * 4096;     // dQ staging: per reduction warp two boxes of 32 queries x 32 floats
+  // K, V, Q stages, dO buffers, dS^T, the dQ staging boxes, then row statistics, barriers and flags; plus
   // alignment slack.  The kernel declares no static shared memory, so the dynamic region normally starts 1024-byte
   // aligned and the slack stays unused; if it ever does not fit, the kernel reports status 2900 instead of running.
-  static constexpr int kTiles = 5 * kTileBytes + kDsBytes + kStageBytes;
-  static constexpr int kSmall = 4 * kTile * 4 + 16 * 8 + 16 + 2 * kMaskRuns * 16;  // statistics, barriers, flags, staged masks
+  static constexpr int kTiles = (2 + kQStages + kDoStages) * kTileBytes + kDsBytes + kStageBytes;
+  static constexpr int kStats = 2 * kQStages * kTile * 4, kBars = 20;
+  static constexpr int kSmall = kStats + kBars * 8 + 16 + kQStages * kMaskRuns * 16;  // statistics, barriers, flags, staged masks
   static constexpr int kSlack = 512;
   static constexpr int kBytes = kTiles + kSmall + kSlack;
-  // tensor-memory columns: dV, dK accumulators, S^T (later P^T / dS^T), dP^T (later dQ^T)
-  static constexpr int kDV = 0, kDK = D, kST = 2 * D, kDPT = 2 * D + 128;
+  // tensor-memory columns: dV, dK accumulators, S^T (later P^T), dP^T (later dQ)
+  static constexpr int kDV = 0, kDK = D, kST = 2 * D, kDPT = 2 * D + 128 * kSBufs;
 };
 
 template <uint32_t N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -150,32 +140,17 @@ __device__ __noinline__ uint4 key_mask(const PlanView& P, const MaskArgs& M, int
 // The row statistics of the 32 queries are read from shared memory; every lane of a warp reads the same addresses.
 // `nl2` / `ndl` hold the NEGATED statistics (-lse2, -delta), so that both phases are one packed multiply-add /
 // add per two queries (fp32x2 instructions; a 16-byte shared-memory load yields two ready operand pairs).
-// mode: 0 = every query allowed, 1 = test the bits of `bw`, 2 = no query allowed (nothing is computed).
-__device__ __forceinline__ void p_chunk(const uint32_t (&s)[32], const float* nl2, uint32_t bw, int mode, float scale_log2,
-                                        uint32_t (&pk)[16]) {
-  if (mode == 2) {
-#pragma unroll
-    for (int e = 0; e < 16; ++e) pk[e] = 0u;
-    return;
-  }
+template <bool kMasked>
+__device__ __forceinline__ void p_body(const uint32_t (&s)[32], const float* nl2, uint32_t bw, float scale_log2, uint32_t (&pk)[16]) {
   const unsigned long long scale2 = pack_f32x2(scale_log2, scale_log2);
 #pragma unroll
   for (int e = 0; e < 32; e += 4) {
     const ulonglong2 n4 = *reinterpret_cast<const ulonglong2*>(nl2 + e);
     float x0, x1, x2, x3;
-#if TS2TS_BWD_X2
     unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[e + 0]), __uint_as_float(s[e + 1])), scale2, n4.x), x0, x1);
     unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), scale2, n4.y), x2, x3);
-#else
-    {
-      float n0, n1, n2, n3;
-      unpack_f32x2(n4.x, n0, n1); unpack_f32x2(n4.y, n2, n3);
-      x0 = fmaf(__uint_as_float(s[e + 0]), scale_log2, n0); x1 = fmaf(__uint_as_float(s[e + 1]), scale_log2, n1);
-      x2 = fmaf(__uint_as_float(s[e + 2]), scale_log2, n2); x3 = fmaf(__uint_as_float(s[e + 3]), scale_log2, n3);
-    }
-#endif
     float p0 = fast_exp2(x0), p1 = fast_exp2(x1), p2 = fast_exp2(x2), p3 = fast_exp2(x3);
-    if (mode == 1) {
+    if (kMasked) {
       p0 = ((bw >> (e + 0)) & 1u) ? p0 : 0.f;
       p1 = ((bw >> (e + 1)) & 1u) ? p1 : 0.f;
       p2 = ((bw >> (e + 2)) & 1u) ? p2 : 0.f;
@@ -185,9 +160,24 @@ __device__ __forceinline__ void p_chunk(const uint32_t (&s)[32], const float* nl
     pk[(e >> 1) + 1] = pack_bf16(p2, p3);
   }
 }
+// mode: 0 = every query allowed, 1 = test the bits of `bw`, 2 = no query allowed (nothing is computed).  kMasked = false is
+// the code of full tiles, which knows no modes.
+template <bool kMasked>
+__device__ __forceinline__ void p_chunk(const uint32_t (&s)[32], const float* nl2, uint32_t bw, int mode, float scale_log2,
+                                        uint32_t (&pk)[16]) {
+  if (!kMasked || mode == 0) {
+    p_body<false>(s, nl2, bw, scale_log2, pk);
+  } else if (mode == 1) {
+    p_body<true>(s, nl2, bw, scale_log2, pk);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) pk[e] = 0u;
+  }
+}
+template <bool kMasked>
 __device__ __forceinline__ void ds_chunk(const uint32_t (&pk)[16], const uint32_t (&dp)[32], const float* ndl, int mode,
                                          uint32_t (&dsk)[16]) {
-  if (mode == 2) {
+  if (kMasked && mode == 2) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) dsk[e] = 0u;
     return;
@@ -199,18 +189,8 @@ __device__ __forceinline__ void ds_chunk(const uint32_t (&pk)[16], const uint32_
     const unsigned long long p01 = pack_f32x2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u));
     const unsigned long long p23 = pack_f32x2(__uint_as_float(c << 16), __uint_as_float(c & 0xffff0000u));
     float r0, r1, r2, r3;
-#if TS2TS_BWD_X2
     unpack_f32x2(mul_f32x2(p01, add_f32x2(pack_f32x2(__uint_as_float(dp[e + 0]), __uint_as_float(dp[e + 1])), d4.x)), r0, r1);
     unpack_f32x2(mul_f32x2(p23, add_f32x2(pack_f32x2(__uint_as_float(dp[e + 2]), __uint_as_float(dp[e + 3])), d4.y)), r2, r3);
-#else
-    {
-      float n0, n1, n2, n3, q0, q1, q2, q3;
-      unpack_f32x2(d4.x, n0, n1); unpack_f32x2(d4.y, n2, n3);
-      unpack_f32x2(p01, q0, q1); unpack_f32x2(p23, q2, q3);
-      r0 = q0 * (__uint_as_float(dp[e + 0]) + n0); r1 = q1 * (__uint_as_float(dp[e + 1]) + n1);
-      r2 = q2 * (__uint_as_float(dp[e + 2]) + n2); r3 = q3 * (__uint_as_float(dp[e + 3]) + n3);
-    }
-#endif
     dsk[(e >> 1) + 0] = pack_bf16(r0, r1);
     dsk[(e >> 1) + 1] = pack_bf16(r2, r3);
   }
@@ -221,7 +201,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
                 const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV,
-                const __grid_constant__ CUtensorMap mapDQ, const __grid_constant__ BwdParams p) {
+                const __grid_constant__ BwdParams p) {
   using Cfg = BwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   // Plain pointer arithmetic (no round trip through an integer) keeps the shared address space visible to the
@@ -229,27 +209,29 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sK = smem;
   uint8_t* sV = smem + Cfg::kTileBytes;           // must follow sK directly (dQ^T operand padding for D = 64)
-  uint8_t* sQ = smem + 2 * Cfg::kTileBytes;       // two stages, Cfg::kTileBytes each
-  uint8_t* sDO = smem + 4 * Cfg::kTileBytes;      // one buffer: reloaded between the dV MMAs of a tile and dP^T of the next
-  uint8_t* sDS = smem + 5 * Cfg::kTileBytes;      // dS^T, halves of 16 KB
+  uint8_t* sQ = smem + 2 * Cfg::kTileBytes;       // Cfg::kQStages stages
+  uint8_t* sDO = sQ + Cfg::kQStages * Cfg::kTileBytes;  // Cfg::kDoStages buffers
+  uint8_t* sDS = sDO + Cfg::kDoStages * Cfg::kTileBytes;  // dS^T, halves of 16 KB
   uint8_t* sStage = sDS + Cfg::kDsBytes;          // dQ staging boxes
   float (*s_lse2)[kTile] = reinterpret_cast<float (*)[kTile]>(smem + Cfg::kTiles);
-  float (*s_delta)[kTile] = reinterpret_cast<float (*)[kTile]>(smem + Cfg::kTiles + 2 * kTile * 4);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kTiles + 4 * kTile * 4);
+  float (*s_delta)[kTile] = s_lse2 + Cfg::kQStages;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kTiles + Cfg::kStats);
   uint64_t& bar_kv = bars[0];
-  uint64_t* bar_q_full = bars + 1;     // [2] Q, lse2, delta of a stage landed
-  uint64_t& bar_do_full = bars[3];     // dO of the tile landed
-  uint64_t& bar_gd = bars[4];          // dV / dK MMAs of the tile completed: its Q stage and the dO buffer may be reloaded
-  uint64_t& bar_st = bars[5];          // S^T and dP^T of the tile are in tensor memory
-  uint64_t* bar_pds = bars + 6;        // [2] P^T / dS^T of a 64-query half written
-  uint64_t& bar_g = bars[8];           // gradient MMAs of the tile completed (dQ^T readable)
-  uint64_t& bar_dqr = bars[9];         // dQ^T read out of tensor memory
-  uint64_t& bar_epi = bars[10];
-  uint64_t* bar_s = bars + 12;         // [2] S^T of a 64-query half of the tile is in tensor memory (dP^T may still be running)
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 16);
-  volatile int* abort_ptr = reinterpret_cast<volatile int*>(reinterpret_cast<uint8_t*>(bars + 16) + 4);
+  uint64_t* bar_q_full = bars + 1;     // [Q stages] Q, lse2, delta of a stage landed
+  uint64_t* bar_do_full = bars + 4;    // [dO buffers] dO of the tile landed
+  uint64_t* bar_gv = bars + 6;         // [dO buffers] dV MMAs of the tile completed: its dO buffer may be reloaded
+  uint64_t* bar_gq = bars + 8;         // [Q stages] dK MMAs of the tile completed: its Q stage may be reloaded
+  uint64_t* bar_s = bars + 11;         // [S^T buffers] S^T of the tile is in tensor memory
+  uint64_t* bar_p = bars + 13;         // [tile & 1] P^T written
+  uint64_t& bar_dp = bars[15];         // dP^T of the tile is in tensor memory
+  uint64_t& bar_ds = bars[16];         // dS^T written
+  uint64_t& bar_g = bars[17];          // dQ of the tile is in tensor memory
+  uint64_t& bar_dqr = bars[18];        // dQ read out of tensor memory
+  uint64_t& bar_epi = bars[19];
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + Cfg::kBars);
+  volatile int* abort_ptr = reinterpret_cast<volatile int*>(reinterpret_cast<uint8_t*>(bars + Cfg::kBars) + 4);
   int* abort_w = const_cast<int*>(abort_ptr);
-  uint4* s_masks = reinterpret_cast<uint4*>(bars + 18);               // [2 stages][kMaskRuns] the pair's masks, by run of the key
+  uint4* s_masks = reinterpret_cast<uint4*>(bars + Cfg::kBars + 2);   // [Q stages][kMaskRuns] the pair's masks, by run of the key
   {  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
     int bad = 0;
     const int32_t* stw = p.plan.status;
@@ -298,18 +280,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   if (tid == 0) {
     *abort_ptr = 0;
     mbar_init(&bar_kv, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 3; ++i) {
       mbar_init(&bar_q_full[i], 1);
-      mbar_init(&bar_pds[i], TS2TS_BWD_ELECT ? 8 : 2 * kTile);  // one arrival per compute warp
+      mbar_init(&bar_gq[i], 1);
     }
-    mbar_init(&bar_do_full, 1);
-    mbar_init(&bar_gd, 1);
-    mbar_init(&bar_st, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_do_full[i], 1);
+      mbar_init(&bar_gv[i], 1);
+      mbar_init(&bar_s[i], 1);
+      mbar_init(&bar_p[i], 8);  // one arrival per compute warp
+    }
+    mbar_init(&bar_dp, 1);
+    mbar_init(&bar_ds, 8);
     mbar_init(&bar_g, 1);
-    mbar_init(&bar_dqr, kTile);
+    mbar_init(&bar_dqr, 4);  // one arrival per reduction warp
     mbar_init(&bar_epi, 2 * kTile);
-    mbar_init(&bar_s[0], 1);
-    mbar_init(&bar_s[1], 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -321,12 +306,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const uint32_t tDV = tmem + Cfg::kDV, tDK = tmem + Cfg::kDK, tST = tmem + Cfg::kST, tDPT = tmem + Cfg::kDPT;
-  // S^T columns [64s + 32h, +32) are read by the compute thread (row, h) in half s and overwritten by it with
-  // P^T bf16 [.., +16) and dS^T bf16 [.. + 16, +16) for its 32 queries.
+  const uint32_t tDV = tmem + Cfg::kDV, tDK = tmem + Cfg::kDK, tST = tmem + Cfg::kST, tDPT = tmem + Cfg::kDPT, tDQ = tDPT;
+  // S^T columns [32c, +32) of a buffer are read by the compute thread of (row, c / 2), which writes P^T bf16 over the first 16 of them.
 
   if (warp >= 12) {
-    reg_dec<88>();
+    if (D == 64) reg_dec<112>(); else reg_dec<88>();
     if (warp == 12 && lane == 0) {
       // ---------------------------------------------------------------- TMA producer
       tma_prefetch_desc(&mapQ); tma_prefetch_desc(&mapK); tma_prefetch_desc(&mapV); tma_prefetch_desc(&mapDO);
@@ -335,10 +319,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         tma_load_4d(sK + s * 16384, &mapK, &bar_kv, s * 64, kb * kTile, h, b);
         tma_load_4d(sV + s * 16384, &mapV, &bar_kv, s * 64, kb * kTile, h, b);
       }
-      auto load_q = [&](int i) {  // Q tile and row statistics of tile i into stage i & 1
+      auto load_q = [&](int i) {  // Q tile and row statistics of tile i into its stage
         const int entry = list[i];
         const int qb = min(entry & ~kFullBit, NB - 1);
-        const int st = i & 1;
+        const int st = i % Cfg::kQStages;
         const bool masks = !(entry & kFullBit) && P.kv_mask != nullptr;  // partial tile: its masks travel with the stage
         mbar_expect_tx(&bar_q_full[st], Cfg::kTileBytes + 2 * kTile * 4 + (masks ? kMaskRuns * 16 : 0));
         if (masks)
@@ -351,155 +335,148 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         bulk_load(s_delta[st], p.delta + stat, kTile * 4, &bar_q_full[st]);
       };
       auto load_do = [&](int i) {
-        const int qb = list[i] & ~kFullBit;
-        mbar_expect_tx(&bar_do_full, Cfg::kTileBytes);
-        for (int s = 0; s < Cfg::kSub; ++s) tma_load_4d(sDO + s * 16384, &mapDO, &bar_do_full, s * 64, qb * kTile, h, b);
+        const int qb = list[i] & ~kFullBit, st = i % Cfg::kDoStages;
+        mbar_expect_tx(&bar_do_full[st], Cfg::kTileBytes);
+        for (int s = 0; s < Cfg::kSub; ++s)
+          tma_load_4d(sDO + st * Cfg::kTileBytes + s * 16384, &mapDO, &bar_do_full[st], s * 64, qb * kTile, h, b);
       };
       load_q(0);
-      load_do(0);
-      if (n > 1) load_q(1);
+      for (int i = 0; i < Cfg::kDoStages && i < n; ++i) load_do(i);
+      for (int i = 1; i < Cfg::kQStages && i < n; ++i) load_q(i);
       for (int i = 0; i + 1 < n; ++i) {
-        if (!mbar_wait(&bar_gd, i & 1, abort_w, 11)) break;  // dV / dK MMAs of tile i done: dO and Q stage i & 1 are free
-        load_do(i + 1);
-        if (i + 2 < n) load_q(i + 2);
+        if (i + Cfg::kDoStages < n) {
+          if (!mbar_wait(&bar_gv[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1, abort_w, 11)) break;  // dP^T, dV MMAs of tile i done
+          load_do(i + Cfg::kDoStages);
+        }
+        if (i + Cfg::kQStages < n) {  // S^T, dK MMAs of tile i done, its statistics read
+          if (!mbar_wait(&bar_gq[i % Cfg::kQStages], (i / Cfg::kQStages) & 1, abort_w, 12)) break;
+          load_q(i + Cfg::kQStages);
+        }
       }
     } else if (warp == 13 && lane == 0) {
       // ---------------------------------------------------------------- MMA issuer
       constexpr uint32_t idesc_st = make_idesc_bf16(128, 128, false, false);  // K-major x K-major
-      constexpr uint32_t idesc_g = make_idesc_bf16(128, D, false, true);      // TMEM A x MN-major B, N = D
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, true, true);    // MN-major A x MN-major B
+      constexpr uint32_t idesc_g = make_idesc_bf16(128, D, false, true);      // TMEM or K-major A x MN-major B, N = D
+      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);      // MN-major A x MN-major B, N = D
       // Descriptor halves (see desc_lo / desc_hi): `hi` is shared by every operand (SBO = 1024); K-major operands
       // carry LBO 16, MN-major ones LBO 16384 (distance between the two 64-element halves of the MN extent).
       constexpr uint32_t hi = desc_hi(1024);
+      constexpr uint32_t kTileStep = Cfg::kTileBytes >> 4;
       const uint32_t k_kmaj = desc_lo(smem_u32(sK), 16), v_kmaj = desc_lo(smem_u32(sV), 16);
-      const uint32_t q_kmaj = desc_lo(smem_u32(sQ), 16), do_kmaj = desc_lo(smem_u32(sDO), 16);
+      const uint32_t q_kmaj = desc_lo(smem_u32(sQ), 16), do_kmaj = desc_lo(smem_u32(sDO), 16), ds_kmaj = desc_lo(smem_u32(sDS), 16);
       const uint32_t q_mn = desc_lo(smem_u32(sQ), 16384), do_mn = desc_lo(smem_u32(sDO), 16384);
       const uint32_t k_mn = desc_lo(smem_u32(sK), 16384), ds_mn = desc_lo(smem_u32(sDS), 16384);
+      auto kstep = [](int kk) -> uint32_t { return ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4; };  // 16 elements along a K-major operand
       // Shared-memory accesses of this thread (barrier waits included) queue behind the MMAs it has issued and only
-      // proceed once the tensor pipe has accepted those, so every wait whose barrier is normally complete already
-      // is placed one or two MMAs before the end of a group: the pipe stays fed while the wait runs.
-      auto issue_st = [&](uint32_t stage) {  // S^T = K Q^T, then tell the compute warps
+      // proceed once the tensor pipe has accepted those.  So every group asks, two MMAs before its end, whether what the
+      // next group waits for has arrived already (`early`): the pipe stays fed while the answer comes.
+      bool early_p = false, early_q = false, early_ds = false, early_do = false;
+      auto q_full = [&](int i) { return mbar_test_wait(&bar_q_full[i % Cfg::kQStages], (i / Cfg::kQStages) & 1); };
+      auto do_full = [&](int i) { return mbar_test_wait(&bar_do_full[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1); };
+      auto wait_q = [&](int i) { return early_q || mbar_wait(&bar_q_full[i % Cfg::kQStages], (i / Cfg::kQStages) & 1, abort_w, 22); };
+      auto wait_do = [&](int i) { return early_do || mbar_wait(&bar_do_full[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1, abort_w, 27); };
+      auto issue_st = [&](int i, auto ask) {  // S^T = K Q^T
+        const uint32_t q = q_kmaj + (i % Cfg::kQStages) * kTileStep, t = tST + (i % Cfg::kSBufs) * 128;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
-          mma_ss2(tST, k_kmaj + off, hi, q_kmaj + stage + off, hi, idesc_st, kk > 0);
+          if (kk == D / 16 - 2) ask();
+          mma_ss2(t, k_kmaj + kstep(kk), hi, q + kstep(kk), hi, idesc_st, kk > 0);
         }
-        mma_commit(&bar_s[0]);
-        mma_commit(&bar_s[1]);
+        mma_commit(&bar_s[i % Cfg::kSBufs]);
       };
-      constexpr uint32_t idesc_st64 = make_idesc_bf16(128, 64, false, false);
-      auto issue_st_half = [&](uint32_t stage, int hq) {  // S^T[:, 64 hq, +64) = K Q[64 hq, +64)^T  (N = 64)
-        const uint32_t rows = (uint32_t)hq * (kSubQ * 128) >> 4;  // 64 query rows x 128 B of the K-major Q tile
+      auto issue_dpt = [&](int i, auto ask) {  // dP^T = V dO^T
+        const uint32_t o = do_kmaj + (i % Cfg::kDoStages) * kTileStep;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
-          mma_ss2(tST + 64 * hq, k_kmaj + off, hi, q_kmaj + stage + rows + off, hi, idesc_st64, kk > 0);
+          if (kk == D / 16 - 2) ask();
+          mma_ss2(tDPT, v_kmaj + kstep(kk), hi, o + kstep(kk), hi, idesc_st, kk > 0);
         }
-        mma_commit(&bar_s[hq]);
+        mma_commit(&bar_dp);
       };
-      auto issue_dpt = [&]() {  // dP^T = V dO^T
+      auto issue_dq = [&](auto ask) {  // dQ = dS K
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
-          mma_ss2(tDPT, v_kmaj + off, hi, do_kmaj + off, hi, idesc_st, kk > 0);
+        for (int kk = 0; kk < kTile / 16; ++kk) {
+          if (kk == kTile / 16 - 2) ask();
+          mma_ss2(tDQ, ds_mn + kk * 128, hi, k_mn + kk * 128, hi, idesc_dq, kk > 0);
         }
-        mma_commit(&bar_st);
-      };
-      auto issue_dqt = [&]() {  // dQ^T = K^T dS^T   (K = 128 keys; M = D, padded to 128 lanes when D = 64)
-#pragma unroll
-        for (int kk = 0; kk < kTile / 16; ++kk) mma_ss2(tDPT, k_mn + kk * 128, hi, ds_mn + kk * 128, hi, idesc_dq, kk > 0);
         mma_commit(&bar_g);
       };
-      // Order per tile i: dV/dK(i) half 0, half 1 | S^T(i+1) | dQ^T(i) | (dQ^T(i) read out) dP^T(i+1).
-      // S^T of the next tile goes first so that the compute warps can do the exponentials of tile i+1 while the
-      // tensor core is busy with dQ^T(i), its read-out and dP^T(i+1).  S^T(i+1) overwrites the P^T / dS^T columns of
-      // tile i; their readers, the dV / dK MMAs of tile i, were issued before it by this thread and the tensor pipe
-      // executes one thread's MMAs in issue order.
-      bool ok = mbar_wait(&bar_kv, 0, abort_w, 21) && mbar_wait(&bar_q_full[0], 0, abort_w, 22);
+      auto issue_dk = [&](int i) {  // dK += dS^T Q
+        const uint32_t q = q_mn + (i % Cfg::kQStages) * kTileStep;
+#pragma unroll
+        for (int kk = 0; kk < kTile / 16; ++kk) mma_ss2(tDK, ds_kmaj + kstep(kk), hi, q + kk * 128, hi, idesc_g, (i > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(&bar_gq[i % Cfg::kQStages]);
+      };
+      auto issue_dv = [&](int i, auto ask) {  // dV += P^T dO
+        const uint32_t o = do_mn + (i % Cfg::kDoStages) * kTileStep, t = tST + (i % Cfg::kSBufs) * 128;
+#pragma unroll
+        for (int kk = 0; kk < kTile / 16; ++kk) {
+          if (kk == kTile / 16 - 2) ask();
+          mma_ts2(tDV, t + (kk >> 1) * 32 + (kk & 1) * 8, o + kk * 128, hi, idesc_g, (i > 0 || kk > 0) ? 1u : 0u);
+        }
+        mma_commit(&bar_gv[i % Cfg::kDoStages]);
+      };
+      auto nothing = []() {};
+      // Order per tile: dV(i), S^T(i+1) (the other way round where S^T has two buffers) | dK(i), dQ(i) | dP^T(i+1).
+      // dV and S^T run while the compute warps work on dS^T(i); dK, dQ and dP^T(i+1) while they work on the exponentials
+      // of tile i+1, so both sides always have a phase's worth of work in hand.  With one buffer S^T(i+1) overwrites the
+      // P^T columns of tile i: their readers, the dV MMAs, were issued before it by this thread and the tensor pipe
+      // executes one thread's MMAs in issue order.  dK before dQ: its Q stage is reloaded sooner, and at D = 128 the next
+      // but one tile's Q otherwise lands too late.
+      bool ok = mbar_wait(&bar_kv, 0, abort_w, 21) && wait_q(0);
       if (ok) {
         tc_fence_after();
-        issue_st(0u);
-        ok = mbar_wait(&bar_do_full, 0, abort_w, 27);
-        if (ok) issue_dpt();
+        issue_st(0, nothing);
+        ok = wait_do(0);
+        if (ok) issue_dpt(0, nothing);
       }
       for (int i = 0; i < n && ok; ++i) {
-        const int st = i & 1;
-        const uint32_t stage = ((uint32_t)st * Cfg::kTileBytes) >> 4;
-        const uint32_t next = ((uint32_t)(st ^ 1) * Cfg::kTileBytes) >> 4;
         const bool more = i + 1 < n;
-        bool fail = false;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          if (!mbar_wait(&bar_pds[s], i & 1, abort_w, 24)) { fail = true; break; }
+        TRACE(0, i, 0);
+        if (Cfg::kSBufs == 2 && more) {
+          if (!(ok = wait_q(i + 1))) break;
           tc_fence_after();
-          TRACE(0, i, 3 + s);
-          const uint32_t half_rows = (uint32_t)s * (kSubQ * 128) >> 4;  // 64 query rows x 128 B
-          const uint32_t acc = (i > 0 || s > 0) ? 1u : 0u;
-#pragma unroll
-          for (int kk = 0; kk < kSubQ / 16; ++kk)  // dV += P^T dO   (K = 64 queries of this half)
-            mma_ts2(tDV, tST + 64 * s + (kk >> 1) * 32 + (kk & 1) * 8, do_mn + half_rows + kk * 128, hi, idesc_g, kk > 0 ? 1u : acc);
-#pragma unroll
-          for (int kk = 0; kk < kSubQ / 16; ++kk)  // dK += dS^T Q
-            mma_ts2(tDK, tST + 64 * s + (kk >> 1) * 32 + 16 + (kk & 1) * 8, q_mn + stage + half_rows + kk * 128, hi, idesc_g, kk > 0 ? 1u : acc);
-#if TS2TS_BWD_SPLIT_ST && !defined(TS2TS_STRICT_ORDER)
-          if (s == 0 && more) {
-            // The first half of S^T(i+1) overwrites the P^T / dS^T columns of half 0 of tile i, whose readers were
-            // issued just above: it runs while the compute warps still work on half 1, so that their exponentials of
-            // tile i+1 can start the moment they are done with tile i.
-            if (!mbar_wait(&bar_q_full[st ^ 1], ((i + 1) >> 1) & 1, abort_w, 22)) { fail = true; break; }
-            tc_fence_after();
-            issue_st_half(next, 0);
-          }
-#endif
+          issue_st(i + 1, [&]() { early_p = mbar_test_wait(&bar_p[i & 1], (i >> 1) & 1); });
         }
-        if (fail) break;
-        mma_commit(&bar_gd);
-#ifdef TS2TS_STRICT_ORDER
-        issue_dqt();
-        TRACE(0, i, 5);
-        if (more) {
-          if (!mbar_wait(&bar_q_full[st ^ 1], ((i + 1) >> 1) & 1, abort_w, 22)) break;
-          if (!mbar_wait(&bar_g, i & 1, abort_w, 26)) break;  // every MMA of tile i complete before S^T(i+1) is issued
+        if (!(ok = early_p || mbar_wait(&bar_p[i & 1], (i >> 1) & 1, abort_w, 24))) break;
+        tc_fence_after();
+        TRACE(0, i, 1);
+        issue_dv(i, [&]() {
+          if (Cfg::kSBufs == 2) early_ds = mbar_test_wait(&bar_ds, i & 1);
+          else early_q = more && q_full(i + 1);
+        });
+        if (Cfg::kSBufs == 1 && more) {
+          if (!(ok = wait_q(i + 1))) break;
           tc_fence_after();
-          issue_st(next);
-        }
-#else
-#if TS2TS_BWD_SPLIT_ST && TS2TS_BWD_DQ_FIRST
-        issue_dqt();  // its read-out by the reduction warps then overlaps the second half of S^T(i+1)
-        TRACE(0, i, 5);
-#endif
-        if (more) {
-#if TS2TS_BWD_SPLIT_ST
-          issue_st_half(next, 1);
-#else
-          if (!mbar_wait(&bar_q_full[st ^ 1], ((i + 1) >> 1) & 1, abort_w, 22)) break;
-          tc_fence_after();
-          issue_st(next);
-#endif
-          TRACE(0, i, 0);
-        }
-#if !(TS2TS_BWD_SPLIT_ST && TS2TS_BWD_DQ_FIRST)
-        issue_dqt();
-        TRACE(0, i, 5);
-#endif
-#endif
-        if (more) {
-          if (!mbar_wait(&bar_dqr, i & 1, abort_w, 23)) break;  // dQ^T(i) read out of the columns dP^T(i+1) overwrites
-          if (!mbar_wait(&bar_do_full, (i + 1) & 1, abort_w, 27)) break;
-          tc_fence_after();
-          TRACE(0, i, 1);
-          issue_dpt();
           TRACE(0, i, 2);
+          issue_st(i + 1, [&]() { early_ds = mbar_test_wait(&bar_ds, i & 1); });
         }
+        TRACE(0, i, 3);
+        if (!(ok = early_ds || mbar_wait(&bar_ds, i & 1, abort_w, 28))) break;
+        tc_fence_after();
+        TRACE(0, i, 4);
+        issue_dk(i);
+        issue_dq([&]() { early_do = more && do_full(i + 1); });
+        TRACE(0, i, 5);
+        early_p = early_q = early_ds = false;
+        if (more) {
+          if (!(ok = wait_do(i + 1) && mbar_wait(&bar_dqr, i & 1, abort_w, 23))) break;  // dQ(i) read out of the columns dP^T(i+1) overwrites
+          tc_fence_after();
+          TRACE(0, i, 6);
+          issue_dpt(i + 1, [&]() {
+            if (Cfg::kSBufs == 2) early_q = i + 2 < n && q_full(i + 2);
+            else early_p = mbar_test_wait(&bar_p[(i + 1) & 1], ((i + 1) >> 1) & 1);
+          });
+        }
+        early_do = false;
+        TRACE(0, i, 7);
       }
     }
   } else if (warp < 8) {
     // ------------------------------------------------------------------ exp / dS warps: thread = (key row, 32 of 64 queries)
-#if TS2TS_BWD_LD2
-    // register pool: 256 x 128 (these warps keep the launch value) + 128 x 168 + 128 x 88 = 512 x 128
-#else
-    reg_dec<120>();
-#endif
+    // register pool: 256 x 128 (the launch value) + 128 x 168 + 128 x 88 = 512 x 128; at D = 64, where the reduction warps hold
+    // half as much, 256 x 120 + 128 x 136 + 128 x 112 (linked 16k 613 -> 600 us: no spills)
+    if (D == 64) reg_dec<120>();
     const int row = tid & (kTile - 1), half = tid >> 7;
     const int kv = kb * kTile + row;
     const bool kv_valid = kv < P.T;
@@ -513,113 +490,101 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
+    int e_next = ld_nc_i32_here(list);
     BTRACE_ACC_DECL
     for (int i = 0; i < n && ok; ++i) {
-      const int st = i & 1;
-      const int entry = list[i];
+      const int st = i % Cfg::kQStages;
+      const int entry = e_next;
+      if (i + 1 < n) e_next = ld_nc_i32_here(list + i + 1);
       const int qb = min(entry & ~kFullBit, NB - 1);
       const bool masked = (entry & kFullBit) == 0;
-      if (!(ok = mbar_wait(&bar_q_full[st], (i >> 1) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
-      uint32_t bits[4] = {0, 0, 0, 0};
-      if (masked) {
-        const uint4 m4 = run < kMaskRuns ? s_masks[st * kMaskRuns + run] : key_mask(P, p.mask, b, qb, kb, row);
-        bits[0] = m4.x; bits[1] = m4.y; bits[2] = m4.z; bits[3] = m4.w;
-        if (!kv_valid) bits[0] = bits[1] = bits[2] = bits[3] = 0u;
-        if (kb == qb) {  // causal inside the diagonal tile: query rows row..127
+      if (!(ok = mbar_wait(&bar_q_full[st], (i / Cfg::kQStages) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
+      // Full and partial tiles are separate code: the full one carries no mask state, so that its two phases fit the
+      // registers and the instruction cache (first phase 2080 -> 1500 clk a tile, causal 4k, D = 128).
+      auto tile = [&](auto masked_tag) {
+        constexpr bool kMasked = decltype(masked_tag)::value;
+        // per 32-query chunk of this thread, uniform over the warp: 0 all allowed, 1 test bits, 2 nothing allowed
+        int mode[2] = {0, 0};
+        uint32_t bw[2] = {0xffffffffu, 0xffffffffu};
+        if (kMasked) {
+          const uint4 m4 = run < kMaskRuns ? s_masks[st * kMaskRuns + run] : key_mask(P, p.mask, b, qb, kb, row);
+          bw[0] = half == 0 ? m4.x : m4.z;
+          bw[1] = half == 0 ? m4.y : m4.w;
 #pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const int lo = row - 32 * w;
-            bits[w] &= lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
+          for (int s = 0; s < 2; ++s) {
+            if (kb == qb) {  // causal inside the diagonal tile: query rows row..127
+              const int lo = row - 64 * half - 32 * s;
+              bw[s] &= lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
+            }
+            if (!kv_valid) bw[s] = 0u;
+            mode[s] = __all_sync(0xffffffffu, bw[s] == 0u) ? 2 : (__all_sync(0xffffffffu, bw[s] == 0xffffffffu) ? 0 : 1);
           }
         }
-      }
-      // per 32-query chunk of this thread, uniform over the warp: 0 all allowed, 1 test bits, 2 nothing allowed
-      int mode[2] = {0, 0};
-      uint32_t bw2[2] = {0xffffffffu, 0xffffffffu};
-      if (masked) {
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          bw2[s] = s == 0 ? (half == 0 ? bits[0] : bits[1]) : (half == 0 ? bits[2] : bits[3]);
-          mode[s] = __all_sync(0xffffffffu, bw2[s] == 0u) ? 2 : (__all_sync(0xffffffffu, bw2[s] == 0xffffffffu) ? 0 : 1);
-        }
-      }
-      if (masked) BTRACE_ACC(0); else BTRACE_ACC(1);
-      // ---- phase 1: exponentials, as soon as the half of S^T is complete
-      if (!(ok = mbar_wait(&bar_s[0], i & 1, abort_w, 35))) break;
-      tc_fence_after();
-      BTRACE_ACC(2);
-      if (tid == 0) TRACE(1, i, 0);
-      uint32_t pk[2][16];
-      {
-        uint32_t sv[2][32];
-#if TS2TS_BWD_LD2
-        tmem_ld32(tST + lane_base + 32 * half, sv[0]);
-        tmem_ld32(tST + lane_base + 64 + 32 * half, sv[1]);
-        tmem_ld_wait();
-#endif
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-#if !TS2TS_BWD_LD2
-          if (s == 1) {
-            if (!(ok = mbar_wait(&bar_s[1], i & 1, abort_w, 36))) break;
-            tc_fence_after();
-          }
-          tmem_ld32(tST + lane_base + 64 * s + 32 * half, sv[s]);
+        if (kMasked) BTRACE_ACC(0); else BTRACE_ACC(1);
+        // ---- phase 1: exponentials, as soon as S^T is complete, 32 columns at a time (the second load in
+        //      flight behind the first half's arithmetic takes registers that spill: 3960 -> 4120 clk a tile)
+        if (!mbar_wait(&bar_s[i % Cfg::kSBufs], (i / Cfg::kSBufs) & 1, abort_w, 35)) return false;
+        tc_fence_after();
+        BTRACE_ACC(2);
+        if ((tid & 127) == 0) TRACE(1 + half, i, 0);
+        const uint32_t tSc = tST + (i % Cfg::kSBufs) * 128 + lane_base + 64 * half;
+        uint32_t pk[2][16];
+        {
+          uint32_t s0[32], s1[32];
+          tmem_ld32(tSc, s0);
           tmem_ld_wait();
-#endif
-          p_chunk(sv[s], s_lse2[st] + s * kSubQ + 32 * half, bw2[s], mode[s], p.scale_log2, pk[s]);
-          tmem_st16(tST + lane_base + 64 * s + 32 * half, pk[s]);
-        }
-      }
-      if (!ok) break;
-      if (tid == 0) TRACE(1, i, 1);
-      BTRACE_ACC(3);
-      // ---- phase 2: dS^T, once dP^T is complete
-      if (!(ok = mbar_wait(&bar_st, i & 1, abort_w, 31))) break;
-      tc_fence_after();
-      BTRACE_ACC(4);
-      if (tid == 0) TRACE(1, i, 2);
-      {
-        uint32_t dp[2][32];
-#if TS2TS_BWD_LD2
-        tmem_ld32(tDPT + lane_base + 32 * half, dp[0]);
-        tmem_ld32(tDPT + lane_base + 64 + 32 * half, dp[1]);
-        tmem_ld_wait();
-#endif
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const uint32_t col = lane_base + 64 * s + 32 * half;
-#if !TS2TS_BWD_LD2
-          tmem_ld32(tDPT + col, dp[s]);
+          p_chunk<kMasked>(s0, s_lse2[st] + half * kSubQ, bw[0], mode[0], p.scale_log2, pk[0]);
+          tmem_st16(tSc, pk[0]);
+          tmem_ld32(tSc + 32, s1);
           tmem_ld_wait();
-#endif
-          uint32_t dsk[16];
-          ds_chunk(pk[s], dp[s], s_delta[st] + s * kSubQ + 32 * half, mode[s], dsk);
-          tmem_st16(tST + col + 16, dsk);
-          // dS^T row `row`, queries [64 s + 32 half, +32): four 16-byte chunks of the 128-byte row of half s
-          uint8_t* ds_row = sDS + s * 16384;
+          p_chunk<kMasked>(s1, s_lse2[st] + half * kSubQ + 32, bw[1], mode[1], p.scale_log2, pk[1]);
+          tmem_st16(tSc + 32, pk[1]);
+          tmem_st_wait();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_p[i & 1]);
+        if ((tid & 127) == 0) TRACE(1 + half, i, 1);
+        BTRACE_ACC(3);
+        // ---- phase 2: dS^T, once dP^T is complete.  dP^T(i) was issued after the MMAs that read dS^T(i-1), so its buffer
+        // is free as well.
+        if (!mbar_wait(&bar_dp, i & 1, abort_w, 31)) return false;
+        tc_fence_after();
+        BTRACE_ACC(4);
+        if ((tid & 127) == 0) TRACE(1 + half, i, 2);
+        {
+          const uint32_t tDc = tDPT + lane_base + 64 * half;
+          uint8_t* ds_row = sDS + half * 16384;  // row `row`: 64 queries, 128 bytes
+          uint32_t d0[32], d1[32], dsk[16];
+          tmem_ld32(tDc, d0);
+          tmem_ld_wait();
+          ds_chunk<kMasked>(pk[0], d0, s_delta[st] + half * kSubQ, mode[0], dsk);
 #pragma unroll
           for (int g = 0; g < 4; ++g)
-            *reinterpret_cast<uint4*>(ds_row + sw128_offset(row, 4 * half + g)) = make_uint4(dsk[g * 4 + 0], dsk[g * 4 + 1], dsk[g * 4 + 2], dsk[g * 4 + 3]);
-          tmem_st_wait();
-          fence_async_smem();
-          tc_fence_before();
-#if TS2TS_BWD_ELECT
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar_pds[s]);
-#else
-          mbar_arrive(&bar_pds[s]);
-#endif
-          if (tid == 0) TRACE(1, i, 3 + 4 * s);
+            *reinterpret_cast<uint4*>(ds_row + sw128_offset(row, g)) = make_uint4(dsk[g * 4 + 0], dsk[g * 4 + 1], dsk[g * 4 + 2], dsk[g * 4 + 3]);
+          tmem_ld32(tDc + 32, d1);
+          tmem_ld_wait();
+          ds_chunk<kMasked>(pk[1], d1, s_delta[st] + half * kSubQ + 32, mode[1], dsk);
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+            *reinterpret_cast<uint4*>(ds_row + sw128_offset(row, 4 + g)) = make_uint4(dsk[g * 4 + 0], dsk[g * 4 + 1], dsk[g * 4 + 2], dsk[g * 4 + 3]);
         }
-      }
+        fence_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_ds);
+        if ((tid & 127) == 0) TRACE(1 + half, i, 3);
+        return true;
+      };
+      ok = masked ? tile(std::true_type{}) : tile(std::false_type{});
+      if (!ok) break;
       BTRACE_ACC(5);
     }
     // ---- epilogue: dV (query-half 0 threads) and scale * dK (half 1) -> bf16 -> swizzled smem -> TMA stores.
-    //      dV goes through the Q stage the last tile did not use, dK through the dO buffer (its last readers, the
-    //      dV MMAs of the last tile, completed before bar_g).
-    const int est = n & 1;
-    if (ok) ok = mbar_wait(&bar_g, (n - 1) & 1, abort_w, 32);
+    //      dV goes through the Q stage the last tile did not use, dK through a dO buffer; what read
+    //      them, and the MMAs that add to dV and dK, completed before bar_gq.
+    const int est = n % Cfg::kQStages;
+    if (ok) ok = mbar_wait(&bar_gq[(n - 1) % Cfg::kQStages], ((n - 1) / Cfg::kQStages) & 1, abort_w, 32);
     tc_fence_after();
     uint8_t* out_dv = sQ + est * Cfg::kTileBytes;
     uint8_t* out_dk = sDO;
@@ -657,52 +622,52 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     BTRACE_ACC(6);
     if ((tid & 127) == 0) BTRACE_ACC_DUMP();
   } else {
-    // ------------------------------------------------------------------ dQ reduction warps 8-11, thread = head-dim lane
-    reg_inc<168>();
-    const int dlane = tid - 2 * kTile;  // 0..127 = TMEM lane = index into D
-    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    // Each warp owns the 32 head-dim lanes d/32 of the dQ tile and two private 128-byte-swizzled fp32 boxes of
-    // [32 queries x 32 floats] in shared memory.  The tile leaves in four rounds of 32 queries: store a round into
-    // one box, hand it to a TMA reduce-add, and store the next round into the other box while the first is read.
-    // Nothing else in the CTA waits for these reads.
-    const int box = dlane >> 5, chunk = (dlane & 31) >> 2, word = dlane & 3;
-    const bool has_box = box * 32 < D;
-    uint8_t* my_stage = sStage + (warp & 3) * 8192;
-    bool ok = true;
+    // ------------------------------------------------------------------ dQ reduction warps 8-11, thread = query row
+    if (D == 64) reg_inc<136>(); else reg_inc<168>();
+    const int w = warp & 3;
+    // Each warp owns 32 queries of the dQ tile and two private 4 KB boxes in shared memory.  The rows leave in rounds of 32
+    // head dimensions: store a round into one box, hand it to a bulk reduce-add, and store the next round into the other
+    // box while the first is read.  Nothing else in the CTA waits for these reads.  The accumulator is laid out
+    // [tile][query / 32][d / 4][query % 32][d % 4]: a thread stores four head dimensions of its query in 16 bytes without
+    // bank conflicts, and a round is 4 KB in one piece there as well as here.  Straight from the registers, as 16-byte
+    // reductions of 512 consecutive bytes a warp, the whole backward was 7 to 10 % slower.
+    const uint32_t tDQr = tDQ + (static_cast<uint32_t>(w * 32) << 16);
+    uint8_t* my_stage = sStage + w * 8192;
+    float* acc = p.dq_acc + ((size_t)b * p.H + h) * p.Tp * D + w * (32 * D);
     for (int i = 0; i < n; ++i) {
-      const int qb = list[i] & ~kFullBit;
-      if (!(ok = mbar_wait(&bar_g, i & 1, abort_w, 41))) break;
+      const int qb = min(list[i] & ~kFullBit, NB - 1);
+      if (!mbar_wait(&bar_g, i & 1, abort_w, 41)) break;
       tc_fence_after();
-      if (tid == 2 * kTile) TRACE(2, i, 0);
-      uint32_t r[2][64];
-      tmem_ld64(tDPT + lane_base, r[0]);
-      tmem_ld64(tDPT + lane_base + 64, r[1]);
+      if (tid == 2 * kTile) TRACE(1, i, 4);
+      uint32_t r[D / 64][64];
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) tmem_ld64(tDQr + 64 * c, r[c]);
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(&bar_dqr);  // the dP^T / dQ^T columns may be overwritten once all four warps have arrived
-      if (tid == 2 * kTile) TRACE(2, i, 1);
-      if (!has_box) continue;
-      if (tid == 2 * kTile) TRACE(2, i, 3);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_dqr);  // the dQ columns may be overwritten once all four warps have arrived
+      if (tid == 2 * kTile) TRACE(1, i, 5);
+      float* dst = acc + (size_t)qb * kTile * D;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < D / 32; ++k) {
         uint8_t* buf = my_stage + (k & 1) * 4096;
         // the box was last used two rounds ago: at most the previous round may still be reading
         if (lane == 0) tma_store_wait_read1();
         __syncwarp();
-        uint8_t* base = buf + word * 4;
+        const uint32_t* v = &r[k >> 1][32 * (k & 1)];
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-          *reinterpret_cast<float*>(base + c * 128 + ((chunk ^ (c & 7)) << 4)) = __uint_as_float(r[k >> 1][32 * (k & 1) + c]) * p.scale;
+        for (int g = 0; g < 8; ++g)
+          *reinterpret_cast<uint4*>(buf + g * 512 + lane * 16) = make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
         fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_reduce_add_4d(&mapDQ, buf, box * 32, qb * kTile + 32 * k, h, b);
+          bulk_reduce_add_f32(dst + k * 1024, buf, 4096);
           tma_store_commit();
         }
       }
-      if (tid == 2 * kTile) TRACE(2, i, 4);
+      if (tid == 2 * kTile) TRACE(1, i, 6);
     }
-    if (lane == 0 && has_box) tma_store_wait_all();
+    if (lane == 0) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -763,23 +728,29 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
   }
 }
 
+// The dQ accumulator [B,H,Tp/32][d / 4][query % 32][d % 4] (fp32, sums of dS K) -> bf16 dq.  A block takes 32 queries of
+// one (b, h): four head dimensions of a query are scaled, turned in shared memory and leave as whole rows.
 template <int D>
-__global__ void __launch_bounds__(256) dq_convert_kernel(const float* acc, __nv_bfloat16* dq, int64_t sb, int64_t sh, int64_t st,
-                                                         int B, int H, int T, int Tp) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // one thread per 8 elements
-  constexpr int kPerRow = D / 8;
-  const int64_t total = (int64_t)B * H * T * kPerRow;
-  if (idx >= total) return;
-  const int c = (int)(idx % kPerRow);
-  const int64_t rt = idx / kPerRow;
-  const int t = (int)(rt % T);
-  const int64_t bh = rt / T;
-  const int h = (int)(bh % H), b = (int)(bh / H);
-  const float4* src = reinterpret_cast<const float4*>(acc + ((bh * Tp + t) * D + c * 8));
-  const float4 a = src[0], e = src[1];
-  uint4 v;
-  v.x = pack_bf16(a.x, a.y); v.y = pack_bf16(a.z, a.w); v.z = pack_bf16(e.x, e.y); v.w = pack_bf16(e.z, e.w);
-  *reinterpret_cast<uint4*>(dq + b * sb + h * sh + (int64_t)t * st + c * 8) = v;
+__global__ void __launch_bounds__(256) dq_convert_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int64_t sb, int64_t sh,
+                                                         int64_t st, int H, int T, int Tp, float scale) {
+  __shared__ __align__(16) __nv_bfloat16 s_row[32][D + 8];
+  const int per_bh = Tp / 32;
+  const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * 32;
+  const float4* src = acc + (size_t)blockIdx.x * (8 * D);
+  float4 v[D / 32];
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i) v[i] = src[i * 256 + threadIdx.x];
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i)
+    *reinterpret_cast<uint2*>(&s_row[threadIdx.x % 32][(i * 8 + threadIdx.x / 32) * 4]) =
+        make_uint2(pack_bf16(v[i].x * scale, v[i].y * scale), pack_bf16(v[i].z * scale, v[i].w * scale));
+  __syncthreads();
+  const int h = bh % H, b = bh / H;
+#pragma unroll
+  for (int i = 0; i < D / 64; ++i) {
+    const int e = threadIdx.x + i * 256, r = e / (D / 8), c = e % (D / 8);
+    if (t0 + r < T) *reinterpret_cast<uint4*>(dq + b * sb + h * sh + (int64_t)(t0 + r) * st + c * 8) = *reinterpret_cast<const uint4*>(&s_row[r][c * 8]);
+  }
 }
 
 size_t bwd_workspace_bytes(int B, int H, int T, int D) {
@@ -799,7 +770,7 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   float* lse2 = reinterpret_cast<float*>(ws);
   float* delta = reinterpret_cast<float*>(ws + plan_align(rows * 4));
   float* dq_acc = reinterpret_cast<float*>(ws + 2 * plan_align(rows * 4));
-  CUtensorMap mq, mk, mv, mdo, mdk, mdv, mdq;
+  CUtensorMap mq, mk, mv, mdo, mdk, mdv;
   int r;
   if ((r = cached_tile_map(&mq, q, 2, B, H, T, D, sq[0], sq[1], sq[2], kTile, 64))) return r;
   if ((r = cached_tile_map(&mk, k, 2, B, H, T, D, sk[0], sk[1], sk[2], kTile, 64))) return r;
@@ -807,7 +778,6 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   if ((r = cached_tile_map(&mdo, dout, 2, B, H, T, D, sdo[0], sdo[1], sdo[2], kTile, 64))) return r;
   if ((r = cached_tile_map(&mdk, dk, 2, B, H, T, D, sdk[0], sdk[1], sdk[2], kTile, 64))) return r;
   if ((r = cached_tile_map(&mdv, dv, 2, B, H, T, D, sdv[0], sdv[1], sdv[2], kTile, 64))) return r;
-  if ((r = cached_tile_map(&mdq, dq_acc, 4, B, H, Tp, D, (int64_t)H * Tp * D, (int64_t)Tp * D, D, 32, 32))) return r;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -834,11 +804,10 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   BTRACE_ATTACH(p, stream);
   {
     ProfileScope timed(1, stream);
-    attn_bwd_kernel<D><<<(unsigned)B * H * P.NB, kBwdThreads, BwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mdo, mdk, mdv, mdq, p);
+    attn_bwd_kernel<D><<<(unsigned)B * H * P.NB, kBwdThreads, BwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mdo, mdk, mdv, p);
   }
-  const int64_t n8 = (int64_t)B * H * T * (D / 8);
-  dq_convert_kernel<D><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), sdq[0], sdq[1],
-                                                                         sdq[2], B, H, T, Tp);
+  dq_convert_kernel<D><<<(unsigned)(rows / 32), 256, 0, stream>>>(reinterpret_cast<const float4*>(dq_acc), static_cast<__nv_bfloat16*>(dq),
+                                                                 sdq[0], sdq[1], sdq[2], H, T, Tp, scale);
   BTRACE_DUMP(stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -121;
 }

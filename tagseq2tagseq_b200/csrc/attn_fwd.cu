@@ -14,16 +14,20 @@
 //             once, so that the issuer can compute S of the NEXT key tile while this one is being exponentiated;
 //             mask (partial tiles only: one select per element against a per-row 128-bit column mask that the pre-pass
 //             worked out; 32-column chunks that are masked for a whole warp are skipped), online softmax in
-//             base 2, P -> bf16 -> shared memory (K-major, 128-byte swizzle)
-//   tcgen05   O += P V                        (both operands from shared memory, V MN-major)
+//             base 2, P -> bf16 -> tensor memory (D = 64) or shared memory (D = 128; K-major, 128-byte swizzle)
+//   tcgen05   O += P V                        (V MN-major; with P in tensor memory the first 64 keys as soon as theirs is there)
+// P needs a place other than the scores it is made from, or S of the next tile could not be computed meanwhile.  At D = 64
+// tensor memory has room for it (S0 | S1 | O0 | O1 | P0 | P1), which takes 128 KB a pair of tiles out of the shared-memory
+// pipe that the MMA operands fill (H = 16, causal 4k batch 4: 239 -> 222 us, linked 16k: 370 -> 348).  At D = 128 it has not: with P
+// over its own scores a team waited 1570 clocks a tile for S where it waits 240 (causal 4k).
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
 // K/V tiles travel through one ring of shared-memory slots in the order K0, K1, V0, K2, V1, ... (K runs one tile
 // ahead of V because S is computed one tile ahead of P V).  At the end of an item each softmax thread reads its
-// row of O out of tensor memory, frees it for the next item and writes the normalised row straight to global
-// memory, while the issuers already work on the next item.
+// row of O out of tensor memory and frees it for the next item; the normalised rows leave through shared memory and TMA stores
+// while the issuers already work on the next item.
 //
-// Tensor memory: S0 | S1 | O0 | O1 = 512 columns.  Shared memory at D = 128: Q0 Q1 (64 KB), P0 P1 (64 KB),
-// three K/V slots (96 KB).
+// Shared memory at D = 128: Q0 Q1 (64 KB), P0 P1 (64 KB), three K/V slots (96 KB); at D = 64: Q0 Q1 (32 KB), O0 O1 (32 KB),
+// eight slots (128 KB).
 //
 // Computes what the reference obtains from PyTorch FlexAttention's forward
 // (model/modules/layer.py:33 via tunalab FlexSelfAttention; semantics in
@@ -98,13 +102,14 @@ template <int D>
 struct FwdSmem {
   static constexpr int kSub = D / 64;
   static constexpr int kTileBytes = kTile * D * 2;
-  static constexpr int kPBytes = kTile * kTile * 2;
-  static constexpr int kStages = D == 128 ? 3 : 6;
+  static constexpr bool kTmemP = D == 64;                    // P in tensor memory
+  static constexpr int kPBytes = kTmemP ? kTileBytes : kTile * kTile * 2;  // output rows always leave through it
+  static constexpr int kStages = D == 128 ? 3 : 8;
   static constexpr int kQ = 0;                               // two Q tiles
-  static constexpr int kP = 2 * kTileBytes;                  // two P tiles
+  static constexpr int kP = 2 * kTileBytes;                  // two P (or O) tiles
   static constexpr int kRing = kP + 2 * kPBytes;             // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
-  static constexpr int kBars = 18 + 2 * kStages;
+  static constexpr int kBars = 20 + 2 * kStages;
   static constexpr int kSmallBytes = kBars * 8 + 16 + 4 * kStages;  // barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
 };
@@ -228,11 +233,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint64_t* bar_q_free = bars + 6;       // [team] last S of the item complete: the Q buffer may be reloaded
   uint64_t* bar_s = bars + 8;            // [team] S of the tile is in tensor memory
   uint64_t* bar_sfree = bars + 10;       // [team] S read into registers: its columns may be overwritten
-  uint64_t* bar_p = bars + 12;           // [team] P of the tile is in shared memory
-  uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P buffer free, O consistent
+  uint64_t* bar_p = bars + 12;           // [team] P of the tile (D = 64: of its last 64 keys) is written
+  uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P free, O consistent
   uint64_t* bar_ofree = bars + 16;       // [team] O of the item read out of tensor memory
-  uint64_t* bar_ring_full = bars + 18;   // [kStages] K or V tile landed in the slot
-  uint64_t* bar_ring_free = bars + 18 + kStages;  // [kStages] both issuers are done with the slot
+  uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled (D = 64)
+  uint64_t* bar_ring_full = bars + 20;   // [kStages] K or V tile landed in the slot
+  uint64_t* bar_ring_free = bars + 20 + kStages;  // [kStages] both issuers are done with the slot
   int* s_item = reinterpret_cast<int*>(bars + Cfg::kBars);  // [2] ticket ring
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
   int* abort_w = s_item + 3;
@@ -261,6 +267,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       mbar_init(&bar_s[i], 1);
       mbar_init(&bar_sfree[i], 4);  // one arrival per softmax warp
       mbar_init(&bar_p[i], 4);
+      mbar_init(&bar_p0[i], 4);
       mbar_init(&bar_pv[i], 1);
       mbar_init(&bar_ofree[i], 4);
     }
@@ -358,6 +365,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const uint32_t k_ring_lo = desc_lo(smem_u32(sRing), 16), v_ring_lo = desc_lo(smem_u32(sRing), 16384);
       const uint32_t tS = tmem + t * kTile;
       const uint32_t tO = tmem + 2 * kTile + t * D;
+      const uint32_t tP = tmem + 2 * kTile + 2 * D + t * 64;  // kTmemP
       const uint32_t mine_bit = kRingTeam0 << t, first_bit = kRingFirst0 << t, last_bit = kRingLast0 << t;
       uint32_t n_s = 0;      // S tiles issued by this team so far
       uint32_t n_pv = 0;     // P V tiles issued so far
@@ -389,7 +397,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           if (info & last_bit) mma_commit(&bar_q_free[t]);
           mma_commit(&bar_ring_free[slot]);
         } else {
-          if (!mbar_wait(&bar_p[t], n_pv & 1, abort_v, 26)) break;
+          if (!mbar_wait(Cfg::kTmemP ? &bar_p0[t] : &bar_p[t], n_pv & 1, abort_v, 26)) break;
           // the first P V of an item overwrites O: the previous item's rows must have been read out
           // (n_items counts this item already, so the previous one is n_items - 2)
           if ((info & first_bit) && n_items > 1 && !mbar_wait(&bar_ofree[t], (n_items - 2) & 1, abort_v, 27)) break;
@@ -397,10 +405,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           FTRACE(2 * t, n_pv, 2);
           const uint32_t v_lo = v_ring_lo + slot * (Cfg::kTileBytes >> 4);
           const uint32_t acc0 = (info & first_bit) ? 0u : 1u;
+          if constexpr (Cfg::kTmemP) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk) {
-            const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
-            mma_ss2(tO, p_lo + off, hi_k, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
+            for (int kk = 0; kk < 4; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
+            if (!mbar_wait(&bar_p[t], n_pv & 1, abort_v, 28)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 4; kk < kTile / 16; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, 1u);
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < kTile / 16; ++kk) {
+              const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+              mma_ss2(tO, p_lo + off, hi_k, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
+            }
           }
           mma_commit(&bar_pv[t]);
           FTRACE(2 * t, n_pv, 3);
@@ -419,6 +436,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tSr = tmem + t * kTile + lane_base;
     const uint32_t tOr = tmem + 2 * kTile + t * D + lane_base;
+    const uint32_t tPr = tmem + 2 * kTile + 2 * D + t * 64 + lane_base;  // kTmemP
     uint8_t* sPt = sP + t * Cfg::kPBytes;
     uint32_t n_tiles = 0;  // tiles this team has processed so far
     uint32_t n_epi = 0;    // items this team has finished
@@ -558,7 +576,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const float m_safe = m_used == -CUDART_INF_F ? 0.f : m_used;
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 3);
         // sweep 2: P = exp2(s * scale - m) with packed fp32 arithmetic (two scores per instruction), row sum in
-        // four partial sums, bf16 pack, P -> shared memory
+        // four partial sums, bf16 pack, P to its place
         const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2), negm2 = pack_f32x2(-m_safe, -m_safe);
         unsigned long long sum2[2] = {0ull, 0ull};
         float sum4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -586,11 +604,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             for (int i = 0; i < 16; ++i) pk[c][i] = 0u;
           }
           if (c == 1) {
-            // P V of the previous tile must be complete before its P buffer is overwritten and before O is touched;
+            // P V of the previous tile must be complete before its P is overwritten and before O is touched;
             // it was issued a whole sweep ago, so this wait normally falls through.
             if (row == 0) FTRACE(2 * t + 1, n_tiles, 4);
             if (n_tiles > 0) fine = mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 33);
-            if (j == 0 && n_epi > 0) {
+            if (!Cfg::kTmemP && j == 0 && n_epi > 0) {
               // the previous item's output left through this buffer: its TMA store must have read it
               if (row == 0) tma_store_wait_read0();
               team_sync(t);
@@ -616,7 +634,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
               tmem_st_wait();
             }
           }
-          if (c >= 1) {
+          if constexpr (Cfg::kTmemP) {
+            if (c == 1) tmem_st16(tPr, pk[0]);
+            if (c >= 1) tmem_st16(tPr + 16 * c, pk[c]);
+            if (c == 1) {
+              tmem_st_wait();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0 && fine) mbar_arrive(&bar_p0[t]);
+            }
+          } else if (c >= 1) {
 #pragma unroll
             for (int cc = (c == 1 ? 0 : c); cc <= c; ++cc)
 #pragma unroll
@@ -633,7 +660,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           l += (s0 + s1) + (s2 + s3) + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
         }
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 6);
-        fence_async_smem();
+        if constexpr (Cfg::kTmemP) tmem_st_wait();
+        else fence_async_smem();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_p[t]);
@@ -651,6 +679,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       if (!ok) break;
       // ---- epilogue: O / l -> bf16 -> the team's P buffer (free after the last P V) -> TMA store
       if (!(ok = mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 34))) break;
+      if (Cfg::kTmemP && n_epi > 0) {  // the buffer's last store must have read it
+        if (row == 0) tma_store_wait_read0();
+        team_sync(t);
+      }
       tc_fence_after();
       {
         const float inv = l > 0.f ? 1.f / l : 0.f;

@@ -208,7 +208,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   // compiler, so every access below becomes a shared-memory instruction instead of a generic one.
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sK = smem;
-  uint8_t* sV = smem + Cfg::kTileBytes;           // must follow sK directly (dQ^T operand padding for D = 64)
+  uint8_t* sV = smem + Cfg::kTileBytes;
   uint8_t* sQ = smem + 2 * Cfg::kTileBytes;       // Cfg::kQStages stages
   uint8_t* sDO = sQ + Cfg::kQStages * Cfg::kTileBytes;  // Cfg::kDoStages buffers
   uint8_t* sDS = sDO + Cfg::kDoStages * Cfg::kTileBytes;  // dS^T, halves of 16 KB

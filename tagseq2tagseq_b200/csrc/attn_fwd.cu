@@ -613,9 +613,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
               if (row == 0) tma_store_wait_read0();
               team_sync(t);
             }
+            tc_fence_after();  // P and O, both read or written by that product, are overwritten below
             if (row == 0) FTRACE(2 * t + 1, n_tiles, 5);
             if (any_need && j > 0) {
-              tc_fence_after();
               const unsigned long long f2 = pack_f32x2(factor, factor);
 #pragma unroll 1
               for (int cc = 0; cc < D / 32; ++cc) {

@@ -498,7 +498,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       if (i + 1 < n) e_next = ld_nc_i32_here(list + i + 1);
       const int qb = min(entry & ~kFullBit, NB - 1);
       const bool masked = (entry & kFullBit) == 0;
-      if (!(ok = mbar_wait(&bar_q_full[st], (i / Cfg::kQStages) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
+      if (!(ok = mbar_wait_warp(&bar_q_full[st], (i / Cfg::kQStages) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
       // Full and partial tiles are separate code: the full one carries no mask state, so that its two phases fit the
       // registers and the instruction cache (first phase 2080 -> 1500 clk a tile, causal 4k, D = 128).
       auto tile = [&](auto masked_tag) {
@@ -523,7 +523,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (kMasked) BTRACE_ACC(0); else BTRACE_ACC(1);
         // ---- phase 1: exponentials, as soon as S^T is complete, 32 columns at a time (the second load in
         //      flight behind the first half's arithmetic takes registers that spill: 3960 -> 4120 clk a tile)
-        if (!mbar_wait(&bar_s[i % Cfg::kSBufs], (i / Cfg::kSBufs) & 1, abort_w, 35)) return false;
+        if (!mbar_wait_warp(&bar_s[i % Cfg::kSBufs], (i / Cfg::kSBufs) & 1, abort_w, 35)) return false;
         tc_fence_after();
         BTRACE_ACC(2);
         if ((tid & 127) == 0) TRACE(1 + half, i, 0);
@@ -548,7 +548,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         BTRACE_ACC(3);
         // ---- phase 2: dS^T, once dP^T is complete.  dP^T(i) was issued after the MMAs that read dS^T(i-1), so its buffer
         // is free as well.
-        if (!mbar_wait(&bar_dp, i & 1, abort_w, 31)) return false;
+        if (!mbar_wait_warp(&bar_dp, i & 1, abort_w, 31)) return false;
         tc_fence_after();
         BTRACE_ACC(4);
         if ((tid & 127) == 0) TRACE(1 + half, i, 2);
@@ -584,7 +584,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     //      dV goes through the Q stage the last tile did not use, dK through a dO buffer; what read
     //      them, and the MMAs that add to dV and dK, completed before bar_gq.
     const int est = n % Cfg::kQStages;
-    if (ok) ok = mbar_wait(&bar_gq[(n - 1) % Cfg::kQStages], ((n - 1) / Cfg::kQStages) & 1, abort_w, 32);
+    if (ok) ok = mbar_wait_warp(&bar_gq[(n - 1) % Cfg::kQStages], ((n - 1) / Cfg::kQStages) & 1, abort_w, 32);
     tc_fence_after();
     uint8_t* out_dv = sQ + est * Cfg::kTileBytes;
     uint8_t* out_dk = sDO;
@@ -636,7 +636,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     float* acc = p.dq_acc + ((size_t)b * p.H + h) * p.Tp * D + w * (32 * D);
     for (int i = 0; i < n; ++i) {
       const int qb = min(list[i] & ~kFullBit, NB - 1);
-      if (!mbar_wait(&bar_g, i & 1, abort_w, 41)) break;
+      if (!mbar_wait_warp(&bar_g, i & 1, abort_w, 41)) break;
       tc_fence_after();
       if (tid == 2 * kTile) TRACE(1, i, 4);
       uint32_t r[D / 64][64];

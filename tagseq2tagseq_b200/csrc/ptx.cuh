@@ -69,6 +69,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same wait by all 32 lanes of a warp, with one answer for all: lanes poll for themselves, so when the abort word is set
+// just as the phase completes some would go on and some leave, and the votes, __syncwarp and tensor-memory instructions
+// that follow a wait need the whole warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_word, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word, code));
+}
+
 // ----------------------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writes -> async proxy (TMA, tcgen05)
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

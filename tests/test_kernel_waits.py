@@ -42,3 +42,14 @@ def _unfenced(text):
 @pytest.mark.parametrize("name", ["attn_fwd.cu", "attn_bwd.cu"])
 def test_tensor_memory_is_touched_behind_a_fence_after_a_wait_for_mmas(name):
     assert _unfenced(_source(name)) == []
+
+
+@pytest.mark.parametrize("name,role", [("attn_fwd.cu", "softmax + epilogue"), ("attn_bwd.cu", "exp / dS warps"), ("attn_bwd.cu", "dQ reduction warps")])
+def test_warps_whose_lanes_all_wait_get_one_answer(name, role):
+    """In roles of whole warps a wait that only some lanes pass would leave the rest missing from the next vote, __syncwarp or
+    tensor-memory instruction: a lane's own answer is for a wait that one thread makes alone, or is not looked at."""
+    body = re.search(r"// -{20,} %s(.*?)(?=// -{20}|__syncthreads\(\))" % re.escape(role), _source(name), re.S).group(1)
+    own = re.findall(r"^.*\b(?:mbar_wait|wait_longer)\(.*$", body, re.M)
+    unasked = r"\s*(?:if \(n_tiles > 0\) mbar_wait|if \(!mbar_try_wait\(.*?\)\) wait_longer)\([^;]*;\s*"
+    voted = r".*(?:tid == 0 && |__all_sync\(0xffffffffu, mbar_wait\().*"
+    assert "mbar_wait_warp(" in body and [line.strip() for line in own if not re.fullmatch(unasked + "|" + voted, line)] == []

@@ -92,14 +92,8 @@ constexpr float kRescaleThreshold = 8.0f;
 #ifndef TS2TS_FWD_DUAL
 #define TS2TS_FWD_DUAL 1
 #endif
-// Barrier among the 128 threads of softmax team t (hardware barrier 1 + t; barrier 0 is __syncthreads).
-__device__ __forceinline__ void team_sync(int t) {
-  if (t == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-  else asm volatile("bar.sync 2, 128;" ::: "memory");
-}
-
-// A wait that is not asked how it ended.  Only its first poll is inline: with the loop of S's wait inside the tile's code, and no
-// exit from it, full tiles took 2 % longer (causal 4k batch 4, D = 64: 226 instead of 220 us).
+// A wait that is not asked how it ended.  Only its first poll is inline: with the loops inside the tile's code, and no exit from
+// them, full tiles took 2 % longer (causal 4k batch 4, D = 64: 226 instead of 220 us).
 __device__ __noinline__ void wait_longer(uint64_t* bar, uint32_t parity, volatile int* abort_word, int code) {
   mbar_wait(bar, parity, abort_word, code);
 }
@@ -115,7 +109,7 @@ struct FwdSmem {
   static constexpr int kP = 2 * kTileBytes;                  // two P (or O) tiles
   static constexpr int kRing = kP + 2 * kPBytes;             // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
-  static constexpr int kBars = 20 + 2 * kStages;
+  static constexpr int kBars = 24 + 2 * kStages;
   static constexpr int kSmallBytes = kBars * 8 + 16 + 4 * kStages;  // barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
 };
@@ -243,8 +237,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P free, O consistent
   uint64_t* bar_ofree = bars + 16;       // [team] O of the item read out of tensor memory
   uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled (D = 64)
-  uint64_t* bar_ring_full = bars + 20;   // [kStages] K or V tile landed in the slot
-  uint64_t* bar_ring_free = bars + 20 + kStages;  // [kStages] both issuers are done with the slot
+  uint64_t* bar_orows = bars + 20;       // [team] the item's output rows are in the team's buffer
+  uint64_t* bar_obuf = bars + 22;        // [team] the TMA store of those rows has read the buffer
+  uint64_t* bar_ring_full = bars + 24;   // [kStages] K or V tile landed in the slot
+  uint64_t* bar_ring_free = bars + 24 + kStages;  // [kStages] both issuers are done with the slot
   int* s_item = reinterpret_cast<int*>(bars + Cfg::kBars);  // [2] ticket ring
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
   int* abort_w = s_item + 3;
@@ -276,6 +272,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       mbar_init(&bar_p0[i], 4);
       mbar_init(&bar_pv[i], 1);
       mbar_init(&bar_ofree[i], 4);
+      mbar_init(&bar_orows[i], 4);
+      mbar_init(&bar_obuf[i], 1);
     }
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&bar_ring_full[i], 1);
@@ -500,6 +498,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       prefetch_mask(e_cur);
       float m_used = -CUDART_INF_F, l = 0.f;
       FTRACE_ACC(0);
+      // The store of the team's last rows must have read its buffer before the item writes there.  The warps of a team never meet in
+      // a named barrier: one that has left, because a wait ran out, would hold the others up for good.
+      if (n_epi > 0) {
+        if (row == 0) {
+          tma_store_wait_read0();
+          mbar_arrive(&bar_obuf[t]);
+        }
+        if (!mbar_try_wait(&bar_obuf[t], (n_epi - 1) & 1)) wait_longer(&bar_obuf[t], (n_epi - 1) & 1, abort_v, 36);
+      }
       for (int j = 0; j < n && ok; ++j) {
         const int entry = e_cur;
         e_cur = e_nxt;
@@ -615,12 +622,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // P V of the previous tile must be complete before its P is overwritten and before O is touched;
             // it was issued a whole sweep ago, so this wait normally falls through.
             if (row == 0) FTRACE(2 * t + 1, n_tiles, 4);
-            if (n_tiles > 0) mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 33);
-            if (!Cfg::kTmemP && j == 0 && n_epi > 0) {
-              // the previous item's output left through this buffer: its TMA store must have read it
-              if (row == 0) tma_store_wait_read0();
-              team_sync(t);
-            }
+            if (n_tiles > 0 && !mbar_try_wait(&bar_pv[t], (n_tiles - 1) & 1)) wait_longer(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 33);
             tc_fence_after();  // P and O, both read or written by that product, are overwritten below
             if (row == 0) FTRACE(2 * t + 1, n_tiles, 5);
             if (any_need && j > 0) {
@@ -683,12 +685,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         ++n_tiles;
       }
       if (!ok) break;
-      // ---- epilogue: O / l -> bf16 -> the team's P buffer (free after the last P V) -> TMA store
+      // ---- epilogue: O / l -> bf16 -> the team's buffer (at D = 128 P's, free after the last P V) -> TMA store
       if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 34) && *abort_v == 0))) break;
-      if (Cfg::kTmemP && n_epi > 0) {  // the buffer's last store must have read it
-        if (row == 0) tma_store_wait_read0();
-        team_sync(t);
-      }
       tc_fence_after();
       {
         const float inv = l > 0.f ? 1.f / l : 0.f;
@@ -714,8 +712,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (q_valid) p.lse[((size_t)b * p.H + h) * P.T + q] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -CUDART_INF_F;
       }
       fence_async_smem();
-      team_sync(t);
-      if (row == 0) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_orows[t]);
+      if (row == 0 && mbar_wait(&bar_orows[t], n_epi & 1, abort_v, 37)) {
         for (int s = 0; s < Cfg::kSub; ++s) tma_store_4d(&mapO, sPt + s * 16384, s * 64, qb * kTile, h, b);
         tma_store_commit();
       }

@@ -50,6 +50,43 @@ def test_warps_whose_lanes_all_wait_get_one_answer(name, role):
     tensor-memory instruction: a lane's own answer is for a wait that one thread makes alone, or is not looked at."""
     body = re.search(r"// -{20,} %s(.*?)(?=// -{20}|__syncthreads\(\))" % re.escape(role), _source(name), re.S).group(1)
     own = re.findall(r"^.*\b(?:mbar_wait|wait_longer)\(.*$", body, re.M)
-    unasked = r"\s*(?:if \(n_tiles > 0\) mbar_wait|if \(!mbar_try_wait\(.*?\)\) wait_longer)\([^;]*;\s*"
-    voted = r".*(?:tid == 0 && |__all_sync\(0xffffffffu, mbar_wait\().*"
-    assert "mbar_wait_warp(" in body and [line.strip() for line in own if not re.fullmatch(unasked + "|" + voted, line)] == []
+    unasked = r"\s*if \((?:n_tiles > 0 && )?!mbar_try_wait\(.*?\)\) wait_longer\([^;]*;\s*"
+    lone_or_voted = r".*(?:tid == 0 && |row == 0 && |__all_sync\(0xffffffffu, mbar_wait\().*"
+    assert "mbar_wait_warp(" in body and [line.strip() for line in own if not re.fullmatch(unasked + "|" + lone_or_voted, line)] == []
+
+
+@pytest.mark.parametrize("name", ["attn_fwd.cu", "attn_bwd.cu"])
+def test_roles_meet_only_where_a_thread_that_has_left_is_not_waited_for(name):
+    """A named barrier (or __syncthreads inside a role) waits for a fixed number of threads without a limit; a thread whose bounded
+    wait ran out never comes."""
+    text = _source(name)
+    roles = text[text.index("// ---"):text.index("if (*abort_")]
+    assert not re.search(r"\b(?:bar|barrier)\.(?:cta\.)?(?:sync|red|arrive)", text) and roles.count("__syncthreads") == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_list_entry_that_is_no_tile_ends_in_a_status(d):
+    """The forward's own check of its lists: the block that meets the entry (as its second or a later item) drains and leaves, the
+    code is in the status word, and the plan built again serves the next call."""
+    import torch
+    from tagseq2tagseq_b200 import build_block_map, read_status
+    from tagseq2tagseq_b200.attention import masked_attn
+    t, h, nb = 4096, 16, 32
+    dev = torch.device("cuda")
+    doc = torch.zeros((1, t), dtype=torch.int32, device=dev)
+    g = torch.Generator(device=dev).manual_seed(1)
+    q, k, v = (torch.randn(1, h, t, d, generator=g, device=dev).bfloat16() for _ in range(3))
+    want, want_lse = masked_attn(q, k, v, doc, plan=build_block_map(doc).plan)
+    plan = build_block_map(doc).plan
+    at = 256                                                    # the layout of csrc/plan.h: status, run_cnt, runs, state, fwd_cnt, fwd_idx
+    for size in (nb * 4, nb * 128 * 16, nb * nb):
+        at = -(-(at + size) // 256) * 256
+    cnt = plan.view(torch.int32)[at // 4:at // 4 + nb]
+    lists = plan.view(torch.int32)[(at + 256) // 4:][:nb * nb].view(nb, nb)
+    assert cnt.tolist() == list(range(1, nb + 1)) and (lists[3, :4] & ~(1 << 30)).tolist() == [0, 1, 2, 3]
+    lists[2, 1] = nb + 5                                        # of the last pair but one in the order of launch
+    masked_attn(q, k, v, doc, plan=plan)
+    assert read_status(plan) in (1014, 1038)                    # the producer or a softmax warp, whoever came first
+    out, lse = masked_attn(q, k, v, doc, plan=build_block_map(doc).plan)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)

@@ -420,8 +420,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       // Order per tile: dV(i), S^T(i+1) (the other way round where S^T has two buffers) | dK(i), dQ(i) | dP^T(i+1).
       // dV and S^T run while the compute warps work on dS^T(i); dK, dQ and dP^T(i+1) while they work on the exponentials
       // of tile i+1, so both sides always have a phase's worth of work in hand.  With one buffer S^T(i+1) overwrites the
-      // P^T columns of tile i: their readers, the dV MMAs, were issued before it by this thread and the tensor pipe
-      // executes one thread's MMAs in issue order.  dK before dQ: its Q stage is reloaded sooner, and at D = 128 the next
+      // P^T columns of tile i and waits for dV(i), which reads them: PTX promises the order of issue only to MMAs with the same
+      // accumulator and shape (linked 16k 815 -> 826 us, causal 4k batch 4 650 -> 652).  With two the last reader, dV(i-1), completed
+      // before dQ(i-1) was read out.  dK before dQ: its Q stage is reloaded sooner, and at D = 128 the next
       // but one tile's Q otherwise lands too late.
       bool ok = mbar_wait(&bar_kv, 0, abort_w, 21) && wait_q(0);
       if (ok) {
@@ -446,7 +447,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           else early_q = more && q_full(i + 1);
         });
         if (Cfg::kSBufs == 1 && more) {
-          if (!(ok = wait_q(i + 1))) break;
+          if (!(ok = wait_q(i + 1) && mbar_wait(&bar_gv[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1, abort_w, 29))) break;
           tc_fence_after();
           TRACE(0, i, 2);
           issue_st(i + 1, [&]() { early_ds = mbar_test_wait(&bar_ds, i & 1); });

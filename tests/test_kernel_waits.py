@@ -64,6 +64,14 @@ def test_roles_meet_only_where_a_thread_that_has_left_is_not_waited_for(name):
     assert not re.search(r"\b(?:bar|barrier)\.(?:cta\.)?(?:sync|red|arrive)", text) and roles.count("__syncthreads") == 1
 
 
+def test_scores_overwrite_the_probabilities_of_the_last_tile_once_their_product_is_complete():
+    """With one S^T buffer S^T(i+1) goes over P^T(i), which dV(i), an MMA with another accumulator, reads: only its completion orders the
+    two, not the order of issue."""
+    text = _source("attn_bwd.cu")
+    one_buffer = text[text.index("if (Cfg::kSBufs == 1 && more) {"):]
+    assert re.match(r"[^{]*\{[^}]*mbar_wait\(&bar_gv\[i % Cfg::kDoStages\], \(i / Cfg::kDoStages\) & 1,[^}]*issue_st\(i \+ 1,", one_buffer)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [64, 128])
 def test_a_list_entry_that_is_no_tile_ends_in_a_status(d):

@@ -86,12 +86,6 @@ constexpr int kFwdItemSlots = 2;
 template <uint32_t N> __device__ __forceinline__ void fwd_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> __device__ __forceinline__ void fwd_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr float kRescaleThreshold = 8.0f;
-#ifndef TS2TS_FWD_X2
-#define TS2TS_FWD_X2 1
-#endif
-#ifndef TS2TS_FWD_DUAL
-#define TS2TS_FWD_DUAL 1
-#endif
 // A wait that is not asked how it ended.  Only its first poll is inline: with the loops inside the tile's code, and no exit from
 // them, full tiles took 2 % longer (causal 4k batch 4, D = 64: 226 instead of 220 us).
 __device__ __noinline__ void wait_longer(uint64_t* bar, uint32_t parity, volatile int* abort_word, int code) {
@@ -516,12 +510,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const int4 mask_cur = mask_pf;
         if (j + 1 < n) prefetch_mask(e_cur);
         FTRACE_ACC(7);
-#if TS2TS_FWD_DUAL
         auto tile = [&](auto masked_tag) {
           constexpr bool kMasked = decltype(masked_tag)::value;
-#else
-        auto tile = [&](bool kMasked) {
-#endif
         uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
         bool dead[4] = {false, false, false, false}, mixed[4] = {false, false, false, false};
         if (kMasked) {
@@ -595,23 +585,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // four partial sums, bf16 pack, P to its place
         const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2), negm2 = pack_f32x2(-m_safe, -m_safe);
         unsigned long long sum2[2] = {0ull, 0ull};
-        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t pk[4][16];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (!kMasked || !dead[c]) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-#if TS2TS_FWD_X2
               float x0, x1;
               unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1])), scale2, negm2), x0, x1);
               const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
               sum2[(i >> 1) & 1] = add_f32x2(sum2[(i >> 1) & 1], pack_f32x2(p0, p1));
-#else
-              const float p0 = fast_exp2(fmaf(__uint_as_float(sv[c][i]), p.scale_log2, -m_safe));
-              const float p1 = fast_exp2(fmaf(__uint_as_float(sv[c][i + 1]), p.scale_log2, -m_safe));
-              sum4[(i >> 1) & 3] += p0 + p1;
-#endif
               pk[c][i >> 1] = pack_bf16(p0, p1);
             }
           } else {
@@ -666,7 +649,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           float s0, s1, s2, s3;
           unpack_f32x2(sum2[0], s0, s1);
           unpack_f32x2(sum2[1], s2, s3);
-          l += (s0 + s1) + (s2 + s3) + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+          l += (s0 + s1) + (s2 + s3);
         }
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 6);
         if constexpr (Cfg::kTmemP) tmem_st_wait();
@@ -677,11 +660,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 7);
         if (kMasked) FTRACE_ACC(6); else FTRACE_ACC(3);
         };
-#if TS2TS_FWD_DUAL
         if (entry & kFullBit) tile(std::false_type{}); else tile(std::true_type{});
-#else
-        tile(!(entry & kFullBit));
-#endif
         ++n_tiles;
       }
       if (!ok) break;
@@ -753,10 +732,10 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
                         PlanView P, MaskArgs M, cudaStream_t stream) {
   CUtensorMap mq, mk, mv, mo;
   int r;
-  if ((r = cached_tile_map(&mq, q, 2, B, H, T, D, sq[0], sq[1], sq[2], kTile, 64))) return r;
-  if ((r = cached_tile_map(&mk, k, 2, B, H, T, D, sk[0], sk[1], sk[2], kTile, 64))) return r;
-  if ((r = cached_tile_map(&mv, v, 2, B, H, T, D, sv[0], sv[1], sv[2], kTile, 64))) return r;
-  if ((r = cached_tile_map(&mo, out, 2, B, H, T, D, so[0], so[1], so[2], kTile, 64))) return r;
+  if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2]))) return r;
+  if ((r = cached_tile_map(&mk, k, B, H, T, D, sk[0], sk[1], sk[2]))) return r;
+  if ((r = cached_tile_map(&mv, v, B, H, T, D, sv[0], sv[1], sv[2]))) return r;
+  if ((r = cached_tile_map(&mo, out, B, H, T, D, so[0], so[1], so[2]))) return r;
   FwdParams p;
   p.plan = P; p.mask = M; p.lse = lse; p.out = static_cast<__nv_bfloat16*>(out);
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];

@@ -10,6 +10,8 @@
 
 #include <mutex>
 
+#include "plan.h"
+
 namespace ts2ts {
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -43,24 +45,21 @@ inline void bind_context() {
   if (fn(&ctx) == CUDA_SUCCESS && ctx == nullptr && cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
 }
 
-// Tensor [B,H,T,D] with D contiguous and element strides (sb, sh, st); tile = box_rows tokens x box_cols
-// elements of one (b,h), written to shared memory with the 128-byte swizzle.  `elem_bytes` is 2 (bf16)
-// or 4 (fp32); box_cols * elem_bytes must be 128.  Rows past T read as zero and are not written.
+// bf16 tensor [B,H,T,D] with D contiguous and element strides (sb, sh, st); tile = kTile tokens x 64 elements of one
+// (b,h), written to shared memory with the 128-byte swizzle.  Rows past T read as zero and are not written.
 // Returns 0 on success.
-inline int make_tile_map(CUtensorMap* out, const void* base, int elem_bytes, int64_t B, int64_t H, int64_t T, int64_t D,
-                         int64_t sb, int64_t sh, int64_t st, int box_rows, int box_cols) {
+inline int make_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return -100;
   bind_context();
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return -101;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)st * elem_bytes, (cuuint64_t)sh * elem_bytes, (cuuint64_t)sb * elem_bytes};
+  cuuint64_t strides[3] = {(cuuint64_t)st * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
   for (int i = 0; i < 3; ++i)
     if (strides[i] % 16 != 0) return -102;
-  cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1, 1};
+  cuuint32_t box[4] = {64, kTile, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  CUresult r = enc(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -103;
 }
@@ -71,11 +70,10 @@ inline int make_tile_map(CUtensorMap* out, const void* base, int elem_bytes, int
 constexpr int kMapCacheSize = 64;
 struct MapKey {
   const void* base;
-  int64_t v[9];
+  int64_t v[7];
   int dev;
 };
-inline int cached_tile_map(CUtensorMap* out, const void* base, int elem_bytes, int64_t B, int64_t H, int64_t T, int64_t D,
-                           int64_t sb, int64_t sh, int64_t st, int box_rows, int box_cols) {
+inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st) {
   struct Entry { MapKey key; CUtensorMap map; bool used; };
   static Entry cache[kMapCacheSize];
   static int next = 0;
@@ -83,8 +81,8 @@ inline int cached_tile_map(CUtensorMap* out, const void* base, int elem_bytes, i
   MapKey key;
   memset(&key, 0, sizeof(key));
   key.base = base;
-  const int64_t vals[9] = {elem_bytes, B, H, T, D, sb, sh, st, (int64_t)box_rows * 65536 + box_cols};
-  for (int i = 0; i < 9; ++i) key.v[i] = vals[i];
+  const int64_t vals[7] = {B, H, T, D, sb, sh, st};
+  for (int i = 0; i < 7; ++i) key.v[i] = vals[i];
   cudaGetDevice(&key.dev);
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < kMapCacheSize; ++i)
@@ -93,7 +91,7 @@ inline int cached_tile_map(CUtensorMap* out, const void* base, int elem_bytes, i
       return 0;
     }
   Entry& e = cache[next];
-  const int r = make_tile_map(&e.map, base, elem_bytes, B, H, T, D, sb, sh, st, box_rows, box_cols);
+  const int r = make_tile_map(&e.map, base, B, H, T, D, sb, sh, st);
   if (r) {
     e.used = false;
     return r;

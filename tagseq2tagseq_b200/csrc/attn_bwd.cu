@@ -10,7 +10,7 @@
 //                           bf16 over the S^T columns just read; then, once dP^T is complete,
 //                           dS^T = P^T (dP^T - delta[q]) as bf16 to shared memory
 //                  tcgen05  dV += P^T dO                          (A from TMEM, B MN-major from smem)
-//                           S^T of the NEXT tile
+//                           S^T of the NEXT tile (D = 128: once dV is complete)
 //                           dK += dS^T Q,  dQ = dS K              (dS^T from smem: K-major for dK, MN-major for dQ)
 //                           dP^T of the next tile once dQ has been read out of the columns they share
 //                  warps 8-11 (thread = query)  dQ -> fp32, 32 head dimensions at a time, through two
@@ -133,7 +133,7 @@ __device__ __noinline__ uint4 key_mask(const PlanView& P, const MaskArgs& M, int
 }
 
 // The per-tile arithmetic of a compute thread, 32 query columns at a time, in two phases so that the first can run
-// while the tensor core still works on dQ^T of the previous tile and dP^T of this one:
+// while the tensor core still works on dK and dQ of the previous tile and dP^T of this one:
 //   p_chunk   P^T = exp2(scale S^T - lse2) under the mask, packed to bf16 pairs (the MMA operand, also kept in
 //             registers for the second phase)
 //   ds_chunk  dS^T = P^T (dP^T - delta), from the bf16 P^T, packed to bf16 pairs
@@ -474,7 +474,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       }
     }
   } else if (warp < 8) {
-    // ------------------------------------------------------------------ exp / dS warps: thread = (key row, 32 of 64 queries)
+    // ------------------------------------------------------------------ exp / dS warps: thread = (key row, 64 of the tile's 128 queries)
     // register pool: 256 x 128 (the launch value) + 128 x 168 + 128 x 88 = 512 x 128; at D = 64, where the reduction warps hold
     // half as much, 256 x 120 + 128 x 136 + 128 x 112 (linked 16k 613 -> 600 us: no spills)
     if (D == 64) reg_dec<120>();

@@ -1,9 +1,8 @@
 // Masked flash-attention forward for sm_100a.
 //
 // Persistent kernel, one CTA per SM.  A work item is a pair of adjacent 128-row query tiles (2p, 2p+1) of one
-// (batch, head); CTAs draw items from a ticket counter in the order the pre-pass wrote (heads one after the
-// other, inside a head the pairs with the most key tiles first), so the tiles that run at the same time share
-// K/V in L2 and the long items start early.  Each query tile of the pair belongs to a "team":
+// (batch, head); CTAs draw items from a ticket counter, group of heads after group of heads, inside a group the pairs with the
+// most key tiles first, so the tiles that run at the same time share K/V in L2 and the long items start early.  Each query tile of the pair belongs to a "team":
 //   softmax team t   4 warps, one thread per query row (setmaxnreg 216)
 //   issuer t         1 thread issuing the team's tcgen05.mma
 // and one producer thread feeds both teams with TMA.  Both teams walk the same ascending stream of key tiles (the

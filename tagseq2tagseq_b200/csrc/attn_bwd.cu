@@ -1,9 +1,11 @@
 // Masked flash-attention backward for sm_100a.
 //
 // Three kernels:
-//   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, padded to whole tiles); zeroes dQ
-//   attn_bwd     one CTA per 128-key tile of one (batch, head); walks the non-skipped 128-query tiles of the
-//                transposed block list.  Scores are transposed so that a tensor-memory lane is a key row:
+//   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, side by side for every 32 queries, padded to
+//                whole tiles); zeroes dQ
+//   attn_bwd     one CTA per 128-key tile of one (batch, head); walks 128-query tiles gathered from the stretches of 32
+//                query rows that hold an allowed pair (PlanLayout::bwd_sub; 11 % fewer tiles on the linked packs, linked 16k, H = 16:
+//                D = 128 1004 -> 956 us, H = 12, D = 64 503 -> 471, warm and at the power limit).  Scores are transposed so that a tensor-memory lane is a key row:
 //                  tcgen05  S^T = K Q^T,  dP^T = V dO^T            [128 keys x 128 queries, fp32 in TMEM]
 //                  warps 0-7 (two threads per key row, 64 queries each), in two phases:
 //                           P^T = exp2(scale S^T - lse2[q]) under the mask, as soon as S^T is complete, written as
@@ -57,8 +59,7 @@ namespace ts2ts {
 struct BwdParams {
   PlanView plan;
   MaskArgs mask;
-  const float* lse2;     // [B,H,Tp]
-  const float* delta;    // [B,H,Tp]
+  const float* stats;    // [B,H,Tp/32][2][32]: -lse2, then -delta
   float* dq_acc;         // [B,H,Tp/32][D/4][32 queries][4], unscaled
   __nv_bfloat16* dk;     // for the empty-list path only
   __nv_bfloat16* dv;
@@ -84,8 +85,9 @@ struct BwdSmem {
   // alignment slack.  The kernel declares no static shared memory, so the dynamic region normally starts 1024-byte
   // aligned and the slack stays unused; if it ever does not fit, the kernel reports status 2900 instead of running.
   static constexpr int kTiles = (2 + kQStages + kDoStages) * kTileBytes + kDsBytes + kStageBytes;
+  static constexpr int kTileSlots = 4;  // a tile's stretch numbers outlive its Q stage until dQ has been read out: one more slot than stages
   static constexpr int kStats = 2 * kQStages * kTile * 4, kBars = 20;
-  static constexpr int kSmall = kStats + kBars * 8 + 16 + kQStages * kMaskRuns * 16;  // statistics, barriers, flags, staged masks
+  static constexpr int kSmall = kStats + kBars * 8 + 16 + kQStages * kMaskRuns * 16 + kTileSlots * 8;  // statistics, barriers, flags, staged masks and stretch numbers
   static constexpr int kSlack = 512;
   static constexpr int kBytes = kTiles + kSmall + kSlack;
   // tensor-memory columns: dV, dK accumulators, S^T (later P^T), dP^T (later dQ)
@@ -95,41 +97,58 @@ struct BwdSmem {
 template <uint32_t N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// 128-bit mask of the query rows of tile qb that may read key `row` of tile kb, before causality, from the run lists: the
-// way out for keys that the plan's mask table does not cover (see kMaskRuns).  "May row class r read my column class" is
-// looked up in the transposed table where the pre-pass built one.
-__device__ __noinline__ uint4 key_mask(const PlanView& P, const MaskArgs& M, int b, int qb, int kb, int row) {
+// A query tile as the kernel walks them: the numbers of four stretches of 32 query rows, kStretchFull set in a full tile
+// (PlanLayout::bwd_sub).  Sequences beyond the table walk whole q tiles.
+__device__ __forceinline__ uint32_t stretch_entry(const uint16_t* subs, const int32_t* list, int i, int j, int NB) {
+  if (subs != nullptr) {
+    uint16_t v;
+    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(v) : "l"(subs + kStretches * i + j));
+    return v;
+  }
+  const int entry = ld_nc_i32_here(list + i);
+  return kStretches * min(static_cast<int>(entry & ~kFullBit), NB - 1) + j | ((entry & kFullBit) ? kStretchFull : 0u);
+}
+// Stretch number of an entry; kStretches * NB stands for no stretch.
+__device__ __forceinline__ int stretch_of(uint32_t entry, int NB) { return min(static_cast<int>(entry & ~kStretchFull), kStretches * NB); }
+
+// Masks of the query rows of two stretches (the numbers in `pair`) that may read key `row` of tile kb, before causality, from
+// the run lists: the way out for keys that the plan's mask table does not cover (see kMaskRuns).  "May row class r read my
+// column class" is looked up in the transposed table where the pre-pass built one.
+__device__ __noinline__ uint2 key_masks(const PlanView& P, const MaskArgs& M, int b, uint32_t pair, int kb, int row) {
   const int kv = kb * kTile + row;
-  if (kv >= P.T) return make_uint4(0u, 0u, 0u, 0u);
+  if (kv >= P.T) return make_uint2(0u, 0u);
   const int kvdoc = M.doc[(size_t)b * P.T + kv], kvcol = M.col[(size_t)b * P.T + kv];
   const bool linked = M.link != nullptr && kvcol >= 0 && kvcol < 64 * M.W;
   const unsigned long long* lt_row = nullptr;
   const int64_t* link_col = nullptr;
   if (linked && P.status[kLinkTRows] == M.R && kvcol < kLinkTMaxCols) lt_row = P.link_t + ((size_t)b * kLinkTMaxCols + kvcol) * kLinkTWords;
   else if (linked) link_col = M.link + (size_t)b * M.R * M.W + (kvcol >> 6);
-  const size_t tq = (size_t)b * P.NB + qb;
-  const int4* runs = reinterpret_cast<const int4*>(P.runs + tq * kTile);
-  const int n = min(__ldg(&P.run_cnt[tq]), kTile), n_valid = min(kTile, P.T - qb * kTile);
-  uint32_t bits[4] = {0u, 0u, 0u, 0u};
-  int4 cur = __ldg(runs);
-  uint32_t lo[4];
-  prefix_mask(cur.x, lo);
-  for (int r = 0; r < n; ++r) {
-    const int4 nx = r + 1 < n ? __ldg(runs + r + 1) : make_int4(n_valid, 0, 0, 0);
-    uint32_t hi[4];
-    prefix_mask(nx.x, hi);  // the run covers rows [cur.x, nx.x)
-    bool allowed = cur.y == kvdoc;
-    if (!allowed && linked && cur.z >= 0 && cur.z < M.R)
-      allowed = lt_row != nullptr ? (__ldg(lt_row + (cur.z >> 6)) >> (cur.z & 63)) & 1ull
-                                  : (static_cast<unsigned long long>(__ldg(link_col + (size_t)cur.z * M.W)) >> (kvcol & 63)) & 1ull;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      if (allowed) bits[w] |= hi[w] & ~lo[w];
-      lo[w] = hi[w];
+  uint32_t bits[2] = {0u, 0u};
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const int sub = stretch_of(pair >> (16 * s) & 0xffffu, P.NB);
+    if (sub == kStretches * P.NB) continue;
+    const int qb = sub / kStretches, from = sub % kStretches * kStretch;
+    const size_t tq = (size_t)b * P.NB + qb;
+    const int4* runs = reinterpret_cast<const int4*>(P.runs + tq * kTile);
+    const int n = min(__ldg(&P.run_cnt[tq]), kTile), n_valid = min(kTile, P.T - qb * kTile);
+    uint32_t mask = 0u;
+    int4 cur = __ldg(runs);
+    for (int r = 0; r < n && cur.x < from + kStretch; ++r) {
+      const int4 nx = r + 1 < n ? __ldg(runs + r + 1) : make_int4(n_valid, 0, 0, 0);
+      const int lo = max(cur.x - from, 0), hi = min(nx.x - from, kStretch);  // the run covers these rows of the stretch
+      if (hi > lo) {
+        bool allowed = cur.y == kvdoc;
+        if (!allowed && linked && cur.z >= 0 && cur.z < M.R)
+          allowed = lt_row != nullptr ? (__ldg(lt_row + (cur.z >> 6)) >> (cur.z & 63)) & 1ull
+                                      : (static_cast<unsigned long long>(__ldg(link_col + (size_t)cur.z * M.W)) >> (kvcol & 63)) & 1ull;
+        if (allowed) mask |= (0xffffffffu >> (kStretch - (hi - lo))) << lo;
+      }
+      cur = nx;
     }
-    cur = nx;
+    if (s == 0) bits[0] = mask; else bits[1] = mask;
   }
-  return make_uint4(bits[0], bits[1], bits[2], bits[3]);
+  return make_uint2(bits[0], bits[1]);
 }
 
 // The per-tile arithmetic of a compute thread, 32 query columns at a time, in two phases so that the first can run
@@ -200,6 +219,7 @@ template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
+                const __grid_constant__ CUtensorMap mapQs, const __grid_constant__ CUtensorMap mapDOs,
                 const __grid_constant__ CUtensorMap mapDK, const __grid_constant__ CUtensorMap mapDV,
                 const __grid_constant__ BwdParams p) {
   using Cfg = BwdSmem<D>;
@@ -213,8 +233,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint8_t* sDO = sQ + Cfg::kQStages * Cfg::kTileBytes;  // Cfg::kDoStages buffers
   uint8_t* sDS = sDO + Cfg::kDoStages * Cfg::kTileBytes;  // dS^T, halves of 16 KB
   uint8_t* sStage = sDS + Cfg::kDsBytes;          // dQ staging boxes
-  float (*s_lse2)[kTile] = reinterpret_cast<float (*)[kTile]>(smem + Cfg::kTiles);
-  float (*s_delta)[kTile] = s_lse2 + Cfg::kQStages;
+  float* s_stats = reinterpret_cast<float*>(smem + Cfg::kTiles);  // [Q stages][kStretches][2][32]: -lse2, then -delta
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kTiles + Cfg::kStats);
   uint64_t& bar_kv = bars[0];
   uint64_t* bar_q_full = bars + 1;     // [Q stages] Q, lse2, delta of a stage landed
@@ -231,7 +250,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + Cfg::kBars);
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(reinterpret_cast<uint8_t*>(bars + Cfg::kBars) + 4);
   int* abort_w = const_cast<int*>(abort_ptr);
-  uint4* s_masks = reinterpret_cast<uint4*>(bars + Cfg::kBars + 2);   // [Q stages][kMaskRuns] the pair's masks, by run of the key
+  uint32_t* s_masks = reinterpret_cast<uint32_t*>(bars + Cfg::kBars + 2);  // [Q stages][kStretches][kMaskRuns] the tile's masks, by run of the key
+  uint32_t* s_tile = s_masks + Cfg::kQStages * kStretches * kMaskRuns;  // [kTileSlots][2] a tile's four stretch entries, 16 bits each
+  static_assert(Cfg::kTileSlots > Cfg::kQStages, "");
   {  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
     int bad = 0;
     const int32_t* stw = p.plan.status;
@@ -259,8 +280,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   const int rank = r2 / gsize;
   const int h = grp * G + (r2 - rank * gsize);
   const int kb = min(max(P.bwd_order[(size_t)b * NB + rank], 0), NB - 1);
-  const int n = min(max(P.bwd_cnt[(size_t)b * NB + kb], 0), NB);
+  const int n = min(max((P.bwd_sub != nullptr ? P.bwd_tiles : P.bwd_cnt)[(size_t)b * NB + kb], 0), NB - kb);  // query tiles to walk
   const int32_t* list = P.bwd_idx + ((size_t)b * NB + kb) * NB;
+  const uint16_t* subs = P.bwd_sub != nullptr ? P.bwd_sub + ((size_t)b * sub_line(NB, NB) + sub_line(NB, kb)) * kStretches : nullptr;
 
   if (n == 0) {
     if (tid < kTile) {
@@ -279,7 +301,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
   if (tid == 0) {
     *abort_ptr = 0;
-    mbar_init(&bar_kv, 1);
+    mbar_init(&bar_kv, 2);
     for (int i = 0; i < 3; ++i) {
       mbar_init(&bar_q_full[i], 1);
       mbar_init(&bar_gq[i], 1);
@@ -311,47 +333,57 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
   if (warp >= 12) {
     if (D == 64) reg_dec<112>(); else reg_dec<88>();
-    if (warp == 12 && lane == 0) {
-      // ---------------------------------------------------------------- TMA producer
-      tma_prefetch_desc(&mapQ); tma_prefetch_desc(&mapK); tma_prefetch_desc(&mapV); tma_prefetch_desc(&mapDO);
-      mbar_expect_tx(&bar_kv, 2 * Cfg::kTileBytes);
-      for (int s = 0; s < Cfg::kSub; ++s) {
-        tma_load_4d(sK + s * 16384, &mapK, &bar_kv, s * 64, kb * kTile, h, b);
-        tma_load_4d(sV + s * 16384, &mapV, &bar_kv, s * 64, kb * kTile, h, b);
+    if (warp == 12 || warp == 14) {
+      // ---------------------------------------------------------------- TMA producers: warp 12 K and Q, warp 14 V and dO
+      // A q tile as it lies in memory comes in one box; a gathered one by a lane each for its stretches, in boxes of 32 rows.  A
+      // stretch past the sequence reads as zeros, has no statistics and no masks, and nothing is computed from it.  Every
+      // copy takes its issuing thread 100-150 clk, and a tile's first product waits for the last of them.
+      const bool is_q = warp == 12, mine = lane < kStretches;
+      const CUtensorMap *whole = is_q ? &mapQ : &mapDO, *part = is_q ? &mapQs : &mapDOs;
+      if (lane == 0) {
+        const CUtensorMap* kv = is_q ? &mapK : &mapV;
+        tma_prefetch_desc(kv); tma_prefetch_desc(whole); tma_prefetch_desc(part);
+        mbar_expect_tx(&bar_kv, Cfg::kTileBytes);
+        tma_load_tile(is_q ? sK : sV, kv, &bar_kv, kb * kTile, 0, h, b);
       }
-      auto load_q = [&](int i) {  // Q tile and row statistics of tile i into its stage
-        const int entry = list[i];
-        const int qb = min(entry & ~kFullBit, NB - 1);
-        const int st = i % Cfg::kQStages;
-        const bool masks = !(entry & kFullBit) && P.kv_mask != nullptr;  // partial tile: its masks travel with the stage
-        mbar_expect_tx(&bar_q_full[st], Cfg::kTileBytes + 2 * kTile * 4 + (masks ? kMaskRuns * 16 : 0));
-        if (masks)
-          bulk_load(s_masks + st * kMaskRuns, P.kv_mask + ((size_t)b * ((size_t)NB * (NB + 1) / 2) + mask_pair(qb, kb)) * kMaskRuns, kMaskRuns * 16,
-                    &bar_q_full[st]);
-        for (int s = 0; s < Cfg::kSub; ++s)
-          tma_load_4d(sQ + st * Cfg::kTileBytes + s * 16384, &mapQ, &bar_q_full[st], s * 64, qb * kTile, h, b);
-        const size_t stat = ((size_t)b * p.H + h) * p.Tp + (size_t)qb * kTile;
-        bulk_load(s_lse2[st], p.lse2 + stat, kTile * 4, &bar_q_full[st]);
-        bulk_load(s_delta[st], p.delta + stat, kTile * 4, &bar_q_full[st]);
-      };
-      auto load_do = [&](int i) {
-        const int qb = list[i] & ~kFullBit, st = i % Cfg::kDoStages;
-        mbar_expect_tx(&bar_do_full[st], Cfg::kTileBytes);
-        for (int s = 0; s < Cfg::kSub; ++s)
-          tma_load_4d(sDO + st * Cfg::kTileBytes + s * 16384, &mapDO, &bar_do_full[st], s * 64, qb * kTile, h, b);
-      };
-      load_q(0);
-      for (int i = 0; i < Cfg::kDoStages && i < n; ++i) load_do(i);
-      for (int i = 1; i < Cfg::kQStages && i < n; ++i) load_q(i);
-      for (int i = 0; i + 1 < n; ++i) {
-        if (i + Cfg::kDoStages < n) {
-          if (!mbar_wait(&bar_gv[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1, abort_w, 11)) break;  // dP^T, dV MMAs of tile i done
-          load_do(i + Cfg::kDoStages);
+      const float* stats = p.stats + ((size_t)b * p.H + h) * p.Tp * 2;
+      const uint32_t* masks = P.kv_mask + (size_t)b * ((size_t)NB * (NB + 1) / 2) * (kStretches * kMaskRuns);
+      const int stages = is_q ? Cfg::kQStages : Cfg::kDoStages;
+      uint8_t* tiles = is_q ? sQ : sDO;
+      uint64_t *full = is_q ? bar_q_full : bar_do_full, *free = is_q ? bar_gq : bar_gv;
+      uint32_t entry = stretch_entry(subs, list, 0, lane & (kStretches - 1), NB);
+      int st = 0, use = 0;
+      for (int i = 0; i < n; ++i) {
+        const int sub = stretch_of(entry, NB);
+        const uint32_t next = i + 1 < n ? stretch_entry(subs, list, i + 1, lane & (kStretches - 1), NB) : 0u;
+        const int first = __shfl_sync(0xffffffffu, sub, 0);
+        const bool joined = __all_sync(0xffffffffu, sub == first + (lane & (kStretches - 1)) && sub < kStretches * NB) && first % kStretches == 0;
+        const bool live = mine && sub < kStretches * NB, masked = !(entry & kStretchFull) && P.kv_mask != nullptr;
+        const uint32_t n_live = __popc(__ballot_sync(0xffffffffu, live));
+        if (use > 0 && !mbar_wait_warp(&free[st], (use - 1) & 1, abort_w, is_q ? 12 : 11)) break;  // dK / dV MMAs of the tile before done
+        if (is_q && mine) reinterpret_cast<uint16_t*>(s_tile)[(i % Cfg::kTileSlots) * kStretches + lane] = entry;
+        __syncwarp();
+        if (lane == 0) mbar_expect_tx(&full[st], Cfg::kTileBytes + (is_q ? n_live * (2 * kStretch * 4 + (masked ? kMaskRuns * 4 : 0)) : 0u));
+        __syncwarp();
+        uint8_t* dst = tiles + st * Cfg::kTileBytes;
+        float* stat = s_stats + st * (2 * kTile) + lane * (2 * kStretch);
+        uint32_t* mask = s_masks + (st * kStretches + lane) * kMaskRuns;
+        const uint32_t* mask_src = masks + (mask_pair(sub / kStretches, kb) * kStretches + sub % kStretches) * kMaskRuns;
+        if (joined) {
+          if (lane == 0) {
+            tma_load_tile(dst, whole, &full[st], sub * kStretch, 0, h, b);
+            if (is_q) bulk_load(stat, stats + sub * (2 * kStretch), 2 * kTile * 4, &full[st]);
+            if (is_q && masked) bulk_load(mask, mask_src, kStretches * kMaskRuns * 4, &full[st]);
+          }
+        } else if (mine) {
+          for (int s = 0; s < Cfg::kSub; ++s) tma_load_tile(dst + s * 16384 + lane * (kStretch * 128), part, &full[st], sub * kStretch, s, h, b);
+          if (is_q && live) {
+            bulk_load(stat, stats + sub * (2 * kStretch), 2 * kStretch * 4, &full[st]);
+            if (masked) bulk_load(mask, mask_src, kMaskRuns * 4, &full[st]);
+          }
         }
-        if (i + Cfg::kQStages < n) {  // S^T, dK MMAs of tile i done, its statistics read
-          if (!mbar_wait(&bar_gq[i % Cfg::kQStages], (i / Cfg::kQStages) & 1, abort_w, 12)) break;
-          load_q(i + Cfg::kQStages);
-        }
+        entry = next;
+        if (++st == stages) { st = 0; ++use; }
       }
     } else if (warp == 13 && lane == 0) {
       // ---------------------------------------------------------------- MMA issuer
@@ -491,15 +523,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
-    int e_next = ld_nc_i32_here(list);
     BTRACE_ACC_DECL
     for (int i = 0; i < n && ok; ++i) {
       const int st = i % Cfg::kQStages;
-      const int entry = e_next;
-      if (i + 1 < n) e_next = ld_nc_i32_here(list + i + 1);
-      const int qb = min(entry & ~kFullBit, NB - 1);
-      const bool masked = (entry & kFullBit) == 0;
-      if (!(ok = mbar_wait_warp(&bar_q_full[st], (i / Cfg::kQStages) & 1, abort_w, 30))) break;  // Q, -lse2, -delta and the masks of this tile landed
+      if (!(ok = mbar_wait_warp(&bar_q_full[st], (i / Cfg::kQStages) & 1, abort_w, 30))) break;  // Q, -lse2, -delta, the masks and the stretch numbers of this tile landed
       // Full and partial tiles are separate code: the full one carries no mask state, so that its two phases fit the
       // registers and the instruction cache (first phase 2080 -> 1500 clk a tile, causal 4k, D = 128).
       auto tile = [&](auto masked_tag) {
@@ -508,16 +535,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         int mode[2] = {0, 0};
         uint32_t bw[2] = {0xffffffffu, 0xffffffffu};
         if (kMasked) {
-          const uint4 m4 = run < kMaskRuns ? s_masks[st * kMaskRuns + run] : key_mask(P, p.mask, b, qb, kb, row);
-          bw[0] = half == 0 ? m4.x : m4.z;
-          bw[1] = half == 0 ? m4.y : m4.w;
+          const uint32_t mine = s_tile[i % Cfg::kTileSlots * 2 + half];  // this thread's two stretches
+          if (run < kMaskRuns) {
+            const uint32_t* m = s_masks + (st * kStretches + 2 * half) * kMaskRuns + run;
+            bw[0] = m[0]; bw[1] = m[kMaskRuns];
+          } else {
+            const uint2 m2 = key_masks(P, p.mask, b, mine, kb, row);
+            bw[0] = m2.x; bw[1] = m2.y;
+          }
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
-            if (kb == qb) {  // causal inside the diagonal tile: query rows row..127
-              const int lo = row - 64 * half - 32 * s;
+            const uint32_t entry = mine >> (16 * s) & 0xffffu;
+            const int sub = stretch_of(entry, NB), lo = row - sub % kStretches * kStretch;
+            if (sub / kStretches == kb)  // causal inside the diagonal tile: query rows row..127
               bw[s] &= lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
-            }
-            if (!kv_valid) bw[s] = 0u;
+            if (!kv_valid || sub == kStretches * NB) bw[s] = 0u;
             mode[s] = __all_sync(0xffffffffu, bw[s] == 0u) ? 2 : (__all_sync(0xffffffffu, bw[s] == 0xffffffffu) ? 0 : 1);
           }
         }
@@ -529,16 +561,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         BTRACE_ACC(2);
         if ((tid & 127) == 0) TRACE(1 + half, i, 0);
         const uint32_t tSc = tST + (i % Cfg::kSBufs) * 128 + lane_base + 64 * half;
+        const float* stats = s_stats + st * (2 * kTile) + half * (2 * kSubQ);
         uint32_t pk[2][16];
         {
           uint32_t s0[32], s1[32];
           tmem_ld32(tSc, s0);
           tmem_ld_wait();
-          p_chunk<kMasked>(s0, s_lse2[st] + half * kSubQ, bw[0], mode[0], p.scale_log2, pk[0]);
+          p_chunk<kMasked>(s0, stats, bw[0], mode[0], p.scale_log2, pk[0]);
           tmem_st16(tSc, pk[0]);
           tmem_ld32(tSc + 32, s1);
           tmem_ld_wait();
-          p_chunk<kMasked>(s1, s_lse2[st] + half * kSubQ + 32, bw[1], mode[1], p.scale_log2, pk[1]);
+          p_chunk<kMasked>(s1, stats + 2 * kStretch, bw[1], mode[1], p.scale_log2, pk[1]);
           tmem_st16(tSc + 32, pk[1]);
           tmem_st_wait();
         }
@@ -559,13 +592,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           uint32_t d0[32], d1[32], dsk[16];
           tmem_ld32(tDc, d0);
           tmem_ld_wait();
-          ds_chunk<kMasked>(pk[0], d0, s_delta[st] + half * kSubQ, mode[0], dsk);
+          ds_chunk<kMasked>(pk[0], d0, stats + kStretch, mode[0], dsk);
 #pragma unroll
           for (int g = 0; g < 4; ++g)
             *reinterpret_cast<uint4*>(ds_row + sw128_offset(row, g)) = make_uint4(dsk[g * 4 + 0], dsk[g * 4 + 1], dsk[g * 4 + 2], dsk[g * 4 + 3]);
           tmem_ld32(tDc + 32, d1);
           tmem_ld_wait();
-          ds_chunk<kMasked>(pk[1], d1, s_delta[st] + half * kSubQ + 32, mode[1], dsk);
+          ds_chunk<kMasked>(pk[1], d1, stats + 3 * kStretch, mode[1], dsk);
 #pragma unroll
           for (int g = 0; g < 4; ++g)
             *reinterpret_cast<uint4*>(ds_row + sw128_offset(row, 4 + g)) = make_uint4(dsk[g * 4 + 0], dsk[g * 4 + 1], dsk[g * 4 + 2], dsk[g * 4 + 3]);
@@ -577,7 +610,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if ((tid & 127) == 0) TRACE(1 + half, i, 3);
         return true;
       };
-      ok = masked ? tile(std::true_type{}) : tile(std::false_type{});
+      ok = (s_tile[i % Cfg::kTileSlots * 2] & kStretchFull) ? tile(std::false_type{}) : tile(std::true_type{});
       if (!ok) break;
       BTRACE_ACC(5);
     }
@@ -613,10 +646,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       mbar_arrive(&bar_epi);
     }
     if (tid == 0 && ok && mbar_wait(&bar_epi, 0, abort_w, 33)) {
-      for (int s = 0; s < Cfg::kSub; ++s) {
-        tma_store_4d(&mapDV, out_dv + s * 16384, s * 64, kb * kTile, h, b);
-        tma_store_4d(&mapDK, out_dk + s * 16384, s * 64, kb * kTile, h, b);
-      }
+      tma_store_tile(&mapDV, out_dv, kb * kTile, 0, h, b);
+      tma_store_tile(&mapDK, out_dk, kb * kTile, 0, h, b);
       tma_store_commit();
       tma_store_wait_all();
     }
@@ -626,7 +657,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     // ------------------------------------------------------------------ dQ reduction warps 8-11, thread = query row
     if (D == 64) reg_inc<136>(); else reg_inc<168>();
     const int w = warp & 3;
-    // Each warp owns 32 queries of the dQ tile and two private 4 KB boxes in shared memory.  The rows leave in rounds of 32
+    // Each warp owns a stretch of the dQ tile and two private 4 KB boxes in shared memory.  The rows leave in rounds of 32
     // head dimensions: store a round into one box, hand it to a bulk reduce-add, and store the next round into the other
     // box while the first is read.  Nothing else in the CTA waits for these reads.  The accumulator is laid out
     // [tile][query / 32][d / 4][query % 32][d % 4]: a thread stores four head dimensions of its query in 16 bytes without
@@ -634,9 +665,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     // reductions of 512 consecutive bytes a warp, the whole backward was 7 to 10 % slower.
     const uint32_t tDQr = tDQ + (static_cast<uint32_t>(w * 32) << 16);
     uint8_t* my_stage = sStage + w * 8192;
-    float* acc = p.dq_acc + ((size_t)b * p.H + h) * p.Tp * D + w * (32 * D);
+    float* acc = p.dq_acc + ((size_t)b * p.H + h) * p.Tp * D;  // + sub * kStretch * D: T <= 2^20 rows of D <= 128, so an int holds it
     for (int i = 0; i < n; ++i) {
-      const int qb = min(list[i] & ~kFullBit, NB - 1);
+      if (!mbar_wait_warp(&bar_ds, i & 1, abort_w, 42)) break;  // from the warps that read the stretch numbers behind the producer's barrier
+      const int sub = stretch_of(reinterpret_cast<const uint16_t*>(s_tile)[i % Cfg::kTileSlots * kStretches + w], NB);
       if (!mbar_wait_warp(&bar_g, i & 1, abort_w, 41)) break;
       tc_fence_after();
       if (tid == 2 * kTile) TRACE(1, i, 4);
@@ -648,7 +680,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_dqr);  // the dQ columns may be overwritten once all four warps have arrived
       if (tid == 2 * kTile) TRACE(1, i, 5);
-      float* dst = acc + (size_t)qb * kTile * D;
+      if (sub == kStretches * NB) continue;
+      float* dst = acc + sub * (kStretch * D);
 #pragma unroll
       for (int k = 0; k < D / 32; ++k) {
         uint8_t* buf = my_stage + (k & 1) * 4096;
@@ -688,8 +721,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 template <int D>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                        const float* __restrict__ lse, int64_t o_sb, int64_t o_sh, int64_t o_st, int64_t d_sb,
-                                                       int64_t d_sh, int64_t d_st, int H, int T, int Tp, float* __restrict__ lse2,
-                                                       float* __restrict__ delta, float* __restrict__ dq_acc) {
+                                                       int64_t d_sh, int64_t d_st, int H, int T, int Tp, float* __restrict__ stats,
+                                                       float* __restrict__ dq_acc) {
   constexpr int kLanes = D / 8, kRows = 256 / kLanes, kEach = kTile / kRows < 4 ? kTile / kRows : 4;  // a block covers kRows * kEach rows of one (b, h)
   const int per_bh = Tp / (kRows * kEach);
   const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * (kRows * kEach);
@@ -723,8 +756,9 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
     for (int s = kLanes / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
     if (c == 0) {
       const float l = t < T ? lse[(int64_t)bh * T + t] : -CUDART_INF_F;
-      lse2[row] = l == -CUDART_INF_F ? -CUDART_INF_F : -l * 1.4426950408889634f;
-      delta[row] = -acc;
+      float* s = stats + row / kStretch * (2 * kStretch) + row % kStretch;
+      s[0] = l == -CUDART_INF_F ? -CUDART_INF_F : -l * 1.4426950408889634f;
+      s[kStretch] = -acc;
     }
   }
 }
@@ -768,17 +802,18 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   const int Tp = P.NB * kTile;
   const size_t rows = (size_t)B * H * Tp;
   char* ws = static_cast<char*>(workspace);
-  float* lse2 = reinterpret_cast<float*>(ws);
-  float* delta = reinterpret_cast<float*>(ws + plan_align(rows * 4));
+  float* stats = reinterpret_cast<float*>(ws);
   float* dq_acc = reinterpret_cast<float*>(ws + 2 * plan_align(rows * 4));
-  CUtensorMap mq, mk, mv, mdo, mdk, mdv;
+  CUtensorMap mq, mk, mv, mdo, mqs, mdos, mdk, mdv;
   int r;
-  if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2]))) return r;
-  if ((r = cached_tile_map(&mk, k, B, H, T, D, sk[0], sk[1], sk[2]))) return r;
-  if ((r = cached_tile_map(&mv, v, B, H, T, D, sv[0], sv[1], sv[2]))) return r;
-  if ((r = cached_tile_map(&mdo, dout, B, H, T, D, sdo[0], sdo[1], sdo[2]))) return r;
-  if ((r = cached_tile_map(&mdk, dk, B, H, T, D, sdk[0], sdk[1], sdk[2]))) return r;
-  if ((r = cached_tile_map(&mdv, dv, B, H, T, D, sdv[0], sdv[1], sdv[2]))) return r;
+  if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mk, k, B, H, T, D, sk[0], sk[1], sk[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mv, v, B, H, T, D, sv[0], sv[1], sv[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mdo, dout, B, H, T, D, sdo[0], sdo[1], sdo[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mqs, q, B, H, T, D, sq[0], sq[1], sq[2], kStretch, 64))) return r;
+  if ((r = cached_tile_map(&mdos, dout, B, H, T, D, sdo[0], sdo[1], sdo[2], kStretch, 64))) return r;
+  if ((r = cached_tile_map(&mdk, dk, B, H, T, D, sdk[0], sdk[1], sdk[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mdv, dv, B, H, T, D, sdv[0], sdv[1], sdv[2], kTile, D))) return r;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -791,9 +826,9 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   constexpr int kPrepRows = 256 / (D / 8) * (kTile / (256 / (D / 8)) < 4 ? kTile / (256 / (D / 8)) : 4);
   bwd_prep_kernel<D><<<(unsigned)(rows / kPrepRows), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1],
-      sdo[2], H, T, Tp, lse2, delta, dq_acc);
+      sdo[2], H, T, Tp, stats, dq_acc);
   BwdParams p;
-  p.plan = P; p.mask = M; p.lse2 = lse2; p.delta = delta; p.dq_acc = dq_acc;
+  p.plan = P; p.mask = M; p.stats = stats; p.dq_acc = dq_acc;
   p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
   for (int i = 0; i < 3; ++i) { p.dk_s[i] = sdk[i]; p.dv_s[i] = sdv[i]; }
   p.H = H; p.Tp = Tp; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
@@ -805,7 +840,7 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   BTRACE_ATTACH(p, stream);
   {
     ProfileScope timed(1, stream);
-    attn_bwd_kernel<D><<<(unsigned)B * H * P.NB, kBwdThreads, BwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mdo, mdk, mdv, p);
+    attn_bwd_kernel<D><<<(unsigned)B * H * P.NB, kBwdThreads, BwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mdo, mqs, mdos, mdk, mdv, p);
   }
   dq_convert_kernel<D><<<(unsigned)(rows / 32), 256, 0, stream>>>(reinterpret_cast<const float4*>(dq_acc), static_cast<__nv_bfloat16*>(dq),
                                                                  sdq[0], sdq[1], sdq[2], H, T, Tp, scale);

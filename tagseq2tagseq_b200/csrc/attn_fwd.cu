@@ -302,8 +302,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         s_ring_info[slot] = info;
         if (map != nullptr) {
           mbar_expect_tx(&bar_ring_full[slot], Cfg::kTileBytes);
-          for (int s = 0; s < Cfg::kSub; ++s)
-            tma_load_4d(sRing + slot * Cfg::kTileBytes + s * 16384, map, &bar_ring_full[slot], s * 64, kb * kTile, h, b);
+          tma_load_tile(sRing + slot * Cfg::kTileBytes, map, &bar_ring_full[slot], kb * kTile, 0, h, b);
         } else {
           mbar_arrive(&bar_ring_full[slot]);  // end marker: nothing to load
         }
@@ -327,8 +326,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           if (item.n[t] == 0) continue;
           if (q_loads[t] > 0 && !mbar_wait(&bar_q_free[t], (q_loads[t] - 1) & 1, abort_v, 13)) { ok = false; break; }
           mbar_expect_tx(&bar_q_full[t], Cfg::kTileBytes);
-          for (int s = 0; s < Cfg::kSub; ++s)
-            tma_load_4d(sQ + t * Cfg::kTileBytes + s * 16384, &mapQ, &bar_q_full[t], s * 64, (item.qb0 + t) * kTile, item.h, item.b);
+          tma_load_tile(sQ + t * Cfg::kTileBytes, &mapQ, &bar_q_full[t], (item.qb0 + t) * kTile, 0, item.h, item.b);
           ++q_loads[t];
         }
         if (!ok) break;
@@ -693,7 +691,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_orows[t]);
       if (row == 0 && mbar_wait(&bar_orows[t], n_epi & 1, abort_v, 37)) {
-        for (int s = 0; s < Cfg::kSub; ++s) tma_store_4d(&mapO, sPt + s * 16384, s * 64, qb * kTile, h, b);
+        tma_store_tile(&mapO, sPt, qb * kTile, 0, h, b);
         tma_store_commit();
       }
       ++n_epi;
@@ -731,10 +729,10 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
                         PlanView P, MaskArgs M, cudaStream_t stream) {
   CUtensorMap mq, mk, mv, mo;
   int r;
-  if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2]))) return r;
-  if ((r = cached_tile_map(&mk, k, B, H, T, D, sk[0], sk[1], sk[2]))) return r;
-  if ((r = cached_tile_map(&mv, v, B, H, T, D, sv[0], sv[1], sv[2]))) return r;
-  if ((r = cached_tile_map(&mo, out, B, H, T, D, so[0], so[1], so[2]))) return r;
+  if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mk, k, B, H, T, D, sk[0], sk[1], sk[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mv, v, B, H, T, D, sv[0], sv[1], sv[2], kTile, D))) return r;
+  if ((r = cached_tile_map(&mo, out, B, H, T, D, so[0], so[1], so[2], kTile, D))) return r;
   FwdParams p;
   p.plan = P; p.mask = M; p.lse = lse; p.out = static_cast<__nv_bfloat16*>(out);
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];

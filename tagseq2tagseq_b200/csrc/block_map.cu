@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
   if (kb0 > qb) {  // above the diagonal
     const int kb = kb0 + threadIdx.x;
     if (threadIdx.x < kStateKb && kb < P.NB) {
-      P.state[tq * P.NB + kb] = kSkip;
+      P.state[tq * P.NB + kb] = 0u;
       if (state_out) state_out[tq * P.NB + kb] = kSkip;
     }
     return;
@@ -200,14 +200,24 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
     // a ragged q tile is never full, a diagonal pair always partial; kv tiles below the diagonal are complete
     uint8_t st = !below || !any_some ? kSkip : (any_none || nvq < kTile ? kPartial : kFull);
     if (kb == qb) st = kPartial;
+    // the q tile's stretches that some key's mask has a row of; keys of later runs have no mask here: any row may be theirs
+    uint32_t live = 0u;
+#pragma unroll
+    for (int w = 0; w < kStretches; ++w) live |= mine < nk && kbits[w] != 0u ? 1u << w : 0u;
+#pragma unroll
+    for (int x = 4; x > 0; x >>= 1) live |= __shfl_xor_sync(0xffffffffu, live, x);
+    if (nk > kMaskRuns) live = (1u << ((nvq + kStretch - 1) / kStretch)) - 1u;
     if (mine == 0 && kb < P.NB) {
-      P.state[tq * P.NB + kb] = st;
+      P.state[tq * P.NB + kb] = st == kSkip ? 0u : st == kFull ? kStateFull | kStateLive : live;
       if (state_out) state_out[tq * P.NB + kb] = st;
     }
     if (st == kPartial && P.q_mask != nullptr) {
-      const size_t at = (pairs + mask_pair(qb, kb)) * kMaskRuns + mine;
-      if (mine < nq) P.q_mask[at] = make_uint4(qbits[0], qbits[1], qbits[2], qbits[3]);
-      if (mine < nk) P.kv_mask[at] = make_uint4(kbits[0], kbits[1], kbits[2], kbits[3]);
+      const size_t pair = pairs + mask_pair(qb, kb);
+      if (mine < nq) P.q_mask[pair * kMaskRuns + mine] = make_uint4(qbits[0], qbits[1], qbits[2], qbits[3]);
+      if (mine < nk) {
+#pragma unroll
+        for (int w = 0; w < kStretches; ++w) P.kv_mask[(pair * kStretches + w) * kMaskRuns + mine] = kbits[w];
+      }
     }
   }
 }
@@ -218,6 +228,70 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
 struct ListOutputs {
   int32_t *part_cnt, *part_idx, *full_cnt, *full_idx;
 };
+// The line of a kv tile where the backward's table exists (at most kMaskMaxTiles tiles): the separate lists as above, and the
+// stretches of the q tiles in the order of PlanLayout::bwd_sub.  A lane owns consecutive q tiles, so that one scan over the
+// lanes gives every entry its place; the states of the line are in registers by then.
+__device__ __forceinline__ void stretch_line(const PlanView& P, const ListOutputs& out, int b, int line, int lane) {
+  constexpr int kMost = kMaskMaxTiles / 32;
+  const int span = P.NB - line, each = (span + 31) / 32, c0 = line + lane * each, n = max(0, min(each, P.NB - c0));
+  const uint8_t* column = P.state + ((size_t)b * P.NB + c0) * P.NB + line;
+  uint32_t sts[kMost];
+#pragma unroll
+  for (int u = 0; u < kMost; ++u) sts[u] = u < n ? column[(size_t)u * P.NB] : 0u;
+  // full tiles, partial tiles, those of them with four live stretches; live stretches of the others (at most 512 and 2048)
+  uint32_t tiles = 0u, subs = 0u;
+#pragma unroll
+  for (int u = 0; u < kMost; ++u) {
+    const uint32_t st = sts[u];
+    if (st == 0u) continue;
+    if (st & kStateFull) tiles += 1u << 16;
+    else if (st == kStateLive) { tiles += 1u; subs += 1u << 16; }
+    else { tiles += 1u; subs += __popc(st); }
+  }
+  uint32_t tiles_to = tiles, subs_to = subs;
+#pragma unroll
+  for (int x = 1; x < 32; x *= 2) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, tiles_to, x), c = __shfl_up_sync(0xffffffffu, subs_to, x);
+    if (lane >= x) { tiles_to += a; subs_to += c; }
+  }
+  const uint32_t tiles_all = __shfl_sync(0xffffffffu, tiles_to, 31), subs_all = __shfl_sync(0xffffffffu, subs_to, 31);
+  const int n_part = tiles_all & 0xffffu, n_full = tiles_all >> 16, n_whole = n_full + (subs_all >> 16);
+  const int n_subs = kStretches * n_whole + (subs_all & 0xffffu);
+  const size_t lb = (size_t)b * P.NB + line;
+  uint16_t* sub = P.bwd_sub + ((size_t)b * sub_line(P.NB, P.NB) + sub_line(P.NB, line)) * kStretches;
+  int at_part = (tiles_to - tiles) & 0xffffu, at_full = (tiles_to - tiles) >> 16;
+  int at_live = n_full + ((subs_to - subs) >> 16), at_rest = kStretches * n_whole + ((subs_to - subs) & 0xffffu);
+#pragma unroll
+  for (int u = 0; u < kMost; ++u) {
+    const uint32_t st = sts[u], first = kStretches * (c0 + u);
+    if (st == 0u) continue;
+    const bool whole = (st & kStateLive) == kStateLive, full = st & kStateFull;
+    if (out.part_idx && !full) out.part_idx[lb * P.NB + at_part] = c0 + u;
+    if (out.full_idx && full) out.full_idx[lb * P.NB + at_full] = c0 + u;
+    if (whole) {
+      const uint32_t lo = (first | (first + 1u) << 16) | (full ? kStretchFull | kStretchFull << 16 : 0u);
+      *reinterpret_cast<uint2*>(sub + kStretches * (full ? at_full : at_live)) = make_uint2(lo, lo + 0x20002u);
+    } else {
+#pragma unroll
+      for (int w = 0; w < kStretches; ++w)
+        if ((st >> w) & 1u) sub[at_rest++] = first + w;
+    }
+    at_full += full;
+    at_part += !full;
+    at_live += whole && !full;
+  }
+  const int n_vt = (n_subs + kStretches - 1) / kStretches;
+  if (lane < kStretches * n_vt - n_subs) sub[n_subs + lane] = kStretches * P.NB;
+  if (out.part_idx) for (int c = n_part + lane; c < P.NB; c += 32) out.part_idx[lb * P.NB + c] = -1;
+  if (out.full_idx) for (int c = n_full + lane; c < P.NB; c += 32) out.full_idx[lb * P.NB + c] = -1;
+  if (lane == 0) {
+    P.bwd_cnt[lb] = n_part + n_full;
+    P.bwd_tiles[lb] = n_vt;
+    if (out.part_cnt) out.part_cnt[lb] = n_part;
+    if (out.full_cnt) out.full_cnt[lb] = n_full;
+  }
+}
+
 // blockIdx.z: 0 lines are q tiles, 1 lines are kv tiles; 2 counts, per pair of adjacent q tiles (2p, 2p+1) -- the forward's
 // work items, which share one stream of K/V tiles -- the kv tiles at least one of the two reads.
 __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_out, ListOutputs bwd_out) {
@@ -231,7 +305,7 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
     const uint8_t* s1 = (2 * line + 1 < P.NB) ? s0 + P.NB : s0;
     int n = 0;
 #pragma unroll 8
-    for (int kb = lane; kb <= min(2 * line + 1, P.NB - 1); kb += 32) n += (s0[kb] | s1[kb]) != kSkip;
+    for (int kb = lane; kb <= min(2 * line + 1, P.NB - 1); kb += 32) n += (s0[kb] | s1[kb]) != 0;
     for (int sh = 16; sh > 0; sh >>= 1) n += __shfl_xor_sync(0xffffffffu, n, sh);
     if (lane == 0) P.pair_cnt[(size_t)b * NP + line] = n;
     return;
@@ -241,6 +315,10 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
   int32_t* full_cnt = transposed ? bwd_out.full_cnt : fwd_out.full_cnt;
   int32_t* full_idx = transposed ? bwd_out.full_idx : fwd_out.full_idx;
   if (line >= P.NB) return;
+  if (transposed && P.bwd_sub != nullptr) {
+    stretch_line(P, bwd_out, b, line, lane);
+    return;
+  }
   const size_t lb = (size_t)b * P.NB + line;
   int32_t* m_idx = (transposed ? P.bwd_idx : P.fwd_idx) + lb * P.NB;
   int n_m = 0, n_p = 0, n_f = 0;
@@ -250,13 +328,13 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       const int c = c0 + 32 * u + lane;
-      sts[u] = kSkip;
+      sts[u] = 0;
       if (c < P.NB) sts[u] = transposed ? P.state[((size_t)b * P.NB + c) * P.NB + line] : P.state[lb * P.NB + c];
     }
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       const int c = c0 + 32 * u + lane;
-      const uint8_t st = sts[u];
+      const uint8_t st = sts[u] == 0 ? kSkip : (sts[u] & kStateFull) ? kFull : kPartial;
       const unsigned bm = __ballot_sync(0xffffffffu, st != kSkip);
       const unsigned bp = __ballot_sync(0xffffffffu, st == kPartial);
       const unsigned bf = __ballot_sync(0xffffffffu, st == kFull);

@@ -16,6 +16,13 @@ constexpr int kTile = 128;
 
 enum : uint8_t { kSkip = 0, kPartial = 1, kFull = 2 };
 
+// The backward gathers its query tiles from stretches of 32 query rows (see bwd_sub).  The plan's `state` byte of a tile pair
+// holds in bits 0-3 which of the q tile's four stretches have an allowed (row, key) pair; kStateFull is set on top where every
+// pair is allowed.  0 is a skipped pair.
+constexpr int kStretch = 32, kStretches = kTile / kStretch;
+constexpr uint8_t kStateFull = 0x80, kStateLive = 0x0f;
+constexpr uint32_t kStretchFull = 0x8000u;  // in an entry of bwd_sub: the stretch belongs to a full tile
+
 // A run is a maximal stretch of tokens inside one tile whose (doc id, row class,
 // column class) triple is constant.  `start` is the offset inside the tile.
 struct alignas(16) Run {
@@ -39,24 +46,28 @@ enum : int {
 constexpr int kLinkTMaxRows = 1024, kLinkTMaxCols = 1024, kLinkTWords = kLinkTMaxRows / 64;
 // Masks of partial tiles, worked out once by the pre-pass for every head and layer: for tile pair (qb, kb) and each of the
 // first kMaskRuns runs of the q tile the 128-bit mask of the key columns its rows may read (q_mask), and for each of the
-// first kMaskRuns runs of the kv tile the mask of the query rows that may read its keys (kv_mask); causality inside the
-// diagonal tile is left to the reader.  16 bytes a mask, 2 x 128 bytes a pair at or below the diagonal, so 8.4 MB a
+// q tile's stretches and each of the first kMaskRuns runs of the kv tile the 32-bit mask of the query rows that may read its
+// keys (kv_mask; 32 bytes a stretch, which one bulk copy takes along); causality inside the diagonal tile is left to the
+// reader.  2 x 128 bytes a pair at or below the diagonal, so 8.4 MB a
 // sequence of 32k; the tables exist up to kMaskMaxTiles tiles, and rows of later runs are worked out from the run lists.
 constexpr int kMaskRuns = 8, kMaskMaxTiles = 512;
 inline __host__ __device__ size_t mask_pair(int qb, int kb) { return (size_t)qb * (qb + 1) / 2 + kb; }
 
-constexpr int32_t kPlanMagic = 0x54533254;  // "TS2T"
+// Start of kv tile kb's line in a table with one slot for every q tile at or below the diagonal, lines one after the other.
+inline __host__ __device__ size_t sub_line(int NB, int kb) { return (size_t)kb * NB - (size_t)kb * (kb - 1) / 2; }
+
+constexpr int32_t kPlanMagic = 0x54533255;  // "TS2" and the layout's own mark: a plan of another layout is refused
 
 struct PlanLayout {
   int B, T, NB;
   size_t status;      // int32[64]   see the kStatus* / kStamp* / k*Ticket words above
   size_t run_cnt;     // int32[B,NB]
   size_t runs;        // Run[B,NB,128]
-  size_t state;       // uint8[B,NB,NB]   state[b,qb,kb]
+  size_t state;       // uint8[B,NB,NB]   state[b,qb,kb], see kStateLive
   size_t fwd_cnt;     // int32[B,NB]      non-skipped kv tiles of q tile qb
   size_t fwd_idx;     // int32[B,NB,NB]   ascending kb, kFullBit set when full
   size_t bwd_cnt;     // int32[B,NB]      non-skipped q tiles of kv tile kb
-  size_t bwd_idx;     // int32[B,NB,NB]   ascending qb, kFullBit set when full
+  size_t bwd_idx;     // int32[B,NB,NB]   ascending qb, kFullBit set when full; written where bwd_sub does not exist
   size_t fwd_order;   // int32[B,NB]      q tiles of batch b by descending fwd_cnt
   size_t bwd_order;   // int32[B,NB]      kv tiles of batch b by descending bwd_cnt
   size_t pair_cnt;    // int32[B,NP]      NP = ceil(NB/2): kv tiles that q tile 2p or 2p+1 reads (forward work items)
@@ -64,7 +75,13 @@ struct PlanLayout {
   size_t link_t;      // uint64[B,kLinkTMaxCols,kLinkTWords]   transposed link bits (see kLinkTRows)
   size_t run_mask;    // uint32[B,NB,kMaskRuns,4]   the tokens of each of a tile's first runs, one bit a token
   size_t q_mask;      // uint32[B,NB(NB+1)/2,kMaskRuns,4]   see kMaskRuns; absent above kMaskMaxTiles
-  size_t kv_mask;     // the same shape
+  size_t kv_mask;     // uint32[B,NB(NB+1)/2,kStretches,kMaskRuns]; absent above kMaskMaxTiles
+  // The query tiles the backward walks for a kv tile, four stretches each.  Full q tiles come first, then partial ones whose
+  // stretches are all live, each as it lies in memory; then the live stretches of the others, gathered, so that stretches without
+  // an allowed pair take no part (linked 16k packs: 2743 tile pairs become 2450 tiles, of which 392 are gathered; linked 32k
+  // 15099 and 13458).  All ascend; the last tile is filled up with stretch number kStretches * NB, which lies past the sequence.
+  size_t bwd_sub;     // uint16[B,NB(NB+1)/2,kStretches]   lines by sub_line(); stretch numbers
+  size_t bwd_tiles;   // int32[B,NB]      tiles of each line; both absent above kMaskMaxTiles
   size_t bytes;
 };
 
@@ -95,6 +112,8 @@ inline PlanLayout plan_layout(int B, int T) {
   const size_t masks = nb <= (size_t)kMaskMaxTiles ? b * (nb * (nb + 1) / 2) * kMaskRuns * 16 : 0;
   L.q_mask = off;     off = plan_align(off + masks);
   L.kv_mask = off;    off = plan_align(off + masks);
+  L.bwd_sub = off;    off = plan_align(off + masks / (kMaskRuns * 16) * kStretches * sizeof(uint16_t));
+  L.bwd_tiles = off;  off = plan_align(off + (masks > 0 ? b * nb * sizeof(int32_t) : 0));
   L.bytes = off;
   return L;
 }
@@ -116,8 +135,10 @@ struct PlanView {
   int32_t* pair_order;
   unsigned long long* link_t;
   uint4* run_mask;
-  uint4* q_mask;   // nullptr when the tables do not exist
-  uint4* kv_mask;
+  uint4* q_mask;   // nullptr when the tables do not exist, like the three after it
+  uint32_t* kv_mask;
+  uint16_t* bwd_sub;
+  int32_t* bwd_tiles;
 };
 
 inline PlanView plan_view(void* base, int B, int T) {
@@ -140,7 +161,9 @@ inline PlanView plan_view(void* base, int B, int T) {
   v.link_t = reinterpret_cast<unsigned long long*>(p + L.link_t);
   v.run_mask = reinterpret_cast<uint4*>(p + L.run_mask);
   v.q_mask = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint4*>(p + L.q_mask) : nullptr;
-  v.kv_mask = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint4*>(p + L.kv_mask) : nullptr;
+  v.kv_mask = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint32_t*>(p + L.kv_mask) : nullptr;
+  v.bwd_sub = L.NB <= kMaskMaxTiles ? reinterpret_cast<uint16_t*>(p + L.bwd_sub) : nullptr;
+  v.bwd_tiles = L.NB <= kMaskMaxTiles ? reinterpret_cast<int32_t*>(p + L.bwd_tiles) : nullptr;
   return v;
 }
 

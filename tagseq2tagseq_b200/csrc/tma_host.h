@@ -45,21 +45,22 @@ inline void bind_context() {
   if (fn(&ctx) == CUDA_SUCCESS && ctx == nullptr && cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
 }
 
-// bf16 tensor [B,H,T,D] with D contiguous and element strides (sb, sh, st); tile = kTile tokens x 64 elements of one
-// (b,h), written to shared memory with the 128-byte swizzle.  Rows past T read as zero and are not written.
+// bf16 tensor [B,H,T,D] with D contiguous and element strides (sb, sh, st); tile = `rows` tokens x `cols` elements of one
+// (b,h), written to shared memory in columns of 64 elements, one after the other, with the 128-byte swizzle.  Rows past T read as zero and are not written.
 // Returns 0 on success.
-inline int make_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st) {
+inline int make_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st,
+                         int rows, int cols) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return -100;
   bind_context();
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return -101;
-  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)st * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
-  for (int i = 0; i < 3; ++i)
+  cuuint64_t dims[5] = {64, (cuuint64_t)T, (cuuint64_t)(D / 64), (cuuint64_t)H, (cuuint64_t)B};
+  cuuint64_t strides[4] = {(cuuint64_t)st * 2, 128, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
+  for (int i = 0; i < 4; ++i)
     if (strides[i] % 16 != 0) return -102;
-  cuuint32_t box[4] = {64, kTile, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint32_t box[5] = {64, (cuuint32_t)rows, (cuuint32_t)(cols / 64), 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -103;
 }
@@ -70,10 +71,11 @@ inline int make_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t 
 constexpr int kMapCacheSize = 64;
 struct MapKey {
   const void* base;
-  int64_t v[7];
+  int64_t v[9];
   int dev;
 };
-inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st) {
+inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st,
+                           int rows, int cols) {
   struct Entry { MapKey key; CUtensorMap map; bool used; };
   static Entry cache[kMapCacheSize];
   static int next = 0;
@@ -81,8 +83,8 @@ inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_
   MapKey key;
   memset(&key, 0, sizeof(key));
   key.base = base;
-  const int64_t vals[7] = {B, H, T, D, sb, sh, st};
-  for (int i = 0; i < 7; ++i) key.v[i] = vals[i];
+  const int64_t vals[9] = {B, H, T, D, sb, sh, st, rows, cols};
+  for (int i = 0; i < 9; ++i) key.v[i] = vals[i];
   cudaGetDevice(&key.dev);
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < kMapCacheSize; ++i)
@@ -91,7 +93,7 @@ inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_
       return 0;
     }
   Entry& e = cache[next];
-  const int r = make_tile_map(&e.map, base, B, H, T, D, sb, sh, st);
+  const int r = make_tile_map(&e.map, base, B, H, T, D, sb, sh, st, rows, cols);
   if (r) {
     e.used = false;
     return r;

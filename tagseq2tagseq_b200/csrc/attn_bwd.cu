@@ -454,8 +454,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       // of tile i+1, so both sides always have a phase's worth of work in hand.  With one buffer S^T(i+1) overwrites the
       // P^T columns of tile i and waits for dV(i), which reads them: PTX promises the order of issue only to MMAs with the same
       // accumulator and shape (linked 16k 815 -> 826 us, causal 4k batch 4 650 -> 652).  With two the last reader, dV(i-1), completed
-      // before dQ(i-1) was read out.  dK before dQ: its Q stage is reloaded sooner, and at D = 128 the next
-      // but one tile's Q otherwise lands too late.
+      // before dQ(i-1) was read out.  At D = 64 dQ comes before dK, which then runs while dQ is read out (linked 16k, H = 12: 471 -> 454 us,
+      // causal 4k batch 4, H = 16: 531 -> 510).  At D = 128, with two Q stages, dK comes first: the stage it frees is asked for before
+      // the copy engine is taken up by dQ's reductions, behind which the next but one tile's Q lands too late (dQ first: 978 -> 1019 us).
       bool ok = mbar_wait(&bar_kv, 0, abort_w, 21) && wait_q(0);
       if (ok) {
         tc_fence_after();
@@ -488,8 +489,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (!(ok = early_ds || mbar_wait(&bar_ds, i & 1, abort_w, 28))) break;
         tc_fence_after();
         TRACE(0, i, 4);
-        issue_dk(i);
-        issue_dq([&]() { early_do = more && do_full(i + 1); });
+        if (D == 64) {
+          issue_dq(nothing);
+          issue_dk(i);
+          early_do = more && do_full(i + 1);
+        } else {
+          issue_dk(i);
+          issue_dq([&]() { early_do = more && do_full(i + 1); });
+        }
         TRACE(0, i, 5);
         early_p = early_q = early_ds = false;
         if (more) {

@@ -23,7 +23,8 @@
 // linked 16k and 32k equal, all at the power limit).
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
 // K/V tiles travel through one ring of shared-memory slots in the order K0, K1, V0, K2, V1, ... (K runs one tile
-// ahead of V because S is computed one tile ahead of P V).  At the end of an item each softmax thread reads its
+// ahead of V because S is computed one tile ahead of P V).  Short launches have the teams share a query tile instead (launch_fwd_t):
+// the tiles of its list go to them in turn, and team 0 adds up both parts at the end, straight from tensor memory.  At the end of an item each softmax thread reads its
 // row of O out of tensor memory and frees it for the next item; the normalised rows leave through shared memory and TMA stores, a
 // warp's 32 rows at a time, while the issuers already work on the next item.
 //
@@ -74,7 +75,7 @@ struct FwdParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_sh, o_st;
   int H;
-  int n_items;           // B * H * ceil(NB / 2)
+  int n_items;           // B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
   int head_group;        // heads whose items are interleaved in the ticket order
   float scale_log2;      // softmax scale * log2(e)
   TS2TS_TRACE_FIELDS
@@ -120,8 +121,8 @@ struct FwdSmem {
   static constexpr int kOut = 2 * kTileBytes;                // eight boxes
   static constexpr int kRing = kOut + 8 * kBoxBytes;         // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
-  static constexpr int kBars = 20 + 2 * kStages;
-  static constexpr int kSmallBytes = kBars * 8 + 24 + 4 * kStages;  // barriers, words
+  static constexpr int kBars = 21 + 2 * kStages;
+  static constexpr int kSmallBytes = kTile * 8 + kBars * 8 + 24 + 4 * kStages;  // row statistics, barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
   // tensor-memory columns of team t
   static __host__ __device__ constexpr int score_col(int t) { return D == 64 ? t * kTile : 2 * kTile; }
@@ -129,36 +130,44 @@ struct FwdSmem {
   static __host__ __device__ constexpr int p_col(int t) { return 384 + t * 64; }
 };
 
-// One work item, decoded from its ticket number by every role on its own.
+// One work item, decoded from its ticket number by every role on its own: the query tiles, key-tile counts and key-tile lists of the two
+// teams.  Teams that share a query tile take every other entry of its list.
 struct FwdItem {
-  int b, h, qb0;
+  int b, h, qb[2];
   int n[2];
   const int32_t* list[2];
 };
 // Ticket order: batch elements one after the other; inside one, groups of G heads; inside a group all heads' heaviest
 // pairs first, then their second heaviest, and so on.  The group bounds the K/V working set that has to stay in L2,
 // and the long items of the last group still start well before the end of the launch.
-__device__ __forceinline__ void decode_item(const PlanView& P, int H, int G, int code, FwdItem& it) {
-  const int NP = (P.NB + 1) / 2;
-  const int per_b = H * NP;
+__device__ __forceinline__ void decode_item(const PlanView& P, int H, int G, int split, int code, FwdItem& it) {
+  const int NI = split ? P.NB : (P.NB + 1) / 2;
+  const int per_b = H * NI;
   it.b = code / per_b;
   const int r1 = code - it.b * per_b;
-  const int g = r1 / (G * NP);
-  const int r2 = r1 - g * G * NP;
+  const int g = r1 / (G * NI);
+  const int r2 = r1 - g * G * NI;
   const int gsize = min(G, H - g * G);
   const int rank = r2 / gsize;
   it.h = g * G + (r2 - rank * gsize);
-  const int pair = min(max(__ldg(&P.pair_order[(size_t)it.b * NP + rank]), 0), NP - 1);
-  it.qb0 = 2 * pair;
-  const size_t row0 = (size_t)it.b * P.NB + it.qb0;
-  it.n[0] = min(max(__ldg(&P.fwd_cnt[row0]), 0), P.NB);
-  it.list[0] = P.fwd_idx + row0 * P.NB;
-  if (it.qb0 + 1 < P.NB) {
-    it.n[1] = min(max(__ldg(&P.fwd_cnt[row0 + 1]), 0), P.NB);
-    it.list[1] = it.list[0] + P.NB;
+  const int at = min(max(__ldg((split ? P.fwd_order : P.pair_order) + (size_t)it.b * NI + rank), 0), NI - 1);
+  it.qb[0] = split ? at : 2 * at;
+  const size_t row0 = (size_t)it.b * P.NB + it.qb[0];
+  const int n0 = min(max(__ldg(&P.fwd_cnt[row0]), 0), P.NB);
+  it.list[0] = it.list[1] = P.fwd_idx + row0 * P.NB;
+  if (split) {
+    it.qb[1] = at;
+    it.n[0] = (n0 + 1) / 2;
+    it.n[1] = n0 / 2;
+    ++it.list[1];
   } else {
+    it.qb[1] = 2 * at + 1;
+    it.n[0] = n0;
     it.n[1] = 0;
-    it.list[1] = it.list[0];
+    if (it.qb[1] < P.NB) {
+      it.n[1] = min(max(__ldg(&P.fwd_cnt[row0 + 1]), 0), P.NB);
+      it.list[1] += P.NB;
+    }
   }
 }
 // What a ring slot holds, written by the producer next to the slot.
@@ -169,15 +178,26 @@ enum : uint32_t {
   kRingLast0 = 32u, kRingLast1 = 64u,   // the team's last tile of the item
   kRingEnd = 128u,                      // no more work
 };
-// Ascending merge of the two key-tile lists of an item.  next() returns the next key tile, -1 at the end, and
+// The key tiles of an item in the order of the ring: the ascending merge of the teams' lists, or the one list of teams that share a
+// query tile, whose tiles go to the teams in turn.  next() returns the next key tile, -1 at the end, and
 // -2 when an entry is not a tile number (the plan does not belong to this call); `info` gets the kRing* bits.
 struct UnionWalk {
   const int32_t *l0, *l1;
   int n0, n1, i0, i1, NB;
-  __device__ __forceinline__ void start(const FwdItem& it, int nb) {
-    l0 = it.list[0]; l1 = it.list[1]; n0 = it.n[0]; n1 = it.n[1]; i0 = i1 = 0; NB = nb;
+  bool split;
+  __device__ __forceinline__ void start(const FwdItem& it, int nb, bool shared) {
+    l0 = it.list[0]; l1 = it.list[1]; n0 = it.n[0]; n1 = it.n[1]; i0 = i1 = 0; NB = nb; split = shared;
   }
   __device__ __forceinline__ int next(uint32_t& info) {
+    if (split) {
+      const int n = n0 + n1;
+      if (i0 >= n) return -1;
+      const int kb = static_cast<int>(__ldg(l0 + i0) & ~kFullBit);
+      if (kb < 0 || kb >= NB) return -2;
+      info = (kRingTeam0 | (i0 < 2 ? kRingFirst0 : 0u) | (i0 >= n - 2 ? kRingLast0 : 0u)) << (i0 & 1);
+      ++i0;
+      return kb;
+    }
     const int a = i0 < n0 ? static_cast<int>(__ldg(l0 + i0) & ~kFullBit) : INT_MAX;
     const int c = i1 < n1 ? static_cast<int>(__ldg(l1 + i1) & ~kFullBit) : INT_MAX;
     const int kb = min(a, c);
@@ -228,7 +248,8 @@ __device__ __noinline__ uint4 row_mask(const PlanView& P, const MaskArgs& M, int
   return make_uint4(bits[0], bits[1], bits[2], bits[3]);
 }
 
-template <int D>
+// kShared: the two teams of a CTA share a query tile and take its key tiles in turn, instead of a query tile of a pair each.
+template <int D, bool kShared>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
@@ -241,7 +262,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint8_t* sQ = smem + Cfg::kQ;
   uint8_t* sOut = smem + Cfg::kOut;
   uint8_t* sRing = smem + Cfg::kRing;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kSmall);
+  float2* s_merge = reinterpret_cast<float2*>(smem + Cfg::kSmall);  // [row] maximum and sum of team 1
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_merge + kTile);
   uint64_t* bar_item_full = bars;        // [2] the producer published a ticket
   uint64_t* bar_item_empty = bars + 2;   // [2] the eight softmax warps copied it
   uint64_t* bar_q_full = bars + 4;       // [team] Q tile landed
@@ -252,8 +274,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P free, O consistent
   uint64_t* bar_ofree = bars + 16;       // [team] O of the item read out of tensor memory
   uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled
-  uint64_t* bar_ring_full = bars + 20;   // [kStages] K or V tile landed in the slot
-  uint64_t* bar_ring_free = bars + 20 + kStages;  // [kStages] both issuers are done with the slot
+  uint64_t* bar_merge = bars + 20;       // team 1's part of a shared query tile is in tensor memory, its row statistics in s_merge
+  uint64_t* bar_ring_full = bars + 21;   // [kStages] K or V tile landed in the slot
+  uint64_t* bar_ring_free = bars + 21 + kStages;  // [kStages] both issuers are done with the slot
   int* s_item = reinterpret_cast<int*>(bars + Cfg::kBars);  // [2] ticket ring
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
   int* abort_w = s_item + 3;
@@ -272,7 +295,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       return;
     }
   }
-
   if (tid == 0) {
     *abort_w = 0;
     s_reads[0] = s_reads[1] = 0u;
@@ -288,6 +310,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       mbar_init(&bar_pv[i], 1);
       mbar_init(&bar_ofree[i], 4);
     }
+    mbar_init(bar_merge, 4);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&bar_ring_full[i], 1);
       mbar_init(&bar_ring_free[i], 2);
@@ -332,7 +355,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       for (uint32_t it = 0; ok; ++it) {
         const uint32_t is = it % kFwdItemSlots;
         if (it >= kFwdItemSlots && !mbar_wait(&bar_item_empty[is], (it / kFwdItemSlots - 1) & 1, abort_v, 12)) break;
-        const int ticket = atomicAdd(&P.status[kFwdTicket], 1);
+        const int ticket = it == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(&P.status[kFwdTicket], 1);  // the first one needs no counter
         const int code = ticket < p.n_items ? ticket : -1;
         s_item[is] = code;
         mbar_arrive(&bar_item_full[is]);
@@ -341,17 +364,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           break;
         }
         FwdItem item;
-        decode_item(P, p.H, p.head_group, code, item);
+        decode_item(P, p.H, p.head_group, kShared, code, item);
         for (int t = 0; t < 2 && ok; ++t) {
           if (item.n[t] == 0) continue;
           if (q_loads[t] > 0 && !mbar_wait(&bar_q_free[t], (q_loads[t] - 1) & 1, abort_v, 13)) { ok = false; break; }
           mbar_expect_tx(&bar_q_full[t], Cfg::kTileBytes);
-          tma_load_tile(sQ + t * Cfg::kTileBytes, &mapQ, &bar_q_full[t], (item.qb0 + t) * kTile, 0, item.h, item.b);
+          tma_load_tile(sQ + t * Cfg::kTileBytes, &mapQ, &bar_q_full[t], item.qb[t] * kTile, 0, item.h, item.b);
           ++q_loads[t];
         }
         if (!ok) break;
         UnionWalk w;
-        w.start(item, NB);
+        w.start(item, NB, kShared);
         uint32_t cur_info = 0, nxt_info = 0;
         int cur = w.next(cur_info);
         if (cur == -2) { atomicCAS(abort_w, 0, 14); break; }
@@ -453,6 +476,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const uint32_t tSr = tmem + Cfg::score_col(t) + lane_base, tOr = tmem + Cfg::out_col(t) + lane_base, tPr = tmem + Cfg::p_col(t) + lane_base;
     uint8_t* box = sOut + warp * Cfg::kBoxBytes;
     uint32_t n_tiles = 0;  // tiles this team has processed so far
+    uint32_t n_merged = 0; // query tiles that both teams had a part of
     FTRACE_ACC_DECL
     // The waits inside a tile are not asked how they ended: one that ran out has set the abort word, or found it set, for good, and
     // whatever is computed from there on stays in this CTA, because every warp looks at the word, as one, before an item's rows
@@ -466,14 +490,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       if (lane == 0) mbar_arrive(&bar_item_empty[is]);
       if (code < 0) break;
       FwdItem item;
-      decode_item(P, p.H, p.head_group, code, item);
-      const int qb = item.qb0 + t;
+      decode_item(P, p.H, p.head_group, kShared, code, item);
+      const int qb = t == 0 ? item.qb[0] : item.qb[1];
       if (qb >= NB) continue;
       const int b = item.b, h = item.h;
       const int n = t == 0 ? item.n[0] : item.n[1];
       const int32_t* list = t == 0 ? item.list[0] : item.list[1];
       const int q = qb * kTile + row;
       const bool q_valid = q < P.T;
+      constexpr int step = kShared ? 2 : 1;
+      const bool shared = kShared && item.n[1] > 0;  // both teams have a part of the query tile
+      if (kShared && t == 1 && n == 0) continue;
       if (n == 0) {  // no readable key tile: defined result, nothing to compute
         if (q_valid) {
           __nv_bfloat16* orow = p.out + (size_t)b * p.o_sb + (size_t)h * p.o_sh + (size_t)q * p.o_st;
@@ -497,7 +524,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       // List entries are fetched two tiles ahead and the mask of a partial tile one tile ahead, so that their latency
       // hides behind the sweeps of the tile before.
       int e_cur = ld_nc_i32_here(list);
-      int e_nxt = n > 1 ? ld_nc_i32_here(list + 1) : 0;
+      int e_nxt = n > 1 ? ld_nc_i32_here(list + step) : 0;
       int4 mask_pf = make_int4(0, 0, 0, 0);
       auto prefetch_mask = [&](int entry) {
         if (entry & kFullBit) return;
@@ -510,7 +537,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       for (int j = 0; j < n && ok; ++j) {
         const int entry = e_cur;
         e_cur = e_nxt;
-        if (j + 2 < n) e_nxt = ld_nc_i32_here(list + j + 2);
+        if (j + 2 < n) e_nxt = ld_nc_i32_here(list + (j + 2) * step);
         const int kb = entry & ~kFullBit;
         if (kb < 0 || kb >= NB) { atomicCAS(abort_w, 0, 38); ok = false; break; }
         const int4 mask_cur = mask_pf;
@@ -664,17 +691,54 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       //      team's warps need not meet; a box is written again once the store before has read it.
       if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 34) && *abort_v == 0))) break;
       tc_fence_after();
+      // Teams that share the query tile: team 1 leaves its part where it is, team 0 scales both to one maximum and adds them up.
+      float f0 = 1.f, f1 = 0.f;
+      if (shared) {
+        if (t == 1) {
+          s_merge[row] = make_float2(m_used, l);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_merge);
+          continue;
+        }
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_merge, n_merged & 1, abort_v, 35) && *abort_v == 0))) break;
+        tc_fence_after();
+        ++n_merged;
+        const float2 other = s_merge[row];
+        const float m = fmaxf(m_used, other.x);
+        f0 = m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m);
+        f1 = other.x == -CUDART_INF_F ? 0.f : fast_exp2(other.x - m);
+        m_used = m;
+        l = l * f0 + other.y * f1;
+      }
       const float inv = l > 0.f ? 1.f / l : 0.f;
+      f0 *= inv;
+      f1 *= inv;
 #pragma unroll 1
       for (int s = 0; s < Cfg::kSub; ++s) {
         uint32_t o[2][32];
         tmem_ld32(tOr + s * 64, o[0]);
         tmem_ld32(tOr + s * 64 + 32, o[1]);
-        tmem_ld_wait();
+        if (shared) {
+          uint32_t o1[2][32];
+          tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64, o1[0]);
+          tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64 + 32, o1[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 64; ++i)
+            o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0 + __uint_as_float(o1[i >> 5][i & 31]) * f1);
+        } else {
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 64; ++i) o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0);
+        }
         if (s == Cfg::kSub - 1) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bar_ofree[t]);  // the next item's first P V may overwrite O
+          if (lane == 0) {  // the next item's first P V may overwrite O
+            mbar_arrive(&bar_ofree[t]);
+            if (shared) mbar_arrive(&bar_ofree[1]);
+          }
         }
         if (lane == 0) tma_store_wait_read0();
         __syncwarp();
@@ -682,10 +746,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         for (int g = 0; g < 8; ++g) {
           const uint32_t* w = &o[g >> 2][(g & 3) * 8];
           uint4 v;
-          v.x = pack_bf16(__uint_as_float(w[0]) * inv, __uint_as_float(w[1]) * inv);
-          v.y = pack_bf16(__uint_as_float(w[2]) * inv, __uint_as_float(w[3]) * inv);
-          v.z = pack_bf16(__uint_as_float(w[4]) * inv, __uint_as_float(w[5]) * inv);
-          v.w = pack_bf16(__uint_as_float(w[6]) * inv, __uint_as_float(w[7]) * inv);
+          v.x = pack_bf16(__uint_as_float(w[0]), __uint_as_float(w[1]));
+          v.y = pack_bf16(__uint_as_float(w[2]), __uint_as_float(w[3]));
+          v.z = pack_bf16(__uint_as_float(w[4]), __uint_as_float(w[5]));
+          v.w = pack_bf16(__uint_as_float(w[6]), __uint_as_float(w[7]));
           *reinterpret_cast<uint4*>(box + sw128_offset(lane, g)) = v;
         }
         fence_async_smem();
@@ -725,10 +789,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 }
 
 // Host launcher.  Tensor strides are in elements; the last dimension is contiguous.
-template <int D>
-static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq,
-                        const int64_t* sk, const int64_t* sv, const int64_t* so, int B, int H, int T, float scale,
-                        PlanView P, MaskArgs M, cudaStream_t stream) {
+template <int D, bool kShared>
+static int launch_fwd_as(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq,
+                         const int64_t* sk, const int64_t* sv, const int64_t* so, int B, int H, int T, float scale,
+                        PlanView P, MaskArgs M, int sms, cudaStream_t stream) {
   CUtensorMap mq, mk, mv, mo;
   int r;
   if ((r = cached_tile_map(&mq, q, B, H, T, D, sq[0], sq[1], sq[2], kTile, D))) return r;
@@ -739,7 +803,7 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
   p.plan = P; p.mask = M; p.lse = lse; p.out = static_cast<__nv_bfloat16*>(out);
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];
   p.H = H; p.scale_log2 = scale * 1.4426950408889634f;
-  const long long items = (long long)B * H * ((P.NB + 1) / 2);
+  const long long items = (long long)B * H * (kShared ? P.NB : (P.NB + 1) / 2);
   p.n_items = (int)items;
   {  // heads per group, from the K and V bytes of one head (2 x T x D bf16 each)
     const long long kv_bytes = 4ll * T * D;
@@ -747,24 +811,43 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
     p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
   }
   static bool attr_done[64] = {};
-  static int sm_count[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -110;
   if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_fwd_kernel<D, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes) != cudaSuccess)
       return -110;
-    if (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0) return -110;
     attr_done[dev] = true;
   }
-  const unsigned grid = (unsigned)(items < sm_count[dev] ? items : sm_count[dev]);
+  const unsigned grid = (unsigned)(items < sms ? items : sms);
   FTRACE_ATTACH(p, stream);
   {
     ProfileScope timed(0, stream);
-    attn_fwd_kernel<D><<<grid, kFwdThreads, FwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mo, p);
+    attn_fwd_kernel<D, kShared><<<grid, kFwdThreads, FwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mo, p);
   }
   FTRACE_DUMP(stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -111;
+}
+
+// Shared query tiles are twice as many and half as long, but bring in every key tile once a query tile instead of once a pair,
+// which costs 15 % (D = 64) to 33 % (D = 128) where the launch is long enough to be bound by throughput.  They win where it is as
+// long as its longest item: when all of them run at once, and, with pairs that do, from 32 tiles on, where lists are long and uneven.
+// Measured, us, pairs -> shared: linked 1024, H = 4, D = 64 23.5 -> 18.8; documents of 2048, H = 8, D = 64 18.8 -> 15.2; causal 2 x 1000, H = 8,
+// D = 128 26.8 -> 20.8; linked 2 x 6767, H = 2, D = 128 53 -> 37; linked 16k, H = 2, D = 64 115 -> 76; causal 4096, H = 8, D = 128 70 -> 49.  Beyond the line: documents of 2048,
+// H = 16, D = 128 (128 pairs) 20.9 -> 23.0, and, inside it, documents of about 100 in 4096, H = 9, D = 128 21.2 -> 23.6; linked 4 x 700, H = 12, D = 64 18.8 -> 20.8; linked 5003, H = 12, D = 64 35 -> 43; causal 4k batch 4, H = 16,
+// D = 128 310 -> 420.
+template <int D>
+static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq, const int64_t* sk, const int64_t* sv,
+                        const int64_t* so, int B, int H, int T, float scale, PlanView P, MaskArgs M, cudaStream_t stream) {
+  static int sm_count[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return -110;
+  if (sm_count[dev] <= 0 && (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0)) return -110;
+  const int sms = sm_count[dev];
+  const long long bh = (long long)B * H;
+  const bool shared = bh * P.NB <= sms || (P.NB >= 32 && bh * ((P.NB + 1) / 2) <= sms);
+  return (shared ? launch_fwd_as<D, true> : launch_fwd_as<D, false>)(q, k, v, out, lse, sq, sk, sv, so, B, H, T, scale, P, M, sms, stream);
 }
 
 int launch_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq, const int64_t* sk,

@@ -1,0 +1,37 @@
+"""Short launches of the forward, where the two teams of a block share a query tile, against the dense mask in fp32."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# tiles of one list (none shared, one each, one and two ...); all items at once and one more; pairs at once from 32 tiles on, and one fewer
+@pytest.mark.parametrize("b,h,t", [(1, 1, 1), (2, 2, 127), (1, 3, 200), (2, 3, 385), (1, 4, 1024), (1, 9, 2048), (2, 37, 256), (2, 37, 257), (4, 8, 600),
+                                   (1, 2, 9472), (1, 2, 9473), (1, 9, 4096), (1, 9, 3968), (1, 9, 4097)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("kind", ["causal", "documents", "linked"])
+def test_forward_of_short_launches(b, h, t, d, kind):
+    from tagseq2tagseq_b200 import build_block_map, read_status, synth
+    from tagseq2tagseq_b200.attention import masked_attn
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(t + d)
+    doc, link = torch.zeros((b, t), dtype=torch.int32, device=dev), None
+    if kind != "causal":
+        doc, link = synth.stack_packs([synth.make_pack(s + 1, t, 150, min(16, t), max(600, t // 8), p_link=0.3 if kind == "linked" else 0.0) for s in range(b)])
+        doc, link = torch.from_numpy(doc).to(dev), None if link is None else torch.from_numpy(link).to(dev)
+    q, k, v = (torch.randn(b, h, t, d, device=dev, generator=g).bfloat16() for _ in range(3))
+    plan = build_block_map(doc, link).plan
+    out, lse = masked_attn(q, k, v, doc, link, plan=plan)
+    assert read_status(plan) == 0
+    for i in range(b):
+        ok = doc[i][:, None] == doc[i][None]
+        if link is not None:
+            words = link[i][doc[i].long()]                                     # [t, W]: what row t's document may read
+            ok |= ((torch.gather(words, 1, (doc[i] >> 6).long()[None].expand(t, -1)) >> (doc[i] & 63).long()[None]) & 1).bool()
+        ok &= torch.ones(t, t, dtype=torch.bool, device=dev).tril()
+        for j in sorted({0, h // 2, h - 1}):
+            s = ((q[i, j].float() @ k[i, j].float().T) * d ** -0.5).masked_fill(~ok, float("-inf"))
+            assert (lse[i, j] - torch.logsumexp(s, -1)).abs().max() <= 1e-2
+            assert (out[i, j].float() - torch.softmax(s, -1) @ v[i, j].float()).abs().max() <= 2e-2
+    again, _ = masked_attn(q, k, v, doc, link, plan=plan)
+    assert torch.equal(out, again)

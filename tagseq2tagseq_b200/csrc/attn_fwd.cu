@@ -65,6 +65,13 @@
 // (8 heads) is 5-7 % faster than 64 MB on the two sparser masks, equal on the densest, 2 % slower on plain causal.
 #define TS2TS_FWD_GROUP_MB 136
 #endif
+#ifndef TS2TS_FWD_FOLD_MB
+// K/V bytes of the whole batch up to which its elements are ordered as one, so that the heaviest items of all of them start first:
+// a little under the L2's 126 MB.  us, one after the other -> as one, D = 64 unless noted: causal 4 x 2039, H = 8 56.3 -> 42.7; linked 4 x 14724, H = 3
+// 248 -> 223; D = 128: documents 4 x 3269, H = 8 51.6 -> 47.7; linked 4 x 14414, H = 3 (88 MB) 265 -> 239; linked 4 x 4096, H = 12 (100 MB)
+// 197 -> 172; but causal 4 x 4096, H = 16 (134 MB) 293 -> 308.  The backward gains nothing from it (its blocks are many).
+#define TS2TS_FWD_FOLD_MB 112
+#endif
 
 namespace ts2ts {
 
@@ -76,6 +83,7 @@ struct FwdParams {
   int64_t o_sb, o_sh, o_st;
   int H;
   int n_items;           // B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
+  int heads;             // heads of a stretch of the ticket order: H, or B * H where the batch elements are one
   int head_group;        // heads whose items are interleaved in the ticket order
   float scale_log2;      // softmax scale * log2(e)
   TS2TS_TRACE_FIELDS
@@ -137,19 +145,22 @@ struct FwdItem {
   int n[2];
   const int32_t* list[2];
 };
-// Ticket order: batch elements one after the other; inside one, groups of G heads; inside a group all heads' heaviest
-// pairs first, then their second heaviest, and so on.  The group bounds the K/V working set that has to stay in L2,
-// and the long items of the last group still start well before the end of the launch.
-__device__ __forceinline__ void decode_item(const PlanView& P, int H, int G, int split, int code, FwdItem& it) {
+// Ticket order: batch elements one after the other, or, in short launches, as one (`heads` = B * H); inside one, groups of G heads;
+// inside a group all heads' heaviest items first, then their second heaviest, and so on.  The group bounds the K/V working set that has
+// to stay in L2, and the long items of the last group still start well before the end of the launch.
+__device__ __forceinline__ void decode_item(const PlanView& P, int H, int heads, int G, int split, int code, FwdItem& it) {
   const int NI = split ? P.NB : (P.NB + 1) / 2;
-  const int per_b = H * NI;
-  it.b = code / per_b;
-  const int r1 = code - it.b * per_b;
+  const int per_b = heads * NI;
+  const int b0 = code / per_b;
+  const int r1 = code - b0 * per_b;
   const int g = r1 / (G * NI);
   const int r2 = r1 - g * G * NI;
-  const int gsize = min(G, H - g * G);
+  const int gsize = min(G, heads - g * G);
   const int rank = r2 / gsize;
   it.h = g * G + (r2 - rank * gsize);
+  const int more = it.h / H;  // batch elements past b0
+  it.b = b0 + more;
+  it.h -= more * H;
   const int at = min(max(__ldg((split ? P.fwd_order : P.pair_order) + (size_t)it.b * NI + rank), 0), NI - 1);
   it.qb[0] = split ? at : 2 * at;
   const size_t row0 = (size_t)it.b * P.NB + it.qb[0];
@@ -364,7 +375,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           break;
         }
         FwdItem item;
-        decode_item(P, p.H, p.head_group, kShared, code, item);
+        decode_item(P, p.H, p.heads, p.head_group, kShared, code, item);
         for (int t = 0; t < 2 && ok; ++t) {
           if (item.n[t] == 0) continue;
           if (q_loads[t] > 0 && !mbar_wait(&bar_q_free[t], (q_loads[t] - 1) & 1, abort_v, 13)) { ok = false; break; }
@@ -490,7 +501,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       if (lane == 0) mbar_arrive(&bar_item_empty[is]);
       if (code < 0) break;
       FwdItem item;
-      decode_item(P, p.H, p.head_group, kShared, code, item);
+      decode_item(P, p.H, p.heads, p.head_group, kShared, code, item);
       const int qb = t == 0 ? item.qb[0] : item.qb[1];
       if (qb >= NB) continue;
       const int b = item.b, h = item.h;
@@ -808,7 +819,8 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   {  // heads per group, from the K and V bytes of one head (2 x T x D bf16 each)
     const long long kv_bytes = 4ll * T * D;
     long long g = (static_cast<long long>(TS2TS_FWD_GROUP_MB) << 20) / (kv_bytes > 0 ? kv_bytes : 1);
-    p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
+    p.heads = kv_bytes * B * H <= (static_cast<long long>(TS2TS_FWD_FOLD_MB) << 20) ? B * H : H;
+    p.head_group = (int)(g < 1 ? 1 : (g > p.heads ? p.heads : g));
   }
   static bool attr_done[64] = {};
   int dev = 0;

@@ -25,6 +25,7 @@
 // Computes what the reference gets from autograd of PyTorch FlexAttention
 // (torch/_higher_order_ops/flex_attention.py:947-1075): P = exp(S - LSE), dV = P^T dO, dP = dO V^T,
 // dS = P (dP - delta), dQ = scale dS K, dK = scale dS^T Q.  Rows whose LSE is -inf get zero gradients.
+#include "launch.cuh"
 #include "plan.h"
 #include "profile.h"
 #include "ptx.cuh"
@@ -260,9 +261,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     else if (smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes) bad = 2900;
     if (bad) {
       if (threadIdx.x == 0) atomicCAS(p.plan.status, 0, bad);
+      wait_previous();
       return;
     }
   }
+  let_next_start();
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -296,6 +299,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         }
       }
     }
+    wait_previous();
     return;
   }
 
@@ -346,6 +350,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_expect_tx(&bar_kv, Cfg::kTileBytes);
         tma_load_tile(is_q ? sK : sV, kv, &bar_kv, kb * kTile, 0, h, b);
       }
+      wait_previous();  // the row statistics; dQ's zeros, which everything that adds to them comes after
       const float* stats = p.stats + ((size_t)b * p.H + h) * p.Tp * 2;
       const uint32_t* masks = P.kv_mask + (size_t)b * ((size_t)NB * (NB + 1) / 2) * (kStretches * kMaskRuns);
       const int stages = is_q ? Cfg::kQStages : Cfg::kDoStages;
@@ -732,6 +737,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
                                                        float* __restrict__ dq_acc) {
   constexpr int kLanes = D / 8, kRows = 256 / kLanes, kEach = kTile / kRows < 4 ? kTile / kRows : 4;  // a block covers kRows * kEach rows of one (b, h)
   const int per_bh = Tp / (kRows * kEach);
+  let_next_start();
   const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * (kRows * kEach);
   const int b = bh / H, h = bh - b * H;
   const int r = threadIdx.x / kLanes, c = threadIdx.x % kLanes;
@@ -773,15 +779,16 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
 // The dQ accumulator [B,H,Tp/32][d / 4][query % 32][d % 4] (fp32, sums of dS K) -> bf16 dq.  A block takes 32 queries of
 // one (b, h): four head dimensions of a query are scaled, turned in shared memory and leave as whole rows.
 template <int D>
-__global__ void __launch_bounds__(256) dq_convert_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int64_t sb, int64_t sh,
+__global__ void __launch_bounds__(256) dq_convert_kernel(const float4* acc, __nv_bfloat16* __restrict__ dq, int64_t sb, int64_t sh,
                                                          int64_t st, int H, int T, int Tp, float scale) {
   __shared__ __align__(16) __nv_bfloat16 s_row[32][D + 8];
   const int per_bh = Tp / 32;
   const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * 32;
   const float4* src = acc + (size_t)blockIdx.x * (8 * D);
   float4 v[D / 32];
+  wait_previous();
 #pragma unroll
-  for (int i = 0; i < D / 32; ++i) v[i] = src[i * 256 + threadIdx.x];
+  for (int i = 0; i < D / 32; ++i) v[i] = ld_v4_here(src + i * 256 + threadIdx.x);
 #pragma unroll
   for (int i = 0; i < D / 32; ++i)
     *reinterpret_cast<uint2*>(&s_row[threadIdx.x % 32][(i * 8 + threadIdx.x / 32) * 4]) =
@@ -845,14 +852,23 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
     p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
   }
   BTRACE_ATTACH(p, stream);
+  // The three launches overlap (launch.cuh) where they are short: the main kernel's blocks set themselves up and bring in K, V, Q and dO
+  // under the preparation, the conversion's blocks wait where SMs have run dry.  us, one after the other -> overlapping: linked 600, H = 8,
+  // D = 64 23.0 -> 16.7; linked 1024, H = 4, D = 64 29.1 -> 22.9; causal 2 x 1000, H = 8, D = 128 38.7 -> 35.3; linked 5003, H = 12, D = 64 72.8 -> 66.9;
+  // causal 4096, H = 8, D = 128 95.9 -> 89.4.  Long launches lose by it: linked 8k, H = 8, D = 128 (512 tiles) 140.6 -> 142.6; linked 16k, H = 16, D = 128
+  // 968 -> 988, H = 12, D = 64 (1536 tiles) 457 -> 461.
+  const bool early = (long long)B * H * P.NB * D <= 384 * 128;
+  cudaError_t launched;
   {
     ProfileScope timed(1, stream);
-    attn_bwd_kernel<D><<<(unsigned)B * H * P.NB, kBwdThreads, BwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mdo, mqs, mdos, mdk, mdv, p);
+    launched = launch_after_if(early, attn_bwd_kernel<D>, dim3((unsigned)B * H * P.NB), kBwdThreads, BwdSmem<D>::kBytes, stream, mq, mk, mv, mdo, mqs, mdos, mdk, mdv, p);
   }
-  dq_convert_kernel<D><<<(unsigned)(rows / 32), 256, 0, stream>>>(reinterpret_cast<const float4*>(dq_acc), static_cast<__nv_bfloat16*>(dq),
-                                                                 sdq[0], sdq[1], sdq[2], H, T, Tp, scale);
+  if (launched == cudaSuccess)
+    launched = launch_after_if(early, dq_convert_kernel<D>, dim3((unsigned)(rows / 32)), 256, 0, stream, reinterpret_cast<const float4*>(dq_acc),
+                            static_cast<__nv_bfloat16*>(dq), sdq[0], sdq[1], sdq[2], H, T, Tp, scale);
   BTRACE_DUMP(stream);
-  return cudaGetLastError() == cudaSuccess ? 0 : -121;
+  const cudaError_t last = cudaGetLastError();
+  return launched == cudaSuccess && last == cudaSuccess ? 0 : -121;
 }
 
 int launch_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse, const int64_t* sq,

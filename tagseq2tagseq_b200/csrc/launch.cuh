@@ -17,8 +17,9 @@ __device__ __forceinline__ void after_previous() {
   wait_previous();
 }
 
+// An ordinary launch unless `early`; the kernel's waits then find nothing to wait for.
 template <typename... Params, typename... Args>
-inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+inline cudaError_t launch_after_if(bool early, void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -26,10 +27,14 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, int thread
   cfg.stream = stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = early;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  return launch_after_if(true, kernel, grid, threads, smem, stream, args...);
 }
 
 }  // namespace ts2ts

@@ -271,6 +271,13 @@ __device__ __forceinline__ int4 ld_nc_v4_here(const void* ptr) {
   return v;
 }
 
+// The same for memory that the launch before wrote, behind the wait for its end (launch.cuh).
+__device__ __forceinline__ float4 ld_v4_here(const float4* ptr) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(ptr) : "memory");
+  return v;
+}
+
 // ----------------------------------------------------------------------------- misc
 // 128-bit mask whose low x bits are set (0 <= x <= 128), as four words.  shl.b32 clamps shift amounts above 31, so a
 // full word comes out as (1 << 32) - 1 = 0 - 1.

@@ -66,33 +66,35 @@ inline int make_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t 
 }
 
 // The same map through a small per-process cache: a training step calls the attention entry points once per layer
-// with the same few (pointer, shape, strides) combinations, and encoding a map costs a driver call each time.
+// with the same few (pointer, shape, strides) combinations, and encoding a map costs a driver call each time.  A key has a set of
+// four entries to itself and the few keys that fall on it, so that a look-up compares four keys however many maps are kept: a
+// forward and backward asks for twelve, and a program that takes turns between a few sets of buffers keeps all of theirs.
 // The map is copied out, so a later request that recycles the cache entry cannot change what a caller holds.
-constexpr int kMapCacheSize = 64;
+constexpr int kMapSets = 128, kMapWays = 4;
 struct MapKey {
   const void* base;
   int64_t v[9];
-  int dev;
+  int64_t dev;
 };
 inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_t H, int64_t T, int64_t D, int64_t sb, int64_t sh, int64_t st,
                            int rows, int cols) {
   struct Entry { MapKey key; CUtensorMap map; bool used; };
-  static Entry cache[kMapCacheSize];
-  static int next = 0;
+  struct Set { Entry entry[kMapWays]; int next; };
+  static Set cache[kMapSets];
   static std::mutex mu;
-  MapKey key;
-  memset(&key, 0, sizeof(key));
-  key.base = base;
-  const int64_t vals[9] = {B, H, T, D, sb, sh, st, rows, cols};
-  for (int i = 0; i < 9; ++i) key.v[i] = vals[i];
-  cudaGetDevice(&key.dev);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const MapKey key = {base, {B, H, T, D, sb, sh, st, rows, cols}, dev};
+  uint64_t h = reinterpret_cast<uintptr_t>(base);
+  for (int i = 0; i < 9; ++i) h = (h ^ static_cast<uint64_t>(key.v[i])) * 0x9e3779b97f4a7c15ull;
+  Set& set = cache[(h ^ (h >> 32) ^ static_cast<uint64_t>(dev)) >> 7 & (kMapSets - 1)];
   std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < kMapCacheSize; ++i)
-    if (cache[i].used && memcmp(&cache[i].key, &key, sizeof(key)) == 0) {
-      *out = cache[i].map;
+  for (Entry& e : set.entry)
+    if (e.used && memcmp(&e.key, &key, sizeof(key)) == 0) {
+      *out = e.map;
       return 0;
     }
-  Entry& e = cache[next];
+  Entry& e = set.entry[set.next];
   const int r = make_tile_map(&e.map, base, B, H, T, D, sb, sh, st, rows, cols);
   if (r) {
     e.used = false;
@@ -101,7 +103,7 @@ inline int cached_tile_map(CUtensorMap* out, const void* base, int64_t B, int64_
   e.key = key;
   e.used = true;
   *out = e.map;
-  next = (next + 1) % kMapCacheSize;
+  set.next = (set.next + 1) % kMapWays;
   return 0;
 }
 

@@ -13,14 +13,14 @@
 //             once, so that the issuer can compute S of the NEXT key tile while this one is being exponentiated;
 //             mask (partial tiles only: one select per element against a per-row 128-bit column mask that the pre-pass
 //             worked out; 32-column chunks that are masked for a whole warp are skipped), online softmax in
-//             base 2, P -> bf16 -> tensor memory
-//   tcgen05   O += P V                        (V MN-major; the first 64 keys as soon as their P is there)
-// P needs a place other than the scores it is made from, or S of the next tile could not be computed meanwhile, and that place is
-// tensor memory, because the MMA operands fill the shared-memory pipe.  At D = 64 the columns are S0 | S1 | O0 | O1 | P0 | P1 (H = 16,
-// causal 4k batch 4: 239 -> 222 us, linked 16k: 370 -> 348, against P in shared memory).  At D = 128 they are O0 | O1 | S | P0 | P1, one score
-// buffer for both teams: a team reads its scores into registers at once, so the buffer is taken for a third of a tile's time and the
-// teams fall into step half a tile apart (H = 16, causal 4k batch 4: 304 -> 296 us against P in shared memory and two score buffers;
-// linked 16k and 32k equal, all at the power limit).
+//             base 2, P -> bf16 -> tensor memory (D = 64) or shared memory (D = 128; K-major, 128-byte swizzle)
+//   tcgen05   O += P V                        (V MN-major; with P in tensor memory the first 64 keys as soon as theirs is there)
+// P needs a place other than the scores it is made from, or S of the next tile could not be computed meanwhile.  At D = 64
+// tensor memory has room for it (S0 | S1 | O0 | O1 | P0 | P1), which takes 128 KB a pair of tiles out of the shared-memory
+// pipe that the MMA operands fill (H = 16, causal 4k batch 4: 239 -> 222 us, linked 16k: 370 -> 348).  At D = 128 it has not: with P
+// over its own scores a team waited 1570 clocks a tile for S where it waits 240 (causal 4k); with P in tensor memory and one score buffer
+// for both teams causal 4k batch 4 took 296 us instead of 304, but linked 16k 408 instead of 390 and two linked 32k packs 4230 instead of
+// 4150, because teams whose tiles differ then wait for each other's reads.
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
 // K/V tiles travel through one ring of shared-memory slots in the order K0, K1, V0, K2, V1, ... (K runs one tile
 // ahead of V because S is computed one tile ahead of P V).  Short launches have the teams share a query tile instead (launch_fwd_t):
@@ -28,8 +28,8 @@
 // row of O out of tensor memory and frees it for the next item; the normalised rows leave through shared memory and TMA stores, a
 // warp's 32 rows at a time, while the issuers already work on the next item.
 //
-// Shared memory at D = 128: Q0 Q1 (64 KB), output boxes (32 KB), four K/V slots (128 KB); at D = 64: Q0 Q1 (32 KB), boxes (32 KB), eight
-// slots (128 KB).
+// Shared memory at D = 128: Q0 Q1 (64 KB), P0 P1 (64 KB), three K/V slots (96 KB); at D = 64: Q0 Q1 (32 KB), O0 O1 (32 KB),
+// eight slots (128 KB).
 //
 // Computes what the reference obtains from PyTorch FlexAttention's forward
 // (model/modules/layer.py:33 via tunalab FlexSelfAttention; semantics in
@@ -102,40 +102,24 @@ __device__ __noinline__ void wait_longer(uint64_t* bar, uint32_t parity, volatil
   mbar_wait(bar, parity, abort_word, code);
 }
 
-// Reads of a score buffer that both teams share, counted: an issuer may be any number of tiles away from the team it waits for, which
-// the one phase bit of an mbarrier cannot tell.
-__device__ __forceinline__ void count_read(uint32_t* word) {
-  asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(word)) : "memory");
-}
-__device__ __forceinline__ bool wait_reads(uint32_t* word, uint32_t want, volatile int* abort_word, int code) {
-  for (uint32_t i = 0; i < TS2TS_SPIN_LIMIT; ++i) {
-    uint32_t have;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(have) : "r"(smem_u32(word)) : "memory");
-    if (static_cast<int>(have - want) >= 0) return true;
-    if ((i & 1023u) == 1023u && *abort_word) return false;
-  }
-  atomicCAS(const_cast<int*>(abort_word), 0, code);
-  return false;
-}
-
 template <int D>
 struct FwdSmem {
   static constexpr int kSub = D / 64;
   static constexpr int kTileBytes = kTile * D * 2;
-  static constexpr int kSBufs = D == 64 ? 2 : 1;             // score buffers in tensor memory: one a team, or one for both
-  static constexpr int kBoxBytes = 32 * 128;                 // output staging of a softmax warp: 32 rows of 64 columns
-  static constexpr int kStages = D == 128 ? 4 : 8;
+  static constexpr bool kTmemP = D == 64;                    // P in tensor memory
+  static constexpr int kPBytes = kTile * D * 2;              // at D = 128 P's place; output rows always leave through it
+  static constexpr int kStages = D == 128 ? 3 : 8;
   static constexpr int kQ = 0;                               // two Q tiles
-  static constexpr int kOut = 2 * kTileBytes;                // eight boxes
-  static constexpr int kRing = kOut + 8 * kBoxBytes;         // K/V slots
+  static constexpr int kP = 2 * kTileBytes;                  // two P (or O) tiles
+  static constexpr int kRing = kP + 2 * kPBytes;             // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
   static constexpr int kBars = 21 + 2 * kStages;
-  static constexpr int kSmallBytes = kTile * 8 + kBars * 8 + 24 + 4 * kStages;  // row statistics, barriers, words
+  static constexpr int kSmallBytes = kTile * 8 + kBars * 8 + 16 + 4 * kStages;  // row statistics, barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
   // tensor-memory columns of team t
-  static __host__ __device__ constexpr int score_col(int t) { return D == 64 ? t * kTile : 2 * kTile; }
-  static __host__ __device__ constexpr int out_col(int t) { return D == 64 ? 2 * kTile + t * D : t * D; }
-  static __host__ __device__ constexpr int p_col(int t) { return 384 + t * 64; }
+  static __host__ __device__ constexpr int score_col(int t) { return t * kTile; }
+  static __host__ __device__ constexpr int out_col(int t) { return 2 * kTile + t * D; }
+  static __host__ __device__ constexpr int p_col(int t) { return 2 * kTile + 2 * D + t * 64; }  // kTmemP
 };
 
 // One work item, decoded from its ticket number by every role on its own: the query tiles, key-tile counts and key-tile lists of the two
@@ -271,7 +255,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   // compiler, so every access below becomes a shared-memory instruction instead of a generic one.
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem + Cfg::kQ;
-  uint8_t* sOut = smem + Cfg::kOut;
+  uint8_t* sP = smem + Cfg::kP;
   uint8_t* sRing = smem + Cfg::kRing;
   float2* s_merge = reinterpret_cast<float2*>(smem + Cfg::kSmall);  // [row] maximum and sum of team 1
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_merge + kTile);
@@ -280,19 +264,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint64_t* bar_q_full = bars + 4;       // [team] Q tile landed
   uint64_t* bar_q_free = bars + 6;       // [team] last S of the item complete: the Q buffer may be reloaded
   uint64_t* bar_s = bars + 8;            // [team] S of the tile is in tensor memory
-  uint64_t* bar_sfree = bars + 10;       // [team] S read into registers: its columns may be overwritten (two score buffers)
-  uint64_t* bar_p = bars + 12;           // [team] P of the tile's last 64 keys is written
+  uint64_t* bar_sfree = bars + 10;       // [team] S read into registers: its columns may be overwritten
+  uint64_t* bar_p = bars + 12;           // [team] P of the tile (D = 64: of its last 64 keys) is written
   uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P free, O consistent
   uint64_t* bar_ofree = bars + 16;       // [team] O of the item read out of tensor memory
-  uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled
+  uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled (D = 64)
   uint64_t* bar_merge = bars + 20;       // team 1's part of a shared query tile is in tensor memory, its row statistics in s_merge
   uint64_t* bar_ring_full = bars + 21;   // [kStages] K or V tile landed in the slot
   uint64_t* bar_ring_free = bars + 21 + kStages;  // [kStages] both issuers are done with the slot
   int* s_item = reinterpret_cast<int*>(bars + Cfg::kBars);  // [2] ticket ring
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
   int* abort_w = s_item + 3;
-  uint32_t* s_reads = reinterpret_cast<uint32_t*>(s_item + 4);      // [team] score tiles read, four warps each (one shared buffer)
-  uint32_t* s_ring_info = reinterpret_cast<uint32_t*>(s_item + 6);  // [kStages] kRing* bits of what each slot holds
+  uint32_t* s_ring_info = reinterpret_cast<uint32_t*>(s_item + 4);  // [kStages] kRing* bits of what each slot holds
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -308,7 +291,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   }
   if (tid == 0) {
     *abort_w = 0;
-    s_reads[0] = s_reads[1] = 0u;
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar_item_full[i], 1);
       mbar_init(&bar_item_empty[i], 8);
@@ -366,7 +348,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       for (uint32_t it = 0; ok; ++it) {
         const uint32_t is = it % kFwdItemSlots;
         if (it >= kFwdItemSlots && !mbar_wait(&bar_item_empty[is], (it / kFwdItemSlots - 1) & 1, abort_v, 12)) break;
-        const int ticket = it == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(&P.status[kFwdTicket], 1);  // the first one needs no counter
+        const int ticket = atomicAdd(&P.status[kFwdTicket], 1);
         const int code = ticket < p.n_items ? ticket : -1;
         s_item[is] = code;
         mbar_arrive(&bar_item_full[is]);
@@ -410,11 +392,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       // 64-column halves; the MN-major operand (V) steps 16 key rows = 2048 B
       constexpr uint32_t hi_k = desc_hi(1024);
       const uint32_t q_lo = desc_lo(smem_u32(sQ + t * Cfg::kTileBytes), 16);
+      const uint32_t p_lo = desc_lo(smem_u32(sP + t * Cfg::kPBytes), 16);
       const uint32_t k_ring_lo = desc_lo(smem_u32(sRing), 16), v_ring_lo = desc_lo(smem_u32(sRing), 16384);
       const uint32_t tS = tmem + Cfg::score_col(t), tO = tmem + Cfg::out_col(t), tP = tmem + Cfg::p_col(t);
       const uint32_t mine_bit = kRingTeam0 << t, first_bit = kRingFirst0 << t, last_bit = kRingLast0 << t;
-      uint32_t n_s[2] = {0, 0};  // S tiles issued so far, per team
-      int last = -1;             // whose S was issued last
+      uint32_t n_s = 0;      // S tiles issued by this team so far
       uint32_t n_pv = 0;     // P V tiles issued so far
       uint32_t n_items = 0;  // items this team has started
       for (uint32_t ring = 0;; ++ring) {
@@ -422,25 +404,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (!mbar_wait(&bar_ring_full[slot], use & 1, abort_v, 23)) break;
         const uint32_t info = s_ring_info[slot];
         if (info & kRingEnd) break;
-        // With one score buffer both teams' tiles pass through it in the order of the ring, team 0's first: a tile waits until the
-        // one before it has been read, whichever team's that was.  Both issuers see every slot, so both know the order.
-        const bool other_first = Cfg::kSBufs == 1 && !(info & kRingIsV) && t == 1 && (info & kRingTeam0);
-        if (other_first) { last = 0; ++n_s[0]; }
         if (!(info & mine_bit)) {
-          if (Cfg::kSBufs == 1 && !(info & kRingIsV) && t == 0) { last = 1; ++n_s[1]; }
           mbar_arrive(&bar_ring_free[slot]);
           continue;
         }
         if (!(info & kRingIsV)) {
           if ((info & first_bit) && !mbar_wait(&bar_q_full[t], n_items & 1, abort_v, 22)) break;
           if (info & first_bit) ++n_items;
-          if (Cfg::kSBufs == 1) {
-            if (last >= 0 && !wait_reads(&s_reads[last], 4 * n_s[last], abort_v, 24)) break;
-          } else if (n_s[t] > 0 && !mbar_wait(&bar_sfree[t], (n_s[t] - 1) & 1, abort_v, 24)) {
-            break;
-          }
+          if (n_s > 0 && !mbar_wait(&bar_sfree[t], (n_s - 1) & 1, abort_v, 24)) break;
           tc_fence_after();
-          FTRACE(2 * t, n_s[t], 0);
+          FTRACE(2 * t, n_s, 0);
           const uint32_t k_lo = k_ring_lo + slot * (Cfg::kTileBytes >> 4);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
@@ -448,14 +421,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mma_ss2(tS, q_lo + off, hi_k, k_lo + off, hi_k, idesc_s, kk > 0);
           }
           mma_commit(&bar_s[t]);
-          FTRACE(2 * t, n_s[t], 1);
-          ++n_s[t];
-          last = t;
-          if (Cfg::kSBufs == 1 && t == 0 && (info & kRingTeam1)) { last = 1; ++n_s[1]; }
+          FTRACE(2 * t, n_s, 1);
+          ++n_s;
           if (info & last_bit) mma_commit(&bar_q_free[t]);
           mma_commit(&bar_ring_free[slot]);
         } else {
-          if (!mbar_wait(&bar_p0[t], n_pv & 1, abort_v, 26)) break;
+          if (!mbar_wait(Cfg::kTmemP ? &bar_p0[t] : &bar_p[t], n_pv & 1, abort_v, 26)) break;
           // the first P V of an item overwrites O: the previous item's rows must have been read out
           // (n_items counts this item already, so the previous one is n_items - 2)
           if ((info & first_bit) && n_items > 1 && !mbar_wait(&bar_ofree[t], (n_items - 2) & 1, abort_v, 27)) break;
@@ -463,12 +434,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           FTRACE(2 * t, n_pv, 2);
           const uint32_t v_lo = v_ring_lo + slot * (Cfg::kTileBytes >> 4);
           const uint32_t acc0 = (info & first_bit) ? 0u : 1u;
+          if constexpr (Cfg::kTmemP) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
-          if (!mbar_wait(&bar_p[t], n_pv & 1, abort_v, 28)) break;
-          tc_fence_after();
+            for (int kk = 0; kk < 4; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
+            if (!mbar_wait(&bar_p[t], n_pv & 1, abort_v, 28)) break;
+            tc_fence_after();
 #pragma unroll
-          for (int kk = 4; kk < kTile / 16; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, 1u);
+            for (int kk = 4; kk < kTile / 16; ++kk) mma_ts2(tO, tP + kk * 8, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, 1u);
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < kTile / 16; ++kk) {
+              const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+              mma_ss2(tO, p_lo + off, hi_k, v_lo + kk * (2048 >> 4), hi_k, idesc_pv, kk > 0 ? 1u : acc0);
+            }
+          }
           mma_commit(&bar_pv[t]);
           FTRACE(2 * t, n_pv, 3);
           ++n_pv;
@@ -485,7 +464,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int row = tid & (kTile - 1);
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tSr = tmem + Cfg::score_col(t) + lane_base, tOr = tmem + Cfg::out_col(t) + lane_base, tPr = tmem + Cfg::p_col(t) + lane_base;
-    uint8_t* box = sOut + warp * Cfg::kBoxBytes;
+    uint8_t* sPt = sP + t * Cfg::kPBytes;
     uint32_t n_tiles = 0;  // tiles this team has processed so far
     uint32_t n_merged = 0; // query tiles that both teams had a part of
     FTRACE_ACC_DECL
@@ -545,6 +524,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       prefetch_mask(e_cur);
       float m_used = -CUDART_INF_F, l = 0.f;
       FTRACE_ACC(0);
+      // The store of the warp's last rows must have read their places, which at D = 128 are P's.
+      if (lane == 0) tma_store_wait_read0();
+      __syncwarp();
       for (int j = 0; j < n && ok; ++j) {
         const int entry = e_cur;
         e_cur = e_nxt;
@@ -593,7 +575,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) Cfg::kSBufs == 1 ? count_read(&s_reads[t]) : mbar_arrive(&bar_sfree[t]);  // the issuer may now overwrite S with the next tile's scores
+        if (lane == 0) mbar_arrive(&bar_sfree[t]);  // the issuer may now overwrite S with the next tile's scores
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 2);
         // masked scores become -inf once; both sweeps below then need no mask (exp2(-inf) = 0)
 #pragma unroll
@@ -671,13 +653,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
               tmem_st_wait();
             }
           }
-          if (c == 1) tmem_st16(tPr, pk[0]);
-          if (c >= 1) tmem_st16(tPr + 16 * c, pk[c]);
-          if (c == 1) {
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_p0[t]);
+          if constexpr (Cfg::kTmemP) {
+            if (c == 1) tmem_st16(tPr, pk[0]);
+            if (c >= 1) tmem_st16(tPr + 16 * c, pk[c]);
+            if (c == 1) {
+              tmem_st_wait();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bar_p0[t]);
+            }
+          } else if (c >= 1) {
+#pragma unroll
+            for (int cc = (c == 1 ? 0 : c); cc <= c; ++cc)
+#pragma unroll
+              for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<uint4*>(sPt + (cc >> 1) * 16384 + sw128_offset(row, (cc & 1) * 4 + g)) =
+                    make_uint4(pk[cc][g * 4 + 0], pk[cc][g * 4 + 1], pk[cc][g * 4 + 2], pk[cc][g * 4 + 3]);
           }
         }
         {
@@ -687,7 +678,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
           l += (s0 + s1) + (s2 + s3);
         }
         if (row == 0) FTRACE(2 * t + 1, n_tiles, 6);
-        tmem_st_wait();
+        if constexpr (Cfg::kTmemP) tmem_st_wait();
+        else fence_async_smem();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_p[t]);
@@ -698,8 +690,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         ++n_tiles;
       }
       if (!ok) break;
-      // ---- epilogue: O / l -> bf16 -> the warp's box, 64 columns at a time -> TMA store.  A warp stores its own 32 rows, so that the
-      //      team's warps need not meet; a box is written again once the store before has read it.
+      // ---- epilogue: O / l -> bf16 -> the warp's rows of the team's buffer (at D = 128 P's, free after the last P V), 64 columns at a time ->
+      //      TMA store.  A warp stores its own 32 rows, so that the team's warps need not meet.
       if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 34) && *abort_v == 0))) break;
       tc_fence_after();
       // Teams that share the query tile: team 1 leaves its part where it is, team 0 scales both to one maximum and adds them up.
@@ -751,8 +743,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             if (shared) mbar_arrive(&bar_ofree[1]);
           }
         }
-        if (lane == 0) tma_store_wait_read0();
-        __syncwarp();
+        uint8_t* box = sPt + s * 16384 + (warp & 3) * (32 * 128);
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
           const uint32_t* w = &o[g >> 2][(g & 3) * 8];

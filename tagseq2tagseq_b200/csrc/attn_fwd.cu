@@ -68,7 +68,7 @@
 #ifndef TS2TS_FWD_FOLD_MB
 // K/V bytes of the whole batch up to which its elements are ordered as one, so that the heaviest items of all of them start first:
 // a little under the L2's 126 MB.  us, one after the other -> as one, D = 64 unless noted: causal 4 x 2039, H = 8 56.3 -> 42.7; linked 4 x 14724, H = 3
-// 248 -> 223; D = 128: documents 4 x 3269, H = 8 51.6 -> 47.7; linked 4 x 14414, H = 3 (88 MB) 265 -> 239; linked 4 x 4096, H = 12 (100 MB)
+// 248 -> 223; D = 128: documents 4 x 3269, H = 8 51.1 -> 47.2; linked 4 x 14414, H = 3 (88 MB) 252 -> 236; linked 4 x 4096, H = 12 (100 MB)
 // 197 -> 172; but causal 4 x 4096, H = 16 (134 MB) 293 -> 308.  The backward gains nothing from it (its blocks are many).
 #define TS2TS_FWD_FOLD_MB 112
 #endif
@@ -836,7 +836,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
 // which costs 15 % (D = 64) to 33 % (D = 128) where the launch is long enough to be bound by throughput.  They win where it is as
 // long as its longest item: when all of them run at once, and, with pairs that do, from 32 tiles on, where lists are long and uneven.
 // Measured, us, pairs -> shared: linked 1024, H = 4, D = 64 23.5 -> 18.8; documents of 2048, H = 8, D = 64 18.8 -> 15.2; causal 2 x 1000, H = 8,
-// D = 128 26.8 -> 20.8; linked 2 x 6767, H = 2, D = 128 53 -> 37; linked 16k, H = 2, D = 64 115 -> 76; causal 4096, H = 8, D = 128 70 -> 49.  Beyond the line: documents of 2048,
+// D = 128 26.9 -> 20.8; linked 2 x 6767, H = 2, D = 128 51.5 -> 40.3; linked 16k, H = 2, D = 64 115 -> 76; causal 4096, H = 8, D = 128 70 -> 51.  Beyond the line: documents of 2048,
 // H = 16, D = 128 (128 pairs) 20.9 -> 23.0, and, inside it, documents of about 100 in 4096, H = 9, D = 128 21.2 -> 23.6; linked 4 x 700, H = 12, D = 64 18.8 -> 20.8; linked 5003, H = 12, D = 64 35 -> 43; causal 4k batch 4, H = 16,
 // D = 128 310 -> 420.
 template <int D>

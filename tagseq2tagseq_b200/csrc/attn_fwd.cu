@@ -82,7 +82,7 @@ struct FwdParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_sh, o_st;
   int H;
-  int n_items;           // B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
+  int n_pairs, n_tiles;  // items: B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
   int heads;             // heads of a stretch of the ticket order: H, or B * H where the batch elements are one
   int head_group;        // heads whose items are interleaved in the ticket order
   float scale_log2;      // softmax scale * log2(e)
@@ -245,9 +245,7 @@ __device__ __noinline__ uint4 row_mask(const PlanView& P, const MaskArgs& M, int
 
 // kShared: the two teams of a CTA share a query tile and take its key tiles in turn, instead of a query tile of a pair each.
 template <int D, bool kShared>
-__global__ void __launch_bounds__(kFwdThreads, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
-                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
+__device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtensorMap& mapK, const CUtensorMap& mapV, const CUtensorMap& mapO, const FwdParams& p) {
   using Cfg = FwdSmem<D>;
   constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -349,7 +347,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const uint32_t is = it % kFwdItemSlots;
         if (it >= kFwdItemSlots && !mbar_wait(&bar_item_empty[is], (it / kFwdItemSlots - 1) & 1, abort_v, 12)) break;
         const int ticket = atomicAdd(&P.status[kFwdTicket], 1);
-        const int code = ticket < p.n_items ? ticket : -1;
+        const int code = ticket < (kShared ? p.n_tiles : p.n_pairs) ? ticket : -1;
         s_item[is] = code;
         mbar_arrive(&bar_item_full[is]);
         if (code < 0) {
@@ -790,8 +788,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   }
 }
 
+// Which work items a launch has: pairs of query tiles, query tiles that the teams share, or whichever of the two the lists call for.
+enum FwdForm { kFwdPairs, kFwdShared, kFwdByLists };
+
+// Every CTA comes to the same answer, because it depends on the plan and the grid (one CTA per SM) alone.  Pairs that all run at once take
+// as long as the longest list; shared tiles, two rounds of them, as long as an SM's share of all lists, two key tiles at a time, at 1.6 times
+// the time of a step whose SM has one team to serve, and two steps for the second item.  Both forms measured on 66 calls of 160 to 288 query
+// tiles (D = 64 and 128, longest list 2 to 128): where this line takes the slower one it is by 2 % at most.
+// A kernel with both bodies runs the one that comes first in its code 0.2-0.7 us (1.5 with one head) slower than a kernel of its own, and the other one 2-3 us;
+// so the pairs, whose launches are the short ones, come first (us, pairs | shared tiles | by the lists: documents of 200 to 300 in 4096, H = 7,
+// D = 128 16.2 | 19.4 | 16.9, D = 64 14.4 | 17.0 | 14.8; causal 4096, H = 8, D = 64 60.5 | 47.6 | 50.5).  One body that asks at run time costs both.
+__device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p) {
+  return 5 * (p.plan.status[kLongestList] - 2) * static_cast<int>(gridDim.x) > 4 * p.plan.status[kAllLists] * p.H;
+}
+
+template <int D, int kForm>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
+  if (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
+  else if (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
+  else if (!lists_call_for_shared(p)) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
+  else fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
+}
+
 // Host launcher.  Tensor strides are in elements; the last dimension is contiguous.
-template <int D, bool kShared>
+template <int D, int kForm>
 static int launch_fwd_as(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq,
                          const int64_t* sk, const int64_t* sv, const int64_t* so, int B, int H, int T, float scale,
                         PlanView P, MaskArgs M, int sms, cudaStream_t stream) {
@@ -805,8 +827,9 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   p.plan = P; p.mask = M; p.lse = lse; p.out = static_cast<__nv_bfloat16*>(out);
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];
   p.H = H; p.scale_log2 = scale * 1.4426950408889634f;
-  const long long items = (long long)B * H * (kShared ? P.NB : (P.NB + 1) / 2);
-  p.n_items = (int)items;
+  p.n_pairs = B * H * ((P.NB + 1) / 2);
+  p.n_tiles = B * H * P.NB;
+  const int items = kForm == kFwdPairs ? p.n_pairs : p.n_tiles;
   {  // heads per group, from the K and V bytes of one head (2 x T x D bf16 each)
     const long long kv_bytes = 4ll * T * D;
     long long g = (static_cast<long long>(TS2TS_FWD_GROUP_MB) << 20) / (kv_bytes > 0 ? kv_bytes : 1);
@@ -818,7 +841,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -110;
   if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<D, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_fwd_kernel<D, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes) != cudaSuccess)
       return -110;
     attr_done[dev] = true;
   }
@@ -826,7 +849,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   FTRACE_ATTACH(p, stream);
   {
     ProfileScope timed(0, stream);
-    attn_fwd_kernel<D, kShared><<<grid, kFwdThreads, FwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mo, p);
+    attn_fwd_kernel<D, kForm><<<grid, kFwdThreads, FwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mo, p);
   }
   FTRACE_DUMP(stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -111;
@@ -834,11 +857,13 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
 
 // Shared query tiles are twice as many and half as long, but bring in every key tile once a query tile instead of once a pair,
 // which costs 15 % (D = 64) to 33 % (D = 128) where the launch is long enough to be bound by throughput.  They win where it is as
-// long as its longest item: when all of them run at once, and, with pairs that do, from 32 tiles on, where lists are long and uneven.
-// Measured, us, pairs -> shared: linked 1024, H = 4, D = 64 23.5 -> 18.8; documents of 2048, H = 8, D = 64 18.8 -> 15.2; causal 2 x 1000, H = 8,
-// D = 128 26.9 -> 20.8; linked 2 x 6767, H = 2, D = 128 51.5 -> 40.3; linked 16k, H = 2, D = 64 115 -> 76; causal 4096, H = 8, D = 128 70 -> 51.  Beyond the line: documents of 2048,
-// H = 16, D = 128 (128 pairs) 20.9 -> 23.0, and, inside it, documents of about 100 in 4096, H = 9, D = 128 21.2 -> 23.6; linked 4 x 700, H = 12, D = 64 18.8 -> 20.8; linked 5003, H = 12, D = 64 35 -> 43; causal 4k batch 4, H = 16,
-// D = 128 310 -> 420.
+// long as its longest item.  That is so when all of them run at once: us, pairs -> shared, documents of up to 32 in 2048, H = 9, D = 64 12.9 -> 12.6,
+// linked 1024, H = 4, D = 64 16.6 -> 12.6; documents of 2048, H = 8, D = 64 18.8 -> 16.1; D = 128 20.8 -> 18.8 at H = 9.  Where all pairs run at once
+// but not all tiles, it depends on the lists from 32 tiles on, and the kernel looks at them: pairs for documents of up to 200 in 4096, H = 9
+// (shared tiles 14.7 -> 18.8 at D = 64, 16.8 -> 20.8 at D = 128), shared tiles for linked 16k, H = 2, D = 64 115 -> 77,
+// documents of up to 2048 in 4096, H = 9, D = 64 34.6 -> 28, causal 4096, H = 8, D = 128 68 -> 53.  With fewer tiles than 32 the lists are too short (documents of 2048, H = 16, D = 128 20.9 -> 23.0;
+// linked 4 x 700, H = 12, D = 64 18.8 -> 20.8), and with more pairs than SMs throughput counts (linked 5003, H = 12, D = 64 35 -> 43; causal 4k batch 4,
+// H = 16, D = 128 310 -> 420).
 template <int D>
 static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq, const int64_t* sk, const int64_t* sv,
                         const int64_t* so, int B, int H, int T, float scale, PlanView P, MaskArgs M, cudaStream_t stream) {
@@ -849,8 +874,9 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
   if (sm_count[dev] <= 0 && (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0)) return -110;
   const int sms = sm_count[dev];
   const long long bh = (long long)B * H;
-  const bool shared = bh * P.NB <= sms || (P.NB >= 32 && bh * ((P.NB + 1) / 2) <= sms);
-  return (shared ? launch_fwd_as<D, true> : launch_fwd_as<D, false>)(q, k, v, out, lse, sq, sk, sv, so, B, H, T, scale, P, M, sms, stream);
+  const bool by_lists = P.NB >= 32 && bh * ((P.NB + 1) / 2) <= sms;
+  const auto launch = bh * P.NB <= sms ? launch_fwd_as<D, kFwdShared> : by_lists ? launch_fwd_as<D, kFwdByLists> : launch_fwd_as<D, kFwdPairs>;
+  return launch(q, k, v, out, lse, sq, sk, sv, so, B, H, T, scale, P, M, sms, stream);
 }
 
 int launch_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq, const int64_t* sk,

@@ -375,6 +375,13 @@ __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows)
   int32_t* order = (which == 2 ? P.pair_order : which == 1 ? P.bwd_order : P.fwd_order) + (size_t)b * n;
   __shared__ int4 s_cnt[256];  // 1024 counts at a time
   const int ci = i < n ? cnt[i] : 0;
+  if (which == 0) {  // what the forward chooses its work items by; the adds are on their way while the tiles are ranked
+    const int longest = __reduce_max_sync(0xffffffffu, ci), sum = __reduce_add_sync(0xffffffffu, sub == 0 ? ci : 0);
+    if (threadIdx.x % 32 == 0) {
+      atomicMax(&P.status[kLongestList], longest);
+      atomicAdd(&P.status[kAllLists], sum);
+    }
+  }
   int rank = 0;
   for (int j0 = 0; j0 < n; j0 += 1024) {
     __syncthreads();

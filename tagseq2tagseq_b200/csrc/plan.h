@@ -37,6 +37,7 @@ constexpr uint32_t kFullBit = 1u << 30;  // set in merged list entries for full 
 // leave (counted in `done`) puts both back to zero, so launches that share a plan must be ordered on one stream.
 enum : int {
   kStatusCode = 0, kStampMagic = 1, kStampB = 2, kStampT = 3,
+  kLongestList = 4, kAllLists = 5,  // the forward's lists: the longest of the batch, and the sum of all of one head
   kFwdTicket = 8, kFwdDone = 9, kBwdTicket = 10, kBwdDone = 11,
   kLinkTRows = 12,  // > 0: link_t holds the transposed link bits of this many row classes
 };
@@ -56,7 +57,7 @@ inline __host__ __device__ size_t mask_pair(int qb, int kb) { return (size_t)qb 
 // Start of kv tile kb's line in a table with one slot for every q tile at or below the diagonal, lines one after the other.
 inline __host__ __device__ size_t sub_line(int NB, int kb) { return (size_t)kb * NB - (size_t)kb * (kb - 1) / 2; }
 
-constexpr int32_t kPlanMagic = 0x54533255;  // "TS2" and the layout's own mark: a plan of another layout is refused
+constexpr int32_t kPlanMagic = 0x54533256;  // "TS2" and the layout's own mark: a plan of another layout is refused
 
 struct PlanLayout {
   int B, T, NB;

@@ -35,3 +35,33 @@ def test_forward_of_short_launches(b, h, t, d, kind):
             assert (out[i, j].float() - torch.softmax(s, -1) @ v[i, j].float()).abs().max() <= 2e-2
     again, _ = masked_attn(q, k, v, doc, link, plan=plan)
     assert torch.equal(out, again)
+
+
+# around 32 tiles and the most pairs and tiles that run at once (148 SMs): one and several elements, one head and several
+@pytest.mark.parametrize("b,h,t", [(1, 9, 4096), (1, 9, 3969), (3, 3, 4096), (1, 2, 18900), (1, 1, 37800)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("kind", ["short", "long"])
+def test_the_form_of_middle_launches_follows_the_lists(b, h, t, d, kind):
+    """All pairs run at once but not all tiles: short lists keep pairs of query tiles, which they are faster with, long ones share tiles.  The
+    two forms round differently, so the bits tell which ran: those of the same heads among more than run at once as pairs, or among as few
+    as run at once as tiles."""
+    from tagseq2tagseq_b200 import build_block_map, read_status, synth
+    from tagseq2tagseq_b200.attention import masked_attn
+    dev = torch.device("cuda")
+    tiles, pairs, sms = -(-t // 128), -(-t // 256), torch.cuda.get_device_properties(0).multi_processor_count
+    assert b * h * pairs <= sms < b * h * tiles
+    other = sms // (b * tiles) if kind == "long" else sms // (b * pairs) + 1
+    if other == 0:
+        pytest.skip("one head alone is more tiles than run at once")
+    doc = torch.zeros((b, t), dtype=torch.int32, device=dev)
+    if kind == "short":
+        doc = torch.from_numpy(synth.stack_packs([synth.make_pack(s + 1, t, 60, 16, 200) for s in range(b)])[0]).to(dev)
+    g = torch.Generator(device=dev).manual_seed(t)
+    q, k, v = (torch.randn(b, max(h, other), t, d, device=dev, generator=g).bfloat16() for _ in range(3))
+    plan, n = build_block_map(doc).plan, min(h, other)
+    out, lse = masked_attn(q[:, :h], k[:, :h], v[:, :h], doc, plan=plan)
+    want, want_lse = masked_attn(q[:, :other], k[:, :other], v[:, :other], doc, plan=plan)
+    assert read_status(plan) == 0
+    assert torch.equal(out[:, :n], want[:, :n]) and torch.equal(lse[:, :n], want_lse[:, :n])
+    again, _ = masked_attn(q[:, :h], k[:, :h], v[:, :h], doc, plan=plan)
+    assert torch.equal(out, again)

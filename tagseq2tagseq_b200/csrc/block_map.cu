@@ -200,15 +200,17 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
     // a ragged q tile is never full, a diagonal pair always partial; kv tiles below the diagonal are complete
     uint8_t st = !below || !any_some ? kSkip : (any_none || nvq < kTile ? kPartial : kFull);
     if (kb == qb) st = kPartial;
-    // the q tile's stretches that some key's mask has a row of; keys of later runs have no mask here: any row may be theirs
+    // a partial pair's stretches that some key's mask has a row of: one reduction for the four pairs of the warp, four bits each
     uint32_t live = 0u;
+    if (__any_sync(0xffffffffu, st == kPartial)) {
 #pragma unroll
-    for (int w = 0; w < kStretches; ++w) live |= mine < nk && kbits[w] != 0u ? 1u << w : 0u;
-#pragma unroll
-    for (int x = 4; x > 0; x >>= 1) live |= __shfl_xor_sync(0xffffffffu, live, x);
-    if (nk > kMaskRuns) live = (1u << ((nvq + kStretch - 1) / kStretch)) - 1u;
+      for (int w = 0; w < kStretches; ++w) live |= kbits[w] != 0u ? 1u << w : 0u;
+      const int at = (lane & 24) >> 1;
+      live = (__reduce_or_sync(0xffffffffu, (mine < nk ? live : 0u) << at) >> at) & kStateLive;
+      if (st == kPartial && nk > kMaskRuns) live = (1u << ((nvq + kStretch - 1) / kStretch)) - 1u;  // keys of later runs have no mask: any row may be theirs
+    }
     if (mine == 0 && kb < P.NB) {
-      P.state[tq * P.NB + kb] = st == kSkip ? 0u : st == kFull ? kStateFull | kStateLive : live;
+      P.state[tq * P.NB + kb] = st == kFull ? kStateFull | kStateLive : live;
       if (state_out) state_out[tq * P.NB + kb] = st;
     }
     if (st == kPartial && P.q_mask != nullptr) {
@@ -222,69 +224,92 @@ __global__ void __launch_bounds__(128) state_kernel(PlanView P, MaskArgs M, uint
   }
 }
 
-// One warp per line.  transposed == 0: line = q tile, scan kv tiles; 1: line = kv tile, scan q tiles.
+// One warp per line.  A line is a q tile, whose kv tiles are scanned, or (transposed) a kv tile, whose q tiles are.
 // Writes the merged list used by the kernels and, when given, the separate partial / full lists in the
 // BlockMask convention (ascending, entries past the count = -1).
 struct ListOutputs {
   int32_t *part_cnt, *part_idx, *full_cnt, *full_idx;
 };
-// The line of a kv tile where the backward's table exists (at most kMaskMaxTiles tiles): the separate lists as above, and the
-// stretches of the q tiles in the order of PlanLayout::bwd_sub.  A lane owns consecutive q tiles, so that one scan over the
-// lanes gives every entry its place; the states of the line are in registers by then.
-__device__ __forceinline__ void stretch_line(const PlanView& P, const ListOutputs& out, int b, int line, int lane) {
-  constexpr int kMost = kMaskMaxTiles / 32;
-  const int span = P.NB - line, each = (span + 31) / 32, c0 = line + lane * each, n = max(0, min(each, P.NB - c0));
+// The line of a kv tile where the backward's table exists (at most kMaskMaxTiles tiles), by kWarps warps: the separate lists as above, and the
+// stretches of the q tiles in the order of PlanLayout::bwd_sub.  A warp owns its share of the line: it loads its states at once, counts
+// them, and with the counts of the warps before it and of all every entry has its place.  (Always one warp a line: B = 2, T = 32768 linked
+// 5.8 us for the launch, of which the sweep over the line 0.7 and its stores 0.8; four warps 4.6; without the table 4.2.  Four sequences
+// of 4096: the whole pre-pass 12.8 us with one warp a line and 14.5 with four, 16384 16.0 and 15.3.)
+constexpr int kOneWarpTiles = 64;
+template <int kWarps>
+__device__ __forceinline__ void stretch_line(const PlanView& P, const ListOutputs& out, int b, int line) {
+  constexpr int kMost = 4;  // tiles of a lane
+  static_assert(kMost * 32 * 4 == kMaskMaxTiles && kMost * 32 >= kOneWarpTiles, "");
+  const int warp = threadIdx.x / 32 % kWarps, lane = threadIdx.x & 31;
+  const int sweeps = (P.NB - line + 32 * kWarps - 1) / (32 * kWarps), c0 = line + warp * 32 * sweeps + lane;
   const uint8_t* column = P.state + ((size_t)b * P.NB + c0) * P.NB + line;
   uint32_t sts[kMost];
 #pragma unroll
-  for (int u = 0; u < kMost; ++u) sts[u] = u < n ? column[(size_t)u * P.NB] : 0u;
-  // full tiles, partial tiles, those of them with four live stretches; live stretches of the others (at most 512 and 2048)
+  for (int u = 0; u < kMost; ++u) sts[u] = u < sweeps && c0 + 32 * u < P.NB ? column[(size_t)(32 * u) * P.NB] : 0u;
+  // full tiles and all that are not skipped; tiles with four live stretches, which the full ones are too, and the stretches of the others
   uint32_t tiles = 0u, subs = 0u;
 #pragma unroll
   for (int u = 0; u < kMost; ++u) {
-    const uint32_t st = sts[u];
-    if (st == 0u) continue;
-    if (st & kStateFull) tiles += 1u << 16;
-    else if (st == kStateLive) { tiles += 1u; subs += 1u << 16; }
-    else { tiles += 1u; subs += __popc(st); }
+    const uint32_t live = sts[u] & kStateLive;
+    tiles += (sts[u] & kStateFull ? 1u << 16 : 0u) + (live != 0u ? 1u : 0u);
+    subs += live == kStateLive ? 1u << 16 : __popc(live);
   }
-  uint32_t tiles_to = tiles, subs_to = subs;
+  tiles = __reduce_add_sync(0xffffffffu, tiles);
+  subs = __reduce_add_sync(0xffffffffu, subs);
+  uint32_t tiles_to = 0u, subs_to = 0u;
+  if (kWarps > 1) {
+    __shared__ uint2 s_counts[kWarps];
+    if (lane == 0) s_counts[warp] = make_uint2(tiles, subs);
+    __syncthreads();
+    tiles = subs = 0u;
 #pragma unroll
-  for (int x = 1; x < 32; x *= 2) {
-    const uint32_t a = __shfl_up_sync(0xffffffffu, tiles_to, x), c = __shfl_up_sync(0xffffffffu, subs_to, x);
-    if (lane >= x) { tiles_to += a; subs_to += c; }
+    for (int w = 0; w < kWarps; ++w) {
+      const uint2 n = s_counts[w];
+      if (w < warp) { tiles_to += n.x; subs_to += n.y; }
+      tiles += n.x; subs += n.y;
+    }
   }
-  const uint32_t tiles_all = __shfl_sync(0xffffffffu, tiles_to, 31), subs_all = __shfl_sync(0xffffffffu, subs_to, 31);
-  const int n_part = tiles_all & 0xffffu, n_full = tiles_all >> 16, n_whole = n_full + (subs_all >> 16);
-  const int n_subs = kStretches * n_whole + (subs_all & 0xffffu);
+  const int n_full = tiles >> 16, n_part = (tiles & 0xffffu) - n_full, n_whole = subs >> 16, n_subs = kStretches * n_whole + (subs & 0xffffu);
+  int at_full = tiles_to >> 16, at_part = (tiles_to & 0xffffu) - at_full;
+  int at_live = n_full + (subs_to >> 16) - at_full, at_rest = kStretches * n_whole + (subs_to & 0xffffu);
   const size_t lb = (size_t)b * P.NB + line;
+  const unsigned below = (1u << lane) - 1u;
   uint16_t* sub = P.bwd_sub + ((size_t)b * sub_line(P.NB, P.NB) + sub_line(P.NB, line)) * kStretches;
-  int at_part = (tiles_to - tiles) & 0xffffu, at_full = (tiles_to - tiles) >> 16;
-  int at_live = n_full + ((subs_to - subs) >> 16), at_rest = kStretches * n_whole + ((subs_to - subs) & 0xffffu);
 #pragma unroll
   for (int u = 0; u < kMost; ++u) {
-    const uint32_t st = sts[u], first = kStretches * (c0 + u);
-    if (st == 0u) continue;
-    const bool whole = (st & kStateLive) == kStateLive, full = st & kStateFull;
-    if (out.part_idx && !full) out.part_idx[lb * P.NB + at_part] = c0 + u;
-    if (out.full_idx && full) out.full_idx[lb * P.NB + at_full] = c0 + u;
+    const uint32_t st = sts[u], qb = c0 + 32 * u, first = kStretches * qb;
+    const bool full = (st & kStateFull) != 0u, whole = (st & kStateLive) == kStateLive;
+    const unsigned b_any = __ballot_sync(0xffffffffu, st != 0u), b_full = __ballot_sync(0xffffffffu, full), b_whole = __ballot_sync(0xffffffffu, whole);
+    if (b_any == 0u) continue;
     if (whole) {
       const uint32_t lo = (first | (first + 1u) << 16) | (full ? kStretchFull | kStretchFull << 16 : 0u);
-      *reinterpret_cast<uint2*>(sub + kStretches * (full ? at_full : at_live)) = make_uint2(lo, lo + 0x20002u);
-    } else {
+      const int at = full ? at_full + __popc(b_full & below) : at_live + __popc(b_whole & ~b_full & below);
+      *reinterpret_cast<uint2*>(sub + kStretches * at) = make_uint2(lo, lo + 0x20002u);
+    }
+    if (b_any != b_whole) {
+      const uint32_t live = whole ? 0u : st & kStateLive;
+      int at = at_rest;
+#pragma unroll
+      for (int w = 0; w < kStretches; ++w) {
+        const unsigned bal = __ballot_sync(0xffffffffu, (live >> w) & 1u);
+        at += __popc(bal & below);
+        at_rest += __popc(bal);
+      }
 #pragma unroll
       for (int w = 0; w < kStretches; ++w)
-        if ((st >> w) & 1u) sub[at_rest++] = first + w;
+        if ((live >> w) & 1u) sub[at++] = first + w;
     }
-    at_full += full;
-    at_part += !full;
-    at_live += whole && !full;
+    if (out.part_idx && st != 0u && !full) out.part_idx[lb * P.NB + at_part + __popc(b_any & ~b_full & below)] = qb;
+    if (out.full_idx && full) out.full_idx[lb * P.NB + at_full + __popc(b_full & below)] = qb;
+    at_part += __popc(b_any & ~b_full);
+    at_full += __popc(b_full);
+    at_live += __popc(b_whole & ~b_full);
   }
-  const int n_vt = (n_subs + kStretches - 1) / kStretches;
-  if (lane < kStretches * n_vt - n_subs) sub[n_subs + lane] = kStretches * P.NB;
-  if (out.part_idx) for (int c = n_part + lane; c < P.NB; c += 32) out.part_idx[lb * P.NB + c] = -1;
-  if (out.full_idx) for (int c = n_full + lane; c < P.NB; c += 32) out.full_idx[lb * P.NB + c] = -1;
-  if (lane == 0) {
+  const int t = threadIdx.x % (32 * kWarps), n_vt = (n_subs + kStretches - 1) / kStretches;
+  if (t < kStretches * n_vt - n_subs) sub[n_subs + t] = kStretches * P.NB;
+  if (out.part_idx) for (int c = n_part + t; c < P.NB; c += 32 * kWarps) out.part_idx[lb * P.NB + c] = -1;
+  if (out.full_idx) for (int c = n_full + t; c < P.NB; c += 32 * kWarps) out.full_idx[lb * P.NB + c] = -1;
+  if (t == 0) {
     P.bwd_cnt[lb] = n_part + n_full;
     P.bwd_tiles[lb] = n_vt;
     if (out.part_cnt) out.part_cnt[lb] = n_part;
@@ -292,13 +317,24 @@ __device__ __forceinline__ void stretch_line(const PlanView& P, const ListOutput
   }
 }
 
-// blockIdx.z: 0 lines are q tiles, 1 lines are kv tiles; 2 counts, per pair of adjacent q tiles (2p, 2p+1) -- the forward's
-// work items, which share one stream of K/V tiles -- the kv tiles at least one of the two reads.
+// Blocks of a batch element: first the lines of kv tiles, one each where four warps share them and four otherwise, then four lines of q tiles each; the rest count, per pair of adjacent q tiles (2p, 2p+1) -- the forward's work items, which share one stream of K/V
+// tiles -- the kv tiles at least one of the two reads, four pairs each.
+__host__ __device__ inline bool kv_line_a_block(const PlanView& P) { return P.bwd_sub != nullptr && P.NB > kOneWarpTiles; }
+static int lists_blocks(const PlanView& P) {
+  const int four = (P.NB + 3) / 4;
+  return (kv_line_a_block(P) ? P.NB : four) + four + ((P.NB + 1) / 2 + 3) / 4;
+}
 __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_out, ListOutputs bwd_out) {
-  const int transposed = blockIdx.z;
-  const int line = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, lane = threadIdx.x & 31;
+  const int four = (P.NB + 3) / 4, kv_blocks = kv_line_a_block(P) ? P.NB : four;
+  const bool transposed = (int)blockIdx.x < kv_blocks, pairs = (int)blockIdx.x >= kv_blocks + four;
+  const int b = blockIdx.y, lane = threadIdx.x & 31;
+  const int line = (blockIdx.x - (transposed ? 0 : pairs ? kv_blocks + four : kv_blocks)) * 4 + (threadIdx.x >> 5);
   after_previous();
-  if (transposed == 2) {
+  if (transposed && kv_line_a_block(P)) {
+    stretch_line<4>(P, bwd_out, b, blockIdx.x);
+    return;
+  }
+  if (pairs) {
     const int NP = (P.NB + 1) / 2;
     if (line >= NP) return;
     const uint8_t* s0 = P.state + ((size_t)b * P.NB + 2 * line) * P.NB;
@@ -316,7 +352,7 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
   int32_t* full_idx = transposed ? bwd_out.full_idx : fwd_out.full_idx;
   if (line >= P.NB) return;
   if (transposed && P.bwd_sub != nullptr) {
-    stretch_line(P, bwd_out, b, line, lane);
+    stretch_line<1>(P, bwd_out, b, line);
     return;
   }
   const size_t lb = (size_t)b * P.NB + line;
@@ -423,6 +459,8 @@ cudaError_t launch_segment_ids(const int32_t* bounds, const int32_t* ids, int n_
 
 // The four launches depend on one another and take a few microseconds each, so each starts while the one before still runs
 // (launch.cuh): with the lists' loads ahead and the shared ranking 29.0 -> 24.3-25.8 us a call at B = 2, T = 32768 with explicit lists.
+// Without them, linked, us: 4096 11.4, 16384 15.1, 32768 19.4, two of them 22.9, four 31.1, 65536 29.6.  What the backward's gathered tiles need of it
+// (masks by stretch and live stretches in `state`, their lines in `lists`) is 0 to 2 of that.
 // Host entry: fills the plan; optional BlockMask-shaped outputs may be null.
 cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t* kv_cnt, int32_t* kv_idx,
                              int32_t* full_cnt, int32_t* full_idx, int32_t* q_cnt, int32_t* q_idx, int32_t* full_q_cnt,
@@ -433,7 +471,7 @@ cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t
   runs_kernel<<<dim3(P.NB + t_words * ((64 * M.W + 127) / 128), P.B), 128, 0, stream>>>(P, M, t_words);
   cudaError_t e = launch_after(state_kernel, dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream, P, M, state_out);
   if (e == cudaSuccess)
-    e = launch_after(lists_kernel, dim3((P.NB + 3) / 4, P.B, 3), 128, 0, stream, P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
+    e = launch_after(lists_kernel, dim3(lists_blocks(P), P.B), 128, 0, stream, P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
                      ListOutputs{q_cnt, q_idx, full_q_cnt, full_q_idx});
   if (e == cudaSuccess) e = launch_after(order_kernel, dim3((P.NB + kOrderTiles - 1) / kOrderTiles, P.B, 3), 256, 0, stream, P, t ? M.R : 0);
   const cudaError_t last = cudaGetLastError();

@@ -54,9 +54,9 @@ def test_stretches_against_the_dense_mask(t, median, lo):
         _check_lines(plan, b, 2, nb, live, full)
 
 
-@pytest.mark.parametrize("nb", [31, 32, 33, 255, 511, 512])
+@pytest.mark.parametrize("nb", [31, 32, 33, 64, 65, 128, 129, 255, 511, 512])
 def test_stretches_of_long_sequences(nb):
-    """Around the tiles that a lane owns and at the most that the table covers, documents alone."""
+    """Around the tiles of a warp's sweep, where one warp a line becomes four, and at the most that the table covers, documents alone."""
     from tagseq2tagseq_b200 import build_block_map
     t = 128 * nb - 70
     doc = torch.arange(t, device="cuda", dtype=torch.int32) // 1111

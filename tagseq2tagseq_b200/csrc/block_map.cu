@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView P, ListOutputs fwd_
 
 // Heaviest-first order inside each batch element: rank by descending count, ties by index.  Eight lanes share a tile and
 // compare its count with an eighth of the others each.
-// which = 0: q tiles by fwd_cnt, 1: kv tiles by bwd_cnt, 2: q-tile pairs by pair_cnt.
+// which = 0: q tiles by fwd_cnt, 1: kv tiles by the query tiles the backward walks for them, 2: q-tile pairs by pair_cnt.
 constexpr int kOrderLanes = 8, kOrderTiles = 256 / kOrderLanes;
 __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows) {
   const int b = blockIdx.y, which = blockIdx.z, sub = threadIdx.x % kOrderLanes;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows)
   }
   const int n = which == 2 ? (P.NB + 1) / 2 : P.NB;
   if ((int)blockIdx.x * kOrderTiles >= n) return;
-  const int32_t* cnt = (which == 2 ? P.pair_cnt : which == 1 ? P.bwd_cnt : P.fwd_cnt) + (size_t)b * n;
+  const int32_t* cnt = (which == 2 ? P.pair_cnt : which == 0 ? P.fwd_cnt : P.bwd_sub != nullptr ? P.bwd_tiles : P.bwd_cnt) + (size_t)b * n;
   int32_t* order = (which == 2 ? P.pair_order : which == 1 ? P.bwd_order : P.fwd_order) + (size_t)b * n;
   __shared__ int4 s_cnt[256];  // 1024 counts at a time
   const int ci = i < n ? cnt[i] : 0;

@@ -33,6 +33,8 @@ def _check_lines(plan, b, B, nb, live, full):
         want = np.concatenate([want, np.full(-want.size % 4, 4 * nb)]).reshape(-1, 4)
         assert tiles[kb] == len(want) and np.array_equal(sub[at:at + len(want)], want), kb
         at += nb - kb
+    order = _plan_part(plan, B, nb, "bwd_order").view(np.int32)[b]
+    assert np.array_equal(order, np.argsort(-tiles, kind="stable"))       # most of these tiles first, ties by number
 
 
 @pytest.mark.parametrize("t", [1, 31, 32, 33, 96, 97, 128, 129, 700, 2047])

@@ -68,7 +68,7 @@ struct PlanLayout {
   size_t fwd_cnt;     // int32[B,NB]      non-skipped kv tiles of q tile qb
   size_t fwd_idx;     // int32[B,NB,NB]   ascending kb, kFullBit set when full
   size_t bwd_cnt;     // int32[B,NB]      non-skipped q tiles of kv tile kb
-  size_t bwd_idx;     // int32[B,NB,NB]   ascending qb, kFullBit set when full; written where bwd_sub does not exist
+  size_t bwd_idx;     // int32[B,NB,NB]   ascending qb, kFullBit set when full; written and read only where bwd_sub does not exist, idle space elsewhere
   size_t fwd_order;   // int32[B,NB]      q tiles of batch b by descending fwd_cnt
   size_t bwd_order;   // int32[B,NB]      kv tiles of batch b by descending bwd_tiles, or bwd_cnt where that does not exist
   size_t pair_cnt;    // int32[B,NP]      NP = ceil(NB/2): kv tiles that q tile 2p or 2p+1 reads (forward work items)

@@ -34,11 +34,9 @@ def test_launch_orders_are_permutations_by_descending_count(nb):
     doc = _two_packs(128 * nb - 5)
     bm = build_block_map(doc, with_lists=True)
     words, at, part = bm.plan.cpu().view(torch.int32).numpy(), 256, {}
-    pairs, tri = (nb + 1) // 2, nb * (nb + 1) // 2 if nb <= 512 else 0   # the last tables exist up to 512 tiles
+    pairs = (nb + 1) // 2
     for name, count, size in (("run_cnt", nb, 4), ("runs", nb * 128, 16), ("state", nb * nb, 1), ("fwd_cnt", nb, 4), ("fwd_idx", nb * nb, 4),  # csrc/plan.h
-                              ("bwd_cnt", nb, 4), ("bwd_idx", nb * nb, 4), ("fwd_order", nb, 4), ("bwd_order", nb, 4), ("pair_cnt", pairs, 4), ("pair_order", pairs, 4),
-                              ("link_t", 1024 * 16 * 2, 4), ("run_mask", nb * 8 * 4, 4), ("q_mask", tri * 8 * 4, 4), ("kv_mask", tri * 8 * 4, 4), ("bwd_sub", tri * 2, 4),
-                              ("bwd_tiles", nb, 4))[:18 if tri else 12]:
+                              ("bwd_cnt", nb, 4), ("bwd_idx", nb * nb, 4), ("fwd_order", nb, 4), ("bwd_order", nb, 4), ("pair_cnt", pairs, 4), ("pair_order", pairs, 4)):
         part[name] = words[at // 4:at // 4 + 2 * count].reshape(2, count) if size == 4 else None
         at = -(-(at + 2 * count * size) // 256) * 256
     for b in range(2):
@@ -46,5 +44,4 @@ def test_launch_orders_are_permutations_by_descending_count(nb):
         both = np.pad(live, ((0, nb % 2), (0, 0))).reshape(pairs, 2, nb).any(axis=1)
         for name, cnt in (("fwd", live.sum(axis=1)), ("bwd", live.sum(axis=0)), ("pair", both.sum(axis=1))):
             assert np.array_equal(part[name + "_cnt"][b], cnt), name
-            weight = part["bwd_tiles"][b] if name == "bwd" and tri else cnt          # the gathered tiles that the backward walks
-            assert np.array_equal(part[name + "_order"][b], np.argsort(-weight, kind="stable")), name
+            assert np.array_equal(part[name + "_order"][b], np.argsort(-cnt, kind="stable")), name

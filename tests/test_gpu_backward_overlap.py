@@ -32,3 +32,31 @@ def test_back_to_back_calls_agree(h, t, d):
         want = alone[i % 2]
         assert torch.equal(dk, want[1]) and torch.equal(dv, want[2])
         assert ((dq.float() - want[0].float()).abs() / want[0].float().abs().clamp_min(1e-2)).max().item() <= 2 ** -6
+
+
+def test_calls_on_two_streams_agree():
+    """Short backwards on two streams at once, each with a plan and inputs of its own: what either overlaps with is its own stream's launch."""
+    from tagseq2tagseq_b200 import build_block_map, read_status, synth
+    from tagseq2tagseq_b200.attention import _attn_bwd, _attn_fwd
+    dev, calls = torch.device("cuda"), []
+    for seed, (h, t, d) in enumerate([(4, 900, 64), (2, 1500, 128)]):
+        doc, link = synth.stack_packs([synth.make_pack(seed + 1, t, 150, 16, 600, p_link=0.2)])
+        doc, link = torch.from_numpy(doc).to(dev), torch.from_numpy(link).to(dev)
+        plan = build_block_map(doc, link).plan
+        g = torch.Generator(device=dev).manual_seed(seed)
+        q, k, v, do = (torch.randn(1, h, t, d, device=dev, generator=g).bfloat16() for _ in range(4))
+        out, lse = _attn_fwd(q, k, v, doc, link, None, None, plan, d ** -0.5)
+        calls.append((q, k, v, out, do, lse, doc, link, None, None, plan, d ** -0.5))
+    alone = [_attn_bwd(*c) for c in calls]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in calls], [[], []]
+    for _ in range(20):
+        for i, c in enumerate(calls):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(_attn_bwd(*c))
+    torch.cuda.synchronize()
+    for i, c in enumerate(calls):
+        assert read_status(c[10]) == 0
+        for dq, dk, dv in got[i]:
+            assert torch.equal(dk, alone[i][1]) and torch.equal(dv, alone[i][2])
+            assert ((dq.float() - alone[i][0].float()).abs() / alone[i][0].float().abs().clamp_min(1e-2)).max().item() <= 2 ** -6

@@ -56,6 +56,55 @@ def test_stretches_against_the_dense_mask(t, median, lo):
         _check_lines(plan, b, 2, nb, live, full)
 
 
+@pytest.mark.parametrize("t", [97, 128, 700, 1500, 2047])
+@pytest.mark.parametrize("classes", [5, 40, 300])
+def test_stretches_of_classes_that_change_inside_documents(t, classes):
+    """Row and column classes with borders of their own, some of them no class, and few documents: the stretches that count are those of the
+    row class; the backward over them agrees with the dense mask in 64 bits (gradients are bf16, their sums of bf16 products)."""
+    from oracle import masks as om
+    from tagseq2tagseq_b200 import build_block_map, read_status
+    from tagseq2tagseq_b200.attention import masked_attn
+    rng = np.random.default_rng(t + classes)
+    def ids(n):
+        cuts = np.sort(rng.choice(np.arange(1, t), min(n, t) - 1, replace=False))
+        return np.repeat(rng.permutation(min(n, t)), np.diff(np.concatenate([[0], cuts, [t]]))).astype(np.int32)
+    doc, row, col = ids(max(2, classes // 8)), ids(classes), ids(classes)
+    row[row % 7 == 3] = -1
+    col[col % 5 == 2] = -1
+    r, w = max(1, classes), -(-max(1, classes) // 64)
+    bits = rng.random((r, 64 * w)) < 0.1
+    link = np.array([[int(np.packbits(bits[i, 64 * j:64 * j + 64], bitorder="little").view(np.int64)[0]) for j in range(w)] for i in range(r)], np.int64)
+    dense = om.class_mask_dense(doc, row, col, link)
+    dev = [torch.from_numpy(x)[None].cuda() for x in (doc, link, row, col)]
+    plan, nb = build_block_map(*dev).plan, (t + 127) // 128
+    ok = np.zeros((128 * nb, 128 * nb), bool)
+    ok[:t, :t] = _before_causality(doc, row, col, link)
+    low = np.tril(np.ones((nb, nb), bool))
+    live, full = ok.reshape(4 * nb, 32, nb, 128).any(axis=(1, 3)) & low.repeat(4, axis=0), ok.reshape(nb, 128, nb, 128).all(axis=(1, 3)) & np.tril(low, -1)
+    runs = _plan_part(plan, 1, nb, "run_cnt").view(np.int32)[0]
+    for kb in np.flatnonzero(runs > 8):
+        live[:, kb] = live[:, kb].reshape(nb, 4).any(axis=1).repeat(4) & (np.arange(4 * nb) * 32 < t)
+    _check_lines(plan, 0, 1, nb, live, full)
+    g = torch.Generator(device="cuda").manual_seed(t)
+    q, k, v, do = (torch.randn(1, 2, t, 64, device="cuda", generator=g).bfloat16() for _ in range(4))
+    qd, kd, vd = (x.clone().requires_grad_(True) for x in (q, k, v))
+    out, _ = masked_attn(qd, kd, vd, dev[0], dev[1], q_row_ids=dev[2], kv_col_ids=dev[3], plan=plan)
+    out.backward(do)
+    assert read_status(plan) == 0
+    q6, k6, v6 = (x.double().requires_grad_(True) for x in (q, k, v))
+    s = (q6 @ k6.transpose(-1, -2) / 8).masked_fill(~torch.from_numpy(dense).cuda(), float("-inf"))
+    (torch.softmax(s, -1) @ v6).backward(do.double())
+    for got, want in ((qd.grad, q6.grad), (kd.grad, k6.grad), (vd.grad, v6.grad)):
+        assert (got.double() - want).norm() <= 1e-2 * want.norm()
+
+
+def _before_causality(doc, row, col, link):
+    """[T, T] of who may read whom, above the diagonal as well: the pre-pass leaves causality inside the diagonal tile to its readers."""
+    table = np.zeros((link.shape[0] + 1, 64 * link.shape[1] + 1), bool)
+    table[:-1, :-1] = np.unpackbits(link.view(np.uint8), axis=1, bitorder="little").astype(bool)
+    return (doc[:, None] == doc[None]) | table[row][:, col]
+
+
 @pytest.mark.parametrize("nb", [31, 32, 33, 64, 65, 128, 129, 255, 511, 512])
 def test_stretches_of_long_sequences(nb):
     """Around the tiles of a warp's sweep, where one warp a line becomes four, and at the most that the table covers, documents alone."""

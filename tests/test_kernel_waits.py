@@ -74,13 +74,15 @@ def test_scores_overwrite_the_probabilities_of_the_last_tile_once_their_product_
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [64, 128])
-def test_a_list_entry_that_is_no_tile_ends_in_a_status(d):
-    """The forward's own check of its lists: the block that meets the entry (as its second or a later item) drains and leaves, the
-    code is in the status word, and the plan built again serves the next call."""
+# pairs of query tiles; query tiles that two teams share, and those as the lists call for them, the entry one of either team's
+@pytest.mark.parametrize("h,place", [(16, 1), (4, 0), (4, 1), (4, 2), (8, 1), (8, 2)])
+def test_a_list_entry_that_is_no_tile_ends_in_a_status(d, h, place):
+    """The forward's own check of its lists: the block that meets the entry (as its second or a later item, or its only one) drains and
+    leaves, the code is in the status word, the same plan with the entry put right serves the next call, and a plan built again too."""
     import torch
     from tagseq2tagseq_b200 import build_block_map, read_status
     from tagseq2tagseq_b200.attention import masked_attn
-    t, h, nb = 4096, 16, 32
+    t, nb = 4096, 32
     dev = torch.device("cuda")
     doc = torch.zeros((1, t), dtype=torch.int32, device=dev)
     g = torch.Generator(device=dev).manual_seed(1)
@@ -93,8 +95,13 @@ def test_a_list_entry_that_is_no_tile_ends_in_a_status(d):
     cnt = plan.view(torch.int32)[at // 4:at // 4 + nb]
     lists = plan.view(torch.int32)[(at + 256) // 4:][:nb * nb].view(nb, nb)
     assert cnt.tolist() == list(range(1, nb + 1)) and (lists[3, :4] & ~(1 << 30)).tolist() == [0, 1, 2, 3]
-    lists[2, 1] = nb + 5                                        # of the last pair but one in the order of launch
+    right = lists[2, place].item()
+    lists[2, place] = nb + 5                                    # of the last pair but one in the order of launch
     masked_attn(q, k, v, doc, plan=plan)
     assert read_status(plan) in (1014, 1038)                    # the producer or a softmax warp, whoever came first
+    assert plan.view(torch.int32)[8:10].tolist() == [0, 0]      # the counters that items are drawn from start again
+    lists[2, place] = right
+    out, lse = masked_attn(q, k, v, doc, plan=plan)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
     out, lse = masked_attn(q, k, v, doc, plan=build_block_map(doc).plan)
     assert torch.equal(out, want) and torch.equal(lse, want_lse)

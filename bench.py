@@ -52,6 +52,15 @@ def measured_traffic():
             "source": f"ncu capture of {d['workload']} at commit {d['commit']}"}
 
 
+def gathered_tiles(plan, B, T):
+    """Query tiles that the backward walks: the sum over the plan's last table (int32 [B, T / 128], csrc/plan.h, up to 512 tiles)."""
+    import torch
+    nb = -(-T // 128)
+    assert nb <= 512
+    at = plan.numel() - -(-4 * B * nb // 256) * 256
+    return int(plan[at:at + 4 * B * nb].view(torch.int32).sum().item())
+
+
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -204,7 +213,8 @@ def run_ours(args, rank, world, device):
     fms, bms = ctypes.c_float(0), ctypes.c_float(0)
     for m in masks:
         bml = build_block_map(m["doc"], m["link"], with_lists=True)
-        m["tiles"] = int((bml.q_cnt.sum() + bml.full_q_cnt.sum()).item())  # non-skipped 128 x 128 tiles
+        m["tiles"] = int((bml.q_cnt.sum() + bml.full_q_cnt.sum()).item())  # non-skipped 128 x 128 tiles, which the forward computes
+        m["bwd_tiles"] = gathered_tiles(bml.plan, *m["doc"].shape)
         del bml
         f_list, b_list, pp_list = [], [], []
         for _ in range(max(3, min(args.steps, 5))):
@@ -217,7 +227,8 @@ def run_ours(args, rank, world, device):
             L.ts2ts_profile_last_ms(0, ctypes.byref(fms)); L.ts2ts_profile_last_ms(1, ctypes.byref(bms))
             f_list.append(fms.value); b_list.append(bms.value); pp_list.append(pe0.elapsed_time(pe1))
         per_mask.append({"mask": m["name"], "density": round(m["density"], 4), "tiles": m["tiles"],
-                         "executed_over_algorithmic": m["tiles"] * 16384.0 / m["pairs"], "fwd_ms": statistics.mean(f_list),
+                         "executed_over_algorithmic": m["tiles"] * 16384.0 / m["pairs"], "bwd_tiles": m["bwd_tiles"],
+                         "bwd_executed_over_algorithmic": m["bwd_tiles"] * 16384.0 / m["pairs"], "fwd_ms": statistics.mean(f_list),
                          "bwd_ms": statistics.mean(b_list), "prepass_ms": statistics.median(pp_list), "fwd_tflops": 4.0 * D * H * m["pairs"] / statistics.mean(f_list) / 1e9,
                          "bwd_tflops": 10.0 * D * H * m["pairs"] / statistics.mean(b_list) / 1e9})
     L.ts2ts_profile_enable(0)
@@ -345,9 +356,10 @@ def run_ours(args, rank, world, device):
                      "fwd": {"achieved": sum(4.0 * D * H * m["pairs"] for m in masks) / sum(p["fwd_ms"] for p in per_mask) / 1e9,
                              "frac": sum(4.0 * D * H * m["pairs"] for m in masks) / sum(p["fwd_ms"] for p in per_mask) / 1e9 / peak_tf,
                              "avg_launch_ms": statistics.mean(p["fwd_ms"] for p in per_mask),
-                             "traffic": None if traffic is None else traffic["fwd_bytes_per_bht"] * (B * H * T)},
-                     # executed = every element of a non-skipped 128 x 128 tile counted, masked or not
-                     "executed_over_algorithmic_flops": sum(m["tiles"] for m in masks) * 16384.0 / sum(m["pairs"] for m in masks)},
+                             "traffic": None if traffic is None else traffic["fwd_bytes_per_bht"] * (B * H * T),
+                             "executed_over_algorithmic_flops": sum(m["tiles"] for m in masks) * 16384.0 / sum(m["pairs"] for m in masks)},
+                     # executed = every element of the 128 x 128 tiles that the kernel walks counted, masked or not
+                     "executed_over_algorithmic_flops": sum(m["bwd_tiles"] for m in masks) * 16384.0 / sum(m["pairs"] for m in masks)},
     }
     if world == 1:
         line["cpu_baseline"] = cpu_baseline(steps=5)

@@ -45,6 +45,27 @@ def test_forward_of_short_launches(b, h, t, d, kind):
     assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("t,few,many", [(506, 2, 75), (1024, 4, 38), (2048, 8, 20)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_sharing_a_query_tile_costs_no_precision(t, few, many, d):
+    """The same heads in a launch that shares query tiles and in one that has a team add up a row alone, against 64 bits: the split is no
+    further off, neither in the row sums nor in the result (five seeds together: what one rounding more or less decides averages out)."""
+    from tagseq2tagseq_b200 import build_block_map
+    from tagseq2tagseq_b200.attention import masked_attn
+    dev = torch.device("cuda")
+    doc = torch.zeros((1, t), dtype=torch.int32, device=dev)
+    plan, off = build_block_map(doc).plan, torch.zeros(2, 2, dtype=torch.float64, device=dev)
+    for seed in range(5):
+        g = torch.Generator(device=dev).manual_seed(seed)
+        q, k, v = (torch.randn(1, many, t, d, device=dev, generator=g).bfloat16() for _ in range(3))
+        s = ((q[:, :few].double() @ k[:, :few].double().transpose(-1, -2)) * d ** -0.5).masked_fill(~torch.ones(t, t, dtype=torch.bool, device=dev).tril(), float("-inf"))
+        want, want_lse = torch.softmax(s, -1) @ v[:, :few].double(), torch.logsumexp(s, -1)
+        for i, n in enumerate((few, many)):
+            out, lse = masked_attn(q[:, :n], k[:, :n], v[:, :n], doc, plan=plan)
+            off[i] += torch.stack([(lse[:, :few].double() - want_lse).square().sum(), (out[:, :few].double() - want).square().sum()])
+    assert (off[0] <= off[1]).all(), (off[0] / off[1]).sqrt().tolist()
+
+
 # around 32 tiles and the most pairs and tiles that run at once (148 SMs): one and several elements, one head and several
 @pytest.mark.parametrize("b,h,t", [(1, 9, 4096), (1, 9, 3969), (3, 3, 4096), (1, 2, 18900), (1, 1, 37800)])
 @pytest.mark.parametrize("d", [64, 128])

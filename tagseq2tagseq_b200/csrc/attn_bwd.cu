@@ -4,8 +4,8 @@
 //   bwd_prep     delta[q] = sum_d O[q,d] dO[q,d],  lse2[q] = LSE[q] * log2(e)   (fp32, side by side for every 32 queries, padded to
 //                whole tiles); zeroes dQ
 //   attn_bwd     one CTA per 128-key tile of one (batch, head); walks 128-query tiles gathered from the stretches of 32
-//                query rows that hold an allowed pair (PlanLayout::bwd_sub; 11 % fewer tiles on the linked packs, linked 16k, H = 16:
-//                D = 128 1004 -> 956 us, H = 12, D = 64 503 -> 471, warm and at the power limit).  Scores are transposed so that a tensor-memory lane is a key row:
+//                query rows that hold an allowed pair (PlanLayout::bwd_sub; 9-19 % fewer tiles on linked 16k packs, 4-11 % on linked 32k ones; linked 16k,
+//                H = 16: D = 128 1004 -> 956 us, H = 12, D = 64 503 -> 471, warm and at the power limit).  Scores are transposed so that a tensor-memory lane is a key row:
 //                  tcgen05  S^T = K Q^T,  dP^T = V dO^T            [128 keys x 128 queries, fp32 in TMEM]
 //                  warps 0-7 (two threads per key row, 64 queries each), in two phases:
 //                           P^T = exp2(scale S^T - lse2[q]) under the mask, as soon as S^T is complete, written as
@@ -71,7 +71,7 @@ struct BwdParams {
   TS2TS_BWD_TRACE_FIELDS
 };
 
-constexpr int kBwdThreads = 512;  // warps 0-7 exp/dS, 8-11 dQ reduction, 12 TMA producer, 13 MMA issuer, 14-15 idle
+constexpr int kBwdThreads = 512;  // warps 0-7 exp/dS, 8-11 dQ reduction, 12 and 14 TMA producers, 13 MMA issuer, 15 idle
 constexpr int kSubQ = 64;         // query columns per compute half
 
 template <int D>
@@ -405,8 +405,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const uint32_t k_mn = desc_lo(smem_u32(sK), 16384), ds_mn = desc_lo(smem_u32(sDS), 16384);
       auto kstep = [](int kk) -> uint32_t { return ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4; };  // 16 elements along a K-major operand
       // Shared-memory accesses of this thread (barrier waits included) queue behind the MMAs it has issued and only
-      // proceed once the tensor pipe has accepted those.  So every group asks, two MMAs before its end, whether what the
-      // next group waits for has arrived already (`early`): the pipe stays fed while the answer comes.
+      // proceed once the tensor pipe has accepted those.  So a group asks, two MMAs before its end, whether what the
+      // next group waits for has arrived already (`early`): the pipe stays fed while the answer comes.  dK does not ask: at D = 128 dQ
+      // follows, which waits for nothing more, and at D = 64, where dK is the last group, the question for dO comes behind it; the next
+      // group there waits for dQ to be read out in any case, and dO has two buffers.
       bool early_p = false, early_q = false, early_ds = false, early_do = false;
       auto q_full = [&](int i) { return mbar_test_wait(&bar_q_full[i % Cfg::kQStages], (i / Cfg::kQStages) & 1); };
       auto do_full = [&](int i) { return mbar_test_wait(&bar_do_full[i % Cfg::kDoStages], (i / Cfg::kDoStages) & 1); };
@@ -852,11 +854,13 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
     p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
   }
   BTRACE_ATTACH(p, stream);
-  // The three launches overlap (launch.cuh) where they are short: the main kernel's blocks set themselves up and bring in K, V, Q and dO
+  // The three launches overlap (launch.cuh) where they are short: the main kernel's blocks set themselves up and bring in K and V
   // under the preparation, the conversion's blocks wait where SMs have run dry.  us, one after the other -> overlapping: linked 600, H = 8,
   // D = 64 23.0 -> 16.7; linked 1024, H = 4, D = 64 29.1 -> 22.9; causal 2 x 1000, H = 8, D = 128 38.7 -> 35.3; linked 5003, H = 12, D = 64 72.8 -> 66.9;
-  // causal 4096, H = 8, D = 128 95.9 -> 89.4.  Long launches lose by it: linked 8k, H = 8, D = 128 (512 tiles) 140.6 -> 142.6; linked 16k, H = 16, D = 128
-  // 968 -> 988, H = 12, D = 64 (1536 tiles) 457 -> 461.
+  // causal 4096, H = 8, D = 128 95.9 -> 89.4.  At the line, D = 128, 384 tiles: documents 6144, H = 8 80.5 -> 75.7,
+  // linked 4096, H = 12 99.3 -> 97.8 (288 tiles 82.4 -> 81.4, 320 84.6 -> 85.5); D = 64, 768 tiles: linked 8k, H = 12 144.3 -> 141.1, documents 93.5 -> 88.3.
+  // Beyond it the gain ends, and long launches lose: linked 8k, H = 8, D = 128 (512 tiles) 140.6 -> 142.6, H = 14 and 16, D = 64 (896 and 1024 tiles)
+  // 170.2 -> 171.0 and 183.4 -> 183.0; linked 16k, H = 16, D = 128 968 -> 988, H = 12, D = 64 (1536 tiles) 457 -> 461.
   const bool early = (long long)B * H * P.NB * D <= 384 * 128;
   cudaError_t launched;
   {

@@ -19,12 +19,13 @@
 // tensor memory has room for it (S0 | S1 | O0 | O1 | P0 | P1), which takes 128 KB a pair of tiles out of the shared-memory
 // pipe that the MMA operands fill (H = 16, causal 4k batch 4: 239 -> 222 us, linked 16k: 370 -> 348).  At D = 128 it has not: with P
 // over its own scores a team waited 1570 clocks a tile for S where it waits 240 (causal 4k); with P in tensor memory and one score buffer
-// for both teams causal 4k batch 4 took 296 us instead of 304, but linked 16k 408 instead of 390 and two linked 32k packs 4230 instead of
-// 4150, because teams whose tiles differ then wait for each other's reads.
+// for both teams causal 4k batch 4 took 296 us instead of 304, but linked 16k 406 instead of 390 and two linked 32k packs 4160 instead of
+// 4125, because teams whose tiles differ then wait for each other's reads.
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
 // K/V tiles travel through one ring of shared-memory slots in the order K0, K1, V0, K2, V1, ... (K runs one tile
 // ahead of V because S is computed one tile ahead of P V).  Short launches have the teams share a query tile instead (launch_fwd_t):
-// the tiles of its list go to them in turn, and team 0 adds up both parts at the end, straight from tensor memory.  At the end of an item each softmax thread reads its
+// the tiles of its list go to them in turn, and team 0 adds up both parts at the end, straight from tensor memory.  A team's next K is then
+// two places ahead in the list and comes behind its current V, so its S is not computed ahead: part of what a shared tile costs.  At the end of an item each softmax thread reads its
 // row of O out of tensor memory and frees it for the next item; the normalised rows leave through shared memory and TMA stores, a
 // warp's 32 rows at a time, while the issuers already work on the next item.
 //
@@ -66,10 +67,12 @@
 #define TS2TS_FWD_GROUP_MB 136
 #endif
 #ifndef TS2TS_FWD_FOLD_MB
-// K/V bytes of the whole batch up to which its elements are ordered as one, so that the heaviest items of all of them start first:
-// a little under the L2's 126 MB.  us, one after the other -> as one, D = 64 unless noted: causal 4 x 2039, H = 8 56.3 -> 42.7; linked 4 x 14724, H = 3
-// 248 -> 223; D = 128: documents 4 x 3269, H = 8 51.1 -> 47.2; linked 4 x 14414, H = 3 (88 MB) 252 -> 236; linked 4 x 4096, H = 12 (100 MB)
-// 197 -> 172; but causal 4 x 4096, H = 16 (134 MB) 293 -> 308.  The backward gains nothing from it (its blocks are many).
+// K/V bytes of the whole batch (in 2^20) up to which its elements are ordered as one: the first ranks of all of them come before any second
+// one, so that every element's heavy items start early.  A little under the L2's 126e6 bytes.  us, one after the other -> as one, D = 64 unless
+// noted: causal 4 x 2039, H = 8 56.3 -> 42.7; linked 4 x 14724, H = 3 248 -> 223; D = 128: documents 4 x 3269, H = 8 51.1 -> 47.2; linked 4 x 4096, H = 12
+// (96) 197 -> 172, H = 14 (112) 169 -> 145; linked 2 x 16384, H = 6 (96) 323 -> 294.  Even elements gain little or nothing: causal 4 x 4096, H = 13 (104)
+// 245 -> 243, 2 x 8192, H = 10 to 14 (80 to 112) +- 1-2 %, linked 2 x 14336, H = 10 to 14, D = 64 (70 to 98) -1 to +1 %.  Beyond the line: linked 4 x 4096, H = 15 (120)
+// 185 -> 162, but causal 4 x 4096, H = 16 (128) 293 -> 308.  The backward gains nothing from it (its blocks are many).
 #define TS2TS_FWD_FOLD_MB 112
 #endif
 

@@ -79,8 +79,8 @@ struct PlanLayout {
   size_t kv_mask;     // uint32[B,NB(NB+1)/2,kStretches,kMaskRuns]; absent above kMaskMaxTiles
   // The query tiles the backward walks for a kv tile, four stretches each.  Full q tiles come first, then partial ones whose
   // stretches are all live, each as it lies in memory; then the live stretches of the others, gathered, so that stretches without
-  // an allowed pair take no part (linked 16k packs: 2743 tile pairs become 2450 tiles, of which 392 are gathered; linked 32k
-  // 15099 and 13458).  All ascend; the last tile is filled up with stretch number kStretches * NB, which lies past the sequence.
+  // an allowed pair take no part (linked 16k packs of the training sizes: 2743 tile pairs become 2450 tiles, of which 392 are gathered,
+  // and 2657 become 2151; linked 32k, documents up to 2048, 15099 become 13458, up to 8192 13948 become 12828).  All ascend; the last tile is filled up with stretch number kStretches * NB, which lies past the sequence.
   size_t bwd_sub;     // uint16[B,NB(NB+1)/2,kStretches]   lines by sub_line(); stretch numbers
   size_t bwd_tiles;   // int32[B,NB]      tiles of each line; both absent above kMaskMaxTiles
   size_t bytes;

@@ -75,7 +75,8 @@ int ts2ts_block_map(const int32_t* doc_ids, const int32_t* q_row_ids, const int3
 int ts2ts_segment_ids(const int32_t* bounds, const int32_t* ids, int n_seg, int T, int32_t* out, void* stream);
 
 /* Forward: out = softmax(scale * q k^T + mask) v, lse = natural-log row sums, fp32 [B,H,T].
- * A row with no allowed key gets out = 0 and lse = -inf.  Replaces the forward of
+ * A row with no allowed key gets out = 0 and lse = -inf.  A call repeats itself bit for bit; how a sequence's rows are rounded
+ * depends on B, H and T, and in middle-sized calls on the mask (short launches add a row up in two parts).  Replaces the forward of
  * flex_attention(q, k, v, block_mask=...) (torch/nn/attention/flex_attention.py:1468). */
 int ts2ts_attn_fwd(const void* q, const void* k, const void* v, const int64_t* q_strides, const int64_t* k_strides,
                    const int64_t* v_strides, int B, int H, int T, int D, float scale, const int32_t* doc_ids,

@@ -246,8 +246,21 @@ __device__ __noinline__ uint4 row_mask(const PlanView& P, const MaskArgs& M, int
   return make_uint4(bits[0], bits[1], bits[2], bits[3]);
 }
 
+// The last CTA to leave puts the ticket counter back to zero for the next launch.
+__device__ __forceinline__ void fwd_leave(const PlanView& P) {
+  __threadfence();
+  const int done = atomicAdd(&P.status[kFwdDone], 1);
+  if (done == static_cast<int>(gridDim.x) - 1) {
+    P.status[kFwdTicket] = 0;
+    P.status[kFwdDone] = 0;
+    __threadfence();
+  }
+}
+
 // kShared: the two teams of a CTA share a query tile and take its key tiles in turn, instead of a query tile of a pair each.
-template <int D, bool kShared>
+// kIdle: the grid may have more CTAs than items; those leave at once, but behind the look at the plan's stamp, because a plan that is
+// refused must not keep a part of the count.
+template <int D, bool kShared, bool kIdle = false>
 __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtensorMap& mapK, const CUtensorMap& mapV, const CUtensorMap& mapO, const FwdParams& p) {
   using Cfg = FwdSmem<D>;
   constexpr int kStages = Cfg::kStages;
@@ -289,6 +302,10 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
       if (tid == 0) atomicCAS(P.status, 0, bad);
       return;
     }
+  }
+  if (kIdle && static_cast<int>(blockIdx.x) >= (kShared ? p.n_tiles : p.n_pairs)) {
+    if (tid == 0) fwd_leave(P);
+    return;
   }
   if (tid == 0) {
     *abort_w = 0;
@@ -786,15 +803,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
   if (warp == kFwdIssuerWarp) tmem_dealloc(tmem, 512);
-  if (tid == 0) {  // the last CTA to leave puts the ticket counter back to zero for the next launch
-    __threadfence();
-    const int done = atomicAdd(&P.status[kFwdDone], 1);
-    if (done == static_cast<int>(gridDim.x) - 1) {
-      P.status[kFwdTicket] = 0;
-      P.status[kFwdDone] = 0;
-      __threadfence();
-    }
-  }
+  if (tid == 0) fwd_leave(P);
 }
 
 // Which work items a launch has: pairs of query tiles, query tiles that the teams share, or whichever of the two the lists call for.
@@ -804,9 +813,9 @@ enum FwdForm { kFwdPairs, kFwdShared, kFwdByLists };
 // as long as the longest list; shared tiles, two rounds of them, as long as an SM's share of all lists, two key tiles at a time, at 1.6 times
 // the time of a step whose SM has one team to serve, and two steps for the second item.  Both forms measured on 66 calls of 160 to 288 query
 // tiles (D = 64 and 128, longest list 2 to 128): where this line takes the slower one it is by 2 % at most.
-// A kernel with both bodies runs the one that comes first in its code 0.2-0.7 us (1.5 with one head) slower than a kernel of its own, and the other one 2-3 us;
+// A kernel with both bodies runs the one that comes first in its code 0.2-0.6 us slower than a kernel of its own, and the other one 2-3 us;
 // so the pairs, whose launches are the short ones, come first (us, pairs | shared tiles | by the lists: documents of 200 to 300 in 4096, H = 7,
-// D = 128 16.2 | 19.4 | 16.9, D = 64 14.4 | 17.0 | 14.8; causal 4096, H = 8, D = 64 60.5 | 47.6 | 50.5).  One body that asks at run time costs both.
+// D = 128 16.4 | 19.6 | 16.6, D = 64 14.3 | 17.0 | 14.9, of 300 to 600 in 30000, one head 21.8 | 24.2 | 22.0; causal 4096, H = 8, D = 64 60.3 | 47.4 | 50.3).  One body that asks at run time costs both.
 __device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p) {
   return 5 * (p.plan.status[kLongestList] - 2) * static_cast<int>(gridDim.x) > 4 * p.plan.status[kAllLists] * p.H;
 }
@@ -817,7 +826,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
   if (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
   else if (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
-  else if (!lists_call_for_shared(p)) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
+  else if (!lists_call_for_shared(p)) fwd_items<D, false, true>(mapQ, mapK, mapV, mapO, p);
   else fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
 }
 

@@ -94,3 +94,24 @@ def test_the_form_of_middle_launches_follows_the_lists(b, h, t, d, kind):
     assert torch.equal(out[:, :n], want[:, :n]) and torch.equal(lse[:, :n], want_lse[:, :n])
     again, _ = masked_attn(q[:, :h], k[:, :h], v[:, :h], doc, plan=plan)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("kind", ["short", "long"])
+def test_a_refused_plan_serves_its_own_call_afterwards(kind):
+    """Blocks of a middle launch that have no item leave early: not before the plan's stamp is looked at, or a plan of another call would keep
+    a part of their count and start its own next launch with it."""
+    from tagseq2tagseq_b200 import build_block_map, read_status, synth
+    from tagseq2tagseq_b200.attention import masked_attn
+    dev, h = torch.device("cuda"), 8
+    doc = torch.zeros((1, 4224), dtype=torch.int32, device=dev)
+    if kind == "short":
+        doc = torch.from_numpy(synth.stack_packs([synth.make_pack(1, 4224, 60, 16, 200)])[0]).to(dev)
+    g = torch.Generator(device=dev).manual_seed(1)
+    q, k, v = (torch.randn(1, h, 4224, 64, device=dev, generator=g).bfloat16() for _ in range(3))
+    plan = build_block_map(doc).plan
+    want, _ = masked_attn(q, k, v, doc, plan=plan)
+    masked_attn(*(x[:, :, :4096] for x in (q, k, v)), doc[:, :4096].contiguous(), plan=plan)
+    assert read_status(plan) == 1900 and plan.view(torch.int32)[8:10].tolist() == [0, 0]
+    for _ in range(3):
+        out, _ = masked_attn(q, k, v, doc, plan=plan)
+        assert torch.equal(out, want) and plan.view(torch.int32)[8:10].tolist() == [0, 0]

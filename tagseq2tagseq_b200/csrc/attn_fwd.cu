@@ -85,10 +85,11 @@ struct FwdParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_sh, o_st;
   int H;
-  int n_pairs, n_tiles;  // items: B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
+  int n_items;           // B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
   int heads;             // heads of a stretch of the ticket order: H, or B * H where the batch elements are one
   int head_group;        // heads whose items are interleaved in the ticket order
   float scale_log2;      // softmax scale * log2(e)
+  int n_pairs;           // items of a launch that may share tiles and does not
   TS2TS_TRACE_FIELDS
 };
 
@@ -303,7 +304,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
       return;
     }
   }
-  if (kIdle && static_cast<int>(blockIdx.x) >= (kShared ? p.n_tiles : p.n_pairs)) {
+  if (kIdle && static_cast<int>(blockIdx.x) >= p.n_pairs) {
     if (tid == 0) fwd_leave(P);
     return;
   }
@@ -367,7 +368,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
         const uint32_t is = it % kFwdItemSlots;
         if (it >= kFwdItemSlots && !mbar_wait(&bar_item_empty[is], (it / kFwdItemSlots - 1) & 1, abort_v, 12)) break;
         const int ticket = atomicAdd(&P.status[kFwdTicket], 1);
-        const int code = ticket < (kShared ? p.n_tiles : p.n_pairs) ? ticket : -1;
+        const int code = ticket < (kIdle ? p.n_pairs : p.n_items) ? ticket : -1;
         s_item[is] = code;
         mbar_arrive(&bar_item_full[is]);
         if (code < 0) {
@@ -784,8 +785,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
         // One rounding less where the sum is one of two parts, for those that adding them up takes: against 64 bits lse was 1-5 % further off
         // there than in a row that one team adds up (attention at T = 219 to 4096), and is 6-11 % closer now.
         constexpr float kLn2 = 0.6931471805599453f;
-        const float lg = log2f(l);
-        p.lse[((size_t)b * p.H + h) * P.T + q] = !(l > 0.f) ? -CUDART_INF_F : shared ? fmaf(m_used, kLn2, lg * kLn2) : (m_used + lg) * kLn2;
+        p.lse[((size_t)b * p.H + h) * P.T + q] = l > 0.f ? (shared ? fmaf(m_used, kLn2, log2f(l) * kLn2) : (m_used + log2f(l)) * kLn2) : -CUDART_INF_F;
       }
       FTRACE_ACC(4);
     }
@@ -824,8 +824,8 @@ template <int D, int kForm>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
-  if (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
-  else if (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
+  if constexpr (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
+  else if constexpr (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
   else if (!lists_call_for_shared(p)) fwd_items<D, false, true>(mapQ, mapK, mapV, mapO, p);
   else fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
 }
@@ -846,8 +846,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];
   p.H = H; p.scale_log2 = scale * 1.4426950408889634f;
   p.n_pairs = B * H * ((P.NB + 1) / 2);
-  p.n_tiles = B * H * P.NB;
-  const int items = kForm == kFwdPairs ? p.n_pairs : p.n_tiles;
+  p.n_items = kForm == kFwdPairs ? p.n_pairs : B * H * P.NB;
   {  // heads per group, from the K and V bytes of one head (2 x T x D bf16 each)
     const long long kv_bytes = 4ll * T * D;
     long long g = (static_cast<long long>(TS2TS_FWD_GROUP_MB) << 20) / (kv_bytes > 0 ? kv_bytes : 1);
@@ -863,7 +862,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
       return -110;
     attr_done[dev] = true;
   }
-  const unsigned grid = (unsigned)(items < sms ? items : sms);
+  const unsigned grid = (unsigned)(p.n_items < sms ? p.n_items : sms);
   FTRACE_ATTACH(p, stream);
   {
     ProfileScope timed(0, stream);

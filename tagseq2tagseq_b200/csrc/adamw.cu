@@ -6,6 +6,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace ts2ts {
 namespace {
 
@@ -33,6 +35,7 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
   p -= t.step_size * m / (sqrtf(v) * t.inv_sqrt_bc2 + a.eps);
 }
 __global__ void __launch_bounds__(kAdamThreads) adamw_kernel(const __grid_constant__ AdamArgs a) {
+  wait_previous();
   int lo = 0, hi = a.count - 1;  // last tensor whose first block is not after this one
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -101,7 +104,8 @@ cudaError_t launch_adamw(int count, float* const* p, const float* const* g, floa
       }
       ++done;
     }
-    if (blocks > 0) adamw_kernel<<<(unsigned)blocks, kAdamThreads, 0, stream>>>(a);
+    const cudaError_t e = blocks > 0 ? launch_after(adamw_kernel, dim3((unsigned)blocks), kAdamThreads, 0, stream, a) : cudaSuccess;
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }

@@ -68,6 +68,7 @@ struct BwdParams {
   int H, Tp;
   int head_group;        // heads whose CTAs are interleaved in the launch order
   float scale, scale_log2;
+  bool early;            // the conversion may start while this kernel runs
   TS2TS_BWD_TRACE_FIELDS
 };
 
@@ -265,7 +266,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       return;
     }
   }
-  let_next_start();
+  if (p.early) let_next_start();
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -736,10 +737,12 @@ template <int D>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                        const float* __restrict__ lse, int64_t o_sb, int64_t o_sh, int64_t o_st, int64_t d_sb,
                                                        int64_t d_sh, int64_t d_st, int H, int T, int Tp, float* __restrict__ stats,
-                                                       float* __restrict__ dq_acc) {
+                                                       float* __restrict__ dq_acc, bool early) {
   constexpr int kLanes = D / 8, kRows = 256 / kLanes, kEach = kTile / kRows < 4 ? kTile / kRows : 4;  // a block covers kRows * kEach rows of one (b, h)
   const int per_bh = Tp / (kRows * kEach);
-  let_next_start();
+  wait_previous();
+  if (early) let_next_start();
+  out = settled(out); dout = settled(dout); lse = settled(lse);
   const int bh = blockIdx.x / per_bh, t0 = (blockIdx.x - bh * per_bh) * (kRows * kEach);
   const int b = bh / H, h = bh - b * H;
   const int r = threadIdx.x / kLanes, c = threadIdx.x % kLanes;
@@ -840,9 +843,6 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
     attr_done[dev] = true;
   }
   constexpr int kPrepRows = 256 / (D / 8) * (kTile / (256 / (D / 8)) < 4 ? kTile / (256 / (D / 8)) : 4);
-  bwd_prep_kernel<D><<<(unsigned)(rows / kPrepRows), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1],
-      sdo[2], H, T, Tp, stats, dq_acc);
   BwdParams p;
   p.plan = P; p.mask = M; p.stats = stats; p.dq_acc = dq_acc;
   p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
@@ -862,13 +862,15 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
   // Beyond it the gain ends, and long launches lose: linked 8k, H = 8, D = 128 (512 tiles) 140.6 -> 142.6, H = 14 and 16, D = 64 (896 and 1024 tiles)
   // 170.2 -> 171.0 and 183.4 -> 183.0; linked 16k, H = 16, D = 128 968 -> 988, H = 12, D = 64 (1536 tiles) 457 -> 461.
   const bool early = (long long)B * H * P.NB * D <= 384 * 128;
-  cudaError_t launched;
-  {
+  p.early = early;
+  cudaError_t launched = launch_after(bwd_prep_kernel<D>, dim3((unsigned)(rows / kPrepRows)), 256, 0, stream, static_cast<const __nv_bfloat16*>(out),
+                                      static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1], sdo[2], H, T, Tp, stats, dq_acc, early);
+  if (launched == cudaSuccess) {
     ProfileScope timed(1, stream);
-    launched = launch_after_if(early, attn_bwd_kernel<D>, dim3((unsigned)B * H * P.NB), kBwdThreads, BwdSmem<D>::kBytes, stream, mq, mk, mv, mdo, mqs, mdos, mdk, mdv, p);
+    launched = launch_after(attn_bwd_kernel<D>, dim3((unsigned)B * H * P.NB), kBwdThreads, BwdSmem<D>::kBytes, stream, mq, mk, mv, mdo, mqs, mdos, mdk, mdv, p);
   }
   if (launched == cudaSuccess)
-    launched = launch_after_if(early, dq_convert_kernel<D>, dim3((unsigned)(rows / 32)), 256, 0, stream, reinterpret_cast<const float4*>(dq_acc),
+    launched = launch_after(dq_convert_kernel<D>, dim3((unsigned)(rows / 32)), 256, 0, stream, reinterpret_cast<const float4*>(dq_acc),
                             static_cast<__nv_bfloat16*>(dq), sdq[0], sdq[1], sdq[2], H, T, Tp, scale);
   BTRACE_DUMP(stream);
   const cudaError_t last = cudaGetLastError();

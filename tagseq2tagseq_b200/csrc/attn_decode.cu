@@ -18,6 +18,7 @@
 //
 // B = 2, H = 16, Tk = 32768, D = 128, 13.9 k allowed keys a sequence (228 MB): two kernels over fixed 128-key tiles with K
 // before V took 75 + 41 us (a third of the copy rate; the merge walked 256 partial results one after the other).
+#include "launch.cuh"
 #include "plan.h"
 #include "ptx.cuh"
 
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_
   const cg::cluster_group cluster = cg::this_cluster();
   const int h = blockIdx.y, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cs = gridDim.x, W = cs * kDecWarps;
+  wait_previous();
   const int qpos = p.q_pos ? min(max(p.q_pos[b], 0), p.Tk - 1) : p.Tk - 1;
   const size_t base = (size_t)b * p.Tk;
   const int32_t* docs = p.mask.doc + base;
@@ -315,11 +317,13 @@ int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq
   cfg.gridDim = dim3(cs, H, B);
   cfg.blockDim = dim3(kDecWarps * 32);
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = cs; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = cs; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch.cuh
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
   if (D == 128) return cudaLaunchKernelEx(&cfg, decode_kernel<128>, p) == cudaSuccess ? 0 : -141;
   if (D == 64) return cudaLaunchKernelEx(&cfg, decode_kernel<64>, p) == cudaSuccess ? 0 : -141;
   return -142;

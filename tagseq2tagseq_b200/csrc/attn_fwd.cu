@@ -36,6 +36,7 @@
 // (model/modules/layer.py:33 via tunalab FlexSelfAttention; semantics in
 // torch/_higher_order_ops/flex_attention.py:218-287): O = softmax(scale QK^T +
 // mask) V, LSE in natural log, a fully masked row gives O = 0 and LSE = -inf.
+#include "launch.cuh"
 #include "plan.h"
 #include "profile.h"
 #include "ptx.cuh"
@@ -824,6 +825,7 @@ template <int D, int kForm>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
+  wait_previous();
   if constexpr (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
   else if constexpr (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
   else if (!lists_call_for_shared(p)) fwd_items<D, false, true>(mapQ, mapK, mapV, mapO, p);
@@ -864,12 +866,14 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   }
   const unsigned grid = (unsigned)(p.n_items < sms ? p.n_items : sms);
   FTRACE_ATTACH(p, stream);
+  cudaError_t launched;
   {
     ProfileScope timed(0, stream);
-    attn_fwd_kernel<D, kForm><<<grid, kFwdThreads, FwdSmem<D>::kBytes, stream>>>(mq, mk, mv, mo, p);
+    launched = launch_after(attn_fwd_kernel<D, kForm>, dim3(grid), kFwdThreads, FwdSmem<D>::kBytes, stream, mq, mk, mv, mo, p);
   }
   FTRACE_DUMP(stream);
-  return cudaGetLastError() == cudaSuccess ? 0 : -111;
+  const cudaError_t last = cudaGetLastError();
+  return launched == cudaSuccess && last == cudaSuccess ? 0 : -111;
 }
 
 // Shared query tiles are twice as many and half as long, but bring in every key tile once a query tile instead of once a pair,

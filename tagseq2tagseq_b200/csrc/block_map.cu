@@ -32,6 +32,7 @@ __device__ __forceinline__ bool link_bit(const int64_t* link_b, int R, int W, in
 // of its own cost more than either.  The first block clears the status words.
 __global__ void __launch_bounds__(128) runs_kernel(PlanView P, MaskArgs M, int t_words) {
   const int tb = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
+  wait_previous();
   let_next_start();
   if (tb == 0 && b == 0 && t < 64) P.status[t] = 0;
   if (tb >= P.NB) {
@@ -443,6 +444,9 @@ __global__ void __launch_bounds__(256) order_kernel(PlanView P, int link_t_rows)
 __global__ void __launch_bounds__(256) segment_ids_kernel(const int32_t* __restrict__ bounds, const int32_t* __restrict__ ids,
                                                           int n_seg, int T, int32_t* __restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  wait_previous();
+  bounds = settled(bounds);
+  ids = settled(ids);
   if (t >= T) return;
   int lo = 0, hi = n_seg + 1;  // first boundary > t, by bisection over bounds[0 .. n_seg]
   while (lo < hi) {
@@ -453,8 +457,7 @@ __global__ void __launch_bounds__(256) segment_ids_kernel(const int32_t* __restr
 }
 
 cudaError_t launch_segment_ids(const int32_t* bounds, const int32_t* ids, int n_seg, int T, int32_t* out, cudaStream_t stream) {
-  segment_ids_kernel<<<(T + 255) / 256, 256, 0, stream>>>(bounds, ids, n_seg, T, out);
-  return cudaGetLastError();
+  return launch_after(segment_ids_kernel, dim3((T + 255) / 256), 256, 0, stream, bounds, ids, n_seg, T, out);
 }
 
 // The four launches depend on one another and take a few microseconds each, so each starts while the one before still runs
@@ -468,8 +471,8 @@ cudaError_t launch_block_map(PlanView P, MaskArgs M, uint8_t* state_out, int32_t
   if (P.NB == 0 || P.B == 0) return cudaSuccess;
   const bool t = M.link != nullptr && M.R > 0 && M.R <= kLinkTMaxRows && 64 * M.W <= kLinkTMaxCols;
   const int t_words = t ? (M.R + 63) / 64 : 0;
-  runs_kernel<<<dim3(P.NB + t_words * ((64 * M.W + 127) / 128), P.B), 128, 0, stream>>>(P, M, t_words);
-  cudaError_t e = launch_after(state_kernel, dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream, P, M, state_out);
+  cudaError_t e = launch_after(runs_kernel, dim3(P.NB + t_words * ((64 * M.W + 127) / 128), P.B), 128, 0, stream, P, M, t_words);
+  if (e == cudaSuccess) e = launch_after(state_kernel, dim3((P.NB + kStateKb - 1) / kStateKb, P.NB, P.B), 128, 0, stream, P, M, state_out);
   if (e == cudaSuccess)
     e = launch_after(lists_kernel, dim3(lists_blocks(P), P.B), 128, 0, stream, P, ListOutputs{kv_cnt, kv_idx, full_cnt, full_idx},
                      ListOutputs{q_cnt, q_idx, full_q_cnt, full_q_idx});

@@ -15,6 +15,7 @@
 // Three kernels: a grid-wide scan (HBM-bound: each token is read once, 4 or 8 bytes; one block per 256 positions)
 // that marks candidates in a dense int32[T] array and counts them per block, a single-block exclusive scan of the
 // block counts, and a grid-wide ordered write-out.
+#include "launch.cuh"
 #include "link_scan.h"
 
 namespace ts2ts {
@@ -33,6 +34,7 @@ __global__ void __launch_bounds__(kScanBlock) link_scan_kernel(LinkScanArgs a, i
   __shared__ int warp_hits[kScanBlock / 32];
   const int t = blockIdx.x * kScanBlock + threadIdx.x;
   int close = -1, start = -1;
+  wait_previous();
   if (t < a.T && load_token(a, t) == a.mid_id) {
     const int lo = max(0, t - a.back_limit);
     for (int i = t - 1; i >= lo && start < 0; --i) {
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(1024) link_offsets_kernel(int32_t* block_count
   __shared__ int warp_sums[32];
   __shared__ int base;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  wait_previous();
   if (tid == 0) base = 0;
   __syncthreads();
   for (int b0 = 0; b0 < nb; b0 += blockDim.x) {
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(kScanBlock) link_write_kernel(const int32_t* d
   __shared__ int warp_hits[kScanBlock / 32];
   const int t = blockIdx.x * kScanBlock + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  wait_previous();
   const int close = t < T ? dense_close[t] : -1;
   const unsigned ballot = __ballot_sync(0xffffffffu, close >= 0);
   if (lane == 0) warp_hits[warp] = __popc(ballot);
@@ -122,10 +126,10 @@ cudaError_t launch_link_scan(const LinkScanArgs& a, int32_t* scratch, int32_t* o
   int32_t* dense_close = scratch;
   int32_t* dense_start = scratch + a.T;
   int32_t* block_count = scratch + 2 * static_cast<size_t>(a.T);
-  link_scan_kernel<<<nb, kScanBlock, 0, stream>>>(a, dense_close, dense_start, block_count);
-  link_offsets_kernel<<<1, 1024, 0, stream>>>(block_count, nb, count);
-  link_write_kernel<<<nb, kScanBlock, 0, stream>>>(dense_close, dense_start, block_count, a.T, out, max_links);
-  return cudaGetLastError();
+  cudaError_t e = launch_after(link_scan_kernel, dim3(nb), kScanBlock, 0, stream, a, dense_close, dense_start, block_count);
+  if (e == cudaSuccess) e = launch_after(link_offsets_kernel, dim3(1), 1024, 0, stream, block_count, nb, count);
+  if (e == cudaSuccess) e = launch_after(link_write_kernel, dim3(nb), kScanBlock, 0, stream, dense_close, dense_start, block_count, a.T, out, max_links);
+  return e;
 }
 
 }  // namespace ts2ts

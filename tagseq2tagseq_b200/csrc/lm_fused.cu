@@ -9,6 +9,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace ts2ts {
@@ -83,18 +84,28 @@ __global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x_in, const __n
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * C;
   float4 v[NV];
+  uint2 d[NV];
   float ss = 0.f;
+  wait_previous();
+  x_in = settled(x_in); a = settled(a); w = settled(w);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (threadIdx.x + i * blockDim.x) * 4;
     if (c < C) {
-      float4 x = *reinterpret_cast<const float4*>(x_in + base + c);
+      v[i] = *reinterpret_cast<const float4*>(x_in + base + c);
+      d[i] = a != nullptr ? *reinterpret_cast<const uint2*>(a + base + c) : make_uint2(0u, 0u);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (c < C) {
+      float4& x = v[i];
       if (a != nullptr) {
-        const float4 d = bf16x4_to_float4(*reinterpret_cast<const uint2*>(a + base + c));
-        x.x += d.x; x.y += d.y; x.z += d.z; x.w += d.w;
+        const float4 f = bf16x4_to_float4(d[i]);
+        x.x += f.x; x.y += f.y; x.z += f.z; x.w += f.w;
       }
       *reinterpret_cast<float4*>(x_out + base + c) = x;
-      v[i] = x;
       ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
     }
   }
@@ -129,6 +140,8 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_bwd_kernel(const __nv_bfloat
   __shared__ float red[2][kRows][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float4 wv[NV], acc[NV];
+  wait_previous();
+  dh = settled(dh); dx_up = settled(dx_up); x = settled(x); w = settled(w); rstd = settled(rstd);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (threadIdx.x + i * blockDim.x) * 4;
@@ -204,6 +217,8 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restric
   __shared__ float4 red[32][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
   const int c = blockIdx.x * 32 + sub * 4;
+  wait_previous();
+  part = settled(part);
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c < C) {
 #pragma unroll 4
@@ -237,6 +252,8 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restric
 __global__ void rope_qk_kernel(__nv_bfloat16* qkv, const float* __restrict__ cs, const float* __restrict__ sn, int T, int H, int D,
                                int64_t n_threads, float sign) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  wait_previous();
+  cs = settled(cs); sn = settled(sn);
   if (idx >= n_threads) return;
   const int vec_per_head = D / 16;  // groups of eight pairs
   int64_t r = idx;
@@ -270,6 +287,8 @@ __global__ void rope_qk_kernel(__nv_bfloat16* qkv, const float* __restrict__ cs,
 // gu [N, 2F]: gate in the first F columns, up in the last F (torch.chunk(2, dim=-1));  act = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, int F, int64_t n_vec) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  wait_previous();
+  gu = settled(gu);
   if (idx >= n_vec) return;
   const int per_row = F / 8;
   const int64_t row = idx / per_row;
@@ -285,6 +304,8 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dact,
                                   __nv_bfloat16* __restrict__ dgu, int F, int64_t n_vec) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  wait_previous();
+  gu = settled(gu); dact = settled(dact);
   if (idx >= n_vec) return;
   const int per_row = F / 8;
   const int64_t row = idx / per_row;
@@ -308,6 +329,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 __global__ void ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ target, float* __restrict__ lse,
                               float* __restrict__ loss, int V) {
   __shared__ float red[32];
+  wait_previous();
+  logits = settled(logits); target = settled(target);
   const __nv_bfloat16* row = logits + (size_t)blockIdx.x * V;
   float m = -CUDART_INF_F, s = 0.f;
   for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
@@ -337,6 +360,8 @@ __global__ void ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const in
 // contributed no loss and get a zero gradient.
 __global__ void ce_bwd_kernel(__nv_bfloat16* logits, const int64_t* __restrict__ target, const float* __restrict__ lse,
                               const float* __restrict__ gscale, float inv_n, int V) {
+  wait_previous();
+  target = settled(target); lse = settled(lse); gscale = settled(gscale);
   __nv_bfloat16* row = logits + (size_t)blockIdx.x * V;
   const int64_t tg = target[blockIdx.x];
   const bool live = tg >= 0 && tg < V;
@@ -364,6 +389,8 @@ __global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* 
   __nv_bfloat16* row = logits + (size_t)blockIdx.x * V;
   const int n_vec = V / 8, per_chunk = (n_vec + kCeChunks - 1) / kCeChunks;  // in 16-byte vectors
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  wait_previous();
+  target = settled(target);
   if (tid == 0) {
     late = 0;
     for (int k = 0; k < kCeChunks; ++k) mbar_init(&bars[k], 1);
@@ -427,12 +454,16 @@ __global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* 
 // x *= gscale[0], and out = bf16(x * gscale[0]).  The first does nothing when the factor is one, which it is unless the
 // caller scaled the loss.
 __global__ void __launch_bounds__(256) scale_f32_kernel(float* x, const float* __restrict__ gscale, int64_t n) {
+  wait_previous();
+  gscale = settled(gscale);
   const float g = gscale[0];
   if (g == 1.f) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] *= g;
 }
 __global__ void __launch_bounds__(256) scale_to_bf16_kernel(const float* __restrict__ x, const float* __restrict__ gscale,
                                                             __nv_bfloat16* __restrict__ out, int64_t n_vec) {
+  wait_previous();
+  x = settled(x); gscale = settled(gscale);
   const float g = gscale[0];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_vec) return;
@@ -466,6 +497,8 @@ __global__ void __launch_bounds__(kEmbThreads) embedding_bwd_kernel(const int64_
   const int col = blockIdx.y * kEmbCols + lane * 4;  // of this lane's first vector; the others follow 128 columns apart
   int count = 0;                                     // queued tokens, the same in every thread
   bool first = true;                                 // nothing of this block's rows written yet
+  wait_previous();
+  idx = settled(idx); dx = settled(dx);
 
   // sum of the queued rows of `id` between two places of the queue, `kVecs` vectors a lane from vector `from` on
   auto sum_rows = [&](auto vecs, int id, int begin, int end, int from, float4* acc) {
@@ -609,12 +642,10 @@ cudaError_t launch_add_rmsnorm_fwd(const float* x_in, const void* a, const float
                                    float eps, cudaStream_t stream) {
   const int threads = norm_threads(C);
   if (C <= 4 * threads)
-    add_rmsnorm_fwd_kernel<1><<<N, threads, 0, stream>>>(x_in, static_cast<const __nv_bfloat16*>(a), w, x_out, static_cast<__nv_bfloat16*>(h),
-                                                         rstd, C, eps);
-  else
-    add_rmsnorm_fwd_kernel<kMaxVec><<<N, threads, 0, stream>>>(x_in, static_cast<const __nv_bfloat16*>(a), w, x_out,
-                                                               static_cast<__nv_bfloat16*>(h), rstd, C, eps);
-  return cudaGetLastError();
+    return launch_after(add_rmsnorm_fwd_kernel<1>, dim3(N), threads, 0, stream, x_in, static_cast<const __nv_bfloat16*>(a), w, x_out,
+                        static_cast<__nv_bfloat16*>(h), rstd, C, eps);
+  return launch_after(add_rmsnorm_fwd_kernel<kMaxVec>, dim3(N), threads, 0, stream, x_in, static_cast<const __nv_bfloat16*>(a), w, x_out,
+                      static_cast<__nv_bfloat16*>(h), rstd, C, eps);
 }
 
 // Blocks of the backward kernel = rows of its dw_part workspace.
@@ -639,48 +670,38 @@ cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const flo
   const int threads = norm_threads(C);
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(dh);
   __nv_bfloat16* a = static_cast<__nv_bfloat16*>(da);
-  if (C <= 4 * threads)
-    add_rmsnorm_bwd_kernel<1, 2><<<grid, threads, 0, stream>>>(g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
-  else
-    add_rmsnorm_bwd_kernel<kMaxVec, 1><<<grid, threads, 0, stream>>>(g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  column_sum_kernel<<<(C + 31) / 32, 1024, 0, stream>>>(dw_part, dw, grid, C);
-  return cudaGetLastError();
+  const cudaError_t e = launch_after(C <= 4 * threads ? add_rmsnorm_bwd_kernel<1, 2> : add_rmsnorm_bwd_kernel<kMaxVec, 1>, dim3(grid), threads, 0, stream,
+                                     g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
+  return e != cudaSuccess ? e : launch_after(column_sum_kernel, dim3((C + 31) / 32), 1024, 0, stream, dw_part, dw, grid, C);
 }
 
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream) {
   const int64_t n = (int64_t)B * T * 2 * H * (D / 16);
   const int threads = 256;
-  rope_qk_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), cs, sn, T, H, D, n, sign);
-  return cudaGetLastError();
+  return launch_after(rope_qk_kernel, dim3((unsigned)((n + threads - 1) / threads)), threads, 0, stream, static_cast<__nv_bfloat16*>(qkv), cs, sn, T, H, D, n, sign);
 }
 
 cudaError_t launch_swiglu_fwd(const void* gu, void* act, int64_t N, int F, cudaStream_t stream) {
   const int64_t n = N * (F / 8);
   const int threads = 256;
-  swiglu_fwd_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, stream>>>(static_cast<const __nv_bfloat16*>(gu),
-                                                                                     static_cast<__nv_bfloat16*>(act), F, n);
-  return cudaGetLastError();
+  return launch_after(swiglu_fwd_kernel, dim3((unsigned)((n + threads - 1) / threads)), threads, 0, stream, static_cast<const __nv_bfloat16*>(gu),
+                      static_cast<__nv_bfloat16*>(act), F, n);
 }
 
 cudaError_t launch_swiglu_bwd(const void* gu, const void* dact, void* dgu, int64_t N, int F, cudaStream_t stream) {
   const int64_t n = N * (F / 8);
   const int threads = 256;
-  swiglu_bwd_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dact), static_cast<__nv_bfloat16*>(dgu), F, n);
-  return cudaGetLastError();
+  return launch_after(swiglu_bwd_kernel, dim3((unsigned)((n + threads - 1) / threads)), threads, 0, stream, static_cast<const __nv_bfloat16*>(gu),
+                      static_cast<const __nv_bfloat16*>(dact), static_cast<__nv_bfloat16*>(dgu), F, n);
 }
 
 cudaError_t launch_ce_fwd(const void* logits, const int64_t* target, float* lse, float* loss, int N, int V, cudaStream_t stream) {
-  ce_fwd_kernel<<<N, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), target, lse, loss, V);
-  return cudaGetLastError();
+  return launch_after(ce_fwd_kernel, dim3(N), 256, 0, stream, static_cast<const __nv_bfloat16*>(logits), target, lse, loss, V);
 }
 
 cudaError_t launch_ce_bwd(void* logits, const int64_t* target, const float* lse, const float* gscale, float inv_n, int N, int V,
                           cudaStream_t stream) {
-  ce_bwd_kernel<<<N, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(logits), target, lse, gscale, inv_n, V);
-  return cudaGetLastError();
+  return launch_after(ce_bwd_kernel, dim3(N), 256, 0, stream, static_cast<__nv_bfloat16*>(logits), target, lse, gscale, inv_n, V);
 }
 
 // -1000: the row does not fit shared memory (the caller takes the two-kernel path).
@@ -695,25 +716,21 @@ int launch_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float i
     if (cudaFuncSetAttribute(ce_fwd_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeRowBytes) != cudaSuccess) return -50;
     attr_done[dev] = true;
   }
-  ce_fwd_grad_kernel<<<N, kCeThreads, bytes, stream>>>(static_cast<__nv_bfloat16*>(logits), target, loss, inv_n, V);
-  return cudaGetLastError() == cudaSuccess ? 0 : -50;
+  return launch_after(ce_fwd_grad_kernel, dim3(N), kCeThreads, bytes, stream, static_cast<__nv_bfloat16*>(logits), target, loss, inv_n, V) == cudaSuccess ? 0 : -50;
 }
 
 cudaError_t launch_scale(float* x, void* out_bf16, const float* gscale, int64_t n, cudaStream_t stream) {
   if (out_bf16 == nullptr) {
     const int64_t blocks = (n + 1023) / 1024;
-    scale_f32_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, stream>>>(x, gscale, n);
-  } else {
-    scale_to_bf16_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, stream>>>(x, gscale, static_cast<__nv_bfloat16*>(out_bf16), n / 8);
+    return launch_after(scale_f32_kernel, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), 256, 0, stream, x, gscale, n);
   }
-  return cudaGetLastError();
+  return launch_after(scale_to_bf16_kernel, dim3((unsigned)((n / 8 + 255) / 256)), 256, 0, stream, x, gscale, static_cast<__nv_bfloat16*>(out_bf16), n / 8);
 }
 
 cudaError_t launch_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(dw, 0, (size_t)V * C * sizeof(float), stream);
   if (e != cudaSuccess) return e;
-  embedding_bwd_kernel<<<dim3(kEmbBuckets, (C + kEmbCols - 1) / kEmbCols), kEmbThreads, 0, stream>>>(idx, dx, dw, (int)N, C, V);
-  return cudaGetLastError();
+  return launch_after(embedding_bwd_kernel, dim3(kEmbBuckets, (C + kEmbCols - 1) / kEmbCols), kEmbThreads, 0, stream, idx, dx, dw, (int)N, C, V);
 }
 
 }  // namespace ts2ts

@@ -1,7 +1,7 @@
 // Masked flash-attention forward for sm_100a.
 //
 // Persistent kernel, one CTA per SM.  A work item is a pair of adjacent 128-row query tiles (2p, 2p+1) of one
-// (batch, head); CTAs draw items from a ticket counter, group of heads after group of heads, inside a group the pairs with the
+// (batch, head); a CTA's first item is its own number, further ones are drawn from a ticket counter, group of heads after group of heads, inside a group the pairs with the
 // most key tiles first, so the tiles that run at the same time share K/V in L2 and the long items start early.  Each query tile of the pair belongs to a "team":
 //   softmax team t   4 warps, one thread per query row (setmaxnreg 216)
 //   issuer t         1 thread issuing the team's tcgen05.mma
@@ -23,9 +23,10 @@
 // 4125, because teams whose tiles differ then wait for each other's reads.
 // The accumulator is rescaled lazily: only when a row's running maximum grows by more than 2^8.
 // K/V tiles travel through one ring of shared-memory slots in the order K0, K1, V0, K2, V1, ... (K runs one tile
-// ahead of V because S is computed one tile ahead of P V).  Short launches have the teams share a query tile instead (launch_fwd_t):
-// the tiles of its list go to them in turn, and team 0 adds up both parts at the end, straight from tensor memory.  A team's next K is then
-// two places ahead in the list and comes behind its current V, so its S is not computed ahead: part of what a shared tile costs.  At the end of an item each softmax thread reads its
+// ahead of V because S is computed one tile ahead of P V).  Launches that are as long as their longest list have the teams share a query tile
+// instead (launch_fwd_t): the tiles of its list go to them in turn, K two tiles ahead of V so that either team's S is computed ahead there too
+// (us with K one tile ahead -> two: causal 4096, H = 8, D = 128 51 -> 45, linked 16k, H = 2, D = 64 75 -> 66, linked 1024, H = 4 18.5 -> 16.6),
+// and team 0 adds up both parts at the end, straight from tensor memory.  At the end of an item each softmax thread reads its
 // row of O out of tensor memory and frees it for the next item; the normalised rows leave through shared memory and TMA stores, a
 // warp's 32 rows at a time, while the issuers already work on the next item.
 //
@@ -86,11 +87,10 @@ struct FwdParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_sh, o_st;
   int H;
-  int n_items;           // B * H * ceil(NB / 2), or B * H * NB where the teams share a query tile
+  int n_pairs, n_tiles;  // B * H * ceil(NB / 2) and B * H * NB: the work items as pairs and as shared query tiles
   int heads;             // heads of a stretch of the ticket order: H, or B * H where the batch elements are one
   int head_group;        // heads whose items are interleaved in the ticket order
   float scale_log2;      // softmax scale * log2(e)
-  int n_pairs;           // items of a launch that may share tiles and does not
   TS2TS_TRACE_FIELDS
 };
 
@@ -98,6 +98,7 @@ constexpr int kFwdThreads = 384;   // warps 0-3 softmax team 0, 4-7 team 1, 8-9 
 constexpr int kFwdIssuerWarp = 8;  // + team
 constexpr int kFwdProducerWarp = 10;
 constexpr int kFwdItemSlots = 2;
+constexpr uint32_t kNoMasks = 0xffffffffu;
 template <uint32_t N> __device__ __forceinline__ void fwd_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> __device__ __forceinline__ void fwd_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr float kRescaleThreshold = 8.0f;
@@ -119,7 +120,7 @@ struct FwdSmem {
   static constexpr int kRing = kP + 2 * kPBytes;             // K/V slots
   static constexpr int kSmall = kRing + kStages * kTileBytes;
   static constexpr int kBars = 21 + 2 * kStages;
-  static constexpr int kSmallBytes = kTile * 8 + kBars * 8 + 16 + 4 * kStages;  // row statistics, barriers, words
+  static constexpr int kSmallBytes = kTile * 8 + kFwdItemSlots * (48 + 32 * (kMaskRuns + 1)) + kBars * 8 + 8 + 4 * kStages;  // row statistics, items, barriers, words
   static constexpr int kBytes = kSmall + kSmallBytes + 1024;  // + alignment slack
   // tensor-memory columns of team t
   static __host__ __device__ constexpr int score_col(int t) { return t * kTile; }
@@ -127,17 +128,21 @@ struct FwdSmem {
   static __host__ __device__ constexpr int p_col(int t) { return 2 * kTile + 2 * D + t * 64; }  // kTmemP
 };
 
-// One work item, decoded from its ticket number by every role on its own: the query tiles, key-tile counts and key-tile lists of the two
-// teams.  Teams that share a query tile take every other entry of its list.
-struct FwdItem {
-  int b, h, qb[2];
-  int n[2];
-  const int32_t* list[2];
+// One work item as the producer publishes it in shared memory, with all that a softmax warp would otherwise fetch from global memory, four accesses one after
+// the other, before its first tile (with the numbers of heads and rows read back from here at the end instead of kept, us: causal 4k batch 4, H = 16, D = 64
+// 222 -> 213, D = 128 298 -> 282, linked 16k, H = 12, D = 64 256 -> 252).  Teams that share a query tile take every other entry of its list.
+struct alignas(16) FwdItem {
+  int code, b, h, qb;           // code < 0: no more work; the first team's query tile (the second one's is the next, or the same where they share it)
+  int n[2], n_runs[2];          // key tiles and runs of each team's query tile
+  int first[2][2];              // the first two list entries of each team
+  Run runs[2][kMaskRuns + 1];   // the first runs of each team's query tile (of the shared one: [0])
 };
+static_assert(sizeof(FwdItem) == 48 + 2 * 16 * (kMaskRuns + 1), "");
 // Ticket order: batch elements one after the other, or, in short launches, as one (`heads` = B * H); inside one, groups of G heads;
 // inside a group all heads' heaviest items first, then their second heaviest, and so on.  The group bounds the K/V working set that has
 // to stay in L2, and the long items of the last group still start well before the end of the launch.
-__device__ __forceinline__ void decode_item(const PlanView& P, int H, int heads, int G, int split, int code, FwdItem& it) {
+// Returns where the plan says which query tile (or pair of them) it is.
+__device__ __forceinline__ const int32_t* item_place(const PlanView& P, int H, int heads, int G, bool split, int code, int& b, int& h) {
   const int NI = split ? P.NB : (P.NB + 1) / 2;
   const int per_b = heads * NI;
   const int b0 = code / per_b;
@@ -146,29 +151,29 @@ __device__ __forceinline__ void decode_item(const PlanView& P, int H, int heads,
   const int r2 = r1 - g * G * NI;
   const int gsize = min(G, heads - g * G);
   const int rank = r2 / gsize;
-  it.h = g * G + (r2 - rank * gsize);
-  const int more = it.h / H;  // batch elements past b0
-  it.b = b0 + more;
-  it.h -= more * H;
-  const int at = min(max(__ldg((split ? P.fwd_order : P.pair_order) + (size_t)it.b * NI + rank), 0), NI - 1);
-  it.qb[0] = split ? at : 2 * at;
-  const size_t row0 = (size_t)it.b * P.NB + it.qb[0];
-  const int n0 = min(max(__ldg(&P.fwd_cnt[row0]), 0), P.NB);
-  it.list[0] = it.list[1] = P.fwd_idx + row0 * P.NB;
-  if (split) {
-    it.qb[1] = at;
-    it.n[0] = (n0 + 1) / 2;
-    it.n[1] = n0 / 2;
-    ++it.list[1];
-  } else {
-    it.qb[1] = 2 * at + 1;
-    it.n[0] = n0;
-    it.n[1] = 0;
-    if (it.qb[1] < P.NB) {
-      it.n[1] = min(max(__ldg(&P.fwd_cnt[row0 + 1]), 0), P.NB);
-      it.list[1] += P.NB;
-    }
-  }
+  h = g * G + (r2 - rank * gsize);
+  const int more = h / H;  // batch elements past b0
+  b = b0 + more;
+  h -= more * H;
+  return (split ? P.fwd_order : P.pair_order) + (size_t)b * NI + rank;
+}
+// The rest of the item, one round of loads.
+__device__ __forceinline__ void read_item(const PlanView& P, bool split, int at, FwdItem& it) {
+  at = min(max(at, 0), (split ? P.NB : (P.NB + 1) / 2) - 1);
+  it.qb = split ? at : 2 * at;
+  const bool two = !split && it.qb + 1 < P.NB;
+  const size_t row0 = (size_t)it.b * P.NB + it.qb, row1 = two ? row0 + 1 : row0;
+  const int32_t *l0 = P.fwd_idx + row0 * P.NB, *l1 = P.fwd_idx + row1 * P.NB;
+  const int c0 = ld_nc_i32_here(&P.fwd_cnt[row0]), c1 = ld_nc_i32_here(&P.fwd_cnt[row1]);
+  const int r0 = ld_nc_i32_here(&P.run_cnt[row0]), r1 = ld_nc_i32_here(&P.run_cnt[row1]);
+  // entries past a list's end are there up to its NB-th and are not looked at
+  const int e00 = ld_nc_i32_here(l0), e01 = ld_nc_i32_here(l0 + min(split ? 2 : 1, P.NB - 1));
+  const int e10 = ld_nc_i32_here(l1 + (split ? min(1, P.NB - 1) : 0)), e11 = ld_nc_i32_here(l1 + min(split ? 3 : 1, P.NB - 1));
+  const int n0 = min(max(c0, 0), P.NB);
+  it.n[0] = split ? (n0 + 1) / 2 : n0;
+  it.n[1] = split ? n0 / 2 : two ? min(max(c1, 0), P.NB) : 0;
+  it.n_runs[0] = r0; it.n_runs[1] = r1;
+  it.first[0][0] = e00; it.first[0][1] = e01; it.first[1][0] = e10; it.first[1][1] = e11;
 }
 // What a ring slot holds, written by the producer next to the slot.
 enum : uint32_t {
@@ -185,8 +190,10 @@ struct UnionWalk {
   const int32_t *l0, *l1;
   int n0, n1, i0, i1, NB;
   bool split;
-  __device__ __forceinline__ void start(const FwdItem& it, int nb, bool shared) {
-    l0 = it.list[0]; l1 = it.list[1]; n0 = it.n[0]; n1 = it.n[1]; i0 = i1 = 0; NB = nb; split = shared;
+  __device__ __forceinline__ void start(const PlanView& P, const FwdItem& it, bool shared) {
+    l0 = P.fwd_idx + ((size_t)it.b * P.NB + it.qb) * P.NB;
+    l1 = shared ? l0 : l0 + P.NB;
+    n0 = it.n[0]; n1 = it.n[1]; i0 = i1 = 0; NB = P.NB; split = shared;
   }
   __device__ __forceinline__ int next(uint32_t& info) {
     if (split) {
@@ -259,88 +266,132 @@ __device__ __forceinline__ void fwd_leave(const PlanView& P) {
   }
 }
 
-// kShared: the two teams of a CTA share a query tile and take its key tiles in turn, instead of a query tile of a pair each.
-// kIdle: the grid may have more CTAs than items; those leave at once, but behind the look at the plan's stamp, because a plan that is
-// refused must not keep a part of the count.
-template <int D, bool kShared, bool kIdle = false>
-__device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtensorMap& mapK, const CUtensorMap& mapV, const CUtensorMap& mapO, const FwdParams& p) {
+// Where the pieces of a CTA's shared memory lie.
+template <int D>
+struct FwdPlaces {
   using Cfg = FwdSmem<D>;
-  constexpr int kStages = Cfg::kStages;
-  extern __shared__ uint8_t smem_raw[];
-  // Plain pointer arithmetic (no round trip through an integer) keeps the shared address space visible to the
-  // compiler, so every access below becomes a shared-memory instruction instead of a generic one.
-  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* sQ = smem + Cfg::kQ;
-  uint8_t* sP = smem + Cfg::kP;
-  uint8_t* sRing = smem + Cfg::kRing;
-  float2* s_merge = reinterpret_cast<float2*>(smem + Cfg::kSmall);  // [row] maximum and sum of team 1
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_merge + kTile);
-  uint64_t* bar_item_full = bars;        // [2] the producer published a ticket
-  uint64_t* bar_item_empty = bars + 2;   // [2] the eight softmax warps copied it
-  uint64_t* bar_q_full = bars + 4;       // [team] Q tile landed
-  uint64_t* bar_q_free = bars + 6;       // [team] last S of the item complete: the Q buffer may be reloaded
-  uint64_t* bar_s = bars + 8;            // [team] S of the tile is in tensor memory
-  uint64_t* bar_sfree = bars + 10;       // [team] S read into registers: its columns may be overwritten
-  uint64_t* bar_p = bars + 12;           // [team] P of the tile (D = 64: of its last 64 keys) is written
-  uint64_t* bar_pv = bars + 14;          // [team] P V of the tile complete: P free, O consistent
-  uint64_t* bar_ofree = bars + 16;       // [team] O of the item read out of tensor memory
-  uint64_t* bar_p0 = bars + 18;          // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled (D = 64)
-  uint64_t* bar_merge = bars + 20;       // team 1's part of a shared query tile is in tensor memory, its row statistics in s_merge
-  uint64_t* bar_ring_full = bars + 21;   // [kStages] K or V tile landed in the slot
-  uint64_t* bar_ring_free = bars + 21 + kStages;  // [kStages] both issuers are done with the slot
-  int* s_item = reinterpret_cast<int*>(bars + Cfg::kBars);  // [2] ticket ring
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_item + 2);
-  int* abort_w = s_item + 3;
-  uint32_t* s_ring_info = reinterpret_cast<uint32_t*>(s_item + 4);  // [kStages] kRing* bits of what each slot holds
+  uint8_t *raw, *smem;
+  uint8_t* sQ;
+  uint8_t* sP;
+  uint8_t* sRing;
+  float2* s_merge;  // [row] maximum and sum of team 1
+  FwdItem* s_item;  // [2]
+  uint64_t* bars;
+  uint64_t* bar_item_full;  // [2] the producer published an item
+  uint64_t* bar_item_empty;  // [2] the eight softmax warps copied it
+  uint64_t* bar_q_full;  // [team] Q tile landed
+  uint64_t* bar_q_free;  // [team] last S of the item complete: the Q buffer may be reloaded
+  uint64_t* bar_s;  // [team] S of the tile is in tensor memory
+  uint64_t* bar_sfree;  // [team] S read into registers: its columns may be overwritten
+  uint64_t* bar_p;  // [team] P of the tile (D = 64: of its last 64 keys) is written
+  uint64_t* bar_pv;  // [team] P V of the tile complete: P free, O consistent
+  uint64_t* bar_ofree;  // [team] O of the item read out of tensor memory
+  uint64_t* bar_p0;  // [team] P of the tile's first 64 keys is in tensor memory and O is rescaled (D = 64)
+  uint64_t* bar_merge;  // team 1's part of a shared query tile is in tensor memory, its row statistics in s_merge
+  uint64_t* bar_ring_full;  // [kStages] K or V tile landed in the slot
+  uint64_t* bar_ring_free;  // [kStages] both issuers are done with the slot
+  uint32_t* tmem_slot;
+  int* abort_w;
+  uint32_t* s_ring_info;  // [kStages] kRing* bits of what each slot holds
+  __device__ __forceinline__ explicit FwdPlaces(uint8_t* base) : raw(base) {
+    // Plain pointer arithmetic (no round trip through an integer) keeps the shared address space visible to the
+    // compiler, so every access becomes a shared-memory instruction instead of a generic one.
+    smem = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
+    sQ = smem + Cfg::kQ;
+    sP = smem + Cfg::kP;
+    sRing = smem + Cfg::kRing;
+    s_merge = reinterpret_cast<float2*>(smem + Cfg::kSmall);
+    s_item = reinterpret_cast<FwdItem*>(s_merge + kTile);
+    bars = reinterpret_cast<uint64_t*>(s_item + kFwdItemSlots);
+    bar_item_full = bars;
+    bar_item_empty = bars + 2;
+    bar_q_full = bars + 4;
+    bar_q_free = bars + 6;
+    bar_s = bars + 8;
+    bar_sfree = bars + 10;
+    bar_p = bars + 12;
+    bar_pv = bars + 14;
+    bar_ofree = bars + 16;
+    bar_p0 = bars + 18;
+    bar_merge = bars + 20;
+    bar_ring_full = bars + 21;
+    bar_ring_free = bars + 21 + Cfg::kStages;
+    tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kBars);
+    abort_w = reinterpret_cast<int*>(tmem_slot + 1);
+    s_ring_info = tmem_slot + 2;
+  }
+};
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const PlanView& P = p.plan;
-  const int NB = P.NB;
-  {  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
-    int bad = 0;
-    if (P.status[kStampMagic] != kPlanMagic || P.status[kStampB] != P.B || P.status[kStampT] != P.T) bad = 1900;
-    else if (smem + Cfg::kSmall + Cfg::kSmallBytes > smem_raw + Cfg::kBytes) bad = 1901;
-    if (bad) {
-      if (tid == 0) atomicCAS(P.status, 0, bad);
-      return;
-    }
-  }
-  if (kIdle && static_cast<int>(blockIdx.x) >= p.n_pairs) {
-    if (tid == 0) fwd_leave(P);
-    return;
-  }
+// Barriers and tensor memory; nothing here looks at memory that an earlier launch may have written.  Returns the tensor memory's address.
+template <int D>
+__device__ __forceinline__ uint32_t fwd_setup(const FwdPlaces<D>& at) {
+  const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
-    *abort_w = 0;
+    *at.abort_w = 0;
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar_item_full[i], 1);
-      mbar_init(&bar_item_empty[i], 8);
-      mbar_init(&bar_q_full[i], 1);
-      mbar_init(&bar_q_free[i], 1);
-      mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_sfree[i], 4);  // one arrival per softmax warp
-      mbar_init(&bar_p[i], 4);
-      mbar_init(&bar_p0[i], 4);
-      mbar_init(&bar_pv[i], 1);
-      mbar_init(&bar_ofree[i], 4);
+      mbar_init(&at.bar_item_full[i], 1);
+      mbar_init(&at.bar_item_empty[i], 8);
+      mbar_init(&at.bar_q_full[i], 1);
+      mbar_init(&at.bar_q_free[i], 1);
+      mbar_init(&at.bar_s[i], 1);
+      mbar_init(&at.bar_sfree[i], 4);  // one arrival per softmax warp
+      mbar_init(&at.bar_p[i], 4);
+      mbar_init(&at.bar_p0[i], 4);
+      mbar_init(&at.bar_pv[i], 1);
+      mbar_init(&at.bar_ofree[i], 4);
     }
-    mbar_init(bar_merge, 4);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&bar_ring_full[i], 1);
-      mbar_init(&bar_ring_free[i], 2);
+    mbar_init(at.bar_merge, 4);
+    for (int i = 0; i < FwdSmem<D>::kStages; ++i) {
+      mbar_init(&at.bar_ring_full[i], 1);
+      mbar_init(&at.bar_ring_free[i], 2);
     }
     fence_mbar_init();
   }
   __syncthreads();
   if (warp == kFwdIssuerWarp) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(at.tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  return *at.tmem_slot;
+}
+
+// kShared: the two teams of a CTA share a query tile and take its key tiles in turn, instead of a query tile of a pair each.
+// `first_at`: for the producer, what the plan says about the CTA's first item.
+template <int D, bool kShared>
+__device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtensorMap& mapK, const CUtensorMap& mapV, const CUtensorMap& mapO, const FwdParams& p,
+                                          const FwdPlaces<D>& at, uint32_t tmem, int first_at) {
+  using Cfg = FwdSmem<D>;
+  constexpr int kStages = Cfg::kStages;
+  uint8_t* const sQ = at.sQ;
+  uint8_t* const sP = at.sP;
+  uint8_t* const sRing = at.sRing;
+  float2* const s_merge = at.s_merge;
+  FwdItem* const s_item = at.s_item;
+  uint64_t* const bars = at.bars;
+  uint64_t* const bar_item_full = at.bar_item_full;
+  uint64_t* const bar_item_empty = at.bar_item_empty;
+  uint64_t* const bar_q_full = at.bar_q_full;
+  uint64_t* const bar_q_free = at.bar_q_free;
+  uint64_t* const bar_s = at.bar_s;
+  uint64_t* const bar_sfree = at.bar_sfree;
+  uint64_t* const bar_p = at.bar_p;
+  uint64_t* const bar_pv = at.bar_pv;
+  uint64_t* const bar_ofree = at.bar_ofree;
+  uint64_t* const bar_p0 = at.bar_p0;
+  uint64_t* const bar_merge = at.bar_merge;
+  uint64_t* const bar_ring_full = at.bar_ring_full;
+  uint64_t* const bar_ring_free = at.bar_ring_free;
+  uint32_t* const tmem_slot = at.tmem_slot;
+  int* const abort_w = at.abort_w;
+  uint32_t* const s_ring_info = at.s_ring_info;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const PlanView& P = p.plan;
+  const int NB = P.NB;
+  const int n_items = kShared ? p.n_tiles : p.n_pairs;
   volatile int* abort_v = abort_w;
-  if (tid == 0) FTRACE_SPAN(0);
 
   if (warp >= 8) {
     fwd_reg_dec<72>();  // register pool: 256 x 216 + 128 x 72 = 384 x 168
@@ -368,37 +419,62 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
       for (uint32_t it = 0; ok; ++it) {
         const uint32_t is = it % kFwdItemSlots;
         if (it >= kFwdItemSlots && !mbar_wait(&bar_item_empty[is], (it / kFwdItemSlots - 1) & 1, abort_v, 12)) break;
-        const int ticket = atomicAdd(&P.status[kFwdTicket], 1);
-        const int code = ticket < (kIdle ? p.n_pairs : p.n_items) ? ticket : -1;
-        s_item[is] = code;
-        mbar_arrive(&bar_item_full[is]);
-        if (code < 0) {
+        // The first item of a CTA is its own number; the next one is drawn once all copies of the last have been asked for: earlier draws
+        // cost balance (at the start of the last item 8-15 %, linked 16k, H = 12, D = 64).
+        int code = it == 0 ? static_cast<int>(blockIdx.x) : static_cast<int>(gridDim.x) + atomicAdd(&P.status[kFwdTicket], 1);
+        if (code >= n_items) {
+          s_item[is].code = -1;
+          mbar_arrive(&bar_item_full[is]);
           fill(nullptr, kRingEnd, 0, 0, 0);
           break;
         }
-        FwdItem item;
-        decode_item(P, p.H, p.heads, p.head_group, kShared, code, item);
+        FwdItem& item = s_item[is];
+        int h, b;
+        const int32_t* place = item_place(P, p.H, p.heads, p.head_group, kShared, code, b, h);
+        item.code = code; item.b = b; item.h = h;
+        read_item(P, kShared, it == 0 ? first_at : ld_nc_i32_here(place), item);
+        const int qb = item.qb, n_own[2] = {item.n[0], item.n[1]};
+        auto publish = [&]() {
+          const int tiles = P.q_mask == nullptr ? 0 : kShared || qb + 1 >= NB ? 1 : 2;
+          mbar_expect_tx(&bar_item_full[is], tiles * (int)sizeof(item.runs[0]));
+          for (int t = 0; t < tiles; ++t) bulk_load(item.runs[t], P.runs + ((size_t)b * NB + qb + t) * kTile, sizeof(item.runs[0]), &bar_item_full[is]);
+        };
+        if (it > 0) publish();  // the first time the tiles' copies are the ones to hurry
         for (int t = 0; t < 2 && ok; ++t) {
-          if (item.n[t] == 0) continue;
+          if (n_own[t] == 0) continue;
           if (q_loads[t] > 0 && !mbar_wait(&bar_q_free[t], (q_loads[t] - 1) & 1, abort_v, 13)) { ok = false; break; }
           mbar_expect_tx(&bar_q_full[t], Cfg::kTileBytes);
-          tma_load_tile(sQ + t * Cfg::kTileBytes, &mapQ, &bar_q_full[t], item.qb[t] * kTile, 0, item.h, item.b);
+          tma_load_tile(sQ + t * Cfg::kTileBytes, &mapQ, &bar_q_full[t], (kShared ? qb : qb + t) * kTile, 0, h, b);
           ++q_loads[t];
         }
         if (!ok) break;
         UnionWalk w;
-        w.start(item, NB, kShared);
-        uint32_t cur_info = 0, nxt_info = 0;
-        int cur = w.next(cur_info);
-        if (cur == -2) { atomicCAS(abort_w, 0, 14); break; }
-        if (cur >= 0) ok = fill(&mapK, cur_info, cur, item.h, item.b);
-        while (cur >= 0 && ok) {
-          const int nxt = w.next(nxt_info);
-          if (nxt == -2) { atomicCAS(abort_w, 0, 14); ok = false; break; }
-          if (nxt >= 0) ok = fill(&mapK, nxt_info, nxt, item.h, item.b);
-          if (ok) ok = fill(&mapV, cur_info | kRingIsV, cur, item.h, item.b);
-          cur = nxt;
-          cur_info = nxt_info;
+        w.start(P, item, kShared);
+        // The tiles whose K is in the ring and whose V is not yet: one, or two where the teams share a query tile, so that either team's
+        // next K comes ahead of its current V and its next S is computed during the softmax of this one.
+        constexpr int kAhead = kShared ? 2 : 1;
+        uint32_t infos[kAhead + 1];
+        int tiles[kAhead + 1];
+        auto next_k = [&](int at) {  // the next tile of the walk into place `at`, its K into the ring
+          tiles[at] = w.next(infos[at]);
+          if (tiles[at] == -2) { atomicCAS(abort_w, 0, 14); return false; }
+          return tiles[at] < 0 || fill(&mapK, infos[at], tiles[at], h, b);
+        };
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          tiles[i] = -1;
+          if (ok && (i == 0 || tiles[i - 1] >= 0)) ok = next_k(i);
+          if (i == 0 && it == 0) publish();
+        }
+        while (tiles[0] >= 0 && ok) {
+          tiles[kAhead] = -1;
+          if (tiles[kAhead - 1] >= 0) ok = next_k(kAhead);
+          if (ok) ok = fill(&mapV, infos[0] | kRingIsV, tiles[0], h, b);
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) {
+            tiles[i] = tiles[i + 1];
+            infos[i] = infos[i + 1];
+          }
         }
       }
     } else if ((warp == kFwdIssuerWarp || warp == kFwdIssuerWarp + 1) && lane == 0) {
@@ -492,69 +568,65 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
     // whatever is computed from there on stays in this CTA, because every warp looks at the word, as one, before an item's rows
     // leave.  A vote for each wait cost 5 % at D = 64 (causal 4k batch 4: 220 -> 232 us), a flag kept per lane 2 %.
     bool ok = true;
+    constexpr int step = kShared ? 2 : 1;
     for (uint32_t it = 0; ok; ++it) {
       const uint32_t is = it % kFwdItemSlots;
       if (!mbar_wait_warp(&bar_item_full[is], (it / kFwdItemSlots) & 1, abort_v, 31)) break;
-      const int code = s_item[is];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_item_empty[is]);
-      if (code < 0) break;
-      FwdItem item;
-      decode_item(P, p.H, p.heads, p.head_group, kShared, code, item);
-      const int qb = t == 0 ? item.qb[0] : item.qb[1];
-      if (qb >= NB) continue;
-      const int b = item.b, h = item.h;
-      const int n = t == 0 ? item.n[0] : item.n[1];
-      const int32_t* list = t == 0 ? item.list[0] : item.list[1];
-      const int q = qb * kTile + row;
-      const bool q_valid = q < P.T;
-      constexpr int step = kShared ? 2 : 1;
-      const bool shared = kShared && item.n[1] > 0;  // both teams have a part of the query tile
-      if (kShared && t == 1 && n == 0) continue;
-      if (n == 0) {  // no readable key tile: defined result, nothing to compute
-        if (q_valid) {
-          __nv_bfloat16* orow = p.out + (size_t)b * p.o_sb + (size_t)h * p.o_sh + (size_t)q * p.o_st;
+      const FwdItem& item = s_item[is];  // stays until the warp is through with it; what only the end of an item needs is read again there
+      if (item.code < 0) break;
+      auto done = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_item_empty[is]);
+      };
+      const int qb = kShared ? item.qb : item.qb + t, n = item.n[t];
+      if (n == 0) {
+        // No readable key tile: a defined result, nothing to compute.  (A second team without a part leaves that to the first.)
+        const int q = qb * kTile + row;
+        if (q < P.T && !(kShared && t == 1)) {
+          __nv_bfloat16* orow = p.out + (size_t)item.b * p.o_sb + (size_t)item.h * p.o_sh + (size_t)q * p.o_st;
           for (int i = 0; i < D; i += 8) *reinterpret_cast<uint4*>(orow + i) = make_uint4(0, 0, 0, 0);
-          p.lse[((size_t)b * p.H + h) * P.T + q] = -CUDART_INF_F;
+          p.lse[((size_t)item.b * p.H + item.h) * P.T + q] = -CUDART_INF_F;
         }
+        done();
         continue;
       }
-      // Row of the plan's mask table for this query row: the number of its run inside the tile.  Rows of runs past the
-      // table, and all rows of sequences without one, work their masks out from the run lists (row_mask).
-      const uint4* masks = nullptr;
-      if (P.q_mask != nullptr) {  // rows past the sequence take the last run's masks: nothing of theirs is stored
-        const size_t tq = (size_t)b * NB + qb;
-        const int nr = __ldg(&P.run_cnt[tq]);
-        int run = -1;
-#pragma unroll
-        for (int r = 0; r < kMaskRuns + 1; ++r)
-          if (r < nr && __ldg(&P.runs[tq * kTile + r].start) <= row) run = r;
-        if (run < kMaskRuns) masks = P.q_mask + ((size_t)b * ((size_t)NB * (NB + 1) / 2) + mask_pair(qb, 0)) * kMaskRuns + run;
-      }
+      const int32_t* list = P.fwd_idx + ((size_t)item.b * NB + qb) * NB + (kShared ? t : 0) + 2 * step;
       // List entries are fetched two tiles ahead and the mask of a partial tile one tile ahead, so that their latency
       // hides behind the sweeps of the tile before.
-      int e_cur = ld_nc_i32_here(list);
-      int e_nxt = n > 1 ? ld_nc_i32_here(list + step) : 0;
+      int e_cur = item.first[t][0], e_nxt = item.first[t][1];
+      // Row of the plan's mask table for this query row: the number of its run inside the tile.  Rows of runs past the
+      // table, and all rows of sequences without one, work their masks out from the run lists (row_mask).
+      // Rows past the sequence take the last run's masks: nothing of theirs is stored.
+      uint32_t masks = kNoMasks;  // place in the table of this row's mask for key tile 0 (the table of as many batch elements as fit the card has fewer places)
+      if (P.q_mask != nullptr) {
+        int run = -1;
+        const int nr = item.n_runs[t];
+#pragma unroll
+        for (int r = 0; r < kMaskRuns + 1; ++r)
+          if (r < nr && item.runs[kShared ? 0 : t][r].start <= row) run = r;
+        if (run < kMaskRuns) masks = (item.b * (uint32_t)(NB * (NB + 1) / 2) + (uint32_t)(qb * (qb + 1) / 2)) * kMaskRuns + run;
+      }
       int4 mask_pf = make_int4(0, 0, 0, 0);
       auto prefetch_mask = [&](int entry) {
         if (entry & kFullBit) return;
-        const int kbp = min(max(entry, 0), qb);
-        if (masks != nullptr) mask_pf = ld_nc_v4_here(masks + (size_t)kbp * kMaskRuns);
+        if (masks != kNoMasks) mask_pf = ld_nc_v4_here(P.q_mask + (masks + min((uint32_t)entry, (uint32_t)qb) * kMaskRuns));
       };
       prefetch_mask(e_cur);
       float m_used = -CUDART_INF_F, l = 0.f;
       FTRACE_ACC(0);
-      // The store of the warp's last rows must have read their places, which at D = 128 are P's.
-      if (lane == 0) tma_store_wait_read0();
-      __syncwarp();
-      for (int j = 0; j < n && ok; ++j) {
+      if constexpr (!Cfg::kTmemP) {  // the store of the warp's last rows must have read their places, which are P's
+        if (lane == 0) tma_store_wait_read0();
+        __syncwarp();
+      }
+      for (int left = n; left > 0; --left) {
         const int entry = e_cur;
         e_cur = e_nxt;
-        if (j + 2 < n) e_nxt = ld_nc_i32_here(list + (j + 2) * step);
+        if (left > 2) e_nxt = ld_nc_i32_here(list);
+        list += step;
         const int kb = entry & ~kFullBit;
-        if (kb < 0 || kb >= NB) { atomicCAS(abort_w, 0, 38); ok = false; break; }
+        if ((uint32_t)kb >= (uint32_t)NB) { atomicCAS(abort_w, 0, 38); ok = false; break; }
         const int4 mask_cur = mask_pf;
-        if (j + 1 < n) prefetch_mask(e_cur);
+        if (left > 1) prefetch_mask(e_cur);
         FTRACE_ACC(7);
         auto tile = [&](auto masked_tag) {
           constexpr bool kMasked = decltype(masked_tag)::value;
@@ -562,10 +634,10 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
         bool dead[4] = {false, false, false, false}, mixed[4] = {false, false, false, false};
         if (kMasked) {
           // 128-bit mask of the key columns this row may read, before causality
-          if (masks != nullptr) {
+          if (masks != kNoMasks) {
             bits[0] = mask_cur.x; bits[1] = mask_cur.y; bits[2] = mask_cur.z; bits[3] = mask_cur.w;
           } else {
-            const uint4 m4 = row_mask(P, p.mask, b, qb, kb, row);
+            const uint4 m4 = row_mask(P, p.mask, item.b, qb, kb, row);
             bits[0] = m4.x; bits[1] = m4.y; bits[2] = m4.z; bits[3] = m4.w;
           }
           if (kb == qb) {  // causal inside the diagonal tile: columns 0..row
@@ -654,7 +726,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
             if (n_tiles > 0 && !mbar_try_wait(&bar_pv[t], (n_tiles - 1) & 1)) wait_longer(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 33);
             tc_fence_after();  // P and O, both read or written by that product, are overwritten below
             if (row == 0) FTRACE(2 * t + 1, n_tiles, 5);
-            if (any_need && j > 0) {
+            if (any_need && left < n) {
               const unsigned long long f2 = pack_f32x2(factor, factor);
 #pragma unroll 1
               for (int cc = 0; cc < D / 32; ++cc) {
@@ -714,80 +786,87 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
       //      TMA store.  A warp stores its own 32 rows, so that the team's warps need not meet.
       if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[t], (n_tiles - 1) & 1, abort_v, 34) && *abort_v == 0))) break;
       tc_fence_after();
+      const int b = item.b, h = item.h, q = qb * kTile + row;
+      const bool shared = kShared && item.n[1] > 0;  // both teams have a part of the query tile
       // Teams that share the query tile: team 1 leaves its part where it is, team 0 scales both to one maximum and adds them up.
-      float f0 = 1.f, f1 = 0.f;
-      if (shared) {
-        if (t == 1) {
-          s_merge[row] = make_float2(m_used, l);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_merge);
-          continue;
-        }
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_merge, n_merged & 1, abort_v, 35) && *abort_v == 0))) break;
-        tc_fence_after();
-        ++n_merged;
-        const float2 other = s_merge[row];
-        const float m = fmaxf(m_used, other.x);
-        f0 = m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m);
-        f1 = other.x == -CUDART_INF_F ? 0.f : fast_exp2(other.x - m);
-        m_used = m;
-        l = l * f0 + other.y * f1;
-      }
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      f0 *= inv;
-      f1 *= inv;
-#pragma unroll 1
-      for (int s = 0; s < Cfg::kSub; ++s) {
-        uint32_t o[2][32];
-        tmem_ld32(tOr + s * 64, o[0]);
-        tmem_ld32(tOr + s * 64 + 32, o[1]);
+      if (shared && t == 1) {
+        s_merge[row] = make_float2(m_used, l);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_merge);
+      } else {
+        float f0 = 1.f, f1 = 0.f;
         if (shared) {
-          uint32_t o1[2][32];
-          tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64, o1[0]);
-          tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64 + 32, o1[1]);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0 + __uint_as_float(o1[i >> 5][i & 31]) * f1);
-        } else {
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 64; ++i) o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0);
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_merge, n_merged & 1, abort_v, 35) && *abort_v == 0))) break;
+          tc_fence_after();
+          ++n_merged;
+          const float2 other = s_merge[row];
+          const float m = fmaxf(m_used, other.x);
+          f0 = m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m);
+          f1 = other.x == -CUDART_INF_F ? 0.f : fast_exp2(other.x - m);
+          m_used = m;
+          l = l * f0 + other.y * f1;
         }
-        if (s == Cfg::kSub - 1) {
-          tc_fence_before();
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        f0 *= inv;
+        f1 *= inv;
+        if constexpr (Cfg::kTmemP) {  // the store of the warp's last rows must have read theirs
+          if (lane == 0) tma_store_wait_read0();
           __syncwarp();
-          if (lane == 0) {  // the next item's first P V may overwrite O
-            mbar_arrive(&bar_ofree[t]);
-            if (shared) mbar_arrive(&bar_ofree[1]);
+        }
+#pragma unroll 1
+        for (int s = 0; s < Cfg::kSub; ++s) {
+          uint32_t o[2][32];
+          tmem_ld32(tOr + s * 64, o[0]);
+          tmem_ld32(tOr + s * 64 + 32, o[1]);
+          if (shared) {
+            uint32_t o1[2][32];
+            tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64, o1[0]);
+            tmem_ld32(tOr + Cfg::out_col(1) - Cfg::out_col(0) + s * 64 + 32, o1[1]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+              o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0 + __uint_as_float(o1[i >> 5][i & 31]) * f1);
+          } else {
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 64; ++i) o[i >> 5][i & 31] = __float_as_uint(__uint_as_float(o[i >> 5][i & 31]) * f0);
+          }
+          if (s == Cfg::kSub - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {  // the next item's first P V may overwrite O
+              mbar_arrive(&bar_ofree[t]);
+              if (shared) mbar_arrive(&bar_ofree[1]);
+            }
+          }
+          uint8_t* box = sPt + s * 16384 + (warp & 3) * (32 * 128);
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const uint32_t* w = &o[g >> 2][(g & 3) * 8];
+            uint4 v;
+            v.x = pack_bf16(__uint_as_float(w[0]), __uint_as_float(w[1]));
+            v.y = pack_bf16(__uint_as_float(w[2]), __uint_as_float(w[3]));
+            v.z = pack_bf16(__uint_as_float(w[4]), __uint_as_float(w[5]));
+            v.w = pack_bf16(__uint_as_float(w[6]), __uint_as_float(w[7]));
+            *reinterpret_cast<uint4*>(box + sw128_offset(lane, g)) = v;
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const int first = qb * kTile + (warp & 3) * 32;
+            if (first < P.T) tma_store_tile(&mapO, box, first, s, h, b);
+            tma_store_commit();
           }
         }
-        uint8_t* box = sPt + s * 16384 + (warp & 3) * (32 * 128);
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const uint32_t* w = &o[g >> 2][(g & 3) * 8];
-          uint4 v;
-          v.x = pack_bf16(__uint_as_float(w[0]), __uint_as_float(w[1]));
-          v.y = pack_bf16(__uint_as_float(w[2]), __uint_as_float(w[3]));
-          v.z = pack_bf16(__uint_as_float(w[4]), __uint_as_float(w[5]));
-          v.w = pack_bf16(__uint_as_float(w[6]), __uint_as_float(w[7]));
-          *reinterpret_cast<uint4*>(box + sw128_offset(lane, g)) = v;
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          const int first = qb * kTile + (warp & 3) * 32;
-          if (first < P.T) tma_store_tile(&mapO, box, first, s, h, b);
-          tma_store_commit();
+        if (q < P.T) {
+          // One rounding less where the sum is one of two parts, for those that adding them up takes: against 64 bits lse was 1-5 % further off
+          // there than in a row that one team adds up (attention at T = 219 to 4096), and is 6-11 % closer now.
+          constexpr float kLn2 = 0.6931471805599453f;
+          p.lse[((size_t)b * p.H + h) * P.T + q] = l > 0.f ? (shared ? fmaf(m_used, kLn2, log2f(l) * kLn2) : (m_used + log2f(l)) * kLn2) : -CUDART_INF_F;
         }
       }
-      if (q_valid) {
-        // One rounding less where the sum is one of two parts, for those that adding them up takes: against 64 bits lse was 1-5 % further off
-        // there than in a row that one team adds up (attention at T = 219 to 4096), and is 6-11 % closer now.
-        constexpr float kLn2 = 0.6931471805599453f;
-        p.lse[((size_t)b * p.H + h) * P.T + q] = l > 0.f ? (shared ? fmaf(m_used, kLn2, log2f(l) * kLn2) : (m_used + log2f(l)) * kLn2) : -CUDART_INF_F;
-      }
+      done();
       FTRACE_ACC(4);
     }
     if (lane == 0) tma_store_wait_all();  // the stores read this CTA's shared memory
@@ -807,29 +886,53 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
   if (tid == 0) fwd_leave(P);
 }
 
-// Which work items a launch has: pairs of query tiles, query tiles that the teams share, or whichever of the two the lists call for.
+// Which work items a launch has: query tiles that the teams share, or pairs of query tiles or shared ones, whichever the lists call for.
 enum FwdForm { kFwdPairs, kFwdShared, kFwdByLists };
 
-// Every CTA comes to the same answer, because it depends on the plan and the grid (one CTA per SM) alone.  Pairs that all run at once take
-// as long as the longest list; shared tiles, two rounds of them, as long as an SM's share of all lists, two key tiles at a time, at 1.6 times
-// the time of a step whose SM has one team to serve, and two steps for the second item.  Both forms measured on 66 calls of 160 to 288 query
-// tiles (D = 64 and 128, longest list 2 to 128): where this line takes the slower one it is by 2 % at most.
-// A kernel with both bodies runs the one that comes first in its code 0.2-0.6 us slower than a kernel of its own, and the other one 2-3 us;
-// so the pairs, whose launches are the short ones, come first (us, pairs | shared tiles | by the lists: documents of 200 to 300 in 4096, H = 7,
-// D = 128 16.4 | 19.6 | 16.6, D = 64 14.3 | 17.0 | 14.9, of 300 to 600 in 30000, one head 21.8 | 24.2 | 22.0; causal 4096, H = 8, D = 64 60.3 | 47.4 | 50.3).  One body that asks at run time costs both.
-__device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p) {
-  return 5 * (p.plan.status[kLongestList] - 2) * static_cast<int>(gridDim.x) > 4 * p.plan.status[kAllLists] * p.H;
+// Every CTA comes to the same answer, because it depends on the plan and the grid (one CTA per SM) alone.  As pairs a launch that is short of items takes as long
+// as its longest list, 2.0 us a tile and 2.2 us at its ends.  As shared tiles it takes an SM's share of all lists, two tiles at a time in 1.65 us (D = 64; 2.0 us at
+// D = 128, where two K/V streams do not fit the ring), and 2.7 us for each of the SM's items.  Shared tiles are taken where they come to less than 0.8 of the pairs'
+// time: of 90 random calls (T = 512 to 20000, 1 to 4 sequences, 2 to 16 heads, all kinds of masks) that picks the slower form by more than 4 % twice (12 and 13 %).  us, pairs | shared:
+// linked 14545, H = 3, D = 128 144 | 89; linked 5169, H = 8, D = 64 87 | 54; causal 4 x 3787, H = 3, D = 128 77 | 56; at the line linked 2 x 3156, H = 12, D = 64
+// 48.0 | 48.3 and 6273, H = 12, D = 128 92 | 91; beyond it linked 2 x 2455, H = 16, D = 64 46 | 50, causal 4 x 2902, H = 12, D = 64 101 | 108.
+// A kernel with both bodies runs either one up to 1.5 us slower than a kernel of its own.
+template <int D>
+__device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p, long long longest, long long all) {
+  return (D == 64 ? 33 : 40) * all * p.H + 108ll * p.n_tiles < gridDim.x * (64 * longest + 70);
 }
 
 template <int D, int kForm>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const FwdPlaces<D> at(smem_raw);
+  const PlanView& P = p.plan;
+  const uint32_t tmem = fwd_setup<D>(at);
+  if (threadIdx.x == 0) FTRACE_SPAN(0);
+  // What came before in the stream ends under the lines above; the plan is read from here on.
   wait_previous();
-  if constexpr (kForm == kFwdPairs) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p);
-  else if constexpr (kForm == kFwdShared) fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
-  else if (!lists_call_for_shared(p)) fwd_items<D, false, true>(mapQ, mapK, mapV, mapO, p);
-  else fwd_items<D, true>(mapQ, mapK, mapV, mapO, p);
+  int first[2] = {0, 0};
+  if (threadIdx.x == kFwdProducerWarp * 32) {  // on their way while the plan's stamp is looked at; inside the plan's buffer whatever it holds
+    int b, h;
+    if (kForm != kFwdShared && static_cast<int>(blockIdx.x) < p.n_pairs) first[0] = ld_nc_i32_here(item_place(P, p.H, p.heads, p.head_group, false, blockIdx.x, b, h));
+    if (kForm != kFwdPairs && static_cast<int>(blockIdx.x) < p.n_tiles) first[1] = ld_nc_i32_here(item_place(P, p.H, p.heads, p.head_group, true, blockIdx.x, b, h));
+  }
+  const int magic = P.status[kStampMagic], plan_b = P.status[kStampB], plan_t = P.status[kStampT], longest = P.status[kLongestList], all = P.status[kAllLists];
+  const bool share = kForm == kFwdShared || (kForm == kFwdByLists && lists_call_for_shared<D>(p, longest, all));
+  // Uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window.  A CTA without an item leaves
+  // behind that, because a plan that is refused must not keep a part of the count.
+  const int bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T ? 1900 : at.smem + FwdSmem<D>::kSmall + FwdSmem<D>::kSmallBytes > at.raw + FwdSmem<D>::kBytes ? 1901 : 0;
+  if (bad || static_cast<int>(blockIdx.x) >= (share ? p.n_tiles : p.n_pairs)) {
+    if (threadIdx.x / 32 == kFwdIssuerWarp) tmem_dealloc(tmem, 512);
+    if (threadIdx.x == 0) {
+      if (bad) atomicCAS(P.status, 0, bad);
+      else fwd_leave(P);
+    }
+    return;
+  }
+  if (kForm == kFwdPairs || (kForm == kFwdByLists && !share)) fwd_items<D, false>(mapQ, mapK, mapV, mapO, p, at, tmem, first[0]);
+  else fwd_items<D, true>(mapQ, mapK, mapV, mapO, p, at, tmem, first[1]);
 }
 
 // Host launcher.  Tensor strides are in elements; the last dimension is contiguous.
@@ -848,7 +951,7 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   p.o_sb = so[0]; p.o_sh = so[1]; p.o_st = so[2];
   p.H = H; p.scale_log2 = scale * 1.4426950408889634f;
   p.n_pairs = B * H * ((P.NB + 1) / 2);
-  p.n_items = kForm == kFwdPairs ? p.n_pairs : B * H * P.NB;
+  p.n_tiles = B * H * P.NB;
   {  // heads per group, from the K and V bytes of one head (2 x T x D bf16 each)
     const long long kv_bytes = 4ll * T * D;
     long long g = (static_cast<long long>(TS2TS_FWD_GROUP_MB) << 20) / (kv_bytes > 0 ? kv_bytes : 1);
@@ -864,7 +967,8 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
       return -110;
     attr_done[dev] = true;
   }
-  const unsigned grid = (unsigned)(p.n_items < sms ? p.n_items : sms);
+  const int most = kForm == kFwdPairs ? p.n_pairs : p.n_tiles;
+  const unsigned grid = (unsigned)(most < sms ? most : sms);
   FTRACE_ATTACH(p, stream);
   cudaError_t launched;
   {
@@ -876,15 +980,11 @@ static int launch_fwd_as(const void* q, const void* k, const void* v, void* out,
   return launched == cudaSuccess && last == cudaSuccess ? 0 : -111;
 }
 
-// Shared query tiles are twice as many and half as long, but bring in every key tile once a query tile instead of once a pair,
-// which costs 15 % (D = 64) to 33 % (D = 128) where the launch is long enough to be bound by throughput.  They win where it is as
-// long as its longest item.  That is so when all of them run at once: us, pairs -> shared, documents of up to 32 in 2048, H = 9, D = 64 12.9 -> 12.6,
-// linked 1024, H = 4, D = 64 16.6 -> 12.6; documents of 2048, H = 8, D = 64 18.8 -> 16.1; D = 128 20.8 -> 18.8 at H = 9.  Where all pairs run at once
-// but not all tiles, it depends on the lists from 32 tiles on, and the kernel looks at them: pairs for documents of up to 200 in 4096, H = 9
-// (shared tiles 14.7 -> 18.8 at D = 64, 16.8 -> 20.8 at D = 128), shared tiles for linked 16k, H = 2, D = 64 115 -> 77,
-// documents of up to 2048 in 4096, H = 9, D = 64 34.6 -> 28, causal 4096, H = 8, D = 128 68 -> 53.  With fewer tiles than 32 the lists are too short (documents of 2048, H = 16, D = 128 20.9 -> 23.0;
-// linked 4 x 700, H = 12, D = 64 18.8 -> 20.8), and with more pairs than SMs throughput counts (linked 5003, H = 12, D = 64 35 -> 43; causal 4k batch 4,
-// H = 16, D = 128 310 -> 420).
+// Shared query tiles are twice as many and half as long, but bring in every key tile once a query tile instead of once a pair, which costs 10 % (D = 64) to 25 %
+// (D = 128) where the launch is long enough to be bound by throughput (causal 4k batch 4, H = 16, D = 64 213 us as pairs, 234 shared; D = 128 282 and 350).  Where all of them run
+// at once they always win (linked 600, H = 8, D = 64 13.1 -> 11.4; linked 1024, H = 4, D = 64 22.8 -> 16).  Up to four pairs an SM it depends on the lists, and the kernel
+// looks at them; with more pairs the lists call for pairs (linked 4 x 17842, H = 2, D = 128, 3.8 an SM 242 as pairs, 250 shared; linked 2 x 14400, H = 8, D = 64, 6.2 an SM 269 and 275) or for neither
+// (linked 16k, H = 12, D = 64, 5.2 an SM 252 and 249).
 template <int D>
 static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, float* lse, const int64_t* sq, const int64_t* sk, const int64_t* sv,
                         const int64_t* so, int B, int H, int T, float scale, PlanView P, MaskArgs M, cudaStream_t stream) {
@@ -895,7 +995,7 @@ static int launch_fwd_t(const void* q, const void* k, const void* v, void* out, 
   if (sm_count[dev] <= 0 && (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0)) return -110;
   const int sms = sm_count[dev];
   const long long bh = (long long)B * H;
-  const bool by_lists = P.NB >= 32 && bh * ((P.NB + 1) / 2) <= sms;
+  const bool by_lists = bh * ((P.NB + 1) / 2) <= 4 * sms;
   const auto launch = bh * P.NB <= sms ? launch_fwd_as<D, kFwdShared> : by_lists ? launch_fwd_as<D, kFwdByLists> : launch_fwd_as<D, kFwdPairs>;
   return launch(q, k, v, out, lse, sq, sk, sv, so, B, H, T, scale, P, M, sms, stream);
 }

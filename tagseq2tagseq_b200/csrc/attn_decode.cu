@@ -8,13 +8,19 @@
 // the same predicate as the training kernels (cross_doc_mask.py:348-357), evaluated per key; no block plan is needed.
 //
 // HBM-bound work: every allowed key's K and V row is read once, 4 D bytes per key and head.  One launch, grid
-// (cluster size, H, B), 16 warps a block.  The warps of a cluster share one (batch, head): warp w of W takes the groups of
-// 32 keys w, w + W, w + 2 W, ..., so that stretches without an allowed key spread over all of them.  It evaluates the mask
-// for up to four groups at a time (lane = key), queues the allowed keys in shared memory, and takes them off the queue
-// kUnroll at a time per row of lanes (D / 8 lanes hold one row, 16 bytes each), the K and V rows of all of them in flight
-// together: masked keys cost no traffic and no lane.  Each row of lanes keeps an online softmax (base 2) of its own; they
-// are merged by shuffles inside a warp, through shared memory inside a block and through distributed shared memory inside
-// the cluster, so no partial result goes to global memory.
+// (cluster size, H, B), 16 warps a block.  The blocks of a cluster share one (batch, head) and take its groups of 32 keys in turn.
+// A block works in rounds of up to 128 groups (one round for 4096 keys a block): its warps evaluate the mask, lane = key, and write the
+// allowed keys into one queue in shared memory, in order; then they take them off it in turn,
+// kUnroll keys at a time per row of lanes (D / 8 lanes hold one row, 16 bytes each), the K and V rows of all of them in flight
+// together: masked keys cost no traffic and no lane, and a document's keys, which lie together, are every warp's work.  Each row of lanes keeps an online
+// softmax (base 2) of its own; they are merged by shuffles inside a warp, through shared memory inside a block and through the first block's shared
+// memory inside the cluster, so no partial result goes to global memory.
+//
+// Warps that took the keys of their own groups waited for the one with most of them (GPU time alone, us, own groups -> one queue: linked 2 x 32768, H = 16,
+// D = 128, 8.3 k allowed keys 36.7 -> 30.3 (21 at the copy rate); 16 x 8192, H = 16, D = 128 45.2 -> 38.5; 20000, H = 16, D = 64 13.7 -> 12.0; all keys allowed, 2 x 32768,
+// 84.3 -> 85.6).  Up to 64 groups a block the queue's two barriers cost more than that (own | one: eight of 1111, H = 12, D = 64 6.2 | 8.0; 4 x 4590 7.2 | 9.8; at the
+// line 8 x 1852, H = 8, D = 128 8.1 | 9.9, all keys of 16 x 2048 46.5 | 51.9), and warps keep their own.  Before the merge went through the first block's memory these
+// were 7.2, 8.5, 9.1 and 50.3.
 //
 // B = 2, H = 16, Tk = 32768, D = 128, 13.9 k allowed keys a sequence (228 MB): two kernels over fixed 128-key tiles with K
 // before V took 75 + 41 us (a third of the copy rate; the merge walked 256 partial results one after the other).
@@ -44,7 +50,11 @@ struct DecodeParams {
   float scale_log2;
 };
 
-constexpr int kDecWarps = 16, kDecGroups = 4, kUnroll = 4;
+constexpr int kDecWarps = 16, kDecGroups = 8, kDecAtOnce = 4, kUnroll = 4, kDecCluster = 8;  // kDecCluster: the largest cluster that every part of the chip takes
+
+// Arrival publishes what the block has written, the other blocks' shared memory included.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void row_dot(const uint4& raw, const float (&q)[8], float& acc) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -69,8 +79,8 @@ __device__ __forceinline__ bool may_read(const DecodeParams& p, const int64_t* l
   return (static_cast<unsigned long long>(__ldg(link_row + (col >> 6))) >> (col & 63)) & 1ull;
 }
 
-// A warp's keys once more, kRows at a time and asking for weights of zero: m, l and o into `r`.  For rows that came out as no
-// number: keys without weight (padded slots, underflow, all before a maximum that outweighs them) add nothing, whatever
+// A block's keys once more, a warp's share in groups, kRows at a time and asking for weights of zero: m, l and o into `r`.  For blocks in which a row came out
+// as no number: keys without weight (padded slots, underflow, all before a maximum that outweighs them) add nothing, whatever
 // their values, but 0 * inf is no number.  Asking at every key of the first pass cost everybody (B = 2, H = 16, Tk = 32768,
 // D = 128: 42.1 -> 45.6 us, or 44.1 us with this pass inlined behind it).
 template <int D>
@@ -88,7 +98,7 @@ __device__ __noinline__ void read_carefully(const DecodeParams& p, int qpos, flo
     o[i] = 0.f;
   }
 #pragma unroll 1
-  for (int g = blockIdx.x * kDecWarps + warp; g < qpos / 32 + 1; g += gridDim.x * kDecWarps) {
+  for (int g = warp * gridDim.x + blockIdx.x; g < qpos / 32 + 1; g += gridDim.x * kDecWarps) {
     const int kv = g * 32 + lane;
     unsigned keys = __ballot_sync(0xffffffffu, kv <= qpos && may_read(p, link_row, qdoc, p.mask.doc[base + kv], p.mask.col[base + kv]));
 #pragma unroll 1
@@ -122,22 +132,39 @@ __device__ __noinline__ void read_carefully(const DecodeParams& p, int qpos, flo
   for (int i = 0; i < 8; ++i) r[2 + i] = o[i];
 }
 
-template <int D>
+// kQueue: the warps of a block share one queue.  Otherwise each has at most kDecAtOnce groups and takes its own keys.
+template <int D, bool kQueue>
 __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_constant__ DecodeParams p) {
   constexpr int kLanes = D / 8;            // lanes that share a row
   constexpr int kRows = 32 / kLanes;       // rows a warp reads at once
   constexpr int kBatch = kRows * kUnroll;  // keys a warp takes off its queue at once
-  __shared__ int s_queue[kDecWarps][kDecGroups * 32 + kBatch];
+  constexpr int kGroups = kQueue ? kDecGroups : kDecAtOnce;  // of a warp in a round
+  __shared__ int s_queue[kDecWarps * kGroups * 32];
+  __shared__ __align__(16) int s_count[kDecWarps * kGroups];
   __shared__ float s_m[kDecWarps], s_l[kDecWarps], s_o[kDecWarps][D];
-  __shared__ float s_block[2 + D];         // the block's maximum, sum and unnormalised output row, read by the cluster's first block
+  __shared__ float s_part[kDecCluster][2 + D];  // in the cluster's first block: every block's maximum, sum and unnormalised output row
   const cg::cluster_group cluster = cg::this_cluster();
   const int h = blockIdx.y, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cs = gridDim.x, W = cs * kDecWarps;
+  const int cs = gridDim.x;
+  cluster_arrive();  // each block is there before another one writes into its shared memory
   wait_previous();
-  const int qpos = p.q_pos ? min(max(p.q_pos[b], 0), p.Tk - 1) : p.Tk - 1;
   const size_t base = (size_t)b * p.Tk;
   const int32_t* docs = p.mask.doc + base;
   const int32_t* cols = p.mask.col + base;
+  // Group u of this warp in the round that starts at the block's group `first`.
+  auto group_at = [&](int first, int u) { return (first + u * kDecWarps + warp) * cs + blockIdx.x; };
+  // The mask inputs of kDecAtOnce groups; tokens past the query are loaded too, and not looked at.
+  int doc[kDecAtOnce], col[kDecAtOnce];
+  auto fetch = [&](int first) {
+#pragma unroll
+    for (int u = 0; u < kDecAtOnce; ++u) {
+      const int kv = group_at(first, u) * 32 + lane;
+      doc[u] = kv < p.Tk ? ld_nc_i32_here(docs + kv) : 0;
+      col[u] = p.mask.link != nullptr && kv < p.Tk ? ld_nc_i32_here(cols + kv) : -1;
+    }
+  };
+  if constexpr (kQueue) fetch(0);  // on their way while the query token's are (ten registers too many where a warp has few groups: eight caches of 1111 6.2 -> 6.7 us)
+  const int qpos = p.q_pos ? min(max(p.q_pos[b], 0), p.Tk - 1) : p.Tk - 1;
   const int qdoc = docs[qpos];
   const int64_t* link_row = nullptr;
   if (p.mask.link != nullptr) {
@@ -157,15 +184,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_
     }
   }
   float m = -CUDART_INF_F, l = 0.f;
-  int* queue = s_queue[warp];
-  int queued = 0;
 
-  // `count` keys off the queue from `from`; slots past the last one repeat it with a score of -inf
-  auto take = [&](int from, int count) {
+  // `count` keys of the queue from `first_key` on; slots past the last one repeat it with a score of -inf
+  auto take = [&](int first_key, int count) {
     uint4 kr[kUnroll], vr[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-      const int key = queue[from + min(u * kRows + sub, count - 1)];
+      const int key = s_queue[first_key + min(u * kRows + sub, count - 1)];
       kr[u] = __ldg(reinterpret_cast<const uint4*>(kbase + (size_t)key * p.k_st));
       vr[u] = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)key * p.v_st));
     }
@@ -193,43 +218,79 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_
     }
   };
 
-  const int n_groups = qpos / 32 + 1;
-  for (int g0 = blockIdx.x * kDecWarps + warp; g0 < n_groups; g0 += kDecGroups * W) {
-    int doc[kDecGroups], col[kDecGroups];
+  // Which keys of the kDecAtOnce groups that `doc` and `col` belong to are allowed, a ballot a group.
+  auto allowed = [&](int first, unsigned (&ok)[kDecAtOnce]) {
+    unsigned long long word[kDecAtOnce];
 #pragma unroll
-    for (int u = 0; u < kDecGroups; ++u) {
-      const int kv = (g0 + u * W) * 32 + lane;
-      doc[u] = kv <= qpos ? docs[kv] : 0;
-      col[u] = link_row != nullptr && kv <= qpos ? cols[kv] : -1;
+    for (int u = 0; u < kDecAtOnce; ++u) {
+      const int kv = group_at(first, u) * 32 + lane;
+      const bool ask = kv <= qpos && doc[u] != qdoc && link_row != nullptr && col[u] >= 0 && col[u] < 64 * p.mask.W;
+      word[u] = ask ? static_cast<unsigned long long>(__ldg(link_row + (col[u] >> 6))) : 0ull;
     }
 #pragma unroll
-    for (int u = 0; u < kDecGroups; ++u) {
-      const int kv = (g0 + u * W) * 32 + lane;
-      bool ok = false;
-      if (kv <= qpos) {
-        ok = doc[u] == qdoc;
-        if (!ok && col[u] >= 0 && col[u] < 64 * p.mask.W)
-          ok = (static_cast<unsigned long long>(__ldg(link_row + (col[u] >> 6))) >> (col[u] & 63)) & 1ull;
+    for (int u = 0; u < kDecAtOnce; ++u) {
+      const int kv = group_at(first, u) * 32 + lane;
+      ok[u] = __ballot_sync(0xffffffffu, kv <= qpos && (doc[u] == qdoc || ((word[u] >> (col[u] & 63)) & 1ull)));
+    }
+  };
+  const unsigned below = (1u << lane) - 1u;
+  if constexpr (!kQueue) {
+    int* queue = s_queue + warp * (kGroups * 32);
+    unsigned ok[kDecAtOnce];
+    fetch(0);
+    allowed(0, ok);
+    int total = 0;
+#pragma unroll
+    for (int u = 0; u < kDecAtOnce; ++u) {
+      if ((ok[u] >> lane) & 1u) queue[total + __popc(ok[u] & below)] = group_at(0, u) * 32 + lane;
+      total += __popc(ok[u]);
+    }
+    __syncwarp();
+    int from = 0;
+    for (; from + kBatch <= total; from += kBatch) take(warp * (kGroups * 32) + from, kBatch);
+    if (from < total) take(warp * (kGroups * 32) + from, total - from);
+  } else {
+    for (int first = 0; first * cs + blockIdx.x < qpos / 32 + 1; first += kDecWarps * kGroups) {
+      if (first > 0) __syncthreads();  // the queue of the last round has been read
+      unsigned ok[kGroups / kDecAtOnce][kDecAtOnce];
+#pragma unroll
+      for (int v = 0; v < kGroups / kDecAtOnce; ++v) {
+        const int from = first + v * kDecAtOnce * kDecWarps;
+        if (from > 0) fetch(from);
+        allowed(from, ok[v]);
+#pragma unroll
+        for (int u = 0; u < kDecAtOnce; ++u)
+          if (lane == 0) s_count[(v * kDecAtOnce + u) * kDecWarps + warp] = __popc(ok[v][u]);
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) queue[queued + __popc(bal & ((1u << lane) - 1u))] = kv;
-      queued += __popc(bal);
+      __syncthreads();
+      // Places in the queue by group: a lane adds up four neighbouring counts; this warp's are the same one of each lane's.
+      static_assert(kDecWarps % 4 == 0 && kDecWarps * kDecGroups == 128, "");
+      const int4 c = reinterpret_cast<const int4*>(s_count)[lane];
+      const int four = c.x + c.y + c.z + c.w, mine = warp & 3;
+      int upto = four;
+#pragma unroll
+      for (int x = 1; x < 32; x <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, upto, x);
+        if (lane >= x) upto += o;
+      }
+      const int total = __shfl_sync(0xffffffffu, upto, 31);
+      const int before = upto - four + (mine > 0 ? c.x : 0) + (mine > 1 ? c.y : 0) + (mine > 2 ? c.z : 0);
+#pragma unroll
+      for (int u = 0; u < kGroups; ++u) {
+        const unsigned keys = ok[u / kDecAtOnce][u % kDecAtOnce];
+        const int place = __shfl_sync(0xffffffffu, before, (u * kDecWarps + warp) / 4);
+        if ((keys >> lane) & 1u) s_queue[place + __popc(keys & below)] = group_at(first, u) * 32 + lane;
+      }
+      __syncthreads();
+      int from = warp * kBatch;
+      for (; from + kBatch <= total; from += kDecWarps * kBatch) take(from, kBatch);
+      if (from < total) take(from, total - from);
     }
-    __syncwarp();
-    int done = 0;
-    for (; queued - done >= kBatch; done += kBatch) take(done, kBatch);
-    const int left = queued - done;
-    const int kept = lane < left ? queue[done + lane] : 0;
-    __syncwarp();
-    if (lane < left) queue[lane] = kept;
-    queued = left;
-    __syncwarp();
   }
-  if (queued > 0) take(0, queued);
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < 8; ++i) bad = bad || o[i] != o[i];
-  if (__any_sync(0xffffffffu, bad)) {
+  if (__syncthreads_or(bad)) {
     float r[10];
     read_carefully<D>(p, qpos, r);
     m = r[0]; l = r[1];
@@ -257,6 +318,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_
   }
   if (lane == 0) { s_m[warp] = mw; s_l[warp] = l; }
   __syncthreads();
+  cluster_wait();
   // warps -> block
   const int d = threadIdx.x;
   if (d < D) {
@@ -270,26 +332,30 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_
       lb = fmaf(f, s_l[w], lb);
       ob = fmaf(f, f == 0.f ? 0.f : s_o[w][d], ob);
     }
-    if (d == 0) { s_block[0] = mb; s_block[1] = lb; }
-    s_block[2 + d] = ob;
+    // blocks -> the first one: written there, so that it reads its own shared memory instead of the others' (two round trips less at the end)
+    float* part = cluster.map_shared_rank(&s_part[blockIdx.x][0], 0);
+    if (d == 0) { part[0] = mb; part[1] = lb; }
+    part[2 + d] = ob;
   }
-  cluster.sync();
-  // blocks -> out
-  if (blockIdx.x == 0 && d < D) {
-    float mc = -CUDART_INF_F;
-    for (int r = 0; r < cs; ++r) mc = fmaxf(mc, *cluster.map_shared_rank(&s_block[0], r));
+  cluster_arrive();
+  if (blockIdx.x > 0) return;
+  cluster_wait();
+  if (d < D) {
+    float mc = s_part[0][0];
+#pragma unroll
+    for (int r = 1; r < kDecCluster; ++r) mc = r < cs ? fmaxf(mc, s_part[r][0]) : mc;
     float lc = 0.f, oc = 0.f;
-    for (int r = 0; r < cs; ++r) {
-      const float mr = *cluster.map_shared_rank(&s_block[0], r), lr = *cluster.map_shared_rank(&s_block[1], r);
-      const float xr = *cluster.map_shared_rank(&s_block[2 + d], r);
+#pragma unroll
+    for (int r = 0; r < kDecCluster; ++r) {
+      if (r >= cs) break;
+      const float mr = s_part[r][0];
       const float f = mr == -CUDART_INF_F ? 0.f : fast_exp2(mr - mc);
-      lc = fmaf(f, lr, lc);
-      oc = fmaf(f, f == 0.f ? 0.f : xr, oc);
+      lc = fmaf(f, s_part[r][1], lc);
+      oc = fmaf(f, f == 0.f ? 0.f : s_part[r][2 + d], oc);
     }
     p.out[(size_t)b * p.o_sb + (size_t)h * p.o_sh + d] = __float2bfloat16(lc > 0.f ? oc / lc : 0.f);
     if (d == 0) p.lse[(size_t)b * p.H + h] = lc > 0.f ? (mc + log2f(lc)) * 0.6931471805599453f : -CUDART_INF_F;
   }
-  cluster.sync();  // the first block has read the others' shared memory
 }
 
 // No partial results go through global memory; the argument stays part of the interface.
@@ -308,11 +374,10 @@ int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq
   p.lse = lse;
   p.H = H; p.Tk = Tk;
   p.scale_log2 = scale * 1.4426950408889634f;
-  // Blocks per (batch, head): twice the SM count in all, as long as every warp gets two groups of keys; eight is the
-  // largest cluster every part of the chip takes.
+  // Blocks per (batch, head): twice the SM count in all, as long as every warp gets two groups of keys.
   const long long groups = (Tk + 31) / 32;
   int cs = 1;
-  while (cs < 8 && (long long)B * H * cs < 2 * 148 && groups >= 2ll * kDecWarps * 2 * cs) cs *= 2;
+  while (cs < kDecCluster && (long long)B * H * cs < 2 * 148 && groups >= 2ll * kDecWarps * 2 * cs) cs *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, H, B);
   cfg.blockDim = dim3(kDecWarps * 32);
@@ -324,8 +389,9 @@ int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
   cfg.numAttrs = 2;
-  if (D == 128) return cudaLaunchKernelEx(&cfg, decode_kernel<128>, p) == cudaSuccess ? 0 : -141;
-  if (D == 64) return cudaLaunchKernelEx(&cfg, decode_kernel<64>, p) == cudaSuccess ? 0 : -141;
+  const bool queue = groups > (long long)cs * kDecWarps * kDecAtOnce;
+  if (D == 128) return cudaLaunchKernelEx(&cfg, queue ? decode_kernel<128, true> : decode_kernel<128, false>, p) == cudaSuccess ? 0 : -141;
+  if (D == 64) return cudaLaunchKernelEx(&cfg, queue ? decode_kernel<64, true> : decode_kernel<64, false>, p) == cudaSuccess ? 0 : -141;
   return -142;
 }
 

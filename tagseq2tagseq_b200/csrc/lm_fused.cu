@@ -9,12 +9,15 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "launch.cuh"
 #include "ptx.cuh"
 
 namespace ts2ts {
 namespace {
 
+template <int N> struct IntTag { static constexpr int value = N; };
 constexpr int kMaxVec = 4;  // float4 per thread and row in the wide variant: C <= 16 * blockDim.x
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -379,23 +382,53 @@ __global__ void ce_bwd_kernel(__nv_bfloat16* logits, const int64_t* __restrict__
 // for the log-sum-exp and again for the gradient, which is written over the logits.  HBM-bound, 4 bytes per logit
 // instead of the 6 of the two kernels above; two blocks of a 50304-logit row share an SM, so that one's copy overlaps the
 // other's arithmetic.  The gradient is that of the mean loss (times inv_n, not times what reaches the loss from above).
-constexpr int kCeThreads = 512, kCeChunks = 4, kCeRowBytes = 216 * 1024;
-__global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* logits, const int64_t* __restrict__ target,
+// What is left beside the copy are two exponentials a logit: maxima are taken of bf16 pairs, four vectors of a thread between two looks at the
+// running one, scale and shift are one packed multiply-add, only the target's vector knows of it.  A block has as many threads as leave each 8 to 16 vectors (12 to 27 from 4096 vectors on).
+// us (floor at the copy rate; one comparison and a maximum a logit, 512 threads whatever the row -> now): 16384 x 50304 (504) 641 -> 555, x 32768 (328) 415 -> 333,
+// x 16384 (164) 230 -> 166, x 4096 (41) 120 -> 49; 1024 x 4096 (3) 14.4 -> 11.1.  512 threads for x 32768 343, 256 for x 50304 574.
+constexpr int kCeRowBytes = 216 * 1024;
+constexpr uint32_t kNoLogits = 0xff80ff80u;  // two of -inf
+constexpr float kLog2e = 1.4426950408889634f;
+template <int kN>
+__device__ __forceinline__ float max_bf16x8(const uint4 (&raw)[kN]) {
+  __nv_bfloat162 most = *reinterpret_cast<const __nv_bfloat162*>(&raw[0].x);
+#pragma unroll
+  for (int u = 0; u < kN; ++u) {
+    const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) most = __hmax2(most, *reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+  }
+  return fmaxf(__low2float(most), __high2float(most));
+}
+// 2^(f log2(e) + shift) of eight values, two to a multiply-add.
+__device__ __forceinline__ void exp2_bf16x8(uint4 raw, float shift, float (&e)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  const unsigned long long scale2 = pack_f32x2(kLog2e, kLog2e), shift2 = pack_f32x2(shift, shift);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a, b;
+    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u)), scale2, shift2), a, b);
+    e[2 * i] = fast_exp2(a);
+    e[2 * i + 1] = fast_exp2(b);
+  }
+}
+template <int kThreads, int kChunks>
+__global__ void __launch_bounds__(kThreads) ce_fwd_grad_kernel(__nv_bfloat16* logits, const int64_t* __restrict__ target,
                                                                  float* __restrict__ loss, float inv_n, int V) {
   extern __shared__ __align__(128) uint8_t ce_row[];
-  __shared__ __align__(8) uint64_t bars[kCeChunks];
-  __shared__ float red_m[kCeThreads / 32], red_s[kCeThreads / 32];
+  __shared__ __align__(8) uint64_t bars[kChunks];
+  __shared__ float red_m[kThreads / 32], red_s[kThreads / 32];
   __shared__ int late;
   __nv_bfloat16* row = logits + (size_t)blockIdx.x * V;
-  const int n_vec = V / 8, per_chunk = (n_vec + kCeChunks - 1) / kCeChunks;  // in 16-byte vectors
+  const int n_vec = V / 8, per_chunk = (n_vec + kChunks - 1) / kChunks;  // in 16-byte vectors
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   wait_previous();
   target = settled(target);
   if (tid == 0) {
     late = 0;
-    for (int k = 0; k < kCeChunks; ++k) mbar_init(&bars[k], 1);
+    for (int k = 0; k < kChunks; ++k) mbar_init(&bars[k], 1);
     fence_mbar_init();
-    for (int k = 0; k < kCeChunks; ++k) {
+    for (int k = 0; k < kChunks; ++k) {
       const int first = min(k * per_chunk, n_vec), count = min(per_chunk, n_vec - first);
       mbar_expect_tx(&bars[k], count * 16);
       if (count > 0) bulk_load(ce_row + first * 16, row + first * 8, count * 16, &bars[k]);
@@ -406,31 +439,44 @@ __global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* 
   __syncthreads();
   const uint4* sv = reinterpret_cast<const uint4*>(ce_row);
   float m = -CUDART_INF_F, s = 0.f;
+  // up to kN vectors of this thread's, `kThreads` apart
+  auto sum_up = [&](auto vecs, int c, int end) {
+    constexpr int kN = decltype(vecs)::value;
+    uint4 raw[kN];
+#pragma unroll
+    for (int u = 0; u < kN; ++u) raw[u] = u == 0 || c + u * kThreads < end ? sv[c + u * kThreads] : make_uint4(kNoLogits, kNoLogits, kNoLogits, kNoLogits);
+    const float m_new = fmaxf(m, max_bf16x8(raw));
+    if (m_new == -CUDART_INF_F) return;
+    // sum of exp(f - m_new) as 2^(f log2(e) + shift); what rounding m_new log2(e) took away is multiplied back in
+    const float shift = -m_new * kLog2e;
+    unsigned long long sum[2] = {0ull, 0ull};
+#pragma unroll
+    for (int u = 0; u < kN; ++u) {
+      float e[8];
+      exp2_bf16x8(raw[u], shift, e);
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) sum[(i >> 1) & 1] = add_f32x2(sum[(i >> 1) & 1], pack_f32x2(e[i], e[i + 1]));
+    }
+    float a, b;
+    unpack_f32x2(add_f32x2(sum[0], sum[1]), a, b);
+    s = s * __expf(m - m_new) + (a + b) * fast_exp2(fmaf(-m_new, kLog2e, -shift));
+    m = m_new;
+  };
   bool ok = true;
-  for (int k = 0; k < kCeChunks; ++k) {
+  for (int k = 0; k < kChunks; ++k) {
     ok = ok && mbar_wait(&bars[k], 0, &late, 1);
     if (!ok) break;
     const int end = min((k + 1) * per_chunk, n_vec);
-    for (int c = k * per_chunk + tid; c < end; c += kCeThreads) {
-      float f[8];
-      bf16x8_to_float(sv[c], f);
-      float mx = f[0];
-#pragma unroll
-      for (int i = 1; i < 8; ++i) mx = fmaxf(mx, f[i]);
-      const float m_new = fmaxf(m, mx);
-      if (m_new == -CUDART_INF_F) continue;
-      float add = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) add += __expf(f[i] - m_new);
-      s = s * __expf(m - m_new) + add;
-      m = m_new;
-    }
+    int c = k * per_chunk + tid;
+    for (; c + 2 * kThreads < end; c += 4 * kThreads) sum_up(IntTag<4>{}, c, end);
+    if (c + kThreads < end) sum_up(IntTag<2>{}, c, end);
+    else if (c < end) sum_up(IntTag<1>{}, c, end);
   }
   const float wm = warp_max(m);
   s = warp_sum(m == -CUDART_INF_F ? 0.f : s * __expf(m - wm));
   if (lane == 0) { red_m[warp] = wm; red_s[warp] = s; }
   __syncthreads();
-  const float pm = lane < kCeThreads / 32 ? red_m[lane] : -CUDART_INF_F;
+  const float pm = lane < kThreads / 32 ? red_m[lane] : -CUDART_INF_F;
   const float m_all = warp_max(pm);
   const float s_all = warp_sum(pm == -CUDART_INF_F ? 0.f : red_s[lane] * __expf(pm - m_all));
   const float l = m_all + logf(s_all);
@@ -440,13 +486,20 @@ __global__ void __launch_bounds__(kCeThreads) ce_fwd_grad_kernel(__nv_bfloat16* 
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     return;
   }
-  const float g = live ? inv_n : 0.f;
-  for (int c = tid; c < n_vec; c += kCeThreads) {
+  const float g = live ? inv_n : 0.f, shift = -l * kLog2e, part = fast_exp2(fmaf(-l, kLog2e, -shift));
+  const unsigned long long scale2 = pack_f32x2(part * g, part * g);
+  const int hit_vec = live ? static_cast<int>(tg >> 3) : -1;
+#pragma unroll 2
+  for (int c = tid; c < n_vec; c += kThreads) {
     float f[8];
-    bf16x8_to_float(sv[c], f);
-    const int64_t first = (int64_t)c * 8;
+    exp2_bf16x8(sv[c], shift, f);
+    if (c != hit_vec) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = (__expf(f[i] - l) - (first + i == tg ? 1.f : 0.f)) * g;
+      for (int i = 0; i < 8; i += 2) unpack_f32x2(mul_f32x2(pack_f32x2(f[i], f[i + 1]), scale2), f[i], f[i + 1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = (f[i] * part - (i == static_cast<int>(tg & 7) ? 1.f : 0.f)) * g;
+    }
     reinterpret_cast<uint4*>(row)[c] = float_to_bf16x8(f);
   }
 }
@@ -486,7 +539,6 @@ __global__ void __launch_bounds__(256) scale_to_bf16_kernel(const float* __restr
 // tokens, 371 and 1317 us).  One id for all tokens is the worst case, 700 us at 16384 x 768.
 constexpr int kEmbBuckets = 256, kEmbThreads = 512, kEmbWarps = kEmbThreads / 32, kEmbEach = 4, kEmbStep = kEmbEach * kEmbThreads;
 constexpr int kEmbList = kEmbStep + 1024, kEmbVec = 4, kEmbCols = 128 * kEmbVec, kEmbHeavy = 64;
-template <int N> struct IntTag { static constexpr int value = N; };
 __device__ __forceinline__ void add4(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
 __global__ void __launch_bounds__(kEmbThreads) embedding_bwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ dx, float* dw, int N,
                                                                     int C, int64_t V) {
@@ -708,15 +760,18 @@ cudaError_t launch_ce_bwd(void* logits, const int64_t* target, const float* lse,
 int launch_ce_fwd_grad(void* logits, const int64_t* target, float* loss, float inv_n, int N, int V, cudaStream_t stream) {
   const int bytes = 2 * V;
   if (bytes > kCeRowBytes) return -1000;
-  static bool attr_done[64] = {};
+  using Kernel = void (*)(__nv_bfloat16*, const int64_t*, float*, float, int);
+  constexpr Kernel kernels[5] = {ce_fwd_grad_kernel<64, 1>, ce_fwd_grad_kernel<64, 4>, ce_fwd_grad_kernel<128, 4>, ce_fwd_grad_kernel<256, 4>, ce_fwd_grad_kernel<512, 4>};
+  const int n_vec = V / 8, which = n_vec <= 256 ? 0 : n_vec <= 1024 ? 1 : n_vec <= 2048 ? 2 : n_vec <= 4096 ? 3 : 4;
+  static bool attr_done[64][5] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -50;
-  if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(ce_fwd_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeRowBytes) != cudaSuccess) return -50;
-    attr_done[dev] = true;
+  if (!attr_done[dev][which]) {
+    if (cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, kCeRowBytes) != cudaSuccess) return -50;
+    attr_done[dev][which] = true;
   }
-  return launch_after(ce_fwd_grad_kernel, dim3(N), kCeThreads, bytes, stream, static_cast<__nv_bfloat16*>(logits), target, loss, inv_n, V) == cudaSuccess ? 0 : -50;
+  return launch_after(kernels[which], dim3(N), which == 0 ? 64 : 32 << which, bytes, stream, static_cast<__nv_bfloat16*>(logits), target, loss, inv_n, V) == cudaSuccess ? 0 : -50;
 }
 
 cudaError_t launch_scale(float* x, void* out_bf16, const float* gscale, int64_t n, cudaStream_t stream) {

@@ -255,17 +255,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t* s_masks = reinterpret_cast<uint32_t*>(bars + Cfg::kBars + 2);  // [Q stages][kStretches][kMaskRuns] the tile's masks, by run of the key
   uint32_t* s_tile = s_masks + Cfg::kQStages * kStretches * kMaskRuns;  // [kTileSlots][2] a tile's four stretch entries, 16 bits each
   static_assert(Cfg::kTileSlots > Cfg::kQStages, "");
-  {  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
-    int bad = 0;
-    const int32_t* stw = p.plan.status;
-    if (stw[kStampMagic] != kPlanMagic || stw[kStampB] != p.plan.B || stw[kStampT] != p.plan.T) bad = 2901;
-    else if (smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes) bad = 2900;
-    if (bad) {
-      if (threadIdx.x == 0) atomicCAS(p.plan.status, 0, bad);
-      wait_previous();
-      return;
-    }
-  }
   if (p.early) let_next_start();
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -283,26 +272,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   const int gsize = min(G, p.H - grp * G);
   const int rank = r2 / gsize;
   const int h = grp * G + (r2 - rank * gsize);
-  const int kb = min(max(P.bwd_order[(size_t)b * NB + rank], 0), NB - 1);
-  const int n = min(max((P.bwd_sub != nullptr ? P.bwd_tiles : P.bwd_cnt)[(size_t)b * NB + kb], 0), NB - kb);  // query tiles to walk
-  const int32_t* list = P.bwd_idx + ((size_t)b * NB + kb) * NB;
-  const uint16_t* subs = P.bwd_sub != nullptr ? P.bwd_sub + ((size_t)b * sub_line(NB, NB) + sub_line(NB, kb)) * kStretches : nullptr;
-
-  if (n == 0) {
-    if (tid < kTile) {
-      const int kv = kb * kTile + tid;
-      if (kv < P.T) {
-        __nv_bfloat16* a = p.dk + (size_t)b * p.dk_s[0] + (size_t)h * p.dk_s[1] + (size_t)kv * p.dk_s[2];
-        __nv_bfloat16* c = p.dv + (size_t)b * p.dv_s[0] + (size_t)h * p.dv_s[1] + (size_t)kv * p.dv_s[2];
-        for (int i = 0; i < D; i += 8) {
-          *reinterpret_cast<uint4*>(a + i) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(c + i) = make_uint4(0, 0, 0, 0);
-        }
-      }
-    }
-    wait_previous();
-    return;
-  }
+  // What the plan says is under way while the barriers and the tensor memory are set up; inside the plan's buffer whatever it holds.
+  const int magic = ld_nc_i32_here(P.status + kStampMagic), plan_b = ld_nc_i32_here(P.status + kStampB), plan_t = ld_nc_i32_here(P.status + kStampT);
+  const int place = ld_nc_i32_here(P.bwd_order + (size_t)b * NB + rank);
 
   if (tid == 0) {
     *abort_ptr = 0;
@@ -321,7 +293,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     mbar_init(&bar_ds, 8);
     mbar_init(&bar_g, 1);
     mbar_init(&bar_dqr, 4);  // one arrival per reduction warp
-    mbar_init(&bar_epi, 2 * kTile);
+    mbar_init(&bar_epi, 8);
     fence_mbar_init();
   }
   __syncthreads();
@@ -329,10 +301,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     tmem_alloc(&tmem_slot, 512);
     tmem_relinquish();
   }
+  const int kb = min(max(place, 0), NB - 1);
+  const int tiles = ld_nc_i32_here((P.bwd_sub != nullptr ? P.bwd_tiles : P.bwd_cnt) + (size_t)b * NB + kb);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  const int n = min(max(tiles, 0), NB - kb);  // query tiles to walk
+  const int32_t* list = P.bwd_idx + ((size_t)b * NB + kb) * NB;
+  const uint16_t* subs = P.bwd_sub != nullptr ? P.bwd_sub + ((size_t)b * sub_line(NB, NB) + sub_line(NB, kb)) * kStretches : nullptr;
+  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
+  const int bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T ? 2901 : smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes ? 2900 : 0;
+  if (bad || n == 0) {
+    if (bad) {
+      if (tid == 0) atomicCAS(P.status, 0, bad);
+    } else if (tid < kTile) {
+      const int kv = kb * kTile + tid;
+      if (kv < P.T) {
+        __nv_bfloat16* a = p.dk + (size_t)b * p.dk_s[0] + (size_t)h * p.dk_s[1] + (size_t)kv * p.dk_s[2];
+        __nv_bfloat16* c = p.dv + (size_t)b * p.dv_s[0] + (size_t)h * p.dv_s[1] + (size_t)kv * p.dv_s[2];
+        for (int i = 0; i < D; i += 8) {
+          *reinterpret_cast<uint4*>(a + i) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(c + i) = make_uint4(0, 0, 0, 0);
+        }
+      }
+    }
+    if (warp == 13) tmem_dealloc(tmem, 512);
+    wait_previous();
+    return;
+  }
   const uint32_t tDV = tmem + Cfg::kDV, tDK = tmem + Cfg::kDK, tST = tmem + Cfg::kST, tDPT = tmem + Cfg::kDPT, tDQ = tDPT;
   // S^T columns [32c, +32) of a buffer are read by the compute thread of (row, c / 2), which writes P^T bf16 over the first 16 of them.
 
@@ -658,13 +655,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         }
       }
       fence_async_smem();
-      mbar_arrive(&bar_epi);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_epi);
     }
     if (tid == 0 && ok && mbar_wait(&bar_epi, 0, abort_w, 33)) {
       tma_store_tile(&mapDV, out_dv, kb * kTile, 0, h, b);
       tma_store_tile(&mapDK, out_dk, kb * kTile, 0, h, b);
       tma_store_commit();
-      tma_store_wait_all();
+      tma_store_wait_read0();  // of this CTA's shared memory
     }
     BTRACE_ACC(6);
     if ((tid & 127) == 0) BTRACE_ACC_DUMP();
@@ -716,7 +714,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       }
       if (tid == 2 * kTile) TRACE(1, i, 6);
     }
-    if (lane == 0) tma_store_wait_all();
+    if (lane == 0) tma_store_wait_read0();
   }
 
   tc_fence_before();

@@ -869,7 +869,7 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
       done();
       FTRACE_ACC(4);
     }
-    if (lane == 0) tma_store_wait_all();  // the stores read this CTA's shared memory
+    if (lane == 0) tma_store_wait_read0();  // the stores read this CTA's shared memory
     if (row == 0) FTRACE_CTA(2 + t, n_tiles);
     if (row == 0) FTRACE_ACC_DUMP(t);
   }

@@ -319,6 +319,12 @@ struct Segments {
   std::vector<int32_t> bounds, ids;
   std::vector<uint64_t> sets;
   int classes = 0;
+  static uint64_t mixed(uint64_t x) {  // spreads small numbers over 64 bits: two odd multipliers and shifts
+    x *= 0x9e3779b97f4a7c15ull;
+    x ^= x >> 29;
+    x *= 0xd6e8feb86659fd93ull;
+    return x ^ (x >> 32);
+  }
   Segments(const std::vector<std::pair<int64_t, int64_t>>& ranges, size_t words) {
     struct Event { int64_t at; int32_t who; bool opens; };
     std::vector<Event> ev;
@@ -329,12 +335,16 @@ struct Segments {
     }
     std::sort(ev.begin(), ev.end(), [](const Event& a, const Event& b) { return a.at < b.at; });
     std::vector<uint64_t> now(words, 0);
-    std::unordered_map<std::string, int32_t> seen;
+    size_t places = 16;
+    while (places < 2 * ev.size()) places *= 2;
+    std::vector<int32_t> seen(places, -1);  // class by the hash of its set, the next free place on a clash
+    uint64_t hash = 0;
     int64_t open = 0;
     for (size_t i = 0; i < ev.size();) {
       const int64_t at = ev[i].at;
       for (; i < ev.size() && ev[i].at == at; ++i) {
         now[ev[i].who >> 6] ^= uint64_t(1) << (ev[i].who & 63);
+        hash ^= mixed(static_cast<uint64_t>(ev[i].who) + 1);
         open += ev[i].opens ? 1 : -1;
       }
       bounds.push_back(static_cast<int32_t>(at));
@@ -343,12 +353,13 @@ struct Segments {
         ids.push_back(-1);
         continue;
       }
-      const auto [it, fresh] = seen.try_emplace(std::string(reinterpret_cast<const char*>(now.data()), words * 8), classes);
-      if (fresh) {
+      size_t at_place = hash & (places - 1);
+      while (seen[at_place] >= 0 && !std::equal(now.begin(), now.end(), sets.begin() + seen[at_place] * words)) at_place = (at_place + 1) & (places - 1);
+      if (seen[at_place] < 0) {
+        seen[at_place] = classes++;
         sets.insert(sets.end(), now.begin(), now.end());
-        ++classes;
       }
-      ids.push_back(it->second);
+      ids.push_back(seen[at_place]);
     }
     if (bounds.empty()) bounds.push_back(0);
   }
@@ -430,13 +441,18 @@ std::vector<Tensor> pack_mask(at::IntArrayRef starts, at::IntArrayRef ends, at::
   if (linked) {
     uint64_t* bits = reinterpret_cast<uint64_t*>(st);
     std::fill(bits, bits + R * W, 0);
+    // which column classes hold a grant's tokens; a row class may read those of its grants
+    std::vector<uint64_t> readers(q.size() * W, 0);
+    auto members = [&](const uint64_t* set, auto visit) {
+      for (size_t w = 0; w < words; ++w)
+        for (uint64_t left = set[w]; left != 0; left &= left - 1) visit(64 * w + __builtin_ctzll(left));
+    };
+    for (int c = 0; c < ks.classes; ++c)
+      members(&ks.sets[c * words], [&](size_t g) { readers[g * W + (c >> 6)] |= uint64_t(1) << (c & 63); });
     for (int r = 0; r < qs.classes; ++r)
-      for (int c = 0; c < ks.classes; ++c) {
-        const uint64_t *a = &qs.sets[r * words], *b = &ks.sets[c * words];
-        uint64_t hit = 0;
-        for (size_t w = 0; w < words; ++w) hit |= a[w] & b[w];
-        if (hit) bits[r * W + (c >> 6)] |= uint64_t(1) << (c & 63);
-      }
+      members(&qs.sets[r * words], [&](size_t g) {
+        for (int64_t w = 0; w < W; ++w) bits[r * W + w] |= readers[g * W + w];
+      });
   }
   table.copy_(stage, /*non_blocking=*/true);
   std::vector<Tensor> r;

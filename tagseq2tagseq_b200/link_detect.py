@@ -13,7 +13,7 @@ exact for byte-level BPE vocabularies (GPT-2's): ')' is a single ASCII byte, whi
 """
 from __future__ import annotations
 
-from typing import Any, Callable, List, Optional, Tuple
+from typing import Any, Callable, Dict, List, Optional, Tuple
 
 import torch
 
@@ -80,13 +80,19 @@ class MarkdownLinkDetector:
 
     # ------------------------------------------------------------------ protocol
     def detect_links(self, input_ids: torch.Tensor) -> List[LinkInfo]:
+        new = tuple.__new__
+        return [new(LinkInfo, link) for link in self._links(input_ids)]
+
+    _own_detect_links = detect_links
+
+    def _links(self, input_ids: torch.Tensor):
+        """(position after the closing token, target) of every link, one after the other."""
         cands, targets = self._scan(input_ids)
-        links: List[LinkInfo] = []
-        decode, new, done = self.decode_fn, tuple.__new__, 0
+        decode, done = self.decode_fn, 0
         for mid, _start, close in cands:
-            n = close - mid
-            target, closed, _ = decode(targets[done:done + n]).partition(")")
-            done += n
+            end = done + close - mid
+            target, closed, _ = decode(targets[done:end]).partition(")")
+            done = end
             if not closed:
                 # the per-token table promised a ')' that the joint decoding does not show (not a byte-level
                 # vocabulary): fall back to the reference's growing window for this candidate
@@ -96,8 +102,20 @@ class MarkdownLinkDetector:
                 close = mid + 1 + at
             target = target.strip()
             if target:
-                links.append(new(LinkInfo, (close + 1, target)))
-        return links
+                yield close + 1, target
+
+    def matched(self, input_ids: torch.Tensor, index: Dict[str, Tuple[int, int]]) -> List[Tuple[int, int]]:
+        """(link_end_pos, document) of every link whose target's document, ``index``'s (doc id, start), starts before it, by position."""
+        get, out, last, ascend = index.get, [], 0, True
+        for pos, target in self._links(input_ids):
+            hit = get(target)
+            if hit is not None and hit[1] < pos:
+                ascend = ascend and pos >= last
+                last = pos
+                out.append((pos, hit[0]))
+        if not ascend:  # only behind a growing window
+            out.sort(key=lambda pair: pair[0])
+        return out
 
     def _grow(self, window: List[int]) -> Tuple[str, int]:
         """(text before ')', index of the token that closes it) of the shortest decodable prefix, or ("", -1)."""

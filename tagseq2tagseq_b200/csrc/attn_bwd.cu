@@ -303,13 +303,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   }
   const int kb = min(max(place, 0), NB - 1);
   const int tiles = ld_nc_i32_here((P.bwd_sub != nullptr ? P.bwd_tiles : P.bwd_cnt) + (size_t)b * NB + kb);
+  const int32_t* list = P.bwd_idx + ((size_t)b * NB + kb) * NB;
+  const uint16_t* subs = P.bwd_sub != nullptr ? P.bwd_sub + ((size_t)b * sub_line(NB, NB) + sub_line(NB, kb)) * kStretches : nullptr;
+  uint32_t entry = 0u;  // the producers' first one
+  if (warp == 12 || warp == 14) entry = stretch_entry(subs, list, 0, lane & (kStretches - 1), NB);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const int n = min(max(tiles, 0), NB - kb);  // query tiles to walk
-  const int32_t* list = P.bwd_idx + ((size_t)b * NB + kb) * NB;
-  const uint16_t* subs = P.bwd_sub != nullptr ? P.bwd_sub + ((size_t)b * sub_line(NB, NB) + sub_line(NB, kb)) * kStretches : nullptr;
   // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
   const int bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T ? 2901 : smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes ? 2900 : 0;
   if (bad || n == 0) {
@@ -354,7 +356,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const int stages = is_q ? Cfg::kQStages : Cfg::kDoStages;
       uint8_t* tiles = is_q ? sQ : sDO;
       uint64_t *full = is_q ? bar_q_full : bar_do_full, *free = is_q ? bar_gq : bar_gv;
-      uint32_t entry = stretch_entry(subs, list, 0, lane & (kStretches - 1), NB);
       int st = 0, use = 0;
       for (int i = 0; i < n; ++i) {
         const int sub = stretch_of(entry, NB);

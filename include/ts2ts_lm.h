@@ -35,6 +35,9 @@ int ts2ts_add_rmsnorm_fwd(const float* x_in, const void* a, const float* w, floa
 size_t ts2ts_add_rmsnorm_bwd_workspace_bytes(int64_t N, int C);
 int ts2ts_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
                           float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream);
+/* The same, but WRITES the weight gradient to dw[C], whatever was there. */
+int ts2ts_add_rmsnorm_bwd_set(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
+                              float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream);
 
 /* Rotary embedding in place on the q and k slices of qkv[B,T,3,H,D] (bf16): pairs (i, i + D/2) are rotated by the
  * angle whose cosine / sine are cos[t,i], sin[t,i] (fp32 [T, D/2]).  sign = +1 rotates, sign = -1 rotates back, which

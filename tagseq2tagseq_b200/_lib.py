@@ -42,6 +42,7 @@ SYMBOLS = {
     "ts2ts_add_rmsnorm_fwd": (c_int, [c_void_p] * 6 + [c_int64, c_int, c_float, c_void_p]),
     "ts2ts_add_rmsnorm_bwd_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "ts2ts_add_rmsnorm_bwd": (c_int, [c_void_p] * 9 + [c_size_t, c_int64, c_int, c_void_p]),
+    "ts2ts_add_rmsnorm_bwd_set": (c_int, [c_void_p] * 9 + [c_size_t, c_int64, c_int, c_void_p]),
     "ts2ts_rope_qk_inplace": (c_int, [c_void_p] * 3 + [c_int] * 4 + [c_float, c_void_p]),
     "ts2ts_swiglu_fwd": (c_int, [c_void_p] * 2 + [c_int64, c_int, c_void_p]),
     "ts2ts_swiglu_bwd": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_void_p]),

@@ -28,7 +28,7 @@ int bwd_static_scratch(void** ptr, size_t* bytes);
 cudaError_t launch_add_rmsnorm_fwd(const float* x_in, const void* a, const float* w, float* x_out, void* h, float* rstd, int N, int C,
                                    float eps, cudaStream_t stream);
 cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx,
-                                   void* da, float* dw, float* dw_part, int N, int C, cudaStream_t stream);
+                                   void* da, float* dw, bool add, float* dw_part, int N, int C, cudaStream_t stream);
 int add_rmsnorm_bwd_blocks(int64_t N, int C);
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream);
 cudaError_t launch_swiglu_fwd(const void* gu, void* act, int64_t N, int F, cudaStream_t stream);
@@ -344,8 +344,8 @@ size_t ts2ts_add_rmsnorm_bwd_workspace_bytes(int64_t N, int C) {
   return (size_t)add_rmsnorm_bwd_blocks(N, C) * C * sizeof(float);
 }
 
-int ts2ts_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
-                          float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream) {
+static int add_rmsnorm_bwd(bool add, const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
+                           float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream) {
   int r;
   if ((r = check_rows(N))) return r;
   if (C < 4 || C > 16384 || C % 4) return fail(-2, "C must be a multiple of 4 in 4..16384 (got %d)", C);
@@ -354,8 +354,16 @@ int ts2ts_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, co
       !aligned(workspace, 16))
     return fail(-5, "add_rmsnorm_bwd: misaligned pointer");
   if (workspace_bytes < ts2ts_add_rmsnorm_bwd_workspace_bytes(N, C)) return fail(-4, "add_rmsnorm_bwd: workspace too small");
-  return launched(launch_add_rmsnorm_bwd(dh, dx_up, x, w, rstd, dx, da, dw, static_cast<float*>(workspace), (int)N, C,
+  return launched(launch_add_rmsnorm_bwd(dh, dx_up, x, w, rstd, dx, da, dw, add, static_cast<float*>(workspace), (int)N, C,
                                          static_cast<cudaStream_t>(stream)), "add_rmsnorm_bwd");
+}
+int ts2ts_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
+                          float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream) {
+  return add_rmsnorm_bwd(true, dh, dx_up, x, w, rstd, dx, da, dw, workspace, workspace_bytes, N, C, stream);
+}
+int ts2ts_add_rmsnorm_bwd_set(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx, void* da,
+                              float* dw, void* workspace, size_t workspace_bytes, int64_t N, int C, void* stream) {
+  return add_rmsnorm_bwd(false, dh, dx_up, x, w, rstd, dx, da, dw, workspace, workspace_bytes, N, C, stream);
 }
 
 int ts2ts_rope_qk_inplace(void* qkv, const float* cos, const float* sin, int B, int T, int H, int D, float sign, void* stream) {

@@ -132,15 +132,16 @@ __global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x_in, const __n
 // with a stride, keep their share of dw in registers and write it to row blockIdx.x of dw_part [gridDim.x, C] at the
 // end (atomics on the C addresses of one dw vector serialise a thousand blocks); a second kernel adds the rows up.
 //
-// HBM-bound, 16 bytes per element: every load of an iteration is issued before its reduction, kRows rows at a time, and
-// the reduction's scratch alternates so that one barrier per iteration suffices.  With one row in flight and the load of
-// dx_up behind the reduction it ran at 62 % of the copy rate (47 us at 16384 x 768, 268 us at 32768 x 2048).
-template <int NV, int kRows>
+// HBM-bound, 16 bytes per element: the loads of the next row are on their way while this one is reduced and stored (kAhead; four vectors a
+// thread and their successors do not fit the registers: 4096 x 8192 142 -> 230 us), and
+// the reduction's scratch alternates so that one barrier per row suffices.  us, two rows at once and none ahead -> one and the next: 16384 x 768 50 -> 46,
+// 32768 x 2048 202 -> 175 (164 at the copy rate), 8192 x 4096 126 -> 95, 1024 x 256 13.3 -> 11.3, each with the sum of its weight gradients.
+template <int NV, bool kAhead>
 __global__ void __launch_bounds__(1024) add_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const float* __restrict__ dx_up,
                                                                const float* __restrict__ x, const float* __restrict__ w,
                                                                const float* __restrict__ rstd, float* __restrict__ dx,
                                                                __nv_bfloat16* __restrict__ da, float* __restrict__ dw_part, int N, int C) {
-  __shared__ float red[2][kRows][32];
+  __shared__ float red[2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float4 wv[NV], acc[NV];
   wait_previous();
@@ -151,59 +152,62 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_bwd_kernel(const __nv_bfloat
     wv[i] = c < C ? *reinterpret_cast<const float4*>(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  struct Row {  // this thread's part of one, dh as it lies in memory
+    float4 x[NV], up[NV];
+    uint2 dh[NV];
+    float rs;
+  } in;
+  auto load = [&](int row) {
+    in.rs = rstd[row];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
+      in.x[i] = in.up[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      in.dh[i] = make_uint2(0u, 0u);
+      if (c < C) {
+        const size_t at = (size_t)row * C + c;
+        in.x[i] = *reinterpret_cast<const float4*>(x + at);
+        in.dh[i] = *reinterpret_cast<const uint2*>(dh + at);
+        if (dx_up != nullptr) in.up[i] = *reinterpret_cast<const float4*>(dx_up + at);
+      }
+    }
+  };
   int buf = 0;
-  for (int row0 = blockIdx.x; row0 < N; row0 += kRows * gridDim.x, buf ^= 1) {
-    float4 xh[kRows][NV], g[kRows][NV], up[kRows][NV];
-    float rs[kRows], dot[kRows];
+  if (kAhead && (int)blockIdx.x < N) load(blockIdx.x);
+  for (int row = blockIdx.x; row < N; row += gridDim.x, buf ^= 1) {
+    if (!kAhead) load(row);
+    const float rs = in.rs;
+    float4 xh[NV], g[NV], up[NV];
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int row = row0 + k * gridDim.x;
-      rs[k] = row < N ? rstd[row] : 0.f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = (threadIdx.x + i * blockDim.x) * 4;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        xh[k][i] = zero; g[k][i] = zero; up[k][i] = zero;
-        if (c < C && row < N) {
-          const size_t at = (size_t)row * C + c;
-          xh[k][i] = *reinterpret_cast<const float4*>(x + at);
-          g[k][i] = bf16x4_to_float4(*reinterpret_cast<const uint2*>(dh + at));
-          if (dx_up != nullptr) up[k][i] = *reinterpret_cast<const float4*>(dx_up + at);
-        }
-      }
+    for (int i = 0; i < NV; ++i) {
+      xh[i] = in.x[i];
+      up[i] = in.up[i];
+      g[i] = bf16x4_to_float4(in.dh[i]);
     }
+    if (kAhead && row + (int)gridDim.x < N) load(row + gridDim.x);
+    float dot = 0.f;
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      dot[k] = 0.f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        float4& h = xh[k][i];
-        float4& d = g[k][i];
-        h.x *= rs[k]; h.y *= rs[k]; h.z *= rs[k]; h.w *= rs[k];
-        acc[i].x += d.x * h.x; acc[i].y += d.y * h.y; acc[i].z += d.z * h.z; acc[i].w += d.w * h.w;
-        d.x *= wv[i].x; d.y *= wv[i].y; d.z *= wv[i].z; d.w *= wv[i].w;
-        dot[k] += d.x * h.x + d.y * h.y + d.z * h.z + d.w * h.w;
-      }
-      dot[k] = warp_sum(dot[k]);
-      if (lane == 0) red[buf][k][warp] = dot[k];
+    for (int i = 0; i < NV; ++i) {
+      float4& h = xh[i];
+      float4& d = g[i];
+      h.x *= rs; h.y *= rs; h.z *= rs; h.w *= rs;
+      acc[i].x += d.x * h.x; acc[i].y += d.y * h.y; acc[i].z += d.z * h.z; acc[i].w += d.w * h.w;
+      d.x *= wv[i].x; d.y *= wv[i].y; d.z *= wv[i].z; d.w *= wv[i].w;
+      dot += d.x * h.x + d.y * h.y + d.z * h.z + d.w * h.w;
     }
+    dot = warp_sum(dot);
+    if (lane == 0) red[buf][warp] = dot;
     __syncthreads();
+    dot = warp_sum(lane < nw ? red[buf][lane] : 0.f) / (float)C;
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int row = row0 + k * gridDim.x;
-      dot[k] = warp_sum(lane < nw ? red[buf][k][lane] : 0.f) / (float)C;
-      if (row >= N) continue;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = (threadIdx.x + i * blockDim.x) * 4;
-        if (c < C) {
-          const size_t at = (size_t)row * C + c;
-          const float4 h = xh[k][i], d = g[k][i], u = up[k][i];
-          const float4 o = make_float4(rs[k] * (d.x - h.x * dot[k]) + u.x, rs[k] * (d.y - h.y * dot[k]) + u.y,
-                                       rs[k] * (d.z - h.z * dot[k]) + u.z, rs[k] * (d.w - h.w * dot[k]) + u.w);
-          *reinterpret_cast<float4*>(dx + at) = o;
-          if (da != nullptr) *reinterpret_cast<uint2*>(da + at) = float4_to_bf16x4(o);
-        }
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
+      if (c < C) {
+        const size_t at = (size_t)row * C + c;
+        const float4 h = xh[i], d = g[i], u = up[i];
+        const float4 o = make_float4(rs * (d.x - h.x * dot) + u.x, rs * (d.y - h.y * dot) + u.y, rs * (d.z - h.z * dot) + u.z, rs * (d.w - h.w * dot) + u.w);
+        *reinterpret_cast<float4*>(dx + at) = o;
+        if (da != nullptr) *reinterpret_cast<uint2*>(da + at) = float4_to_bf16x4(o);
       }
     }
   }
@@ -213,10 +217,10 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_bwd_kernel(const __nv_bfloat
     if (c < C) *reinterpret_cast<float4*>(dw_part + (size_t)blockIdx.x * C + c) = acc[i];
   }
 }
-// dw[c] += sum over the rows of dw_part[rows, C].  A block owns 32 columns: eight lanes of a warp read one row's 128
+// dw[c] = (`add` to what is there) the sum over the rows of dw_part[rows, C].  A block owns 32 columns: eight lanes of a warp read one row's 128
 // bytes, so that 128 rows are in flight per block; one thread per column was a serial chain of loads (66 us per call at
 // 1480 x 768, more than the kernel whose partial sums it adds).
-__global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ part, float* dw, int rows, int C) {
+__global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ part, float* dw, int rows, int C, bool add) {
   __shared__ float4 red[32][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
   const int c = blockIdx.x * 32 + sub * 4;
@@ -244,7 +248,7 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restric
 #pragma unroll
     for (int i = 0; i < 32; ++i) t += reinterpret_cast<const float*>(red[i])[threadIdx.x];
     const int col = blockIdx.x * 32 + threadIdx.x;
-    if (col < C) dw[col] += t;
+    if (col < C) dw[col] = add ? dw[col] + t : t;
   }
 }
 
@@ -717,14 +721,14 @@ int add_rmsnorm_bwd_blocks(int64_t N, int C) {
 }
 
 cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx,
-                                   void* da, float* dw, float* dw_part, int N, int C, cudaStream_t stream) {
+                                   void* da, float* dw, bool add, float* dw_part, int N, int C, cudaStream_t stream) {
   const int grid = add_rmsnorm_bwd_blocks(N, C);
   const int threads = norm_threads(C);
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(dh);
   __nv_bfloat16* a = static_cast<__nv_bfloat16*>(da);
-  const cudaError_t e = launch_after(C <= 4 * threads ? add_rmsnorm_bwd_kernel<1, 2> : add_rmsnorm_bwd_kernel<kMaxVec, 1>, dim3(grid), threads, 0, stream,
+  const cudaError_t e = launch_after(C <= 4 * threads ? add_rmsnorm_bwd_kernel<1, true> : add_rmsnorm_bwd_kernel<kMaxVec, false>, dim3(grid), threads, 0, stream,
                                      g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
-  return e != cudaSuccess ? e : launch_after(column_sum_kernel, dim3((C + 31) / 32), 1024, 0, stream, dw_part, dw, grid, C);
+  return e != cudaSuccess ? e : launch_after(column_sum_kernel, dim3((C + 31) / 32), 1024, 0, stream, dw_part, dw, grid, C, add);
 }
 
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream) {

@@ -518,12 +518,12 @@ struct AddRMSNorm : torch::autograd::Function<AddRMSNorm> {
     const auto bf16 = x.options().dtype(at::kBFloat16);
     const Tensor dh = grads[1].defined() ? grads[1].contiguous() : at::zeros(x.sizes(), bf16);  // h had no user
     const Tensor up = grads[0].defined() ? grads[0].contiguous() : Tensor();
-    Tensor dx = at::empty_like(x), da = has_a ? at::empty(x.sizes(), bf16) : Tensor(), dw = at::zeros_like(w);
+    Tensor dx = at::empty_like(x), da = has_a ? at::empty(x.sizes(), bf16) : Tensor(), dw = w.numel() == C ? at::empty_like(w) : at::zeros_like(w);
     Tensor ws = at::empty({static_cast<int64_t>(ts2ts_add_rmsnorm_bwd_workspace_bytes(N, static_cast<int>(C)))}, x.options().dtype(at::kByte));
-    check(ts2ts_add_rmsnorm_bwd(dh.const_data_ptr(), up.defined() ? fptr(up) : nullptr, fptr(x), fptr(w), fptr(rstd), mfptr(dx),
+    check(ts2ts_add_rmsnorm_bwd_set(dh.const_data_ptr(), up.defined() ? fptr(up) : nullptr, fptr(x), fptr(w), fptr(rstd), mfptr(dx),
                                 has_a ? da.mutable_data_ptr() : nullptr, mfptr(dw), ws.mutable_data_ptr(), ws.numel(), N, static_cast<int>(C),
                                 stream_of(x)),
-          "ts2ts_add_rmsnorm_bwd");
+          "ts2ts_add_rmsnorm_bwd_set");
     refuse_gradient("ts2ts::add_rmsnorm backward", {grads[0], grads[1], x, w}, {&dx, &da, &dw});
     return {dx, da, dw, Tensor()};
   }

@@ -68,6 +68,9 @@ int ts2ts_scale(float* x, void* out, const float* gscale, int64_t n, void* strea
  * ignored).  C % 4 == 0, V < 2^31.  The additions are made in an order that depends on idx alone. */
 int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t N, int C, int64_t V, void* stream);
 
+/* dst[i][0..n[i]) (bf16) = src[i][0..n[i]) (fp32), rounded to nearest even, for `count` tensors.  src, dst: host arrays of device pointers. */
+int ts2ts_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, void* stream);
+
 /* One AdamW step over `count` fp32 tensors.  p, g, m, v: host arrays of device pointers (parameter, gradient, first and
  * second moment); n: host array of element counts; steps: host array, the number of this step per tensor (from 1).
  *   p <- p (1 - lr wd);  m <- b1 m + (1 - b1) g;  v <- b2 v + (1 - b2) g^2;

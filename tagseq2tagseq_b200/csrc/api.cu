@@ -30,6 +30,7 @@ cudaError_t launch_add_rmsnorm_fwd(const float* x_in, const void* a, const float
 cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const float* x, const float* w, const float* rstd, float* dx,
                                    void* da, float* dw, bool add, float* dw_part, int N, int C, cudaStream_t stream);
 int add_rmsnorm_bwd_blocks(int64_t N, int C);
+cudaError_t launch_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, cudaStream_t stream);
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream);
 cudaError_t launch_swiglu_fwd(const void* gu, void* act, int64_t N, int F, cudaStream_t stream);
 cudaError_t launch_swiglu_bwd(const void* gu, const void* dact, void* dgu, int64_t N, int F, cudaStream_t stream);
@@ -439,6 +440,14 @@ int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t 
   if (!idx || !dx || !dw) return fail(-3, "embedding_bwd: null pointer");
   if (!aligned(dx, 16) || !aligned(dw, 16)) return fail(-5, "embedding_bwd: misaligned pointer");
   return launched(launch_embedding_bwd(idx, dx, dw, N, C, V, static_cast<cudaStream_t>(stream)), "embedding_bwd");
+}
+
+int ts2ts_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, void* stream) {
+  if (count < 0) return fail(-1, "count must not be negative");
+  if (count > 0 && (!src || !dst || !n)) return fail(-3, "cast_bf16: null pointer");
+  for (int i = 0; i < count; ++i)
+    if (n[i] < 0 || (n[i] > 0 && (!src[i] || !dst[i]))) return fail(-3, "cast_bf16: tensor %d has a null pointer or a negative size", i);
+  return launched(launch_cast_bf16(count, src, dst, n, static_cast<cudaStream_t>(stream)), "cast_bf16");
 }
 
 int ts2ts_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,

@@ -252,6 +252,42 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restric
   }
 }
 
+// ---------------------------------------------------------------------------------------------- bf16 copies
+// All of a step's weights in one launch instead of one each: a block takes kCastChunk consecutive elements of one tensor.  HBM-bound, 6 bytes
+// an element.  us: the 17 weights of four layers at d_model 768 with 50304 words (76 M elements, 70 at the copy rate) 111 -> 72; nine of 3.6 M in all 17 in nine launches, below 5 in one.
+constexpr int kCastTensors = 128, kCastThreads = 256, kCastChunk = 8192;
+struct CastArgs {
+  const float* src[kCastTensors];
+  __nv_bfloat16* dst[kCastTensors];
+  int64_t n[kCastTensors];
+  int first_block[kCastTensors];
+  int count;
+};
+__global__ void __launch_bounds__(kCastThreads) cast_bf16_kernel(const __grid_constant__ CastArgs a) {
+  int lo = 0, hi = a.count - 1;  // last tensor whose first block is not after this one
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.first_block[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  wait_previous();
+  const float* src = settled(a.src[lo]);
+  __nv_bfloat16* dst = a.dst[lo];
+  const int64_t begin = (int64_t)((int)blockIdx.x - a.first_block[lo]) * kCastChunk, end = min(begin + (int64_t)kCastChunk, a.n[lo]);
+  int64_t i = begin;
+  if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0) {
+    const int64_t vend = begin + (end - begin) / 8 * 8;
+#pragma unroll 4
+    for (int64_t j = begin + 8 * threadIdx.x; j < vend; j += 8 * kCastThreads) {
+      float f[8];
+      *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src + j);
+      *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + j + 4);
+      *reinterpret_cast<uint4*>(dst + j) = float_to_bf16x8(f);
+    }
+    i = vend;
+  }
+  for (i += threadIdx.x; i < end; i += kCastThreads) dst[i] = __float2bfloat16_rn(src[i]);
+}
+
 // ---------------------------------------------------------------------------------------------- rotary embedding
 // In place on the q (part 0) and k (part 1) slices of qkv [B,T,3,H,D]: pairs (i, i + D/2),
 //   y1 = x1 cos - sign * x2 sin,  y2 = x2 cos + sign * x1 sin;  sign = -1 turns a gradient back (the inverse rotation).
@@ -729,6 +765,25 @@ cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const flo
   const cudaError_t e = launch_after(C <= 4 * threads ? add_rmsnorm_bwd_kernel<1, true> : add_rmsnorm_bwd_kernel<kMaxVec, false>, dim3(grid), threads, 0, stream,
                                      g, dx_up, x, w, rstd, dx, a, dw_part, N, C);
   return e != cudaSuccess ? e : launch_after(column_sum_kernel, dim3((C + 31) / 32), 1024, 0, stream, dw_part, dw, grid, C, add);
+}
+
+cudaError_t launch_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, cudaStream_t stream) {
+  CastArgs a;
+  for (int done = 0; done < count;) {
+    int64_t blocks = 0;
+    a.count = 0;
+    for (; done < count && a.count < kCastTensors; ++done) {
+      const int64_t need = (n[done] + kCastChunk - 1) / kCastChunk;
+      if (need == 0) continue;
+      if (a.count > 0 && blocks + need > 0x7fffffff) break;
+      a.src[a.count] = src[done]; a.dst[a.count] = static_cast<__nv_bfloat16*>(dst[done]); a.n[a.count] = n[done];
+      a.first_block[a.count++] = (int)blocks;
+      blocks += need;
+    }
+    const cudaError_t e = blocks > 0 ? launch_after(cast_bf16_kernel, dim3((unsigned)blocks), kCastThreads, 0, stream, a) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream) {

@@ -674,11 +674,37 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossE
 // conversion pass (6 bytes per weight) on the way to the parameter.  x is saved as it was passed, so that writing to it
 // before the backward is noticed; of w only the bf16 copy is needed, and a changed w does not matter.  A gradient that may be
 // differentiated again (create_graph) is made of ordinary operators on x and w themselves.
+// `copy`, the weight in bf16 where the caller has made one (cast_weights), or a copy of this call's own.
+Tensor bf16_of(const Tensor& w, const OptTensor& copy) {
+  if (!copy.has_value()) return w.to(at::kBFloat16);
+  TORCH_CHECK_VALUE(copy->scalar_type() == at::kBFloat16 && copy->sizes() == w.sizes() && copy->device() == w.device(), "the weight's copy is bf16 and of its size");
+  return *copy;
+}
+// The bf16 copies of fp32 weights, all in one launch.
+std::vector<Tensor> cast_weights(at::TensorList ws) {
+  std::vector<Tensor> out;
+  if (ws.empty()) return out;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const CUDAGuard guard(ws[0].device());
+  std::vector<const float*> src;
+  std::vector<void*> dst;
+  std::vector<int64_t> n;
+  for (const Tensor& w : ws) {
+    TORCH_CHECK_VALUE(w.is_cuda() && w.device() == ws[0].device() && w.scalar_type() == at::kFloat && w.is_contiguous(), "cast_weights: contiguous fp32 CUDA tensors of one device");
+    out.push_back(at::empty(w.sizes(), w.options().dtype(at::kBFloat16)));
+    src.push_back(fptr(w));
+    dst.push_back(out.back().mutable_data_ptr());
+    n.push_back(w.numel());
+  }
+  check(ts2ts_cast_bf16(static_cast<int>(src.size()), src.data(), dst.data(), n.data(), stream_of(ws[0])), "ts2ts_cast_bf16");
+  return out;
+}
+
 struct Linear : torch::autograd::Function<Linear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& copy) {
     need_cuda(x);
     at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor wb = w.to(at::kBFloat16);
+    const Tensor wb = bf16_of(w, copy);
     ctx->save_for_backward({x, wb});
     if (w.requires_grad() && !w.is_inference()) {
       ctx->saved_data["w"] = w;
@@ -705,23 +731,23 @@ struct Linear : torch::autograd::Function<Linear> {
       }
       if (ctx->needs_input_grad(0)) dx = at::mm(dy, wb).view(s[0].sizes());
       if (ctx->needs_input_grad(1)) dw = at::mm(dy.t().to(at::kFloat), s[0].reshape({-1, s[0].size(-1)}).to(at::kFloat));
-      return {dx, dw};
+      return {dx, dw, Tensor()};
     }
     if (ctx->needs_input_grad(0)) dx = at::mm(dy, s[1]).view(s[0].sizes());
     if (ctx->needs_input_grad(1)) dw = at::mm(dy.t(), s[0].reshape({-1, s[0].size(-1)}), at::kFloat);
-    return {dx, dw};
+    return {dx, dw, Tensor()};
   }
 };
-Tensor linear(const Tensor& x, const Tensor& w) { return Linear::apply(x, w); }
+Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& copy) { return Linear::apply(x, w, copy); }
 
 // Mean cross-entropy of the output head, logits = h w^T.  The loss kernel leaves the gradient of the mean loss in the
 // logits' buffer; what reaches the loss from above multiplies the two small results instead of the logits.
 struct HeadLoss : torch::autograd::Function<HeadLoss> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& target_in) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& target_in, const OptTensor& copy) {
     need_cuda(h);
     at::AutoDispatchBelowADInplaceOrView below;
     const CUDAGuard guard(h.device());
-    const Tensor h2 = h.reshape({-1, h.size(-1)}), wb = w.to(at::kBFloat16), target = target_in.reshape({-1}).to(at::kLong).contiguous();
+    const Tensor h2 = h.reshape({-1, h.size(-1)}), wb = bf16_of(w, copy), target = target_in.reshape({-1}).to(at::kLong).contiguous();
     const int64_t N = h2.size(0), V = w.size(0);
     TORCH_CHECK_VALUE(target.numel() == N, "head_loss: one target per row of h");
     Tensor logits = at::mm(h2, wb.t()), loss = at::empty({N}, h.options().dtype(at::kFloat));
@@ -752,10 +778,10 @@ struct HeadLoss : torch::autograd::Function<HeadLoss> {
       }
     }
     refuse_gradient("ts2ts::head_loss backward", {grads[0], s[0], ctx->saved_data["w"].toTensor()}, {&dh, &dw});
-    return {dh, dw, Tensor()};
+    return {dh, dw, Tensor(), Tensor()};
   }
 };
-Tensor head_loss(const Tensor& h, const Tensor& w, const Tensor& target) { return HeadLoss::apply(h, w, target); }
+Tensor head_loss(const Tensor& h, const Tensor& w, const Tensor& target, const OptTensor& copy) { return HeadLoss::apply(h, w, target, copy); }
 
 struct Embedding : torch::autograd::Function<Embedding> {
   static Tensor forward(AutogradContext* ctx, const Tensor& w, const Tensor& idx) {
@@ -826,8 +852,9 @@ TORCH_LIBRARY(ts2ts, m) {
         "Tensor plan, int n_heads, int head_dim) -> Tensor", qkv_attention);
   m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
   m.def("cross_entropy(Tensor logits, Tensor target) -> Tensor", cross_entropy);
-  m.def("linear(Tensor x, Tensor w) -> Tensor", linear);
-  m.def("head_loss(Tensor h, Tensor w, Tensor target) -> Tensor", head_loss);
+  m.def("cast_weights(Tensor[] ws) -> Tensor[]", cast_weights);
+  m.def("linear(Tensor x, Tensor w, Tensor? copy=None) -> Tensor", linear);
+  m.def("head_loss(Tensor h, Tensor w, Tensor target, Tensor? copy=None) -> Tensor", head_loss);
   m.def("embedding(Tensor w, Tensor idx) -> Tensor", embedding);
   m.def("adamw(Tensor(a!)[] params, Tensor[] grads, Tensor(b!)[] exp_avgs, Tensor(c!)[] exp_avg_sqs, Tensor(d!)[] steps, float lr, float beta1, "
         "float beta2, float eps, float weight_decay) -> ()", adamw);

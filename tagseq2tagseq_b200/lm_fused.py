@@ -15,7 +15,7 @@ from torch.autograd import forward_ad as fwAD
 from . import _lib
 from .mask_spec import MaskSpec
 
-__all__ = ["add_rmsnorm", "qkv_attention", "swiglu", "cross_entropy", "head_loss", "embedding", "rope_half_tables", "Linear", "AdamW"]
+__all__ = ["add_rmsnorm", "qkv_attention", "swiglu", "cross_entropy", "head_loss", "embedding", "rope_half_tables", "cast_weights", "Linear", "AdamW"]
 
 _lib.load_if_built()
 _MAX_HEAD_COLUMNS = 110592  # a row of logits that ts2ts_ce_fwd_grad keeps in shared memory
@@ -73,15 +73,16 @@ def cross_entropy(logits: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     return _call(_lib.ops().cross_entropy.default, logits, target)
 
 
-def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
-    """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call."""
+def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor, copy: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call.  ``copy``: the
+    weight in bf16, for a caller that has it."""
     if target.numel() != h.shape[:-1].numel():
         raise ValueError("head_loss: one target per row of h")
     _need_cuda(h, weight, target)
     V = weight.shape[0]
     if (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad) and h.dtype == torch.bfloat16 and weight.dtype == torch.float32
             and V % 8 == 0 and V <= _MAX_HEAD_COLUMNS and h.shape[-1] % 8 == 0):
-        return _call(_lib.ops().head_loss.default, h, weight, target)
+        return _call(_lib.ops().head_loss.default, h, weight, target, copy)
     logits = F.linear(h, weight.to(h.dtype))
     return cross_entropy(logits.to(torch.bfloat16).view(-1, V), target.reshape(-1))
 
@@ -99,6 +100,12 @@ def transformed() -> bool:
     return torch._C._functorch.peek_interpreter_stack() is not None or fwAD._current_level >= 0
 
 
+def cast_weights(weights) -> list:
+    """bf16 copies of contiguous fp32 CUDA weights, all in one launch."""
+    _need_cuda(*weights)
+    return _call(_lib.ops().cast_weights.default, weights)
+
+
 class Linear(nn.Linear):
     """A bias-free linear layer with an fp32 weight.  Under bf16 autocast, bf16 activations multiply the weight's bf16 copy,
     and the weight gradient is produced in fp32; anything else is torch's own layer."""
@@ -106,10 +113,11 @@ class Linear(nn.Linear):
     def __init__(self, in_features: int, out_features: int):
         super().__init__(in_features, out_features, bias=False)
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, copy: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``copy``: the weight in bf16, for a caller that has made one (``cast_weights``)."""
         if (x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
                 and torch.get_autocast_dtype("cuda") == torch.bfloat16 and (torch.compiler.is_compiling() or not transformed())):
-            return _call(_lib.ops().linear.default, x, self.weight)
+            return _call(_lib.ops().linear.default, x, self.weight, copy)
         return super().forward(x)
 
 

@@ -24,7 +24,7 @@ import torch.nn.modules.module as _module
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 
-from .lm_fused import AdamW, Linear, add_rmsnorm, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
+from .lm_fused import AdamW, Linear, add_rmsnorm, cast_weights, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -94,12 +94,16 @@ class Block(nn.Module):
         self.gate_up = Linear(cfg.d_model, 2 * cfg.mlp_hidden)
         self.down = Linear(cfg.mlp_hidden, cfg.d_model)
 
-    def forward(self, x, a, mask: MaskSpec, cos, sin):
-        c = self.cfg
+    def linears(self):
+        return (self.qkv, self.proj, self.gate_up, self.down)
+
+    def forward(self, x, a, mask: MaskSpec, cos, sin, copies=((),) * 4):
+        """``copies``: what each of ``linears()`` gets beside its input, the weight's bf16 copy or nothing."""
+        c, (qkv, proj, gate_up, down) = self.cfg, copies
         x, h = add_rmsnorm(x, a, self.ln1.weight, RMS_EPS)
-        attn = qkv_attention(self.qkv(h), cos, sin, mask, c.n_heads, c.head_dim)   # rotary + masked attention, layer.py:32-35
-        x, h = add_rmsnorm(x, self.proj(attn), self.ln2.weight, RMS_EPS)
-        return x, self.down(swiglu(self.gate_up(h)))
+        attn = qkv_attention(self.qkv(h, *qkv), cos, sin, mask, c.n_heads, c.head_dim)   # rotary + masked attention, layer.py:32-35
+        x, h = add_rmsnorm(x, self.proj(attn, *proj), self.ln2.weight, RMS_EPS)
+        return x, self.down(swiglu(self.gate_up(h, *gate_up)), *down)
 
 
 class DecoderLM(nn.Module):
@@ -142,6 +146,19 @@ class DecoderLM(nn.Module):
                 t.record_stream(here)
         return tables
 
+    def _weight_copies(self):
+        """The bf16 copies that this forward's linear layers keep for their backward, ((copy,), ...) by layer and then the head's, made in one launch.  None
+        where a layer would not take one, or somebody's code could look at a weight, or change it, on the way."""
+        layers = [m for blk in self.blocks if _plain(blk, Block) for m in blk.linears()] + [self.head]
+        if (len(layers) != 4 * len(self.blocks) + 1 or torch.compiler.is_compiling() or not torch.is_grad_enabled() or transformed()
+                or not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") != torch.bfloat16
+                or not all(_plain(m, Linear) and m.bias is None for m in layers)):
+            return None
+        weights = [m.weight for m in layers]
+        if not all(type(w) in (nn.Parameter, torch.Tensor) and w.is_cuda and w.device == weights[0].device and w.dtype == torch.float32 and w.is_contiguous() for w in weights):
+            return None
+        return [(c,) for c in cast_weights(weights)]
+
     def forward(self, tokens: torch.Tensor, mask: MaskSpec, rope=None) -> torch.Tensor:
         """tokens int64 [B, T+1]; returns the mean next-token cross-entropy (training_module.py:195-211).  Runs under
         bf16 autocast: the linear layers compute in bf16, the residual stream, norms, rotary angles and the loss in fp32.
@@ -154,11 +171,12 @@ class DecoderLM(nn.Module):
             x = e(inp).float()
         cos, sin = self._rope_tables(inp.shape[1], inp.device) if rope is None else rope
         a = None
-        for blk in self.blocks:
-            x, a = blk(x, a, mask, cos, sin)
+        copies = self._weight_copies()
+        for i, blk in enumerate(self.blocks):
+            x, a = blk(x, a, mask, cos, sin, copies[4 * i:4 * i + 4]) if copies else blk(x, a, mask, cos, sin)
         _, h = add_rmsnorm(x, a, self.norm.weight, RMS_EPS)
         if _plain(self.head, Linear) and self.head.bias is None:
-            return head_loss(h, self.head.weight, tgt)
+            return head_loss(h, self.head.weight, tgt, *(copies[-1] if copies else ()))
         logits = self.head(h)
         return cross_entropy(logits.to(torch.bfloat16).view(-1, logits.shape[-1]), tgt.reshape(-1))
 

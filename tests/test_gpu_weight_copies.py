@@ -1,0 +1,53 @@
+"""The bf16 copies of a step's weights, made in one launch: what a conversion of each gives, and the same step with and without."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+
+
+def test_copies_are_those_of_torch():
+    from tagseq2tagseq_b200.lm_fused import cast_weights
+    g = torch.Generator(device=DEV).manual_seed(1)
+    shapes = [(1, 1), (3, 5), (8, 1024), (1, 8191), (1, 8192), (1, 8193), (257, 768), (50, 1)] + [(7, 3)] * 140  # more than one launch takes
+    ws = [torch.randn(s, device=DEV, generator=g) * 10.0 ** (i % 9 - 4) for i, s in enumerate(shapes)]
+    ws.append(torch.empty(33 * 7 + 1, device=DEV).uniform_(-1, 1)[1:].view(33, 7))                              # not at a 16-byte boundary
+    ws.append(torch.tensor([[0.0, -0.0, float("inf"), -float("inf"), 1e-40, 3.4e38, 1.00390625, 1.01171875]], device=DEV))  # ends, ties to even
+    got = cast_weights(ws)
+    assert all(torch.equal(a, w.bfloat16()) and a.shape == w.shape for a, w in zip(got, ws))
+    nan = torch.full((2, 9), float("nan"), device=DEV)
+    assert cast_weights([nan])[0].isnan().all() and cast_weights([]) == []
+    with pytest.raises(ValueError):
+        cast_weights([ws[0], ws[2].t()])
+
+
+def test_a_step_with_copies_is_the_step_without():
+    """A hook that does nothing makes every layer convert its own weight: same loss, same gradients, bit for bit (two documents of one tile: attention's
+    dq adds nothing up in the order of arrival)."""
+    from tagseq2tagseq_b200 import MaskSpec
+    from tagseq2tagseq_b200.train_step import DecoderLM, LMConfig
+    torch.manual_seed(3)
+    vocab = 4096
+    with torch.device(DEV):
+        model = DecoderLM(LMConfig(2, 128, 2, 64, 256, vocab))
+    tokens = torch.randint(0, vocab, (1, 129), device=DEV)
+    spec = MaskSpec((torch.arange(128, device=DEV, dtype=torch.int32) // 70)[None], None)
+
+    def run():
+        model.zero_grad()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            loss = model(tokens, spec)
+        loss.backward()
+        return [loss.detach().clone()] + [p.grad.clone() for p in model.parameters()]
+
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert len(model._weight_copies()) == 9
+    want = run()
+    handle = model.blocks[1].proj.register_forward_pre_hook(lambda m, a: None)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert model._weight_copies() is None
+    for a, b in zip(run(), want):
+        assert torch.equal(a, b)
+    handle.remove()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        assert model._weight_copies() is None and torch.equal(model(tokens, spec), want[0])

@@ -68,7 +68,6 @@ struct BwdParams {
   int H, Tp;
   int head_group;        // heads whose CTAs are interleaved in the launch order
   float scale, scale_log2;
-  bool early;            // the conversion may start while this kernel runs
   TS2TS_BWD_TRACE_FIELDS
 };
 
@@ -255,7 +254,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t* s_masks = reinterpret_cast<uint32_t*>(bars + Cfg::kBars + 2);  // [Q stages][kStretches][kMaskRuns] the tile's masks, by run of the key
   uint32_t* s_tile = s_masks + Cfg::kQStages * kStretches * kMaskRuns;  // [kTileSlots][2] a tile's four stretch entries, 16 bits each
   static_assert(Cfg::kTileSlots > Cfg::kQStages, "");
-  if (p.early) let_next_start();
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -853,15 +851,12 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
     p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
   }
   BTRACE_ATTACH(p, stream);
-  // The three launches overlap (launch.cuh) where they are short: the main kernel's blocks set themselves up and bring in K and V
-  // under the preparation, the conversion's blocks wait where SMs have run dry.  us, one after the other -> overlapping: linked 600, H = 8,
-  // D = 64 23.0 -> 16.7; linked 1024, H = 4, D = 64 29.1 -> 22.9; causal 2 x 1000, H = 8, D = 128 38.7 -> 35.3; linked 5003, H = 12, D = 64 72.8 -> 66.9;
-  // causal 4096, H = 8, D = 128 95.9 -> 89.4.  At the line, D = 128, 384 tiles: documents 6144, H = 8 80.5 -> 75.7,
-  // linked 4096, H = 12 99.3 -> 97.8 (288 tiles 82.4 -> 81.4, 320 84.6 -> 85.5); D = 64, 768 tiles: linked 8k, H = 12 144.3 -> 141.1, documents 93.5 -> 88.3.
-  // Beyond it the gain ends, and long launches lose: linked 8k, H = 8, D = 128 (512 tiles) 140.6 -> 142.6, H = 14 and 16, D = 64 (896 and 1024 tiles)
-  // 170.2 -> 171.0 and 183.4 -> 183.0; linked 16k, H = 16, D = 128 968 -> 988, H = 12, D = 64 (1536 tiles) 457 -> 461.
+  // The main kernel's blocks set themselves up and bring in K and V under the preparation where the launches are short.  us, one after the other -> overlapping: documents
+  // 2048, H = 8, D = 64 19.2 -> 17.4; linked 1024, H = 4, D = 64 22.4 -> 21.1; causal 1024, H = 4, D = 128 28.2 -> 26.7; causal 4096, H = 4, D = 128 82.8 -> 80.9; linked 5003, H = 12,
+  // D = 64 63.9 -> 62.5; 2 x 1771, H = 12, D = 128 64.6 -> 63.6.  Beyond 384 tiles at D = 128 and 768 at D = 64 the gain ends and long launches lose: linked 8k, H = 12, D = 64 (768 tiles)
+  // 91.5 -> 93.6; below it two linked 6767, H = 2, D = 128 do, too (85.4 -> 88.0).  The conversion does not start under the main kernel: its blocks would wait where SMs
+  // have run dry, but a trigger in the main kernel costs more (the first five of the calls above 18.0, 21.2, 27.2, 82.2, 63.6; linked 16k, H = 16, D = 128 961 -> 982, H = 12, D = 64 441 -> 458).
   const bool early = (long long)B * H * P.NB * D <= 384 * 128;
-  p.early = early;
   cudaError_t launched = launch_after(bwd_prep_kernel<D>, dim3((unsigned)(rows / kPrepRows)), 256, 0, stream, static_cast<const __nv_bfloat16*>(out),
                                       static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1], sdo[2], H, T, Tp, stats, dq_acc, early);
   if (launched == cudaSuccess) {

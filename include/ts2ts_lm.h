@@ -70,6 +70,8 @@ int ts2ts_embedding_bwd(const int64_t* idx, const float* dx, float* dw, int64_t 
 
 /* dst[i][0..n[i]) (bf16) = src[i][0..n[i]) (fp32), rounded to nearest even, for `count` tensors.  src, dst: host arrays of device pointers. */
 int ts2ts_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, void* stream);
+/* bytes[i] bytes from src[i] to dst[i], at any alignment, for `count` tensors that do not overlap.  src, dst: host arrays of device pointers. */
+int ts2ts_copy(int count, const void* const* src, void* const* dst, const int64_t* bytes, void* stream);
 
 /* One AdamW step over `count` fp32 tensors.  p, g, m, v: host arrays of device pointers (parameter, gradient, first and
  * second moment); n: host array of element counts; steps: host array, the number of this step per tensor (from 1).

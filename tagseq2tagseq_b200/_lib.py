@@ -52,6 +52,7 @@ SYMBOLS = {
     "ts2ts_scale": (c_int, [c_void_p] * 3 + [c_int64, c_void_p]),
     "ts2ts_embedding_bwd": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_void_p]),
     "ts2ts_cast_bf16": (c_int, [c_int] + [c_void_p] * 4),
+    "ts2ts_copy": (c_int, [c_int] + [c_void_p] * 4),
     "ts2ts_adamw": (c_int, [c_int] + [c_void_p] * 6 + [c_double] * 5 + [c_void_p]),
 }
 

@@ -31,6 +31,7 @@ cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const flo
                                    void* da, float* dw, bool add, float* dw_part, int N, int C, cudaStream_t stream);
 int add_rmsnorm_bwd_blocks(int64_t N, int C);
 cudaError_t launch_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, cudaStream_t stream);
+cudaError_t launch_copy(int count, const void* const* src, void* const* dst, const int64_t* bytes, cudaStream_t stream);
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream);
 cudaError_t launch_swiglu_fwd(const void* gu, void* act, int64_t N, int F, cudaStream_t stream);
 cudaError_t launch_swiglu_bwd(const void* gu, const void* dact, void* dgu, int64_t N, int F, cudaStream_t stream);
@@ -448,6 +449,14 @@ int ts2ts_cast_bf16(int count, const float* const* src, void* const* dst, const 
   for (int i = 0; i < count; ++i)
     if (n[i] < 0 || (n[i] > 0 && (!src[i] || !dst[i]))) return fail(-3, "cast_bf16: tensor %d has a null pointer or a negative size", i);
   return launched(launch_cast_bf16(count, src, dst, n, static_cast<cudaStream_t>(stream)), "cast_bf16");
+}
+
+int ts2ts_copy(int count, const void* const* src, void* const* dst, const int64_t* bytes, void* stream) {
+  if (count < 0) return fail(-1, "count must not be negative");
+  if (count > 0 && (!src || !dst || !bytes)) return fail(-3, "copy: null pointer");
+  for (int i = 0; i < count; ++i)
+    if (bytes[i] < 0 || (bytes[i] > 0 && (!src[i] || !dst[i]))) return fail(-3, "copy: tensor %d has a null pointer or a negative size", i);
+  return launched(launch_copy(count, src, dst, bytes, static_cast<cudaStream_t>(stream)), "copy");
 }
 
 int ts2ts_adamw(int count, float* const* p, const float* const* g, float* const* m, float* const* v, const int64_t* n,

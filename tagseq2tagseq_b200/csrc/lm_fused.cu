@@ -252,32 +252,24 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restric
   }
 }
 
-// ---------------------------------------------------------------------------------------------- bf16 copies
-// All of a step's weights in one launch instead of one each: a block takes kCastChunk consecutive elements of one tensor.  HBM-bound, 6 bytes
-// an element.  us: the 17 weights of four layers at d_model 768 with 50304 words (76 M elements, 70 at the copy rate) 111 -> 72; nine of 3.6 M in all 17 in nine launches, below 5 in one.
-constexpr int kCastTensors = 128, kCastThreads = 256, kCastChunk = 8192;
-struct CastArgs {
-  const float* src[kCastTensors];
-  __nv_bfloat16* dst[kCastTensors];
-  int64_t n[kCastTensors];
-  int first_block[kCastTensors];
+// ---------------------------------------------------------------------------------------------- copies of many tensors
+// All of a step's weights to bf16, or all gradients of a step as they are, in one launch instead of one each: a block takes kMoveBytes consecutive bytes of
+// one source.  HBM-bound, 6 and 8 bytes an element.  us, bf16: the 17 weights of four layers at d_model 768 with 50304 words (76 M elements, 70 at the copy rate)
+// 111 -> 72; nine of 3.6 M in all 17 in nine launches, below 5 in one.  Copies: 15 gradients of 3.6 M elements and the loss 13.6 + 1.4 by torch's launches -> 7.
+constexpr int kMoveTensors = 128, kMoveThreads = 256, kMoveBytes = 32768;
+struct MoveArgs {
+  const void* src[kMoveTensors];
+  void* dst[kMoveTensors];
+  int64_t n[kMoveTensors];  // elements to convert, or bytes to copy
+  int first_block[kMoveTensors];
   int count;
 };
-__global__ void __launch_bounds__(kCastThreads) cast_bf16_kernel(const __grid_constant__ CastArgs a) {
-  int lo = 0, hi = a.count - 1;  // last tensor whose first block is not after this one
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.first_block[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-  }
-  wait_previous();
-  const float* src = settled(a.src[lo]);
-  __nv_bfloat16* dst = a.dst[lo];
-  const int64_t begin = (int64_t)((int)blockIdx.x - a.first_block[lo]) * kCastChunk, end = min(begin + (int64_t)kCastChunk, a.n[lo]);
+__device__ __forceinline__ void move_cast(const float* src, __nv_bfloat16* dst, int64_t begin, int64_t end) {
   int64_t i = begin;
   if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0) {
     const int64_t vend = begin + (end - begin) / 8 * 8;
 #pragma unroll 4
-    for (int64_t j = begin + 8 * threadIdx.x; j < vend; j += 8 * kCastThreads) {
+    for (int64_t j = begin + 8 * threadIdx.x; j < vend; j += 8 * kMoveThreads) {
       float f[8];
       *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src + j);
       *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + j + 4);
@@ -285,7 +277,38 @@ __global__ void __launch_bounds__(kCastThreads) cast_bf16_kernel(const __grid_co
     }
     i = vend;
   }
-  for (i += threadIdx.x; i < end; i += kCastThreads) dst[i] = __float2bfloat16_rn(src[i]);
+  for (i += threadIdx.x; i < end; i += kMoveThreads) dst[i] = __float2bfloat16_rn(src[i]);
+}
+// Bytes from `begin` on in pieces of Unit; returns where the last whole one ends.
+template <typename Unit> __device__ __forceinline__ int64_t move_units(const char* src, char* dst, int64_t begin, int64_t end) {
+  const int64_t uend = begin + (end - begin) / (int64_t)sizeof(Unit) * (int64_t)sizeof(Unit);
+#pragma unroll 8
+  for (int64_t j = begin + (int64_t)sizeof(Unit) * threadIdx.x; j < uend; j += sizeof(Unit) * kMoveThreads)
+    *reinterpret_cast<Unit*>(dst + j) = *reinterpret_cast<const Unit*>(src + j);
+  return uend;
+}
+template <bool kCast>
+__global__ void __launch_bounds__(kMoveThreads) move_kernel(const __grid_constant__ MoveArgs a) {
+  int lo = 0, hi = a.count - 1;  // last tensor whose first block is not after this one
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.first_block[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  wait_previous();
+  constexpr int kChunk = kCast ? kMoveBytes / 4 : kMoveBytes;
+  const void* src = settled(a.src[lo]);
+  const int64_t begin = (int64_t)((int)blockIdx.x - a.first_block[lo]) * kChunk, end = min(begin + (int64_t)kChunk, a.n[lo]);
+  if constexpr (kCast) {
+    move_cast(static_cast<const float*>(src), static_cast<__nv_bfloat16*>(a.dst[lo]), begin, end);
+  } else {
+    const char* from = static_cast<const char*>(src);
+    char* to = static_cast<char*>(a.dst[lo]);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(from) | reinterpret_cast<uintptr_t>(to);
+    int64_t i = begin;
+    if ((at & 15u) == 0) i = move_units<uint4>(from, to, i, end);
+    else if ((at & 3u) == 0) i = move_units<uint32_t>(from, to, i, end);
+    move_units<char>(from, to, i, end);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------- rotary embedding
@@ -767,23 +790,31 @@ cudaError_t launch_add_rmsnorm_bwd(const void* dh, const float* dx_up, const flo
   return e != cudaSuccess ? e : launch_after(column_sum_kernel, dim3((C + 31) / 32), 1024, 0, stream, dw_part, dw, grid, C, add);
 }
 
-cudaError_t launch_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, cudaStream_t stream) {
-  CastArgs a;
+template <bool kCast>
+cudaError_t launch_move(int count, const void* const* src, void* const* dst, const int64_t* n, cudaStream_t stream) {
+  constexpr int kChunk = kCast ? kMoveBytes / 4 : kMoveBytes;
+  MoveArgs a;
   for (int done = 0; done < count;) {
     int64_t blocks = 0;
     a.count = 0;
-    for (; done < count && a.count < kCastTensors; ++done) {
-      const int64_t need = (n[done] + kCastChunk - 1) / kCastChunk;
+    for (; done < count && a.count < kMoveTensors; ++done) {
+      const int64_t need = (n[done] + kChunk - 1) / kChunk;
       if (need == 0) continue;
       if (a.count > 0 && blocks + need > 0x7fffffff) break;
-      a.src[a.count] = src[done]; a.dst[a.count] = static_cast<__nv_bfloat16*>(dst[done]); a.n[a.count] = n[done];
+      a.src[a.count] = src[done]; a.dst[a.count] = dst[done]; a.n[a.count] = n[done];
       a.first_block[a.count++] = (int)blocks;
       blocks += need;
     }
-    const cudaError_t e = blocks > 0 ? launch_after(cast_bf16_kernel, dim3((unsigned)blocks), kCastThreads, 0, stream, a) : cudaSuccess;
+    const cudaError_t e = blocks > 0 ? launch_after(move_kernel<kCast>, dim3((unsigned)blocks), kMoveThreads, 0, stream, a) : cudaSuccess;
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+cudaError_t launch_cast_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, cudaStream_t stream) {
+  return launch_move<true>(count, reinterpret_cast<const void* const*>(src), dst, n, stream);
+}
+cudaError_t launch_copy(int count, const void* const* src, void* const* dst, const int64_t* bytes, cudaStream_t stream) {
+  return launch_move<false>(count, src, dst, bytes, stream);
 }
 
 cudaError_t launch_rope_qk(void* qkv, const float* cs, const float* sn, int B, int T, int H, int D, float sign, cudaStream_t stream) {

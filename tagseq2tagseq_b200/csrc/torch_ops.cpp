@@ -700,6 +700,29 @@ std::vector<Tensor> cast_weights(at::TensorList ws) {
   return out;
 }
 
+// dst[i] = src[i].  Those that lie alike and whole go in one launch, the others through torch one by one.
+void copy_tensors(at::TensorList dst, at::TensorList src) {
+  TORCH_CHECK_VALUE(dst.size() == src.size(), "copy_tensors: lists of equal length");
+  std::vector<const void*> from;
+  std::vector<void*> to;
+  std::vector<int64_t> bytes;
+  c10::optional<c10::Device> device;
+  for (size_t i = 0; i < dst.size(); ++i) {
+    const Tensor &d = dst[i], &s = src[i];
+    if (d.is_cuda() && s.device() == d.device() && (!device.has_value() || *device == d.device()) && d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() &&
+        d.is_contiguous() && s.is_contiguous() && !d.requires_grad() && !s.is_neg() && !s.is_conj()) {
+      device = d.device();
+      from.push_back(s.const_data_ptr()); to.push_back(d.mutable_data_ptr()); bytes.push_back(static_cast<int64_t>(d.nbytes()));
+      if (!d.is_inference()) d.unsafeGetTensorImpl()->bump_version();
+    } else {
+      d.copy_(s);
+    }
+  }
+  if (from.empty()) return;
+  const CUDAGuard guard(*device);
+  check(ts2ts_copy(static_cast<int>(from.size()), from.data(), to.data(), bytes.data(), at::cuda::getCurrentCUDAStream(device->index()).stream()), "ts2ts_copy");
+}
+
 struct Linear : torch::autograd::Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& copy) {
     need_cuda(x);
@@ -853,6 +876,7 @@ TORCH_LIBRARY(ts2ts, m) {
   m.def("swiglu(Tensor gate_up) -> Tensor", swiglu);
   m.def("cross_entropy(Tensor logits, Tensor target) -> Tensor", cross_entropy);
   m.def("cast_weights(Tensor[] ws) -> Tensor[]", cast_weights);
+  m.def("copy_tensors(Tensor(a!)[] dst, Tensor[] src) -> ()", copy_tensors);
   m.def("linear(Tensor x, Tensor w, Tensor? copy=None) -> Tensor", linear);
   m.def("head_loss(Tensor h, Tensor w, Tensor target, Tensor? copy=None) -> Tensor", head_loss);
   m.def("embedding(Tensor w, Tensor idx) -> Tensor", embedding);

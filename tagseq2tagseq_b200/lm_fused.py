@@ -15,7 +15,7 @@ from torch.autograd import forward_ad as fwAD
 from . import _lib
 from .mask_spec import MaskSpec
 
-__all__ = ["add_rmsnorm", "qkv_attention", "swiglu", "cross_entropy", "head_loss", "embedding", "rope_half_tables", "cast_weights", "Linear", "AdamW"]
+__all__ = ["add_rmsnorm", "qkv_attention", "swiglu", "cross_entropy", "head_loss", "embedding", "rope_half_tables", "cast_weights", "copy_tensors", "Linear", "AdamW"]
 
 _lib.load_if_built()
 _MAX_HEAD_COLUMNS = 110592  # a row of logits that ts2ts_ce_fwd_grad keeps in shared memory
@@ -104,6 +104,11 @@ def cast_weights(weights) -> list:
     """bf16 copies of contiguous fp32 CUDA weights, all in one launch."""
     _need_cuda(*weights)
     return _call(_lib.ops().cast_weights.default, weights)
+
+
+def copy_tensors(dst, src) -> None:
+    """``d.copy_(s)`` for every pair, in one launch for those on the GPU that are of one type and size and contiguous."""
+    _call(_lib.ops().copy_tensors.default, dst, src)
 
 
 class Linear(nn.Linear):

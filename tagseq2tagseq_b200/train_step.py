@@ -24,7 +24,7 @@ import torch.nn.modules.module as _module
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 
-from .lm_fused import AdamW, Linear, add_rmsnorm, cast_weights, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
+from .lm_fused import AdamW, Linear, add_rmsnorm, cast_weights, copy_tensors, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -258,18 +258,14 @@ class _StepGraph:
         self.mask._block_map = None  # built by the graph, into its own pool
 
     def _load(self, tokens, mask):
-        self.tokens.copy_(tokens)
         m = self.mask
-        m.doc_ids.copy_(mask.doc_ids)
-        if m.q_row_ids is not None:
-            m.q_row_ids.copy_(mask.q_row_ids)
-        if m.kv_col_ids is not None:
-            m.kv_col_ids.copy_(mask.kv_col_ids)
+        pairs = [(self.tokens, tokens), (m.doc_ids, mask.doc_ids), (m.q_row_ids, mask.q_row_ids), (m.kv_col_ids, mask.kv_col_ids)]
         if m.link_bits is not None:
             R, W = mask.link_bits.shape[1:]
             if m.link_bits.shape[1:] != (R, W):
                 m.link_bits.zero_()
-            m.link_bits[:, :R, :W].copy_(mask.link_bits)
+            pairs.append((m.link_bits[:, :R, :W], mask.link_bits))
+        copy_tensors(*zip(*(p for p in pairs if p[0] is not None)))
 
     def run(self, tokens, mask) -> torch.Tensor:
         here = torch.cuda.current_stream()
@@ -283,10 +279,11 @@ class _StepGraph:
         self._load(tokens, mask)
         self.graph.replay()
         grads = [torch.empty_like(p) for p in self.params]  # the graph's own buffers are written again by the next step
-        torch._foreach_copy_(grads, self.grads)
+        loss = torch.empty_like(self.loss)
+        copy_tensors([*grads, loss], [*self.grads, self.loss])
         for p, g in zip(self.params, grads):
             p.grad = g
-        return self.loss.clone()
+        return loss
 
 
 class TrainStep:

@@ -278,7 +278,7 @@ struct FwdPlaces {
   FwdItem* s_item;  // [2]
   uint64_t* bars;
   uint64_t* bar_item_full;  // [2] the producer published an item
-  uint64_t* bar_item_empty;  // [2] the eight softmax warps copied it
+  uint64_t* bar_item_empty;  // [2] the eight softmax warps are through with it
   uint64_t* bar_q_full;  // [team] Q tile landed
   uint64_t* bar_q_free;  // [team] last S of the item complete: the Q buffer may be reloaded
   uint64_t* bar_s;  // [team] S of the tile is in tensor memory
@@ -892,10 +892,11 @@ enum FwdForm { kFwdPairs, kFwdShared, kFwdByLists };
 // Every CTA comes to the same answer, because it depends on the plan and the grid (one CTA per SM) alone.  As pairs a launch that is short of items takes as long
 // as its longest list, 2.0 us a tile and 2.2 us at its ends.  As shared tiles it takes an SM's share of all lists, two tiles at a time in 1.65 us (D = 64; 2.0 us at
 // D = 128, where two K/V streams do not fit the ring), and 2.7 us for each of the SM's items.  Shared tiles are taken where they come to less than 0.8 of the pairs'
-// time: of 90 random calls (T = 512 to 20000, 1 to 4 sequences, 2 to 16 heads, all kinds of masks) that picks the slower form by more than 4 % twice (12 and 13 %).  us, pairs | shared:
+// time: of 85 random calls (T = 512 to 20000, 1 to 4 sequences, 2 to 16 heads, all kinds of masks) that picks the slower form by more than 4 % three times (6, 9 and
+// 10 %, all three H = 12, D = 64 just above one pair an SM: 2 x 2006, 2 x 1609, causal 4 x 731).  us, pairs | shared:
 // linked 14545, H = 3, D = 128 144 | 89; linked 5169, H = 8, D = 64 87 | 54; causal 4 x 3787, H = 3, D = 128 77 | 56; at the line linked 2 x 3156, H = 12, D = 64
 // 48.0 | 48.3 and 6273, H = 12, D = 128 92 | 91; beyond it linked 2 x 2455, H = 16, D = 64 46 | 50, causal 4 x 2902, H = 12, D = 64 101 | 108.
-// A kernel with both bodies runs either one up to 1.5 us slower than a kernel of its own.
+// A kernel with both bodies runs either one 0 to 2.4 us slower than a kernel of its own.
 template <int D>
 __device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p, long long longest, long long all) {
   return (D == 64 ? 33 : 40) * all * p.H + 108ll * p.n_tiles < gridDim.x * (64 * longest + 70);

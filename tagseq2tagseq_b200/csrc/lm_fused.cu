@@ -446,9 +446,9 @@ __global__ void ce_bwd_kernel(__nv_bfloat16* logits, const int64_t* __restrict__
 // instead of the 6 of the two kernels above; two blocks of a 50304-logit row share an SM, so that one's copy overlaps the
 // other's arithmetic.  The gradient is that of the mean loss (times inv_n, not times what reaches the loss from above).
 // What is left beside the copy are two exponentials a logit: maxima are taken of bf16 pairs, four vectors of a thread between two looks at the
-// running one, scale and shift are one packed multiply-add, only the target's vector knows of it.  A block has as many threads as leave each 8 to 16 vectors (12 to 27 from 4096 vectors on).
-// us (floor at the copy rate; one comparison and a maximum a logit, 512 threads whatever the row -> now): 16384 x 50304 (504) 641 -> 555, x 32768 (328) 415 -> 333,
-// x 16384 (164) 230 -> 166, x 4096 (41) 120 -> 49; 1024 x 4096 (3) 14.4 -> 11.1.  512 threads for x 32768 343, 256 for x 50304 574.
+// running one, difference and scale are packed, only the target's vector knows of it.  A block has as many threads as leave each 8 to 16 vectors (12 to 27 from 4096 vectors on).
+// us (floor at the copy rate; one comparison and a maximum a logit, 512 threads whatever the row -> now): 16384 x 50304 (504) 650 -> 557, x 32768 (328) 422 -> 338,
+// x 16384 (164) 235 -> 167, x 4096 (41) 120 -> 50; 1024 x 4096 (3) 15.8 -> 12.8.  512 threads for x 32768 343, 256 for x 50304 574.
 constexpr int kCeRowBytes = 216 * 1024;
 constexpr uint32_t kNoLogits = 0xff80ff80u;  // two of -inf
 constexpr float kLog2e = 1.4426950408889634f;
@@ -463,14 +463,15 @@ __device__ __forceinline__ float max_bf16x8(const uint4 (&raw)[kN]) {
   }
   return fmaxf(__low2float(most), __high2float(most));
 }
-// 2^(f log2(e) + shift) of eight values, two to a multiply-add.
-__device__ __forceinline__ void exp2_bf16x8(uint4 raw, float shift, float (&e)[8]) {
+// exp(f - most) of eight values, two to an operation.  The difference is taken before the scaling: where logits are large (the lowest value stands for a class that is
+// ruled out) a scaled maximum is off by more than an exponent can be, or past what fp32 holds.  One multiply-add for both would save 1 % (16384 x 50304 552 us).
+__device__ __forceinline__ void exp_bf16x8(uint4 raw, float most, float (&e)[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  const unsigned long long scale2 = pack_f32x2(kLog2e, kLog2e), shift2 = pack_f32x2(shift, shift);
+  const unsigned long long scale2 = pack_f32x2(kLog2e, kLog2e), less2 = pack_f32x2(-most, -most);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float a, b;
-    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u)), scale2, shift2), a, b);
+    unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u)), less2), scale2), a, b);
     e[2 * i] = fast_exp2(a);
     e[2 * i + 1] = fast_exp2(b);
   }
@@ -510,19 +511,17 @@ __global__ void __launch_bounds__(kThreads) ce_fwd_grad_kernel(__nv_bfloat16* lo
     for (int u = 0; u < kN; ++u) raw[u] = u == 0 || c + u * kThreads < end ? sv[c + u * kThreads] : make_uint4(kNoLogits, kNoLogits, kNoLogits, kNoLogits);
     const float m_new = fmaxf(m, max_bf16x8(raw));
     if (m_new == -CUDART_INF_F) return;
-    // sum of exp(f - m_new) as 2^(f log2(e) + shift); what rounding m_new log2(e) took away is multiplied back in
-    const float shift = -m_new * kLog2e;
     unsigned long long sum[2] = {0ull, 0ull};
 #pragma unroll
     for (int u = 0; u < kN; ++u) {
       float e[8];
-      exp2_bf16x8(raw[u], shift, e);
+      exp_bf16x8(raw[u], m_new, e);
 #pragma unroll
       for (int i = 0; i < 8; i += 2) sum[(i >> 1) & 1] = add_f32x2(sum[(i >> 1) & 1], pack_f32x2(e[i], e[i + 1]));
     }
     float a, b;
     unpack_f32x2(add_f32x2(sum[0], sum[1]), a, b);
-    s = s * __expf(m - m_new) + (a + b) * fast_exp2(fmaf(-m_new, kLog2e, -shift));
+    s = s * __expf(m - m_new) + (a + b);
     m = m_new;
   };
   bool ok = true;
@@ -549,19 +548,19 @@ __global__ void __launch_bounds__(kThreads) ce_fwd_grad_kernel(__nv_bfloat16* lo
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     return;
   }
-  const float g = live ? inv_n : 0.f, shift = -l * kLog2e, part = fast_exp2(fmaf(-l, kLog2e, -shift));
-  const unsigned long long scale2 = pack_f32x2(part * g, part * g);
+  const float g = live ? inv_n : 0.f;
+  const unsigned long long scale2 = pack_f32x2(g, g);
   const int hit_vec = live ? static_cast<int>(tg >> 3) : -1;
 #pragma unroll 2
   for (int c = tid; c < n_vec; c += kThreads) {
     float f[8];
-    exp2_bf16x8(sv[c], shift, f);
+    exp_bf16x8(sv[c], l, f);
     if (c != hit_vec) {
 #pragma unroll
       for (int i = 0; i < 8; i += 2) unpack_f32x2(mul_f32x2(pack_f32x2(f[i], f[i + 1]), scale2), f[i], f[i + 1]);
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = (f[i] * part - (i == static_cast<int>(tg & 7) ? 1.f : 0.f)) * g;
+      for (int i = 0; i < 8; ++i) f[i] = (f[i] - (i == static_cast<int>(tg & 7) ? 1.f : 0.f)) * g;
     }
     reinterpret_cast<uint4*>(row)[c] = float_to_bf16x8(f);
   }

@@ -152,6 +152,7 @@ class DecoderLM(nn.Module):
         layers = [m for blk in self.blocks if _plain(blk, Block) for m in blk.linears()] + [self.head]
         if (len(layers) != 4 * len(self.blocks) + 1 or torch.compiler.is_compiling() or not torch.is_grad_enabled() or transformed()
                 or not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") != torch.bfloat16
+                or any(cls.forward is not _OWN_FORWARD[cls] for cls in (Block, Linear))
                 or not all(_plain(m, Linear) and m.bias is None for m in layers)):
             return None
         weights = [m.weight for m in layers]

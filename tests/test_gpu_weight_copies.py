@@ -51,3 +51,43 @@ def test_a_step_with_copies_is_the_step_without():
     handle.remove()
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
         assert model._weight_copies() is None and torch.equal(model(tokens, spec), want[0])
+
+
+def _small(vocab=4096):
+    from tagseq2tagseq_b200 import MaskSpec
+    from tagseq2tagseq_b200.train_step import DecoderLM, LMConfig
+    torch.manual_seed(3)
+    with torch.device(DEV):
+        model = DecoderLM(LMConfig(2, 128, 2, 64, 256, vocab))
+    tokens = torch.randint(0, vocab, (1, 129), device=DEV)
+    spec = MaskSpec((torch.arange(128, device=DEV, dtype=torch.int32) // 70)[None], None)
+
+    def run():
+        model.zero_grad()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            loss = model(tokens, spec)
+        loss.backward()
+        return [loss.detach().clone()] + [p.grad.clone() for p in model.parameters()]
+    return model, run
+
+
+@pytest.mark.parametrize("which", ["Linear", "Block"])
+def test_a_forward_replaced_on_the_class_gets_the_arguments_it_always_got(which, monkeypatch):
+    from tagseq2tagseq_b200 import train_step
+    model, run = _small()
+    want = run()
+    cls, calls = getattr(train_step, which), []
+    own = cls.forward
+
+    def linear(self, x):
+        calls.append(self)
+        return own(self, x)
+
+    def block(self, x, a, mask, cos, sin):
+        calls.append(self)
+        return own(self, x, a, mask, cos, sin)
+
+    monkeypatch.setattr(cls, "forward", linear if which == "Linear" else block)
+    for a, b in zip(run(), want):
+        assert torch.equal(a, b)
+    assert len(calls) == (8 if which == "Linear" else 2)

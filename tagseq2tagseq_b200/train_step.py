@@ -150,7 +150,7 @@ class DecoderLM(nn.Module):
         """The bf16 copies that this forward's linear layers keep for their backward, ((copy,), ...) by layer and then the head's, made in one launch.  None
         where a layer would not take one, or somebody's code could look at a weight, or change it, on the way."""
         layers = [m for blk in self.blocks if _plain(blk, Block) for m in blk.linears()] + [self.head]
-        if (len(layers) != 4 * len(self.blocks) + 1 or torch.compiler.is_compiling() or not torch.is_grad_enabled() or transformed()
+        if (len(layers) != 4 * len(self.blocks) + 1 or torch.compiler.is_compiling() or not torch.is_grad_enabled() or _observed()
                 or not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") != torch.bfloat16
                 or any(cls.forward is not _OWN_FORWARD[cls] for cls in (Block, Linear))
                 or not all(_plain(m, Linear) and m.bias is None for m in layers)):

@@ -91,3 +91,43 @@ def test_a_forward_replaced_on_the_class_gets_the_arguments_it_always_got(which,
     for a, b in zip(run(), want):
         assert torch.equal(a, b)
     assert len(calls) == (8 if which == "Linear" else 2)
+
+
+def test_no_copies_ahead_where_something_of_the_callers_is_called_on_the_way():
+    """Saved tensors that go to the host as they are saved, and modes that see every operator: each layer converts its own weight when it is its turn."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from tagseq2tagseq_b200 import MaskSpec
+    from tagseq2tagseq_b200.train_step import DecoderLM, LMConfig
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    small, _ = _small()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        for mode in (Function(), Dispatch(), torch.autograd.graph.save_on_cpu()):
+            with mode:
+                assert small._weight_copies() is None
+        assert len(small._weight_copies()) == 9
+
+    with torch.device(DEV):
+        model = DecoderLM(LMConfig(6, 512, 8, 64, 2048, 8192))         # 25 M + 4 M weights
+    tokens = torch.randint(0, 8192, (1, 129), device=DEV)
+    spec = MaskSpec(torch.zeros((1, 128), device=DEV, dtype=torch.int32), None)
+
+    def peak():
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        with torch.autocast("cuda", dtype=torch.bfloat16), torch.autograd.graph.save_on_cpu():
+            model(tokens, spec)
+        return torch.cuda.max_memory_allocated() - before
+    peak()                                                            # the plan, the rotation tables
+    got = peak()
+    model.blocks[0].proj.register_forward_pre_hook(lambda m, a: None)  # with a hook no copies are made ahead
+    assert got <= peak() + (1 << 20)

@@ -158,6 +158,9 @@ class DecoderLM(nn.Module):
         weights = [m.weight for m in layers]
         if not all(type(w) in (nn.Parameter, torch.Tensor) and w.is_cuda and w.device == weights[0].device and w.dtype == torch.float32 and w.is_contiguous() for w in weights):
             return None
+        # Frozen weights below the first one that learns are kept by nobody.
+        if not (weights[0].requires_grad or getattr(getattr(self.embed, "weight", None), "requires_grad", False)):
+            return None
         return [(c,) for c in cast_weights(weights)]
 
     def forward(self, tokens: torch.Tensor, mask: MaskSpec, rope=None) -> torch.Tensor:

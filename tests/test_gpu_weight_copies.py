@@ -131,3 +131,33 @@ def test_no_copies_ahead_where_something_of_the_callers_is_called_on_the_way():
     got = peak()
     model.blocks[0].proj.register_forward_pre_hook(lambda m, a: None)  # with a hook no copies are made ahead
     assert got <= peak() + (1 << 20)
+
+
+@pytest.mark.parametrize("frozen", ["all", "embedding and first layers"])
+def test_copies_that_no_backward_keeps_are_not_held(frozen):
+    from tagseq2tagseq_b200 import MaskSpec
+    from tagseq2tagseq_b200.train_step import DecoderLM, LMConfig
+    with torch.device(DEV):
+        model = DecoderLM(LMConfig(6, 512, 8, 64, 2048, 8192))
+    for name, p in model.named_parameters():
+        p.requires_grad_(frozen != "all" and name.startswith(("blocks.5", "norm", "head")))
+    tokens = torch.randint(0, 8192, (1, 129), device=DEV)
+    spec = MaskSpec(torch.zeros((1, 128), device=DEV, dtype=torch.int32), None)
+
+    def peak():
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            model(tokens, spec)
+        return torch.cuda.max_memory_allocated() - before
+    peak()                                                            # the plan, the rotation tables
+    got = peak()
+    model.blocks[0].proj.register_forward_pre_hook(lambda m, a: None)  # with a hook no copies are made ahead
+    assert got <= peak() + (1 << 20)
+    for p in (model.embed.weight, model.blocks[0].qkv.weight):        # either makes every layer keep its own
+        model.blocks[0].proj._forward_pre_hooks.clear()
+        model.requires_grad_(False)
+        p.requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert len(model._weight_copies()) == 25

@@ -674,10 +674,11 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& target) { return CrossE
 // conversion pass (6 bytes per weight) on the way to the parameter.  x is saved as it was passed, so that writing to it
 // before the backward is noticed; of w only the bf16 copy is needed, and a changed w does not matter.  A gradient that may be
 // differentiated again (create_graph) is made of ordinary operators on x and w themselves.
-// `copy`, the weight in bf16 where the caller has made one (cast_weights), or a copy of this call's own.
+// `copy`, the weight in bf16 where the caller has made one (cast_weights; what it holds is taken as it is), or a copy of this call's own.
 Tensor bf16_of(const Tensor& w, const OptTensor& copy) {
   if (!copy.has_value()) return w.to(at::kBFloat16);
   TORCH_CHECK_VALUE(copy->scalar_type() == at::kBFloat16 && copy->sizes() == w.sizes() && copy->device() == w.device(), "the weight's copy is bf16 and of its size");
+  TORCH_CHECK_VALUE(!copy->requires_grad(), "the weight's copy does not require grad: the weight itself gets the gradient");
   return *copy;
 }
 // The bf16 copies of fp32 weights, all in one launch.

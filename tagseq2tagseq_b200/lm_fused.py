@@ -74,8 +74,8 @@ def cross_entropy(logits: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
 
 
 def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor, copy: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call.  ``copy``: the
-    weight in bf16, for a caller that has it."""
+    """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call.  ``copy``: what
+    ``cast_weights`` made of the weight as it is now, for a caller that has it; its values are not looked at, and the gradient is the weight's."""
     if target.numel() != h.shape[:-1].numel():
         raise ValueError("head_loss: one target per row of h")
     _need_cuda(h, weight, target)
@@ -119,7 +119,7 @@ class Linear(nn.Linear):
         super().__init__(in_features, out_features, bias=False)
 
     def forward(self, x: torch.Tensor, copy: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """``copy``: the weight in bf16, for a caller that has made one (``cast_weights``)."""
+        """``copy``: as for ``head_loss``."""
         if (x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
                 and torch.get_autocast_dtype("cuda") == torch.bfloat16 and (torch.compiler.is_compiling() or not transformed())):
             return _call(_lib.ops().linear.default, x, self.weight, copy)

@@ -161,3 +161,20 @@ def test_copies_that_no_backward_keeps_are_not_held(frozen):
         p.requires_grad_(True)
         with torch.autocast("cuda", dtype=torch.bfloat16):
             assert len(model._weight_copies()) == 25
+
+
+def test_a_copy_is_bf16_of_the_weights_size_and_without_a_gradient():
+    from tagseq2tagseq_b200.lm_fused import Linear, cast_weights, head_loss
+    with torch.device(DEV):
+        layer, x, target = Linear(64, 128), torch.randn(9, 64).bfloat16(), torch.randint(0, 128, (9,))
+    good, = cast_weights([layer.weight])
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = layer(x), head_loss(x, layer.weight, target)
+        assert torch.equal(layer(x, good), want[0]) and torch.equal(head_loss(x, layer.weight, target, good), want[1])
+        for bad in (good.float(), good[:64], good.clone().requires_grad_(), layer.weight.to(torch.bfloat16)):
+            with pytest.raises(ValueError):
+                layer(x, bad)
+            with pytest.raises(ValueError):
+                head_loss(x, layer.weight, target, bad)
+    head_loss(x, layer.weight, target, good).backward()
+    assert layer.weight.grad is not None and good.grad is None

@@ -8,6 +8,7 @@
 #include "../../include/ts2ts_lm.h"
 
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -701,27 +702,59 @@ std::vector<Tensor> cast_weights(at::TensorList ws) {
   return out;
 }
 
-// dst[i] = src[i].  Those that lie alike and whole go in one launch, the others through torch one by one.
+// Whether d.copy_(s) moves bytes and does nothing else.
+bool bytes_only(const Tensor& d, const Tensor& s) {
+  for (const Tensor* t : {&d, &s})
+    if (!t->is_cuda() || at::isTensorSubclassLike(*t) || t->is_nested() || t->layout() != at::kStrided || t->_is_zerotensor() || t->is_neg() || t->is_conj() ||
+        !t->is_contiguous() || t->_fw_grad(0).defined())
+      return false;
+  return s.device() == d.device() && d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() && !d.requires_grad() && !d.is_inference() &&
+         !(at::GradMode::is_enabled() && s.requires_grad());
+}
+// Whether some pair's target shares memory with another tensor of the list: the pairs then depend on their order.
+bool targets_overlap(const std::vector<std::pair<Tensor, Tensor>>& pairs) {
+  struct Range { uintptr_t begin, end; bool target; };
+  std::vector<Range> ranges;
+  for (const auto& [d, s] : pairs)
+    for (const Tensor* t : {&d, &s})
+      if (const auto at = reinterpret_cast<uintptr_t>(t->const_data_ptr()); t->nbytes() > 0) ranges.push_back({at, at + t->nbytes(), t == &d});
+  std::sort(ranges.begin(), ranges.end(), [](const Range& a, const Range& b) { return a.begin < b.begin; });
+  uintptr_t any = 0, target = 0;  // where what came before ends
+  for (const Range& r : ranges) {
+    if (r.begin < (r.target ? any : target)) return true;
+    any = std::max(any, r.end);
+    if (r.target) target = std::max(target, r.end);
+  }
+  return false;
+}
+void copy_together(std::vector<std::pair<Tensor, Tensor>>& pairs) {
+  if (pairs.empty()) return;
+  if (targets_overlap(pairs)) {
+    for (auto& [d, s] : pairs) d.copy_(s);
+  } else {
+    std::vector<const void*> from;
+    std::vector<void*> to;
+    std::vector<int64_t> bytes;
+    for (auto& [d, s] : pairs) {
+      from.push_back(s.const_data_ptr()); to.push_back(d.mutable_data_ptr()); bytes.push_back(static_cast<int64_t>(d.nbytes()));
+      d.unsafeGetTensorImpl()->bump_version();
+    }
+    const CUDAGuard guard(pairs[0].first.device());
+    check(ts2ts_copy(static_cast<int>(from.size()), from.data(), to.data(), bytes.data(), stream_of(pairs[0].first)), "ts2ts_copy");
+  }
+  pairs.clear();
+}
+// dst[i].copy_(src[i]), one after the other as far as that can be told: neighbours that only move bytes, of tensors apart from each other, go in one launch.
 void copy_tensors(at::TensorList dst, at::TensorList src) {
   TORCH_CHECK_VALUE(dst.size() == src.size(), "copy_tensors: lists of equal length");
-  std::vector<const void*> from;
-  std::vector<void*> to;
-  std::vector<int64_t> bytes;
-  c10::optional<c10::Device> device;
+  std::vector<std::pair<Tensor, Tensor>> together;
   for (size_t i = 0; i < dst.size(); ++i) {
-    const Tensor &d = dst[i], &s = src[i];
-    if (d.is_cuda() && s.device() == d.device() && (!device.has_value() || *device == d.device()) && d.scalar_type() == s.scalar_type() && d.sizes() == s.sizes() &&
-        d.is_contiguous() && s.is_contiguous() && !d.requires_grad() && !s.is_neg() && !s.is_conj()) {
-      device = d.device();
-      from.push_back(s.const_data_ptr()); to.push_back(d.mutable_data_ptr()); bytes.push_back(static_cast<int64_t>(d.nbytes()));
-      if (!d.is_inference()) d.unsafeGetTensorImpl()->bump_version();
-    } else {
-      d.copy_(s);
-    }
+    const bool joins = bytes_only(dst[i], src[i]);
+    if (!joins || (!together.empty() && together[0].first.device() != dst[i].device())) copy_together(together);
+    if (joins) together.emplace_back(dst[i], src[i]);
+    else dst[i].copy_(src[i]);
   }
-  if (from.empty()) return;
-  const CUDAGuard guard(*device);
-  check(ts2ts_copy(static_cast<int>(from.size()), from.data(), to.data(), bytes.data(), at::cuda::getCurrentCUDAStream(device->index()).stream()), "ts2ts_copy");
+  copy_together(together);
 }
 
 struct Linear : torch::autograd::Function<Linear> {

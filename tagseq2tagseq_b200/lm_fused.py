@@ -107,8 +107,12 @@ def cast_weights(weights) -> list:
 
 
 def copy_tensors(dst, src) -> None:
-    """``d.copy_(s)`` for every pair, in one launch for those on the GPU that are of one type and size and contiguous."""
-    _call(_lib.ops().copy_tensors.default, dst, src)
+    """``d.copy_(s)`` for every pair, in order; neighbours on one GPU that are of one type and size, contiguous and apart from each other in one launch."""
+    if transformed() and not torch.compiler.is_compiling():
+        for d, s in zip(dst, src, strict=True):
+            d.copy_(s)
+    else:
+        _call(_lib.ops().copy_tensors.default, dst, src)
 
 
 class Linear(nn.Linear):

@@ -27,3 +27,49 @@ def test_every_pair_is_copied_and_nothing_else():
     copy_tensors([], [])
     with pytest.raises(ValueError):
         copy_tensors(dsts[:2], srcs[:1])
+
+
+def test_pairs_that_share_memory_are_copied_in_order():
+    from tagseq2tagseq_b200.lm_fused import copy_tensors
+
+    def chain(copy):
+        base = torch.arange(300000, device=DEV, dtype=torch.float32)
+        a, b, c = base[:100000], base[100000:200000], base[200000:]
+        copy([b, c, a, b], [a, b, c, torch.full_like(b, 7)])      # each reads what the one before wrote, two write to one place
+        copy([c.view(200, 500).t(), a[:100000]], [a.view(500, 200), c])  # a strided target between
+        copy([a, a], [a, b])                                      # onto itself
+        return base
+    one_by_one = lambda dst, src: [d.copy_(s) for d, s in zip(dst, src)]
+    assert torch.equal(chain(copy_tensors), chain(one_by_one))
+
+
+def test_what_a_copy_does_besides_moving_bytes():
+    from tagseq2tagseq_b200.lm_fused import copy_tensors
+    x = torch.randn(5, device=DEV, requires_grad=True)
+    w = torch.randn(5, device=DEV)
+    d, e = torch.empty(5, device=DEV), torch.empty(5, device=DEV)
+    copy_tensors([d, e], [x * 3, w])                              # the history of a source
+    assert torch.equal(e, w) and torch.equal(torch.autograd.grad(d.sum(), x)[0], torch.full_like(w, 3))
+    with torch.no_grad():
+        d = torch.empty(5, device=DEV)
+        copy_tensors([d, x], [x, w])
+    assert not d.requires_grad and torch.equal(x.detach(), w)
+    with pytest.raises(RuntimeError):                             # a leaf that learns
+        copy_tensors([x], [w])
+    copy_tensors([d], [torch._efficientzerotensor(5, device=DEV)])
+    assert torch.equal(d, torch.zeros(5, device=DEV))
+    with torch.inference_mode():
+        frozen = torch.zeros(5, device=DEV)
+    with pytest.raises(RuntimeError):                             # no writes to it outside
+        copy_tensors([frozen], [w])
+    with torch.autograd.forward_ad.dual_level():
+        d = torch.empty(5, device=DEV)
+        copy_tensors([d], [torch.autograd.forward_ad.make_dual(w, 2 * w)])
+        assert torch.equal(torch.autograd.forward_ad.unpack_dual(d).tangent, 2 * w)
+
+    def twice(a):
+        out = torch.empty_like(a)
+        copy_tensors([out], [a])
+        return 2 * out
+    rows = torch.randn(3, 5, device=DEV)
+    assert torch.equal(torch.func.vmap(twice)(rows), 2 * rows)

@@ -345,6 +345,8 @@ class CrossDocLinkMaskCreator:
                 out[pos] = [hit[0]]
         return out
 
+    _own_match_links_to_docs = _match_links_to_docs
+
     def __call__(self, tokens: torch.Tensor, doc_spans: List[Any], **kwargs) -> MaskSpec:
         seq_len = tokens.shape[-1]
         detector = self.link_detector
@@ -352,7 +354,7 @@ class CrossDocLinkMaskCreator:
         # the time the caller's decode function: 608 -> 520 us; with classes hashed and link bits joined grant by grant in native code 438).
         kind = type(detector)
         if (tokens.is_cuda and getattr(kind, "detect_links", None) is getattr(kind, "_own_detect_links", 0) and "detect_links" not in vars(detector)
-                and type(self)._match_links_to_docs is CrossDocLinkMaskCreator._match_links_to_docs and "_match_links_to_docs" not in vars(self)):
+                and type(self)._match_links_to_docs is CrossDocLinkMaskCreator._own_match_links_to_docs and "_match_links_to_docs" not in vars(self)):
             pairs = detector.matched(tokens[0], self._index(doc_spans))
             cap = self._current_max_grants()
             self._step += 1

@@ -47,3 +47,26 @@ def test_a_growing_window_may_close_behind_the_next_link():
     links = [tuple(link) for link in detector.detect_links(tokens)]
     assert links == [(6, "a b"), (5, "b")]
     assert detector.matched(tokens, creator._index(spans)) == [(5, 8), (6, 7)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["class", "subclass", "object"])
+def test_a_matching_of_the_callers_own_is_asked(where, monkeypatch):
+    detector = _Scanned(lambda ids: "".join(WORDS[i] for i in ids))
+    tokens = torch.tensor([[0, 0, 0, 0, 0, 2, 6, 0]], device="cuda")
+    detector.given = [[4, 4, 6]]                               # "a)"
+    spans = [DocSpan(0, "", 0, 4, False, [], "a"), DocSpan(1, "", 4, 8, False, [], "b")]
+    assert CrossDocLinkMaskCreator(detector)(tokens, spans).link_bits is not None
+    calls = []
+
+    def nothing(self, links, doc_spans):
+        calls.append([tuple(link) for link in links])
+        return {}
+
+    kind = type("Own", (CrossDocLinkMaskCreator,), {"_match_links_to_docs": nothing}) if where == "subclass" else CrossDocLinkMaskCreator
+    if where == "class":
+        monkeypatch.setattr(CrossDocLinkMaskCreator, "_match_links_to_docs", nothing)
+    creator = kind(detector)
+    if where == "object":
+        creator._match_links_to_docs = nothing.__get__(creator)
+    assert creator(tokens, spans).link_bits is None and calls == [[(7, "a")]]

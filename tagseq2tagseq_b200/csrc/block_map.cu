@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(128) runs_kernel(PlanView P, MaskArgs M, int t
     const int per_word = (64 * M.W + 127) / 128, at = tb - P.NB;
     const int w = at / per_word, c = (at - w * per_word) * 128 + t;
     if (w >= t_words || c >= 64 * M.W) return;
-    const int64_t* link_b = M.link + (size_t)b * M.R * M.W + (c >> 6);
+    const int64_t* link_b = settled(M.link) + (size_t)b * M.R * M.W + (c >> 6);
     const int r0 = 64 * w, n = min(64, M.R - r0);
     unsigned long long out = 0ull;
 #pragma unroll 8

@@ -72,6 +72,28 @@ def test_scores_overwrite_the_probabilities_of_the_last_tile_once_their_product_
     assert re.match(r"[^{]*\{[^}]*mbar_wait\(&bar_gv\[i % Cfg::kDoStages\], \(i / Cfg::kDoStages\) & 1,[^}]*issue_st\(i \+ 1,", one_buffer)
 
 
+def _unsettled(text):
+    """Pointers that a kernel with a wait of its own for the launch before it reads through the read-only path without settled() behind that wait: its
+    __restrict__ parameters to constant memory, and what it passes to __ldg."""
+    bad = []
+    for kernel in re.finditer(r"__global__ void (?:__launch_bounds__\([^)]*\) )?(\w+)\((.*?)\) \{\n(.*?)\n\}", text, re.S):
+        name, params, body = kernel.groups()
+        wait = re.search(r"\bwait_previous\(\);", body)
+        if wait is None:  # the kernels inside a chain: what they read without having made it was complete before the chain
+            assert "after_previous();" in body, name
+            continue
+        pointers = set(re.findall(r"const \w+\* __restrict__ (\w+)", params)) | set(re.findall(r"__ldg\((?:reinterpret_cast<[^>]*>\()?&?(\w+)", body))
+        bad += [(name, p) for p in sorted(pointers) if not re.search(r"\b%s = settled\(" % p, body[wait.end():])]
+    return bad
+
+
+@pytest.mark.parametrize("name", ["adamw.cu", "block_map.cu", "link_scan.cu", "lm_fused.cu"])
+def test_read_only_loads_stay_behind_the_wait_for_the_launch_before(name):
+    """A read-only load whose address is known at the start may be moved up across the wait (the attention kernels' addresses come from what they load)."""
+    text = _source(name)
+    assert len(re.findall(r"__global__", text)) == len(re.findall(r"\b(?:wait|after)_previous\(\);", text)) and _unsettled(text) == []
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [64, 128])
 # pairs of query tiles; query tiles that two teams share, and those as the lists call for them, the entry one of either team's

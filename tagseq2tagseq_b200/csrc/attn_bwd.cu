@@ -254,6 +254,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint32_t* s_masks = reinterpret_cast<uint32_t*>(bars + Cfg::kBars + 2);  // [Q stages][kStretches][kMaskRuns] the tile's masks, by run of the key
   uint32_t* s_tile = s_masks + Cfg::kQStages * kStretches * kMaskRuns;  // [kTileSlots][2] a tile's four stretch entries, 16 bits each
   static_assert(Cfg::kTileSlots > Cfg::kQStages, "");
+  if (smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes) {  // a misplaced shared-memory window, the same in all CTAs: refused before anything is written there
+    if (threadIdx.x == 0) atomicCAS(p.plan.status, 0, 2900);
+    wait_previous();
+    return;
+  }
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PlanView& P = p.plan;
@@ -310,11 +315,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const int n = min(max(tiles, 0), NB - kb);  // query tiles to walk
-  // uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window
-  const int bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T ? 2901 : smem + Cfg::kTiles + Cfg::kSmall > smem_raw + Cfg::kBytes ? 2900 : 0;
+  const bool bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T;  // uniform across the grid: refuse a plan that was not built for this (B, T)
   if (bad || n == 0) {
     if (bad) {
-      if (tid == 0) atomicCAS(P.status, 0, bad);
+      if (tid == 0) atomicCAS(P.status, 0, 2901);
     } else if (tid < kTile) {
       const int kv = kb * kTile + tid;
       if (kv < P.T) {

@@ -909,6 +909,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   const FwdPlaces<D> at(smem_raw);
   const PlanView& P = p.plan;
+  if (at.smem + FwdSmem<D>::kSmall + FwdSmem<D>::kSmallBytes > at.raw + FwdSmem<D>::kBytes) {  // a misplaced shared-memory window, the same in all CTAs: refused before anything is written there
+    wait_previous();
+    if (threadIdx.x == 0) atomicCAS(P.status, 0, 1901);
+    return;
+  }
   const uint32_t tmem = fwd_setup<D>(at);
   if (threadIdx.x == 0) FTRACE_SPAN(0);
   // What came before in the stream ends under the lines above; the plan is read from here on.
@@ -921,13 +926,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   }
   const int magic = P.status[kStampMagic], plan_b = P.status[kStampB], plan_t = P.status[kStampT], longest = P.status[kLongestList], all = P.status[kAllLists];
   const bool share = kForm == kFwdShared || (kForm == kFwdByLists && lists_call_for_shared<D>(p, longest, all));
-  // Uniform across the grid: refuse a plan that was not built for this (B, T), or a misplaced shared-memory window.  A CTA without an item leaves
-  // behind that, because a plan that is refused must not keep a part of the count.
-  const int bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T ? 1900 : at.smem + FwdSmem<D>::kSmall + FwdSmem<D>::kSmallBytes > at.raw + FwdSmem<D>::kBytes ? 1901 : 0;
+  // Uniform across the grid: refuse a plan that was not built for this (B, T).  A CTA without an item leaves behind that, because a plan that is refused must not
+  // keep a part of the count.
+  const bool bad = magic != kPlanMagic || plan_b != P.B || plan_t != P.T;
   if (bad || static_cast<int>(blockIdx.x) >= (share ? p.n_tiles : p.n_pairs)) {
     if (threadIdx.x / 32 == kFwdIssuerWarp) tmem_dealloc(tmem, 512);
     if (threadIdx.x == 0) {
-      if (bad) atomicCAS(P.status, 0, bad);
+      if (bad) atomicCAS(P.status, 0, 1900);
       else fwd_leave(P);
     }
     return;

@@ -72,6 +72,13 @@ def test_scores_overwrite_the_probabilities_of_the_last_tile_once_their_product_
     assert re.match(r"[^{]*\{[^}]*mbar_wait\(&bar_gv\[i % Cfg::kDoStages\], \(i / Cfg::kDoStages\) & 1,[^}]*issue_st\(i \+ 1,", one_buffer)
 
 
+@pytest.mark.parametrize("name,code,uses", [("attn_fwd.cu", "1901", r"fwd_setup<D>\(at\)"), ("attn_bwd.cu", "2900", r"mbar_init\(|tmem_alloc\(")])
+def test_a_misplaced_shared_memory_window_is_refused_before_it_is_written(name, code, uses):
+    kernel = re.search(r"__global__ void __launch_bounds__\(\w+, 1\)\nattn_\w+_kernel\(.*?\n}", _source(name), re.S).group()
+    refused = re.search(r"atomicCAS\([\w.]*status, 0, %s\);(?:\s*wait_previous\(\);)?\s*return;" % code, kernel)
+    assert refused and refused.end() < re.search(uses, kernel).start() and "wait_previous();" in kernel[:refused.end()]
+
+
 def _unsettled(text):
     """Pointers that a kernel with a wait of its own for the launch before it reads through the read-only path without settled() behind that wait: its
     __restrict__ parameters to constant memory, and what it passes to __ldg."""

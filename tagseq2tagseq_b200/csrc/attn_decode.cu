@@ -133,8 +133,9 @@ __device__ __noinline__ void read_carefully(const DecodeParams& p, int qpos, flo
 }
 
 // kQueue: the warps of a block share one queue.  Otherwise each has at most kDecAtOnce groups and takes its own keys.
-template <int D, bool kQueue>
-__global__ void __launch_bounds__(kDecWarps * 32, 2) decode_kernel(const __grid_constant__ DecodeParams p) {
+// kPerSm: blocks an SM is to hold, which sets the registers; with two, 64 a thread, the loads of a batch wait for one another.
+template <int D, bool kQueue, int kPerSm>
+__global__ void __launch_bounds__(kDecWarps * 32, kPerSm) decode_kernel(const __grid_constant__ DecodeParams p) {
   constexpr int kLanes = D / 8;            // lanes that share a row
   constexpr int kRows = 32 / kLanes;       // rows a warp reads at once
   constexpr int kBatch = kRows * kUnroll;  // keys a warp takes off its queue at once
@@ -390,9 +391,15 @@ int launch_decode(const void* q, const void* k, const void* v, const int64_t* sq
   cfg.attrs = attrs;
   cfg.numAttrs = 2;
   const bool queue = groups > (long long)cs * kDecWarps * kDecAtOnce;
-  if (D == 128) return cudaLaunchKernelEx(&cfg, queue ? decode_kernel<128, true> : decode_kernel<128, false>, p) == cudaSuccess ? 0 : -141;
-  if (D == 64) return cudaLaunchKernelEx(&cfg, queue ? decode_kernel<64, true> : decode_kernel<64, false>, p) == cudaSuccess ? 0 : -141;
-  return -142;
+  // One block an SM where all blocks find a place that way: a cluster needs its SMs in one part of the chip, so 148 single blocks do, 128 in clusters of two or four, 96 of eight, but
+  // not 128 of eight.  us, two -> one: all keys of 16 x 1846, H = 8, D = 128 27.0 -> 24.8, 8 x 2000, H = 12 25.7 -> 22.9, 2 x 7723, H = 8 (four) 23.7 -> 21.5, linked 39109, H = 12,
+  // D = 64 (eight) 15.9 -> 14.8; beyond the lines all keys of 16 x 2000, H = 12, D = 128 35.8 -> 45.9, 32768, H = 16 (eight) 59.6 -> 83.3.
+  const bool alone = (long long)B * H * cs <= (cs == 1 ? 148 : cs < 8 ? 128 : 96);
+  using Kernel = void (*)(DecodeParams);
+  constexpr Kernel kernels[2][2][2] = {{{decode_kernel<64, false, 2>, decode_kernel<64, false, 1>}, {decode_kernel<64, true, 2>, decode_kernel<64, true, 1>}},
+                                       {{decode_kernel<128, false, 2>, decode_kernel<128, false, 1>}, {decode_kernel<128, true, 2>, decode_kernel<128, true, 1>}}};
+  if (D != 64 && D != 128) return -142;
+  return cudaLaunchKernelEx(&cfg, kernels[D == 128][queue][alone], p) == cudaSuccess ? 0 : -141;
 }
 
 }  // namespace ts2ts

@@ -59,3 +59,24 @@ def test_keys_without_weight_add_nothing_whatever_their_values(tk):
         want, want_lse = _reference(q[i], k[i], v[i], torch.ones(tk, dtype=torch.bool, device=dev), d)
         assert (out[i].double() - want).abs().max().item() <= 2 ** -8 * max(1.0, want.abs().max().item())
         assert (lse[i].double() - want_lse).abs().max().item() <= 1e-4
+
+
+# one block an SM or two: 148 blocks and 149, 128 in clusters of two and of four and a few more, 96 and 104 in clusters of eight; own keys and a shared queue
+@pytest.mark.parametrize("b,h,tk", [(4, 37, 1000), (1, 149, 1000), (4, 37, 2100), (1, 149, 2100), (4, 16, 3000), (5, 13, 3000), (2, 16, 7000), (3, 11, 7000), (1, 12, 17000), (1, 13, 17000), (1, 12, 33000), (1, 13, 33000)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_one_or_two_blocks_an_sm_give_the_same(b, h, tk, d):
+    from tagseq2tagseq_b200 import synth
+    from tagseq2tagseq_b200.attention import masked_attn_decode
+    dev = torch.device("cuda")
+    doc, link = synth.stack_packs([synth.make_pack(7 + i, tk, 300, 16, tk // 2, p_link=0.3) for i in range(b)])
+    doc, link = torch.from_numpy(doc).to(dev), torch.from_numpy(link).to(dev)
+    g = torch.Generator(device=dev).manual_seed(tk + d)
+    q = torch.randn(b, h, 1, d, device=dev, generator=g).bfloat16()
+    k, v = (torch.randn(b, h, tk, d, device=dev, generator=g).bfloat16() for _ in range(2))
+    out, lse = masked_attn_decode(q, k, v, doc, link)
+    for i in range(b):
+        ok = (doc[i] == doc[i, -1]) | ((link[i][doc[i, -1].long()][(doc[i] >> 6).long()] >> (doc[i] & 63).long()) & 1).bool()
+        want, want_lse = _reference(q[i], k[i], v[i], ok, d)
+        # one bf16 rounding of a mean of unit normals, fp32 sums of at most 33000 products
+        assert (out[i].double() - want).abs().max().item() <= 2 ** -8 * max(1.0, want.abs().max().item())
+        assert (lse[i].double() - want_lse).abs().max().item() <= 1e-4

@@ -890,16 +890,15 @@ __device__ __forceinline__ void fwd_items(const CUtensorMap& mapQ, const CUtenso
 enum FwdForm { kFwdPairs, kFwdShared, kFwdByLists };
 
 // Every CTA comes to the same answer, because it depends on the plan and the grid (one CTA per SM) alone.  As pairs a launch that is short of items takes as long
-// as its longest list, 2.0 us a tile and 2.2 us at its ends.  As shared tiles it takes an SM's share of all lists, two tiles at a time in 1.65 us (D = 64; 2.0 us at
-// D = 128, where two K/V streams do not fit the ring), and 2.7 us for each of the SM's items.  Shared tiles are taken where they come to less than 0.8 of the pairs'
-// time: of 85 random calls (T = 512 to 20000, 1 to 4 sequences, 2 to 16 heads, all kinds of masks) that picks the slower form by more than 4 % three times (6, 9 and
-// 10 %, all three H = 12, D = 64 just above one pair an SM: 2 x 2006, 2 x 1609, causal 4 x 731).  us, pairs | shared:
-// linked 14545, H = 3, D = 128 144 | 89; linked 5169, H = 8, D = 64 87 | 54; causal 4 x 3787, H = 3, D = 128 77 | 56; at the line linked 2 x 3156, H = 12, D = 64
-// 48.0 | 48.3 and 6273, H = 12, D = 128 92 | 91; beyond it linked 2 x 2455, H = 16, D = 64 46 | 50, causal 4 x 2902, H = 12, D = 64 101 | 108.
-// A kernel with both bodies runs either one 0 to 2.4 us slower than a kernel of its own.
+// as its longest list, 2.0 us a tile.  As shared tiles it takes an SM's share of all lists, two tiles at a time in 1.65 us (D = 64; 1.8 us at D = 128, where two K/V
+// streams do not fit the ring), and 3.2 us for each of the SM's items.  Shared tiles are taken where they come to less than 0.8 of the pairs' time: fitted to both forms
+// of 330 random calls with more tiles than SMs and up to four pairs an SM; of 330 others it takes a form that is slower by more than 4 % six times, by 16 % at most.
+// us, pairs | shared, each as a kernel of its own: linked 5133, H = 12, D = 128 63.6 | 52.3; 4 x 682, H = 12, D = 64 19.9 | 16.8; at the line documents 4 x 2639, H = 4, D = 64
+// 20.8 | 20.0 and linked 8 x 608, H = 6, D = 128 17.3 | 17.9; beyond it linked 2 x 1278, H = 16, D = 64 24.3 | 26.3 and 4 x 8154, H = 3, D = 128 91.8 | 99.4.
+// A kernel with both bodies runs the pairs 0.6 us slower than a kernel of its own, the shared tiles 1.2 us.
 template <int D>
 __device__ __forceinline__ bool lists_call_for_shared(const FwdParams& p, long long longest, long long all) {
-  return (D == 64 ? 33 : 40) * all * p.H + 108ll * p.n_tiles < gridDim.x * (64 * longest + 70);
+  return (D == 64 ? 33 : 36) * all * p.H + 126ll * p.n_tiles < gridDim.x * (64 * longest + 30);
 }
 
 template <int D, int kForm>

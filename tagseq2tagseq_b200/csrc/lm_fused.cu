@@ -80,35 +80,39 @@ __device__ __forceinline__ uint4 float_to_bf16x8(const float (&f)[8]) {
 }
 
 // ---------------------------------------------------------------------------------------------- residual add + RMSNorm
-// x_out = x_in + a (a may be null), h = x_out * rstd * w with rstd = 1 / sqrt(mean(x_out^2) + eps).  One block per row.
-template <int NV>  // float4 per thread and row: 1 when C <= 4 * blockDim.x, else kMaxVec
-__global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x_in, const __nv_bfloat16* __restrict__ a, const float* __restrict__ w,
-                                       float* x_out, __nv_bfloat16* __restrict__ h, float* __restrict__ rstd, int C, float eps) {
+// x_out = x_in + a (kAdd, or x_in alone), h = x_out * rstd * w with rstd = 1 / sqrt(mean(x_out^2) + eps).  One block per row.
+// With 32 registers two blocks of 1024 threads share an SM: with 40, for the loads of x_in and a of all four vectors at once, they do not (2100 x 16384 69 -> 86 us).
+template <int NV, bool kAdd>  // float4 per thread and row: 1 when C <= 4 * blockDim.x, else kMaxVec
+__global__ void __launch_bounds__(1024, 2) add_rmsnorm_fwd_kernel(const float* __restrict__ x_in, const __nv_bfloat16* __restrict__ a, const float* __restrict__ w,
+                                                                  float* x_out, __nv_bfloat16* __restrict__ h, float* __restrict__ rstd, int C, float eps) {
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * C;
   float4 v[NV];
-  uint2 d[NV];
   float ss = 0.f;
   wait_previous();
   x_in = settled(x_in); a = settled(a); w = settled(w);
+  auto load = [&](int c) { return *reinterpret_cast<const float4*>(x_in + base + c); };
+  if (!kAdd) {
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (threadIdx.x + i * blockDim.x) * 4;
-    if (c < C) {
-      v[i] = *reinterpret_cast<const float4*>(x_in + base + c);
-      d[i] = a != nullptr ? *reinterpret_cast<const uint2*>(a + base + c) : make_uint2(0u, 0u);
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
+      if (c < C) v[i] = load(c);
     }
   }
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (threadIdx.x + i * blockDim.x) * 4;
     if (c < C) {
-      float4& x = v[i];
-      if (a != nullptr) {
-        const float4 f = bf16x4_to_float4(d[i]);
+      float4 x;
+      if (kAdd) {
+        x = load(c);
+        const float4 f = bf16x4_to_float4(*reinterpret_cast<const uint2*>(a + base + c));
         x.x += f.x; x.y += f.y; x.z += f.z; x.w += f.w;
+      } else {
+        x = v[i];
       }
       *reinterpret_cast<float4*>(x_out + base + c) = x;
+      v[i] = x;
       ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
     }
   }
@@ -755,11 +759,9 @@ int norm_threads(int C) {
 cudaError_t launch_add_rmsnorm_fwd(const float* x_in, const void* a, const float* w, float* x_out, void* h, float* rstd, int N, int C,
                                    float eps, cudaStream_t stream) {
   const int threads = norm_threads(C);
-  if (C <= 4 * threads)
-    return launch_after(add_rmsnorm_fwd_kernel<1>, dim3(N), threads, 0, stream, x_in, static_cast<const __nv_bfloat16*>(a), w, x_out,
-                        static_cast<__nv_bfloat16*>(h), rstd, C, eps);
-  return launch_after(add_rmsnorm_fwd_kernel<kMaxVec>, dim3(N), threads, 0, stream, x_in, static_cast<const __nv_bfloat16*>(a), w, x_out,
-                      static_cast<__nv_bfloat16*>(h), rstd, C, eps);
+  const auto kernel = C <= 4 * threads ? a != nullptr ? add_rmsnorm_fwd_kernel<1, true> : add_rmsnorm_fwd_kernel<1, false>
+                                       : a != nullptr ? add_rmsnorm_fwd_kernel<kMaxVec, true> : add_rmsnorm_fwd_kernel<kMaxVec, false>;
+  return launch_after(kernel, dim3(N), threads, 0, stream, x_in, static_cast<const __nv_bfloat16*>(a), w, x_out, static_cast<__nv_bfloat16*>(h), rstd, C, eps);
 }
 
 // Blocks of the backward kernel = rows of its dw_part workspace.

@@ -600,8 +600,8 @@ __global__ void __launch_bounds__(256) scale_to_bf16_kernel(const float* __restr
 // the ids v with v % kEmbBuckets == bucket: it reads all of idx, 8 bytes a token from L2, and queues its tokens in
 // ascending order; a warp then adds up one id's rows at a time.  Ids of more than kEmbHeavy queued rows are shared by the
 // block: each warp takes a stretch of the queue, and the sixteen partial rows are added in order.  dw is zeroed before.
-// HBM-bound (dx read once, dw written twice at most).  Pass with its memset, uniform ids into 50304 rows: 73 us at
-// 16384 x 768, 218 us at 32768 x 2048 (atomics in the order of arrival 51 and 181 us; torch's kernel, which sorts the
+// HBM-bound (dx read once, dw written twice at most).  Pass with its memset, uniform ids into 50304 rows: 69 us at
+// 16384 x 768, 208 us at 32768 x 2048 (atomics in the order of arrival 51 and 181 us; torch's kernel, which sorts the
 // tokens, 371 and 1317 us).  One id for all tokens is the worst case, 700 us at 16384 x 768.
 constexpr int kEmbBuckets = 256, kEmbThreads = 512, kEmbWarps = kEmbThreads / 32, kEmbEach = 4, kEmbStep = kEmbEach * kEmbThreads;
 constexpr int kEmbList = kEmbStep + 1024, kEmbVec = 4, kEmbCols = 128 * kEmbVec, kEmbHeavy = 64;
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(kEmbThreads) embedding_bwd_kernel(const int64_
   int count = 0;                                     // queued tokens, the same in every thread
   bool first = true;                                 // nothing of this block's rows written yet
   wait_previous();
-  idx = settled(idx); dx = settled(dx);
+  idx = settled(idx);  // where dx is read depends on it; dx settled, too, cost registers (spills: 32768 x 2048 207 -> 231 us)
 
   // sum of the queued rows of `id` between two places of the queue, `kVecs` vectors a lane from vector `from` on
   auto sum_rows = [&](auto vecs, int id, int begin, int end, int from, float4* acc) {

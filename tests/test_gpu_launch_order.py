@@ -55,3 +55,63 @@ def test_dependent_calls_back_to_back(n, c):
                 assert torch.equal(a, b), (i, k)
             else:                                             # dq of the attention is added up in the order of arrival, in fp32, and rounded to bf16
                 assert (a - b).norm() <= 2 ** -9 * b.norm()
+
+
+def _step(inputs, wait):
+    """What a training loop has follow one another: tokens and targets written on the device, the mask from them, a head with a scaled loss, its gradients copied, an optimizer
+    step on them and the weights' copies for the next."""
+    from tagseq2tagseq_b200 import CrossDocLinkMaskCreator, DocSpan
+    from tagseq2tagseq_b200.link_detect import MarkdownLinkDetector
+    from tagseq2tagseq_b200.lm_fused import AdamW, Linear, cast_weights, copy_tensors, embedding, head_loss
+    plain, link_at, h, weight = inputs
+    n, v = plain.numel(), weight.shape[0]
+    text = {1: "[", 2: "](", 3: ")"}
+    detector = MarkdownLinkDetector(lambda ids: "".join(text.get(i, "w%d" % i) for i in ids), window_tokens=8, link_start_token_ids=(1,), link_mid_token_id=2, vocab_size=64)
+    spans = [DocSpan(i, "", i * n // 4, (i + 1) * n // 4, False, [], "w%d" % (10 + i)) for i in range(4)]
+    creator = CrossDocLinkMaskCreator(detector)
+    with torch.device(plain.device):
+        head = Linear(h.shape[1], v)
+        table = torch.nn.Parameter(weight[:64].clone())
+    with torch.no_grad():
+        head.weight.copy_(weight)
+    opt = AdamW([head.weight, table], lr=0.1)
+    copies, out = [c for c in cast_weights([head.weight, table])], []
+
+    def done(*ts):
+        if wait:
+            torch.cuda.synchronize()
+        out.extend(t.detach().clone() for t in ts)
+
+    for step in range(3):
+        tokens = plain.clone()
+        for k, tok in enumerate((1, 20, 2, 10 + step % 3, 3)):   # a link in the last document, written just before the scan
+            tokens[link_at + k] = tok
+        spec = creator(tokens[None], spans)
+        done(spec.doc_ids, *(t for t in (spec.link_bits, spec.q_row_ids, spec.kv_col_ids) if t is not None), spec.block_map(with_lists=True).state)
+        x = (h + embedding(table, tokens).repeat(1, h.shape[1] // table.shape[1])).bfloat16()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            loss = head_loss(x, head.weight, tokens, copies[0])
+        done(loss)
+        grads = torch.autograd.grad(3.0 * loss, (head.weight, table))
+        kept = [torch.empty_like(g) for g in grads]
+        copy_tensors(kept, grads)
+        del grads                                                # their memory is the next allocation's
+        head.weight.grad, table.grad = kept
+        opt.step()
+        copies = cast_weights([head.weight, table])
+        done(*kept, head.weight, table, *copies)
+    return out
+
+
+@pytest.mark.parametrize("n,c,v", [(64, 64, 64), (1000, 256, 4096), (5000, 128, 1024)])
+def test_a_loop_of_steps_back_to_back(n, c, v):
+    dev, sets = torch.device("cuda"), []
+    for seed in range(2):
+        g = torch.Generator(device=dev).manual_seed(10 + seed)
+        weight = torch.randn(v, c, device=dev, generator=g) * 0.05
+        sets.append((torch.randint(20, 60, (n,), device=dev, generator=g), n - 8, torch.randn(n, c, device=dev, generator=g), weight))
+    want = [_step(s, True) for s in sets]
+    torch.cuda.synchronize()
+    for i in range(6):
+        for k, (a, b) in enumerate(zip(_step(sets[i % 2], False), want[i % 2], strict=True)):
+            assert torch.equal(a, b), (i, k)

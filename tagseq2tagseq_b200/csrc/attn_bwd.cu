@@ -855,12 +855,10 @@ static int launch_bwd_t(const void* q, const void* k, const void* v, const void*
     p.head_group = (int)(g < 1 ? 1 : (g > H ? H : g));
   }
   BTRACE_ATTACH(p, stream);
-  // The main kernel's blocks set themselves up and bring in K and V under the preparation where the launches are short.  us, one after the other -> overlapping: documents
-  // 2048, H = 8, D = 64 19.2 -> 17.4; linked 1024, H = 4, D = 64 22.4 -> 21.1; causal 1024, H = 4, D = 128 28.2 -> 26.7; causal 4096, H = 4, D = 128 82.8 -> 80.9; linked 5003, H = 12,
-  // D = 64 63.9 -> 62.5; 2 x 1771, H = 12, D = 128 64.6 -> 63.6.  Beyond 384 tiles at D = 128 and 768 at D = 64 the gain ends and long launches lose: linked 8k, H = 12, D = 64 (768 tiles)
-  // 91.5 -> 93.6.  Between one tile an SM and that line it goes either way by 1 to 4 %: at D = 128 documents 2 x 2600, H = 8 59.8 -> 57.4, 6144, H = 8 67.0 -> 65.8, causal 4096,
-  // H = 10 126.3 -> 124.8, but linked 4096, H = 7 83.0 -> 86.9 and H = 12 87.0 -> 89.3, 2 x 6767, H = 2 85.4 -> 88.0; at D = 64 linked 6144, H = 12 99.5 -> 102.8.  The conversion does not start under the main kernel: its blocks would wait where SMs
-  // have run dry, but a trigger in the main kernel costs more (the first five of the calls above 18.0, 21.2, 27.2, 82.2, 63.6; linked 16k, H = 16, D = 128 961 -> 982, H = 12, D = 64 441 -> 458).
+  // The main kernel's blocks set themselves up and bring in K and V under the preparation where the launches are short.  us, one after the other -> overlapping: linked 1024,
+  // H = 4, D = 64 22.4 -> 21.1; causal 1024, H = 4, D = 128 28.2 -> 26.7.  Between one tile an SM and the line it goes either way by 1 to 4 % (D = 128, documents 2 x 2600, H = 8
+  // 59.8 -> 57.4, linked 4096, H = 7 83.0 -> 86.9); beyond 384 tiles at D = 128 and 768 at D = 64 launches lose (linked 8k, H = 12, D = 64, 768 tiles 91.5 -> 93.6).
+  // The conversion does not start under the main kernel: a trigger there costs more than it gives (linked 5003, H = 12, D = 64 62.5 -> 63.6, 16k, H = 16, D = 128 961 -> 982).
   const bool early = (long long)B * H * P.NB * D <= 384 * 128;
   cudaError_t launched = launch_after(bwd_prep_kernel<D>, dim3((unsigned)(rows / kPrepRows)), 256, 0, stream, static_cast<const __nv_bfloat16*>(out),
                                       static_cast<const __nv_bfloat16*>(dout), lse, so[0], so[1], so[2], sdo[0], sdo[1], sdo[2], H, T, Tp, stats, dq_acc, early);

@@ -7,7 +7,8 @@
 // A kernel touches no memory that another launch may have written or may still read before it has waited, and waits in at least one
 // thread of every block, so that a kernel's end implies the end of all before it.  The first kernel of a chain (pre-pass, backward) calls let_next_start()
 // behind its own wait: all that came before the chain has ended when its later kernels start, and these wait for what the chain itself has written.
-// What may have been written just before is read with plain loads, bulk copies or through settled(): a read-only load could be moved up across the wait.
+// What may have been written just before is read with plain loads, bulk copies, through settled() or at addresses that come from such loads: another read-only load could be
+// moved up across the wait.
 #pragma once
 #include <cuda_runtime.h>
 

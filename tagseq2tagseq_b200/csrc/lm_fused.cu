@@ -450,7 +450,8 @@ __global__ void ce_bwd_kernel(__nv_bfloat16* logits, const int64_t* __restrict__
 // instead of the 6 of the two kernels above; two blocks of a 50304-logit row share an SM, so that one's copy overlaps the
 // other's arithmetic.  The gradient is that of the mean loss (times inv_n, not times what reaches the loss from above).
 // What is left beside the copy are two exponentials a logit: maxima are taken of bf16 pairs, four vectors of a thread between two looks at the
-// running one, difference and scale are packed, only the target's vector knows of it.  A block has as many threads as leave each 8 to 16 vectors (12 to 27 from 4096 vectors on).
+// running one, difference and scale are packed, only the target's vector knows of it.  A row of up to 1024 vectors of eight has 64 threads (up to 16 vectors each), up to 2048
+// 128, up to 4096 256 (8 to 16 each), beyond 512 (8 to 27).
 // us (floor at the copy rate; one comparison and a maximum a logit, 512 threads whatever the row -> now): 16384 x 50304 (504) 650 -> 557, x 32768 (328) 422 -> 338,
 // x 16384 (164) 235 -> 167, x 4096 (41) 120 -> 50; 1024 x 4096 (3) 15.8 -> 12.8.  512 threads for x 32768 343, 256 for x 50304 574.
 constexpr int kCeRowBytes = 216 * 1024;

@@ -73,6 +73,11 @@ def cross_entropy(logits: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     return _call(_lib.ops().cross_entropy.default, logits, target)
 
 
+def one_pass_head(vocab: int, width: int) -> bool:
+    """Whether the loss of a head of this size is the one-pass kernel's, which takes a copy of the weight."""
+    return vocab % 8 == 0 and vocab <= _MAX_HEAD_COLUMNS and width % 8 == 0
+
+
 def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor, copy: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Mean cross-entropy of the output head ``h @ weight.T`` against ``target``; the logits never leave this call.  ``copy``: what
     ``cast_weights`` made of the weight as it is now, for a caller that has it; its values are not looked at, and the gradient is the weight's."""
@@ -81,7 +86,7 @@ def head_loss(h: torch.Tensor, weight: torch.Tensor, target: torch.Tensor, copy:
     _need_cuda(h, weight, target)
     V = weight.shape[0]
     if (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad) and h.dtype == torch.bfloat16 and weight.dtype == torch.float32
-            and V % 8 == 0 and V <= _MAX_HEAD_COLUMNS and h.shape[-1] % 8 == 0):
+            and one_pass_head(V, h.shape[-1])):
         return _call(_lib.ops().head_loss.default, h, weight, target, copy)
     logits = F.linear(h, weight.to(h.dtype))
     return cross_entropy(logits.to(torch.bfloat16).view(-1, V), target.reshape(-1))

@@ -24,7 +24,7 @@ import torch.nn.modules.module as _module
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 
-from .lm_fused import AdamW, Linear, add_rmsnorm, cast_weights, copy_tensors, cross_entropy, embedding, head_loss, qkv_attention, rope_half_tables, swiglu, transformed
+from .lm_fused import AdamW, Linear, add_rmsnorm, cast_weights, copy_tensors, cross_entropy, embedding, head_loss, one_pass_head, qkv_attention, rope_half_tables, swiglu, transformed
 from .mask_spec import MaskSpec
 
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what nn.RMSNorm uses for fp32 input when eps is None
@@ -147,8 +147,8 @@ class DecoderLM(nn.Module):
         return tables
 
     def _weight_copies(self):
-        """The bf16 copies that this forward's linear layers keep for their backward, ((copy,), ...) by layer and then the head's, made in one launch.  None
-        where a layer would not take one, or somebody's code could look at a weight, or change it, on the way."""
+        """The bf16 copies that this forward's linear layers keep for their backward, ((copy,), ...) by layer and then the head's (() where its loss takes none), made in
+        one launch.  None where a layer would not take one, or somebody's code could look at a weight, or change it, on the way."""
         layers = [m for blk in self.blocks if _plain(blk, Block) for m in blk.linears()] + [self.head]
         if (len(layers) != 4 * len(self.blocks) + 1 or torch.compiler.is_compiling() or not torch.is_grad_enabled() or _observed()
                 or not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") != torch.bfloat16
@@ -161,7 +161,8 @@ class DecoderLM(nn.Module):
         # Frozen weights below the first one that learns are kept by nobody.
         if not (weights[0].requires_grad or getattr(getattr(self.embed, "weight", None), "requires_grad", False)):
             return None
-        return [(c,) for c in cast_weights(weights)]
+        head = one_pass_head(*weights[-1].shape)
+        return [(c,) for c in cast_weights(weights if head else weights[:-1])] + ([] if head else [()])
 
     def forward(self, tokens: torch.Tensor, mask: MaskSpec, rope=None) -> torch.Tensor:
         """tokens int64 [B, T+1]; returns the mean next-token cross-entropy (training_module.py:195-211).  Runs under

@@ -178,3 +178,16 @@ def test_a_copy_is_bf16_of_the_weights_size_and_without_a_gradient():
                 head_loss(x, layer.weight, target, bad)
     head_loss(x, layer.weight, target, good).backward()
     assert layer.weight.grad is not None and good.grad is None
+
+
+@pytest.mark.parametrize("vocab", [4096, 110592, 110600])
+def test_a_head_whose_loss_takes_no_copy_gets_none(vocab):
+    """The head's loss in two kernels (rows that do not fit shared memory) converts the weight itself."""
+    model, run = _small(vocab)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        copies = model._weight_copies()
+    assert len(copies) == 9 and [len(c) for c in copies] == [1] * 8 + [int(vocab <= 110592)]
+    want = run()
+    model.blocks[1].proj.register_forward_pre_hook(lambda m, a: None)
+    for a, b in zip(run(), want):
+        assert torch.equal(a, b)
